@@ -1203,13 +1203,14 @@ int dispatch_dvc(int dvc, const void* q, const PagedKV& c, const int32_t* cu_q, 
 
 using namespace cvllm;
 
-// prefill_attn_bias.cu: the tcgen05 / TMEM / TMA pipeline for 16-bit storage, D = Dv = 128, pages of a multiple of 128
-// rows and an even number of query heads per KV head
+// prefill_attn_bias.cu: the tcgen05 / TMEM / TMA pipeline for portions
+bool cvllm_prefill_bias_serves(int D, int Dv, int page_size, int dist_rows);
 int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows, void* out,
                               const int32_t* seq_start, const float* slopes, const int32_t* page_table,
-                              const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ, int HKV,
+                              const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ, int HKV, int HD,
                               int PS, int NLP, int max_seqlen_q, float scale, int chunk, int window, int keep, int sink,
-                              const float* sink_logits, int64_t o_stride, cudaStream_t st);
+                              const float* sink_logits, const float* dist_bias, int dist_rows, int64_t o_stride,
+                              cudaStream_t st);
 
 // latent_attn_umma.cu: tcgen05 / TMEM / TMA for one key/value head whose values are columns of its key rows, 16-bit
 bool cvllm_latent_attn_umma_serves(int D, int Dv, int page_size, int64_t out_stride, const void* q, const void* cache,
@@ -1378,12 +1379,16 @@ extern "C" int cvllm_bias_attn_varlen_dist(const void* q, const void* k_cache, c
                              out_stride, B, max_new, H, G, D, Dv, st)
   // 0 product, 1 fp32 FMA kernel, 2 no tcgen05 kernel, 3 the latent tcgen05 kernel wherever it serves
   const int path = test_options().bias_attn_fma.load();
-  if (dtype == CVLLM_BF16 && D == 128 && Dv == 128 && v_stride == Dv && page_size % 128 == 0 && (H / G) % 2 == 0 &&
-      path == 0 && dist_bias == nullptr && out_stride % 8 == 0 &&
+  // (buffers off the 16-byte grid: whole tiles of 128-wide heads refuse them, the shapes around those take mma.sync)
+  if (dtype == CVLLM_BF16 && cvllm_prefill_bias_serves(D, Dv, page_size, dist_bias ? dist_rows : 0) && v_stride == Dv &&
+      (H / G) % 2 == 0 && path == 0 && out_stride % 8 == 0 &&
+      ((D == 128 && page_size % 128 == 0 && dist_bias == nullptr) ||
+       (aligned16(q) && aligned16(out) && aligned16(k_cache) && aligned16(v_cache))) &&
       table_stride_head == pages_per_head && table_stride_slot == (int64_t)G * pages_per_head && cache_rows > 0)
     return cvllm_launch_prefill_bias(q, k_cache, v_cache, cache_rows, out, seq_start, slopes, page_table,
-                                     batch_mapping, cu_seqlens_q, B, total_tokens, H, G, page_size, pages_per_head,
-                                     max_new, scale, chunk, window, keep_first, sink, sink_logits, out_stride, st);
+                                     batch_mapping, cu_seqlens_q, B, total_tokens, H, G, D, page_size, pages_per_head,
+                                     max_new, scale, chunk, window, keep_first, sink, sink_logits, dist_bias, dist_rows,
+                                     out_stride, st);
   // latent rows that the pipeline above has not taken
   if (dtype == CVLLM_BF16 && G == 1 && v_cache == k_cache && v_stride == D && slopes == nullptr && dist_bias == nullptr &&
       cache_rows > 0 && (path == 0 || path == 3) &&

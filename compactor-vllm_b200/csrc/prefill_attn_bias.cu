@@ -1,13 +1,20 @@
-// Attention with a distance bias, a chunk mask and a softmax sink on the tcgen05 pipeline of prefill_attn2.cu, for the
-// case that pipeline serves: 16-bit storage, key and value size 128, pages that are multiples of 128 rows, an even
-// number of query heads per KV head.  Same roles (warps 0-7 softmax of two heads, warp 8 TMA producer, warp 9 UMMA
+// Attention with a distance bias, a chunk mask and a softmax sink on the tcgen05 pipeline of prefill_attn2.cu: bfloat16
+// storage, key and value size 128 or 64, pages of 16, 32, 64 or a multiple of 128 rows, an even number of query heads per
+// KV head.  Same roles (warps 0-7 softmax of two heads, warp 8 TMA producer, warp 9 UMMA
 // issuer), same ring of five 32 KB slots, same TMEM layout and hand-offs; what differs:
 //   * every key - the step's own tokens included - is already in the paged cache, so all K / V tiles are cache tiles
 //     [128 j, 128 j + 127] of the sequence and the causal mask is positional: key position <= query position;
 //   * tiles before the chunk (or the sliding window) of the query tile's first row are never loaded: the tile list is
 //     the tiles that hold kept first tokens, if any, then the tiles from j_begin on;
 //   * the softmax adds slope * (key position - query position) in log2 units to the scaled logits, masks keys outside
-//     the row's chunk or window (the kept first tokens stay visible), and starts from (max 0, sum 1) when there is a sink.
+//     the row's chunk or window (the kept first tokens stay visible), and starts from (max 0, sum 1) when there is a sink;
+//   * a learned bias per distance (DIST) comes out of shared memory: the two heads' columns of the table lie there in
+//     log2 units with the slope's part added, so a row reads its 128 biases of a tile at consecutive addresses (and
+//     the 32 rows of a warp 32 neighbouring words); tiles wholly beyond the table add one constant.  With heads of 128 the
+//     ring gives up one of its five slots for the table.  One 4096-token portion, 32 / 8 heads of 128, window 1024, a table
+//     of 1024 rows, with the q / k norms and the cache write: 725 us on mma.sync, 154 us here;
+//   * pages shorter than a tile arrive in pieces of a page each; pieces past the last query's page are not loaded (the same
+//     portion without a window: pages of 64 1294 -> 214 us, heads of 64 601 -> 183 us).
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -16,13 +23,15 @@
 namespace cvllm {
 
 namespace pb {
-constexpr int kBM = 128, kBN = 128, kHD = 128;
-constexpr int kSlots = 5;
-constexpr int kTileBytes = kBN * kHD * 2;  // 32 KB
-constexpr int kBoxBytes = kTileBytes / 2;  // one [128 x 64] swizzled box
+constexpr int kBM = 128, kBN = 128;
+constexpr int kBoxBytes = kBN * 64 * 2;    // one [128 x 64] swizzled box
+// distances -kTabFront .. rows - 1 + kTabBack of a bias table lie in shared memory: a tile's rows and columns reach 254
+// before distance 0 (masked) and, unless the whole tile is past the table, 254 beyond its last row (which they repeat)
+constexpr int kTabFront = 256, kTabBack = 256, kTab = 4096;
+constexpr int kMaxDistRows = kTab - kTabFront - kTabBack;
 constexpr int kThreads = 384;              // 3 warpgroups
 constexpr int kRegsSoftmax = 224, kRegsOther = 56;  // 2*128*224 + 128*56 = 64512 <= 65536
-}  // namespace p2
+}  // namespace pb
 
 struct PrefillBiasParams {
   void* out;
@@ -40,13 +49,19 @@ struct PrefillBiasParams {
   int keep;                   // the sequence's first positions that stay visible whatever window and chunk say
   float sink;                 // 1 = a sink in the denominator, 0 = none
   const float* sink_logits;   // [HQ] the sink's score per head, or NULL (score 0)
+  const float* dist_bias;     // [dist_rows][HQ] added to the score by distance (the last row beyond), DIST only
+  int dist_rows;
 };
 
+template <int HD, bool DIST>
 struct PrefillBiasSmem {
-  unsigned char q[2][pb::kTileBytes];
-  unsigned char kv[pb::kSlots][pb::kTileBytes];
+  static constexpr int kTileBytes = pb::kBN * HD * 2;
+  static constexpr int kSlots = HD == 128 && DIST ? 4 : 5;
+  unsigned char q[2][kTileBytes];
+  unsigned char kv[kSlots][kTileBytes];
+  float table[DIST ? 2 : 1][DIST ? pb::kTab : 4];
   uint64_t q_full;
-  uint64_t full[pb::kSlots], empty[pb::kSlots];
+  uint64_t full[kSlots], empty[kSlots];
   uint64_t s_full[2], p_full[2];
   uint64_t p_half[2];   // P of the tile's first 64 keys is in TMEM: the PV UMMAs of those keys may start
   uint64_t o_done[2];   // one phase per PV_t(i)
@@ -98,14 +113,16 @@ __device__ long long g_pb_trace[8][256];
 #define P2_TRACE(rowi, jj) do { } while (0)
 #endif
 
-template <bool BF16>
+template <int kHD, bool DIST>
 __global__ void __launch_bounds__(pb::kThreads, 1)
 prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kc,
                          const __grid_constant__ CUtensorMap tm_vc, const PrefillBiasParams p) {
   using namespace pb;
+  using Smem = PrefillBiasSmem<kHD, DIST>;
+  constexpr bool BF16 = true;
+  constexpr int kSlots = Smem::kSlots, kTileBytes = Smem::kTileBytes, kBoxes = kHD / 64;
   extern __shared__ unsigned char smem_raw[];
-  PrefillBiasSmem& sm = *reinterpret_cast<PrefillBiasSmem*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.z;
@@ -157,6 +174,17 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     tma_prefetch_desc(&tm_kc);
     tma_prefetch_desc(&tm_vc);
   }
+  if constexpr (DIST) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const float slope = p.slopes ? p.slopes[hq0 + t] : 0.f;
+      for (int i = threadIdx.x; i < p.dist_rows + kTabFront + kTabBack; i += kThreads) {
+        const int n = i - kTabFront;
+        const float r = p.dist_bias[(int64_t)min(max(n, 0), p.dist_rows - 1) * p.HQ + hq0 + t];
+        sm.table[t][i] = (r - slope * (float)n) * 1.4426950408889634f;
+      }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -168,10 +196,11 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     if (lane == 0) {
       mbar_expect_tx(&sm.q_full, 2 * kTileBytes);
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        tma_load_3d(sm.q[t], &tm_q, &sm.q_full, 0, hq0 + t, q_beg + q0);
-        tma_load_3d(sm.q[t] + kBoxBytes, &tm_q, &sm.q_full, 64, hq0 + t, q_beg + q0);
-      }
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int x = 0; x < kBoxes; ++x)
+          tma_load_3d(sm.q[t] + x * kBoxBytes, &tm_q, &sm.q_full, 64 * x, hq0 + t, q_beg + q0);
+      const int piece = min(p.PS, kBN), last_page = p_last / p.PS;   // rows of a box
       const int32_t* pt = p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + hkv) * p.NLP;
       for (int n = 0; n < 2 * n_tiles; ++n) {
         const int j = n >> 1;
@@ -180,17 +209,21 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const uint32_t ph = (n / kSlots) & 1;
         const int t0 = tile_base(j);
         const int pg = t0 / p.PS;
-        const int row = pt[pg] * p.PS + (t0 - pg * p.PS);
         mbar_wait(&sm.empty[slot], ph ^ 1);
 #ifdef CVLLM_PROBE_NO_TMA  // timing probe only (wrong results): K / V tiles are never fetched
         mbar_arrive(&sm.full[slot]);
         continue;
 #endif
-        mbar_expect_tx(&sm.full[slot], kTileBytes);
         unsigned char* dst = sm.kv[slot];
         const CUtensorMap* m = is_v ? &tm_vc : &tm_kc;
-        tma_load_2d(dst, m, &sm.full[slot], 0, row);
-        tma_load_2d(dst + kBoxBytes, m, &sm.full[slot], 64, row);
+        const int pieces = min(kBN / piece, last_page - pg + 1);
+        mbar_expect_tx(&sm.full[slot], pieces * piece * kHD * 2);
+        for (int i = 0; i < pieces; ++i) {
+          const int row = pt[pg + i] * p.PS + (t0 - pg * p.PS);   // the offset is 0 in pages shorter than a tile
+#pragma unroll
+          for (int x = 0; x < kBoxes; ++x)
+            tma_load_2d(dst + x * kBoxBytes + i * piece * 128, m, &sm.full[slot], 64 * x, row);
+        }
       }
     }
   } else if (warp == 9) {
@@ -261,8 +294,8 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const int valid = last_valid;
         uint4* v4 = reinterpret_cast<uint4*>(sm.kv[slot_of(n)]);
         const uint4 z = make_uint4(0, 0, 0, 0);
-        for (int idx = lane; idx < (kBN - valid) * 16; idx += 32) {
-          const int r = valid + idx / 16, c = idx % 16;  // 16 x 16B per row across the 2 boxes
+        for (int idx = lane; idx < (kBN - valid) * 8 * kBoxes; idx += 32) {
+          const int r = valid + idx / (8 * kBoxes), c = idx % (8 * kBoxes);  // 8 x 16B per row and box
           v4[(c >> 3) * (kBoxBytes / 16) + r * 8 + (c & 7)] = z;
         }
         fence_proxy_async_smem();
@@ -310,6 +343,8 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const int lo_i = first_key(pi);
     const int lo_max = first_key(p_last);
     const float slope2 = p.slopes ? p.slopes[hq0 + t] * 1.4426950408889634f : 0.f;
+    // what the table's last row adds to every score beyond it
+    const float far_bias = DIST ? p.dist_bias[(int64_t)(p.dist_rows - 1) * p.HQ + hq0 + t] * 1.4426950408889634f : 0.f;
 
     for (int j = 0; j < n_tiles; ++j) {
       mbar_wait(&sm.s_full[t], j & 1);
@@ -336,14 +371,29 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       const int base = tile_base(j);
       {
         const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), sl2 = make_float2(slope2, slope2);
-        const float off = slope2 * (float)(base - pi);
-        const float2 off2 = make_float2(off, off);
+        bool table = false;
+        float off = slope2 * (float)(base - pi);
+        if constexpr (DIST) {
+          table = p0 - base - (kBN - 1) < p.dist_rows - 1;   // some row of the tile has a distance inside the table
+          off += far_bias;
+        }
+        if (DIST && table) {
+          const float* tb = sm.table[t] + kTabFront + (pi - base);
 #pragma unroll
-        for (int c = 0; c < kBN; c += 2) {
-          const float2 bias = __ffma2_rn(make_float2((float)c, (float)(c + 1)), sl2, off2);
-          const float2 v = __ffma2_rn(make_float2(s[c], s[c + 1]), sc2, bias);
-          s[c] = v.x;
-          s[c + 1] = v.y;
+          for (int c = 0; c < kBN; c += 2) {
+            const float2 v = __ffma2_rn(make_float2(s[c], s[c + 1]), sc2, make_float2(tb[-c], tb[-c - 1]));
+            s[c] = v.x;
+            s[c + 1] = v.y;
+          }
+        } else {
+          const float2 off2 = make_float2(off, off);
+#pragma unroll
+          for (int c = 0; c < kBN; c += 2) {
+            const float2 bias = __ffma2_rn(make_float2((float)c, (float)(c + 1)), sl2, off2);
+            const float2 v = __ffma2_rn(make_float2(s[c], s[c + 1]), sc2, bias);
+            s[c] = v.x;
+            s[c + 1] = v.y;
+          }
         }
       }
       // ---- masks (boundary tiles only): keys after the query, keys before the row's chunk or window ----
@@ -484,24 +534,48 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
 using namespace cvllm;
 
+// What the kernel serves, beside bfloat16 storage, an even number of query heads per KV head and contiguous page tables.
+bool cvllm_prefill_bias_serves(int D, int Dv, int page_size, int dist_rows) {
+  return D == Dv && (D == 128 || D == 64) &&
+         (page_size % 128 == 0 || page_size == 64 || page_size == 32 || page_size == 16) && dist_rows <= pb::kMaxDistRows;
+}
+
+namespace {
+
+template <int HD, bool DIST>
+int launch_bias(const CUtensorMap& tm_q, const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, const PrefillBiasParams& p,
+                int max_seqlen_q, cudaStream_t st) {
+  const size_t smem = sizeof(PrefillBiasSmem<HD, DIST>) + 1024;
+  static_assert(sizeof(PrefillBiasSmem<HD, DIST>) + 1024 <= 227 * 1024, "shared memory");
+  const dim3 grid((max_seqlen_q + pb::kBM - 1) / pb::kBM, p.HQ / 2, p.B);
+  static std::atomic<uint64_t> attr{0};
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn_bias_kernel<HD, DIST>, (int)smem, attr));
+  prefill_attn_bias_kernel<HD, DIST><<<grid, pb::kThreads, smem, st>>>(tm_q, tm_kc, tm_vc, p);
+  CVLLM_CHECK_LAUNCH();
+  return CVLLM_OK;
+}
+
+}  // namespace
+
 // Launch.  Called by cvllm_bias_attn_varlen (bias_attn.cu) for the shapes named at the top; returns a CVLLM_* code.
 int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows, void* out,
                               const int32_t* seq_start, const float* slopes, const int32_t* page_table,
-                              const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ, int HKV,
+                              const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ, int HKV, int HD,
                               int PS, int NLP, int max_seqlen_q, float scale, int chunk, int window, int keep, int sink,
-                              const float* sink_logits, int64_t o_stride, cudaStream_t st) {
+                              const float* sink_logits, const float* dist_bias, int dist_rows, int64_t o_stride,
+                              cudaStream_t st) {
   using namespace pb;
   CVLLM_CHECK_ALIGN(aligned16(q) && aligned16(out) && aligned16(k_cache) && aligned16(v_cache));
   CUtensorMap tm_q, tm_kc, tm_vc;
   {
     const uint32_t box3[3] = {64, 1, (uint32_t)kBM};
-    const uint64_t dq[3] = {(uint64_t)kHD, (uint64_t)HQ, (uint64_t)N};
-    const uint64_t sq[2] = {(uint64_t)kHD * 2, (uint64_t)HQ * kHD * 2};
+    const uint64_t dq[3] = {(uint64_t)HD, (uint64_t)HQ, (uint64_t)N};
+    const uint64_t sq[2] = {(uint64_t)HD * 2, (uint64_t)HQ * HD * 2};
     int rc = make_tmap_16b(&tm_q, q, 3, dq, sq, box3, true);
     if (rc) return rc;
-    const uint32_t box2[2] = {64, (uint32_t)kBN};
-    const uint64_t dc[2] = {(uint64_t)kHD, (uint64_t)cache_rows};
-    const uint64_t sc[1] = {(uint64_t)kHD * 2};
+    const uint32_t box2[2] = {64, (uint32_t)(PS < kBN ? PS : kBN)};
+    const uint64_t dc[2] = {(uint64_t)HD, (uint64_t)cache_rows};
+    const uint64_t sc[1] = {(uint64_t)HD * 2};
     rc = make_tmap_16b(&tm_kc, k_cache, 2, dc, sc, box2, true);
     if (rc) return rc;
     rc = make_tmap_16b(&tm_vc, v_cache, 2, dc, sc, box2, true);
@@ -523,13 +597,13 @@ int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_
   p.keep = keep;
   p.sink = sink ? 1.f : 0.f;
   p.sink_logits = sink ? sink_logits : nullptr;
-  const size_t smem = sizeof(PrefillBiasSmem) + 1024;
-  const dim3 grid((max_seqlen_q + kBM - 1) / kBM, HQ / 2, B);
-  static std::atomic<uint64_t> attr_bf{0};
-  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn_bias_kernel<true>, (int)smem, attr_bf));
-  prefill_attn_bias_kernel<true><<<grid, kThreads, smem, st>>>(tm_q, tm_kc, tm_vc, p);
-  CVLLM_CHECK_LAUNCH();
-  return CVLLM_OK;
+  p.dist_bias = dist_bias;
+  p.dist_rows = dist_rows;
+  if (HD == 128)
+    return dist_bias ? launch_bias<128, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
+                     : launch_bias<128, false>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
+  return dist_bias ? launch_bias<64, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
+                   : launch_bias<64, false>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
 }
 
 #ifdef CVLLM_PREFILL_TRACE

@@ -549,8 +549,9 @@ int cvllm_bias_attn_decode(const void* q, const void* k_cache, const void* v_cac
  * gets dist_bias[min(n, dist_rows - 1), h] (fp32 [dist_rows, H]; NULL = none), unscaled.  The caller makes the
  * table, so any rule from distance to bias (buckets of a smaller learned table) is served.  keep_first > 0: the
  * sequence's first keep_first positions stay visible to every later query whatever window and chunk say.  out_stride:
- * elements between the outputs of neighbouring tokens (0 = H * Dv).  A bias table runs on the mma.sync and fp32 FMA
- * kernels only; windows and kept tokens on all of them.
+ * elements between the outputs of neighbouring tokens (0 = H * Dv).  Portions with bias tables of up to 3584 rows run on the
+ * tcgen05 kernel where it serves (bfloat16, D = Dv = 128 or 64, pages of 16, 32, 64 or a multiple of 128 rows, H / G even,
+ * 16-byte aligned buffers), larger ones on the mma.sync and fp32 FMA kernels; windows and kept tokens on all of them.
  * cache_rows (decode; 0 = unknown) = rows of k_cache.  bfloat16 rows of D <= 576 numbers whose values are columns of the
  * keys (G = 1, v_cache = k_cache, v_stride = D, Dv <= 512, sizes multiples of 8, pages multiples of 64) take the tcgen05
  * kernel of csrc/latent_attn_umma.cu: portions unless the one named above serves them, decode from 8 heads on; its

@@ -1,0 +1,138 @@
+"""Portions of the biased attention over the head sizes, page sizes and bias tables that its tensor-core kernel serves (and
+their neighbours that it leaves to the others), against the formula in 64 bits.
+
+Tolerance: scores are sums of exact 16-bit products in 32 bits, P and the result are rounded to bfloat16 once each (2^-9
+relative, so 2^-9 / sqrt(3) root mean square each): 2.8e-3 relative in the 2-norm is the most that both leave; 6e-3 is
+twice that."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def make(H, G, D, page, spans, seed, **kw):
+    """A module with its cache: rows up to every sequence's last position written, all others NaN."""
+    from compactor_vllm.layers.attention import BiasedChunkAttention
+
+    g = torch.Generator().manual_seed(seed)
+    with torch.device(DEV):
+        m = BiasedChunkAttention(H, G, D, D, D ** -0.5, **kw).to(DEV)
+    ends = [s + n for s, n in spans]
+    B, P = len(spans), max(-(-e // page) for e in ends)
+    rows = (B + 1) * G * P * page
+    m.page_table = torch.randperm((B + 1) * G * P, generator=g).to(torch.int32).view(B + 1, G, P).to(DEV)
+    m.k_cache = torch.full((rows, D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    m.v_cache = m.k_cache.clone()
+    m.page_size = page
+    keys = []
+    for b, e in enumerate(ends):
+        k, v = (torch.randn(e, G, D, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+        p = torch.arange(e, device=DEV)
+        for h in range(G):
+            at = m.page_table[b + 1, h].long()[p // page] * page + p % page
+            m.k_cache[at], m.v_cache[at] = k[:, h], v[:, h]
+        keys.append((k.double(), v.double()))
+    q = torch.randn(sum(n for _, n in spans), H, D, generator=g).to(torch.bfloat16).to(DEV)
+    return m, q, keys
+
+
+def context(spans, decode):
+    from compactor_vllm.utils.context import set_context
+
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu = [0]
+    for _, n in spans:
+        cu.append(cu[-1] + n)
+    set_context(is_prefill=not decode, cu_seqlens_q=i32(cu), max_seqlen_q=max(n for _, n in spans),
+                max_seqlen_k=max(s + n for s, n in spans), batch_mapping=i32(range(1, len(spans) + 1)),
+                positions_i32=i32([p for s, n in spans for p in range(s, s + n)]), seq_start=i32([s for s, _ in spans]))
+
+
+def formula(m, q, keys, spans):
+    H, G, D = m.num_heads, m.num_kv_heads, m.head_dim
+    out, at = [], 0
+    for (k, v), (start, n) in zip(keys, spans):
+        i = torch.arange(start, start + n, device=DEV)[:, None]
+        j = torch.arange(k.shape[0], device=DEV)[None]
+        ok = torch.ones_like(i - j, dtype=torch.bool)
+        if m.chunk:
+            ok &= i // m.chunk == j // m.chunk
+        if m.window:
+            ok &= i - j < m.window
+        ok = (ok | (j < m.keep_first)) & (j <= i)
+        kk, vv = (x.repeat_interleave(H // G, dim=1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double(), kk) * m.scale
+        dist = (i - j).clamp(min=0)
+        if m.slopes is not None:
+            s -= m.slopes.double()[:, None, None] * dist
+        if m.dist_bias is not None:
+            s += m.dist_bias.double()[dist.clamp(max=m.dist_bias.shape[0] - 1)].permute(2, 0, 1)
+        s = s.masked_fill(~ok, -math.inf)
+        sink = torch.full((H, n, 1), 0.0 if m.sink else -math.inf, dtype=torch.float64, device=DEV)
+        if m.sink_logits is not None:
+            sink += m.sink_logits.double()[:, None, None]
+        p = torch.softmax(torch.cat([s, sink], dim=-1), dim=-1)[..., :-1]
+        out.append(torch.einsum("hqk,khd->qhd", p, vv).reshape(n, H * D))
+        at += n
+    return torch.cat(out)
+
+
+def options(seed, H, rows, slopes, sink, window, keep, chunk):
+    from compactor_vllm.layers.attention import linear_bias_slopes
+
+    kw = dict(window=window, keep_first=keep, chunk=chunk, sink=sink != "none", learned_sink=sink == "learned")
+    if slopes:
+        kw["slopes"] = linear_bias_slopes(H)
+    return kw
+
+
+def dress(m, rows, seed):
+    g = torch.Generator().manual_seed(seed)
+    with torch.no_grad():
+        if m.sink_logits is not None:
+            m.sink_logits.copy_(torch.randn(m.num_heads, generator=g))
+    if rows:
+        m.dist_bias = torch.randn(rows, m.num_heads, generator=g).to(DEV)
+        m.rel = torch.nn.Parameter(m.dist_bias)
+
+
+# portions that begin and end on and off the 128-row tiles and the pages, one of a single token
+SPANS = [(0, 300), (255, 130), (640, 1), (511, 129), (129, 127)]
+
+# H, G, D, page, table rows, slopes, sink, window, kept tokens, chunk
+CASES = [
+    (4, 2, 128, 128, 0, True, "zero", 0, 0, 0),
+    (4, 2, 128, 128, 1, False, "learned", 0, 0, 0),
+    (4, 2, 128, 128, 200, True, "none", 0, 0, 0),
+    (4, 2, 128, 64, 130, False, "learned", 257, 0, 0),
+    (2, 1, 128, 32, 700, True, "zero", 128, 5, 0),
+    (2, 1, 128, 16, 0, True, "none", 0, 130, 200),
+    (8, 1, 128, 256, 3584, False, "zero", 0, 0, 0),
+    (2, 1, 128, 128, 3585, False, "zero", 0, 0, 0),      # a table past what lies in shared memory
+    (4, 2, 64, 128, 0, False, "learned", 0, 0, 0),
+    (4, 2, 64, 64, 90, True, "none", 0, 0, 0),
+    (8, 2, 64, 32, 300, False, "zero", 100, 140, 0),
+    (4, 2, 64, 16, 0, True, "zero", 0, 0, 300),
+    (3, 1, 64, 64, 40, True, "zero", 0, 0, 0),           # an odd group
+    (4, 2, 128, 48, 40, True, "zero", 0, 0, 0),          # pages that do not divide a tile
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c)))
+def test_portions(case):
+    from compactor_vllm.utils.context import reset_context
+
+    H, G, D, page, rows, slopes, sink, window, keep, chunk = case
+    m, q, keys = make(H, G, D, page, SPANS, 11, **options(1, H, rows, slopes, sink, window, keep, chunk))
+    dress(m, rows, 2)
+    context(SPANS, False)
+    try:
+        got = m.attend(q).double()
+    finally:
+        reset_context()
+    want = formula(m, q, keys, SPANS)
+    assert torch.isfinite(got).all()
+    assert ((got - want).norm() / want.norm()).item() < 6e-3
