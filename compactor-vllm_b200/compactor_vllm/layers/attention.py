@@ -304,6 +304,18 @@ class BiasedChunkAttention(nn.Module):
                 and k.dtype == torch.bfloat16 and self.head_dim % 8 == 0 and self.v_head_dim % 8 == 0
                 and self.v_head_dim <= 512 and self.slopes is None and self.rel is None and int(self.page_size) % 64 == 0)
 
+    def streaming_decode_kernel(self, batch: int, max_keys: int) -> bool:
+        """Whether a decode step goes to the streaming kernel of csrc/decode_attn.cu (the library takes it when the sizes
+        allow and the workspace holds its scratch): where the keys a query may see are two of its units of 128 or more.
+        Measured at 32 / 8 heads of 64, 32 sequences (streaming / key splits): up to 140 keys 19 / 14 us, up to 280 keys
+        21.2 / 21.3 us; heads of 128, up to 280 keys 25 / 31 us, 8 x 4096 keys 37 / 104 us."""
+        if self.chunk:
+            max_keys = min(max_keys, self.chunk)
+        if self.window:
+            max_keys = min(max_keys, self.window)
+        return (max_keys >= 256 and not self.values_in_keys and self.head_dim == self.v_head_dim
+                and self.head_dim in (64, 128) and self.num_heads // self.num_kv_heads <= 8)
+
     def forward(self, qkv: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         from compactor_vllm import _native as N
 
@@ -378,7 +390,10 @@ class BiasedChunkAttention(nn.Module):
         else:
             assert ctx.batch_mapping.numel() == T
             splits = self.decode_splits(T, int(ctx.max_seqlen_k))
-            ws = N.workspace(dev, 4 * T * H * splits * (2 + Dv), "bias_attn_decode") if splits > 1 else None
+            ws_bytes = 4 * T * H * splits * (2 + Dv) if splits > 1 else 0
+            if self.streaming_decode_kernel(T, int(ctx.max_seqlen_k)):
+                ws_bytes = max(ws_bytes, lib.cvllm_bias_decode_workspace_bytes(T, H, G, D))
+            ws = N.workspace(dev, ws_bytes, "bias_attn_decode") if ws_bytes else None
             N.check(lib.cvllm_bias_attn_decode_dist(
                 N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.positions_i32),
                 N.ptr(ctx.batch_mapping), N.ptr(self.slopes), self.chunk, *dist, int(self.sink), N.ptr(self.sink_logits),

@@ -24,6 +24,13 @@
 //     a scratch slot; the CTA that completes a head merges (atomic ticket),
 //     every warp folding a strided subset of the slots with independent loads
 // HBM-bound: 4*D bytes per cached (token, head).
+//
+// BIAS: the same streaming for the biased attention's decode steps (cvllm_launch_bias_decode, called by
+// cvllm_bias_attn_decode): heads of 128 or 64, keys 0 .. position of a sequence cut by its chunk or window (the unit list
+// starts at the first visible key's unit, behind the units of kept first tokens), a distance bias and a sink in the softmax.
+// What that path computes in 32 bits stays so: P is the sum of two 16-bit numbers (2^-17 relative), whose low parts take
+// the query columns 4 .. 7 that groups of up to four heads leave free.  Partial states are folded by a second kernel
+// (its workspace needs no zeroed tickets).
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -37,7 +44,7 @@ constexpr int kDecWarps = 8;      // consumer warps: 8 x 16 keys = one unit
 constexpr int kDecCons = kDecWarps * 32;
 constexpr int kDecThreads = kDecCons + 32;  // + producer warp
 constexpr int kMaxSlots = 6;      // ring slots (one K unit or one V unit each): 6 when G <= 4, else 5
-constexpr int kSlotBytes = kUnit * 256;     // 32 KB at D = 128, 16-bit
+constexpr int kSlotBytes = kUnit * 256;     // 32 KB at D = 128, 16-bit (half of it used at D = 64)
 constexpr int kHalfBytes = kUnit * 128;     // one 64-column half of a slot
 
 struct DecodeParams {
@@ -54,6 +61,15 @@ struct DecodeParams {
   int lens_by_slot;   // seq_lens_bh is the cache's [Bmax+1, HKV] table, indexed through batch_mapping
   int mode;           // 0 = normal; 1 = consumers only drain the ring (load ceiling, profiling only)
   float scale_log2;
+  // biased attention only
+  const int32_t* positions;   // [B] position of every sequence's token
+  int64_t pt_slot, pt_head;   // page table strides
+  int64_t o_stride;           // output row stride (elements)
+  const float* slopes;        // [HQ] or NULL
+  const float* dist_bias;     // [dist_rows][HQ] or NULL
+  int dist_rows, chunk, window, keep, reserved_slot;
+  float sink;                 // 1 = a sink in the denominator
+  const float* sink_logits;   // [HQ] or NULL (score 0)
 #ifdef CVLLM_DECODE_TRACE
   unsigned long long* trace;  // profiling build only (tools/trace_decode.py): 8 globaltimer stamps per CTA
 #endif
@@ -71,10 +87,28 @@ __device__ __forceinline__ unsigned long long gtime() {
 #define DEC_TRACE(slot) do { } while (0)
 #endif
 
-// One warp's 16-key slice: K rows r / r+8 (4 chunks each), V for 4 keys x 2 chunks.
+// One warp's 16-key slice: K rows r / r+8 (D / 32 chunks each), V for 4 keys x D / 64 chunks.
+template <int D>
 struct Slice {
-  uint4 k_lo[4], k_hi[4];  // rows r, r+8; 16-byte chunk kchunk(j, c)
-  uint4 v[4][2];           // keys {2j,2j+1,2j+8,2j+9}; chunks r (d 8r..8r+7), 8+r
+  uint4 k_lo[D / 32], k_hi[D / 32];  // rows r, r+8; 16-byte chunk kchunk(j, c)
+  uint4 v[4][D / 64];                // keys {2j,2j+1,2j+8,2j+9}; chunks r (d 8r..8r+7), 8+r
+};
+
+// The keys that a sequence's token sees, as a list of kUnit-key units: the units that hold kept first tokens and lie
+// before the unit of the first key inside chunk and window, then the units from that one to the token's own.
+struct UnitList {
+  int pi, lo, begin, kept, count;
+  UnitList() = default;
+  __device__ __forceinline__ UnitList(const DecodeParams& p, int b) {
+    const bool live = p.batch_mapping[b] != p.reserved_slot;
+    pi = p.positions[b];
+    lo = p.chunk > 0 ? pi / p.chunk * p.chunk : 0;
+    if (p.window > 0) lo = max(lo, pi - p.window + 1);
+    begin = lo / kUnit;
+    kept = min(cdiv(min(p.keep, lo), kUnit), begin);
+    count = live ? kept + pi / kUnit - begin + 1 : 0;
+  }
+  __device__ __forceinline__ int base(int u) const { return (u < kept ? u : u - kept + begin) * kUnit; }
 };
 
 // Lane j owns the 16-byte chunks {2j, 2j+1} of each 128-byte half of a row; c = 0..3 walks them.
@@ -95,15 +129,27 @@ __device__ __forceinline__ uint32_t slot_addr(uint32_t slot, int t, int ch) {
   return slot + (uint32_t)((ch >> 3) * kHalfBytes + t * 128 + (((ch & 7) ^ (t & 7)) << 4));
 }
 
+// 1 / denominator of a biased head's row whose running maximum is m (log2 units) and whose sum is l, sink included: the
+// row's values are relative to m, and so is what the sink adds
+__device__ __forceinline__ float bias_inv(const DecodeParams& p, int hq, float m, float l) {
+  if (p.sink > 0.f) {
+    const float sm = (p.sink_logits ? p.sink_logits[hq] : 0.f) * 1.4426950408889634f;
+    if (sm - m > 120.f) return 0.f;   // a sink far above every key takes all the weight
+    l += ex2(sm - m);
+  }
+  return l > 0.f ? 1.f / l : 0.f;
+}
+
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kDecCons) : "memory"); }
 
-template <bool BF16, int D>
+template <bool BF16, int D, bool BIAS = false>
 __global__ void __launch_bounds__(kDecThreads, 1)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const DecodeParams p) {
-  static_assert(D == 128, "decode kernel is specialised for head_dim 128");
+  static_assert(D == 128 || (BIAS && D == 64), "head sizes");
   constexpr int KSTEPS = D / 16;  // 8
   constexpr int MT = D / 16;      // 8 output m-tiles (16 d each)
+  constexpr int KC = D / 32;      // 16-byte chunks of a row per lane
   constexpr int ROW = D + 2;      // merged row: O[D], m, l
   constexpr int NW = kDecThreads / 32;
 
@@ -126,9 +172,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const int G = p.G;
   // rows cached for flattened head i = b * HKV + h
   auto len_of = [&](int i) -> int {
+    if constexpr (BIAS) return p.positions[i / p.HKV] + 1;
     if (!p.lens_by_slot) return p.seq_lens_bh[i];
     const int b = i / p.HKV;
     return p.seq_lens_bh[p.batch_mapping[b] * p.HKV + (i - b * p.HKV)];
+  };
+  auto units_of = [&](int i) -> int {
+    if constexpr (BIAS) return UnitList(p, i / p.HKV).count;
+    else return cdiv(len_of(i), kUnit);
+  };
+  auto out_row = [&](int b, int h) -> uint32_t* {   // the G heads of (b, h), as pairs
+    if constexpr (BIAS) return reinterpret_cast<uint32_t*>(p.out) + b * (p.o_stride / 2) + h * G * (D / 2);
+    else return reinterpret_cast<uint32_t*>(p.out) + ((int64_t)b * p.HQ + h * G) * (D / 2);
   };
 
   if (tid == 0) DEC_TRACE(0);
@@ -149,7 +204,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int per = cdiv(BH, kDecThreads);
     const int beg = min(BH, tid * per), end = min(BH, beg + per);
     int local = 0;
-    for (int i = beg; i < end; ++i) local += cdiv(len_of(i), kUnit);
+    for (int i = beg; i < end; ++i) local += units_of(i);
     int incl = local;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -163,7 +218,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     int run = base + incl - local;
     for (int i = beg; i < end; ++i) {
       s_prefix[i] = run;
-      run += cdiv(len_of(i), kUnit);
+      run += units_of(i);
     }
     if (tid == kDecThreads - 1) s_prefix[BH] = run;
     __syncthreads();
@@ -175,7 +230,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   for (int i = c; i < BH; i += C) {
     if (s_prefix[i + 1] == s_prefix[i]) {
       const int b = i / p.HKV, h = i % p.HKV;
-      uint32_t* o = reinterpret_cast<uint32_t*>(p.out) + ((int64_t)b * p.HQ + h * G) * (D / 2);
+      uint32_t* o = out_row(b, h);
       for (int e = tid; e < G * D / 2; e += kDecThreads) o[e] = 0u;
     }
   }
@@ -209,14 +264,16 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       nvp = 0;
       if (my_unit < u_end) {
         const int head = find_head(my_unit);
-        const int t0 = (my_unit - s_prefix[head]) * kUnit;
+        int t0 = (my_unit - s_prefix[head]) * kUnit;
+        if constexpr (BIAS) t0 = UnitList(p, head / p.HKV).base(my_unit - s_prefix[head]);
         const int L = len_of(head);
         nvp = min(pieces, cdiv(L - t0, BR));  // pages past the head's length are not mapped
         if (my_piece < nvp) {
           const int b = head / p.HKV, h = head % p.HKV;
           const int tok = t0 + my_piece * BR;
           const int pg = tok / p.PS;
-          const int32_t* pt = p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + h) * p.NLP;
+          const int32_t* pt = BIAS ? p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head
+                                   : p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + h) * p.NLP;
           row = pt[pg] * p.PS + (tok - pg * p.PS);
         }
       }
@@ -239,13 +296,13 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           const CUtensorMap* tm = kv ? &tm_v : &tm_k;
           if (lane == 0) {
             mbar_wait(&bar_empty[slot], par ^ 1u);
-            mbar_expect_tx(&bar_full[slot], (uint32_t)(nv * BR * 256));
+            mbar_expect_tx(&bar_full[slot], (uint32_t)(nv * BR * D * 2));
           }
           for (int pc = 0; pc < nv; ++pc) {
             const int r0 = __shfl_sync(0xffffffffu, row, i * pieces + pc);
             if (lane == 0) {
               tma_load_2d(dst + pc * BR * 128, tm, &bar_full[slot], 0, r0);
-              tma_load_2d(dst + kHalfBytes + pc * BR * 128, tm, &bar_full[slot], 64, r0);
+              if constexpr (D == 128) tma_load_2d(dst + kHalfBytes + pc * BR * 128, tm, &bar_full[slot], 64, r0);
             }
           }
         }
@@ -270,6 +327,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int ua = u - h_beg, ub = seg_end - h_beg;  // units of this head
     const int b = head / p.HKV, h = head % p.HKV;
     const int L = len_of(head);
+    const UnitList list = [&]() {
+      if constexpr (BIAS) return UnitList(p, b);
+      else return UnitList{};
+    }();
+    // biased attention: this lane's query columns 2j, 2j + 1 (columns 4 .. 7 of a small group carry the low parts of P)
+    const bool low_cols = BIAS && G <= 4 && j >= 2;
+    const int qc = low_cols ? 2 * j - 4 : 2 * j;
+    float slope0 = 0.f, slope1 = 0.f;
+    if (BIAS && p.slopes) {
+      slope0 = qc < G ? p.slopes[h * G + qc] * 1.4426950408889634f : 0.f;
+      slope1 = qc + 1 < G ? p.slopes[h * G + qc + 1] * 1.4426950408889634f : 0.f;
+    }
 
     // ---- Q^T as B operand (n = query r, k = permuted d) ----
     uint32_t qb[KSTEPS][2];
@@ -277,7 +346,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       const uint4 z = make_uint4(0, 0, 0, 0);
       const char* qrow = reinterpret_cast<const char*>(p.q) + ((int64_t)b * p.HQ + h * G + r) * (D * 2);
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
+      for (int cc = 0; cc < KC; ++cc) {
         const uint4 v = (r < G) ? *reinterpret_cast<const uint4*>(qrow + kchunk(j, cc) * 16) : z;
         qb[2 * cc][0] = v.x; qb[2 * cc][1] = v.y;
         qb[2 * cc + 1][0] = v.z; qb[2 * cc + 1][1] = v.w;
@@ -299,15 +368,33 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if (++c_slot == kSlots) { c_slot = 0; c_par ^= 1u; }
       const uint32_t k_base = ring_u32 + ks_slot * kSlotBytes, v_base = ring_u32 + vs_slot * kSlotBytes;
       const int t0 = warp * 16;                               // this warp's rows inside the unit
-      const int n_valid = min(16, L - (uu * kUnit + t0));     // <= 0: nothing for this warp
+      const int unit0 = BIAS ? list.base(uu) : uu * kUnit;    // position of the unit's first key
+      const int n_valid = min(16, L - (unit0 + t0));          // <= 0: nothing for this warp
+      // what distance and head add to this lane's four logits, requested before the unit's data is waited for
+      float bias0 = 0.f, bias1 = 0.f, bias2 = 0.f, bias3 = 0.f;
+      if constexpr (BIAS) {
+        const int n_lo = list.pi - (unit0 + t0 + r), n_hi = n_lo - 8;
+        bias0 = -slope0 * (float)n_lo; bias1 = -slope1 * (float)n_lo;
+        bias2 = -slope0 * (float)n_hi; bias3 = -slope1 * (float)n_hi;
+        if (p.dist_bias && qc < G) {
+          const float* t_lo = p.dist_bias + (int64_t)min(max(n_lo, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
+          const float* t_hi = p.dist_bias + (int64_t)min(max(n_hi, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
+          bias0 = fmaf(t_lo[0], 1.4426950408889634f, bias0);
+          bias2 = fmaf(t_hi[0], 1.4426950408889634f, bias2);
+          if (qc + 1 < G) {
+            bias1 = fmaf(t_lo[1], 1.4426950408889634f, bias1);
+            bias3 = fmaf(t_hi[1], 1.4426950408889634f, bias3);
+          }
+        }
+      }
 
       // every warp waits (so nobody can run a full ring ahead) and releases the slots
       mbar_wait(&bar_full[ks_slot], k_par);
       if (tid == 0 && u == u_begin && uu == ua) DEC_TRACE(2);
       if (n_valid > 0 && p.mode == 0) {
-        Slice cur;
+        Slice<D> cur;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
+        for (int cc = 0; cc < KC; ++cc) {
           cur.k_lo[cc] = lds_v4(slot_addr(k_base, t0 + r, kchunk(j, cc)));
           cur.k_hi[cc] = lds_v4(slot_addr(k_base, t0 + r + 8, kchunk(j, cc)));
         }
@@ -320,9 +407,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int key = 2 * j + (i & 1) + ((i >> 1) << 3);
-            const bool ok = key < n_valid;
+            bool ok = key < n_valid;
+            if constexpr (BIAS) ok = ok && (unit0 + t0 + key >= list.lo || unit0 + t0 + key < p.keep);
             cur.v[i][0] = ok ? lds_v4(slot_addr(v_base, t0 + key, r)) : z;
-            cur.v[i][1] = ok ? lds_v4(slot_addr(v_base, t0 + key, 8 + r)) : z;
+            if constexpr (D == 128) cur.v[i][D / 64 - 1] = ok ? lds_v4(slot_addr(v_base, t0 + key, 8 + r)) : z;
           }
         }
         // ---- S^T[16 keys x 8 queries]: two accumulators halve the dependent mma chain ----
@@ -341,17 +429,30 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         for (int e = 0; e < 4; ++e) s[e] += s_b[e];
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);  // K rows are in registers: free the slot now
-        const bool ok_lo = r < n_valid, ok_hi = r + 8 < n_valid;
-        const float x0 = ok_lo ? s[0] * p.scale_log2 : -INFINITY;
-        const float x1 = ok_lo ? s[1] * p.scale_log2 : -INFINITY;
-        const float x2 = ok_hi ? s[2] * p.scale_log2 : -INFINITY;
-        const float x3 = ok_hi ? s[3] * p.scale_log2 : -INFINITY;
+        bool ok_lo = r < n_valid, ok_hi = r + 8 < n_valid;
+        if constexpr (BIAS) {
+          const int kp = unit0 + t0 + r;
+          ok_lo = ok_lo && (kp >= list.lo || kp < p.keep);
+          ok_hi = ok_hi && (kp + 8 >= list.lo || kp + 8 < p.keep);
+          if (G <= 4) {   // columns 4 .. 7 repeat the scores of columns 0 .. 3: same maximum, same probabilities
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float other = __shfl_xor_sync(0xffffffffu, s[e], 2);
+              if (low_cols) s[e] = other;
+            }
+          }
+        }
+        const float x0 = ok_lo ? (BIAS ? fmaf(s[0], p.scale_log2, bias0) : s[0] * p.scale_log2) : -INFINITY;
+        const float x1 = ok_lo ? (BIAS ? fmaf(s[1], p.scale_log2, bias1) : s[1] * p.scale_log2) : -INFINITY;
+        const float x2 = ok_hi ? (BIAS ? fmaf(s[2], p.scale_log2, bias2) : s[2] * p.scale_log2) : -INFINITY;
+        const float x3 = ok_hi ? (BIAS ? fmaf(s[3], p.scale_log2, bias3) : s[3] * p.scale_log2) : -INFINITY;
         float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) {
           mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
           mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
         }
+        if constexpr (BIAS) { m0 = fmaxf(m0, -1e30f); m1 = fmaxf(m1, -1e30f); }   // a first unit may be all masked
         float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
         // a NaN/-inf column max (garbage q) must not poison the rest
         if (!(mn0 > -INFINITY)) mn0 = 0.f;
@@ -367,19 +468,32 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             acc[t][0] *= al0; acc[t][1] *= al1; acc[t][2] *= al0; acc[t][3] *= al1;
           }
         }
-        const uint32_t pb0 = movmatrix_trans(pack2<BF16>(p0, p1));
-        const uint32_t pb1 = movmatrix_trans(pack2<BF16>(p2, p3));
+        uint32_t hi01 = pack2<BF16>(p0, p1), hi23 = pack2<BF16>(p2, p3), lo01 = 0u, lo23 = 0u;
+        if constexpr (BIAS) {
+          lo01 = pack2<true>(p0 - __uint_as_float(hi01 << 16), p1 - __uint_as_float(hi01 & 0xffff0000u));
+          lo23 = pack2<true>(p2 - __uint_as_float(hi23 << 16), p3 - __uint_as_float(hi23 & 0xffff0000u));
+          if (low_cols) { hi01 = lo01; hi23 = lo23; }
+        }
+        const uint32_t pb0 = movmatrix_trans(hi01);
+        const uint32_t pb1 = movmatrix_trans(hi23);
 
         // ---- O^T[D x 8] += V^T[D x 16] . P^T[16 x 8] ----
+        // tile t: rows r and r + 8 are numbers 8 r + t and 64 + 8 r + t (D = 64: 8 r + t and 8 r + 4 + t) of the value rows
+        auto add_pv = [&](uint32_t b0, uint32_t b1) {
 #pragma unroll
-        for (int t = 0; t < MT; ++t) {
-          const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
-          const int w = t >> 1;
-          const uint32_t a0 = __byte_perm(u4_get(cur.v[0][0], w), u4_get(cur.v[1][0], w), sel);
-          const uint32_t a1 = __byte_perm(u4_get(cur.v[0][1], w), u4_get(cur.v[1][1], w), sel);
-          const uint32_t a2 = __byte_perm(u4_get(cur.v[2][0], w), u4_get(cur.v[3][0], w), sel);
-          const uint32_t a3 = __byte_perm(u4_get(cur.v[2][1], w), u4_get(cur.v[3][1], w), sel);
-          mma16816<BF16>(acc[t], a0, a1, a2, a3, pb0, pb1);
+          for (int t = 0; t < MT; ++t) {
+            const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
+            const int w = t >> 1, c2 = D / 64 - 1, w2 = D == 128 ? w : w + 2;
+            const uint32_t a0 = __byte_perm(u4_get(cur.v[0][0], w), u4_get(cur.v[1][0], w), sel);
+            const uint32_t a1 = __byte_perm(u4_get(cur.v[0][c2], w2), u4_get(cur.v[1][c2], w2), sel);
+            const uint32_t a2 = __byte_perm(u4_get(cur.v[2][0], w), u4_get(cur.v[3][0], w), sel);
+            const uint32_t a3 = __byte_perm(u4_get(cur.v[2][c2], w2), u4_get(cur.v[3][c2], w2), sel);
+            mma16816<BF16>(acc[t], a0, a1, a2, a3, b0, b1);
+          }
+        };
+        add_pv(pb0, pb1);
+        if constexpr (BIAS) {
+          if (G > 4) add_pv(movmatrix_trans(lo01), movmatrix_trans(lo23));   // no free columns: a second product
         }
       } else {
         if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);
@@ -396,14 +510,23 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       l0 += __shfl_xor_sync(0xffffffffu, l0, o);
       l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     }
+    if constexpr (BIAS) {
+      if (G <= 4) {   // the low parts' products join their columns
+#pragma unroll
+        for (int t = 0; t < MT; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[t][e] += __shfl_xor_sync(0xffffffffu, acc[t][e], 2);
+      }
+    }
     {
       float* mw = s_merge + warp * G * ROW;
       const int q0 = 2 * j, q1 = 2 * j + 1;  // query columns of this lane; only q < G exist
+      constexpr int kRow2 = D == 128 ? 64 : 4;   // where a tile's second eight rows lie (see add_pv)
       if (q0 < G) {
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
           mw[q0 * ROW + 8 * r + t] = acc[t][0];
-          mw[q0 * ROW + 64 + 8 * r + t] = acc[t][2];
+          mw[q0 * ROW + kRow2 + 8 * r + t] = acc[t][2];
         }
         if (r == 0) { mw[q0 * ROW + D] = m0; mw[q0 * ROW + D + 1] = l0; }
       }
@@ -411,7 +534,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
         for (int t = 0; t < MT; ++t) {
           mw[q1 * ROW + 8 * r + t] = acc[t][1];
-          mw[q1 * ROW + 64 + 8 * r + t] = acc[t][3];
+          mw[q1 * ROW + kRow2 + 8 * r + t] = acc[t][3];
         }
         if (r == 0) { mw[q1 * ROW + D] = m1; mw[q1 * ROW + D + 1] = l1; }
       }
@@ -441,11 +564,12 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     };
     auto write_out = [&]() {
-      uint32_t* orow = reinterpret_cast<uint32_t*>(p.out) + ((int64_t)b * p.HQ + h * G) * (D / 2);
+      uint32_t* orow = out_row(b, h);
       for (int e = tid; e < G * D / 2; e += kDecCons) {
         const int q = e / (D / 2), d2 = e - q * (D / 2);
         const float lq = s_final[q * ROW + D + 1];
-        const float inv = lq > 0.f ? 1.f / lq : 0.f;
+        float inv = lq > 0.f ? 1.f / lq : 0.f;
+        if constexpr (BIAS) inv = bias_inv(p, h * G + q, s_final[q * ROW + D], lq);
         orow[e] = pack2<BF16>(s_final[q * ROW + 2 * d2] * inv, s_final[q * ROW + 2 * d2 + 1] * inv);
       }
     };
@@ -459,6 +583,11 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       // publish the partial, then take a ticket; the CTA completing the head merges
       float* slot = p.scratch + (int64_t)(head + c) * G * ROW;
       for (int e = tid; e < G * ROW; e += kDecCons) __stcg(slot + e, s_final[e]);
+      if constexpr (BIAS) {
+        cons_bar();   // s_merge / s_final reused by the next segment; bias_decode_fold_kernel merges
+        u = seg_end;
+        continue;
+      }
       __threadfence();
       cons_bar();
       if (tid == 0) {
@@ -531,6 +660,76 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
 #endif
     u = seg_end;
+  }
+}
+
+// Folds the partial states of the heads that the split cut (BIAS): a CTA per query head, which recomputes the split; a warp
+// per every eighth slot, whose loads are all independent (a single KV head's rows may lie in as many slots as there are
+// CTAs: with a CTA per KV head and the slots one after the other 1 x 16000 keys of
+// 8 / 1 heads took 122 us with norms and cache write, 26 us so).
+template <int D>
+__global__ void __launch_bounds__(256) bias_decode_fold_kernel(const DecodeParams p, int C) {
+  constexpr int ROW = D + 2, PER = D / 32;
+  const int hq = blockIdx.x % p.HQ, b = blockIdx.x / p.HQ, G = p.G, h = hq / G, q = hq - h * G, head = b * p.HKV + h;
+  __shared__ float s_o[8][D];
+  __shared__ float s_l[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int before = 0, all = 0;   // units of the sequences before, and of all
+  for (int i = lane; i < p.B; i += 32) {
+    const int n = UnitList(p, i).count;
+    all += n;
+    if (i < b) before += n;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+    all += __shfl_xor_sync(0xffffffffu, all, o);
+  }
+  const int n = UnitList(p, b).count;
+  if (n == 0) return;
+  const int64_t U = (int64_t)all * p.HKV, h_beg = (int64_t)before * p.HKV + (int64_t)h * n, h_end = h_beg + n;
+  const int c_first = (int)(((h_beg + 1) * C - 1) / U), c_last = (int)((h_end * C - 1) / U);
+  if (c_first == c_last) return;   // one CTA had the whole head and has written it
+  auto used = [&](int c) { return U * c / C < U * (c + 1) / C; };   // CTAs without units wrote nothing
+  auto row = [&](int c) { return p.scratch + ((int64_t)(head + c) * G + q) * ROW; };
+  float M = -INFINITY;
+  for (int c = c_first + lane; c <= c_last; c += 32)
+    if (used(c)) M = fmaxf(M, __ldcg(row(c) + D));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  float acc[PER], l = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
+#pragma unroll 4
+  for (int c = c_first + warp; c <= c_last; c += 8) {
+    if (!used(c)) continue;
+    const float* x = row(c);
+    const float w = ex2(__ldcg(x + D) - M);
+    l = fmaf(__ldcg(x + D + 1), w, l);
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(x + i * 32 + 2 * lane));
+      acc[i] = fmaf(v.x, w, acc[i]);
+      acc[i + 1] = fmaf(v.y, w, acc[i + 1]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PER; i += 2) {
+    s_o[warp][i * 32 + 2 * lane] = acc[i];
+    s_o[warp][i * 32 + 2 * lane + 1] = acc[i + 1];
+  }
+  if (lane == 0) s_l[warp] = l;
+  __syncthreads();
+  if (threadIdx.x < D / 2) {
+    float x = 0.f, y = 0.f, sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      x += s_o[w][2 * threadIdx.x];
+      y += s_o[w][2 * threadIdx.x + 1];
+      sum += s_l[w];
+    }
+    const float inv = bias_inv(p, hq, M, sum);
+    reinterpret_cast<uint32_t*>(p.out)[b * (p.o_stride / 2) + hq * (D / 2) + threadIdx.x] = pack2<true>(x * inv, y * inv);
   }
 }
 
@@ -633,6 +832,67 @@ static int launch_decode_attn(const void* q, void* out, const void* k_cache, con
     decode_attn_kernel<true, 128><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
   } else {
     decode_attn_kernel<false, 128><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+  }
+  CVLLM_CHECK_LAUNCH();
+  return CVLLM_OK;
+}
+
+// What the streaming kernel serves of the biased attention's decode steps (bfloat16, contiguous 16-byte aligned rows), and
+// the scratch that it needs there.
+bool cvllm_bias_decode_serves(int H, int G, int D, int Dv, int page_size, int64_t o_stride) {
+  return D == Dv && (D == 128 || D == 64) && H / G <= 8 && o_stride % 2 == 0 &&
+         (page_size % kUnit == 0 || page_size == 64 || page_size == 32 || page_size == 16);
+}
+extern "C" size_t cvllm_bias_decode_workspace_bytes(int B, int H, int G, int D) {
+  if (B <= 0 || H <= 0 || G <= 0) return 0;
+  return ((size_t)B * G + (size_t)sm_count()) * (H / G) * (D + 2) * sizeof(float);
+}
+
+int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows, void* out,
+                             int64_t o_stride, const int32_t* positions, const int32_t* batch_mapping,
+                             const int32_t* page_table, int64_t pt_slot, int64_t pt_head, int B, int H, int G, int D, int PS,
+                             float scale, const float* slopes, int chunk, int window, int keep, const float* dist_bias,
+                             int dist_rows, int sink, const float* sink_logits, int reserved_slot, float* workspace,
+                             cudaStream_t st) {
+  DecodeParams p = {};
+  p.q = q; p.out = out;
+  p.page_table = page_table; p.batch_mapping = batch_mapping;
+  p.scratch = workspace;
+  p.B = B; p.HQ = H; p.HKV = G; p.G = H / G; p.PS = PS;
+  p.box_rows = PS < kUnit ? PS : kUnit;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.positions = positions; p.pt_slot = pt_slot; p.pt_head = pt_head; p.o_stride = o_stride;
+  p.slopes = slopes; p.dist_bias = dist_bias; p.dist_rows = dist_rows;
+  p.chunk = chunk; p.window = window; p.keep = keep; p.reserved_slot = reserved_slot;
+  p.sink = sink ? 1.f : 0.f; p.sink_logits = sink ? sink_logits : nullptr;
+  CUtensorMap tm_k, tm_v;
+  {
+    const uint32_t box[2] = {64, (uint32_t)p.box_rows};
+    const uint64_t dims[2] = {(uint64_t)D, (uint64_t)cache_rows};
+    const uint64_t strides[1] = {(uint64_t)D * 2};
+    int rc = make_tmap_16b(&tm_k, k_cache, 2, dims, strides, box, true);
+    if (rc) return rc;
+    rc = make_tmap_16b(&tm_v, v_cache, 2, dims, strides, box, true);
+    if (rc) return rc;
+  }
+  constexpr int kMaxSmem = 224 * 1024;
+  const int BH = B * G, C = sm_count();
+  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)(kDecWarps + 1) * p.G * (D + 2) * 4 + ((size_t)BH + 1) * 4;
+  CVLLM_CHECK_SUPPORTED(fixed + 2 * (size_t)kSlotBytes <= (size_t)kMaxSmem);
+  p.slots = (int)(((size_t)kMaxSmem - fixed) / kSlotBytes);
+  if (p.slots > kMaxSlots) p.slots = kMaxSlots;
+  const size_t smem = fixed + (size_t)p.slots * kSlotBytes;
+  static std::atomic<uint64_t> attr_128{0}, attr_64{0};
+  if (D == 128) {
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128, true>, kMaxSmem, attr_128));
+    decode_attn_kernel<true, 128, true><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_LAUNCH();
+    bias_decode_fold_kernel<128><<<B * H, 256, 0, st>>>(p, C);
+  } else {
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 64, true>, kMaxSmem, attr_64));
+    decode_attn_kernel<true, 64, true><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_LAUNCH();
+    bias_decode_fold_kernel<64><<<B * H, 256, 0, st>>>(p, C);
   }
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;

@@ -563,6 +563,10 @@ int cvllm_bias_attn_varlen_dist(const void* q, const void* k_cache, const void* 
                                 const float* dist_bias, int dist_rows, int sink, const float* sink_logits, float scale,
                                 void* out, int64_t out_stride, int B, int max_new, int H, int G, int D, int Dv, int total_tokens, int64_t cache_rows, int pages_per_head,
                                 int64_t v_stride, int dtype, cvllm_stream_t stream);
+/* Decode in bfloat16 with D = Dv = 128 or 64, pages of 16, 32, 64 or a multiple of 128 rows, H / G <= 8 and cache_rows given
+ * takes the streaming kernel of csrc/decode_attn.cu when workspace_bytes >= cvllm_bias_decode_workspace_bytes(B, H, G, D)
+ * (`splits` then counts for nothing; the workspace needs no initial contents). */
+size_t cvllm_bias_decode_workspace_bytes(int B, int H, int G, int D);
 int cvllm_bias_attn_decode_dist(const void* q, const void* k_cache, const void* v_cache, const int32_t* page_table,
                                 int64_t table_stride_slot, int64_t table_stride_head, int page_size,
                                 const int32_t* positions, const int32_t* batch_mapping, const float* slopes, int chunk,

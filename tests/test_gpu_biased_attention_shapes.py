@@ -136,3 +136,51 @@ def test_portions(case):
     want = formula(m, q, keys, SPANS)
     assert torch.isfinite(got).all()
     assert ((got - want).norm() / want.norm()).item() < 6e-3
+
+
+# decoding: positions at and around unit, window and chunk borders, one at position 0, one on the reserved slot
+DECODE = [(p, 1) for p in (0, 1, 127, 128, 255, 299, 300, 511, 640, 1100)]
+
+
+def decode(m, q, option=0):
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import get_context, reset_context
+
+    context(DECODE, True)
+    get_context().batch_mapping[4] = 0       # a padding row
+    N.set_test_option("bias_attn_fma", option)
+    try:
+        return m.attend(q).double()
+    finally:
+        N.set_test_option("bias_attn_fma", 0)
+        reset_context()
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[1] * 8 >= c[0]] + [(16, 2, 128, 128, 50, True, "learned", 0, 0, 0),
+                                                                           (5, 1, 64, 64, 0, True, "zero", 200, 3, 0)],
+                         ids=lambda c: "-".join(map(str, c)))
+def test_decoding(case):
+    """The streaming kernel keeps P in 32 bits (as two 16-bit parts), so only the result's rounding is left: 2^-9 / sqrt(3)
+    = 1.2e-3; 2.5e-3 is twice that.  It is no further from the formula than the FMA kernel, whose P is one 32-bit number."""
+    H, G, D, page, rows, slopes, sink, window, keep, chunk = case
+    m, q, keys = make(H, G, D, page, DECODE, 12, **options(1, H, rows, slopes, sink, window, keep, chunk))
+    dress(m, rows, 3)
+    want = formula(m, q, keys, DECODE)
+    want[4] = 0
+    err = lambda x: ((x - want).norm() / want.norm()).item()
+    got, fma = decode(m, q), decode(m, q, 1)
+    assert torch.isfinite(got).all() and (got[4] == 0).all()
+    assert err(got) < 2.5e-3 and err(got) < 1.05 * err(fma) + 1e-6
+
+
+def test_decoding_far_sinks_and_scores():
+    """Sinks far above and far below every key, scores large enough that only the running maximum keeps them finite."""
+    m, q, keys = make(4, 2, 128, 128, DECODE, 13, sink=True, learned_sink=True)
+    q = (q * 8).contiguous()
+    with torch.no_grad():
+        m.sink_logits.copy_(torch.tensor([500.0, -500.0, 60.0, 0.0]))
+    want = formula(m, q, keys, DECODE)
+    want[4] = 0
+    got = decode(m, q)
+    assert torch.isfinite(got).all()
+    assert ((got - want).norm() / want.norm()).item() < 2.5e-3
