@@ -316,160 +316,6 @@ __device__ __forceinline__ void store_state(const float2 (&S)[R / 2], const Recu
   }
 }
 
-// Gated delta rule.  qkv [T, 2 G D + H Dv] fp32 = (q | k | v) after the short convolution; beta and decay logits are
-// columns b_off + h and a_off + h of proj (model type).  Head h reads q / k head h / (H / G).
-// Algebra per token, from the state S before the token:  dk = S^T k, dq = S^T q (one pass over the registers),
-// u = beta (v - g dk),  o = g dq + (k . q) u,  S <- g S + k u^T   - the same numbers as decaying first, writing, then
-// reading, with one pass less over the state.
-template <typename T, int R, int MAXT>
-__global__ void __launch_bounds__(MAXT) delta_rule_kernel(const float* __restrict__ qkv, int64_t qkv_stride,
-                                                          const T* __restrict__ proj, int64_t proj_stride, int b_off,
-                                                          int a_off, const float* __restrict__ A_log,
-                                                          const float* __restrict__ dt_bias, int G, RecurArgs a) {
-  using L = Lay<R>;
-  extern __shared__ __align__(16) float sm[];
-  const int D = a.D, Dv = a.Dv, H = a.H, KS = a.KS, CW = a.CW, kTok = a.tok;
-  const int ROW = KS * L::SL;
-  float* sq = sm;                       // [kTok][ROW]
-  float* sk = sq + kTok * ROW;          // [kTok][ROW]
-  float* sv = sk + kTok * ROW;          // [kTok][CW]
-  float* so = sv + kTok * CW;           // [kTok][CW]
-  float* sc = so + kTok * CW;           // [kTok][4]: decay, beta, k . q
-  float* part = sc + kTok * 4;          // [2][kTokMax]
-  float* sinv = part + 2 * kTokMax;     // [kTokMax]
-  const int h = blockIdx.x / a.VT, vt = blockIdx.x % a.VT, b = blockIdx.y;
-  int t0, n_new, start;
-  portion(a.g, b, t0, n_new, start);
-  if (n_new <= 0) return;               // the same for every CTA of the cluster
-  const int slot = a.g.slots[b];
-  const int kvh = h / (H / G);
-  const int c0 = vt * CW, ncol = min(CW, Dv - c0);
-  const int tid = threadIdx.x, j = tid / KS, ks = tid % KS;
-  const bool valid = j < ncol;
-  const int warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
-  for (int i = tid; i < 2 * kTok * ROW; i += blockDim.x) sm[i] = 0.f;   // pads and rows beyond D stay zero
-  float2 S[R / 2];
-  load_state<R>(S, a, slot, h, c0 + j, valid, ks, start > 0);
-  const float neg_a = -expf(A_log[h]), dtb = dt_bias[h];
-  const float q_scale = rsqrtf((float)D);
-  const int q_col = kvh * D, k_col = G * D + kvh * D, v_col = 2 * G * D + h * Dv + c0;
-  __syncthreads();
-  // a stage's inputs are loaded into registers one stage ahead, so that their latency hides behind the tokens before
-  float pq[kPF], pk[kPF], pv[kPFG];
-  T pg[kPFG];
-  auto prefetch = [&](int j0n) {
-    const int nn = min(kTok, n_new - j0n);
-    TileWalk w(D);
-#pragma unroll
-    for (int u = 0; u < kPF; ++u, w.next())
-      if (w.c < nn) {
-        const float* row = qkv + (int64_t)(t0 + j0n + w.c) * qkv_stride;
-        pq[u] = row[q_col + w.d];
-        pk[u] = row[k_col + w.d];
-      }
-    TileWalk wv(ncol);
-#pragma unroll
-    for (int u = 0; u < kPFG; ++u, wv.next())
-      if (wv.c < nn) pv[u] = qkv[(int64_t)(t0 + j0n + wv.c) * qkv_stride + v_col + wv.d];
-  };
-  prefetch(0);
-  int stage = 0;
-  for (int j0 = 0; j0 < n_new; j0 += kTok, ++stage) {
-    const int n = min(kTok, n_new - j0);
-    {
-      TileWalk w(D);
-#pragma unroll
-      for (int u = 0; u < kPF; ++u, w.next())
-        if (w.c < n) {
-          sq[w.c * ROW + L::at(w.d)] = pq[u];
-          sk[w.c * ROW + L::at(w.d)] = pk[u];
-        }
-      for (; w.c < n; w.next()) {
-        const float* row = qkv + (int64_t)(t0 + j0 + w.c) * qkv_stride;
-        sq[w.c * ROW + L::at(w.d)] = row[q_col + w.d];
-        sk[w.c * ROW + L::at(w.d)] = row[k_col + w.d];
-      }
-      TileWalk wv(ncol);
-#pragma unroll
-      for (int u = 0; u < kPFG; ++u, wv.next())
-        if (wv.c < n) sv[wv.c * CW + wv.d] = pv[u];
-      for (; wv.c < n; wv.next()) sv[wv.c * CW + wv.d] = qkv[(int64_t)(t0 + j0 + wv.c) * qkv_stride + v_col + wv.d];
-    }
-    for (int c = tid; c < n; c += blockDim.x) {   // the tokens' decays and betas
-      const T* pr = proj + (int64_t)(t0 + j0 + c) * proj_stride;
-      sc[c * 4 + 0] = expf(neg_a * softplus_f(to_f<T>(pr[a_off + h]) + dtb));
-      sc[c * 4 + 1] = sigmoid_f(to_f<T>(pr[b_off + h]));
-    }
-    __syncthreads();
-    if (j0 + kTok < n_new) prefetch(j0 + kTok);
-    prefetch_gates<T>(a, pg, h, c0, ncol, t0 + j0, n);
-    for (int c = warp; c < n; c += warps) {   // unit q and k, the token's scalars
-      float qq = 0.f, kk = 0.f, qk = 0.f;
-      for (int d = lane; d < D; d += 32) {
-        const float qv = sq[c * ROW + L::at(d)], kv = sk[c * ROW + L::at(d)];
-        qq += qv * qv;
-        kk += kv * kv;
-        qk += qv * kv;
-      }
-      qq = warp_sum(qq);
-      kk = warp_sum(kk);
-      qk = warp_sum(qk);
-      const float qi = q_scale / sqrtf(qq + 1e-6f), ki = 1.0f / sqrtf(kk + 1e-6f);
-      for (int d = lane; d < D; d += 32) {
-        sq[c * ROW + L::at(d)] *= qi;
-        sk[c * ROW + L::at(d)] *= ki;
-      }
-      if (lane == 0) sc[c * 4 + 2] = qk * qi * ki;
-    }
-    __syncthreads();
-    // One token: its key / query slices are in registers already (loaded while the token before ran); the next token's
-    // are requested first.  Four partial sums per dot product keep the multiply-add chains short.
-    auto step = [&](const float2 (&kc)[R / 2], const float2 (&qc)[R / 2], float2 (&kn)[R / 2], float2 (&qn)[R / 2], int c,
-                    bool ahead) {
-      if (ahead && c + 1 < n) {
-        load_slice<R>(kn, sk + (c + 1) * ROW + ks * L::SL);
-        load_slice<R>(qn, sq + (c + 1) * ROW + ks * L::SL);
-      }
-      const float gd = sc[c * 4 + 0], beta = sc[c * 4 + 1], kq_dot = sc[c * 4 + 2];
-      const float vj = valid ? sv[c * CW + j] : 0.f;
-      float2 dk[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, dq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-      for (int r = 0; r < R / 2; ++r) {
-        dk[r & 1] = __ffma2_rn(S[r], kc[r], dk[r & 1]);
-        dq[r & 1] = __ffma2_rn(S[r], qc[r], dq[r & 1]);
-      }
-      float dks = (dk[0].x + dk[0].y) + (dk[1].x + dk[1].y), dqs = (dq[0].x + dq[0].y) + (dq[1].x + dq[1].y);
-      slice_sum2(dks, dqs, KS);
-      const float u = beta * (vj - gd * dks);
-      if (ks == 0 && valid) so[c * CW + j] = fmaf(kq_dot, u, gd * dqs);
-      const float2 u2 = make_float2(u, u), g2 = make_float2(gd, gd);
-#pragma unroll
-      for (int r = 0; r < R / 2; ++r) S[r] = __ffma2_rn(kc[r], u2, __fmul2_rn(g2, S[r]));
-    };
-    if constexpr (R <= 16) {
-      float2 ka[R / 2], qa[R / 2], kb[R / 2], qb[R / 2];
-      load_slice<R>(ka, sk + ks * L::SL);
-      load_slice<R>(qa, sq + ks * L::SL);
-      for (int c = 0; c < n; c += 2) {
-        step(ka, qa, kb, qb, c, true);
-        if (c + 1 < n) step(kb, qb, ka, qa, c + 1, true);
-      }
-    } else {   // long slices: no registers to spare for the token ahead
-      float2 ka[R / 2], qa[R / 2];
-      for (int c = 0; c < n; ++c) {
-        load_slice<R>(ka, sk + c * ROW + ks * L::SL);
-        load_slice<R>(qa, sq + c * ROW + ks * L::SL);
-        step(ka, qa, ka, qa, c, false);
-      }
-    }
-    __syncthreads();
-    gated_unit_norm_rows<T>(a, so, part, sinv, stage, pg, h, c0, ncol, t0 + j0, n);
-    __syncthreads();
-  }
-  if (slot != a.reserved_slot) store_state<R>(S, a, slot, h, c0 + j, valid, ks);
-  if (a.VT > 1) cooperative_groups::this_cluster().sync();   // nobody leaves while its sums may still be read
-}
-
 // wkv.  r, k, v: [T, H * D] rows of the model type (row strides given); w_raw [T, H * D] decay logits (model type):
 // w = exp(-exp(w_raw + w0)); bonus [H * D] multiplies the current token's own k v^T in its read-out only.  Dv = D.
 template <typename T, int R, int MAXT>
@@ -1054,6 +900,156 @@ __device__ __forceinline__ void stage_rows(T* dst, int pitch, const T* src, int6
   }
 }
 
+// The outputs of `n` staged tokens (so [tok][CW] fp32, this CTA's columns c0 .. c0 + ncol - 1; their gate logits sg [tok][CP])
+// -> unit norm over ALL Dv columns of the head (the cluster's CTAs exchange their sums of squares, `mine` being this
+// CTA's), weight, gate; eight lanes per token.  Every CTA of the cluster calls this the same number of times.
+template <typename T>
+__device__ __forceinline__ void tile_norm_rows(const RecurArgs& a, const float* so, const T* sg, int CP, float* mine, float* sinv,
+                                               int h, int c0, int ncol, int tok0, int n, int out_pairs) {
+  namespace cg = cooperative_groups;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+  const int Dv = a.Dv, CW = a.CW;
+  for (int cb = warp * 4; cb < n; cb += warps * 4) {
+    const int c = cb + (lane >> 3);
+    float ss = 0.f;
+    if (c < n)
+      for (int j = lane & 7; j < ncol; j += 8) ss = fmaf(so[c * CW + j], so[c * CW + j], ss);
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    if ((lane & 7) == 0 && c < n) mine[c] = ss;
+  }
+  if (a.VT > 1) cg::this_cluster().sync();
+  else __syncthreads();
+  for (int c = tid; c < n; c += blockDim.x) {
+    float ss = 0.f;
+    if (a.VT > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      for (int v = 0; v < a.VT; ++v) ss += cl.map_shared_rank(mine, v)[c];
+    } else {
+      ss = mine[c];
+    }
+    sinv[c] = 1.0f / sqrtf(ss / (float)Dv + a.eps);
+  }
+  __syncthreads();
+  if (ncol > 0) {
+    T* out = static_cast<T*>(a.out);
+    auto value = [&](int c, int j) {
+      const float gz = to_f<T>(sg[c * CP + j]);
+      return so[c * CW + j] * sinv[c] * a.norm_w[h * a.norm_head_stride + c0 + j] *
+             (a.gate_kind ? sigmoid_f(gz) : silu_f(gz));
+    };
+    if (sizeof(T) == 2 && out_pairs) {
+      TileWalk w(ncol / 2);
+      for (; w.c < n; w.next())
+        *reinterpret_cast<uint32_t*>(out + (int64_t)(tok0 + w.c) * a.out_stride + h * Dv + c0 + 2 * w.d) =
+            pack2<true>(value(w.c, 2 * w.d), value(w.c, 2 * w.d + 1));
+    } else {
+      TileWalk w(ncol);
+      for (; w.c < n; w.next())
+        out[(int64_t)(tok0 + w.c) * a.out_stride + h * Dv + c0 + w.d] = from_f<T>(value(w.c, w.d));
+    }
+  }
+}
+
+// A thread's tile of the state: S[j][r] = rows (2 r, 2 r + 1 of the thread's eight) of column col0 + j.  The pool keeps
+// [slots, H, Dv, D]: a value column's key rows are contiguous, moved as 16-byte pieces when the key size allows.
+template <int KS, int C>
+__device__ __forceinline__ void load_tile(float2 (&S)[C][kGlaRows / 2], const RecurArgs& a, int slot, int h, int c0, int col0,
+                                          int ncol, int ks, bool from_pool) {
+  const int D = a.D;
+#pragma unroll
+  for (int j = 0; j < C; ++j) {
+    const bool on = from_pool && col0 + j < ncol;
+    const float* p = a.state + (((int64_t)slot * a.H + h) * a.Dv + c0 + col0 + j) * D;
+#pragma unroll
+    for (int q4 = 0; q4 < 2; ++q4) {
+      const int i = q4 * KS * 4 + ks * 4;
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on) {
+        if ((D & 3) == 0) {
+          if (i < D) t = *reinterpret_cast<const float4*>(p + i);
+        } else {
+          if (i < D) t.x = p[i];
+          if (i + 1 < D) t.y = p[i + 1];
+          if (i + 2 < D) t.z = p[i + 2];
+          if (i + 3 < D) t.w = p[i + 3];
+        }
+      }
+      S[j][q4 * 2] = make_float2(t.x, t.y);
+      S[j][q4 * 2 + 1] = make_float2(t.z, t.w);
+    }
+  }
+}
+
+template <int KS, int C>
+__device__ __forceinline__ void store_tile(const float2 (&S)[C][kGlaRows / 2], const RecurArgs& a, int slot, int h, int c0,
+                                           int col0, int ncol, int ks) {
+  const int D = a.D;
+#pragma unroll
+  for (int j = 0; j < C; ++j) {
+    if (col0 + j >= ncol) continue;
+    float* p = a.state + (((int64_t)slot * a.H + h) * a.Dv + c0 + col0 + j) * D;
+#pragma unroll
+    for (int q4 = 0; q4 < 2; ++q4) {
+      const int i = q4 * KS * 4 + ks * 4;
+      const float2 lo = S[j][q4 * 2], hi = S[j][q4 * 2 + 1];
+      if ((D & 3) == 0) {
+        if (i < D) *reinterpret_cast<float4*>(p + i) = make_float4(lo.x, lo.y, hi.x, hi.y);
+      } else {
+        if (i < D) p[i] = lo.x;
+        if (i + 1 < D) p[i + 1] = lo.y;
+        if (i + 2 < D) p[i + 2] = hi.x;
+        if (i + 3 < D) p[i + 3] = hi.y;
+      }
+    }
+  }
+}
+
+// Sums of N numbers each over 2^k neighbouring lanes (`me`: the lane's number among them), all together: every exchange
+// halves what a lane is left with (then, with one number left, adds).  Returns the index of the first of the `kept`
+// sums that end up in o[0 ..] of this lane.
+template <int LANES, int N>
+struct LaneSums {
+  static constexpr int kept = LANES < N ? N / LANES : 1;
+  __device__ static __forceinline__ int run(float (&o)[N], int me) {
+    int left = N, first = 0;
+#pragma unroll
+    for (int d = 1; d < LANES; d <<= 1) {
+      if (left > 1) {
+        const bool up = (me & d) != 0;
+        left >>= 1;
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j)
+          if (j < left) {
+            const float send = up ? o[j] : o[j + left], keep = up ? o[j + left] : o[j];
+            o[j] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+          }
+        if (up) first += left;
+      } else {
+        o[0] += __shfl_xor_sync(0xffffffffu, o[0], d);
+      }
+    }
+    return first;
+  }
+  // the way back: every lane gets all N numbers, number i in o[i]
+  __device__ static __forceinline__ void spread(float (&o)[N], int me) {
+#pragma unroll
+    for (int d = LANES / 2; d >= 1; d >>= 1) {
+      const int have = N / (2 * d);      // numbers a lane holds before this exchange (0: this exchange only added)
+      if (have >= 1) {
+        const bool up = (me & d) != 0;
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j)
+          if (j < have) {
+            const float mine = o[j], other = __shfl_xor_sync(0xffffffffu, mine, d);
+            o[j] = up ? other : mine;
+            o[j + have] = up ? mine : other;
+          }
+      }
+    }
+  }
+};
+
 template <typename T, int KS, int C, int U>
 __global__ void __launch_bounds__(512) gla_scan_kernel(const T* __restrict__ proj, GlaArgs ga, RecurArgs a) {
   namespace cg = cooperative_groups;
@@ -1099,33 +1095,8 @@ __global__ void __launch_bounds__(512) gla_scan_kernel(const T* __restrict__ pro
     for (int i = n * CP + tid; i < (n + U - 1) / U * U * CP; i += blockDim.x) sv[i] = from_f<T>(0.f);
   };
   issue(0, 0);
-  // state tile: S[j][r] = rows (2 r, 2 r + 1 of the thread's eight) of column col0 + j
   float2 S[C][kGlaRows / 2];
-  {
-    const bool from_pool = start > 0;
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const bool on = from_pool && col0 + j < ncol;
-      const float* p = a.state + (((int64_t)slot * a.H + h) * Dv + c0 + col0 + j) * D;
-#pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
-        const int i = q4 * KS * 4 + ks * 4;
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (on) {
-          if ((D & 3) == 0) {
-            if (i < D) t = *reinterpret_cast<const float4*>(p + i);
-          } else {
-            if (i < D) t.x = p[i];
-            if (i + 1 < D) t.y = p[i + 1];
-            if (i + 2 < D) t.z = p[i + 2];
-            if (i + 3 < D) t.w = p[i + 3];
-          }
-        }
-        S[j][q4 * 2] = make_float2(t.x, t.y);
-        S[j][q4 * 2 + 1] = make_float2(t.z, t.w);
-      }
-    }
-  }
+  load_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks, start > 0);
   if (D != DP)   // rows beyond D: zero keys, queries and decays, written once
     for (int i = tid; i < (2 * tok + tok / U) * DP; i += blockDim.x) tq[i] = 0.f;
   int stage = 0;
@@ -1175,24 +1146,8 @@ __global__ void __launch_bounds__(512) gla_scan_kernel(const T* __restrict__ pro
       if constexpr (U == 1) {
         pp[0] = warp_sum(pp[0]);
         if (lane == 0) tp[blk] = pp[0];
-      } else {   // U * U <= 32 sums over the lanes: each exchange halves what a lane is left with
-        int left = U * U, first = 0;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          if (left > 1) {
-            const bool up = (lane & d) != 0;
-            left >>= 1;
-#pragma unroll
-            for (int j = 0; j < U * U / 2; ++j)
-              if (j < left) {
-                const float send = up ? pp[j] : pp[j + left], keep = up ? pp[j + left] : pp[j];
-                pp[j] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-              }
-            if (up) first += left;
-          } else {
-            pp[0] += __shfl_xor_sync(0xffffffffu, pp[0], d);
-          }
-        }
+      } else {
+        const int first = LaneSums<32, U * U>::run(pp, lane);
         if (lane < U * U) tp[blk * U * U + first] = pp[0];
       }
     }
@@ -1244,25 +1199,10 @@ __global__ void __launch_bounds__(512) gla_scan_kernel(const T* __restrict__ pro
             S[j][3] = __ffma2_rn(make_float2(k1.z, k1.w), v2, S[j][3]);
           }
         }
-        // sums over the key lanes of all U * C outputs together, halving as above; the lane a sum ends up with adds what
-        // the token reads of the block itself
-        int left = NV, first = 0;
-#pragma unroll
-        for (int d = 1; d < KS; d <<= 1) {
-          if (left > 1) {
-            const bool up = (ks & d) != 0;
-            left >>= 1;
-#pragma unroll
-            for (int j = 0; j < NV / 2; ++j)
-              if (j < left) {
-                const float send = up ? o[j] : o[j + left], keep = up ? o[j + left] : o[j];
-                o[j] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-              }
-            if (up) first += left;
-          } else {
-            o[0] += __shfl_xor_sync(0xffffffffu, o[0], d);
-          }
-        }
+        // sums over the key lanes of all U * C outputs together; the lane a sum ends up with adds what the token reads of
+        // the block itself
+        constexpr int left = LaneSums<KS, NV>::kept;
+        const int first = LaneSums<KS, NV>::run(o, ks);
         if (KS <= NV || ks < NV) {
 #pragma unroll
           for (int j = 0; j < NV; ++j)
@@ -1280,72 +1220,555 @@ __global__ void __launch_bounds__(512) gla_scan_kernel(const T* __restrict__ pro
       }
     }
     __syncthreads();
-    // unit norm over ALL Dv columns of the head (the cluster's CTAs exchange their sums of squares), weight, gate;
-    // eight lanes per token
-    float* mine = part + (stage & 1) * kGlaTok;
-    for (int cb = warp * 4; cb < n; cb += warps * 4) {
-      const int c = cb + (lane >> 3);
-      float ss = 0.f;
-      if (c < n)
-        for (int j = lane & 7; j < ncol; j += 8) ss = fmaf(so[c * CW + j], so[c * CW + j], ss);
-#pragma unroll
-      for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-      if ((lane & 7) == 0 && c < n) mine[c] = ss;
-    }
-    if (a.VT > 1) cg::this_cluster().sync();
-    else __syncthreads();
-    for (int c = tid; c < n; c += blockDim.x) {
-      float ss = 0.f;
-      if (a.VT > 1) {
-        cg::cluster_group cl = cg::this_cluster();
-        for (int v = 0; v < a.VT; ++v) ss += cl.map_shared_rank(mine, v)[c];
-      } else {
-        ss = mine[c];
-      }
-      sinv[c] = 1.0f / sqrtf(ss / (float)Dv + a.eps);
-    }
-    __syncthreads();
-    if (ncol > 0) {
-      T* out = static_cast<T*>(a.out);
-      auto value = [&](int c, int j) {
-        const float gz = to_f<T>(sg[c * CP + j]);
-        return so[c * CW + j] * sinv[c] * a.norm_w[h * a.norm_head_stride + c0 + j] *
-               (a.gate_kind ? sigmoid_f(gz) : silu_f(gz));
-      };
-      if (sizeof(T) == 2 && ga.out_pairs) {
-        TileWalk w(ncol / 2);
-        for (; w.c < n; w.next())
-          *reinterpret_cast<uint32_t*>(out + (int64_t)(t0 + j0 + w.c) * a.out_stride + h * Dv + c0 + 2 * w.d) =
-              pack2<true>(value(w.c, 2 * w.d), value(w.c, 2 * w.d + 1));
-      } else {
-        TileWalk w(ncol);
-        for (; w.c < n; w.next())
-          out[(int64_t)(t0 + j0 + w.c) * a.out_stride + h * Dv + c0 + w.d] = from_f<T>(value(w.c, w.d));
-      }
-    }
+    tile_norm_rows<T>(a, so, sg, CP, part + (stage & 1) * kGlaTok, sinv, h, c0, ncol, t0 + j0, n, ga.out_pairs);
     __syncthreads();
   }
-  if (slot != a.reserved_slot) {
+  if (slot != a.reserved_slot) store_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks);
+  if (a.VT > 1) cg::this_cluster().sync();   // nobody leaves while its sums may still be read
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Gated delta rule.  qkv [T, 2 G D + H Dv] fp32 = (q | k | v) after the short convolution; beta and decay logits are
+// columns b_off + h and a_off + h of proj (model type).  Head h reads q / k head h / (H / G).  The state tile of a thread
+// is the gated linear attention's, and so are the blocks of U tokens.  With S the state before a block, its tokens
+// counted 0 .. U - 1, q and k the unit vectors, w_ts = g_(s+1) .. g_t and g_0t = g_0 .. g_t (products, never quotients),
+// what token t writes is k_t u_t^T with
+//   u_t = beta_t (v_t - g_0t S^T k_t) - sum_(s < t) beta_t w_ts (k_t . k_s) u_s
+// - a triangular system of U unknowns whose matrix the value columns share.  With M its inverse (times diag(beta)) and
+// P = (w_ts (q_t . k_s)) M,
+//   u_t = sum_s M_ts (v_s - g_0s S^T k_s)
+//   o_t = g_0t S^T q_t + sum_s P_ts (v_s - g_0s S^T k_s)
+//   S  <- g_0(U-1) S + sum_s w_(U-1)s k_s u_s^T
+// so a block takes one pass over the registers for 2 U dot products with the rows as they come and one for the update,
+// where token by token the state takes U of each; only the sums S^T k (over the key lanes) stand between a block and the
+// next.  The unit lengths, decays and betas are all in the block's coefficients (DeltaCoef), made once per CTA.
+// ---------------------------------------------------------------------------------------------------------
+struct DeltaArgs {
+  int b_off, a_off, G;
+  int64_t qkv_stride, proj_stride;
+  const float *A_log, *dt_bias;
+  int vec_key, vec_val;   // key rows / value rows move as 16-byte pieces
+  int CP;                 // staged value row: CW rounded up to 8
+};
+
+// A block's coefficients on its raw rows: uv, uk: [U][U] w_(U-1)t u_t = sum_s uv_ts v_s - uk_ts S^T k_s;  ov, ok: [U][U] and
+// oq [U]: o_t = oq_t S^T q_t + sum_s ov_ts v_s - ok_ts S^T k_s;  decay of the state.
+template <int U>
+struct DeltaCoef {
+  static constexpr int kTri = U * (U + 1) / 2;
+  static constexpr int kDots = U == 1 ? 4 : 32;   // q_t . q_t | k_t . k_s, s <= t | q_t . k_s, s <= t
+  static_assert(U + 2 * kTri <= kDots, "one sum per lane");
+  static constexpr int uv = 0, uk = U * U, ov = 2 * U * U, ok = 3 * U * U, oq = 4 * U * U, decay = 4 * U * U + U;
+  static constexpr int size = (4 * U * U + U + 1 + 3) / 4 * 4;
+
+  // one warp: the block's dot products -> dots[kDots]; rows zero beyond D up to DP
+  template <int DP>
+  __device__ static __forceinline__ void make_dots(const float* rq, const float* rk, float* dots) {
+    const int lane = threadIdx.x & 31;
+    float p[kDots];
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      if (col0 + j >= ncol) continue;
-      float* p = a.state + (((int64_t)slot * a.H + h) * Dv + c0 + col0 + j) * D;
+    for (int i = 0; i < kDots; ++i) p[i] = 0.f;
+    auto dot4 = [](float4 x, float4 y, float acc) {
+      return fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, acc))));
+    };
 #pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
-        const int i = q4 * KS * 4 + ks * 4;
-        const float2 lo = S[j][q4 * 2], hi = S[j][q4 * 2 + 1];
-        if ((D & 3) == 0) {
-          if (i < D) *reinterpret_cast<float4*>(p + i) = make_float4(lo.x, lo.y, hi.x, hi.y);
-        } else {
-          if (i < D) p[i] = lo.x;
-          if (i + 1 < D) p[i + 1] = lo.y;
-          if (i + 2 < D) p[i + 2] = hi.x;
-          if (i + 3 < D) p[i + 3] = hi.y;
+    for (int it = 0; it < (DP + 127) / 128; ++it) {
+      const int d = it * 128 + lane * 4;
+      if (d < DP) {
+        float4 q[U], k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          q[u] = *reinterpret_cast<const float4*>(rq + u * DP + d);
+          k[u] = *reinterpret_cast<const float4*>(rk + u * DP + d);
+        }
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+          p[t] = dot4(q[t], q[t], p[t]);
+#pragma unroll
+          for (int s = 0; s <= t; ++s) {
+            p[U + t * (t + 1) / 2 + s] = dot4(k[t], k[s], p[U + t * (t + 1) / 2 + s]);
+            p[U + kTri + t * (t + 1) / 2 + s] = dot4(q[t], k[s], p[U + kTri + t * (t + 1) / 2 + s]);
+          }
         }
       }
     }
+    const int first = LaneSums<32, kDots>::run(p, lane);
+    if (lane < kDots) dots[first] = p[0];
   }
+  // inverse lengths of a block's token t from its dot products
+  __device__ static __forceinline__ float q_inv(const float* dots, int t, float q_scale) {
+    return q_scale / sqrtf(dots[t] + 1e-6f);
+  }
+  __device__ static __forceinline__ float k_inv(const float* dots, int t) {
+    return 1.0f / sqrtf(dots[U + t * (t + 1) / 2 + t] + 1e-6f);
+  }
+
+  // one thread: the coefficients from the dot products, decays, betas and the inverse lengths of q (scaled) and k; missing
+  // tokens come with decay 1, beta 0 and zero rows
+  __device__ static __forceinline__ void make(const float* dots, const float (&g)[U], const float (&be)[U],
+                                              const float (&qi)[U], const float (&ki)[U], float* cf) {
+    float g0[U], M[U][U];
+#pragma unroll
+    for (int t = 0; t < U; ++t) g0[t] = t ? g0[t > 0 ? t - 1 : 0] * g[t] : g[t];
+#pragma unroll
+    for (int t = 0; t < U; ++t) {   // row t of the inverse, by forward substitution
+#pragma unroll
+      for (int s = 0; s < U; ++s) M[t][s] = s == t ? be[t] : 0.f;
+      float w = g[t];
+#pragma unroll
+      for (int r = t - 1; r >= 0; --r) {
+        const float x = be[t] * w * (dots[U + t * (t + 1) / 2 + r] * ki[t] * ki[r]);
+#pragma unroll
+        for (int s = 0; s <= r; ++s) M[t][s] = fmaf(-x, M[r][s], M[t][s]);
+        w *= g[r];
+      }
+    }
+    float we[U];   // w_(U-1)t, with the unit length of the key that it multiplies
+    {
+      float w = 1.f;
+#pragma unroll
+      for (int s = U - 1; s >= 0; --s) {
+        we[s] = w * ki[s];
+        w *= g[s];
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < U; ++t) {
+      float P[U];
+#pragma unroll
+      for (int s = 0; s < U; ++s) P[s] = 0.f;
+      float w = 1.f;
+#pragma unroll
+      for (int r = t; r >= 0; --r) {
+        const float x = w * (dots[U + kTri + t * (t + 1) / 2 + r] * qi[t] * ki[r]);
+#pragma unroll
+        for (int s = 0; s <= r; ++s) P[s] = fmaf(x, M[r][s], P[s]);
+        w *= g[r];
+      }
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        const float gk = g0[s] * ki[s];
+        cf[uv + t * U + s] = we[t] * M[t][s];
+        cf[uk + t * U + s] = we[t] * (M[t][s] * gk);
+        cf[ov + t * U + s] = P[s];
+        cf[ok + t * U + s] = P[s] * gk;
+      }
+      cf[oq + t] = g0[t] * qi[t];
+    }
+    cf[decay] = g0[U - 1];
+  }
+};
+
+// What a block does to a thread's tile, in two parts: `block` brings the tile from before the block to behind it and leaves
+// what the read-outs need in a Pending; `finish` sums the read-outs over the key lanes and stores them.  A warp stands
+// still while its sums cross the lanes, so a block's `finish` is put beside the next block's products.
+template <int KS, int C, int U>
+struct DeltaTile {
+  using Coef = DeltaCoef<U>;
+  static constexpr int DP = KS * kGlaRows, NV = U * C;
+  static constexpr int kept = LaneSums<KS, NV>::kept;   // sums that land in a lane, numbered token * C + column
+
+  struct Pending {
+    float dq[NV], w[NV], v[U][C];   // the lane's part of S^T q; S^T k and the value rows
+    const float* cf;
+    float* so;
+  };
+
+  __device__ static __forceinline__ void load_row(float2 (&x)[kGlaRows / 2], const float* row, int at) {
+    const float4 a = *reinterpret_cast<const float4*>(row + at), b = *reinterpret_cast<const float4*>(row + KS * 4 + at);
+    x[0] = make_float2(a.x, a.y);
+    x[1] = make_float2(a.z, a.w);
+    x[2] = make_float2(b.x, b.y);
+    x[3] = make_float2(b.z, b.w);
+  }
+  template <int N>
+  __device__ static __forceinline__ void load_n(float (&x)[N], const float* p) {   // N numbers at a multiple of N
+    if constexpr (N == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(p);
+      x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+    } else if constexpr (N == 2) {
+      const float2 t = *reinterpret_cast<const float2*>(p);
+      x[0] = t.x, x[1] = t.y;
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] = p[i];
+    }
+  }
+  __device__ static __forceinline__ void dot(float (&sums)[NV], int t, const float2 (&S)[C][kGlaRows / 2],
+                                             const float2 (&x)[kGlaRows / 2]) {
+    float2 o2[C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) o2[j] = __fmul2_rn(x[0], S[j][0]);
+#pragma unroll
+    for (int r = 1; r < kGlaRows / 2; ++r)
+#pragma unroll
+      for (int j = 0; j < C; ++j) o2[j] = __ffma2_rn(x[r], S[j][r], o2[j]);
+#pragma unroll
+    for (int j = 0; j < C; ++j) sums[t * C + j] = o2[j].x + o2[j].y;
+  }
+
+  // CP: pitch of the output rows; of the thread's columns `cols` exist
+  __device__ static __forceinline__ void finish(Pending& p, int CP, int cols, int ks) {
+    const int first = LaneSums<KS, NV>::run(p.dq, ks);
+#pragma unroll
+    for (int j = 0; j < kept; ++j) {
+      const int t = (first + j) / C, c = (first + j) % C;
+      float pv[U], pk[U];
+      load_n<U>(pv, p.cf + Coef::ov + t * U);
+      load_n<U>(pk, p.cf + Coef::ok + t * U);
+      float o = p.cf[Coef::oq + t] * p.dq[j];
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        float vs = p.v[s][0], ws = p.w[s * C];
+#pragma unroll
+        for (int i = 1; i < C; ++i) {
+          vs = c == i ? p.v[s][i] : vs;
+          ws = c == i ? p.w[s * C + i] : ws;
+        }
+        o = fmaf(pv[s], vs, fmaf(-pk[s], ws, o));
+      }
+      if (c < cols && (KS <= NV || ks < NV)) p.so[t * CP + c] = o;
+    }
+  }
+
+  // rk, rq: the block's key and query rows (pitch DP), cf its coefficients; sv its value rows and so its output rows (pitch
+  // CP), both from the thread's first column on.  PREV: `pend` holds the block before, which is finished on the way.
+  template <bool PREV>
+  __device__ static __forceinline__ void block(float2 (&S)[C][kGlaRows / 2], Pending& pend, const float* rk, const float* rq,
+                                               const float* cf, const float* sv, float* so, int CP, int cols, int ks) {
+    const int at = ks * 4;
+    float2 k[U][kGlaRows / 2];
+    float w[NV];
+#pragma unroll
+    for (int t = 0; t < U; ++t) load_row(k[t], rk + t * DP, at);
+#pragma unroll
+    for (int t = 0; t < U; ++t) dot(w, t, S, k[t]);
+    if constexpr (PREV) finish(pend, CP, cols, ks);
+    LaneSums<KS, NV>::run(w, ks);
+#pragma unroll
+    for (int t = 0; t < U; ++t) {
+      float2 q[kGlaRows / 2];
+      load_row(q, rq + t * DP, at);
+      dot(pend.dq, t, S, q);
+    }
+#pragma unroll
+    for (int s = 0; s < U; ++s) load_n<C>(pend.v[s], sv + s * CP);
+    LaneSums<KS, NV>::spread(w, ks);
+    const float2 g2 = make_float2(cf[Coef::decay], cf[Coef::decay]);
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+#pragma unroll
+      for (int r = 0; r < kGlaRows / 2; ++r) S[j][r] = __fmul2_rn(g2, S[j][r]);
+#pragma unroll
+    for (int t = 0; t < U; ++t) {
+      float uv[U], uk[U], u[C];
+      load_n<U>(uv, cf + Coef::uv + t * U);
+      load_n<U>(uk, cf + Coef::uk + t * U);
+#pragma unroll
+      for (int j = 0; j < C; ++j) u[j] = 0.f;
+#pragma unroll
+      for (int s = 0; s <= t; ++s)
+#pragma unroll
+        for (int j = 0; j < C; ++j) u[j] = fmaf(uv[s], pend.v[s][j], fmaf(-uk[s], w[s * C + j], u[j]));
+#pragma unroll
+      for (int j = 0; j < C; ++j)
+#pragma unroll
+        for (int r = 0; r < kGlaRows / 2; ++r) S[j][r] = __ffma2_rn(k[t][r], make_float2(u[j], u[j]), S[j][r]);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) pend.w[i] = w[i];
+    pend.cf = cf;
+    pend.so = so;
+  }
+};
+
+// One token per sequence: the state's trip through the registers is the step.
+template <typename T, int KS>
+__global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict__ qkv, const T* __restrict__ proj,
+                                                         DeltaArgs da, RecurArgs a) {
+  namespace cg = cooperative_groups;
+  constexpr int C = 4, DP = KS * kGlaRows;
+  using Tile = DeltaTile<KS, C, 1>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int D = a.D, Dv = a.Dv, CW = a.CW, CP = da.CP;
+  float* raw = reinterpret_cast<float*>(smraw);   // [2][DP] q, k
+  float* cf = raw + 2 * DP;                       // [8] coefficients
+  float* dots = cf + 8;                           // [4]
+  float* sv = dots + 4;                           // [CP]
+  float* so = sv + CP;                            // [CP]
+  float* part = so + CP;                          // [4]: this CTA's sum of squares, 1 / rms
+  T* sg = reinterpret_cast<T*>(part + 4);         // [CP]
+  const int h = blockIdx.x / a.VT, vt = blockIdx.x % a.VT, b = blockIdx.y;
+  int t0, n_new, start;
+  portion(a.g, b, t0, n_new, start);
+  if (n_new <= 0) return;               // the same for every CTA of the cluster
+  const int slot = a.g.slots[b];
+  const int kvh = h / (a.H / da.G);
+  const int c0 = vt * CW, ncol = max(0, min(CW, Dv - c0));
+  const int tid = threadIdx.x, ks = tid % KS, col0 = tid / KS * C;
+  float2 S[C][kGlaRows / 2];
+  load_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks, start > 0);
+  const float* row = qkv + (int64_t)t0 * da.qkv_stride;
+  const T* gate = static_cast<const T*>(a.gate) + (int64_t)t0 * a.gate_stride + a.gate_off + h * Dv + c0;
+  for (int i = tid; i < DP; i += blockDim.x) {
+    raw[i] = i < D ? row[kvh * D + i] : 0.f;
+    raw[DP + i] = i < D ? row[da.G * D + kvh * D + i] : 0.f;
+  }
+  for (int i = tid; i < CP; i += blockDim.x) {
+    sv[i] = i < ncol ? row[2 * da.G * D + h * Dv + c0 + i] : 0.f;
+    if (i < ncol) sg[i] = gate[i];
+  }
+  const T* pr = proj + (int64_t)t0 * da.proj_stride;
+  const float g[1] = {expf(-expf(da.A_log[h]) * softplus_f(to_f<T>(pr[da.a_off + h]) + da.dt_bias[h]))};
+  const float be[1] = {sigmoid_f(to_f<T>(pr[da.b_off + h]))};
+  __syncthreads();
+  if (tid < 32) {
+    DeltaCoef<1>::make_dots<DP>(raw, raw + DP, dots);
+    __syncwarp();
+    if (tid == 0) {
+      const float qi[1] = {DeltaCoef<1>::q_inv(dots, 0, rsqrtf((float)D))}, ki[1] = {DeltaCoef<1>::k_inv(dots, 0)};
+      DeltaCoef<1>::make(dots, g, be, qi, ki, cf);
+    }
+  }
+  __syncthreads();
+  typename Tile::Pending pend;
+  Tile::template block<false>(S, pend, raw + DP, raw, cf, sv + col0, so + col0, CP, ncol - col0, ks);
+  Tile::finish(pend, CP, ncol - col0, ks);
+  if (slot != a.reserved_slot) store_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks);
+  __syncthreads();
+  tile_norm_rows<T>(a, so, sg, CP, part, part + 1, h, c0, ncol, t0, 1, 0);
   if (a.VT > 1) cg::this_cluster().sync();   // nobody leaves while its sums may still be read
+}
+
+// Portions.  A cluster of VT CTAs serves one (head, sequence); each keeps CW value columns.  Warps have one of two roles:
+// `warps` main warps take the blocks through their state tiles; four others work for the stages (`tok` tokens) around the
+// one the main warps are in: they load q, k and v of the stage after next (cp.async), make the next stage's coefficients
+// and finish the outputs of the stages before (sums of squares, exchanged through distributed shared memory, then norm,
+// weight, gate).  One cluster barrier per stage orders all of it:
+//   iteration s, main warps: blocks of stage s, from R[s % 3], coefficients [s & 1] and V[s % 3]; outputs to O[s % 3]
+//                others:     R, V[(s + 2) % 3] <- stage s + 2;  coefficients [(s + 1) & 1] <- R[(s + 1) % 3];
+//                            sums of squares of stage s - 1;  outputs of stage s - 2
+// Measured on the way (one portion of 4096 tokens, 32 heads of 128 x 128, with convolution and output product, which take
+// 0.19 ms): token by token 2.35 ms; blocks, with the phases of a stage of 32 tokens one after the other, 1.63 ms (cycles a
+// stage: key and query rows transformed by the coefficients 4.7 k, loads 3.4 k, blocks 9.6 k, norm 4.5 k); transformed rows
+// sent to the cluster's other CTAs as plain stores into distributed shared memory 3.6 ms (12 k 16-byte stores a stage); raw
+// rows, roles, a block's read-outs finished before the next block starts 1.67 ms (main warps 13 k cycles a stage, the
+// others 21 k: divisions, loads waited for at their conversion); this form 1.31 ms (12.8 k and 16.5 k).
+// What bounds it: instruction issue of the blocks (about half of it the 3.25 multiply-adds per state number and token) and
+// the latency of the exchange over the key lanes, two main warps a scheduler.
+constexpr int kDeltaHelpers = 4;   // warps
+constexpr int kDeltaMain = 8;      // most main warps
+
+template <typename T, int KS, int C>
+__global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers) * 32, 1)
+delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, DeltaArgs da, RecurArgs a) {
+  namespace cg = cooperative_groups;
+  constexpr int U = kGlaBlock, DP = KS * kGlaRows;
+  using Coef = DeltaCoef<U>;
+  using Tile = DeltaTile<KS, C, U>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int D = a.D, Dv = a.Dv, H = a.H, CW = a.CW, CP = da.CP, tok = a.tok, VT = a.VT;
+  float* R = reinterpret_cast<float*>(smraw);             // [3][q, k][tok][DP]
+  float* cf = R + 6 * tok * DP;                           // [2][tok / U][Coef::size]
+  float* V = cf + 2 * (tok / U) * Coef::size;             // [3][tok][CP]
+  float* O = V + 3 * tok * CP;                            // [3][tok][CP]
+  float* dots = O + 3 * tok * CP;                         // [tok / U][kDots]
+  float* part = dots + tok / U * Coef::kDots;             // [2][VT][tok] sums of squares of the cluster's CTAs
+  const int h = blockIdx.x / VT, vt = blockIdx.x % VT, b = blockIdx.y;
+  int t0, n_new, start;
+  portion(a.g, b, t0, n_new, start);
+  if (n_new <= 0) return;               // the same for every CTA of the cluster
+  const int slot = a.g.slots[b];
+  const int kvh = h / (H / da.G);
+  const int c0 = vt * CW, ncol = max(0, min(CW, Dv - c0));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int main_warps = (blockDim.x >> 5) - kDeltaHelpers;
+  const bool helper = warp >= main_warps;
+  const int stages = cdiv(n_new, tok);
+  auto sync_all = [&]() {
+    if (VT > 1) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  if (D != DP)   // rows beyond D stay zero
+    for (int i = tid; i < 6 * tok * DP; i += blockDim.x) R[i] = 0.f;
+  sync_all();   // before the first copies into R, and: every CTA of the cluster runs before another writes to it
+
+  // ---- main warps ----
+  const int ks = tid % KS, col0 = tid / KS * C;   // first column (of the CTA's) of a main thread
+  float2 S[C][kGlaRows / 2];
+  if (!helper) load_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks, start > 0);
+
+  // ---- the others ----
+  const int hw = warp - main_warps, ht = hw * 32 + lane;
+  constexpr int kHT = kDeltaHelpers * 32;
+  const float neg_a = -expf(da.A_log[h]), dtb = da.dt_bias[h];
+  const float q_scale = rsqrtf((float)D);
+  T la = from_f<T>(0.f), lb = la;   // decay and beta logits of the next stage's token `lane` (first of these warps)
+  // `rows` rows of `len` numbers -> shared rows of `pitch`, 16 bytes at a time where `vec`
+  auto stage_in = [&](float* dst, int pitch, const float* src, int len, int rows, bool vec) {
+    const int E = vec ? 4 : 1, per = len / E;
+    if (per <= 0) return;
+    int c = ht / per, d = ht - c * per;
+    const int sc = kHT / per, sd = kHT - sc * per;
+    while (c < rows) {
+      if (vec) cp_async16(dst + c * pitch + d * 4, src + c * da.qkv_stride + d * 4);
+      else dst[c * pitch + d] = src[c * da.qkv_stride + d];
+      c += sc;
+      d += sd;
+      if (d >= per) { d -= per; ++c; }
+    }
+  };
+  auto issue = [&](int s) {
+    const int n = min(tok, n_new - s * tok);
+    const float* row = qkv + (int64_t)(t0 + s * tok) * da.qkv_stride;
+    float *dq = R + s % 3 * 2 * tok * DP, *sv = V + s % 3 * tok * CP;
+    stage_in(dq, DP, row + kvh * D, D, n, da.vec_key);
+    stage_in(dq + tok * DP, DP, row + da.G * D + kvh * D, D, n, da.vec_key);
+    stage_in(sv, CP, row + 2 * da.G * D + h * Dv + c0, ncol, n, da.vec_val);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // the last block's missing tokens: zero rows (0 * garbage)
+    const int n_up = cdiv(n, U) * U;
+    if (n_up != n) {
+      for (int i = n * CP + ht; i < n_up * CP; i += kHT) sv[i] = 0.f;
+      for (int i = n * DP + ht; i < n_up * DP; i += kHT) dq[i] = dq[tok * DP + i] = 0.f;
+    }
+    if (hw == 0 && lane < n) {
+      const T* pr = proj + (int64_t)(t0 + s * tok + lane) * da.proj_stride;
+      la = pr[da.a_off + h];
+      lb = pr[da.b_off + h];
+    }
+  };
+  auto help_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kHT) : "memory"); };
+  // outputs: such a thread keeps to one column (its weight in a register) and takes every out_rows-th token
+  constexpr int kGate = 16;   // gate logits that it loads ahead of their use
+  const bool by_column = ncol > 0 && ncol <= kHT;
+  const int out_rows = by_column ? kHT / ncol : 1, out_c = by_column ? ht / ncol : 0;
+  const int out_j = by_column ? ht - out_c * ncol : 0;
+  const bool out_on = helper && by_column && out_c < out_rows;
+  const float out_w = out_on ? a.norm_w[h * a.norm_head_stride + c0 + out_j] : 0.f;
+  T* const out = static_cast<T*>(a.out) + (int64_t)t0 * a.out_stride + h * Dv + c0;
+  const T* const gate = static_cast<const T*>(a.gate) + (int64_t)t0 * a.gate_stride + a.gate_off + h * Dv + c0;
+
+  if (helper) issue(0);
+  for (int s = -1; s <= stages + 1; ++s) {
+    if (!helper) {
+      if (s >= 0 && s < stages) {
+        const int blocks = cdiv(min(tok, n_new - s * tok), U);
+        const float *rq = R + s % 3 * 2 * tok * DP, *c = cf + (s & 1) * (tok / U) * Coef::size;
+        const float *rk = rq + tok * DP, *sv = V + s % 3 * tok * CP + col0;
+        float* so = O + s % 3 * tok * CP + col0;
+        typename Tile::Pending pend;
+        Tile::template block<false>(S, pend, rk, rq, c, sv, so, CP, ncol - col0, ks);
+        for (int blk = 1; blk < blocks; ++blk) {
+          rk += U * DP;
+          rq += U * DP;
+          c += Coef::size;
+          sv += U * CP;
+          so += U * CP;
+          Tile::template block<true>(S, pend, rk, rq, c, sv, so, CP, ncol - col0, ks);
+        }
+        Tile::finish(pend, CP, ncol - col0, ks);
+      }
+    } else {
+      // gates of stage s - 2, used at the end
+      const int e = s - 2, n_e = e >= 0 ? min(tok, n_new - e * tok) : 0;
+      T pg[kGate];
+      {
+        const T* g = gate + (int64_t)(e * tok + out_c) * a.gate_stride + out_j;
+#pragma unroll
+        for (int u = 0; u < kGate; ++u) {
+          if (out_on && out_c + u * out_rows < n_e) pg[u] = *g;
+          g += (int64_t)out_rows * a.gate_stride;
+        }
+      }
+      if (s + 1 < stages) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        help_sync();
+        const float g_tok = expf(neg_a * softplus_f(to_f<T>(la) + dtb)), b_tok = sigmoid_f(to_f<T>(lb));
+        if (s + 2 < stages) issue(s + 2);
+        const int n = min(tok, n_new - (s + 1) * tok), blocks = cdiv(n, U);
+        const float* rq = R + (s + 1) % 3 * 2 * tok * DP;
+        for (int blk = hw; blk < blocks; blk += kDeltaHelpers)
+          Coef::template make_dots<DP>(rq + blk * U * DP, rq + (tok + blk * U) * DP, dots + blk * Coef::kDots);
+        help_sync();
+        if (hw == 0) {   // a lane per token, then a lane per block
+          const float* dt = dots + min(lane / U, blocks - 1) * Coef::kDots;
+          const float q_tok = Coef::q_inv(dt, lane % U, q_scale), k_tok = Coef::k_inv(dt, lane % U);
+          float g[U], be[U], qi[U], ki[U];
+#pragma unroll
+          for (int t = 0; t < U; ++t) {
+            const int from = (lane * U + t) & 31;
+            g[t] = __shfl_sync(0xffffffffu, g_tok, from);
+            be[t] = __shfl_sync(0xffffffffu, b_tok, from);
+            qi[t] = __shfl_sync(0xffffffffu, q_tok, from);
+            ki[t] = __shfl_sync(0xffffffffu, k_tok, from);
+            if (lane * U + t >= n) g[t] = 1.f, be[t] = 0.f;
+          }
+          if (lane < blocks)
+            Coef::make(dots + lane * Coef::kDots, g, be, qi, ki, cf + (((s + 1) & 1) * (tok / U) + lane) * Coef::size);
+        }
+      }
+      if (s >= 1 && s <= stages) {   // sums of squares of stage s - 1, eight lanes per token
+        const int n = min(tok, n_new - (s - 1) * tok);
+        const float* so = O + (s - 1) % 3 * tok * CP;
+        for (int c = ht >> 3; c - (ht >> 3) < n; c += kHT / 8) {
+          float ss = 0.f;
+          if (c < n)
+            for (int j = lane & 7; j < ncol; j += 8) ss = fmaf(so[c * CP + j], so[c * CP + j], ss);
+#pragma unroll
+          for (int d = 4; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+          float* at = part + ((s - 1) & 1) * VT * tok + vt * tok + c;
+          if (VT == 1) {
+            if ((lane & 7) == 0 && c < n) *at = ss;
+          } else if ((lane & 7) < VT && c < n) {
+            *cg::this_cluster().map_shared_rank(at, lane & 7) = ss;
+          }
+        }
+      }
+      if (e >= 0 && ncol > 0) {   // outputs of stage s - 2
+        const float* so = O + e % 3 * tok * CP;
+        float inv = 0.f;          // of token `lane` (a stage has at most 32)
+        if (lane < n_e) {
+          const float* sums = part + (e & 1) * VT * tok + lane;
+          float ss = 0.f;
+          for (int v = 0; v < VT; ++v) ss += sums[v * tok];
+          inv = 1.0f / sqrtf(ss / (float)Dv + a.eps);
+        }
+        auto value = [&](float x, float w, float gz) { return from_f<T>(x * w * (a.gate_kind ? sigmoid_f(gz) : silu_f(gz))); };
+        if (by_column) {
+          T* o = out + (int64_t)(e * tok + out_c) * a.out_stride + out_j;
+          const float* x = so + out_c * CP + out_j;
+#pragma unroll
+          for (int u = 0; u < kGate; ++u) {
+            const int c = out_c + u * out_rows;
+            if (u * out_rows < n_e) {
+              const float iv = __shfl_sync(0xffffffffu, inv, c & 31);
+              if (out_on && c < n_e) *o = value(*x * iv, out_w, to_f<T>(pg[u]));
+            }
+            o += (int64_t)out_rows * a.out_stride;
+            x += out_rows * CP;
+          }
+          for (int u = kGate; u * out_rows < n_e; ++u) {
+            const int c = out_c + u * out_rows;
+            const float iv = __shfl_sync(0xffffffffu, inv, c & 31);
+            if (out_on && c < n_e)
+              out[(int64_t)(e * tok + c) * a.out_stride + out_j] =
+                  value(so[c * CP + out_j] * iv, out_w, to_f<T>(gate[(int64_t)(e * tok + c) * a.gate_stride + out_j]));
+          }
+        } else {
+          for (int c = 0; c < n_e; ++c) {
+            const float iv = __shfl_sync(0xffffffffu, inv, c);
+            for (int j = ht; j < ncol; j += kHT)
+              out[(int64_t)(e * tok + c) * a.out_stride + j] =
+                  value(so[c * CP + j] * iv, a.norm_w[h * a.norm_head_stride + c0 + j],
+                        to_f<T>(gate[(int64_t)(e * tok + c) * a.gate_stride + j]));
+          }
+        }
+      }
+    }
+    if (s <= stages) sync_all();
+  }
+  if (!helper && slot != a.reserved_slot) store_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks);
 }
 
 // How a (head, sequence) of the gated linear attention is laid out: KS key lanes, C columns per thread, `warps` warps per
@@ -1380,6 +1803,50 @@ inline GlaShape gla_shape(int D, int Dv, int64_t pairs, int max_new, size_t elem
   s.tok = s.U;
   while (s.tok < kGlaTok && s.tok < max_new) s.tok <<= 1;
   while (s.tok > s.U && s.smem(elem) > 110 * 1024) s.tok >>= 1;
+  return s;
+}
+
+// ... of the delta rule: the same tiles.  Portions: at most eight main warps per CTA (two per scheduler); two columns per
+// thread instead of four while that leaves schedulers idle, and a head spread over more CTAs while that leaves SMs idle
+// (up to four: clusters of eight do not fill the GPU's processing clusters; 16 heads of 128 x 128, 3000 tokens: 0.89 ms
+// over four CTAs each, 1.34 ms over eight).  Stages of 32 tokens, shorter ones for short portions and where key rows are long (three stages' rows are held).
+struct DeltaShape {
+  int KS, C, VT, warps, CW, CP, tok;
+  size_t smem(size_t elem) const {
+    const size_t DP = (size_t)KS * kGlaRows, U = kGlaBlock;
+    if (tok == 0) return sizeof(float) * (2 * DP + 16 + 2 * (size_t)CP) + elem * CP;   // single tokens
+    return sizeof(float) * (6 * tok * DP + tok / U * (2 * DeltaCoef<kGlaBlock>::size + DeltaCoef<kGlaBlock>::kDots) +
+                            6 * (size_t)tok * CP + 2 * (size_t)VT * tok);
+  }
+};
+
+inline DeltaShape delta_shape(int D, int Dv, int64_t pairs, int max_new) {
+  DeltaShape s{};
+  s.KS = 1;
+  while (s.KS * kGlaRows < D) s.KS <<= 1;
+  auto warps_of = [&](int C) { return cdiv(Dv, 32 / s.KS * C); };
+  s.C = 4;
+  s.VT = 1;
+  if (max_new == 1) {   // many small CTAs
+    while (s.VT < 8 && s.VT * 16 < warps_of(4)) s.VT *= 2;
+  } else {
+    const int forced = test_options().gla_layout.load();   // 100 * VT + C (tests and measurements)
+    if (pairs * warps_of(4) < 4 * (int64_t)sm_count() && warps_of(2) <= 8 * kDeltaMain) s.C = 2;
+    if (forced > 0) s.C = forced % 100 == 2 && warps_of(2) <= 8 * kDeltaMain ? 2 : 4;
+    const int w = warps_of(s.C);
+    while (s.VT < 8 &&
+           (cdiv(w, s.VT) > kDeltaMain || (s.VT < 4 && pairs * s.VT * 2 <= sm_count() && s.VT * 2 <= w)))
+      s.VT *= 2;
+    if (forced >= 100 && forced / 100 <= 8 && cdiv(w, forced / 100) <= kDeltaMain) s.VT = forced / 100;
+  }
+  s.warps = cdiv(warps_of(s.C), s.VT);
+  s.CW = s.warps * (32 / s.KS) * s.C;
+  s.CP = cdiv(s.CW, 8) * 8;
+  if (max_new > 1) {
+    s.tok = kGlaBlock;
+    while (s.tok < kGlaTok && s.tok < max_new) s.tok <<= 1;
+    while (s.tok > kGlaBlock && s.smem(4) > 200 * 1024) s.tok >>= 1;
+  }
   return s;
 }
 
@@ -1503,25 +1970,49 @@ int dispatch_gla(const GlaShape& sh, dim3 grid, cudaStream_t st, const void* pro
 #undef CVLLM_GLA
 }
 
+template <typename T, int KS, int C>
+int launch_delta(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* qkv, const void* proj, const DeltaArgs& da,
+                 const RecurArgs& a) {
+  static std::atomic<uint64_t> attr{0};
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_scan_kernel<T, KS, C>, 200 * 1024, attr));
+  CVLLM_CHECK_CUDA(launch_clustered(delta_scan_kernel<T, KS, C>, grid, (sh.warps + kDeltaHelpers) * 32, sh.smem(sizeof(T)), st,
+                                    sh.VT, qkv, static_cast<const T*>(proj), da, a));
+  CVLLM_CHECK_LAUNCH();
+  return CVLLM_OK;
+}
+
+template <typename T, int KS>
+int launch_delta_step(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* qkv, const void* proj, const DeltaArgs& da,
+                      const RecurArgs& a) {
+  CVLLM_CHECK_CUDA(launch_clustered(delta_step_kernel<T, KS>, grid, sh.warps * 32, sh.smem(sizeof(T)), st, sh.VT, qkv,
+                                    static_cast<const T*>(proj), da, a));
+  CVLLM_CHECK_LAUNCH();
+  return CVLLM_OK;
+}
+
+template <typename T>
+int dispatch_delta(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* qkv, const void* proj, const DeltaArgs& da,
+                   const RecurArgs& a) {
+#define CVLLM_DELTA(KK) \
+  return sh.tok == 0 ? launch_delta_step<T, KK>(sh, grid, st, qkv, proj, da, a)    \
+         : sh.C == 2 ? launch_delta<T, KK, 2>(sh, grid, st, qkv, proj, da, a)      \
+                     : launch_delta<T, KK, 4>(sh, grid, st, qkv, proj, da, a)
+  switch (sh.KS) {
+    case 1: CVLLM_DELTA(1);
+    case 2: CVLLM_DELTA(2);
+    case 4: CVLLM_DELTA(4);
+    case 8: CVLLM_DELTA(8);
+    case 16: CVLLM_DELTA(16);
+    default: CVLLM_DELTA(32);
+  }
+#undef CVLLM_DELTA
+}
+
 template <int R>
 constexpr int max_recur_smem(int key_rows) {
   // key rows of at most kMaxKeyDim numbers: KS <= kMaxKeyDim / R slices of R + 4 floats
   (void)key_rows;
   return 200 * 1024;   // a ceiling for every shape; a launch asks for what its stage size needs (pick_tok: <= 96 KB)
-}
-
-template <typename T, int R, int MAXT>
-int launch_delta(dim3 grid, const RecurShape& sh, cudaStream_t st, const float* qkv, int64_t qkv_stride,
-                 const void* proj, int64_t proj_stride, int b_off, int a_off, const float* A_log, const float* dt_bias,
-                 int G, const RecurArgs& a) {
-  // the attribute is set once per kernel: to what the largest shape needs, not to this launch's size
-  static std::atomic<uint64_t> attr{0};
-  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_rule_kernel<T, R, MAXT>, max_recur_smem<R>(2), attr));
-  CVLLM_CHECK_CUDA(launch_clustered(delta_rule_kernel<T, R, MAXT>, grid, sh.threads, sh.smem(2), st, sh.VT, qkv,
-                                    qkv_stride, static_cast<const T*>(proj), proj_stride, b_off, a_off, A_log, dt_bias,
-                                    G, a));
-  CVLLM_CHECK_LAUNCH();
-  return CVLLM_OK;
 }
 
 template <typename T, int R, int MAXT>
@@ -1626,17 +2117,18 @@ extern "C" int cvllm_delta_rule(const float* qkv, int64_t qkv_stride, const void
   CVLLM_CHECK_ARG(cu_seqlens_q ? seq_start != nullptr : (positions != nullptr && max_new == 1));
   CVLLM_CHECK_SUPPORTED(D <= kMaxKeyDim && Dv <= kMaxValueDim && H <= 65535 && B <= 65535);
   auto st = static_cast<cudaStream_t>(stream);
-  RecurShape sh = recur_shape(D, Dv, H * B, max_new);
-  sh.pick_tok(max_new, 2);
-  CVLLM_CHECK_SUPPORTED(sh.threads > 0 && sh.threads <= 1024 && (int64_t)H * sh.VT <= 2147483647);
-  RecurArgs a{{cu_seqlens_q, seq_start, positions, batch_mapping}, state, gate, gate_stride, gate_off, norm_w,
-              norm_head_stride, eps, out, out_stride, H, D, Dv, reserved_slot, sh.KS, sh.VT, sh.CW, sh.tok};
+  const size_t elem = dtype == CVLLM_BF16 ? 2 : 4;
+  const DeltaShape sh = delta_shape(D, Dv, (int64_t)H * B, max_new);
+  CVLLM_CHECK_SUPPORTED(sh.warps >= 1 && sh.warps <= (max_new > 1 ? kDeltaMain : 16) && sh.smem(elem) <= 200 * 1024 &&
+                        (int64_t)H * sh.VT <= 2147483647);
+  const int vec_key = aligned16(qkv) && qkv_stride % 4 == 0 && D % 4 == 0;
+  const int vec_val = vec_key && Dv % 4 == 0 && sh.CW % 4 == 0;
+  const DeltaArgs da{b_off, a_off, G, qkv_stride, proj_stride, A_log, dt_bias, vec_key, vec_val, sh.CP};
+  const RecurArgs a{{cu_seqlens_q, seq_start, positions, batch_mapping}, state, gate, gate_stride, gate_off, norm_w,
+                    norm_head_stride, eps, out, out_stride, H, D, Dv, reserved_slot, sh.KS, sh.VT, sh.CW, sh.tok};
   const dim3 grid(H * sh.VT, B);
-#define CVLLM_DELTA(T, RR, MT) \
-  launch_delta<T, RR, MT>(grid, sh, st, qkv, qkv_stride, proj, proj_stride, b_off, a_off, A_log, dt_bias, G, a)
-  if (dtype == CVLLM_BF16) { CVLLM_RECUR_BY_R(CVLLM_DELTA, __nv_bfloat16) }
-  CVLLM_RECUR_BY_R(CVLLM_DELTA, float)
-#undef CVLLM_DELTA
+  if (dtype == CVLLM_BF16) return dispatch_delta<__nv_bfloat16>(sh, grid, st, qkv, proj, da, a);
+  return dispatch_delta<float>(sh, grid, st, qkv, proj, da, a);
 }
 
 extern "C" int cvllm_wkv_scan(const void* r, int64_t r_stride, const void* k, int64_t k_stride, const void* v,
