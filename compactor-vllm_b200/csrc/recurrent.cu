@@ -1541,7 +1541,7 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict
 }
 
 // Portions.  A cluster of VT CTAs serves one (head, sequence); each keeps CW value columns.  Warps have one of two roles:
-// `warps` main warps take the blocks through their state tiles; four others work for the stages (`tok` tokens) around the
+// `warps` main warps take the blocks through their state tiles; the others work for the stages (`tok` tokens) around the
 // one the main warps are in: they load q, k and v of the stage after next (cp.async), make the next stage's coefficients
 // and finish the outputs of the stages before (sums of squares, exchanged through distributed shared memory, then norm,
 // weight, gate).  One cluster barrier per stage orders all of it:
@@ -1553,17 +1553,19 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict
 // stage: key and query rows transformed by the coefficients 4.7 k, loads 3.4 k, blocks 9.6 k, norm 4.5 k); transformed rows
 // sent to the cluster's other CTAs as plain stores into distributed shared memory 3.6 ms (12 k 16-byte stores a stage); raw
 // rows, roles, a block's read-outs finished before the next block starts 1.67 ms (main warps 13 k cycles a stage, the
-// others 21 k: divisions, loads waited for at their conversion); this form 1.31 ms (12.8 k and 16.5 k).
+// others 21 k: divisions, loads waited for at their conversion); without those 1.31 ms (12.8 k and 16.5 k); eight other
+// warps, rows copied by pointers that only add up: 1.12 ms (13.1 k and 9.4 k).
 // What bounds it: instruction issue of the blocks (about half of it the 3.25 multiply-adds per state number and token) and
 // the latency of the exchange over the key lanes, two main warps a scheduler.
-constexpr int kDeltaHelpers = 4;   // warps
-constexpr int kDeltaMain = 8;      // most main warps
+template <int C>
+constexpr int kDeltaHelpers = C == 2 ? 8 : 4;   // warps (four columns per thread leave registers for four)
+constexpr int kDeltaMain = 8;                   // most main warps
 
 template <typename T, int KS, int C>
-__global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers) * 32, 1)
+__global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers<C>) * 32, 1)
 delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, DeltaArgs da, RecurArgs a) {
   namespace cg = cooperative_groups;
-  constexpr int U = kGlaBlock, DP = KS * kGlaRows;
+  constexpr int U = kGlaBlock, DP = KS * kGlaRows, HW = kDeltaHelpers<C>;
   using Coef = DeltaCoef<U>;
   using Tile = DeltaTile<KS, C, U>;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1582,7 +1584,7 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
   const int kvh = h / (H / da.G);
   const int c0 = vt * CW, ncol = max(0, min(CW, Dv - c0));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int main_warps = (blockDim.x >> 5) - kDeltaHelpers;
+  const int main_warps = (blockDim.x >> 5) - HW;
   const bool helper = warp >= main_warps;
   const int stages = cdiv(n_new, tok);
   auto sync_all = [&]() {
@@ -1600,31 +1602,56 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
 
   // ---- the others ----
   const int hw = warp - main_warps, ht = hw * 32 + lane;
-  constexpr int kHT = kDeltaHelpers * 32;
+  constexpr int kHT = HW * 32;
   const float neg_a = -expf(da.A_log[h]), dtb = da.dt_bias[h];
   const float q_scale = rsqrtf((float)D);
   T la = from_f<T>(0.f), lb = la;   // decay and beta logits of the next stage's token `lane` (first of these warps)
-  // `rows` rows of `len` numbers -> shared rows of `pitch`, 16 bytes at a time where `vec`
-  auto stage_in = [&](float* dst, int pitch, const float* src, int len, int rows, bool vec) {
-    const int E = vec ? 4 : 1, per = len / E;
-    if (per <= 0) return;
-    int c = ht / per, d = ht - c * per;
-    const int sc = kHT / per, sd = kHT - sc * per;
-    while (c < rows) {
-      if (vec) cp_async16(dst + c * pitch + d * 4, src + c * da.qkv_stride + d * 4);
-      else dst[c * pitch + d] = src[c * da.qkv_stride + d];
-      c += sc;
-      d += sd;
-      if (d >= per) { d -= per; ++c; }
+  // A row's 16-byte pieces go to neighbouring threads, each of which keeps to its piece and takes every so-many-th row.
+  struct Pieces {
+    int row, at, step;   // first row, first number, rows per pass (0: not this thread)
+    __device__ __forceinline__ Pieces(int t, int len) {
+      const int per = max(len / 4, 1);
+      step = kHT / per;
+      row = t / per;
+      at = (t - row * per) * 4;
+      if (row >= step || len < 4) step = 0;
     }
   };
+  const Pieces key(ht, D), val(ht, ncol);
   auto issue = [&](int s) {
     const int n = min(tok, n_new - s * tok);
     const float* row = qkv + (int64_t)(t0 + s * tok) * da.qkv_stride;
     float *dq = R + s % 3 * 2 * tok * DP, *sv = V + s % 3 * tok * CP;
-    stage_in(dq, DP, row + kvh * D, D, n, da.vec_key);
-    stage_in(dq + tok * DP, DP, row + da.G * D + kvh * D, D, n, da.vec_key);
-    stage_in(sv, CP, row + 2 * da.G * D + h * Dv + c0, ncol, n, da.vec_val);
+    const float *q = row + kvh * D, *k = q + da.G * D, *v = row + 2 * da.G * D + h * Dv + c0;
+    if (da.vec_key) {
+      if (key.step > 0) {
+        const int64_t first = key.row * da.qkv_stride + key.at, step = key.step * da.qkv_stride;
+        const float *pq = q + first, *pk = k + first;
+        float* d = dq + key.row * DP + key.at;
+        for (int c = key.row; c < n; c += key.step, pq += step, pk += step, d += key.step * DP) {
+          cp_async16(d, pq);
+          cp_async16(d + tok * DP, pk);
+        }
+      }
+    } else {
+      for (int i = ht; i < n * D; i += kHT) {
+        const int c = i / D, d = i - c * D;
+        dq[c * DP + d] = q[c * da.qkv_stride + d];
+        dq[(tok + c) * DP + d] = k[c * da.qkv_stride + d];
+      }
+    }
+    if (da.vec_val) {
+      if (val.step > 0) {
+        const float* pv = v + val.row * da.qkv_stride + val.at;
+        float* d = sv + val.row * CP + val.at;
+        for (int c = val.row; c < n; c += val.step, pv += val.step * da.qkv_stride, d += val.step * CP) cp_async16(d, pv);
+      }
+    } else {
+      for (int i = ht; i < n * ncol; i += kHT) {
+        const int c = i / ncol, d = i - c * ncol;
+        sv[c * CP + d] = v[c * da.qkv_stride + d];
+      }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
     // the last block's missing tokens: zero rows (0 * garbage)
     const int n_up = cdiv(n, U) * U;
@@ -1640,7 +1667,7 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
   };
   auto help_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kHT) : "memory"); };
   // outputs: such a thread keeps to one column (its weight in a register) and takes every out_rows-th token
-  constexpr int kGate = 16;   // gate logits that it loads ahead of their use
+  constexpr int kGate = C == 2 ? 8 : 16;   // gate logits that it loads ahead of their use
   const bool by_column = ncol > 0 && ncol <= kHT;
   const int out_rows = by_column ? kHT / ncol : 1, out_c = by_column ? ht / ncol : 0;
   const int out_j = by_column ? ht - out_c * ncol : 0;
@@ -1673,6 +1700,8 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
       // gates of stage s - 2, used at the end
       const int e = s - 2, n_e = e >= 0 ? min(tok, n_new - e * tok) : 0;
       T pg[kGate];
+#pragma unroll
+      for (int u = 0; u < kGate; ++u) pg[u] = from_f<T>(0.f);
       {
         const T* g = gate + (int64_t)(e * tok + out_c) * a.gate_stride + out_j;
 #pragma unroll
@@ -1688,7 +1717,7 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
         if (s + 2 < stages) issue(s + 2);
         const int n = min(tok, n_new - (s + 1) * tok), blocks = cdiv(n, U);
         const float* rq = R + (s + 1) % 3 * 2 * tok * DP;
-        for (int blk = hw; blk < blocks; blk += kDeltaHelpers)
+        for (int blk = hw; blk < blocks; blk += HW)
           Coef::template make_dots<DP>(rq + blk * U * DP, rq + (tok + blk * U) * DP, dots + blk * Coef::kDots);
         help_sync();
         if (hw == 0) {   // a lane per token, then a lane per block
@@ -1739,14 +1768,20 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
           T* o = out + (int64_t)(e * tok + out_c) * a.out_stride + out_j;
           const float* x = so + out_c * CP + out_j;
 #pragma unroll
-          for (int u = 0; u < kGate; ++u) {
-            const int c = out_c + u * out_rows;
-            if (u * out_rows < n_e) {
+          for (int u0 = 0; u0 < kGate; u0 += 4) {   // four at a time: their exponentials and quotients side by side
+            if (u0 * out_rows >= n_e) break;
+            T y[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int c = out_c + (u0 + u) * out_rows;
               const float iv = __shfl_sync(0xffffffffu, inv, c & 31);
-              if (out_on && c < n_e) *o = value(*x * iv, out_w, to_f<T>(pg[u]));
+              y[u] = value(c < n_e ? x[u * out_rows * CP] * iv : 0.f, out_w, to_f<T>(pg[u0 + u]));
             }
-            o += (int64_t)out_rows * a.out_stride;
-            x += out_rows * CP;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (out_on && out_c + (u0 + u) * out_rows < n_e) o[(int64_t)u * out_rows * a.out_stride] = y[u];
+            o += (int64_t)4 * out_rows * a.out_stride;
+            x += 4 * out_rows * CP;
           }
           for (int u = kGate; u * out_rows < n_e; ++u) {
             const int c = out_c + u * out_rows;
@@ -1975,7 +2010,7 @@ int launch_delta(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* 
                  const RecurArgs& a) {
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_scan_kernel<T, KS, C>, 200 * 1024, attr));
-  CVLLM_CHECK_CUDA(launch_clustered(delta_scan_kernel<T, KS, C>, grid, (sh.warps + kDeltaHelpers) * 32, sh.smem(sizeof(T)), st,
+  CVLLM_CHECK_CUDA(launch_clustered(delta_scan_kernel<T, KS, C>, grid, (sh.warps + kDeltaHelpers<C>) * 32, sh.smem(sizeof(T)), st,
                                     sh.VT, qkv, static_cast<const T*>(proj), da, a));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
