@@ -6,6 +6,7 @@ caller gets an exception.  PyTorch is used only for device memory and streams.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from pathlib import Path
 
@@ -187,7 +188,21 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # the handle without a Stream object around it
+
+
+def index_tensor(t: torch.Tensor, device: torch.device) -> torch.Tensor:
+    """t as a contiguous int32 tensor on the device (t itself when it is one)."""
+    if t.dtype is torch.int32 and t.device == device and t.is_contiguous():
+        return t
+    return t.to(dtype=torch.int32, device=device).contiguous()
+
+
 def stream(device: torch.device | None = None) -> int:
+    """Handle of the device's current stream.  A decode step is one kernel of about 10 us: what a call costs on the host
+    is what such a step costs, and the Stream objects were the largest part of it (two a call, 1.5 us each)."""
+    if device is not None and device.index is not None and _raw_stream is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -211,12 +226,18 @@ def block_dtype_code(dt: torch.dtype) -> int:
 _WORKSPACES: dict = {}
 
 
-def workspace(device: torch.device, nbytes: int, tag: str = "", zero: bool = False) -> torch.Tensor:
+@functools.lru_cache(maxsize=4096)
+def sized(name: str, *sizes: int) -> int:
+    """A size function of the library (its result depends on nothing but its arguments), remembered per argument list."""
+    return getattr(lib(), name)(*sizes)
+
+
+def workspace(device: torch.device, nbytes: int, tag="", zero: bool = False) -> torch.Tensor:
     """Grow-only per-(device, stream, tag) byte scratch from torch's caching allocator.
 
     zero=True: the buffer is zero-filled when it is (re)allocated — for kernels whose contract is
     "control words zero on entry, restored to zero on exit" (decode attention's head tickets)."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, tag)
+    key = (device.index, stream(device), tag)
     buf = _WORKSPACES.get(key)
     if buf is None or buf.numel() < nbytes:
         alloc = torch.zeros if zero else torch.empty

@@ -49,17 +49,18 @@ def head_sparse_decode_attention(
     assert k.is_contiguous() and v.is_contiguous() and k.dtype == q.dtype == v.dtype
     assert global_page_table.is_contiguous() and global_page_table.dtype == torch.int32
     assert batch_mapping.dtype == torch.int32 and batch_mapping.is_contiguous()
-    seq_lens_bh = seq_lens_bh.to(torch.int32).contiguous()
+    if seq_lens_bh.dtype != torch.int32 or not seq_lens_bh.is_contiguous():
+        seq_lens_bh = seq_lens_bh.to(torch.int32).contiguous()
     sm_scale = 1 / math.sqrt(D) if sm_scale is None else sm_scale
     dev = q.device
     out = torch.empty_like(q)
     if B == 0:
         return out
     L = N.lib()
-    ws_bytes = L.cvllm_decode_attention_workspace_bytes(B, HQ, HKV, D, 0)
+    ws_bytes = N.sized("cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
     # one workspace per (B, HQ, HKV): the ticket region's size depends on B*HKV, and the "zero on
     # entry, zero on exit" contract only holds while the layout stays the same
-    ws = N.workspace(dev, ws_bytes, f"decode_attn:{B}:{HQ}:{HKV}", zero=True)
+    ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
     rc = L.cvllm_decode_attention(
         N.ptr(q), N.ptr(out), N.ptr(k), N.ptr(v), N.ptr(seq_lens_bh), N.ptr(global_page_table),
         N.ptr(batch_mapping), N.ptr(ws), ws.numel(), B, HQ, HKV, D, int(PAGE_SIZE),
@@ -103,8 +104,8 @@ def decode_append_and_attend(
     if B == 0:
         return out
     L = N.lib()
-    ws_bytes = L.cvllm_decode_attention_workspace_bytes(B, HQ, HKV, D, 0)
-    ws = N.workspace(dev, ws_bytes, f"decode_attn:{B}:{HQ}:{HKV}", zero=True)
+    ws_bytes = N.sized("cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
+    ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
     rc = L.cvllm_decode_step(
         N.ptr(key), N.ptr(value), key.stride(0), key.stride(1), value.stride(0), value.stride(1),
         N.ptr(q), N.ptr(out), N.ptr(k_cache), N.ptr(v_cache), N.ptr(bh_seq_lens), N.ptr(global_page_table),

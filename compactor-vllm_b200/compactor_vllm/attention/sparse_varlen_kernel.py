@@ -53,9 +53,7 @@ def causal_sparse_varlen_with_cache(
     assert k_cache.is_contiguous() and v_cache.is_contiguous()
     assert q.dtype == k.dtype == v.dtype == k_cache.dtype == v_cache.dtype
     dev = q.device
-    cu = cu_seqlens_q.to(dtype=torch.int32, device=dev).contiguous()
-    lens = seq_lens_bh.to(dtype=torch.int32, device=dev).contiguous()
-    bm = batch_mapping.to(dtype=torch.int32, device=dev).contiguous()
+    cu, lens, bm = (N.index_tensor(t, dev) for t in (cu_seqlens_q, seq_lens_bh, batch_mapping))
     pt = global_page_table
     assert pt.dtype == torch.int32 and pt.is_contiguous()
     if sm_scale is None:

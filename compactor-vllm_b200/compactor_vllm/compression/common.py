@@ -133,9 +133,8 @@ def extract_and_store_top_kv(
     assert batch_mapping.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()
     assert new_keys.stride(-1) == 1 and new_vals.stride(-1) == 1
     dev = new_keys.device
-    cu = cu_seqlens_k.to(device=dev, dtype=torch.int32).contiguous()
+    cu, retain = N.index_tensor(cu_seqlens_k, dev), N.index_tensor(num_tokens_to_retain, dev)
     bm = batch_mapping.to(torch.int32)
-    retain = num_tokens_to_retain.to(device=dev, dtype=torch.int32).contiguous()
     L = N.lib()
     ws_bytes = L.cvllm_select_store_workspace_bytes(B, H, N_total)
     ws = N.workspace(dev, ws_bytes, "select_store")

@@ -220,7 +220,7 @@ def non_causal_attn_scores(
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(D)
     dev = q.device
-    cu = cu_seqlens_qk.to(device=dev, dtype=torch.int32).contiguous()
+    cu = N.index_tensor(cu_seqlens_qk, dev)
     out = torch.empty((Ntok, HKV), dtype=torch.float32, device=dev)
     if Ntok == 0:
         return out

@@ -10,6 +10,7 @@ import copy
 from typing import Optional
 
 import torch
+from compactor_vllm import _native as N
 from compactor_vllm.attention.sparse_decode_kernel import decode_append_and_attend, head_sparse_decode_attention
 from compactor_vllm.attention.sparse_varlen_kernel import causal_sparse_varlen_with_cache
 from compactor_vllm.compression.common import extract_and_store_top_kv
@@ -253,6 +254,13 @@ class BiasedChunkAttention(nn.Module):
         other.k_cache = other.v_cache = other.page_table = other.bh_seq_lens = other.page_size = None
         return other
 
+    def _field(self, name: str):
+        """A parameter, buffer or plain attribute by name, past Module.__getattr__ (0.5 us a name, and a step reads eight)."""
+        value = self._parameters.get(name)
+        if value is None:
+            value = self._buffers.get(name)
+        return self.__dict__.get(name) if value is None else value
+
     @torch.no_grad()
     def refresh_distance_bias(self, rel: Optional[torch.Tensor] = None) -> None:
         """`rel` (given: the new table, any number of rows) spread out per distance: dist_bias[n, h] =
@@ -304,7 +312,7 @@ class BiasedChunkAttention(nn.Module):
                 and k.dtype == torch.bfloat16 and self.head_dim % 8 == 0 and self.v_head_dim % 8 == 0
                 and self.v_head_dim <= 512 and self.slopes is None and self.rel is None and int(self.page_size) % 64 == 0)
 
-    def streaming_decode_kernel(self, batch: int, max_keys: int) -> bool:
+    def streaming_decode_kernel(self, max_keys: int) -> bool:
         """Whether a decode step goes to the streaming kernel of csrc/decode_attn.cu (the library takes it when the sizes
         allow and the workspace holds its scratch): where the keys a query may see are two of its units of 128 or more.
         Measured at 32 / 8 heads of 64, 32 sequences (streaming / key splits): up to 140 keys 19 / 14 us, up to 280 keys
@@ -313,12 +321,12 @@ class BiasedChunkAttention(nn.Module):
             max_keys = min(max_keys, self.chunk)
         if self.window:
             max_keys = min(max_keys, self.window)
-        return (max_keys >= 256 and not self.values_in_keys and self.head_dim == self.v_head_dim
-                and self.head_dim in (64, 128) and self.num_heads // self.num_kv_heads <= 8)
+        D, page = self.head_dim, int(self.page_size)
+        return (max_keys >= 256 and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
+                and self.num_heads // self.num_kv_heads <= 8 and self.k_cache.dtype == torch.bfloat16
+                and (page % 128 == 0 or page in (16, 32, 64)))
 
     def forward(self, qkv: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        from compactor_vllm import _native as N
-
         ctx: Context = get_context()
         s = self.source
         if s is not None and self.k_cache is None:      # the source's cache views, once the cache manager has made them
@@ -332,19 +340,19 @@ class BiasedChunkAttention(nn.Module):
         q = torch.empty((T, H, D), dtype=qkv.dtype, device=dev)
         pt = self.page_table
         table = (N.ptr(pt), pt.stride(0), pt.stride(1), int(self.page_size))
-        rot = self.inv_freq
+        rot, q_w, k_w = self._field("inv_freq"), self._field("q_norm_weight"), self._field("k_norm_weight")
         if self.row_norm:
             caches = (None, None) if s is not None else (N.ptr(self.k_cache), N.ptr(self.v_cache))
             N.check(lib.cvllm_row_norm_rope_store(
-                N.ptr(qkv), qkv.stride(0), N.ptr(rot), 0 if rot is None else 2 * rot.numel(), N.ptr(self.q_norm_weight),
-                N.ptr(self.k_norm_weight), self.eps, N.ptr(ctx.positions_i32), N.ptr(ctx.token_slot), N.ptr(q), *caches,
+                N.ptr(qkv), qkv.stride(0), N.ptr(rot), 0 if rot is None else 2 * rot.numel(), N.ptr(q_w),
+                N.ptr(k_w), self.eps, N.ptr(ctx.positions_i32), N.ptr(ctx.token_slot), N.ptr(q), *caches,
                 *table, N.ptr(self.bh_seq_lens), T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
                 "cvllm_row_norm_rope_store")
             return self.attend(q, out=out)
         N.check(lib.cvllm_rope_qknorm_store(
             N.ptr(qkv), qkv.stride(0), N.ptr(rot), 0 if rot is None else 2 * rot.numel(),
             int(self.norm) + 2 * int(self.value_norm),
-            N.ptr(self.q_norm_weight), N.ptr(self.k_norm_weight), self.eps,
+            N.ptr(q_w), N.ptr(k_w), self.eps,
             N.ptr(ctx.positions_i32), N.ptr(ctx.token_slot), N.ptr(q), N.ptr(self.k_cache), N.ptr(self.v_cache),
             *table, N.ptr(self.bh_seq_lens), T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
             "cvllm_rope_qknorm_store")
@@ -353,8 +361,6 @@ class BiasedChunkAttention(nn.Module):
     def attend(self, q: torch.Tensor, flat: bool = True, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """q [T, H, D] (normed / rotated already, the step's keys in the cache) -> [T, H * Dv], or with flat=False
         [T, H, Dv] (possibly a view of wider rows).  `out` [T, H * Dv] (row stride free): where to write."""
-        from compactor_vllm import _native as N
-
         ctx: Context = get_context()
         T = q.shape[0]
         H, G, D, Dv = self.num_heads, self.num_kv_heads, self.head_dim, self.v_head_dim
@@ -376,27 +382,28 @@ class BiasedChunkAttention(nn.Module):
         else:
             assert out.shape == (T, H * Dv) and out.stride(1) == 1 and out.dtype == q.dtype
             o_stride = out.stride(0)
-        if self.rel is not None and self.dist_bias is None:
+        if self._field("dist_bias") is None and self._field("rel") is not None:
             self.refresh_distance_bias()
-        db = self.dist_bias
+        db, slopes, sink_logits = self._field("dist_bias"), self._field("slopes"), self._field("sink_logits")
         dist = (self.window, self.keep_first, N.ptr(db), 0 if db is None else db.shape[0])
         if ctx.is_prefill:
             B = ctx.batch_mapping.numel()
             N.check(lib.cvllm_bias_attn_varlen_dist(
                 N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.cu_seqlens_q),
-                N.ptr(ctx.seq_start), N.ptr(ctx.batch_mapping), N.ptr(self.slopes), self.chunk, *dist, int(self.sink),
-                N.ptr(self.sink_logits), self.scale, N.ptr(out), o_stride, B, int(ctx.max_seqlen_q), H, G, D, Dv, T,
+                N.ptr(ctx.seq_start), N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink),
+                N.ptr(sink_logits), self.scale, N.ptr(out), o_stride, B, int(ctx.max_seqlen_q), H, G, D, Dv, T,
                 self.k_cache.shape[0], pt.shape[-1], v_stride, code, N.stream(dev)), "cvllm_bias_attn_varlen")
         else:
             assert ctx.batch_mapping.numel() == T
-            splits = self.decode_splits(T, int(ctx.max_seqlen_k))
-            ws_bytes = 4 * T * H * splits * (2 + Dv) if splits > 1 else 0
-            if self.streaming_decode_kernel(T, int(ctx.max_seqlen_k)):
-                ws_bytes = max(ws_bytes, lib.cvllm_bias_decode_workspace_bytes(T, H, G, D))
+            if self.streaming_decode_kernel(int(ctx.max_seqlen_k)):
+                splits, ws_bytes = 1, N.sized("cvllm_bias_decode_workspace_bytes", T, H, G, D)
+            else:
+                splits = self.decode_splits(T, int(ctx.max_seqlen_k))
+                ws_bytes = 4 * T * H * splits * (2 + Dv) if splits > 1 else 0
             ws = N.workspace(dev, ws_bytes, "bias_attn_decode") if ws_bytes else None
             N.check(lib.cvllm_bias_attn_decode_dist(
                 N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.positions_i32),
-                N.ptr(ctx.batch_mapping), N.ptr(self.slopes), self.chunk, *dist, int(self.sink), N.ptr(self.sink_logits),
+                N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
                 self.scale, N.ptr(out), o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits, N.ptr(ws), ws.numel() if ws is not None else 0, v_stride, code,
                 N.stream(dev)), "cvllm_bias_attn_decode")
         if keep != Dv:
