@@ -92,13 +92,14 @@ struct TestOptions {
   std::atomic<int> snap_v1{0};                // 1: the mma.sync SnapKV kernels
   std::atomic<int> chunk_scores_v1{0};        // 1: the mma.sync chunk scorer (A/B against the tcgen05 one)
   std::atomic<int> pdl{0};                    // 1: launch the selection chain with programmatic dependent launch (A/B; off in the product)
+  std::atomic<int> select_passes{0};          // 1: the selection as a chain of launches also where one cluster would do
   std::atomic<int> grs_pairs{0};              // > 0: cap the CTA pairs of gemm_reduce
   std::atomic<int> grs_probe{0};              // gemm_reduce timing probes (bit mask; results are wrong)
   std::atomic<uint64_t> grs_debug_host_ptr{0};  // pinned host buffer for gemm_reduce's timeout records
   std::atomic<int> grs_rows_per_round{0};     // > 0: rows per reduce round of gemm_reduce (multiple of 256)
   std::atomic<int> bias_attn_fma{0};          // 1: 16-bit portions of the biased attention on the fp32 FMA kernel
   std::atomic<int> ssm_segment{0};            // > 0: tokens per segment of the state-space scan (0: chosen per step)
-  std::atomic<int> gla_layout{0};             // > 0: 100 * CTAs per (head, sequence) + columns per thread (2, 4) of the gated linear attention
+  std::atomic<int> gla_layout{0};             // > 0: 100 * CTAs per (head, sequence) + columns per thread (2, 4) of the gated linear attention and the delta rule
   std::atomic<int> recur_layout{0};           // > 0: 100 * CTAs per (head, sequence) + register slice of the matrix-state mixers (0: chosen per step)
 };
 TestOptions& test_options();

@@ -15,8 +15,13 @@
 // Every phase is a grid of (token tiles x sequences) CTAs: the keys of a 32K-token sequence are
 // 1 MB and live in L2, each pass is a few microseconds instead of a single-SM walk.  The CTA that
 // takes the last ticket of a sequence folds the global histogram into the next digit.
+// Phases 1 to 4 of sequences whose keys fit the shared memory of a cluster of up to eight CTAs (350 K keys at 8 heads) are
+// ONE kernel (sel_cluster_kernel): twelve short launches of 4 to 12 us each, one waiting for the other, were three quarters
+// of an eviction.  Longer ones take the launches.
 // Order everywhere: key descending, ties by ascending flat index tok*H + head, NaN above +inf.
 // Rows land in ascending token order per head (the reference's order is atomic-nondeterministic).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "select_common.cuh"
 
@@ -70,15 +75,17 @@ __global__ void sel_init_kernel(const int32_t* __restrict__ cu, const int32_t* _
 }
 
 // digit pick: 256-bin histogram (descending) -> digit holding the `remaining`-th entry.
-// Executed by one full warp; returns through lane-uniform refs.
-__device__ __forceinline__ void pick_digit(const uint32_t* hist /*global, 256*/, uint32_t remaining,
-                                           uint32_t& digit, uint32_t& new_remaining) {
+// Executed by one full warp; returns through lane-uniform refs.  bin(i): count of digit i.
+// `held`: how many entries that digit holds.
+template <typename Bin>
+__device__ __forceinline__ void pick_digit(Bin bin, uint32_t remaining, uint32_t& digit, uint32_t& new_remaining,
+                                           uint32_t& held) {
   const int lane = threadIdx.x & 31;
   uint32_t h8[8];
   uint32_t own = 0;
 #pragma unroll
   for (int t = 0; t < 8; ++t) {
-    h8[t] = __ldcg(hist + 255 - 8 * lane - t);
+    h8[t] = bin(255 - 8 * lane - t);
     own += h8[t];
   }
   uint32_t incl = own;
@@ -89,7 +96,7 @@ __device__ __forceinline__ void pick_digit(const uint32_t* hist /*global, 256*/,
   }
   const uint32_t above = incl - own;
   const bool mine = (above < remaining) && (remaining <= incl);
-  uint32_t d = 0, rem = 0;
+  uint32_t d = 0, rem = 0, n = 0;
   if (mine) {
     uint32_t acc = above;
     int t = 0;
@@ -99,11 +106,14 @@ __device__ __forceinline__ void pick_digit(const uint32_t* hist /*global, 256*/,
     }
     d = (uint32_t)(255 - 8 * lane - t);
     rem = remaining - acc;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) n = u == t ? h8[u] : n;
   }
   const uint32_t who = __ballot_sync(0xffffffffu, mine);
   const int src = who ? (__ffs(who) - 1) : 0;
   digit = __shfl_sync(0xffffffffu, d, src);
   new_remaining = __shfl_sync(0xffffffffu, rem, src);
+  held = __shfl_sync(0xffffffffu, n, src);
 }
 
 // ---------------------------------------------------------------------------
@@ -168,8 +178,8 @@ __global__ void __launch_bounds__(kPassThreads) sel_pass_kernel(const float* __r
   const int warp = tid >> 5, lane = tid & 31;
   for (int s = warp; s < nseg; s += kPassThreads / 32) {
     if (s_active[s]) {
-      uint32_t digit, rem;
-      pick_digit(hist + s * 256, st[s].remaining, digit, rem);
+      uint32_t digit, rem, held;
+      pick_digit([&](int i) { return __ldcg(hist + s * 256 + i); }, st[s].remaining, digit, rem, held);
       if (lane == 0) {
         st[s].prefix = s_prefix[s] | (digit << shift);
         st[s].remaining = rem;
@@ -356,6 +366,263 @@ __global__ void __launch_bounds__(kPassThreads) sel_count_heads_kernel(const flo
   }
   __syncthreads();
   if (tid < H) w.tile_cnt[((int64_t)b * w.tiles + tile) * H + tid] = make_uint2(s_gt[tid], s_tie[tid]);
+}
+
+// ---------------------------------------------------------------------------
+// Phases 1 to 4 in one launch: a cluster of CS CTAs per sequence, each with a run of whole tiles whose keys stay in its shared
+// memory.  A pass counts digits in its own histogram (256 x 32 words: a column per head and neighbouring token, so that the
+// lanes of a warp never meet in a word or a bank), the cluster's CTAs add up each other's sums through distributed shared
+// memory, each for itself, behind one cluster barrier (two buffers: whoever writes a buffer again has passed a barrier that
+// all readers have reached).  The first digit of the per-head passes is counted together with the first of the whole
+// sequence.  A pass is the last one when its digit's entries are all taken: the low bits then make no difference (keys from
+// the prefix up are kept, "ties" with it all).  Bound by latency: up to seven rounds of a pass over the CTA's keys and an
+// exchange, 5 to 8 k cycles a round.  Whole evictions in a graph, chain of launches / one launch: 700 tokens of 8 heads
+// 83 / 41 us, 5000 87 / 46 us, 32768 99 / 72 us (half of it the copy), six of 6000 148 / 103 us.
+// ---------------------------------------------------------------------------
+constexpr int kClThreads = 1024;
+
+inline size_t sel_cluster_smem(int tiles_per_cta, int H) {
+  return sizeof(uint32_t) * ((size_t)tiles_per_cta * kTileTok * H + 256 * 32 + 2 * 256 + 4 * (size_t)H * 256);
+}
+
+__global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
+    const float* __restrict__ scores, int64_t stride_n, const int32_t* __restrict__ cu, const int32_t* __restrict__ num_retain,
+    const int32_t* __restrict__ batch_mapping, const int32_t* __restrict__ bh_lens, int H, int PS, int pad_to_page,
+    int reserved_batch, int keys_cap, SelWs w) {
+  namespace cg = cooperative_groups;
+  extern __shared__ uint32_t sm[];
+  uint32_t* keys = sm;                    // [keys_cap] token major, head minor
+  uint32_t* col = keys + keys_cap;        // [256][32] the pass's counts, zero between passes
+  uint32_t* g = col + 256 * 32;           // [2][256] this CTA's counts over all heads
+  uint32_t* hh = g + 2 * 256;             // [3][H][256] ... per head: first digit | two buffers
+  uint32_t* tot = hh + 3 * H * 256;       // [H][256] the cluster's sums
+  __shared__ uint32_t s_gt[kMaxH], s_tie[kMaxH], s_sel[kMaxH];
+  __shared__ uint32_t s_prefix[kMaxH], s_remaining[kMaxH], s_active[kMaxH], s_open[kMaxH];
+  __shared__ uint32_t s_all_gt[kMaxH], s_all_tie[kMaxH], s_all_sel[kMaxH], s_before;
+  __shared__ uint32_t s_pick[3];   // digit, remaining, whether its entries are all taken
+  __shared__ int s_warp[32];
+  cg::cluster_group cl = cg::this_cluster();
+  const int CS = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int beg = cu[b], len = cu[b + 1] - beg;
+  const uint32_t k = (uint32_t)max(0, min(num_retain[b], len * H));
+  const bool active = batch_mapping[b] != reserved_batch && k > 0;
+  if (rank == 0 && tid < H) w.len0[b * H + tid] = bh_lens[b * H + tid];
+  if (!active) {   // the same for every CTA of the cluster
+    if (rank == 0 && tid < H) w.state_h[b * H + tid] = SegState{0, 0, 0, 0};
+    return;
+  }
+  const int tiles_b = cdiv(len, kTileTok), tpc = cdiv(tiles_b, CS);
+  const int tile0 = min(rank * tpc, tiles_b), tile1 = min(tile0 + tpc, tiles_b);
+  const int tok0 = tile0 * kTileTok, ntok = max(0, min(len, tile1 * kTileTok) - tok0), nkeys = ntok * H;
+  // a thread keeps to one head: it takes every (stride / H)-th token
+  const int stride = kClThreads / H * H, my_h = tid % H, my_tok = tid / H;
+  const bool on = tid < stride;
+  int lg = 5;   // columns per head (log2)
+  while (lg > 0 && (H << lg) > 32) --lg;
+  const int copies = 1 << lg, col_head = lane >> lg;
+  const bool col_first = (lane & (copies - 1)) == 0 && col_head < H;
+  // sum over the cluster of word i of a shared array: all loads in flight together (a cluster has at most eight CTAs)
+  auto cluster_sum = [&](uint32_t* array, int i) {
+    uint32_t v[8], t = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = r < CS ? cl.map_shared_rank(array, r)[i] : 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) t += v[r];
+    return t;
+  };
+  const int my_col = my_h * copies + (my_tok & (copies - 1));
+  if (on) {
+    const float* src = scores + (int64_t)(beg + tok0 + my_tok) * stride_n + my_h;
+    const int64_t step = (int64_t)(stride / H) * stride_n;
+#pragma unroll 4
+    for (int i = tid; i < nkeys; i += stride, src += step) keys[i] = score_key(__float_as_uint(__ldg(src)));
+  }
+  for (int i = tid; i < 256 * 32; i += kClThreads) col[i] = 0;
+  __syncthreads();
+  // counts of digit `shift` of the keys that match (prefix, mask); pre: this thread's head's prefix
+  auto count = [&](uint32_t pre, uint32_t mask, int shift, bool want) {
+    if (on && want) {
+#pragma unroll 4
+      for (int i = tid; i < nkeys; i += stride) {
+        const uint32_t key = keys[i];
+        if ((key & mask) == pre) atomicAdd(&col[((key >> shift) & 255u) * 32 + my_col], 1u);
+      }
+    }
+    __syncthreads();
+  };
+  // columns -> per-head counts (dst) and, where asked, counts over all heads (all); the columns are zero afterwards
+  auto collect = [&](uint32_t* dst, uint32_t* all) {
+    constexpr int ROWS = 256 / (kClThreads / 32);
+    uint32_t v[ROWS];
+    uint32_t* mine = col + warp * ROWS * 32 + lane;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      v[r] = mine[r * 32];
+      mine[r * 32] = 0;
+    }
+    if (all) {
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const uint32_t t = __reduce_add_sync(0xffffffffu, v[r]);
+        if (lane == 0) all[warp * ROWS + r] = t;
+      }
+    }
+    if (dst) {
+      for (int o = 1; o < copies; o <<= 1) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) v[r] += __shfl_xor_sync(0xffffffffu, v[r], o);
+      }
+      if (col_first) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) dst[col_head * 256 + warp * ROWS + r] = v[r];
+      }
+    }
+  };
+  // ---- phase 1: the sequence's threshold ----
+  uint32_t prefix = 0, remaining = k;
+  for (int pass = 0; pass < 4; ++pass) {
+    const int shift = 24 - 8 * pass;
+    count(prefix, pass == 0 ? 0u : 0xffffffffu << (32 - 8 * pass), shift, true);
+    uint32_t* mine = g + (pass & 1) * 256;
+    collect(pass == 0 ? hh : nullptr, mine);
+    cl.sync();
+    if (tid < 256) tot[tid] = cluster_sum(mine, tid);
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t digit, rem, held;
+      pick_digit([&](int i) { return tot[i]; }, remaining, digit, rem, held);
+      if (lane == 0) s_pick[0] = digit, s_pick[1] = rem, s_pick[2] = held == rem;
+    }
+    __syncthreads();
+    prefix |= s_pick[0] << shift;
+    remaining = s_pick[1];
+    if (s_pick[2]) {   // (the same in every CTA)
+      remaining = 0xffffffffu;
+      break;
+    }
+  }
+  // ---- phase 2: keys above it per head, ties in flat order ----
+  if (tid < H) s_gt[tid] = s_tie[tid] = s_sel[tid] = 0;
+  __syncthreads();
+  {
+    uint32_t gt = 0, tie = 0;
+    if (on)
+      for (int i = tid; i < nkeys; i += stride) {
+        gt += keys[i] > prefix;
+        tie += keys[i] == prefix;
+      }
+    if (gt) atomicAdd(&s_gt[my_h], gt);
+    if (tie) atomicAdd(&s_tie[my_h], tie);
+  }
+  cl.sync();
+  if (tid < H) {
+    s_all_gt[tid] = cluster_sum(s_gt, tid);
+    s_all_tie[tid] = cluster_sum(s_tie, tid);
+  }
+  if (warp == 1) {   // ties of the CTAs before this one
+    uint32_t t = 0;
+    for (int i = lane; i < rank * H; i += 32) t += cl.map_shared_rank(s_tie, i / H)[i % H];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) s_before = t;
+  }
+  __syncthreads();
+  uint32_t ties = 0, own_ties = 0;
+  for (int h = 0; h < H; ++h) {
+    ties += s_all_tie[h];
+    own_ties += s_tie[h];
+  }
+  if (remaining < ties) {   // (the same in every CTA) some are left out: the first `remaining` in flat order are taken
+    const uint32_t before = s_before;
+    if (before + own_ties <= remaining) {
+      if (tid < H) s_sel[tid] = s_tie[tid];
+    } else if (before < remaining) {
+      const uint32_t need = remaining - before;
+      uint32_t seen = 0;
+      for (int base = 0; base < nkeys && seen < need; base += kClThreads) {
+        const int i = base + tid;
+        const bool tie = i < nkeys && keys[i] == prefix;
+        int tot;
+        const uint32_t at = seen + block_excl_count(tie, s_warp, tot);
+        if (tie && at < need) atomicAdd(&s_sel[i % H], 1u);
+        seen += tot;
+      }
+    }
+    cl.sync();
+    if (tid < H) s_all_sel[tid] = cluster_sum(s_sel, tid);
+  } else if (tid < H) {
+    s_all_sel[tid] = s_all_tie[tid];
+  }
+  if (tid < H) {
+    const int c = (int)(s_all_gt[tid] + s_all_sel[tid]);
+    int n = c;
+    if (pad_to_page) n += pad_amount(bh_lens[b * H + tid] + c, len, PS);
+    n = min(n, len);
+    s_prefix[tid] = 0;
+    s_remaining[tid] = (uint32_t)n;
+    s_active[tid] = s_open[tid] = n > 0;
+  }
+  cl.sync();   // from here on the heads' states are written by the CTAs that own the heads
+  // ---- phase 3: every head's own threshold ----
+  for (int pass = 0; pass < 4; ++pass) {
+    const int shift = 24 - 8 * pass;
+    uint32_t* mine = hh;
+    if (pass > 0) {
+      mine = hh + (1 + (pass & 1)) * H * 256;
+      count(s_prefix[my_h], 0xffffffffu << (32 - 8 * pass), shift, s_open[my_h] != 0);
+      collect(mine, nullptr);
+      cl.sync();
+    }
+    // head h belongs to CTA h mod CS: each sums and picks its heads' digits and tells all (every CTA summing every head's
+    // bins moved 64 KB into each CTA, 6 k cycles a pass)
+    for (int i = tid; i < (H - rank + CS - 1) / CS * 256; i += kClThreads) {
+      const int at = (rank + (i >> 8) * CS) * 256 + (i & 255);
+      tot[at] = cluster_sum(mine, at);
+    }
+    __syncthreads();
+    const int head = rank + warp * CS;
+    if (head < H && s_open[head]) {
+      uint32_t digit, rem, held;
+      pick_digit([&](int i) { return tot[head * 256 + i]; }, s_remaining[head], digit, rem, held);
+      const uint32_t pre = s_prefix[head] | (digit << shift);
+      __syncwarp();
+      if (lane < CS) {
+        cl.map_shared_rank(s_prefix, lane)[head] = pre;
+        cl.map_shared_rank(s_remaining, lane)[head] = held == rem ? 0xffffffffu : rem;
+        cl.map_shared_rank(s_open, lane)[head] = held != rem;
+      }
+    }
+    cl.sync();
+    bool open = false;
+    for (int h = 0; h < H; ++h) open |= s_open[h] != 0;
+    if (!open) break;   // (the same in every CTA)
+  }
+  if (rank == 0 && tid < H)
+    w.state_h[b * H + tid] = SegState{s_prefix[tid], s_remaining[tid], s_active[tid], 0};
+  // ---- phase 4: per tile / head: (#keys > T_h, #keys == T_h), a warp per tile ----
+  const int subs = 32 / H;
+  for (int t = tile0 + warp; t < tile1; t += kClThreads / 32) {
+    const int h = lane % H, sub = lane / H;
+    uint32_t gt = 0, tie = 0;
+    if (sub < subs) {
+      const uint32_t thr = s_prefix[h];
+      const uint32_t* kt = keys + (t - tile0) * kTileTok * H + h;
+      const int n = min(kTileTok, len - t * kTileTok);
+      for (int i = sub; i < n; i += subs) {
+        const uint32_t key = kt[i * H];
+        gt += key > thr;
+        tie += key == thr;
+      }
+    }
+    uint32_t gs = gt, ts = tie;   // lanes h, h + H, ..: the tile's counts of head h
+    for (int j = 1; j < subs; ++j) {
+      gs += __shfl_down_sync(0xffffffffu, gt, j * H);
+      ts += __shfl_down_sync(0xffffffffu, tie, j * H);
+    }
+    if (lane < H) w.tile_cnt[((int64_t)b * w.tiles + t) * H + lane] = make_uint2(gs, ts);
+  }
+  cl.sync();   // nobody leaves while its counts may still be read
 }
 
 // ---------------------------------------------------------------------------
@@ -577,22 +844,49 @@ extern "C" int cvllm_select_store_topk(const float* scores, int64_t s_stride_n, 
   w.tile_cnt = reinterpret_cast<uint2*>(base + l.tile_cnt);
   w.tiles = l.tiles;
   auto st = static_cast<cudaStream_t>(stream);
-  CVLLM_CHECK_CUDA(cudaMemsetAsync(base, 0, l.zero_end, st));
   const dim3 grid((N + kTileTok - 1) / kTileTok, B);
-  sel_init_kernel<<<(B * HKV + 255) / 256, 256, 0, st>>>(cu_seqlens_k, num_retain, batch_mapping, bh_lens,
-                                                         B, HKV, reserved_batch, w);
-  // eleven short kernels in a row, each dependent on the one before; launch_pdl is a plain launch unless the test
-  // option "pdl" is set (common.cuh has the measurements)
-  const dim3 pb(kPassThreads);
-  for (int pass = 0; pass < 4; ++pass)
-    CVLLM_CHECK_CUDA(launch_pdl(sel_pass_kernel<false>, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, pass, w));
-  CVLLM_CHECK_CUDA(launch_pdl(sel_count_global_kernel, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, w));
-  CVLLM_CHECK_CUDA(launch_pdl(sel_resolve_kernel, dim3(B), pb, 0, st, scores, s_stride_n, cu_seqlens_k, batch_mapping,
-                              HKV, PS, pad_to_page, reserved_batch, w));
-  for (int pass = 0; pass < 4; ++pass)
-    CVLLM_CHECK_CUDA(launch_pdl(sel_pass_kernel<true>, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, pass, w));
-  CVLLM_CHECK_CUDA(launch_pdl(sel_count_heads_kernel, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, w));
-  CVLLM_CHECK_LAUNCHES(12);
+  // One cluster per sequence while its share of the keys (a sequence may be all of N) fits a CTA's shared memory; smaller
+  // clusters for fewer keys: an exchange costs more than 16 K keys less per CTA save.
+  int cluster = 1;
+  while (cluster < 8 && (int64_t)N * HKV > (int64_t)cluster * 16384) cluster *= 2;
+  const int tiles_per_cta = cdiv((int)grid.x, cluster);
+  const size_t cl_smem = sel_cluster_smem(tiles_per_cta, HKV);
+  constexpr size_t kClSmemMax = 226 * 1024;   // beside the static arrays
+  if (cl_smem <= kClSmemMax && test_options().select_passes.load() == 0) {
+    static std::atomic<uint64_t> attr{0};
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)sel_cluster_kernel, (int)kClSmemMax, attr));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster, B);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = cl_smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CVLLM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sel_cluster_kernel, scores, s_stride_n, cu_seqlens_k, num_retain, batch_mapping,
+                                        (const int32_t*)bh_lens, HKV, PS, pad_to_page, reserved_batch,
+                                        tiles_per_cta * kTileTok * HKV, w));
+    CVLLM_CHECK_LAUNCH();
+  } else {
+    CVLLM_CHECK_CUDA(cudaMemsetAsync(base, 0, l.zero_end, st));
+    sel_init_kernel<<<(B * HKV + 255) / 256, 256, 0, st>>>(cu_seqlens_k, num_retain, batch_mapping, bh_lens,
+                                                           B, HKV, reserved_batch, w);
+    // eleven short kernels in a row, each dependent on the one before; launch_pdl is a plain launch unless the test
+    // option "pdl" is set (common.cuh has the measurements)
+    const dim3 pb(kPassThreads);
+    for (int pass = 0; pass < 4; ++pass)
+      CVLLM_CHECK_CUDA(launch_pdl(sel_pass_kernel<false>, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, pass, w));
+    CVLLM_CHECK_CUDA(launch_pdl(sel_count_global_kernel, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, w));
+    CVLLM_CHECK_CUDA(launch_pdl(sel_resolve_kernel, dim3(B), pb, 0, st, scores, s_stride_n, cu_seqlens_k, batch_mapping,
+                                HKV, PS, pad_to_page, reserved_batch, w));
+    for (int pass = 0; pass < 4; ++pass)
+      CVLLM_CHECK_CUDA(launch_pdl(sel_pass_kernel<true>, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, pass, w));
+    CVLLM_CHECK_CUDA(launch_pdl(sel_count_heads_kernel, grid, pb, 0, st, scores, s_stride_n, cu_seqlens_k, HKV, w));
+    CVLLM_CHECK_LAUNCHES(12);
+  }
   // enough copy CTAs to fill the chip a few times over: 4 per tile at long prompts, 1 when the grid is already wide
   const int64_t gtiles = (int64_t)grid.x * grid.y;
   const dim3 ggrid(grid.x, grid.y, gtiles >= 4 * sm_count() ? 1 : 4);

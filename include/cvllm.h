@@ -70,7 +70,9 @@ uint64_t cvllm_launch_count(void);
  *                            2 mma.sync also where the tcgen05 kernel would serve (A/B), 3 the tcgen05 kernel for latent
  *                            rows wherever it serves (portions and decode)
  *   "ssm_segment" n          tokens per segment of cvllm_ssm_scan (0 = the product's choice; tests use short segments)
- *   "gla_layout" n           100 * CTAs per (head, sequence) + columns per thread of cvllm_gla_scan (0 = chosen per step)
+ *   "gla_layout" n           100 * CTAs per (head, sequence) + columns per thread of cvllm_gla_scan and of the portions of
+ *                            cvllm_delta_rule (0 = chosen per step)
+ *   "select_passes" 1|0      cvllm_select_store_topk: the chain of launches also where one cluster per sequence would do
  *   "grs_debug_host_ptr" p   pinned host buffer (64 words per CTA) for cvllm_gemm_allreduce's timeout records
  * Returns CVLLM_E_ARG for an unknown name. */
 int cvllm_set_test_option(const char* name, double value);

@@ -1,0 +1,89 @@
+"""Selection and compaction: the one-launch selection (a cluster per sequence) against the chain of launches, exactly, over
+head counts, ragged batches, score strides, ties, infinities and NaN, and the sizes where clusters grow."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+D, PS = 64, 128
+
+
+def scores_of(kind, n, H, g):
+    s = torch.randn(n, H, generator=g)
+    if kind == "ties":                       # a handful of values: nearly every threshold is a tie
+        s = torch.randint(0, 5, (n, H), generator=g).float()
+    elif kind == "equal":
+        s.zero_()
+    elif kind == "special":
+        r = torch.rand(n, H, generator=g)
+        s[r < 0.05] = float("inf")
+        s[(r >= 0.05) & (r < 0.1)] = float("-inf")
+        s[(r >= 0.1) & (r < 0.13)] = float("nan")
+        s[(r >= 0.13) & (r < 0.2)] = -0.0
+        s[(r >= 0.2) & (r < 0.25)] = 0.0
+        s[(r >= 0.25) & (r < 0.3)] = torch.finfo(torch.float32).min
+    return s
+
+
+def evict(scores, lens, retain, H, wide, slots, pad, option):
+    from compactor_vllm import _native as N
+    from compactor_vllm.compression.common import extract_and_store_top_kv
+
+    n, B = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(5)
+    k, v = (torch.randn(n, H, D, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    lens0 = torch.randint(0, 300, (B, H), generator=g).to(torch.int32).to(DEV)
+    P = -(-(max(lens) + 300 + PS) // PS)
+    rows = (B + 2) * H * P * PS
+    table = torch.randperm((B + 2) * H * P, generator=g).to(torch.int32).view(B + 2, H, P).to(DEV)
+    kc, vc = (torch.zeros(rows, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    buf = torch.zeros(n, H + (3 if wide else 0), device=DEV)
+    buf[:, :H] = scores.to(DEV)
+    cu = [0]
+    for x in lens:
+        cu.append(cu[-1] + x)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    N.set_test_option("select_passes", option)
+    try:
+        extract_and_store_top_kv(scores=buf[:, :H], cu_seqlens_k=i32(cu), max_k_len=max(lens), top_k=max(lens) * H, H=H,
+                                 new_keys=k, new_vals=v, num_tokens_to_retain=i32(retain), page_table=table,
+                                 batch_mapping=i32(slots), bh_lens=lens0, k_cache=kc, v_cache=vc, PAGE_SIZE=PS,
+                                 PAD_TO_PAGE_SIZE=pad)
+    finally:
+        N.set_test_option("select_passes", 0)
+    return lens0, kc, vc
+
+
+LENS = {"one": [700], "ragged": [1, 2500, 0, 256, 257, 1023], "cluster2": [2600, 40], "cluster8": [15000, 3000, 7], "tiny": [3]}
+
+
+@pytest.mark.parametrize("kind", ["random", "ties", "equal", "special"])
+@pytest.mark.parametrize("lens", sorted(LENS))
+@pytest.mark.parametrize("H", [1, 3, 8, 16])
+def test_one_launch_equals_the_chain(H, lens, kind):
+    L = LENS[lens]
+    B = len(L)
+    g = torch.Generator().manual_seed(H * 100 + B)
+    scores = scores_of(kind, sum(L), H, g)
+    slots = list(range(1, B + 1))
+    if B > 3:
+        slots[3] = 0                         # a reserved slot
+    for ratio, pad, wide in ((0.5, True, False), (0.03, False, True), (1.0, True, False), (0.0, True, True)):
+        retain = [int(round(ratio * x * H)) for x in L]
+        if ratio == 0.03:
+            retain = [max(1, r) for r in retain]
+        a = evict(scores, L, retain, H, wide, slots, pad, 0)
+        b = evict(scores, L, retain, H, wide, slots, pad, 1)
+        for x, y in zip(a, b):
+            assert torch.equal(x, y), (ratio, pad)
+
+
+@pytest.mark.parametrize("n,H", [(40960, 8), (41216, 8), (16384, 16), (22000, 16)])
+def test_where_the_clusters_end(n, H):
+    """The largest sequences that a cluster's shared memory holds, and the first that it does not."""
+    g = torch.Generator().manual_seed(n)
+    scores = scores_of("random", n, H, g)
+    a = evict(scores, [n], [n * H // 4], H, False, [1], True, 0)
+    b = evict(scores, [n], [n * H // 4], H, False, [1], True, 1)
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
