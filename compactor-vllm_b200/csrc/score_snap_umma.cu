@@ -1,17 +1,28 @@
 // SnapKV observation-window scorer on tcgen05 (reference: compression/snapkv.py:39-276,332-448; K12 + K13).
 //
-// Rows = the last w query tokens x the G query heads of one kv head (w * G <= 128: one UMMA M tile; the mma.sync
-// kernels of score_attn.cu serve larger windows), columns = 128-key tiles of the sequence's non-window keys:
-//   S = Qwin [128 x 128 d] . K_tile^T   one `tcgen05.mma` chain of 8 x (128 x 128 x 16) per key tile.
-// Two launches over the same (key split, kv head, sequence) grid, one CTA per split of kSnapSplit keys:
-//   pass 1  running (max, sum) of every row over the split's keys          -> stats[part][row]
-//   pass 2  column sums of exp2(s - m_row) / l_row with the FINAL row statistics (all parts combined), causal
-//           kpool-tap mean inside pool_segment-key segments, window keys <- +inf                 -> out[key, hk]
+// Rows = the last w query tokens x the G query heads of one kv head (w * G <= 128: one UMMA tile; the mma.sync
+// kernels of score_attn.cu serve larger windows), columns = 128-key tiles of the sequence's non-window keys.
+// Two launches over the same (key split, kv head, sequence) grid, one CTA per split:
+//   pass 1  S = Qwin . K_tile^T (lane = row, column = key): running (max, sum) of every row over the split's
+//           keys -> stats[part][row]
+//   pass 2  S^T = K_tile . Qwin^T (lane = key, column = row): column sums of exp2(s - m_row) / l_row with the
+//           FINAL row statistics (all parts combined), causal kpool-tap mean inside pool_segment-key segments,
+//           window keys <- +inf                                                            -> out[key, hk]
 // Roles per CTA as in score_chunk_umma.cu: warp 8 TMA producer (Q window once: a 3-D box {64 d, G heads, w tokens}
 // lands in shared memory already in row order (token, g); K tiles through a 4-slot ring), warp 9 UMMA issuer (four
-// 128-column TMEM buffers), warps 0-7 two warpgroups that each own one half of the key columns of every tile: a
-// thread keeps its row's 64 logits in registers from one tcgen05.ld on.  The two halves never exchange anything in
-// pass 1 (each writes its own partial statistics: parts = 2 x splits) and only meet in pass 2's column sums.
+// 128-column TMEM buffers), warps 0-7 two warpgroups.  Pass 1: each warpgroup owns one half of the key columns of
+// every tile, a thread keeps its row's 64 logits in registers, and each half writes its own partial statistics
+// (parts = 2 x splits).  Pass 2: the warpgroups take alternate tiles; with the operands swapped a thread owns one
+// KEY, so the sum over the rows stays in its registers, with the rows' statistics read from shared memory as
+// broadcasts.  With lane = row it took 62 shuffles a thread, two barriers of all eight warps a tile and nothing
+// to overlap them with.  40960 keys, 32 / 8 heads, both passes and the call: 88 -> 50 us with the splits below, 131072
+// keys 288 -> 130 us; error against 64 bits (rms, relative) 9.3e-8 -> 5.2e-8.
+// What bounds the passes: pass 1 the read of K, pass 2 the exponentials (128 x 128 a tile at 16 per clock: 1024
+// clocks).  A CTA holds the SM (TMEM, 160 KB of shared memory), so the grid runs in waves of 148 CTAs and a start
+// (barriers, TMEM, the first tile's latency, in pass 2 the statistics) costs as much as four tiles: see
+// snap_split() for how many CTAs a call is cut into.
+#include <algorithm>
+
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -24,7 +35,8 @@ constexpr int kBoxBytes = kTileBytes / 2;
 constexpr int kSlots = 4;
 constexpr int kThreads = 384;
 constexpr int kRegsSoftmax = 224, kRegsOther = 56;
-constexpr int kSplit = 1024;  // keys per CTA
+constexpr int kMaxTilesManyCtas = 8;  // key tiles per CTA where (sequence, head) pairs alone fill the chip
+constexpr int kSms = 148;
 }  // namespace sn
 
 struct SnapUmmaParams {
@@ -32,33 +44,23 @@ struct SnapUmmaParams {
   const int32_t* cu_k;
   float* stats;  // [B, HKV, parts, 128, 2] partial (m, l) per row; parts = 2 * n_splits
   float* out;    // [Nk, HKV]
-  int HKV, G, w, n_splits, kpool, pool_segment;
+  int HKV, G, w, n_splits, split, kpool, pool_segment;  // split: keys per CTA, a multiple of 128
   float scale_log2;
 };
 
 struct SnapUmmaSmem {
   unsigned char q[sn::kTileBytes];
   unsigned char ring[sn::kSlots][sn::kTileBytes];
-  float col[4][sn::kTile];
-  float raw[sn::kTile];
+  float2 row_stat[2 * sn::kTile];  // pass 2: (-m, 1 / l) of every row; the second half: (m, l) of the other warpgroup
+  float raw[2][2][sn::kTile];      // pass 2: [warpgroup][its tile's parity] column sums before the mean over taps
   uint64_t q_full;
   uint64_t full[sn::kSlots], empty[sn::kSlots];
   uint64_t s_full[4], s_empty[4];
   uint32_t tmem_base;
 };
 
-template <int N, int O>
-__device__ __forceinline__ void snap_colsum_stage(float (&acc)[sn::kHalf], int lane) {
-  const bool hi = (lane & O) != 0;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const float keep = hi ? acc[i + N] : acc[i];
-    const float send = hi ? acc[i] : acc[i + N];
-    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-  }
-}
-
 __device__ __forceinline__ void snap_bar_256() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void snap_bar_wg(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory"); }
 
 template <bool BF16, bool PASS2>
 __global__ void __launch_bounds__(sn::kThreads, 1)
@@ -73,8 +75,8 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int kb = p.cu_k[b], len = p.cu_k[b + 1] - kb, q_end = p.cu_q[b + 1];
   const int rows = p.w * p.G;
   const int n_scored = len - p.w;  // keys [0, L - w) are scored, the window keys get +inf
-  const int k_lo = sp * kSplit;
-  const int k_hi = min(n_scored, k_lo + kSplit);  // scored keys of this split
+  const int k_lo = sp * p.split;
+  const int k_hi = min(n_scored, k_lo + p.split);  // scored keys of this split
   const int n_tiles = k_hi > k_lo ? (k_hi - k_lo + kTile - 1) / kTile : 0;
   const int parts = 2 * p.n_splits;
   float* st_base = p.stats + ((int64_t)b * p.HKV + hk) * parts * kTile * 2;
@@ -90,7 +92,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     } else {
       const float v = n_scored > 0 ? INFINITY : 0.f;
-      for (int k = k_lo + threadIdx.x; k < min(len, k_lo + kSplit); k += kThreads)
+      for (int k = k_lo + threadIdx.x; k < min(len, k_lo + p.split); k += kThreads)
         p.out[(int64_t)(kb + k) * p.HKV + hk] = v;
     }
     return;
@@ -99,7 +101,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(&sm.q_full, 1);
     for (int i = 0; i < kSlots; ++i) { mbar_init(&sm.full[i], 1); mbar_init(&sm.empty[i], 1); }
-    for (int i = 0; i < 4; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], 256); }
+    for (int i = 0; i < 4; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], PASS2 ? 128 : 256); }
     mbar_fence_init();
   }
   if (warp == 9) {
@@ -149,7 +151,8 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int kk = 0; kk < kHD / 16; ++kk) {
           const uint32_t off = (kk >> 2) * kBoxBytes + (kk & 3) * 32;
-          umma_ss(tmem_u + buf * kTile, umma_desc_add(q_desc, off), umma_desc_add(k_desc, off), idesc, kk > 0 ? 1u : 0u);
+          const uint64_t qd = umma_desc_add(q_desc, off), kd = umma_desc_add(k_desc, off);
+          umma_ss(tmem_u + buf * kTile, PASS2 ? kd : qd, PASS2 ? qd : kd, idesc, kk > 0 ? 1u : 0u);
         }
         umma_commit(&sm.s_full[buf]);
         umma_commit(&sm.empty[slot]);
@@ -160,98 +163,127 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // ====================== softmax statistics / column sums ======================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     const int wg = warp >> 2, quad = warp & 3;
-    const int row = quad * 32 + lane;
-    const int st = threadIdx.x;  // 0..255
+    const int row = quad * 32 + lane;  // TMEM lane: the query row (pass 1) or the key of the tile (pass 2)
+    const int st = threadIdx.x;        // 0..255
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-    float m_run = -INFINITY, l_run = 0.f;  // pass 1: this half's running statistics of the row
-    float neg_m = 0.f, inv_l = 0.f;        // pass 2: the row's final statistics
-    if (PASS2) {
-      float M = -INFINITY;
-      for (int s = 0; s < parts; ++s) M = fmaxf(M, st_base[((int64_t)s * kTile + row) * 2]);
-      float L = 0.f;
-      for (int s = 0; s < parts; ++s) {
-        const float ms = st_base[((int64_t)s * kTile + row) * 2];
-        if (ms > -INFINITY) L += st_base[((int64_t)s * kTile + row) * 2 + 1] * ex2(ms - M);
-      }
-      neg_m = (M > -INFINITY) ? -M : 0.f;
-      inv_l = (row < rows && L > 0.f) ? 1.f / L : 0.f;
-    }
-    for (int t = 0; t < n_tiles; ++t) {
-      const int buf = t & 3;
-      const int nk = min(kTile, k_hi - (k_lo + t * kTile));  // scored keys in this tile
-      mbar_wait(&sm.s_full[buf], (t >> 2) & 1);
-      tc_fence_after();
-      uint32_t r0[32], r1[32];
-      tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base, r0);
-      tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base + 32, r1);
-      tc_wait_ld();
-      tc_fence_before();
-      mbar_arrive(&sm.s_empty[buf]);
-      float sv[kHalf];
+    if constexpr (!PASS2) {
+      float m_run = -INFINITY, l_run = 0.f;  // this half's running statistics of the row
+      for (int t = 0; t < n_tiles; ++t) {
+        const int buf = t & 3;
+        const int nk = min(kTile, k_hi - (k_lo + t * kTile));  // scored keys in this tile
+        mbar_wait(&sm.s_full[buf], (t >> 2) & 1);
+        tc_fence_after();
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base, r0);
+        tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base + 32, r1);
+        tc_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&sm.s_empty[buf]);
+        float sv[kHalf];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        sv[i] = __uint_as_float(r0[i]) * p.scale_log2;
-        sv[32 + i] = __uint_as_float(r1[i]) * p.scale_log2;
-      }
-      if (nk < kTile) {
+        for (int i = 0; i < 32; ++i) {
+          sv[i] = __uint_as_float(r0[i]) * p.scale_log2;
+          sv[32 + i] = __uint_as_float(r1[i]) * p.scale_log2;
+        }
+        if (nk < kTile) {
 #pragma unroll
-        for (int i = 0; i < kHalf; ++i)
-          if (wg * kHalf + i >= nk) sv[i] = -INFINITY;
-      }
-      if (!PASS2) {
+          for (int i = 0; i < kHalf; ++i)
+            if (wg * kHalf + i >= nk) sv[i] = -INFINITY;
+        }
         float m0 = sv[0], m1 = sv[1], m2 = sv[2], m3 = sv[3];
 #pragma unroll
         for (int i = 4; i < kHalf; i += 4) {
           m0 = fmaxf(m0, sv[i]); m1 = fmaxf(m1, sv[i + 1]); m2 = fmaxf(m2, sv[i + 2]); m3 = fmaxf(m3, sv[i + 3]);
         }
-        const float m_new = fmaxf(m_run, fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)));
+        // The reference point is rounded up to a whole number: every later change of it, here and where the parts
+        // meet, is then a power of two and adds no error (ex2's is one-sided and would add up along the chain).
+        const float m_new = fmaxf(m_run, ceilf(fmaxf(fmaxf(m0, m1), fmaxf(m2, m3))));
         if (m_new > -INFINITY) {  // else: every key of this half is masked so far
-          float s0 = 0.f, s1 = 0.f;
+          float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-          for (int i = 0; i < kHalf; i += 2) {
+          for (int i = 0; i < kHalf; i += 4) {
             s0 += ex2(sv[i] - m_new);
             s1 += ex2(sv[i + 1] - m_new);
+            s2 += ex2(sv[i + 2] - m_new);
+            s3 += ex2(sv[i + 3] - m_new);
           }
-          l_run = l_run * ex2(m_run - m_new) + (s0 + s1);  // ex2(-inf) = 0 on the first live tile
+          l_run = l_run * ex2(m_run - m_new) + ((s0 + s1) + (s2 + s3));  // ex2(-inf) = 0 on the first live tile
           m_run = m_new;
         }
-      } else {
-        float acc[kHalf];
-#pragma unroll
-        for (int i = 0; i < kHalf; ++i) acc[i] = ex2(sv[i] + neg_m) * inv_l;
-        snap_colsum_stage<32, 16>(acc, lane);
-        snap_colsum_stage<16, 8>(acc, lane);
-        snap_colsum_stage<8, 4>(acc, lane);
-        snap_colsum_stage<4, 2>(acc, lane);
-        snap_colsum_stage<2, 1>(acc, lane);
-        *reinterpret_cast<float2*>(&sm.col[quad][wg * kHalf + 2 * lane]) = make_float2(acc[0], acc[1]);
-        snap_bar_256();
-        if (st < kTile) sm.raw[st] = ((sm.col[0][st] + sm.col[1][st]) + sm.col[2][st]) + sm.col[3][st];
-        snap_bar_256();
-        // causal kpool-tap mean inside pool_segment-key segments (snapkv.py:253-262); window keys <- +inf
-        if (st < kTile) {
-          const int kabs = k_lo + t * kTile + st;
-          if (kabs < len) {
-            float v = INFINITY;
-            if (st < nk) {
-              const int lo = max(st - (p.kpool - 1), (st / p.pool_segment) * p.pool_segment);
-              float s = 0.f;
-              for (int u = lo; u <= st; ++u) s += sm.raw[u];
-              v = s / (float)(st + 1 - lo);
-            }
-            p.out[(int64_t)(kb + kabs) * p.HKV + hk] = v;
-          }
-        }
-        // sm.raw / sm.col are rewritten only behind the next tile's first barrier, which every reader passes first
       }
-    }
-    if (!PASS2) {
       float* stp = st_base + ((int64_t)(2 * sp + wg) * kTile + row) * 2;
       stp[0] = m_run;
       stp[1] = l_run;
     } else {
+      // the rows' final statistics: a thread combines one row's parts of one half (part & 1 == wg), then the
+      // first 128 threads the two halves
+      {
+        const float2* parts_of = reinterpret_cast<const float2*>(st_base) + (int64_t)wg * kTile + row;
+        float M = -INFINITY, L = 0.f;
+#pragma unroll 4
+        for (int s = 0; s < p.n_splits; ++s) M = fmaxf(M, parts_of[(int64_t)s * 2 * kTile].x);
+#pragma unroll 4
+        for (int s = 0; s < p.n_splits; ++s) {
+          const float2 ml = parts_of[(int64_t)s * 2 * kTile];
+          if (ml.x > -INFINITY) L += ml.y * ex2(ml.x - M);
+        }
+        if (wg == 1) sm.row_stat[kTile + row] = make_float2(M, L);
+        snap_bar_256();
+        if (wg == 0) {
+          const float2 o = sm.row_stat[kTile + row];
+          const float Mt = fmaxf(M, o.x);
+          float Lt = 0.f;
+          if (M > -INFINITY) Lt += L * ex2(M - Mt);
+          if (o.x > -INFINITY) Lt += o.y * ex2(o.x - Mt);
+          sm.row_stat[row] = make_float2(Mt > -INFINITY ? -Mt : 0.f, (row < rows && Lt > 0.f) ? 1.f / Lt : 0.f);
+        }
+        snap_bar_256();
+      }
+      const int blocks = (rows + 31) >> 5;  // 32-row column blocks that hold rows
+      for (int t = wg; t < n_tiles; t += 2) {
+        const int buf = t & 3;
+        const int nk = min(kTile, k_hi - (k_lo + t * kTile));  // scored keys in this tile
+        mbar_wait(&sm.s_full[buf], (t >> 2) & 1);
+        tc_fence_after();
+        float total = 0.f;  // of at most four blocks, each a tree over eight chains of four: short chains of roundings
+        for (int c = 0; c < blocks; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + buf * kTile + lane_base + 32 * c, r);
+          tc_wait_ld();
+          const float4* rs = reinterpret_cast<const float4*>(sm.row_stat + 32 * c);
+          float a[8];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float4 u = rs[i / 2];  // (-m, 1 / l) of two rows
+            const float e0 = ex2(fmaf(__uint_as_float(r[i]), p.scale_log2, u.x));
+            const float e1 = ex2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, u.z));
+            a[i % 8] = i < 8 ? e0 * u.y : fmaf(e0, u.y, a[i % 8]);
+            a[i % 8 + 1] = i < 8 ? e1 * u.w : fmaf(e1, u.w, a[i % 8 + 1]);
+          }
+          total += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+        }
+        tc_fence_before();
+        mbar_arrive(&sm.s_empty[buf]);
+        // causal kpool-tap mean inside pool_segment-key segments (snapkv.py:253-262); window keys <- +inf.  The
+        // buffer of this parity is written again two tiles on, behind the next tile's barrier, which every
+        // reader of this one passes first
+        float* raw = sm.raw[wg][(t >> 1) & 1];
+        raw[row] = total;
+        snap_bar_wg(wg);
+        const int kabs = k_lo + t * kTile + row;
+        if (kabs < len) {
+          float v = INFINITY;
+          if (row < nk) {
+            const int lo = max(row - (p.kpool - 1), (row / p.pool_segment) * p.pool_segment);
+            float s = 0.f;
+            for (int u = lo; u <= row; ++u) s += raw[u];
+            v = s / (float)(row + 1 - lo);
+          }
+          p.out[(int64_t)(kb + kabs) * p.HKV + hk] = v;
+        }
+      }
       // window keys of this split that lie beyond its last scored tile
-      for (int k = k_lo + n_tiles * kTile + st; k < min(len, k_lo + kSplit); k += 256)
+      for (int k = k_lo + n_tiles * kTile + st; k < min(len, k_lo + p.split); k += 256)
         p.out[(int64_t)(kb + k) * p.HKV + hk] = INFINITY;
     }
   } else {
@@ -267,8 +299,36 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
 using namespace cvllm;
 
+// Key tiles per CTA.  A CTA holds its SM, and its start costs about four tiles, so few (sequence, head) pairs are
+// cut so that all CTAs run at once: `waves` x 148 CTAs over the heads, less one per further sequence (whose last
+// split is short on average), with a second or third wave only where several sequences, which may differ in
+// length, would otherwise get fewer than four splits each.  From 74 pairs on the pairs themselves fill the chip and
+// a CTA takes 8 tiles, which keeps sequences of unequal length balanced.  Fixed splits of 1024
+// keys were 2.2 waves at 40960 keys and 8 heads, and 8 CTAs at 1000: 4096 and 12000 keys took 34.5 us, now 26.5; with
+// four sequences of 8000 or of 500-20000 keys 69 and 72.5 -> 65 and 69.
+static int snap_waves(int B, int HKV) {
+  if ((int64_t)B * HKV > sn::kSms / 2) return 0;
+  int waves = 1;
+  while (waves * sn::kSms / HKV - (B - 1) < (B > 1 ? 4 * B : 1)) ++waves;
+  return waves;
+}
+
+static int snap_split_tiles(int B, int HKV, int Nk, int max_seqlen_k) {
+  const int waves = snap_waves(B, HKV);
+  if (waves == 0) return sn::kMaxTilesManyCtas;
+  const int64_t longest = (max_seqlen_k + sn::kTile - 1) / sn::kTile;
+  // at least the longest sequence, so that its splits are no more than `ctas` even if max_seqlen_k exceeds Nk
+  const int64_t tiles =
+      std::max(longest, std::min<int64_t>((Nk + sn::kTile - 1) / sn::kTile + (B - 1), longest * B));
+  const int64_t ctas = waves * sn::kSms / HKV - (B - 1);
+  return (int)std::max<int64_t>(1, (tiles + ctas - 1) / ctas);
+}
+
 size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV) {
-  const size_t n_splits = (size_t)(max_seqlen_k + sn::kSplit - 1) / sn::kSplit;
+  const size_t tiles = (size_t)(max_seqlen_k + sn::kTile - 1) / sn::kTile;
+  size_t n_splits = (tiles + sn::kMaxTilesManyCtas - 1) / sn::kMaxTilesManyCtas;
+  // the most that snap_split_tiles() can make of it, whatever the total of the keys
+  if (const int waves = snap_waves(B, HKV)) n_splits = std::max(n_splits, std::min(tiles, (size_t)(waves * sn::kSms / HKV)));
   return (size_t)B * HKV * 2 * (n_splits ? n_splits : 1) * sn::kTile * 2 * sizeof(float);
 }
 
@@ -291,7 +351,8 @@ int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int
   if (rc) return rc;
   SnapUmmaParams p;
   p.cu_q = cu_q; p.cu_k = cu_k; p.stats = stats; p.out = out; p.HKV = HKV; p.G = G; p.w = w;
-  p.n_splits = (max_seqlen_k + sn::kSplit - 1) / sn::kSplit;
+  p.split = snap_split_tiles(B, HKV, Nk, max_seqlen_k) * sn::kTile;
+  p.n_splits = (max_seqlen_k + p.split - 1) / p.split;
   p.kpool = kpool; p.pool_segment = pool_segment; p.scale_log2 = scale_log2;
   const dim3 grid(p.n_splits, HKV, B);
   const int smem = (int)sizeof(SnapUmmaSmem) + 1024;
