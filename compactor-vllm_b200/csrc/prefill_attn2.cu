@@ -26,6 +26,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "tile_order.cuh"
 #include "tma.cuh"
 
 namespace cvllm {
@@ -107,7 +108,7 @@ __device__ long long g_p2_trace[8][256];
 #define P2_TRACE(rowi, jj) do { } while (0)
 #endif
 
-template <bool BF16>
+template <bool BF16, bool BY_TILE>
 __global__ void __launch_bounds__(p2::kThreads, 1)
 prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kc,
@@ -118,14 +119,17 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.z;
-  const int hq0 = 2 * blockIdx.y;  // heads hq0, hq0 + 1 share KV head hkv (G even)
+  // (a form of its own for each order: with the choice at run time the loop below it ran 1 % slower at 32768 tokens)
+  TileOrder at;
+  if constexpr (BY_TILE) at = tile_order(p.seq_lens_bh, kBM);
+  const int b = BY_TILE ? at.b : blockIdx.z;
+  const int hq0 = 2 * (BY_TILE ? at.pair : blockIdx.y);  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
   const int q_beg = p.cu_seqlens_q[b];
   const int La = p.cu_seqlens_q[b + 1] - q_beg;
   const int n_qt = (La + kBM - 1) / kBM;
-  const int qt = n_qt - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
-  if (qt < 0) return;
+  const int qt = BY_TILE ? at.qt : n_qt - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
+  if (qt < 0 || qt >= n_qt) return;
   const int q0 = qt * kBM;
   const int Lc = p.seq_lens_bh[b * p.HKV + hkv];
   const int n_pre = (Lc + kBN - 1) / kBN;
@@ -498,11 +502,17 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
   p.rescale_threshold = rescale_threshold;
   const size_t smem = sizeof(Prefill2Smem) + 1024;
   const dim3 grid((max_seqlen_q + p2::kBM - 1) / p2::kBM, HQ / 2, B);
-  static std::atomic<uint64_t> attr_bf{0}, attr_h{0};
-  if (bf16) CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn2_kernel<true>, (int)smem, attr_bf));
-  else CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn2_kernel<false>, (int)smem, attr_h));
-  if (bf16) prefill_attn2_kernel<true><<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
-  else prefill_attn2_kernel<false><<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
+  const bool by_tile = (int64_t)grid.x * grid.y * grid.z <= kOrderCtas;
+  auto launch = [&](auto kernel, std::atomic<uint64_t>& attr) -> int {
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)kernel, (int)smem, attr));
+    kernel<<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
+    return CVLLM_OK;
+  };
+  static std::atomic<uint64_t> attr[4] = {{0}, {0}, {0}, {0}};
+  int rc;
+  if (bf16) rc = by_tile ? launch(prefill_attn2_kernel<true, true>, attr[0]) : launch(prefill_attn2_kernel<true, false>, attr[1]);
+  else rc = by_tile ? launch(prefill_attn2_kernel<false, true>, attr[2]) : launch(prefill_attn2_kernel<false, false>, attr[3]);
+  if (rc) return rc;
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }

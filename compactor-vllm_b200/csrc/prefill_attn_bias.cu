@@ -18,6 +18,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "tile_order.cuh"
 #include "tma.cuh"
 
 namespace cvllm {
@@ -125,14 +126,16 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.z;
-  const int hq0 = 2 * blockIdx.y;  // heads hq0, hq0 + 1 share KV head hkv (G even)
+  TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
+  if ((int64_t)gridDim.x * gridDim.y * gridDim.z <= kOrderCtas) at = tile_order(p.seq_start, kBM);
+  const int b = at.b;
+  const int hq0 = 2 * at.pair;  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
   const int q_beg = p.cu_seqlens_q[b];
   const int La = p.cu_seqlens_q[b + 1] - q_beg;
   const int n_qt = (La + kBM - 1) / kBM;
-  const int qt = n_qt - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
-  if (qt < 0) return;
+  const int qt = at.qt;  // heaviest (latest) tiles first
+  if (qt >= n_qt) return;
   const int q0 = qt * kBM;
   const int p0 = p.seq_start[b] + q0;                      // position of the tile's first query
   const int p_last = p0 + min(kBM, La - q0) - 1;           // ... and of its last valid one

@@ -1888,7 +1888,7 @@ inline DeltaShape delta_shape(int D, int Dv, int64_t pairs, int max_new) {
 // How a (head, sequence) is laid out on CTAs and threads.
 struct RecurShape {
   int R, KS, VT, CW, threads, tok;
-  size_t smem(int key_rows) const {   // key_rows: staged key-sized rows per token (2 delta, 3 wkv)
+  size_t smem(int key_rows) const {   // key_rows: staged key-sized rows per token
     return sizeof(float) * ((size_t)key_rows * tok * KS * (R + 4) + (size_t)2 * tok * CW + tok * 4 + 4 * kTokMax);
   }
   // tokens per stage: as many as a portion has, up to kTokMax, within 96 KB of shared memory (longer stages outrun the registers that load a stage ahead: 64 tokens measured 2-4 % slower than 32 at heads of 128 x 128 and 64 x 64)
