@@ -502,7 +502,7 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
   p.rescale_threshold = rescale_threshold;
   const size_t smem = sizeof(Prefill2Smem) + 1024;
   const dim3 grid((max_seqlen_q + p2::kBM - 1) / p2::kBM, HQ / 2, B);
-  const bool by_tile = (int64_t)grid.x * grid.y * grid.z <= kOrderCtas;
+  const bool by_tile = order_by_tile(grid.x, grid.y, grid.z);
   auto launch = [&](auto kernel, std::atomic<uint64_t>& attr) -> int {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)kernel, (int)smem, attr));
     kernel<<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);

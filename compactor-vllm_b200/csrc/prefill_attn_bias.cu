@@ -127,7 +127,7 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
-  if ((int64_t)gridDim.x * gridDim.y * gridDim.z <= kOrderCtas) at = tile_order(p.seq_start, kBM);
+  if (order_by_tile(gridDim.x, gridDim.y, gridDim.z)) at = tile_order(p.seq_start, kBM);
   const int b = at.b;
   const int hq0 = 2 * at.pair;  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;

@@ -17,13 +17,19 @@
 
 namespace cvllm {
 
-constexpr int64_t kOrderCtas = 12 * 148;
+// Launches of one wave start all their tiles at once: no order to choose, and no past to read first.
+constexpr int64_t kOneWave = 148, kOrderCtas = 12 * kOneWave;
+
+__host__ __device__ __forceinline__ bool order_by_tile(unsigned tiles, unsigned pairs, unsigned seqs) {
+  const int64_t ctas = (int64_t)tiles * pairs * seqs;
+  return ctas > kOneWave && ctas <= kOrderCtas;
+}
 
 struct TileOrder {
   int qt, pair, b;  // query tile (may lie beyond the sequence's tiles), head pair, sequence
 };
 
-// Grid (tiles, pairs, sequences) of at most kOrderCtas CTAs; `past`: the first sequence's.
+// Grid (tiles, pairs, sequences) for which order_by_tile() holds; `past`: the first sequence's.
 __device__ __forceinline__ TileOrder tile_order(const int32_t* past, int tile_rows) {
   if (2 * (int64_t)*past > (int64_t)gridDim.x * tile_rows)
     return {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
