@@ -1425,7 +1425,9 @@ struct DeltaTile {
           vs = c == i ? p.v[s][i] : vs;
           ws = c == i ? p.w[s * C + i] : ws;
         }
-        o = fmaf(pv[s], vs, fmaf(-pk[s], ws, o));
+        // later tokens' coefficients are zero, but their rows may be infinite or NaN: left out, not multiplied
+        const float with = fmaf(pv[s], vs, fmaf(-pk[s], ws, o));
+        o = s <= t ? with : o;
       }
       if (c < cols && (KS <= NV || ks < NV)) p.so[t * CP + c] = o;
     }

@@ -107,3 +107,39 @@ def run(size, lens, layout, dtype):
         assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5, ls
         assert torch.equal(state.matrix_state[0], untouched)
         assert math.isfinite(got.sum().item())
+
+
+@pytest.mark.parametrize("layout", [0, 102, 104, 404])
+@pytest.mark.parametrize("at", [1, 6, 7, 34, 63])
+def test_what_is_not_finite_stays_behind_its_token(at, layout):
+    """An infinite or NaN entry of one token's row changes no bit of the tokens before it or of other sequences, whatever
+    place of its block the token has."""
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context, set_context
+
+    heads, kv, dim, vdim = 2, 1, 64, 64
+    lens, starts = [70, 9], [3, 0]
+    channels = 2 * kv * dim + heads * vdim
+    # a query, a key, a value, the gate, beta and the decay
+    places = [3, kv * dim + 5, 2 * kv * dim + 7, channels + 2, channels + heads * vdim, channels + heads * vdim + heads]
+
+    def once(place, value):
+        m, state, cols, ctx = setup(heads, kv, dim, vdim, lens, starts, torch.float32, 21)
+        if place is not None:
+            cols[at, place] = value
+        set_context(**ctx)
+        N.set_test_option("gla_layout", layout)
+        try:
+            return m(None, cols, state), state.matrix_state
+        finally:
+            N.set_test_option("gla_layout", 0)
+            reset_context()
+
+    clean, clean_state = once(None, None)
+    assert torch.isfinite(clean).all()
+    for place in places:
+        for value in (math.inf, -math.inf, math.nan):
+            got, state = once(place, value)
+            assert torch.equal(got[:at], clean[:at]) and torch.equal(got[lens[0]:], clean[lens[0]:]), (place, value)
+            assert torch.equal(state[2], clean_state[2])
+            assert value == value or not torch.isfinite(got[at:lens[0]]).all()
