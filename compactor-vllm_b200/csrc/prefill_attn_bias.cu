@@ -12,9 +12,17 @@
 //     log2 units with the slope's part added, so a row reads its 128 biases of a tile at consecutive addresses (and
 //     the 32 rows of a warp 32 neighbouring words); tiles wholly beyond the table add one constant.  With heads of 128 the
 //     ring gives up one of its five slots for the table.  One 4096-token portion, 32 / 8 heads of 128, window 1024, a table
-//     of 1024 rows, with the q / k norms and the cache write: 725 us on mma.sync, 154 us here;
+//     of 1024 rows, with the q / k norms and the cache write: 725 us on mma.sync, 170 us here;
+//   * EXACT: bias tables, heads of 64 and short pages came from bias_attn_varlen_mma_kernel, and must not be further from the
+//     formula than there.  Every exponential is ex2, and P is the sum of two bfloat16 numbers (2^-17 relative), whose low
+//     parts lie behind the high ones in the score's TMEM columns and take a second product with V.  With P in one part, a
+//     polynomial for 3 of 8 pairs and a reference up to 2^8 below the row's maximum (which then is not an exact 1 in P)
+//     these rows were 3 to 18 % further from 64 bits than on mma.sync; now they are 12 to 23 % nearer (the result's own
+//     rounding is left).  P in one part with the reference at every new maximum takes as long and is 0.3 to 0.7 % further.
+//     With the polynomial it is slower (the extra instructions are what bounds the tile).  Heads of 128 in whole pages without
+//     a table have always run here with the polynomial and one part;
 //   * pages shorter than a tile arrive in pieces of a page each; pieces past the last query's page are not loaded (the same
-//     portion without a window: pages of 64 1294 -> 214 us, heads of 64 601 -> 183 us).
+//     portion without a window: pages of 64 1293 -> 217 us, heads of 64 599 -> 174 us).
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -104,6 +112,12 @@ __device__ __forceinline__ float2 ex2_poly2_b(float2 x) {
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
 }
 
+// What rounding two probabilities to bfloat16 has left over, itself as bfloat16.
+__device__ __forceinline__ uint32_t rounded_off(float2 e, uint32_t hi) {
+  const float2 r = __fadd2_rn(e, make_float2(-__uint_as_float(hi << 16), -__uint_as_float(hi & 0xffff0000u)));
+  return pack2<true>(r.x, r.y);
+}
+
 #ifdef CVLLM_PREFILL_TRACE  // profiling build only (tools/trace_prefill.py): clock64 stamps of CTA (0,0,0), first 256 KV tiles
 __device__ long long g_pb_trace[8][256];
 #define P2_TRACE(rowi, jj)                                                                              \
@@ -114,13 +128,14 @@ __device__ long long g_pb_trace[8][256];
 #define P2_TRACE(rowi, jj) do { } while (0)
 #endif
 
-template <int kHD, bool DIST>
+template <int kHD, bool DIST, bool EXACT>
 __global__ void __launch_bounds__(pb::kThreads, 1)
 prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kc,
                          const __grid_constant__ CUtensorMap tm_vc, const PrefillBiasParams p) {
   using namespace pb;
   using Smem = PrefillBiasSmem<kHD, DIST>;
   constexpr bool BF16 = true;
+    constexpr int kPoly = EXACT ? 0 : kPolyPairsB;
   constexpr int kSlots = Smem::kSlots, kTileBytes = Smem::kTileBytes, kBoxes = kHD / 64;
   extern __shared__ unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -264,25 +279,26 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       const uint64_t v_desc = umma_smem_desc(smem_u32(sm.kv[slot_of(2 * j + 1)]), kBoxBytes, 1024);
       const uint32_t p_tmem = tmem_u + t * kBN;
       const uint32_t o_tmem = tmem_u + 256 + t * kHD;
+      auto pv = [&](int kk, bool first) {   // 16 keys
+        umma_ts_warp(o_tmem, p_tmem + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, first ? 0u : 1u);
+        if constexpr (EXACT) umma_ts_warp(o_tmem, p_tmem + kBN / 2 + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, 1u);
+      };
 #if CVLLM_PREFILL_P_SPLIT > 0
       mbar_wait(&sm.p_half[t], j & 1);
       P2_TRACE(2 * t, j);
       tc_fence_after();
 #pragma unroll
-      for (int kk = 0; kk < 2 * kPSplitB; ++kk)
-        umma_ts_warp(o_tmem, p_tmem + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+      for (int kk = 0; kk < 2 * kPSplitB; ++kk) pv(kk, j == 0 && kk == 0);
       mbar_wait(&sm.p_full[t], j & 1);
       tc_fence_after();
 #pragma unroll
-      for (int kk = 2 * kPSplitB; kk < kBN / 16; ++kk)
-        umma_ts_warp(o_tmem, p_tmem + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, 1u);
+      for (int kk = 2 * kPSplitB; kk < kBN / 16; ++kk) pv(kk, false);
 #else
       mbar_wait(&sm.p_full[t], j & 1);
       P2_TRACE(2 * t, j);
       tc_fence_after();
 #pragma unroll
-      for (int kk = 0; kk < kBN / 16; ++kk)
-        umma_ts_warp(o_tmem, p_tmem + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+      for (int kk = 0; kk < kBN / 16; ++kk) pv(kk, j == 0 && kk == 0);
 #endif
       if (t == 1) umma_commit_warp(&sm.empty[slot_of(2 * j + 1)]);
       umma_commit_warp(&sm.o_done[t]);
@@ -448,7 +464,7 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         float2 l2a = make_float2(0.f, 0.f), l2b = make_float2(0.f, 0.f);
 #pragma unroll
         for (int c = 0; c < kBN / 32; ++c) {
-          uint32_t pk[16];
+          uint32_t pk[16], lo[EXACT ? 16 : 1];
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
             const float2 t0 = __ffma2_rn(make_float2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), sc2, nm2);
@@ -456,12 +472,12 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #ifdef CVLLM_PROBE_NO_EXP  // timing probe only (wrong results): the loop without its MUFU work — 7.6 ms, unchanged
             const float2 e0 = t0, e1 = t1;
 #else
-            // kPolyPairsB = e: e of every 8 logit pairs (two loop trips, four pairs each... slots b0 b2 b1 b3 a1 a3 a0 a2)
+            // kPoly = e: e of every 8 logit pairs (two loop trips, four pairs each... slots b0 b2 b1 b3 a1 a3 a0 a2)
             const int slot = (i >> 1) & 3;
-            const bool p1 = (kPolyPairsB >= 1 && slot == 0) || (kPolyPairsB >= 2 && slot == 2) ||
-                            (kPolyPairsB >= 3 && slot == 1) || (kPolyPairsB >= 4 && slot == 3);
-            const bool p0 = (kPolyPairsB >= 5 && slot == 1) || (kPolyPairsB >= 6 && slot == 3) ||
-                            (kPolyPairsB >= 7 && slot == 0) || (kPolyPairsB >= 8 && slot == 2);
+            const bool p1 = (kPoly >= 1 && slot == 0) || (kPoly >= 2 && slot == 2) || (kPoly >= 3 && slot == 1) ||
+                            (kPoly >= 4 && slot == 3);
+            const bool p0 = (kPoly >= 5 && slot == 1) || (kPoly >= 6 && slot == 3) || (kPoly >= 7 && slot == 0) ||
+                            (kPoly >= 8 && slot == 2);
             const float2 e0 = p0 ? ex2_poly2_b(t0) : make_float2(ex2(t0.x), ex2(t0.y));
             const float2 e1 = p1 ? ex2_poly2_b(t1) : make_float2(ex2(t1.x), ex2(t1.y));
 #endif
@@ -469,8 +485,13 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             l2b = __fadd2_rn(l2b, e1);
             pk[i] = pack2<BF16>(e0.x, e0.y);
             pk[i + 1] = pack2<BF16>(e1.x, e1.y);
+            if constexpr (EXACT) {
+              lo[i] = rounded_off(e0, pk[i]);
+              lo[i + 1] = rounded_off(e1, pk[i + 1]);
+            }
           }
           tmem_st16(s_tmem + c * 16, pk);
+          if constexpr (EXACT) tmem_st16(s_tmem + kBN / 2 + c * 16, lo);
 #if CVLLM_PREFILL_P_SPLIT > 0
           if (c == kPSplitB - 1) {  // the first part of P (and any O rescale before it) is in TMEM
             tc_wait_st();
@@ -545,15 +566,15 @@ bool cvllm_prefill_bias_serves(int D, int Dv, int page_size, int dist_rows) {
 
 namespace {
 
-template <int HD, bool DIST>
+template <int HD, bool DIST, bool EXACT>
 int launch_bias(const CUtensorMap& tm_q, const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, const PrefillBiasParams& p,
                 int max_seqlen_q, cudaStream_t st) {
   const size_t smem = sizeof(PrefillBiasSmem<HD, DIST>) + 1024;
   static_assert(sizeof(PrefillBiasSmem<HD, DIST>) + 1024 <= 227 * 1024, "shared memory");
   const dim3 grid((max_seqlen_q + pb::kBM - 1) / pb::kBM, p.HQ / 2, p.B);
   static std::atomic<uint64_t> attr{0};
-  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn_bias_kernel<HD, DIST>, (int)smem, attr));
-  prefill_attn_bias_kernel<HD, DIST><<<grid, pb::kThreads, smem, st>>>(tm_q, tm_kc, tm_vc, p);
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn_bias_kernel<HD, DIST, EXACT>, (int)smem, attr));
+  prefill_attn_bias_kernel<HD, DIST, EXACT><<<grid, pb::kThreads, smem, st>>>(tm_q, tm_kc, tm_vc, p);
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }
@@ -595,6 +616,7 @@ int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_
     const float t = test_options().prefill_threshold.load(std::memory_order_relaxed);
     if (t >= 0.f) p.rescale_threshold = t;
   }
+  const bool exact = HD == 64 || dist_bias || PS % kBN;   // see the top
   p.chunk = chunk;
   p.window = window;
   p.keep = keep;
@@ -602,11 +624,12 @@ int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_
   p.sink_logits = sink ? sink_logits : nullptr;
   p.dist_bias = dist_bias;
   p.dist_rows = dist_rows;
-  if (HD == 128)
-    return dist_bias ? launch_bias<128, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
-                     : launch_bias<128, false>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
-  return dist_bias ? launch_bias<64, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
-                   : launch_bias<64, false>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
+  if (HD == 64)
+    return dist_bias ? launch_bias<64, true, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
+                     : launch_bias<64, false, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
+  if (dist_bias) return launch_bias<128, true, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
+  return exact ? launch_bias<128, false, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
+               : launch_bias<128, false, false>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);
 }
 
 #ifdef CVLLM_PREFILL_TRACE
