@@ -104,6 +104,8 @@ _SIGNATURES = {
     "cvllm_bias_attn_decode": (_i, [_p, _p, _p, _p, _i64, _i64, _i, _p, _p, _p, _i, _i, _p, _f, _p,
                                     _i, _i, _i, _i, _i, _i, _i, _p, _sz, _i64, _i, _p]),
     "cvllm_bias_decode_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "cvllm_bias_attn_decode_stream": (_i, [_p, _p, _p, _i64, _p, _i64, _i64, _i, _p, _p, _p, _i, _i, _i, _p, _i, _i, _p, _f,
+                                           _p, _i64, _i, _i, _i, _i, _i, _p, _sz, _p]),
     "cvllm_residual_norm": (_i, [_p, _i64, _p, _i64, _i, _p, _i64, _p, _i64, _p, _p, _p, _i64, _i, _i, _i, _f, _i, _p]),
     "cvllm_embed_norm": (_i, [_p, _p, _i, _p, _p, _i, _p, _i64, _p, _i64, _i, _i, _i, _f, _p]),
     "cvllm_pair_hash_embed": (_i, [_p, _p, _p, _p, _p, _f, _i64, _i64, _i64, _p, _p, _i64, _i, _i, _i, _i, _p]),

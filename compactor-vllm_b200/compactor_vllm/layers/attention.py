@@ -312,19 +312,20 @@ class BiasedChunkAttention(nn.Module):
                 and k.dtype == torch.bfloat16 and self.head_dim % 8 == 0 and self.v_head_dim % 8 == 0
                 and self.v_head_dim <= 512 and self.slopes is None and self.rel is None and int(self.page_size) % 64 == 0)
 
-    def streaming_decode_kernel(self, max_keys: int) -> bool:
-        """Whether a decode step goes to the streaming kernel of csrc/decode_attn.cu (the library takes it when the sizes
-        allow and the workspace holds its scratch): where the keys a query may see are two of its units of 128 or more.
-        Measured at 32 / 8 heads of 64, 32 sequences (streaming / key splits): up to 140 keys 19 / 14 us, up to 280 keys
-        21.2 / 21.3 us; heads of 128, up to 280 keys 25 / 31 us, 8 x 4096 keys 37 / 104 us."""
-        if self.chunk:
-            max_keys = min(max_keys, self.chunk)
+    def streaming_decode_kernel(self, max_keys: int, batch: int = 1) -> bool:
+        """Whether a decode step goes to the streaming kernel of csrc/decode_attn.cu: where it serves the sizes and the keys
+        that a query may see (kept first tokens among them) are two of its units of 128 or more.  It reads the cache at the
+        rate of the plain decode kernel but has a prologue, and a fold behind it.  Layer step with norms and cache write in
+        a graph, 32 / 8 heads of 128 (streaming / key splits): 8 x 4096 keys 37 / 104 us, 8 x 200 14 / 21, 1 x 200 13 / 20,
+        32 x 200 25 / 31; heads of 64, 32 sequences: up to 140 keys 19 / 14 us, up to 280 keys 21.2 / 21.3."""
+        keys = min(max_keys, self.chunk) if self.chunk else max_keys
         if self.window:
-            max_keys = min(max_keys, self.window)
+            keys = min(keys, self.window)
+        keys = min(keys + self.keep_first, max_keys)
         D, page = self.head_dim, int(self.page_size)
-        return (max_keys >= 256 and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
-                and self.num_heads // self.num_kv_heads <= 8 and self.k_cache.dtype == torch.bfloat16
-                and (page % 128 == 0 or page in (16, 32, 64)))
+        return (keys >= 256 and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
+                and self.num_heads // self.num_kv_heads <= 8 and batch * self.num_kv_heads <= 4096
+                and self.k_cache.dtype == torch.bfloat16 and (page % 128 == 0 or page in (16, 32, 64)))
 
     def forward(self, qkv: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         ctx: Context = get_context()
@@ -395,17 +396,23 @@ class BiasedChunkAttention(nn.Module):
                 self.k_cache.shape[0], pt.shape[-1], v_stride, code, N.stream(dev)), "cvllm_bias_attn_varlen")
         else:
             assert ctx.batch_mapping.numel() == T
-            if self.streaming_decode_kernel(int(ctx.max_seqlen_k)):
-                splits, ws_bytes = 1, N.sized("cvllm_bias_decode_workspace_bytes", T, H, G, D)
+            max_keys = int(ctx.max_seqlen_k)
+            if (self.streaming_decode_kernel(max_keys, T) and o_stride % 2 == 0 and out.data_ptr() % 4 == 0
+                    and (q.data_ptr() | self.k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
+                ws = N.workspace(dev, N.sized("cvllm_bias_decode_workspace_bytes", T, H, G, D), "bias_attn_stream")
+                N.check(lib.cvllm_bias_attn_decode_stream(
+                    N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), self.k_cache.shape[0], *table, N.ptr(ctx.positions_i32),
+                    N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
+                    self.scale, N.ptr(out), o_stride, T, H, G, D, RESERVED_BATCH, N.ptr(ws), ws.numel(), N.stream(dev)),
+                    "cvllm_bias_attn_decode_stream")
             else:
-                splits = self.decode_splits(T, int(ctx.max_seqlen_k))
-                ws_bytes = 4 * T * H * splits * (2 + Dv) if splits > 1 else 0
-            ws = N.workspace(dev, ws_bytes, "bias_attn_decode") if ws_bytes else None
-            N.check(lib.cvllm_bias_attn_decode_dist(
-                N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.positions_i32),
-                N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
-                self.scale, N.ptr(out), o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits, N.ptr(ws), ws.numel() if ws is not None else 0, v_stride, code,
-                N.stream(dev)), "cvllm_bias_attn_decode")
+                splits = self.decode_splits(T, max_keys)
+                ws = N.workspace(dev, 4 * T * H * splits * (2 + Dv), "bias_attn_decode") if splits > 1 else None
+                N.check(lib.cvllm_bias_attn_decode_dist(
+                    N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.positions_i32),
+                    N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
+                    self.scale, N.ptr(out), o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits,
+                    N.ptr(ws), ws.numel() if ws is not None else 0, v_stride, code, N.stream(dev)), "cvllm_bias_attn_decode")
         if keep != Dv:
             out = out.view(T, H, Dv)[:, :, :keep]
             return out.reshape(T, H * keep) if flat else out

@@ -1212,8 +1212,8 @@ int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_
                               const float* sink_logits, const float* dist_bias, int dist_rows, int64_t o_stride,
                               cudaStream_t st);
 
-// decode_attn.cu: the streaming decode kernel (TMA ring, mma.sync, 32-bit P as two 16-bit parts)
-bool cvllm_bias_decode_serves(int H, int G, int D, int Dv, int page_size, int64_t o_stride);
+// decode_attn.cu: the streaming decode kernel (TMA ring, mma.sync, P as the sum of two bfloat16 numbers)
+bool cvllm_bias_decode_serves(int B, int H, int G, int D, int page_size, int64_t o_stride);
 int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows, void* out,
                              int64_t o_stride, const int32_t* positions, const int32_t* batch_mapping,
                              const int32_t* page_table, int64_t pt_slot, int64_t pt_head, int B, int H, int G, int D, int PS,
@@ -1477,18 +1477,6 @@ extern "C" int cvllm_bias_attn_decode_dist(const void* q, const void* k_cache, c
     CVLLM_CHECK_LAUNCH();
     return CVLLM_OK;
   }
-  // The streaming kernel reads the cache at the rate of the plain decode kernel but has a prologue and a fold behind it:
-  // steps of 200 keys and more win, layer step with norms and cache write in a graph, 32 / 8 heads (streaming / splits):
-  // 8 x 4096 keys 37 / 104 us, 8 x 200 14 / 21, 1 x 200 13 / 20, 32 x 200 25 / 31 (heads of 64: 21.2 / 21.3); with a unit
-  // of keys per head, 32 x 100, splits win, 14 / 19 us with heads of 64.  The caller sends steps of up to 255 keys there by
-  // not bringing the workspace.
-  if (dtype == CVLLM_BF16 && path == 0 && cvllm_bias_decode_serves(H, G, D, Dv, page_size, out_stride) && v_stride == Dv &&
-      cache_rows > 0 && workspace != nullptr && workspace_bytes >= cvllm_bias_decode_workspace_bytes(B, H, G, D) &&
-      (int64_t)B * G <= 4096 && aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(workspace) &&
-      reinterpret_cast<uintptr_t>(out) % 4 == 0)
-    return cvllm_launch_bias_decode(q, k_cache, v_cache, cache_rows, out, out_stride, positions, batch_mapping, page_table,
-                                    table_stride_slot, table_stride_head, B, H, G, D, page_size, scale, slopes, chunk, window,
-                                    keep_first, dist_bias, dist_rows, sink, sink_logits, reserved_slot, workspace, st);
   if (D % 8 == 0 && Dv % 8 == 0 && D <= 256 && Dv <= 256 && v_stride % 8 == 0 && aligned16(k_cache) &&
       aligned16(v_cache)) {
     if (splits > 1) {
@@ -1518,4 +1506,37 @@ extern "C" int cvllm_bias_attn_decode_dist(const void* q, const void* k_cache, c
         static_cast<float*>(out), out_stride, H, G, D, Dv, reserved_slot);
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
+}
+
+// The caller chooses this entry (cvllm_bias_attn_decode_dist never comes here, whatever its workspace holds).
+extern "C" int cvllm_bias_attn_decode_stream(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows,
+                                             const int32_t* page_table, int64_t table_stride_slot,
+                                             int64_t table_stride_head, int page_size, const int32_t* positions,
+                                             const int32_t* batch_mapping, const float* slopes, int chunk, int window,
+                                             int keep_first, const float* dist_bias, int dist_rows, int sink,
+                                             const float* sink_logits, float scale, void* out, int64_t out_stride, int B,
+                                             int H, int G, int D, int reserved_slot, float* workspace,
+                                             size_t workspace_bytes, cvllm_stream_t stream) {
+  CVLLM_CHECK_ARG(B >= 0 && H > 0 && G > 0 && H % G == 0 && D > 0 && chunk >= 0 && cache_rows > 0 && page_size > 0);
+  CVLLM_CHECK_ARG(window >= 0 && keep_first >= 0 && (dist_bias == nullptr || dist_rows > 0));
+  CVLLM_CHECK_ARG(out_stride == 0 || out_stride >= (int64_t)H * D);
+  if (out_stride == 0) out_stride = (int64_t)H * D;
+  if (B == 0) return CVLLM_OK;
+  CVLLM_CHECK_ARG(q && k_cache && v_cache && page_table && positions && batch_mapping && out && workspace);
+  if (test_options().bias_attn_fma.load() != 0)   // tests: the key-split kernel with one part
+    return cvllm_bias_attn_decode_dist(q, k_cache, v_cache, page_table, table_stride_slot, table_stride_head, page_size,
+                                       positions, batch_mapping, slopes, chunk, window, keep_first, dist_bias, dist_rows,
+                                       sink, sink_logits, scale, out, out_stride, B, H, G, D, D, cache_rows, reserved_slot,
+                                       1, nullptr, 0, D, CVLLM_BF16, stream);
+  CVLLM_CHECK_SUPPORTED(cvllm_bias_decode_serves(B, H, G, D, page_size, out_stride));
+  CVLLM_CHECK_ALIGN(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(workspace) &&
+                    reinterpret_cast<uintptr_t>(out) % 4 == 0);
+  if (workspace_bytes < cvllm_bias_decode_workspace_bytes(B, H, G, D)) {
+    set_last_error("decode workspace too small");
+    return CVLLM_E_WORKSPACE;
+  }
+  return cvllm_launch_bias_decode(q, k_cache, v_cache, cache_rows, out, out_stride, positions, batch_mapping, page_table,
+                                  table_stride_slot, table_stride_head, B, H, G, D, page_size, scale, slopes, chunk, window,
+                                  keep_first, dist_bias, dist_rows, sink, sink_logits, reserved_slot, workspace,
+                                  static_cast<cudaStream_t>(stream));
 }

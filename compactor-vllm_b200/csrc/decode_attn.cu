@@ -26,7 +26,7 @@
 // HBM-bound: 4*D bytes per cached (token, head).
 //
 // BIAS: the same streaming for the biased attention's decode steps (cvllm_launch_bias_decode, called by
-// cvllm_bias_attn_decode): heads of 128 or 64, keys 0 .. position of a sequence cut by its chunk or window (the unit list
+// cvllm_bias_attn_decode_stream): heads of 128 or 64, keys 0 .. position of a sequence cut by its chunk or window (the unit list
 // starts at the first visible key's unit, behind the units of kept first tokens), a distance bias and a sink in the softmax.
 // What that path computes in 32 bits stays so: P is the sum of two 16-bit numbers (2^-17 relative), whose low parts take
 // the query columns 4 .. 7 that groups of up to four heads leave free.  Partial states are folded by a second kernel
@@ -839,8 +839,8 @@ static int launch_decode_attn(const void* q, void* out, const void* k_cache, con
 
 // What the streaming kernel serves of the biased attention's decode steps (bfloat16, contiguous 16-byte aligned rows), and
 // the scratch that it needs there.
-bool cvllm_bias_decode_serves(int H, int G, int D, int Dv, int page_size, int64_t o_stride) {
-  return D == Dv && (D == 128 || D == 64) && H / G <= 8 && o_stride % 2 == 0 &&
+bool cvllm_bias_decode_serves(int B, int H, int G, int D, int page_size, int64_t o_stride) {
+  return (D == 128 || D == 64) && H / G <= 8 && (int64_t)B * G <= 4096 && o_stride % 2 == 0 &&
          (page_size % kUnit == 0 || page_size == 64 || page_size == 32 || page_size == 16);
 }
 extern "C" size_t cvllm_bias_decode_workspace_bytes(int B, int H, int G, int D) {

@@ -565,10 +565,6 @@ int cvllm_bias_attn_varlen_dist(const void* q, const void* k_cache, const void* 
                                 const float* dist_bias, int dist_rows, int sink, const float* sink_logits, float scale,
                                 void* out, int64_t out_stride, int B, int max_new, int H, int G, int D, int Dv, int total_tokens, int64_t cache_rows, int pages_per_head,
                                 int64_t v_stride, int dtype, cvllm_stream_t stream);
-/* Decode in bfloat16 with D = Dv = 128 or 64, pages of 16, 32, 64 or a multiple of 128 rows, H / G <= 8 and cache_rows given
- * takes the streaming kernel of csrc/decode_attn.cu when workspace_bytes >= cvllm_bias_decode_workspace_bytes(B, H, G, D)
- * (`splits` then counts for nothing; the workspace needs no initial contents). */
-size_t cvllm_bias_decode_workspace_bytes(int B, int H, int G, int D);
 int cvllm_bias_attn_decode_dist(const void* q, const void* k_cache, const void* v_cache, const int32_t* page_table,
                                 int64_t table_stride_slot, int64_t table_stride_head, int page_size,
                                 const int32_t* positions, const int32_t* batch_mapping, const float* slopes, int chunk,
@@ -576,6 +572,19 @@ int cvllm_bias_attn_decode_dist(const void* q, const void* k_cache, const void* 
                                 const float* sink_logits, float scale, void* out, int64_t out_stride, int B, int H,
                                 int G, int D, int Dv, int64_t cache_rows, int reserved_slot, int splits, float* workspace, size_t workspace_bytes, int64_t v_stride, int dtype,
                                 cvllm_stream_t stream);
+
+/* The same decode step on the streaming kernel of csrc/decode_attn.cu, where it serves: bfloat16, keys and values of D = 128
+ * or 64 numbers, pages of 16, 32, 64 or a multiple of 128 rows, H / G <= 8, B * G <= 4096, an even out_stride, q, caches and
+ * workspace on 16 bytes, out on 4 (anything else is refused).  workspace: cvllm_bias_decode_workspace_bytes bytes, no
+ * initial contents.  The caller chooses between the two entries by the keys that its queries may see. */
+size_t cvllm_bias_decode_workspace_bytes(int B, int H, int G, int D);
+int cvllm_bias_attn_decode_stream(const void* q, const void* k_cache, const void* v_cache, int64_t cache_rows,
+                                  const int32_t* page_table, int64_t table_stride_slot, int64_t table_stride_head,
+                                  int page_size, const int32_t* positions, const int32_t* batch_mapping,
+                                  const float* slopes, int chunk, int window, int keep_first, const float* dist_bias,
+                                  int dist_rows, int sink, const float* sink_logits, float scale, void* out,
+                                  int64_t out_stride, int B, int H, int G, int D, int reserved_slot, float* workspace,
+                                  size_t workspace_bytes, cvllm_stream_t stream);
 
 /* How many CTAs of the latent tcgen05 kernel have given up on a wait since the library was loaded (their outputs are
  * NaN); synchronises. */

@@ -216,3 +216,49 @@ def test_decoding_far_sinks_and_scores():
     got = decode(m, q)
     assert torch.isfinite(got).all()
     assert ((got - want).norm() / want.norm()).item() < 2.5e-3
+
+
+def test_decode_kernel_does_not_depend_on_earlier_steps():
+    """What a step runs on follows from the step: a step on three key splits gives the same bits before and after a step that
+    left a large workspace behind, and those are not the streaming kernel's."""
+    m, q, keys = make(8, 2, 128, 128, DECODE, 15, sink=True)
+    streamed = decode(m, q)
+    m.streaming_decode_kernel, m.decode_splits = lambda *_: False, lambda *_: 3
+    before = decode(m, q)
+    assert not torch.equal(before, streamed)
+    long, q_long, _ = make(8, 2, 128, 128, [(300, 1)] * 150, 16, sink=True)
+    context([(300, 1)] * 150, True)
+    long.attend(q_long)
+    assert torch.equal(decode(m, q), before)
+
+
+def test_kept_tokens_count_for_the_choice_of_the_decode_kernel():
+    m, q, keys = make(4, 2, 128, 128, [(40, 1)], 18, window=128, keep_first=512)
+    assert m.streaming_decode_kernel(4096) and m.streaming_decode_kernel(256) and not m.streaming_decode_kernel(255)
+
+
+@pytest.mark.parametrize("what", ["out", "query", "width"])
+def test_decoding_into_rows_that_the_streaming_kernel_refuses(what):
+    """Outputs off the 4-byte grid, at odd row strides, or queries off the 16-byte grid take the key splits, as many as
+    the step's keys ask for."""
+    from compactor_vllm.utils.context import reset_context
+
+    m, q, keys = make(8, 2, 64, 64, DECODE, 19, sink=True)
+    T, width = q.shape[0], 8 * 64
+    if what == "query":
+        flat = torch.zeros(q.numel() + 1, dtype=q.dtype, device=DEV)
+        flat[1:] = q.flatten()
+        q = flat[1:].view_as(q)
+    rows = width + (1 if what == "width" else 2)
+    out = torch.zeros(T * rows + 1, dtype=q.dtype, device=DEV)[1 if what == "out" else 0:][:T * rows].view(T, rows)[:, :width]
+    want = formula(m, q, keys, DECODE)
+    context(DECODE, True)
+    asked = []
+    splits = m.decode_splits
+    m.decode_splits = lambda *a: asked.append(splits(*a)) or asked[-1]
+    try:
+        got = m.attend(q, out=out if what != "query" else None).double()
+    finally:
+        reset_context()
+    assert asked and asked[0] > 1
+    assert ((got - want).norm() / want.norm()).item() < 2.5e-3
