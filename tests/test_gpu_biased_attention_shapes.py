@@ -174,11 +174,11 @@ def test_portions_lose_no_precision(case):
 DECODE = [(p, 1) for p in (0, 1, 127, 128, 255, 299, 300, 511, 640, 1100)]
 
 
-def decode(m, q, option=0):
+def decode(m, q, option=0, spans=DECODE):
     from compactor_vllm import _native as N
     from compactor_vllm.utils.context import get_context, reset_context
 
-    context(DECODE, True)
+    context(spans, True)
     get_context().batch_mapping[4] = 0       # a padding row
     N.set_test_option("bias_attn_fma", option)
     try:
@@ -216,6 +216,25 @@ def test_decoding_far_sinks_and_scores():
     got = decode(m, q)
     assert torch.isfinite(got).all()
     assert ((got - want).norm() / want.norm()).item() < 2.5e-3
+
+
+# whole units lie between the kept tokens and the window or the chunk of the last ones
+KEPT = [(p, 1) for p in (0, 255, 256, 383, 511, 640, 767, 1100, 1535, 1900)]
+
+
+@pytest.mark.parametrize("window,keep,chunk", [(256, 5, 0), (300, 130, 0), (256, 400, 0), (0, 140, 256), (700, 3, 512), (257, 1, 0)])
+@pytest.mark.parametrize("D,page", [(128, 128), (128, 64), (64, 128), (64, 16)])
+def test_decoding_with_kept_tokens(D, page, window, keep, chunk):
+    """Kept first tokens on the streaming kernel: fewer than a unit, several units, up to and into the window's first."""
+    m, q, keys = make(8, 2, D, page, KEPT, 14, **options(1, 8, 60, True, "zero", window, keep, chunk))
+    dress(m, 60, 5)
+    assert m.streaming_decode_kernel(1901)
+    want = formula(m, q, keys, KEPT)
+    want[4] = 0
+    err = lambda x: ((x - want).norm() / want.norm()).item()
+    got = decode(m, q, spans=KEPT)
+    assert torch.isfinite(got).all() and (got[4] == 0).all()
+    assert err(got) < 2.5e-3 and err(got) < 1.05 * err(decode(m, q, 1, KEPT)) + 1e-6
 
 
 def test_decode_kernel_does_not_depend_on_earlier_steps():
