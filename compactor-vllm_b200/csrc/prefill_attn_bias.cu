@@ -17,7 +17,7 @@
 //     formula than there.  Every exponential is ex2, and P is the sum of two bfloat16 numbers (2^-17 relative), whose low
 //     parts lie behind the high ones in the score's TMEM columns and take a second product with V.  With P in one part, a
 //     polynomial for 3 of 8 pairs and a reference up to 2^8 below the row's maximum (which then is not an exact 1 in P)
-//     these rows were 3 to 18 % further from 64 bits than on mma.sync; now they are 12 to 23 % nearer (the result's own
+//     these rows were 2.5 to 19 % further from 64 bits than on mma.sync; now they are 12 to 23 % nearer (the result's own
 //     rounding is left).  P in one part with the reference at every new maximum takes as long and is 0.3 to 0.7 % further.
 //     With the polynomial it is slower (the extra instructions are what bounds the tile).  Heads of 128 in whole pages without
 //     a table have always run here with the polynomial and one part;
@@ -135,7 +135,7 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   using namespace pb;
   using Smem = PrefillBiasSmem<kHD, DIST>;
   constexpr bool BF16 = true;
-    constexpr int kPoly = EXACT ? 0 : kPolyPairsB;
+  constexpr int kPoly = EXACT ? 0 : kPolyPairsB;
   constexpr int kSlots = Smem::kSlots, kTileBytes = Smem::kTileBytes, kBoxes = kHD / 64;
   extern __shared__ unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -319,6 +319,20 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         }
         fence_proxy_async_smem();
         __syncwarp();
+      }
+      if constexpr (EXACT) {
+        // nor do keys before the first row's chunk or window, which share its tile, reach any row of this CTA: their
+        // values may be infinite or NaN
+        const int base = tile_base(j), hidden = min(lo0 - base, kBN), shown = max(p.keep - base, 0);   // rows shown .. hidden - 1
+        if (hidden > shown) {
+          uint4* v4 = reinterpret_cast<uint4*>(sm.kv[slot_of(n)]);
+          for (int idx = lane; idx < (hidden - shown) * 8 * kBoxes; idx += 32) {
+            const int r = shown + idx / (8 * kBoxes), c = idx % (8 * kBoxes);
+            v4[(c >> 3) * (kBoxBytes / 16) + r * 8 + (c & 7)] = make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
       }
       tc_fence_after();
     };

@@ -281,3 +281,41 @@ def test_decoding_into_rows_that_the_streaming_kernel_refuses(what):
         reset_context()
     assert asked and asked[0] > 1
     assert ((got - want).norm() / want.norm()).item() < 2.5e-3
+
+
+@pytest.mark.parametrize("D,page,rows", [(128, 64, 0), (128, 128, 40), (64, 128, 0), (64, 16, 40)])
+@pytest.mark.parametrize("window,keep,chunk", [(300, 0, 0), (300, 5, 0), (0, 130, 256)])
+def test_values_that_no_row_sees(D, page, rows, window, keep, chunk):
+    """Values outside every query's window or chunk that share a tile with seen ones may be infinite or NaN."""
+    from compactor_vllm.utils.context import reset_context
+
+    start, n = 1100, 50
+    m, q, keys = make(4, 2, D, page, [(start, n)], 21, **options(1, 4, rows, False, "zero", window, keep, chunk))
+    dress(m, rows, 6)
+    (k, v), p = keys[0], torch.arange(start + n, device=DEV)
+    seen = p >= (start - window + 1 if window else start // chunk * chunk)
+    hidden = p[~seen & (p >= keep)]
+    for h in range(2):
+        at = m.page_table[1, h].long()[hidden // page] * page + hidden % page
+        m.v_cache[at] = torch.tensor([math.inf, math.nan, -math.inf], device=DEV).to(torch.bfloat16)[hidden % 3][:, None]
+    want = formula(m, q, keys, [(start, n)])
+    context([(start, n)], False)
+    try:
+        got = m.attend(q).double()
+    finally:
+        reset_context()
+    assert torch.isfinite(got).all()
+    assert ((got - want).norm() / want.norm()).item() < 6e-3
+    last = [(start + n - 1, 1)]
+    got, want = decode_one(m, q[-1:].contiguous(), last), formula(m, q[-1:].contiguous(), keys, last)
+    assert ((got - want).norm() / want.norm()).item() < 2.5e-3
+
+
+def decode_one(m, q, spans):
+    from compactor_vllm.utils.context import reset_context
+
+    context(spans, True)
+    try:
+        return m.attend(q).double()
+    finally:
+        reset_context()
