@@ -452,7 +452,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
           mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
         }
-        if constexpr (BIAS) { m0 = fmaxf(m0, -1e30f); m1 = fmaxf(m1, -1e30f); }   // a first unit may be all masked
+        if constexpr (BIAS) {   // a first unit may be all masked: the lowest finite reference, so that every score can pass it
+          m0 = fmaxf(m0, -3.402823466e38f);
+          m1 = fmaxf(m1, -3.402823466e38f);
+        }
         float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
         // a NaN/-inf column max (garbage q) must not poison the rest
         if (!(mn0 > -INFINITY)) mn0 = 0.f;

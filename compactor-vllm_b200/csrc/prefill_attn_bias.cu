@@ -447,8 +447,9 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           mx2 = fmaxf(mx2, s[c + 2]);
           mx3 = fmaxf(mx3, s[c + 3]);
         }
-        // a row that sees no key of this tile (it lies before the row's chunk or window) keeps a finite reference
-        return fmaxf(fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)), -1e30f);
+        // a row that sees no key of this tile (it lies before the row's chunk or window) keeps a finite reference; the
+        // lowest there is, since any higher one would make lower scores weigh nothing among themselves
+        return fmaxf(fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)), -3.402823466e38f);
       };
       // O *= alpha, l *= alpha, m_ref <- m_to.  O holds PV(0..j-1); PV(j-1) may still be in flight.
       auto rescale_to = [&](float m_to) {

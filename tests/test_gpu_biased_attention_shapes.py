@@ -319,3 +319,30 @@ def decode_one(m, q, spans):
         return m.attend(q).double()
     finally:
         reset_context()
+
+
+@pytest.mark.parametrize("D,page", [(128, 64), (64, 128)])
+def test_scores_far_below(D, page):
+    """Scores of -10^32 are scores: they weigh nothing beside others and the same among themselves."""
+    from compactor_vllm.utils.context import reset_context
+
+    spans = [(0, 200), (300, 90)]
+    m, q, keys = make(4, 2, D, page, spans, 22)
+    m.dist_bias = torch.zeros(150, 4, device=DEV)
+    m.dist_bias[:140] = -1e32
+    m.rel = torch.nn.Parameter(m.dist_bias)
+    context(spans, False)
+    try:
+        got = m.attend(q).double()
+    finally:
+        reset_context()
+    want = formula(m, q, keys, spans)
+    assert torch.isfinite(got).all()
+    assert ((got - want).norm() / want.norm()).item() < 6e-3
+    m.dist_bias[140:] = -1e32
+    at = [(389, 1)]
+    m2, q2, keys2 = make(4, 2, D, page, at, 23)
+    m2.dist_bias, m2.rel = m.dist_bias, m.rel
+    got, want = decode_one(m2, q2, at), formula(m2, q2, keys2, at)
+    assert m2.streaming_decode_kernel(390)
+    assert ((got - want).norm() / want.norm()).item() < 2.5e-3
