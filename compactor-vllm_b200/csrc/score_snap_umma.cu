@@ -20,7 +20,7 @@
 // What bounds the passes: pass 1 the read of K, pass 2 the exponentials (128 x 128 a tile at 16 per clock: 1024
 // clocks).  A CTA holds the SM (TMEM, 160 KB of shared memory), so the grid runs in waves of 148 CTAs and a start
 // (barriers, TMEM, the first tile's latency, in pass 2 the statistics) costs as much as four tiles: see
-// snap_split() for how many CTAs a call is cut into.
+// snap_split_tiles() for how many CTAs a call is cut into.
 #include <algorithm>
 
 #include "common.cuh"
@@ -299,40 +299,41 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
 using namespace cvllm;
 
-// Key tiles per CTA.  A CTA holds its SM, and its start costs about four tiles, so few (sequence, head) pairs are
-// cut so that all CTAs run at once: `waves` x 148 CTAs over the heads, less one per further sequence (whose last
-// split is short on average), with a second or third wave only where several sequences, which may differ in
-// length, would otherwise get fewer than four splits each.  From 74 pairs on the pairs themselves fill the chip and
-// a CTA takes 8 tiles, which keeps sequences of unequal length balanced.  Fixed splits of 1024
-// keys were 2.2 waves at 40960 keys and 8 heads, and 8 CTAs at 1000: 4096 and 12000 keys took 34.5 us, now 26.5; with
-// four sequences of 8000 or of 500-20000 keys 69 and 72.5 -> 65 and 69.
-static int snap_waves(int B, int HKV) {
-  if ((int64_t)B * HKV > sn::kSms / 2) return 0;
-  int waves = 1;
-  while (waves * sn::kSms / HKV - (B - 1) < (B > 1 ? 4 * B : 1)) ++waves;
-  return waves;
+// Key tiles per CTA.  A CTA holds its SM, and its start costs about four tiles.  Few (sequence, head) pairs are cut into as
+// many splits as make the waves of CTAs, each of a start and a split, shortest; the splits beyond a shorter sequence's
+// end (the caller's bound may be all the keys of a batch) also take their turn on an SM, about 0.02 tiles of the whole
+// launch each.  From 74 pairs on the pairs themselves fill the chip and a CTA takes 8 tiles, which keeps sequences of
+// unequal length balanced.
+// In a graph, 32 / 8 heads, us, fixed splits of 8 tiles / at least four splits a sequence in up to three waves / this:
+// 1220 + 1987 + 1640 + 1076 keys 30.7 / 34.8 / 26.6, six of 864 to 1550 34.8 / 41.0 / 32.8, four of 8000
+// 73.7 / 71.7 / 57.3, 500 + 20000 + 3000 + 9000 73.8 / 71.7 / 61.4; one sequence (the same as the second): 1000 30.7 / 16.4, 4096 30.7 / 20.5, 40960 96.2 / 55.3.
+static int snap_split_tiles(int B, int HKV, int Nk, int max_seqlen_k) {
+  if ((int64_t)B * HKV > sn::kSms / 2) return sn::kMaxTilesManyCtas;
+  const int64_t longest = std::max(1, (max_seqlen_k + sn::kTile - 1) / sn::kTile);
+  int64_t best = longest, best_cost = INT64_MAX;
+  for (int64_t splits = 1; splits <= std::min<int64_t>(longest, sn::kSms / HKV); ++splits) {
+    const int64_t tiles = (longest + splits - 1) / splits, padded = B * ((longest + tiles - 1) / tiles);
+    const int64_t live = std::min(padded, Nk / (tiles * sn::kTile) + B);   // at most a partial split per sequence
+    const int64_t waves = (live * HKV + sn::kSms - 1) / sn::kSms;
+    const int64_t cost = waves * (4 + tiles) * sn::kSms + 3 * (padded - live) * HKV;
+    if (cost < best_cost) best_cost = cost, best = tiles;
+  }
+  return (int)best;
 }
 
-static int snap_split_tiles(int B, int HKV, int Nk, int max_seqlen_k) {
-  const int waves = snap_waves(B, HKV);
-  if (waves == 0) return sn::kMaxTilesManyCtas;
-  const int64_t longest = (max_seqlen_k + sn::kTile - 1) / sn::kTile;
-  // at least the longest sequence, so that its splits are no more than `ctas` even if max_seqlen_k exceeds Nk
-  const int64_t tiles =
-      std::max(longest, std::min<int64_t>((Nk + sn::kTile - 1) / sn::kTile + (B - 1), longest * B));
-  const int64_t ctas = waves * sn::kSms / HKV - (B - 1);
-  return (int)std::max<int64_t>(1, (tiles + ctas - 1) / ctas);
+// Tests: key tiles per CTA of such a call.
+extern "C" int cvllm_selftest_snap_split(int B, int HKV, int Nk, int max_seqlen_k) {
+  return B > 0 && HKV > 0 ? snap_split_tiles(B, HKV, Nk, max_seqlen_k) : 0;
 }
 
 size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV) {
   const size_t tiles = (size_t)(max_seqlen_k + sn::kTile - 1) / sn::kTile;
-  size_t n_splits = (tiles + sn::kMaxTilesManyCtas - 1) / sn::kMaxTilesManyCtas;
   // the most that snap_split_tiles() can make of it, whatever the total of the keys
-  if (const int waves = snap_waves(B, HKV)) n_splits = std::max(n_splits, std::min(tiles, (size_t)(waves * sn::kSms / HKV)));
+  const size_t n_splits = (int64_t)B * HKV > sn::kSms / 2 ? (tiles + sn::kMaxTilesManyCtas - 1) / sn::kMaxTilesManyCtas
+                                                          : std::min(tiles, (size_t)(sn::kSms / HKV));
   return (size_t)B * HKV * 2 * (n_splits ? n_splits : 1) * sn::kTile * 2 * sizeof(float);
 }
 
-// Launcher used by cvllm_snapkv_scores (score_attn.cu) when w * G <= 128.
 int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
                            const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nq, int Nk, int HQ, int HKV,
                            int max_seqlen_k, float scale_log2, int kpool, int pool_segment, float* out, float* stats,

@@ -400,6 +400,8 @@ int cvllm_selftest_eig(const float* gram, double* lam_out, double* vec_out, floa
 /* ------------------------------------------------------------------------
  * Self tests (device sanity for descriptor encodings; used by tests only)
  * --------------------------------------------------------------------- */
+/* Key tiles of 128 that a CTA of the SnapKV scorer takes in a call of these sizes (tests). */
+int cvllm_selftest_snap_split(int B, int HKV, int Nk, int max_seqlen_k);
 int cvllm_selftest_umma(const void* a, const void* b, float* d, int mode,
                         uint32_t lbo, uint32_t sbo, int dtype, cvllm_stream_t stream);
 

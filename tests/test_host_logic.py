@@ -110,3 +110,21 @@ def test_shape_envelope_is_checked_at_construction():
     with pytest.raises(ValueError, match="page_size 64"):
         _check_shape_envelope(NS(head_dim=128, hidden_size=4096, num_attention_heads=32, num_key_value_heads=8),
                               NS(kvcache_page_size=64, leverage_sketch_size=48))
+
+
+def test_window_scorer_cuts_short_batches_into_one_wave():
+    """CTAs of the SnapKV scorer that have keys, over calls of a few sequences: no second wave of CTAs for the sake of more
+    splits, and no more splits than the workspace holds statistics of."""
+    from compactor_vllm import _native as N
+
+    for lens, heads in (([1220, 1987, 1640, 1076], 8), ([864, 1335, 1550, 1280, 1107, 1548], 8), ([8000] * 4, 8), ([500, 20000, 3000, 9000], 8),
+                        ([2059, 1223, 2307], 8), ([8447, 6569, 3238, 9140, 3352], 4), ([40960], 8), ([1000], 8), ([300] * 9, 8)):
+        for bound in (sum(lens), max(lens)):
+            tiles = N.lib().cvllm_selftest_snap_split(len(lens), heads, sum(lens), bound)
+            live = sum(-(-n // (128 * tiles)) for n in lens) * heads
+            assert 0 < live <= 148, (lens, bound, tiles, live)
+            splits = -(-bound // (128 * tiles))
+            held = N.lib().cvllm_snapkv_scores_workspace_bytes(len(lens), bound, 4 * heads, heads, 32)
+            assert len(lens) * heads * 2 * splits * 128 * 2 * 4 <= held
+    assert N.lib().cvllm_selftest_snap_split(10, 8, 10000, 1000) == 8      # pairs enough: the fixed split
+    assert N.lib().cvllm_selftest_snap_split(1, 8, 1000, 1000) == 1
