@@ -54,6 +54,8 @@ _SIGNATURES = {
                                           _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i,
                                           _p, _sz, _p]),
     "cvllm_select_store_workspace_bytes": (_sz, [_i, _i, _i]),
+    "cvllm_select_store_topk_bounded": (_i, [_p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p, _p, _p, _p, _p,
+                                             _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _sz, _p]),
     "cvllm_select_store_topk": (_i, [_p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p, _p, _p, _p, _p,
                                      _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _sz, _p]),
     "cvllm_decode_attention_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),

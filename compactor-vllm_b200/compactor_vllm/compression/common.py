@@ -140,11 +140,11 @@ def extract_and_store_top_kv(
     ws = N.workspace(dev, ws_bytes, "select_store")
     sk_n, sk_h, _ = new_keys.stride()
     sv_n, sv_h, _ = new_vals.stride()
-    rc = L.cvllm_select_store_topk(
+    rc = L.cvllm_select_store_topk_bounded(
         N.ptr(scores), scores.stride(0), N.ptr(new_keys), N.ptr(new_vals), sk_n, sk_h, sv_n, sv_h,
         N.ptr(retain), N.ptr(cu), N.ptr(bm), N.ptr(bh_lens), N.ptr(page_table),
         N.ptr(k_cache), N.ptr(v_cache), B, N_total, H, D, int(PAGE_SIZE), page_table.shape[2],
-        new_keys.element_size(), int(bool(PAD_TO_PAGE_SIZE)), int(_RESERVED),
+        new_keys.element_size(), int(bool(PAD_TO_PAGE_SIZE)), int(_RESERVED), max_k_len,
         N.ptr(ws), ws.numel(), N.stream(dev),
     )
     N.check(rc, "cvllm_select_store_topk")

@@ -15,9 +15,9 @@
 // Every phase is a grid of (token tiles x sequences) CTAs: the keys of a 32K-token sequence are
 // 1 MB and live in L2, each pass is a few microseconds instead of a single-SM walk.  The CTA that
 // takes the last ticket of a sequence folds the global histogram into the next digit.
-// Phases 1 to 4 of sequences whose keys fit the shared memory of a cluster of up to eight CTAs (350 K keys at 8 heads) are
-// ONE kernel (sel_cluster_kernel): twelve short launches of 4 to 12 us each, one waiting for the other, were three quarters
-// of an eviction.  Longer ones take the launches.
+// Phases 1 to 4 are ONE kernel (sel_cluster_kernel) where the keys of the longest sequence fit the shared memory of a cluster
+// of up to eight CTAs (160 tiles at 8 heads: 40960 tokens, 327680 keys): twelve short launches of 4 to 12 us each, one
+// waiting for the other, were three quarters of an eviction.  Calls with a longer sequence take the launches.
 // Order everywhere: key descending, ties by ascending flat index tok*H + head, NaN above +inf.
 // Rows land in ascending token order per head (the reference's order is atomic-nondeterministic).
 #include <cooperative_groups.h>
@@ -415,6 +415,9 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
   const int tiles_b = cdiv(len, kTileTok), tpc = cdiv(tiles_b, CS);
   const int tile0 = min(rank * tpc, tiles_b), tile1 = min(tile0 + tpc, tiles_b);
   const int tok0 = tile0 * kTileTok, ntok = max(0, min(len, tile1 * kTileTok) - tok0), nkeys = ntok * H;
+  // keys in shared memory: whole tiles, all of them unless the sequence is longer than the caller's bound; the others are
+  // read again from `scores` in every pass
+  const int held = min(nkeys, keys_cap);
   // a thread keeps to one head: it takes every (stride / H)-th token
   const int stride = kClThreads / H * H, my_h = tid % H, my_tok = tid / H;
   const bool on = tid < stride;
@@ -436,19 +439,27 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
     const float* src = scores + (int64_t)(beg + tok0 + my_tok) * stride_n + my_h;
     const int64_t step = (int64_t)(stride / H) * stride_n;
 #pragma unroll 4
-    for (int i = tid; i < nkeys; i += stride, src += step) keys[i] = score_key(__float_as_uint(__ldg(src)));
+    for (int i = tid; i < held; i += stride, src += step) keys[i] = score_key(__float_as_uint(__ldg(src)));
   }
+  auto far_key = [&](int i) {
+    return score_key(__float_as_uint(__ldg(scores + (int64_t)(beg + tok0 + i / H) * stride_n + i % H)));
+  };
+  auto each_key = [&](auto use) {   // all keys of this thread
+    int i = tid;
+#pragma unroll 4
+    for (; i < held; i += stride) use(keys[i]);
+    if (nkeys > held)
+#pragma unroll 1
+      for (; i < nkeys; i += stride) use(far_key(i));
+  };
   for (int i = tid; i < 256 * 32; i += kClThreads) col[i] = 0;
   __syncthreads();
   // counts of digit `shift` of the keys that match (prefix, mask); pre: this thread's head's prefix
   auto count = [&](uint32_t pre, uint32_t mask, int shift, bool want) {
-    if (on && want) {
-#pragma unroll 4
-      for (int i = tid; i < nkeys; i += stride) {
-        const uint32_t key = keys[i];
+    if (on && want)
+      each_key([&](uint32_t key) {
         if ((key & mask) == pre) atomicAdd(&col[((key >> shift) & 255u) * 32 + my_col], 1u);
-      }
-    }
+      });
     __syncthreads();
   };
   // columns -> per-head counts (dst) and, where asked, counts over all heads (all); the columns are zero afterwards
@@ -508,10 +519,10 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
   {
     uint32_t gt = 0, tie = 0;
     if (on)
-      for (int i = tid; i < nkeys; i += stride) {
-        gt += keys[i] > prefix;
-        tie += keys[i] == prefix;
-      }
+      each_key([&](uint32_t key) {
+        gt += key > prefix;
+        tie += key == prefix;
+      });
     if (gt) atomicAdd(&s_gt[my_h], gt);
     if (tie) atomicAdd(&s_tie[my_h], tie);
   }
@@ -542,7 +553,7 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
       uint32_t seen = 0;
       for (int base = 0; base < nkeys && seen < need; base += kClThreads) {
         const int i = base + tid;
-        const bool tie = i < nkeys && keys[i] == prefix;
+        const bool tie = i < nkeys && (i < held ? keys[i] : far_key(i)) == prefix;
         int tot;
         const uint32_t at = seen + block_excl_count(tie, s_warp, tot);
         if (tie && at < need) atomicAdd(&s_sel[i % H], 1u);
@@ -607,12 +618,20 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
     uint32_t gt = 0, tie = 0;
     if (sub < subs) {
       const uint32_t thr = s_prefix[h];
-      const uint32_t* kt = keys + (t - tile0) * kTileTok * H + h;
-      const int n = min(kTileTok, len - t * kTileTok);
-      for (int i = sub; i < n; i += subs) {
-        const uint32_t key = kt[i * H];
-        gt += key > thr;
-        tie += key == thr;
+      const int first = (t - tile0) * kTileTok * H + h, n = min(kTileTok, len - t * kTileTok);
+      if (first < held) {   // whole tiles are held
+        for (int i = sub; i < n; i += subs) {
+          const uint32_t key = keys[first + i * H];
+          gt += key > thr;
+          tie += key == thr;
+        }
+      } else {
+#pragma unroll 1
+        for (int i = sub; i < n; i += subs) {
+          const uint32_t key = far_key(first + i * H);
+          gt += key > thr;
+          tie += key == thr;
+        }
       }
     }
     uint32_t gs = gt, ts = tie;   // lanes h, h + H, ..: the tile's counts of head h
@@ -809,13 +828,13 @@ static void launch_sel_gather(dim3 grid, cudaStream_t st, const float* scores, i
              (const uint4*)vals, sk_n, sk_h, sv_n, sv_h, cu, bm, pt, bh_lens, (uint4*)kc, (uint4*)vc, H, PS, NLP, w);
 }
 
-extern "C" int cvllm_select_store_topk(const float* scores, int64_t s_stride_n, const void* keys,
+extern "C" int cvllm_select_store_topk_bounded(const float* scores, int64_t s_stride_n, const void* keys,
                                        const void* vals, int64_t sk_n, int64_t sk_h, int64_t sv_n,
                                        int64_t sv_h, const int32_t* num_retain,
                                        const int32_t* cu_seqlens_k, const int32_t* batch_mapping,
                                        int32_t* bh_lens, const int32_t* page_table, void* k_cache,
                                        void* v_cache, int B, int N, int HKV, int D, int PS, int NLP,
-                                       int elem_bytes, int pad_to_page, int reserved_batch,
+                                       int elem_bytes, int pad_to_page, int reserved_batch, int max_len,
                                        void* workspace, size_t workspace_bytes, cvllm_stream_t stream) {
   CVLLM_CHECK_ARG(B > 0 && N >= 0 && HKV > 0 && D > 0 && PS > 0 && NLP > 0);
   CVLLM_CHECK_ARG(scores && keys && vals && num_retain && cu_seqlens_k && batch_mapping && bh_lens &&
@@ -845,11 +864,19 @@ extern "C" int cvllm_select_store_topk(const float* scores, int64_t s_stride_n, 
   w.tiles = l.tiles;
   auto st = static_cast<cudaStream_t>(stream);
   const dim3 grid((N + kTileTok - 1) / kTileTok, B);
-  // One cluster per sequence while its share of the keys (a sequence may be all of N) fits a CTA's shared memory; smaller
-  // clusters for fewer keys: an exchange costs more than 16 K keys less per CTA save.
+  // One cluster per sequence while its share of the longest sequence's keys fits a CTA's shared memory; smaller clusters
+  // for fewer keys: an exchange costs more than 16 K keys less per CTA save.  While all CTAs take up to 0.7 of the SMs,
+  // which the others would only leave idle, twice as many for half the keys is the better trade; beyond that a CTA,
+  // which fills its SM, waits for another (clusters of eight for each of many short sequences ran in waves).  Whole
+  // evictions in a graph, 8 heads, chain of launches / clusters by N alone / this, us:
+  // 128 of 100 tokens 166 / 230 / 71, 64 of 500 217 / 196 / 102, 25 of 1000 162 / 121 / 96, 16 of 3000 180 / 180 / 109,
+  // 12 of 6000 190 / 190 / 119, 8 of 4000 146 / 98 / 96, one of 32768 118 / 88 / 88.
+  const int longest = min(max(max_len, 1), N);
+  auto room = [&](int c) { return c < 8 && 20 * (int64_t)B * c <= 7 * (int64_t)sm_count(); };
   int cluster = 1;
-  while (cluster < 8 && (int64_t)N * HKV > (int64_t)cluster * 16384) cluster *= 2;
-  const int tiles_per_cta = cdiv((int)grid.x, cluster);
+  while (cluster < 8 && (int64_t)longest * HKV > (int64_t)cluster * 16384) cluster *= 2;
+  while (room(cluster) && (int64_t)N * HKV > (int64_t)cluster * 16384) cluster *= 2;
+  const int tiles_per_cta = cdiv(cdiv(longest, kTileTok), cluster);
   const size_t cl_smem = sel_cluster_smem(tiles_per_cta, HKV);
   constexpr size_t kClSmemMax = 226 * 1024;   // beside the static arrays
   if (cl_smem <= kClSmemMax && test_options().select_passes.load() == 0) {
@@ -906,4 +933,17 @@ extern "C" int cvllm_select_store_topk(const float* scores, int64_t s_stride_n, 
 #undef G
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
+}
+
+extern "C" int cvllm_select_store_topk(const float* scores, int64_t s_stride_n, const void* keys,
+                                       const void* vals, int64_t sk_n, int64_t sk_h, int64_t sv_n,
+                                       int64_t sv_h, const int32_t* num_retain,
+                                       const int32_t* cu_seqlens_k, const int32_t* batch_mapping,
+                                       int32_t* bh_lens, const int32_t* page_table, void* k_cache,
+                                       void* v_cache, int B, int N, int HKV, int D, int PS, int NLP,
+                                       int elem_bytes, int pad_to_page, int reserved_batch,
+                                       void* workspace, size_t workspace_bytes, cvllm_stream_t stream) {
+  return cvllm_select_store_topk_bounded(scores, s_stride_n, keys, vals, sk_n, sk_h, sv_n, sv_h, num_retain, cu_seqlens_k,
+                                         batch_mapping, bh_lens, page_table, k_cache, v_cache, B, N, HKV, D, PS, NLP,
+                                         elem_bytes, pad_to_page, reserved_batch, N, workspace, workspace_bytes, stream);
 }

@@ -244,8 +244,21 @@ int cvllm_prefill_store_topk_idx(const void* keys, const void* vals,
  * radix-select (global top num_retain[b], then per-head top n_h) -> gather
  * into the paged cache.  Same kept sets as rank + store_topk_idx with the full
  * ranking (top_k >= max_len*H, the engine's setting, utils/arguments.py
- * :208-211). */
+ * :208-211).
+ * The _bounded form takes max_len, the tokens of the longest sequence: the selection is laid out for it (a cluster of CTAs
+ * per sequence that holds max_len tokens' keys, or a chain of launches where none does).  A sequence that is longer than
+ * max_len after all gets the same result, slower; without the bound every sequence is taken to be as long as all N. */
 size_t cvllm_select_store_workspace_bytes(int B, int H, int N);
+int cvllm_select_store_topk_bounded(const float* scores, int64_t s_stride_n,
+                                    const void* keys, const void* vals,
+                                    int64_t sk_n, int64_t sk_h, int64_t sv_n, int64_t sv_h,
+                                    const int32_t* num_retain, const int32_t* cu_seqlens_k,
+                                    const int32_t* batch_mapping, int32_t* bh_lens,
+                                    const int32_t* page_table, void* k_cache, void* v_cache,
+                                    int B, int N, int HKV, int D, int PS, int NLP,
+                                    int elem_bytes, int pad_to_page, int reserved_batch, int max_len,
+                                    void* workspace, size_t workspace_bytes,
+                                    cvllm_stream_t stream);
 int cvllm_select_store_topk(const float* scores, int64_t s_stride_n,
                             const void* keys, const void* vals,
                             int64_t sk_n, int64_t sk_h, int64_t sv_n, int64_t sv_h,

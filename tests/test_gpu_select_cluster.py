@@ -25,7 +25,7 @@ def scores_of(kind, n, H, g):
     return s
 
 
-def evict(scores, lens, retain, H, wide, slots, pad, option):
+def evict(scores, lens, retain, H, wide, slots, pad, option, max_len=None):
     from compactor_vllm import _native as N
     from compactor_vllm.compression.common import extract_and_store_top_kv
 
@@ -45,7 +45,7 @@ def evict(scores, lens, retain, H, wide, slots, pad, option):
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     N.set_test_option("select_passes", option)
     try:
-        extract_and_store_top_kv(scores=buf[:, :H], cu_seqlens_k=i32(cu), max_k_len=max(lens), top_k=max(lens) * H, H=H,
+        extract_and_store_top_kv(scores=buf[:, :H], cu_seqlens_k=i32(cu), max_k_len=max_len or max(lens), top_k=max(lens) * H, H=H,
                                  new_keys=k, new_vals=v, num_tokens_to_retain=i32(retain), page_table=table,
                                  batch_mapping=i32(slots), bh_lens=lens0, k_cache=kc, v_cache=vc, PAGE_SIZE=PS,
                                  PAD_TO_PAGE_SIZE=pad)
@@ -85,5 +85,40 @@ def test_where_the_clusters_end(n, H):
     scores = scores_of("random", n, H, g)
     a = evict(scores, [n], [n * H // 4], H, False, [1], True, 0)
     b = evict(scores, [n], [n * H // 4], H, False, [1], True, 1)
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+
+
+def launches(scores, lens, H, **kw):
+    from compactor_vllm import _native as N
+
+    count = N.lib().cvllm_launch_count
+    before = count()
+    out = evict(scores, lens, [n * H // 2 for n in lens], H, False, list(range(1, len(lens) + 1)), True, 0, **kw)
+    return count() - before, out
+
+
+def test_the_longest_sequence_chooses_the_path():
+    """Sequences that each fit a cluster take the two launches whatever their number; one that does not, the chain."""
+    g = torch.Generator().manual_seed(3)
+    for lens, want in (([6000] * 12, 2), ([40960, 300], 2), ([41216, 300], 13), ([200] * 300, 2)):
+        scores = scores_of("random", sum(lens), 8, g)
+        n, got = launches(scores, lens, 8)
+        assert n == want, (lens[0], len(lens), n)
+        chain = evict(scores, lens, [x * 4 for x in lens], 8, False, list(range(1, len(lens) + 1)), True, 1)
+        for x, y in zip(got, chain):
+            assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("kind", ["random", "ties", "special"])
+@pytest.mark.parametrize("H,bound", [(8, 1), (8, 300), (8, 5000), (3, 256), (16, 2049)])
+def test_sequences_longer_than_the_bound(H, bound, kind):
+    """max_k_len below the longest sequence: keys beyond a cluster's share are read where they are, with the same result."""
+    lens = [700, 9001, 256, 0, 2300]
+    g = torch.Generator().manual_seed(H + bound)
+    scores = scores_of(kind, sum(lens), H, g)
+    retain, slots = [n * H // 3 for n in lens], [1, 2, 3, 4, 5]
+    a = evict(scores, lens, retain, H, True, slots, True, 0, max_len=bound)
+    b = evict(scores, lens, retain, H, True, slots, True, 1)
     for x, y in zip(a, b):
         assert torch.equal(x, y)
