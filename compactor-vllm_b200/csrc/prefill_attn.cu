@@ -437,7 +437,7 @@ using namespace cvllm;
 int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                           const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, void* out,
                           const int32_t* seq_lens_bh, const int32_t* page_table,
-                          const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int HQ,
+                          const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ,
                           int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q,
                           float scale_log2, float rescale_threshold, bool bf16, cudaStream_t st);
 
@@ -504,7 +504,7 @@ extern "C" int cvllm_prefill_attention(const void* q, const void* k, const void*
   // (prefill_attn2.cu).  Test option "prefill_v1" forces the one-head-per-CTA kernel (tests cover both).
   if ((HQ / HKV) % 2 == 0 && !test_options().prefill_v1.load(std::memory_order_relaxed))
     return cvllm_launch_prefill2(tm_q, tm_k, tm_v, tm_kc, tm_vc, out, seq_lens_bh, page_table,
-                                 batch_mapping, cu_seqlens_q, B, HQ, HKV, PS, NLP, o_stride_n,
+                                 batch_mapping, cu_seqlens_q, B, N, HQ, HKV, PS, NLP, o_stride_n,
                                  max_seqlen_q, p.scale_log2, p.rescale_threshold, bf16, st);
   const size_t smem = sizeof(PrefillSmem) + 1024;
   const dim3 grid((max_seqlen_q + kBM - 1) / kBM, HQ, B);

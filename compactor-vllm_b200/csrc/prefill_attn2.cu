@@ -121,7 +121,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (a form of its own for each order: with the choice at run time the loop below it ran 1 % slower at 32768 tokens)
   TileOrder at;
-  if constexpr (BY_TILE) at = tile_order(p.seq_lens_bh, kBM);
+  if constexpr (BY_TILE) at = tile_order(p.seq_lens_bh, p.B * p.HKV, kBM);
   const int b = BY_TILE ? at.b : blockIdx.z;
   const int hq0 = 2 * (BY_TILE ? at.pair : blockIdx.y);  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
@@ -490,7 +490,7 @@ using namespace cvllm;
 int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                           const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, void* out,
                           const int32_t* seq_lens_bh, const int32_t* page_table,
-                          const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int HQ,
+                          const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ,
                           int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q,
                           float scale_log2, float rescale_threshold, bool bf16, cudaStream_t st) {
   Prefill2Params p;
@@ -502,7 +502,7 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
   p.rescale_threshold = rescale_threshold;
   const size_t smem = sizeof(Prefill2Smem) + 1024;
   const dim3 grid((max_seqlen_q + p2::kBM - 1) / p2::kBM, HQ / 2, B);
-  const bool by_tile = order_by_tile(grid.x, grid.y, grid.z);
+  const bool by_tile = order_by_tile(grid, N, p2::kBM);
   auto launch = [&](auto kernel, std::atomic<uint64_t>& attr) -> int {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)kernel, (int)smem, attr));
     kernel<<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
@@ -525,3 +525,27 @@ extern "C" int cvllm_debug_prefill_trace_read(void* host_out) {
   return CVLLM_OK;
 }
 #endif
+
+namespace cvllm {
+__global__ void tile_order_kernel(const int32_t* past, int n, int by_tile, int tile_rows, int32_t* out) {
+  TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
+  if (by_tile) at = tile_order(past, n, tile_rows);
+  if (threadIdx.x == 0) {
+    int32_t* o = out + 3 * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+    o[0] = at.qt;
+    o[1] = at.pair;
+    o[2] = at.b;
+  }
+}
+}  // namespace cvllm
+
+// Tests: the order that a launch of (tiles, pairs, seqs) CTAs over `tokens` new tokens takes.
+extern "C" int cvllm_selftest_tile_order(const int32_t* past, int n, int tiles, int pairs, int seqs, int tokens,
+                                         int tile_rows, int32_t* out, int* by_tile, cvllm_stream_t stream) {
+  CVLLM_CHECK_ARG(past && n > 0 && tiles > 0 && pairs > 0 && seqs > 0 && tokens >= 0 && tile_rows > 0 && out && by_tile);
+  const dim3 grid(tiles, pairs, seqs);
+  *by_tile = order_by_tile(grid, tokens, tile_rows);
+  tile_order_kernel<<<grid, 32, 0, static_cast<cudaStream_t>(stream)>>>(past, n, *by_tile, tile_rows, out);
+  CVLLM_CHECK_LAUNCH();
+  return CVLLM_OK;
+}

@@ -60,6 +60,7 @@ struct PrefillBiasParams {
   const float* sink_logits;   // [HQ] the sink's score per head, or NULL (score 0)
   const float* dist_bias;     // [dist_rows][HQ] added to the score by distance (the last row beyond), DIST only
   int dist_rows;
+  bool by_tile;               // the order of the query tiles (tile_order.cuh)
 };
 
 template <int HD, bool DIST>
@@ -142,7 +143,7 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
-  if (order_by_tile(gridDim.x, gridDim.y, gridDim.z)) at = tile_order(p.seq_start, kBM);
+  if (p.by_tile) at = tile_order(p.seq_start, p.B, kBM);
   const int b = at.b;
   const int hq0 = 2 * at.pair;  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
@@ -639,6 +640,7 @@ int cvllm_launch_prefill_bias(const void* q, const void* k_cache, const void* v_
   p.sink_logits = sink ? sink_logits : nullptr;
   p.dist_bias = dist_bias;
   p.dist_rows = dist_rows;
+  p.by_tile = order_by_tile(dim3((max_seqlen_q + kBM - 1) / kBM, HQ / 2, B), N, kBM);
   if (HD == 64)
     return dist_bias ? launch_bias<64, true, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st)
                      : launch_bias<64, false, true>(tm_q, tm_kc, tm_vc, p, max_seqlen_q, st);

@@ -413,6 +413,11 @@ int cvllm_selftest_eig(const float* gram, double* lam_out, double* vec_out, floa
 /* ------------------------------------------------------------------------
  * Self tests (device sanity for descriptor encodings; used by tests only)
  * --------------------------------------------------------------------- */
+/* The order in which the prefill kernels' CTAs take their query tiles (csrc/tile_order.cuh; tests): for a grid of
+ * (tiles, pairs, seqs) over `tokens` new tokens in tiles of tile_rows rows, with the pasts [n] on the device:
+ * out[3 * cta] = tile, pair, sequence; *by_tile = whether such a launch looks at the pasts at all. */
+int cvllm_selftest_tile_order(const int32_t* past, int n, int tiles, int pairs, int seqs, int tokens, int tile_rows,
+                              int32_t* out, int* by_tile, cvllm_stream_t stream);
 /* Key tiles of 128 that a CTA of the SnapKV scorer takes in a call of these sizes (tests). */
 int cvllm_selftest_snap_split(int B, int HKV, int Nk, int max_seqlen_k);
 int cvllm_selftest_umma(const void* a, const void* b, float* d, int mode,

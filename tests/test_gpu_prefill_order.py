@@ -43,3 +43,37 @@ def test_order_changes_nothing(dtype, new, past, calls):
     for call in calls[1:]:
         for i, o in _run(call, new, past, pools).items():
             assert torch.equal(o, want[i]), i
+
+
+def _order(past, tiles, pairs, seqs, tokens):
+    """What the CTAs of a launch take, (tile, pair, sequence) each in launch order, and whether the rule looked at the pasts."""
+    import ctypes
+    from compactor_vllm import _native as N
+
+    p = torch.tensor(past, dtype=torch.int32, device=DEV)
+    out = torch.full((tiles * pairs * seqs, 3), -1, dtype=torch.int32, device=DEV)
+    by_tile = ctypes.c_int()
+    N.check(N.lib().cvllm_selftest_tile_order(N.ptr(p), p.numel(), tiles, pairs, seqs, tokens, 128, N.ptr(out),
+                                              ctypes.byref(by_tile), N.stream(p.device)), "cvllm_selftest_tile_order")
+    return [tuple(x) for x in out.tolist()], bool(by_tile.value)
+
+
+def test_the_order_does_not_depend_on_which_sequence_is_first():
+    """The same batch in another order of its sequences takes the same schedule; every CTA gets a tile of its own."""
+    tiles, pairs, seqs = 16, 8, 5
+    everything = {(t, p, b) for t in range(tiles) for p in range(pairs) for b in range(seqs)}
+    for past in ([0, 8000, 8000, 8000, 8000], [0, 0, 0, 0, 4000], [1023] * 5, [1025] * 5):
+        kinds = set()
+        for turn in range(seqs):
+            got, looked = _order(past[turn:] + past[:turn], tiles, pairs, seqs, tiles * 128 * seqs)
+            assert looked and set(got) == everything
+            kinds.add([t for t, _, _ in got] == sorted((t for t, _, _ in got), reverse=True))   # by tiles?
+        assert kinds == {2 * sum(past) <= seqs * tiles * 128}, past
+
+
+def test_tiles_past_the_end_of_short_sequences_do_not_count():
+    """4000 + 2077 + 911 + 3301 tokens, 16 pairs: 2048 CTAs in the grid, at most (80 + 4) * 16 = 1344 with work."""
+    n = 4000 + 2077 + 911 + 3301
+    assert _order([0] * 4, 32, 16, 4, n)[1]
+    assert not _order([0] * 4, 32, 16, 4, 32 * 128 * 4)[1]
+    assert not _order([0], 9, 16, 1, 1100)[1]     # one wave
