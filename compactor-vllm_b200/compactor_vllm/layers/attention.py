@@ -255,11 +255,12 @@ class BiasedChunkAttention(nn.Module):
         return other
 
     def _field(self, name: str):
-        """A parameter, buffer or plain attribute by name, past Module.__getattr__ (0.5 us a name, and a step reads eight)."""
-        value = self._parameters.get(name)
-        if value is None:
-            value = self._buffers.get(name)
-        return self.__dict__.get(name) if value is None else value
+        """A parameter, buffer or plain attribute by name, past Module.__getattr__ (0.5 us a name, and a step reads eight).  A
+        name that is none of these (a parametrized one is a property of the class) goes the usual way."""
+        for held in (self._parameters, self._buffers, self.__dict__):
+            if name in held:
+                return held[name]
+        return getattr(self, name)
 
     @torch.no_grad()
     def refresh_distance_bias(self, rel: Optional[torch.Tensor] = None) -> None:

@@ -128,3 +128,27 @@ def test_window_scorer_cuts_short_batches_into_one_wave():
             assert len(lens) * heads * 2 * splits * 128 * 2 * 4 <= held
     assert N.lib().cvllm_selftest_snap_split(10, 8, 10000, 1000) == 8      # pairs enough: the fixed split
     assert N.lib().cvllm_selftest_snap_split(1, 8, 1000, 1000) == 1
+
+
+def test_fields_of_a_parametrized_attention():
+    """The attention's shortcut past Module.__getattr__ finds what the attribute finds, a parametrized weight too."""
+    import torch
+    from torch.nn.utils import parametrize
+
+    from compactor_vllm.layers.attention import BiasedChunkAttention
+
+    class Twice(torch.nn.Module):
+        def forward(self, x):
+            return 2 * x
+
+    m = BiasedChunkAttention(4, 2, 64, 64, 0.125, qk_norm=True, sink=True, learned_sink=True, bucket_bias=(8, 64))
+    names = ("inv_freq", "q_norm_weight", "k_norm_weight", "dist_bias", "rel", "slopes", "sink_logits")
+    for name in names:
+        assert m._field(name) is getattr(m, name), name
+    for name in ("q_norm_weight", "sink_logits"):
+        parametrize.register_parametrization(m, name, Twice())
+        with torch.no_grad():
+            m.parametrizations[name].original.fill_(3.0)
+        assert torch.equal(m._field(name), getattr(m, name)) and (m._field(name) == 6.0).all(), name
+    for name in names:
+        assert (m._field(name) is None) == (getattr(m, name) is None), name
