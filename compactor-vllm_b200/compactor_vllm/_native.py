@@ -233,9 +233,10 @@ _WORKSPACES: dict = {}
 
 
 @functools.lru_cache(maxsize=4096)
-def sized(name: str, *sizes: int) -> int:
-    """A size function of the library (its result depends on nothing but its arguments), remembered per argument list."""
-    return getattr(lib(), name)(*sizes)
+def sized(device: int, name: str, *sizes: int) -> int:
+    """A size function of the library, remembered per device (its number of SMs decides how a call is split) and arguments."""
+    with torch.cuda.device(device):
+        return getattr(lib(), name)(*sizes)
 
 
 def workspace(device: torch.device, nbytes: int, tag="", zero: bool = False) -> torch.Tensor:

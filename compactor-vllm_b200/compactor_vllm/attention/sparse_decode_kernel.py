@@ -57,7 +57,7 @@ def head_sparse_decode_attention(
     if B == 0:
         return out
     L = N.lib()
-    ws_bytes = N.sized("cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
+    ws_bytes = N.sized(dev.index, "cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
     # one workspace per (B, HQ, HKV): the ticket region's size depends on B*HKV, and the "zero on
     # entry, zero on exit" contract only holds while the layout stays the same
     ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
@@ -104,7 +104,7 @@ def decode_append_and_attend(
     if B == 0:
         return out
     L = N.lib()
-    ws_bytes = N.sized("cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
+    ws_bytes = N.sized(dev.index, "cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
     ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
     rc = L.cvllm_decode_step(
         N.ptr(key), N.ptr(value), key.stride(0), key.stride(1), value.stride(0), value.stride(1),

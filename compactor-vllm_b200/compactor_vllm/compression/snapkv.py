@@ -68,7 +68,7 @@ def query_aware_key_scores(
     out = torch.empty((N_k, Hk), dtype=torch.float32, device=dev)
     cu_q, cu_k = N.index_tensor(cu_seqlens_q, dev), N.index_tensor(cu_seqlens_k, dev)
     L = N.lib()
-    ws_bytes = N.sized("cvllm_snapkv_scores_workspace_bytes", B, N_k, Hq, Hk, w)
+    ws_bytes = N.sized(dev.index, "cvllm_snapkv_scores_workspace_bytes", B, N_k, Hq, Hk, w)
     ws = N.workspace(dev, ws_bytes, "snapkv")
     rc = L.cvllm_snapkv_scores(
         N.ptr(q), N.ptr(k), q.stride(0), k.stride(0), N.ptr(cu_q), N.ptr(cu_k), w, B, N_k, Hq, Hk,

@@ -400,7 +400,7 @@ class BiasedChunkAttention(nn.Module):
             max_keys = int(ctx.max_seqlen_k)
             if (self.streaming_decode_kernel(max_keys, T) and o_stride % 2 == 0 and out.data_ptr() % 4 == 0
                     and (q.data_ptr() | self.k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
-                ws = N.workspace(dev, N.sized("cvllm_bias_decode_workspace_bytes", T, H, G, D), "bias_attn_stream")
+                ws = N.workspace(dev, N.sized(dev.index, "cvllm_bias_decode_workspace_bytes", T, H, G, D), "bias_attn_stream")
                 N.check(lib.cvllm_bias_attn_decode_stream(
                     N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), self.k_cache.shape[0], *table, N.ptr(ctx.positions_i32),
                     N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),

@@ -36,7 +36,6 @@ constexpr int kSlots = 4;
 constexpr int kThreads = 384;
 constexpr int kRegsSoftmax = 224, kRegsOther = 56;
 constexpr int kMaxTilesManyCtas = 8;  // key tiles per CTA where (sequence, head) pairs alone fill the chip
-constexpr int kSms = 148;
 }  // namespace sn
 
 struct SnapUmmaParams {
@@ -308,14 +307,15 @@ using namespace cvllm;
 // 1220 + 1987 + 1640 + 1076 keys 30.7 / 34.8 / 26.6, six of 864 to 1550 34.8 / 41.0 / 32.8, four of 8000
 // 73.7 / 71.7 / 57.3, 500 + 20000 + 3000 + 9000 73.8 / 71.7 / 61.4; one sequence (the same as the second): 1000 30.7 / 16.4, 4096 30.7 / 20.5, 40960 96.2 / 55.3.
 static int snap_split_tiles(int B, int HKV, int Nk, int max_seqlen_k) {
-  if ((int64_t)B * HKV > sn::kSms / 2) return sn::kMaxTilesManyCtas;
+  const int sms = sm_count();
+  if ((int64_t)B * HKV > sms / 2) return sn::kMaxTilesManyCtas;
   const int64_t longest = std::max(1, (max_seqlen_k + sn::kTile - 1) / sn::kTile);
   int64_t best = longest, best_cost = INT64_MAX;
-  for (int64_t splits = 1; splits <= std::min<int64_t>(longest, sn::kSms / HKV); ++splits) {
+  for (int64_t splits = 1; splits <= std::min<int64_t>(longest, sms / HKV); ++splits) {
     const int64_t tiles = (longest + splits - 1) / splits, padded = B * ((longest + tiles - 1) / tiles);
     const int64_t live = std::min(padded, Nk / (tiles * sn::kTile) + B);   // at most a partial split per sequence
-    const int64_t waves = (live * HKV + sn::kSms - 1) / sn::kSms;
-    const int64_t cost = waves * (4 + tiles) * sn::kSms + 3 * (padded - live) * HKV;
+    const int64_t waves = (live * HKV + sms - 1) / sms;
+    const int64_t cost = waves * (4 + tiles) * sms + 3 * (padded - live) * HKV;
     if (cost < best_cost) best_cost = cost, best = tiles;
   }
   return (int)best;
@@ -328,9 +328,10 @@ extern "C" int cvllm_selftest_snap_split(int B, int HKV, int Nk, int max_seqlen_
 
 size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV) {
   const size_t tiles = (size_t)(max_seqlen_k + sn::kTile - 1) / sn::kTile;
+  const int sms = sm_count();
   // the most that snap_split_tiles() can make of it, whatever the total of the keys
-  const size_t n_splits = (int64_t)B * HKV > sn::kSms / 2 ? (tiles + sn::kMaxTilesManyCtas - 1) / sn::kMaxTilesManyCtas
-                                                          : std::min(tiles, (size_t)(sn::kSms / HKV));
+  const size_t n_splits = (int64_t)B * HKV > sms / 2 ? (tiles + sn::kMaxTilesManyCtas - 1) / sn::kMaxTilesManyCtas
+                                                          : std::min(tiles, (size_t)(sms / HKV));
   return (size_t)B * HKV * 2 * (n_splits ? n_splits : 1) * sn::kTile * 2 * sizeof(float);
 }
 

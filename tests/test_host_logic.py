@@ -152,3 +152,30 @@ def test_fields_of_a_parametrized_attention():
         assert torch.equal(m._field(name), getattr(m, name)) and (m._field(name) == 6.0).all(), name
     for name in names:
         assert (m._field(name) is None) == (getattr(m, name) is None), name
+
+
+def test_remembered_sizes_are_per_device(monkeypatch):
+    """A size that depends on the device's number of SMs is asked for once per device, on that device."""
+    import contextlib
+
+    from compactor_vllm import _native as N
+
+    at, asked = [0], []
+
+    class Library:
+        def bytes(self, n):
+            asked.append((at[0], n))
+            return n * (100, 148)[at[0]]
+
+    @contextlib.contextmanager
+    def device(index):
+        before, at[0] = at[0], index
+        yield
+        at[0] = before
+
+    monkeypatch.setattr(N, "lib", Library)
+    monkeypatch.setattr(N.torch.cuda, "device", device)
+    N.sized.cache_clear()
+    assert [N.sized(0, "bytes", 2), N.sized(1, "bytes", 2), N.sized(0, "bytes", 2), N.sized(1, "bytes", 3)] == [200, 296, 200, 444]
+    assert asked == [(0, 2), (1, 2), (1, 3)]
+    N.sized.cache_clear()
