@@ -318,13 +318,19 @@ class BiasedChunkAttention(nn.Module):
         that a query may see (kept first tokens among them) are two of its units of 128 or more.  It reads the cache at the
         rate of the plain decode kernel but has a prologue, and a fold behind it.  Layer step with norms and cache write in
         a graph, 32 / 8 heads of 128 (streaming / key splits): 8 x 4096 keys 37 / 104 us, 8 x 200 14 / 21, 1 x 200 13 / 20,
-        32 x 200 25 / 31; heads of 64, 32 sequences: up to 140 keys 19 / 14 us, up to 280 keys 21.2 / 21.3."""
+        32 x 200 25 / 31.  Heads of 64, whose rows are short beside the prologue, want more keys when there are more heads than
+        CTAs (L2 flushed): 32 sequences at 260 keys 30.7 / 26.6, at 320 28.7 / 28.7, 64 sequences at 320 38.9 / 34.8, at 512
+        45.1 / 45.1; up to 16 sequences the streaming kernel is level or ahead from 256 keys on.
+        A captured step is chosen by its bound `max_keys` and replayed at any length, where the splits are those of the bound
+        too: with 8192 or more the streaming kernel is level or ahead at every length (32 sequences, heads of 64: 100 keys
+        26.6 / 34.8, 4000 keys 98 / 154), with 2048 it is behind at short ones (100 keys 26.6 / 22.5, 1000 keys 43 / 59)."""
         keys = min(max_keys, self.chunk) if self.chunk else max_keys
         if self.window:
             keys = min(keys, self.window)
         keys = min(keys + self.keep_first, max_keys)
         D, page = self.head_dim, int(self.page_size)
-        return (keys >= 256 and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
+        least = 256 if D != 64 else min(max(256, batch * self.num_kv_heads + 64), 512)
+        return (keys >= least and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
                 and self.num_heads // self.num_kv_heads <= 8 and batch * self.num_kv_heads <= 4096
                 and self.k_cache.dtype == torch.bfloat16 and (page % 128 == 0 or page in (16, 32, 64)))
 

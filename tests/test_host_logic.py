@@ -179,3 +179,21 @@ def test_remembered_sizes_are_per_device(monkeypatch):
     assert [N.sized(0, "bytes", 2), N.sized(1, "bytes", 2), N.sized(0, "bytes", 2), N.sized(1, "bytes", 3)] == [200, 296, 200, 444]
     assert asked == [(0, 2), (1, 2), (1, 3)]
     N.sized.cache_clear()
+
+
+def test_heads_of_64_stream_from_where_it_pays():
+    import torch
+
+    from compactor_vllm.layers.attention import BiasedChunkAttention
+
+    def choice(heads, kv, dim, keys, batch, **kw):
+        m = BiasedChunkAttention(heads, kv, dim, dim, dim ** -0.5, **kw)
+        m.k_cache, m.page_size = torch.empty(0, dim, dtype=torch.bfloat16), 128
+        return m.streaming_decode_kernel(keys, batch)
+
+    assert [choice(32, 8, 64, 256, b) for b in (1, 16, 24, 25, 32)] == [True, True, True, False, False]
+    assert [choice(32, 8, 64, k, 32) for k in (319, 320)] == [False, True]
+    assert [choice(32, 8, 64, k, 512) for k in (511, 512)] == [False, True]
+    assert choice(32, 8, 128, 256, 512) and not choice(32, 8, 128, 255, 1)
+    assert not choice(32, 8, 128, 4096, 513)          # more heads than its split covers
+    assert choice(32, 8, 128, 4096, 1, window=128, keep_first=128) and not choice(32, 8, 128, 4096, 1, window=128)
