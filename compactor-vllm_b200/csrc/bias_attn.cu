@@ -1388,8 +1388,15 @@ extern "C" int cvllm_bias_attn_varlen_dist(const void* q, const void* k_cache, c
                              out_stride, B, max_new, H, G, D, Dv, st)
   // 0 product, 1 fp32 FMA kernel, 2 no tcgen05 kernel, 3 the latent tcgen05 kernel wherever it serves
   const int path = test_options().bias_attn_fma.load();
+  const bool latent = dtype == CVLLM_BF16 && G == 1 && v_cache == k_cache && v_stride == D && slopes == nullptr &&
+                      dist_bias == nullptr && cache_rows > 0 && (path == 0 || path == 3) &&
+                      cvllm_latent_attn_umma_serves(D, Dv, page_size, out_stride, q, k_cache, out);
+  // Heads of 64 that are their own values are served by both tcgen05 kernels.  The one for latent rows packs all heads'
+  // queries into its tiles and is ahead while those are one wave (us, latent / this one): 8 heads, 300 tokens 14.3 / 18.4,
+  // 2000 43.0 / 47.1, 4096 103 / 82; 32 heads, 300 tokens 16.4 / 18.4, 600 24.6 / 22.5, 4096 285 / 156.
+  const bool one_wave = latent && D == 64 && ((int64_t)total_tokens * H + 127) / 128 <= sm_count();
   // (buffers off the 16-byte grid: whole tiles of 128-wide heads refuse them, the shapes around those take mma.sync)
-  if (dtype == CVLLM_BF16 && cvllm_prefill_bias_serves(D, Dv, page_size, dist_bias ? dist_rows : 0) && v_stride == Dv &&
+  if (!one_wave && dtype == CVLLM_BF16 && cvllm_prefill_bias_serves(D, Dv, page_size, dist_bias ? dist_rows : 0) && v_stride == Dv &&
       (H / G) % 2 == 0 && path == 0 && out_stride % 8 == 0 &&
       ((D == 128 && page_size % 128 == 0 && dist_bias == nullptr) ||
        (aligned16(q) && aligned16(out) && aligned16(k_cache) && aligned16(v_cache))) &&
@@ -1399,9 +1406,7 @@ extern "C" int cvllm_bias_attn_varlen_dist(const void* q, const void* k_cache, c
                                      max_new, scale, chunk, window, keep_first, sink, sink_logits, dist_bias, dist_rows,
                                      out_stride, st);
   // latent rows that the pipeline above has not taken
-  if (dtype == CVLLM_BF16 && G == 1 && v_cache == k_cache && v_stride == D && slopes == nullptr && dist_bias == nullptr &&
-      cache_rows > 0 && (path == 0 || path == 3) &&
-      cvllm_latent_attn_umma_serves(D, Dv, page_size, out_stride, q, k_cache, out))
+  if (latent)
     return cvllm_launch_latent_attn_umma(q, k_cache, cache_rows, out, out_stride, seq_start, cu_seqlens_q, batch_mapping,
                                          page_table, table_stride_slot, B, total_tokens, max_new, H, D, Dv, page_size,
                                          scale, chunk, window, keep_first, sink, sink_logits, 1, nullptr, -1, st);

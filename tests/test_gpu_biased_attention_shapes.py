@@ -346,3 +346,27 @@ def test_scores_far_below(D, page):
     got, want = decode_one(m2, q2, at), formula(m2, q2, keys2, at)
     assert m2.streaming_decode_kernel(390)
     assert ((got - want).norm() / want.norm()).item() < 2.5e-3
+
+
+@pytest.mark.parametrize("H,spans,latent", [(8, [(0, 2368)], True), (8, [(0, 2369)], False), (32, [(100, 300), (0, 200)], True),
+                                            (32, [(0, 700)], False), (2, [(0, 90)], True)])
+def test_rows_of_64_that_are_their_own_values(H, spans, latent):
+    """One wave of packed query rows stays on the kernel for latent rows (option 3 asks for it everywhere), more do not."""
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context
+
+    m, q, keys = make(H, 1, 64, 64, spans, 24, values_in_keys=True, sink=True)
+    keys = [(k, k) for k, _ in keys]
+    out = []
+    for option in (0, 3):
+        context(spans, False)
+        N.set_test_option("bias_attn_fma", option)
+        try:
+            out.append(m.attend(q))
+        finally:
+            N.set_test_option("bias_attn_fma", 0)
+            reset_context()
+    assert torch.equal(*out) == latent
+    want = formula(m, q, keys, spans)
+    for got in out:
+        assert ((got.double() - want).norm() / want.norm()).item() < 6e-3
