@@ -32,6 +32,7 @@
 // the query columns 4 .. 7 that groups of up to four heads leave free.  Partial states are folded by a second kernel
 // (its workspace needs no zeroed tickets).
 #include <stdlib.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "mma.cuh"
@@ -61,7 +62,12 @@ struct DecodeParams {
   int lens_by_slot;   // seq_lens_bh is the cache's [Bmax+1, HKV] table, indexed through batch_mapping
   int mode;           // 0 = normal; 1 = consumers only drain the ring (load ceiling, profiling only)
   float scale_log2;
-  // biased attention only
+#ifdef CVLLM_DECODE_TRACE
+  unsigned long long* trace;  // profiling build only (tools/trace_decode.py): 8 globaltimer stamps per CTA
+#endif
+};
+
+struct BiasDecodeParams : DecodeParams {   // what the biased attention adds
   const int32_t* positions;   // [B] position of every sequence's token
   int64_t pt_slot, pt_head;   // page table strides
   int64_t o_stride;           // output row stride (elements)
@@ -70,9 +76,6 @@ struct DecodeParams {
   int dist_rows, chunk, window, keep, reserved_slot;
   float sink;                 // 1 = a sink in the denominator
   const float* sink_logits;   // [HQ] or NULL (score 0)
-#ifdef CVLLM_DECODE_TRACE
-  unsigned long long* trace;  // profiling build only (tools/trace_decode.py): 8 globaltimer stamps per CTA
-#endif
 };
 
 __device__ __forceinline__ unsigned long long gtime() {
@@ -99,7 +102,7 @@ struct Slice {
 struct UnitList {
   int pi, lo, begin, kept, count;
   UnitList() = default;
-  __device__ __forceinline__ UnitList(const DecodeParams& p, int b) {
+  __device__ __forceinline__ UnitList(const BiasDecodeParams& p, int b) {
     const bool live = p.batch_mapping[b] != p.reserved_slot;
     pi = p.positions[b];
     lo = p.chunk > 0 ? pi / p.chunk * p.chunk : 0;
@@ -131,7 +134,7 @@ __device__ __forceinline__ uint32_t slot_addr(uint32_t slot, int t, int ch) {
 
 // 1 / denominator of a biased head's row whose running maximum is m (log2 units) and whose sum is l, sink included: the
 // row's values are relative to m, and so is what the sink adds
-__device__ __forceinline__ float bias_inv(const DecodeParams& p, int hq, float m, float l) {
+__device__ __forceinline__ float bias_inv(const BiasDecodeParams& p, int hq, float m, float l) {
   if (p.sink > 0.f) {
     const float sm = (p.sink_logits ? p.sink_logits[hq] : 0.f) * 1.4426950408889634f;
     if (sm - m > 120.f) return 0.f;   // a sink far above every key takes all the weight
@@ -145,7 +148,7 @@ __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, %0;" ::"n
 template <bool BF16, int D, bool BIAS = false>
 __global__ void __launch_bounds__(kDecThreads, 1)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                   const DecodeParams p) {
+                   const std::conditional_t<BIAS, BiasDecodeParams, DecodeParams> p) {
   static_assert(D == 128 || (BIAS && D == 64), "head sizes");
   constexpr int KSTEPS = D / 16;  // 8
   constexpr int MT = D / 16;      // 8 output m-tiles (16 d each)
@@ -272,8 +275,9 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           const int b = head / p.HKV, h = head % p.HKV;
           const int tok = t0 + my_piece * BR;
           const int pg = tok / p.PS;
-          const int32_t* pt = BIAS ? p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head
-                                   : p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + h) * p.NLP;
+          const int32_t* pt;
+          if constexpr (BIAS) pt = p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head;
+          else pt = p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + h) * p.NLP;
           row = pt[pg] * p.PS + (tok - pg * p.PS);
         }
       }
@@ -335,9 +339,11 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const bool low_cols = BIAS && G <= 4 && j >= 2;
     const int qc = low_cols ? 2 * j - 4 : 2 * j;
     float slope0 = 0.f, slope1 = 0.f;
-    if (BIAS && p.slopes) {
-      slope0 = qc < G ? p.slopes[h * G + qc] * 1.4426950408889634f : 0.f;
-      slope1 = qc + 1 < G ? p.slopes[h * G + qc + 1] * 1.4426950408889634f : 0.f;
+    if constexpr (BIAS) {
+      if (p.slopes) {
+        slope0 = qc < G ? p.slopes[h * G + qc] * 1.4426950408889634f : 0.f;
+        slope1 = qc + 1 < G ? p.slopes[h * G + qc + 1] * 1.4426950408889634f : 0.f;
+      }
     }
 
     // ---- Q^T as B operand (n = query r, k = permuted d) ----
@@ -671,7 +677,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 // CTAs: with a CTA per KV head and the slots one after the other 1 x 16000 keys of
 // 8 / 1 heads took 122 us with norms and cache write, 26 us so).
 template <int D>
-__global__ void __launch_bounds__(256) bias_decode_fold_kernel(const DecodeParams p, int C) {
+__global__ void __launch_bounds__(256) bias_decode_fold_kernel(const BiasDecodeParams p, int C) {
   constexpr int ROW = D + 2, PER = D / 32;
   const int hq = blockIdx.x % p.HQ, b = blockIdx.x / p.HQ, G = p.G, h = hq / G, q = hq - h * G, head = b * p.HKV + h;
   __shared__ float s_o[8][D];
@@ -857,7 +863,7 @@ int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_c
                              float scale, const float* slopes, int chunk, int window, int keep, const float* dist_bias,
                              int dist_rows, int sink, const float* sink_logits, int reserved_slot, float* workspace,
                              cudaStream_t st) {
-  DecodeParams p = {};
+  BiasDecodeParams p = {};
   p.q = q; p.out = out;
   p.page_table = page_table; p.batch_mapping = batch_mapping;
   p.scratch = workspace;
