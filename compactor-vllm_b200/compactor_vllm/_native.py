@@ -63,6 +63,9 @@ _SIGNATURES = {
                                     _f, _i, _i, _p]),
     "cvllm_decode_step": (_i, [_p, _p, _i64, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p, _p, _p, _sz,
                                _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _p]),
+    "cvllm_prefill_attention_bounded": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p,
+                                             _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i, _i,
+                                             _f, _i, _p]),
     "cvllm_prefill_attention": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p,
                                      _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64, _i,
                                      _f, _i, _p]),

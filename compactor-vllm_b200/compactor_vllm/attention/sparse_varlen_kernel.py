@@ -32,8 +32,8 @@ def causal_sparse_varlen_with_cache(
     For every sequence b, kv head h and query head g of h:
     softmax(scale * q . [Kcache_bh || Kapp_b]^T, causal on the appended part) .
     [Vcache_bh || Vapp_b]; the prefix length is per (b, h).
-    `max_seqlen_k_cache` is accepted for signature parity (the reference only
-    uses it as an autotune key, :164).
+    `max_seqlen_k_cache`, the longest prefix, only chooses the order of the work
+    (the reference uses it as an autotune key, :164); a wrong one costs speed.
     """
     assert q.ndim == 3, "q should be [N, HQ, D]"
     Ntok, HQ, D = q.shape
@@ -59,11 +59,12 @@ def causal_sparse_varlen_with_cache(
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(D)
     out = torch.empty((Ntok, HQ, D), dtype=q.dtype, device=dev)
-    rc = N.lib().cvllm_prefill_attention(
+    max_past = min(max_seqlen_k_cache, 2 ** 31 - 1) if isinstance(max_seqlen_k_cache, int) else -1
+    rc = N.lib().cvllm_prefill_attention_bounded(
         N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(k_cache), N.ptr(v_cache),
         N.ptr(lens), N.ptr(pt), N.ptr(bm), N.ptr(cu),
         B, Ntok, HQ, HKV, D, int(PAGE_SIZE), pt.shape[-1], CACHE_SIZE,
-        q.stride(0), k.stride(0), v.stride(0), out.stride(0), int(max_seqlen_q),
+        q.stride(0), k.stride(0), v.stride(0), out.stride(0), int(max_seqlen_q), max_past,
         float(sm_scale), N.dtype_code(q.dtype), N.stream(dev),
     )
     N.check(rc, "cvllm_prefill_attention")

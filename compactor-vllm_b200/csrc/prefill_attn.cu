@@ -438,17 +438,17 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
                           const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, void* out,
                           const int32_t* seq_lens_bh, const int32_t* page_table,
                           const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ,
-                          int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q,
+                          int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q, int max_past,
                           float scale_log2, float rescale_threshold, bool bf16, cudaStream_t st);
 
-extern "C" int cvllm_prefill_attention(const void* q, const void* k, const void* v, void* out,
-                                       const void* k_cache, const void* v_cache,
-                                       const int32_t* seq_lens_bh, const int32_t* page_table,
-                                       const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B,
-                                       int N, int HQ, int HKV, int D, int PS, int NLP, int64_t cache_rows,
-                                       int64_t q_stride_n, int64_t k_stride_n, int64_t v_stride_n,
-                                       int64_t o_stride_n, int max_seqlen_q, float sm_scale, int dtype,
-                                       cvllm_stream_t stream) {
+extern "C" int cvllm_prefill_attention_bounded(const void* q, const void* k, const void* v, void* out,
+                                               const void* k_cache, const void* v_cache,
+                                               const int32_t* seq_lens_bh, const int32_t* page_table,
+                                               const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B,
+                                               int N, int HQ, int HKV, int D, int PS, int NLP, int64_t cache_rows,
+                                               int64_t q_stride_n, int64_t k_stride_n, int64_t v_stride_n,
+                                               int64_t o_stride_n, int max_seqlen_q, int max_past, float sm_scale,
+                                               int dtype, cvllm_stream_t stream) {
   CVLLM_CHECK_ARG(B > 0 && N >= 0 && HQ > 0 && HKV > 0 && PS > 0 && NLP > 0 && max_seqlen_q >= 0);
   if (N == 0 || max_seqlen_q == 0) return CVLLM_OK;
   CVLLM_CHECK_ARG(q && k && v && out && k_cache && v_cache && seq_lens_bh && page_table &&
@@ -505,7 +505,7 @@ extern "C" int cvllm_prefill_attention(const void* q, const void* k, const void*
   if ((HQ / HKV) % 2 == 0 && !test_options().prefill_v1.load(std::memory_order_relaxed))
     return cvllm_launch_prefill2(tm_q, tm_k, tm_v, tm_kc, tm_vc, out, seq_lens_bh, page_table,
                                  batch_mapping, cu_seqlens_q, B, N, HQ, HKV, PS, NLP, o_stride_n,
-                                 max_seqlen_q, p.scale_log2, p.rescale_threshold, bf16, st);
+                                 max_seqlen_q, max_past, p.scale_log2, p.rescale_threshold, bf16, st);
   const size_t smem = sizeof(PrefillSmem) + 1024;
   const dim3 grid((max_seqlen_q + kBM - 1) / kBM, HQ, B);
   static std::atomic<uint64_t> attr_bf{0}, attr_h{0};
@@ -518,6 +518,19 @@ extern "C" int cvllm_prefill_attention(const void* q, const void* k, const void*
   }
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
+}
+
+extern "C" int cvllm_prefill_attention(const void* q, const void* k, const void* v, void* out,
+                                       const void* k_cache, const void* v_cache,
+                                       const int32_t* seq_lens_bh, const int32_t* page_table,
+                                       const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B,
+                                       int N, int HQ, int HKV, int D, int PS, int NLP, int64_t cache_rows,
+                                       int64_t q_stride_n, int64_t k_stride_n, int64_t v_stride_n,
+                                       int64_t o_stride_n, int max_seqlen_q, float sm_scale, int dtype,
+                                       cvllm_stream_t stream) {
+  return cvllm_prefill_attention_bounded(q, k, v, out, k_cache, v_cache, seq_lens_bh, page_table, batch_mapping,
+                                         cu_seqlens_q, B, N, HQ, HKV, D, PS, NLP, cache_rows, q_stride_n, k_stride_n,
+                                         v_stride_n, o_stride_n, max_seqlen_q, -1, sm_scale, dtype, stream);
 }
 
 extern "C" int cvllm_selftest_umma(const void* a, const void* b, float* d, int mode, uint32_t lbo,

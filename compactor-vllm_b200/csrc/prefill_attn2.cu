@@ -119,16 +119,16 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // (a form of its own for each order: with the choice at run time the loop below it ran 1 % slower at 32768 tokens)
-  TileOrder at;
-  if constexpr (BY_TILE) at = tile_order(p.seq_lens_bh, p.B * p.HKV, kBM);
-  const int b = BY_TILE ? at.b : blockIdx.z;
-  const int hq0 = 2 * (BY_TILE ? at.pair : blockIdx.y);  // heads hq0, hq0 + 1 share KV head hkv (G even)
+  // (a form of its own for each order: with the choice at run time the loop below it ran 1 % slower, 32768 tokens and the
+  // ragged continuation of tile_order.cuh alike)
+  // grid (tiles, pairs, sequences), or by tiles (pairs, sequences, tiles)
+  const int b = BY_TILE ? blockIdx.y : blockIdx.z;
+  const int hq0 = 2 * (BY_TILE ? blockIdx.x : blockIdx.y);  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
   const int q_beg = p.cu_seqlens_q[b];
   const int La = p.cu_seqlens_q[b + 1] - q_beg;
   const int n_qt = (La + kBM - 1) / kBM;
-  const int qt = BY_TILE ? at.qt : n_qt - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
+  const int qt = BY_TILE ? (int)(gridDim.z - 1 - blockIdx.z) : n_qt - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
   if (qt < 0 || qt >= n_qt) return;
   const int q0 = qt * kBM;
   const int Lc = p.seq_lens_bh[b * p.HKV + hkv];
@@ -491,7 +491,7 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
                           const CUtensorMap& tm_kc, const CUtensorMap& tm_vc, void* out,
                           const int32_t* seq_lens_bh, const int32_t* page_table,
                           const int32_t* batch_mapping, const int32_t* cu_seqlens_q, int B, int N, int HQ,
-                          int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q,
+                          int HKV, int PS, int NLP, int64_t o_stride_n, int max_seqlen_q, int max_past,
                           float scale_log2, float rescale_threshold, bool bf16, cudaStream_t st) {
   Prefill2Params p;
   p.out = out; p.seq_lens_bh = seq_lens_bh; p.page_table = page_table;
@@ -502,10 +502,10 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
   p.rescale_threshold = rescale_threshold;
   const size_t smem = sizeof(Prefill2Smem) + 1024;
   const dim3 grid((max_seqlen_q + p2::kBM - 1) / p2::kBM, HQ / 2, B);
-  const bool by_tile = order_by_tile(grid, N, p2::kBM);
+  const bool by_tile = order_by_tile(grid, N, p2::kBM) && grid.x <= 65535 && past_is_short(max_past, max_seqlen_q);
   auto launch = [&](auto kernel, std::atomic<uint64_t>& attr) -> int {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)kernel, (int)smem, attr));
-    kernel<<<grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
+    kernel<<<by_tile ? dim3(grid.y, grid.z, grid.x) : grid, p2::kThreads, smem, st>>>(tm_q, tm_k, tm_v, tm_kc, tm_vc, p);
     return CVLLM_OK;
   };
   static std::atomic<uint64_t> attr[4] = {{0}, {0}, {0}, {0}};
@@ -529,7 +529,7 @@ extern "C" int cvllm_debug_prefill_trace_read(void* host_out) {
 namespace cvllm {
 __global__ void tile_order_kernel(const int32_t* past, int n, int by_tile, int tile_rows, int32_t* out) {
   TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
-  if (by_tile) at = tile_order(past, n, tile_rows);
+  if (by_tile && pasts_are_short(past, n, tile_rows)) at = tile_order();
   if (threadIdx.x == 0) {
     int32_t* o = out + 3 * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
     o[0] = at.qt;

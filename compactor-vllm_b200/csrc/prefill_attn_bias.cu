@@ -143,17 +143,20 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
-  if (p.by_tile) at = tile_order(p.seq_start, p.B, kBM);
+  int q_beg = p.cu_seqlens_q[at.b], q_end = p.cu_seqlens_q[at.b + 1], start = p.seq_start[at.b];
+  if (p.by_tile && pasts_are_short(p.seq_start, p.B, kBM)) {   // (behind the loads above: see prefill_attn2.cu)
+    at = tile_order();
+    q_beg = p.cu_seqlens_q[at.b], q_end = p.cu_seqlens_q[at.b + 1], start = p.seq_start[at.b];
+  }
   const int b = at.b;
   const int hq0 = 2 * at.pair;  // heads hq0, hq0 + 1 share KV head hkv (G even)
   const int hkv = hq0 / p.G;
-  const int q_beg = p.cu_seqlens_q[b];
-  const int La = p.cu_seqlens_q[b + 1] - q_beg;
+  const int La = q_end - q_beg;
   const int n_qt = (La + kBM - 1) / kBM;
   const int qt = at.qt;  // heaviest (latest) tiles first
   if (qt >= n_qt) return;
   const int q0 = qt * kBM;
-  const int p0 = p.seq_start[b] + q0;                      // position of the tile's first query
+  const int p0 = start + q0;                               // position of the tile's first query
   const int p_last = p0 + min(kBM, La - q0) - 1;           // ... and of its last valid one
   auto first_key = [&](int pi) {                           // first position a query at pi sees through chunk and window
     int lo = p.chunk > 0 ? (pi / p.chunk) * p.chunk : 0;

@@ -6,8 +6,9 @@
 // begins again with its longest tile, the last one included.  But CTAs that run side by side read K and V at about
 // the rate that L2 can give, and tiles of one head at adjacent places share those reads.
 // So the order by tiles (all pairs and sequences inside) is taken for launches of at most twelve waves of CTAs that have
-// work and a mean past (over sequences and heads, whatever their order) of at most half the longest prompt; the order by
-// pairs otherwise.
+// work and a short past; the order by pairs otherwise.  Short is, in prefill_attn2.cu, a longest past (the caller's bound) of
+// at most three quarters of the longest prompt, and in prefill_attn_bias.cu, whose callers bring no bound, a mean past (over
+// sequences, whatever their order; read by every CTA) of at most half of it.
 // Measured in turn in one process, by pairs -> by tiles (whatever the rule says of the case), us, 32 / 8 heads of 128 unless
 // said:
 //   prompts of 1000: 25 -> 25     2048: 56 -> 42     4096: 141 -> 121     8192: 513 -> 465     12000: 1053 -> 999
@@ -17,6 +18,8 @@
 //   portions with slopes, 4096: 206 -> 177; with a window: 156 -> 148; 2000 + 700 + 3000 after 9000: 1053 -> 1092
 //   4000 + 2077 + 911 + 3301: 269 -> 257     one of 4000 among three of 100: 150 -> 140     twelve of 500, the first
 //   without a past, the others after 4000: 328 -> 342
+//   4000 + 2077 + 911 + 3301 after up to 1440 tokens a head 446 -> 438, 3480 608 -> 630, 7200 943 -> 1031; 4096 after up to
+//   3000 255 -> 249, 5400 329 -> 331; 2000 + 700 + 3000 after up to 2400 274 -> 266; 3000 (16 / 4 heads) after 3000 94 -> 93
 #pragma once
 #include <algorithm>
 
@@ -33,20 +36,26 @@ inline bool order_by_tile(dim3 grid, int tokens, int tile_rows) {
   return live > sm_count() && live <= 12 * (int64_t)sm_count();
 }
 
+// A caller without a bound says -1.
+inline bool past_is_short(int max_past, int longest) { return max_past >= 0 && 4 * (int64_t)max_past <= 3 * (int64_t)longest; }
+
 struct TileOrder {
   int qt, pair, b;  // query tile (may lie beyond the sequence's tiles), head pair, sequence
 };
 
 // Grid (tiles, pairs, sequences) for which order_by_tile() holds; past [n]: tokens before the new ones, of every sequence or
-// of every (sequence, head).  Called by whole warps.
-__device__ __forceinline__ TileOrder tile_order(const int32_t* past, int n, int tile_rows) {
+// of every (sequence, head).  If they are short on the mean, the order is by tiles.  Called by whole warps.
+__device__ __forceinline__ bool pasts_are_short(const int32_t* past, int n, int tile_rows) {
   // a sum that the compiler knows to be the warp's own: with shuffles, what follows from the order (the sequence, its
   // addresses) is kept per lane, and the whole kernel runs 13 to 17 % slower.  No overflow: n is at most 12 CTAs an SM
   unsigned own = 0;
   for (int i = threadIdx.x & 31; i < n; i += 32) own += (unsigned)min(past[i], 1 << 20);
   const unsigned sum = __reduce_add_sync(0xffffffffu, own);
-  if (2 * (long long)sum > (long long)gridDim.x * tile_rows * n)
-    return {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
+  return 2 * (long long)sum <= (long long)gridDim.x * tile_rows * n;
+}
+
+// This CTA's place in the order by tiles.
+__device__ __forceinline__ TileOrder tile_order() {
   const unsigned idx = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   const unsigned h = idx / gridDim.y;
   return {(int)(gridDim.x - 1 - h / gridDim.z), (int)(idx % gridDim.y), (int)(h % gridDim.z)};

@@ -307,7 +307,17 @@ int cvllm_decode_step(const void* key, const void* value, int64_t sk_b, int64_t 
 
 /* causal_sparse_varlen_with_cache — attention/sparse_varlen_kernel.py:11-197
  * (K1 :265-519).  Causal attention of the packed new tokens over
- * [cached prefix of (b,h) || new K/V of b]; tcgen05/TMEM/TMA kernel. */
+ * [cached prefix of (b,h) || new K/V of b]; tcgen05/TMEM/TMA kernel.
+ * The _bounded form takes max_past, the longest cached prefix (-1: not known): with it a launch of few waves takes its query
+ * tiles in the better order.  The results do not depend on it. */
+int cvllm_prefill_attention_bounded(const void* q, const void* k, const void* v, void* out,
+                                    const void* k_cache, const void* v_cache,
+                                    const int32_t* seq_lens_bh, const int32_t* page_table,
+                                    const int32_t* batch_mapping, const int32_t* cu_seqlens_q,
+                                    int B, int N, int HQ, int HKV, int D, int PS, int NLP,
+                                    int64_t cache_rows, int64_t q_stride_n, int64_t k_stride_n,
+                                    int64_t v_stride_n, int64_t o_stride_n, int max_seqlen_q, int max_past,
+                                    float sm_scale, int dtype, cvllm_stream_t stream);
 int cvllm_prefill_attention(const void* q, const void* k, const void* v, void* out,
                             const void* k_cache, const void* v_cache,
                             const int32_t* seq_lens_bh, const int32_t* page_table,
@@ -414,7 +424,7 @@ int cvllm_selftest_eig(const float* gram, double* lam_out, double* vec_out, floa
  * Self tests (device sanity for descriptor encodings; used by tests only)
  * --------------------------------------------------------------------- */
 /* The order in which the prefill kernels' CTAs take their query tiles (csrc/tile_order.cuh; tests): for a grid of
- * (tiles, pairs, seqs) over `tokens` new tokens in tiles of tile_rows rows, with the pasts [n] on the device:
+ * (tiles, pairs, seqs) over `tokens` new tokens in tiles of tile_rows rows, with the pasts [n] on the device (biased form):
  * out[3 * cta] = tile, pair, sequence; *by_tile = whether such a launch looks at the pasts at all. */
 int cvllm_selftest_tile_order(const int32_t* past, int n, int tiles, int pairs, int seqs, int tokens, int tile_rows,
                               int32_t* out, int* by_tile, cvllm_stream_t stream);

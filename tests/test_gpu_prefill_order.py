@@ -1,5 +1,5 @@
-"""The order in which a launch takes its query tiles (by tiles, by pairs because of the first sequence's past, by pairs
-because of the launch's size) changes no bit of a sequence's output."""
+"""The order in which a launch takes its query tiles (by tiles, by pairs because of the pasts, by pairs because of the
+launch's size) changes no bit of a sequence's output."""
 from __future__ import annotations
 
 import pytest
@@ -14,14 +14,15 @@ DEV = "cuda"
 HQ, HKV, PS, D = 32, 8, 128, 128
 
 
-def _run(seqs, new, past, pools):
-    """Outputs per sequence of one call over the sequences `seqs`, in that order."""
+def _run(seqs, new, past, pools, bound=None):
+    """Outputs per sequence of one call over the sequences `seqs`, in that order; `bound`: what it is told of the pasts."""
     q, k, v, cu, kc, vc, pt, bm = pools
     rows = torch.cat([torch.arange(int(cu[i]), int(cu[i + 1])) for i in seqs]).to(DEV)
     cu_call = torch.tensor([0] + [new[i] for i in seqs]).cumsum(0).to(torch.int32)
     lens = torch.tensor([[past[i]] * HKV for i in seqs], dtype=torch.int32, device=DEV)
     out = causal_sparse_varlen_with_cache(q[rows], k[rows], v[rows], kc, vc, lens, pt, bm[list(seqs)].contiguous(),
-                                          cu_call.to(DEV), max(new[i] for i in seqs), int(lens.max()), HKV, PS, None)
+                                          cu_call.to(DEV), max(new[i] for i in seqs), int(lens.max()) if bound is None else bound,
+                                          HKV, PS, None)
     torch.cuda.synchronize()
     return dict(zip(seqs, out.split([new[i] for i in seqs])))
 
@@ -30,7 +31,8 @@ def _run(seqs, new, past, pools):
 @pytest.mark.parametrize("new,past,calls", [
     # whole tiles of 128: a ragged tail's tile also holds rows of whatever sequence comes next, and the rows of a warp
     # move their softmax reference point together (ragged tails against the oracle: test_gpu_prefill.py)
-    ([640, 256, 128], [0, 600, 1], [(0, 1, 2), (1, 0, 2), (2, 1, 0)]),          # the first past: 0, 600, 1
+    ([640, 256, 128], [0, 600, 1], [(0, 1, 2), (1, 0, 2), (2, 1, 0)]),          # by pairs for the pasts, in three batch orders
+    ([1280, 640, 128], [0, 2600, 1], [(0, 1, 2), (2, 0), (2, 1, 0), (1, 2)]),   # by pairs for the pasts; by tiles; pairs; one wave
     ([384] * 40, [0, 70] * 20, [tuple(range(40)), tuple(range(20)), tuple(range(20, 40))]),   # 1920 CTAs; 960
 ])
 def test_order_changes_nothing(dtype, new, past, calls):
@@ -45,8 +47,20 @@ def test_order_changes_nothing(dtype, new, past, calls):
             assert torch.equal(o, want[i]), i
 
 
+@pytest.mark.parametrize("bound", [0, 959, 961, 2 ** 40, -1])
+def test_the_bound_of_the_pasts_only_orders(bound):
+    """By tiles up to three quarters of the longest prompt (960), by pairs beyond; a bound that is wrong costs speed alone."""
+    new, past = [1280, 384, 128], [500, 2600, 0]
+    kc, vc, pt, bm = make_paged(3, HKV, D, PS, [[n] * HKV for n in past], torch.bfloat16, DEV, seed=5, poison=True)
+    cu = torch.tensor([0] + new).cumsum(0)
+    q, k, v = fused_qkv(int(cu[-1]), HQ, HKV, D, torch.bfloat16, DEV, seed=6)
+    pools = (q, k, v, cu, kc, vc, pt, bm)
+    want, got = _run((0, 1, 2), new, past, pools), _run((0, 1, 2), new, past, pools, bound)
+    assert all(torch.equal(got[i], want[i]) and torch.isfinite(got[i]).all() for i in want)
+
+
 def _order(past, tiles, pairs, seqs, tokens):
-    """What the CTAs of a launch take, (tile, pair, sequence) each in launch order, and whether the rule looked at the pasts."""
+    """What the CTAs of a biased launch take, (tile, pair, sequence) each in launch order, and whether it looked at the pasts."""
     import ctypes
     from compactor_vllm import _native as N
 
