@@ -257,10 +257,14 @@ class BiasedChunkAttention(nn.Module):
     def _field(self, name: str):
         """A parameter, buffer or plain attribute by name, past Module.__getattr__ (0.5 us a name, and a step reads eight).  A
         name that is none of these (a parametrized one is a property of the class) goes the usual way."""
-        for held in (self._parameters, self._buffers, self.__dict__):
-            if name in held:
-                return held[name]
-        return getattr(self, name)
+        own = self.__dict__
+        held = own["_parameters"]
+        if name in held:
+            return held[name]
+        held = own["_buffers"]
+        if name in held:
+            return held[name]
+        return own[name] if name in own else getattr(self, name)
 
     @torch.no_grad()
     def refresh_distance_bias(self, rel: Optional[torch.Tensor] = None) -> None:
@@ -324,15 +328,16 @@ class BiasedChunkAttention(nn.Module):
         A captured step is chosen by its bound `max_keys` and replayed at any length, where the splits are those of the bound
         too: with 8192 or more the streaming kernel is level or ahead at every length (32 sequences, heads of 64: 100 keys
         26.6 / 34.8, 4000 keys 98 / 154), with 2048 it is behind at short ones (100 keys 26.6 / 22.5, 1000 keys 43 / 59)."""
-        keys = min(max_keys, self.chunk) if self.chunk else max_keys
-        if self.window:
-            keys = min(keys, self.window)
+        chunk, window, D, G, page = self.chunk, self.window, self.head_dim, self.num_kv_heads, int(self.page_size)
+        keys = chunk if 0 < chunk < max_keys else max_keys
+        if 0 < window < keys:
+            keys = window
         keys = min(keys + self.keep_first, max_keys)
-        D, page = self.head_dim, int(self.page_size)
-        least = 256 if D != 64 else min(max(256, batch * self.num_kv_heads + 64), 512)
+        rows = batch * G
+        least = 256 if D != 64 else min(max(256, rows + 64), 512)
         return (keys >= least and not self.values_in_keys and D == self.v_head_dim and D in (64, 128)
-                and self.num_heads // self.num_kv_heads <= 8 and batch * self.num_kv_heads <= 4096
-                and self.k_cache.dtype == torch.bfloat16 and (page % 128 == 0 or page in (16, 32, 64)))
+                and self.num_heads // G <= 8 and rows <= 4096
+                and self.k_cache.dtype is torch.bfloat16 and (page % 128 == 0 or page in (16, 32, 64)))
 
     def forward(self, qkv: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         ctx: Context = get_context()
@@ -348,7 +353,8 @@ class BiasedChunkAttention(nn.Module):
         q = torch.empty((T, H, D), dtype=qkv.dtype, device=dev)
         pt = self.page_table
         table = (N.ptr(pt), pt.stride(0), pt.stride(1), int(self.page_size))
-        rot, q_w, k_w = self._field("inv_freq"), self._field("q_norm_weight"), self._field("k_norm_weight")
+        field = self._field
+        rot, q_w, k_w = field("inv_freq"), field("q_norm_weight"), field("k_norm_weight")
         if self.row_norm:
             caches = (None, None) if s is not None else (N.ptr(self.k_cache), N.ptr(self.v_cache))
             N.check(lib.cvllm_row_norm_rope_store(
@@ -390,9 +396,12 @@ class BiasedChunkAttention(nn.Module):
         else:
             assert out.shape == (T, H * Dv) and out.stride(1) == 1 and out.dtype == q.dtype
             o_stride = out.stride(0)
-        if self._field("dist_bias") is None and self._field("rel") is not None:
+        field = self._field
+        db = field("dist_bias")
+        if db is None and field("rel") is not None:
             self.refresh_distance_bias()
-        db, slopes, sink_logits = self._field("dist_bias"), self._field("slopes"), self._field("sink_logits")
+            db = field("dist_bias")
+        slopes, sink_logits = field("slopes"), field("sink_logits")
         dist = (self.window, self.keep_first, N.ptr(db), 0 if db is None else db.shape[0])
         if ctx.is_prefill:
             B = ctx.batch_mapping.numel()
@@ -404,21 +413,22 @@ class BiasedChunkAttention(nn.Module):
         else:
             assert ctx.batch_mapping.numel() == T
             max_keys = int(ctx.max_seqlen_k)
-            if (self.streaming_decode_kernel(max_keys, T) and o_stride % 2 == 0 and out.data_ptr() % 4 == 0
-                    and (q.data_ptr() | self.k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
+            q_at, k_at, v_at, o_at = N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), N.ptr(out)
+            if (self.streaming_decode_kernel(max_keys, T) and o_stride % 2 == 0 and o_at % 4 == 0
+                    and (q_at | k_at | v_at) % 16 == 0):
                 ws = N.workspace(dev, N.sized(dev.index, "cvllm_bias_decode_workspace_bytes", T, H, G, D), "bias_attn_stream")
                 N.check(lib.cvllm_bias_attn_decode_stream(
-                    N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), self.k_cache.shape[0], *table, N.ptr(ctx.positions_i32),
+                    q_at, k_at, v_at, self.k_cache.shape[0], *table, N.ptr(ctx.positions_i32),
                     N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
-                    self.scale, N.ptr(out), o_stride, T, H, G, D, RESERVED_BATCH, N.ptr(ws), ws.numel(), N.stream(dev)),
+                    self.scale, o_at, o_stride, T, H, G, D, RESERVED_BATCH, N.ptr(ws), ws.numel(), N.stream(dev)),
                     "cvllm_bias_attn_decode_stream")
             else:
                 splits = self.decode_splits(T, max_keys)
                 ws = N.workspace(dev, 4 * T * H * splits * (2 + Dv), "bias_attn_decode") if splits > 1 else None
                 N.check(lib.cvllm_bias_attn_decode_dist(
-                    N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.positions_i32),
+                    q_at, k_at, v_at, *table, N.ptr(ctx.positions_i32),
                     N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
-                    self.scale, N.ptr(out), o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits,
+                    self.scale, o_at, o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits,
                     N.ptr(ws), ws.numel() if ws is not None else 0, v_stride, code, N.stream(dev)), "cvllm_bias_attn_decode")
         if keep != Dv:
             out = out.view(T, H, Dv)[:, :, :keep]
