@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark of the attention + KV-compression hot path (BASELINE.json's metric).
+"""Headline benchmark of the attention + KV-compression hot path (prefill, decode and compression).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 \

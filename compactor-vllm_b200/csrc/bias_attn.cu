@@ -9,7 +9,9 @@
 // Optional masks and biases beside these: a sliding window with kept first tokens, a learned bias per distance
 // (DistBias), and a learned sink score per head.
 // The new tokens' keys are in the cache before the attention launches read it, so both read keys from one place.
-// All arithmetic is fp32; 16-bit storage only rounds q, k, v and the output.
+// Scores, softmax and sums are fp32; 16-bit storage rounds q, k, v and the output, and the mma.sync portion kernel also its
+// probabilities (bfloat16, 2^-9).  The tcgen05 portions (prefill_attn_bias.cu) and the streaming decode steps (decode_attn.cu)
+// say for themselves how they hold theirs.
 #include "common.cuh"
 #include "mma.cuh"
 

@@ -389,7 +389,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       };
       // P = exp2(S*scale - m_ref) packed to 16 bit over the S columns; returns the row sum of this tile.
       // Packed fp32 pairs: one fp32x2 FMA scales and shifts two logits, one fp32x2 add sums two probabilities (A/B on B200,
-      // r02d: 7.62-7.68 ms vs 7.95-8.05 ms scalar at 32K).
+      // 7.62-7.68 ms vs 7.95-8.05 ms scalar at 32K).
       auto write_p = [&]() -> float {
         const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
         const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(neg_m, neg_m);
@@ -432,7 +432,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
       // The row maximum of the tile is known before the first exponential.  Taking it off the critical path
       // (exponentials against the previous tiles' reference, rescale deferred by one tile) was measured on B200
-      // and changed nothing: 7.70-7.91 ms vs 7.60-7.80 ms at 32K (r02i) — the chain of maxima already hides under the
+      // and changed nothing: 7.70-7.91 ms vs 7.60-7.80 ms at 32K — the chain of maxima already hides under the
       // TMEM load latency.
       {
         const float m_new = fmaxf(m_ref, row_max());

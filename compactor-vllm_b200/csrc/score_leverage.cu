@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const Lev
     // Centre (one tile: the uncentred sketch is still resident; several tiles: re-derived centred), zero the
     // padded token columns (partial k16 steps must contribute nothing) and hand the centred sketch to the score
     // kernel — one vectorised pass, a warp per sketch row, 8 tokens per lane.  (A flat `i / nt` element loop
-    // here was 65 % of the kernel's instructions: ncu r02g.)
+    // here was 65 % of the kernel's instructions, by ncu.)
     const bool resident = c_len <= kTokTile;
     if (!resident) {
       sketch_tile<BF16>(sm, p, h, c_beg + t0, nt, true);

@@ -1,4 +1,4 @@
-"""BASELINE.json's configurations 2-5 at their FULL sizes through the reference-shaped API
+"""The headline configurations 2-5 at their FULL sizes through the reference-shaped API
 (plugin scoring -> Attention.forward -> decode), checked by what stays affordable at that size:
 
 * attention: a device-side fp32 restatement on SAMPLED query rows (the CPU oracle would take minutes);

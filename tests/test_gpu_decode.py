@@ -10,7 +10,7 @@ from helpers import make_paged
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-TOL = {torch.float16: 3e-3, torch.bfloat16: 2e-2}  # reference test atol 3e-3 (fp16); north_star 2e-2 bf16
+TOL = {torch.float16: 3e-3, torch.bfloat16: 2e-2}  # reference test atol 3e-3 (fp16); 2e-2 bf16
 
 
 def _check(q, kc, vc, lens, pt, bm, HKV, PS, dtype, scale=None):

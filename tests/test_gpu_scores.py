@@ -197,9 +197,8 @@ def test_leverage_golden(name):
     d = (raw.float().cpu() - g["raw"].float()).abs()
     # Chunks shorter than the sketch (48 columns) have a rank-deficient Gram whose small
     # eigenvalues are bf16 rounding noise: swapping the reference's own factorisation
-    # (fp32 svd -> fp64 svd or eigh) moves those scores by 0.03-0.05 on this very fixture
-    # (tools/leverage_sensitivity.py), so they get the noise-floor bound; full-rank chunks the
-    # north_star bound.
+    # (fp32 svd -> fp64 svd or eigh) moves those scores by 0.03-0.05 on this very fixture,
+    # so they get the noise-floor bound; full-rank chunks the tight one.
     _, chunk_lens = osc.split_into_chunks(lens, g["chunk_size"])
     off = 0
     for L in chunk_lens:
@@ -261,8 +260,8 @@ def test_leverage_vs_oracle_well_conditioned(dtype, lens, H, chunk):
 def test_leverage_low_rank_keys_statistics(dtype, lens, H, chunk):
     """Low-rank keys (what real K looks like): the 16-bit Gram is indefinite, its small |lambda| (~1
     against lambda_max ~1e5) are rounding noise of the Gram itself, and x^T |G|^-1 x is ill-conditioned
-    in the reference too: one ulp in one entry of the 16-bit column mean (a summation-order effect,
-    tools/debug_leverage2.py) moves ~1 % of a chunk's scores by O(1), and the reference's own fp32 SVD
+    in the reference too: one ulp in one entry of the 16-bit column mean (a summation-order effect)
+    moves ~1 % of a chunk's scores by O(1), and the reference's own fp32 SVD
     sits as far from the exact factorisation ("eigh64") of the same Gram as we do.  What is stable —
     and asserted — is the bulk: median distance to the exact answer no worse than the reference
     arithmetic's, scores finite and >= 0, and (full-rank chunks) the z-scored top half agreeing with the
