@@ -119,6 +119,10 @@ _SIGNATURES = {
     "cvllm_token_shift_mix": (_i, [_p, _i64, _p, _i, _i, _p, _p, _p, _p, _p, _i, _i, _p, _i64, _i, _i, _p]),
     "cvllm_delta_rule": (_i, [_p, _i64, _p, _i64, _i, _i, _p, _p, _p, _p, _i64, _i, _p, _i, _f, _p, _p, _p, _p, _i, _i,
                               _p, _i64, _i, _i, _i, _i, _i, _i, _p]),
+    "cvllm_delta_rule_chunks_workspace_bytes": (_sz, [_i64, _i, _i, _i, _i, _i, _i]),
+    "cvllm_delta_rule_chunks": (_i, [_p, _i64, _p, _i64, _i, _i, _p, _p, _p, _p, _i64, _i, _p, _i, _f, _p, _p, _p, _i64, _i, _i,
+                                     _p, _i64, _i, _i, _i, _i, _i, _i, _p, _sz, _p]),
+    "cvllm_delta_chunk_aborts": (_i, [_p]),
     "cvllm_bias_attn_varlen_dist": (_i, [_p, _p, _p, _p, _i64, _i64, _i, _p, _p, _p, _p, _i, _i, _i, _p, _i, _i, _p, _f,
                                          _p, _i64, _i, _i, _i, _i, _i, _i, _i, _i64, _i, _i64, _i, _p]),
     "cvllm_bias_attn_decode_dist": (_i, [_p, _p, _p, _p, _i64, _i64, _i, _p, _p, _p, _i, _i, _i, _p, _i, _i, _p, _f, _p,

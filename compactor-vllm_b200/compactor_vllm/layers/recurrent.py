@@ -116,11 +116,23 @@ class DeltaRuleMixer(nn.Module):
         out = torch.empty((T, H * Dv), dtype=cols.dtype, device=dev)
         g_off = C
         b_off = C + H * Dv
-        N.check(lib.cvllm_delta_rule(N.ptr(qkv), qkv.stride(0), N.ptr(cols), cols.stride(0), b_off, b_off + H,
-                                     N.ptr(self.A_log), N.ptr(self.dt_bias), N.ptr(state.matrix_state), N.ptr(cols),
-                                     cols.stride(0), g_off, N.ptr(self.norm_weight), 0, self.eps, *geom, N.ptr(slots),
-                                     B, max_new, N.ptr(out), out.stride(0), H, G, D, Dv, RESERVED_BATCH, code, st),
-                "cvllm_delta_rule")
+        rows = (N.ptr(qkv), qkv.stride(0), N.ptr(cols), cols.stride(0), b_off, b_off + H, N.ptr(self.A_log),
+                N.ptr(self.dt_bias), N.ptr(state.matrix_state), N.ptr(cols), cols.stride(0), g_off, N.ptr(self.norm_weight),
+                0, self.eps)
+        # portions in chunks on the tensor cores where the library has them for these sizes and rows lie on 16 bytes
+        need = 0
+        if geom[2] is None and all(x % 16 == 0 for x in (qkv.data_ptr(), cols.data_ptr(), out.data_ptr(),
+                                                         cols.stride(0) * cols.element_size(), g_off * cols.element_size(),
+                                                         out.stride(0) * out.element_size(), C * 4)):
+            need = lib.cvllm_delta_rule_chunks_workspace_bytes(T, B, max_new, H, G, D, Dv)
+        if need:
+            ws = N.workspace(dev, need, "delta_rule_chunks")
+            N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], N.ptr(slots), T, B, max_new, N.ptr(out),
+                                                out.stride(0), H, G, D, Dv, RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st),
+                    "cvllm_delta_rule_chunks")
+        else:
+            N.check(lib.cvllm_delta_rule(*rows, *geom, N.ptr(slots), B, max_new, N.ptr(out), out.stride(0), H, G, D, Dv,
+                                         RESERVED_BATCH, code, st), "cvllm_delta_rule")
         return self.o_proj(out)
 
 

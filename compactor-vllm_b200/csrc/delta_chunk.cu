@@ -1,0 +1,1092 @@
+// Gated delta rule over portions of prompts, in chunks of 64 tokens on tcgen05 / TMEM (the recurrence, its gates and norm:
+// recurrent.cu, whose kernels keep short portions, single tokens and other sizes).
+//
+// With S [D, Dv] a head's state before a chunk, its tokens counted 0 .. 63, q and k the unit vectors, w_ts = g_(s+1) .. g_t
+// and G_t = g_0 .. g_t (products, never quotients), token t writes k_t u_t^T with
+//   u_t = beta_t (v_t - G_t S^T k_t) - sum_(s < t) beta_t w_ts (k_t . k_s) u_s
+// - a triangular system that the value columns share.  With T its inverse (times diag(beta)), P = (w_ts (q_t . k_s)) for
+// s <= t, C = K^T diag(w_63) T, and R = V - diag(G) K S,
+//   S <- G_63 S + C R;   O = diag(G) Q S + (P T) R
+// C and P T depend on the inputs alone: delta_rows_kernel and delta_coef_kernel make them for all chunks at once.
+// delta_chunk_kernel walks a sequence's chunks with two products in sequence, [K; Q] S and C R, and P T R beside them.
+//
+// 32 bits on a 16-bit tensor pipe: every operand is the sum of three bfloat16 numbers (24 bits of fraction; the rest is below
+// 2^-26 of the value), every product takes the six pairs of parts down to 2^-18, and pairs of one magnitude share an
+// accumulator: with the three parts of the right operand side by side in N, the left operand's first part meets all three
+// parts, its second part the first two (32 accumulator columns further on) and its third part the first.  Three products
+// of 96, 64 and 32 columns read the left operand three times instead of six, and the three sums are added smallest first.
+//
+// A chunk's images (operands as they lie in shared memory, 128-byte swizzle) are written once by the first kernels and copied
+// by untiled bulk copies.
+//
+// A cluster of Dv / 32 CTAs serves one (head, sequence); each keeps 32 value columns of S in registers (a thread per key
+// channel and 16 columns), rewritten as three parts into shared memory after every chunk.  Unit norms need all columns
+// of a head: the CTAs exchange their sums of squares through distributed shared memory.
+//
+// What is not finite stays behind its token: an element of R that is infinite or NaN would meet zeros of P T in earlier
+// tokens' rows, so it enters the products as 0 and its column becomes NaN from that token on.
+//
+// Every wait has a limit.  A wait that runs out sets the CTA's abort flag; all roles then leave their loops, copies and
+// products in flight are waited for (with a limit), the CTA's state becomes NaN and a counter that the host can read
+// (cvllm_delta_chunk_aborts) goes up.
+#include <algorithm>
+
+#include "mma.cuh"
+#include "recur_common.cuh"
+#include "tma.cuh"
+
+namespace cvllm {
+
+__device__ int g_delta_chunk_aborts;
+
+namespace {
+
+constexpr int kChunk = 64;                       // tokens
+constexpr int kCols = 32;                        // value columns of a CTA
+constexpr int kPanel = 128 * 128;                // 128 rows of 64 16-bit numbers
+constexpr int kParts = 3;
+constexpr uint32_t kSpins = 1u << 20;            // tries of a wait, each up to kSleep ns: about two seconds
+constexpr uint32_t kSleep = 2000;
+
+struct DeltaChunkArgs {
+  const float* qkv;            // [tokens, 2 G D + H Dv] (q | k | v) after the convolution
+  int64_t qkv_stride, proj_stride, gate_stride, out_stride;
+  const void *proj, *gate;
+  int b_off, a_off, gate_off;
+  const float *A_log, *dt_bias, *norm_w;
+  int norm_head_stride;
+  float eps;
+  float* state;
+  void* out;
+  int H, G, Dv, reserved_slot;
+  StepGeom g;
+  // a launch takes the chunks [first, first + per_seq) of every sequence; their images lie at slot(b, chunk)
+  int first, per_seq, compact;
+  unsigned char* kq;           // [slots, G, parts, D / 64, panel]: rows 0 .. 63 k, 64 .. 127 q
+  unsigned char* cp;           // [slots, H, parts, D + 64 rows of 128 bytes]: rows 0 .. D - 1 C, then P T
+  float* dots;                 // [slots, G, 2, 10, 16, 16]: lower blocks of K K^T and Q K^T
+  float* gw;                   // [slots, H, 64]: G_t
+  float* carry;                // [B, H, Dv, D] between launches
+  __device__ __forceinline__ int slot(int b, int t0, int c) const { return compact ? t0 / kChunk + b + c : b * per_seq + c - first; }
+};
+
+// x = hi + mid + lo, each a bfloat16; two numbers a word
+__device__ __forceinline__ void split3(float2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const float2 minus = make_float2(-1.f, -1.f);
+  hi = pack2<true>(x.x, x.y);
+  x = __ffma2_rn(unpack2<true>(hi), minus, x);
+  mid = pack2<true>(x.x, x.y);
+  x = __ffma2_rn(unpack2<true>(mid), minus, x);
+  lo = pack2<true>(x.x, x.y);
+}
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  split3(make_float2(x, y), hi, mid, lo);
+}
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// acc of two 8-column tiles (i: which) += A . B on three parts each; the largest pair apart from the others
+__device__ __forceinline__ void mma_parts(float (&big)[4], float (&rest)[4], const uint32_t (&fa)[3][4], const uint32_t (&fb)[3][4],
+                                          int i) {
+  auto mul = [&](float (&acc)[4], int ea, int eb) {
+    mma16816<true>(acc, fa[ea][0], fa[ea][1], fa[ea][2], fa[ea][3], fb[eb][2 * i], fb[eb][2 * i + 1]);
+  };
+  mul(rest, 0, 2);
+  mul(rest, 1, 1);
+  mul(rest, 2, 0);
+  mul(big, 0, 0);
+  mul(rest, 0, 1);
+  mul(rest, 1, 0);
+}
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+// A try sleeps until the phase ends (kSleep at most): a dozen warps that poll shared memory instead slow the products' operand
+// reads down.
+__device__ __forceinline__ bool dc_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+               "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(kSleep) : "memory");
+  return ok != 0;
+}
+
+// byte offset of (row, 16-byte piece) in a panel
+__device__ __forceinline__ int panel_at(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
+
+// ---------------------------------------------------------------------------------------------------------
+// Unit rows and their products.  grid (chunks, G, B), 256 threads: k and q rows to unit length and into parts, the image out
+// by a bulk copy; K K^T and Q K^T (lower blocks of 16) from the parts on mma.sync.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int kPrepThreads = 256;
+constexpr int kUnits = 20;    // lower blocks of 16 x 16 of two matrices
+__device__ __forceinline__ void unit_of(int u, int& m, int& mt, int& nt) {
+  m = u / 10;
+  const int i = u % 10;
+  mt = i < 1 ? 0 : i < 3 ? 1 : i < 6 ? 2 : 3;
+  nt = i - mt * (mt + 1) / 2;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const DeltaChunkArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  const int b = blockIdx.z, grp = blockIdx.y, c = a.first + blockIdx.x;
+  int t0, n_new, start;
+  portion(a.g, b, t0, n_new, start);
+  const int n = min(kChunk, n_new - c * kChunk);
+  if (n <= 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = a.slot(b, t0, c);
+  unsigned char* img = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  constexpr int kPartBytes = (D / 64) * kPanel;
+
+  // ---- unit rows in parts: a thread has four numbers of 2 x 8 (heads of 64: 2 x 4) rows ----
+  {
+    constexpr int LR = D / 4, RW = 32 / LR, kPasses = kChunk / (8 * RW), kRows = 2 * kPasses;
+    const int sub = lane / LR, l = lane % LR, d = l * 4;
+    const float* base = a.qkv + (int64_t)(t0 + c * kChunk) * a.qkv_stride + grp * D + d;
+    const int off0 = (d >> 6) * kPanel + (d & 7) * 2, piece = (d & 63) >> 3;
+    float4 x[kRows];           // q rows, then k rows
+    float ss[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int t = (i % kPasses) * (8 * RW) + warp * RW + sub;
+      x[i] = t < n ? *reinterpret_cast<const float4*>(base + (int64_t)t * a.qkv_stride + (i / kPasses) * a.G * D)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      ss[i] = fmaf(x[i].w, x[i].w, fmaf(x[i].z, x[i].z, fmaf(x[i].y, x[i].y, x[i].x * x[i].x)));
+    // sums over a row's lanes, all rows together: every exchange halves the sums that a lane is left with
+    int mine = 0;
+#pragma unroll
+    for (int o = 1, left = kRows; o < LR; o <<= 1) {
+      if (left > 1) {
+        const bool up = (l & o) != 0;
+        left >>= 1;
+#pragma unroll
+        for (int i = 0; i < kRows / 2; ++i)
+          if (i < left) {
+            const float send = up ? ss[i] : ss[i + left], keep = up ? ss[i + left] : ss[i];
+            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        if (up) mine += left;
+      } else {
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+      }
+    }
+    const float inv_mine = (mine < kPasses ? rsqrtf((float)D) : 1.0f) / sqrtf(ss[0] + 1e-6f);
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      // the lane that row i's sum ended up in: bit k of its number is set where the k-th exchange kept the upper half
+      int from = 0;
+#pragma unroll
+      for (int o = 1, left = kRows, at = i; left > 1; o <<= 1) {
+        left >>= 1;
+        if (at >= left) from |= o, at -= left;
+      }
+      const float inv = __shfl_sync(0xffffffffu, inv_mine, from, LR);
+      uint32_t p[kParts][2];
+      split3(x[i].x * inv, x[i].y * inv, p[0][0], p[1][0], p[2][0]);
+      split3(x[i].z * inv, x[i].w * inv, p[0][1], p[1][1], p[2][1]);
+      const int t = (i % kPasses) * (8 * RW) + warp * RW + sub, row = i < kPasses ? kChunk + t : t;
+#pragma unroll
+      for (int e = 0; e < kParts; ++e)
+        *reinterpret_cast<uint2*>(img + e * kPartBytes + off0 + panel_at(row, piece)) = make_uint2(p[e][0], p[e][1]);
+    }
+  }
+  fence_proxy_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    unsigned char* dst = a.kq + ((int64_t)slot * a.G + grp) * (kParts * kPartBytes);
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(img)),
+                 "r"(kParts * kPartBytes)
+                 : "memory");
+    bulk_commit();
+  }
+
+  // ---- K K^T and Q K^T: 20 lower blocks over eight warps ----
+  constexpr int kRounds = (kUnits + 7) / 8;
+#pragma unroll 1
+  for (int r = 0; r < kRounds; ++r) {
+    float big[2][4], rest[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) big[i][e] = rest[i][e] = 0.f;
+    const int u = warp + 8 * r;
+    if (u < kUnits) {
+      int m, mt, nt;
+      unit_of(u, m, mt, nt);
+      const int row_a = m * kChunk + mt * 16 + (lane & 15), row_b = nt * 16 + (lane & 7) + ((lane >> 4) << 3);
+      const uint32_t base = smem_u32(img);
+#pragma unroll 2
+      for (int ks = 0; ks < D / 16; ++ks) {
+        const int pa = ks * 2 + (lane >> 4), pb = ks * 2 + ((lane >> 3) & 1);
+        uint32_t fa[kParts][4], fb[kParts][4];
+#pragma unroll
+        for (int e = 0; e < kParts; ++e) {
+          ldmatrix4(fa[e], base + e * kPartBytes + (pa >> 3) * kPanel + panel_at(row_a, pa & 7));
+          ldmatrix4(fb[e], base + e * kPartBytes + (pb >> 3) * kPanel + panel_at(row_b, pb & 7));
+        }
+        mma_parts(big[0], rest[0], fa, fb, 0);
+        mma_parts(big[1], rest[1], fa, fb, 1);
+      }
+      float* dst = a.dots + (((int64_t)slot * a.G + grp) * kUnits + u) * 256;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          *reinterpret_cast<float2*>(dst + ((lane >> 2) + 8 * e) * 16 + i * 8 + (lane & 3) * 2) =
+              make_float2(big[i][2 * e] + rest[i][2 * e], big[i][2 * e + 1] + rest[i][2 * e + 1]);
+    }
+  }
+  if (tid == 0) bulk_wait<0>();
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Coefficients of the chunks.  grid (chunks, H, B), 256 threads: decays; A (beta_t w_ts k_t . k_s, t > s) and P; the inverse X
+// of I + A in blocks of 16 tokens - diagonal blocks by forward substitution, a column per thread, then halves of 32 and of 64
+// from X_21 = -X_22 (A_21 X_11), half a block per warp; C = K^T diag(w_63) X diag(beta) from three parts on mma.sync; and
+// P X diag(beta).  Row t of X and of P X is made of rows up to t alone, by sums that stop at t: what is not finite stays behind
+// its token.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int kPitchX = 68;   // X: rows read four columns at a time
+constexpr int kPitchA = 65;   // the others: sixteen rows' entries of a column at a time
+template <int D>
+struct CoefSmem {
+  static constexpr int kRow = kChunk * 128;                  // one part's panel of K rows
+  static constexpr int k = 0;                                // [parts][D / 64][64 rows], then C's image
+  static constexpr int a = kParts * (D / 64) * kRow;         // A, then the parts of diag(w) T, then P T's image
+  static constexpr int p = a + kParts * kRow;
+  static constexpr int x = p + kChunk * kPitchA * 4;
+  static constexpr int total = x + kChunk * kPitchX * 4;
+};
+
+// acc[4] += (row `row` of `left`, 16 numbers) x (16 rows of `right`, four columns from col).  CAUSAL: number k only where
+// k <= row.
+template <bool CAUSAL>
+__device__ __forceinline__ void block_mul(float (&acc)[4], const float* left, int pitch, const float* right, int row, int col) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const float4 r = *reinterpret_cast<const float4*>(right + k * kPitchX + col);
+    const float l = left[row * pitch + k];
+    if (!CAUSAL || k <= row) {
+      acc[0] = fmaf(l, r.x, acc[0]);
+      acc[1] = fmaf(l, r.y, acc[1]);
+      acc[2] = fmaf(l, r.z, acc[2]);
+      acc[3] = fmaf(l, r.w, acc[3]);
+    }
+  }
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const DeltaChunkArgs a) {
+  using L = CoefSmem<D>;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ float2 s_tok[kChunk];          // decays and betas
+  __shared__ uint64_t s_bar;
+  __shared__ float s_w[kChunk], s_rest[32]; // products of the decays behind token s: of the chunk's, of the first 32
+  const int b = blockIdx.z, h = blockIdx.y, c = a.first + blockIdx.x, grp = h / (a.H / a.G);
+  int t0, n_new, start;
+  portion(a.g, b, t0, n_new, start);
+  const int n = min(kChunk, n_new - c * kChunk);
+  if (n <= 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = a.slot(b, t0, c);
+  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  float *A = reinterpret_cast<float*>(sm + L::a), *P = reinterpret_cast<float*>(sm + L::p), *X = reinterpret_cast<float*>(sm + L::x);
+
+  float z_decay = 0.f, z_beta = 0.f;
+  if (tid < n) {
+    const T* pr = static_cast<const T*>(a.proj) + (int64_t)(t0 + c * kChunk + tid) * a.proj_stride;
+    z_decay = to_f<T>(pr[a.a_off + h]) + a.dt_bias[h];
+    z_beta = to_f<T>(pr[a.b_off + h]);
+  }
+  const float rate = a.A_log[h];
+  if (tid == 0) {       // k's rows, used by the product at the end
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+    const unsigned char* kq = a.kq + ((int64_t)slot * a.G + grp) * (kParts * (D / 64) * kPanel);
+    mbar_expect_tx(&s_bar, kParts * (D / 64) * L::kRow);
+    for (int i = 0; i < kParts * (D / 64); ++i) bulk_load(sm + L::k + i * L::kRow, kq + i * kPanel, L::kRow, &s_bar);
+  }
+  // the dots' blocks to their places in A and P
+  {
+    const float4* src = reinterpret_cast<const float4*>(a.dots + ((int64_t)slot * a.G + grp) * kUnits * 256);
+    float4 x[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) x[i] = src[i * kPrepThreads + tid];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int e = i * kPrepThreads + tid;     // four numbers each; 64 per block
+      int m, mt, nt;
+      unit_of(e >> 6, m, mt, nt);
+      float* dst = (m ? P : A) + (mt * 16 + ((e >> 2) & 15)) * kPitchA + nt * 16 + (e & 3) * 4;
+      dst[0] = x[i].x;
+      dst[1] = x[i].y;
+      dst[2] = x[i].z;
+      dst[3] = x[i].w;
+    }
+  }
+  if (tid < kChunk)     // missing tokens: decay 1, beta 0
+    s_tok[tid] = tid < n ? make_float2(exp_1ulp(-expf(rate) * softplus_f(z_decay)), sigmoid_f(z_beta)) : make_float2(1.f, 0.f);
+  __syncthreads();
+  if (warp == 0) {      // G_t and w_63t by scans of products, two tokens a lane
+    const float ga = s_tok[2 * lane].x, gb = s_tok[2 * lane + 1].x;
+    float up = ga * gb, down = up, low = up;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float lo = __shfl_up_sync(0xffffffffu, up, o), hi = __shfl_down_sync(0xffffffffu, down, o);
+      const float in = __shfl_down_sync(0xffffffffu, low, o);
+      if (lane >= o) up *= lo;
+      if (lane + o < 32) down *= hi;
+      if ((lane & 15) + o < 16) low *= in;
+    }
+    const float before = __shfl_up_sync(0xffffffffu, up, 1), behind = __shfl_down_sync(0xffffffffu, down, 1);
+    const float in = __shfl_down_sync(0xffffffffu, low, 1);
+    const float prev = lane ? before : 1.f, next = lane < 31 ? behind : 1.f, next_low = lane < 15 ? in : 1.f;
+    if (lane < 16) {
+      s_rest[2 * lane] = next_low * gb;
+      s_rest[2 * lane + 1] = next_low;
+    }
+    s_w[2 * lane] = next * gb;
+    s_w[2 * lane + 1] = next;
+    *reinterpret_cast<float2*>(a.gw + ((int64_t)slot * a.H + h) * kChunk + 2 * lane) = make_float2(prev * ga, up);
+  }
+  __syncthreads();
+
+  // ---- A and P in the dots' place: a thread per column and half of it ----
+  {
+    const int s = tid & 63, upper = (tid >> 6) & 1, of_q = tid >> 7;
+    float* m = of_q ? P : A;
+    const int lo = upper ? max(32, s + 1) : s + 1, hi = upper ? kChunk : 32;
+    float w = upper && s < 32 ? s_rest[s] : 1.f;
+#pragma unroll 1
+    for (int t8 = lo & ~7; t8 < hi; t8 += 8) {   // eight at a time: their loads before their stores
+      float x[8];
+      float2 tok[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        x[i] = m[(t8 + i) * kPitchA + s];
+        tok[i] = s_tok[t8 + i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (t8 + i >= lo) {
+          w *= tok[i].x;
+          m[(t8 + i) * kPitchA + s] = x[i] * (of_q ? w : tok[i].y * w);
+        }
+    }
+  }
+  __syncthreads();
+
+  // ---- X ----
+  if (tid < kChunk) {      // diagonal blocks
+    const int blk = tid >> 4, col = tid & 15;
+    const float* d = A + blk * 16 * kPitchA + blk * 16;
+    float x[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      float acc0 = t == col ? 1.f : 0.f, acc1 = 0.f;
+#pragma unroll
+      for (int s = 0; s < t; ++s) {
+        const float r = d[t * kPitchA + s];
+        if (s & 1) acc1 = fmaf(-r, x[s], acc1);
+        else acc0 = fmaf(-r, x[s], acc0);
+      }
+      x[t] = acc0 + acc1;
+    }
+#pragma unroll
+    for (int t = 0; t < 16; ++t) X[(blk * 16 + t) * kPitchX + blk * 16 + col] = t < col ? 0.f : x[t];
+  }
+  // half a block per warp: a row and four columns a lane
+  const int row = lane >> 1, col = (warp & 1) * 8 + (lane & 1) * 4, q4 = warp >> 1;
+  auto A_at = [&](int i, int j) { return A + i * 16 * kPitchA + j * 16; };
+  auto P_at = [&](int i, int j) { return P + i * 16 * kPitchA + j * 16; };
+  auto X_at = [&](int i, int j) { return X + i * 16 * kPitchX + j * 16; };
+  auto put = [&](float* m, const float (&v)[4], float sign) {
+    *reinterpret_cast<float4*>(m + row * kPitchX + col) = make_float4(sign * v[0], sign * v[1], sign * v[2], sign * v[3]);
+  };
+  __syncthreads();
+  if (q4 < 2) {            // blocks (1, 0) and (3, 2); sums on the way lie in the blocks above the diagonal
+    const int i = 2 * q4 + 1, j = 2 * q4;
+    float acc[4] = {}, res[4] = {};
+    block_mul<false>(acc, A_at(i, j), kPitchA, X_at(j, j), row, col);
+    put(X_at(j, i), acc, -1.f);
+    __syncwarp();
+    block_mul<true>(res, X_at(i, i), kPitchX, X_at(j, i), row, col);
+    put(X_at(i, j), res, 1.f);
+  }
+  __syncthreads();
+  {
+    const int i = 2 + (q4 >> 1), j = q4 & 1;     // blocks (2, 0), (2, 1), (3, 0), (3, 1)
+    float acc[4] = {};
+    if (j == 0) {
+      block_mul<false>(acc, A_at(i, 0), kPitchA, X_at(0, 0), row, col);
+      block_mul<false>(acc, A_at(i, 1), kPitchA, X_at(1, 0), row, col);
+    } else {
+      block_mul<false>(acc, A_at(i, 1), kPitchA, X_at(1, 1), row, col);
+    }
+    put(X_at(j, i), acc, -1.f);
+    __syncthreads();
+    float res[4] = {};
+    if (i == 3) block_mul<false>(res, X_at(3, 2), kPitchX, X_at(j, 2), row, col);
+    block_mul<true>(res, X_at(i, i), kPitchX, X_at(j, i), row, col);
+    put(X_at(i, j), res, 1.f);
+  }
+  __syncthreads();
+
+  // ---- diag(w) X diag(beta) in parts (a later token's beta may be NaN: left out, not multiplied) ----
+  for (int i = tid; i < kChunk * 8; i += kPrepThreads) {
+    const int t = i >> 3, s0 = (i & 7) * 8;
+    const float w = s_w[t];
+    uint32_t p[kParts][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int s = s0 + 2 * q;
+      float2 v = make_float2(0.f, 0.f);
+      if (s <= t) {
+        v = *reinterpret_cast<const float2*>(X + t * kPitchX + s);
+        v.x *= w * s_tok[s].y;
+        v.y = s < t ? v.y * (w * s_tok[s + 1].y) : 0.f;
+      }
+      split3(v, p[0][q], p[1][q], p[2][q]);
+    }
+#pragma unroll
+    for (int e = 0; e < kParts; ++e)
+      *reinterpret_cast<uint4*>(sm + L::a + e * L::kRow + panel_at(t, i & 7)) = make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
+  }
+  __syncthreads();
+  {
+    uint32_t spins = 0;
+    while (!dc_try(&s_bar, 0))
+      if (++spins > kSpins) {     // the chunk's coefficients are void: its decays, and with them the state, become NaN
+        if (tid < kChunk) a.gw[((int64_t)slot * a.H + h) * kChunk + tid] = __int_as_float(0x7fc00000);
+        if (tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
+        break;
+      }
+  }
+
+  // ---- C: 16 channels a warp, all 64 columns; column block nb has rows of token blocks kb >= nb ----
+  float big[4][2][4], rest[4][2][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) big[i][j][e] = rest[i][j][e] = 0.f;
+  if (warp < D / 16) {
+    const uint32_t kb_at = smem_u32(sm + L::k), tb_at = smem_u32(sm + L::a);
+    const int piece_a = 2 * warp + ((lane >> 3) & 1), row_a = (lane & 7) + ((lane >> 4) << 3), row_b = (lane & 7) + (((lane >> 3) & 1) << 3);
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb) {
+      uint32_t fa[kParts][4];
+#pragma unroll
+      for (int e = 0; e < kParts; ++e)
+        ldmatrix4_trans(fa[e], kb_at + (e * (D / 64) + (piece_a >> 3)) * L::kRow + panel_at(kb * 16 + row_a, piece_a & 7));
+#pragma unroll
+      for (int nb = 0; nb <= kb; ++nb) {
+        uint32_t fb[kParts][4];
+#pragma unroll
+        for (int e = 0; e < kParts; ++e) ldmatrix4_trans(fb[e], tb_at + e * L::kRow + panel_at(kb * 16 + row_b, nb * 2 + (lane >> 4)));
+        mma_parts(big[nb][0], rest[nb][0], fa, fb, 0);
+        mma_parts(big[nb][1], rest[nb][1], fa, fb, 1);
+      }
+    }
+  }
+  __syncthreads();   // K and the parts are read: the images take their places
+  if (warp < D / 16) {
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          uint32_t p[kParts];
+          split3(big[nb][i][2 * e] + rest[nb][i][2 * e], big[nb][i][2 * e + 1] + rest[nb][i][2 * e + 1], p[0], p[1], p[2]);
+          const int at = panel_at(warp * 16 + (lane >> 2) + 8 * e, nb * 2 + i) + (lane & 3) * 4;
+#pragma unroll
+          for (int q = 0; q < kParts; ++q) *reinterpret_cast<uint32_t*>(sm + L::k + q * D * 128 + at) = p[q];
+        }
+  }
+  // ---- P X diag(beta): the ten lower blocks, five block products a pair of warps; blocks above the diagonal are zero ----
+  auto put_pt = [&](int i, int j, const float (&acc)[4]) {
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = i > j || (i == j && col + q <= row) ? acc[q] * s_tok[j * 16 + col + q].y : 0.f;
+    uint32_t p[kParts][2];
+    split3(v[0], v[1], p[0][0], p[1][0], p[2][0]);
+    split3(v[2], v[3], p[0][1], p[1][1], p[2][1]);
+#pragma unroll
+    for (int e = 0; e < kParts; ++e)
+      *reinterpret_cast<uint2*>(sm + L::a + e * L::kRow + panel_at(i * 16 + row, (j * 16 + col) >> 3) + (col & 4) * 2) =
+          make_uint2(p[e][0], p[e][1]);
+  };
+  const uint32_t blocks = q4 == 0 ? 0x0030u : q4 == 1 ? 0x3220u : q4 == 2 ? 0x1031u : 0x33221121u;   // a byte each: row, column
+#pragma unroll 1
+  for (int q = 0; q < (q4 == 3 ? 4 : 2); ++q) {
+    const int i = (blocks >> (8 * q + 4)) & 15, j = (blocks >> (8 * q)) & 15;
+    float acc[4] = {};
+#pragma unroll 1
+    for (int k = j; k < i; ++k) block_mul<false>(acc, P_at(i, k), kPitchA, X_at(k, j), row, col);
+    block_mul<true>(acc, P_at(i, i), kPitchA, X_at(i, j), row, col);
+    put_pt(i, j, acc);
+  }
+  {
+    const float zero[4] = {};
+    for (int q = q4; q < 6; q += 4) {
+      const int i = q < 3 ? 0 : q < 5 ? 1 : 2, j = q < 3 ? q + 1 : q < 5 ? q - 1 : 3;
+      put_pt(i, j, zero);
+    }
+  }
+  fence_proxy_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    unsigned char* dst = a.cp + ((int64_t)slot * a.H + h) * (kParts * (D + kChunk) * 128);
+    for (int e = 0; e < kParts; ++e) {
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + e * (D + kChunk) * 128),
+                   "r"(smem_u32(sm + L::k + e * D * 128)), "r"(D * 128)
+                   : "memory");
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + e * (D + kChunk) * 128 + D * 128),
+                   "r"(smem_u32(sm + L::a + e * L::kRow)), "r"(L::kRow)
+                   : "memory");
+    }
+    bulk_commit();
+    bulk_wait<0>();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// The chunks of one (head, sequence).  grid (H * Dv / 32, B), clusters of Dv / 32; 512 threads: warps 0 - 7 turn products
+// into operands (TMEM lane = row: token or key channel; warps 4 - 7 the second 16 columns), warp 8 issues the products,
+// warp 9 the copies; warps 10, 11, 14 and 15 read the lanes of Q S and P T R and make the outputs (12 and 13 only fill the
+// place that gives those warps their quarter of TMEM).
+// ---------------------------------------------------------------------------------------------------------
+template <int D>
+struct ChunkSmem {
+  static constexpr int kqPart = (D / 64) * kPanel;          // [K; Q], one part
+  static constexpr int cpPart = (D + kChunk) * 128;         // [C; P T], one part
+  static constexpr int kq = 0;
+  static constexpr int cp = kParts * kqPart;
+  static constexpr int s = cp + kParts * cpPart;            // [parts][D rows][64 bytes]
+  static constexpr int sPart = D * kCols * 2;
+  static constexpr int r = s + kParts * sPart;              // [parts][64 rows][64 bytes]
+  static constexpr int rPart = kChunk * kCols * 2;
+  static constexpr int total = r + kParts * rPart;
+};
+
+struct ChunkBars {
+  uint64_t kq_full[kParts], cp_full;
+  uint64_t y_done, s_done, o_done;       // the products [K; Q] S, C R and P T R
+  uint64_t s_full, r_full;               // their right operands
+  uint64_t o_free;                       // P T R is read
+  uint64_t norm[2], drain;
+  float part[2][16][kChunk];             // sums of squares: [CTA * 2 + column half][token]
+  float norm_w[kCols];
+  int bad[2][kCols], any_bad[2];         // first token of the chunk whose R is not finite, per column
+  uint32_t tmem_base;
+  volatile uint32_t abort;
+};
+
+__device__ __forceinline__ bool dc_wait(uint64_t* bar, uint32_t parity, ChunkBars& b) {
+  uint32_t spins = 0;
+  while (!dc_try(bar, parity)) {
+    if (b.abort) return false;
+    if (++spins > kSpins) {
+      b.abort = 1;
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool dc_wait_warp(uint64_t* bar, uint32_t parity, ChunkBars& b) {
+  return __all_sync(0xffffffffu, dc_wait(bar, parity, b));
+}
+// right operands: N runs along the rows of memory (64 bytes of 32 columns a part), 64-byte swizzle
+__device__ __forceinline__ uint64_t cols_desc(uint32_t addr, int part_bytes) {
+  return (umma_smem_desc(addr, part_bytes, 512) & ~((uint64_t)7 << 61)) | ((uint64_t)4 << 61);
+}
+// 16 columns (`half` of the 32) of row `row` -> the three parts of a right operand
+__device__ __forceinline__ void put_parts(unsigned char* base, int part_bytes, int row, int half, const float2 (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    uint32_t p[kParts][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split3(v[4 * q + i], p[0][i], p[1][i], p[2][i]);
+    const int at = row * 64 + (((half * 2 + q) ^ ((row >> 1) & 3)) << 4);
+#pragma unroll
+    for (int e = 0; e < kParts; ++e)
+      *reinterpret_cast<uint4*>(base + e * part_bytes + at) = make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
+  }
+}
+// the three sums of a product, smallest first
+__device__ __forceinline__ void take_product(uint32_t addr, float2 (&v)[8]) {
+  uint32_t x[3][16];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) tmem_ld16(addr + e * kCols, x[e]);
+  tc_wait_ld();
+  auto pair = [&](int e, int j) { return make_float2(__uint_as_float(x[e][2 * j]), __uint_as_float(x[e][2 * j + 1])); };
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = __fadd2_rn(pair(0, j), __fadd2_rn(pair(1, j), pair(2, j)));
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArgs a) {
+  using L = ChunkSmem<D>;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ ChunkBars bars;
+  const int VT = a.Dv / kCols, h = blockIdx.x / VT, vt = blockIdx.x % VT, b = blockIdx.y;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int t0, n_all, start;
+  portion(a.g, b, t0, n_all, start);
+  const int chunks = min(a.per_seq, cdiv(max(n_all, 0), kChunk) - a.first);
+  if (chunks <= 0) return;                 // the same for every CTA of the cluster
+  const int seq_slot = a.g.slots[b], grp = h / (a.H / a.G);
+  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+
+  if (tid == 0) {
+    for (int e = 0; e < kParts; ++e) mbar_init(&bars.kq_full[e], 1);
+    mbar_init(&bars.cp_full, 1);
+    mbar_init(&bars.y_done, 1);
+    mbar_init(&bars.s_done, 1);
+    mbar_init(&bars.o_done, 1);
+    mbar_init(&bars.s_full, 384);          // eight warps of the state, four of the outputs (Q S is read)
+    mbar_init(&bars.r_full, 128);
+    mbar_init(&bars.o_free, 128);
+    mbar_init(&bars.norm[0], 1);
+    mbar_init(&bars.norm[1], 1);
+    mbar_init(&bars.drain, 1);
+    bars.any_bad[0] = bars.any_bad[1] = 0;
+    bars.abort = 0;
+    mbar_fence_init();
+  }
+  if (tid < kCols) {
+    bars.norm_w[tid] = a.norm_w[h * a.norm_head_stride + vt * kCols + tid];
+    bars.bad[0][tid] = bars.bad[1][tid] = kChunk;
+  }
+  if (warp == 8) {
+    tmem_alloc(&bars.tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (VT > 1) cluster_sync_all();          // barriers exist before a neighbour writes to them
+  const uint32_t tmem = bars.tmem_base;
+  constexpr uint32_t kY = 0, kS = 128, kO = 256;   // TMEM columns of the products
+  const int first_slot = a.slot(b, t0, a.first);
+  bool ok = true;
+
+  if (warp == 9) {
+    // ------------------------------ copies ------------------------------
+    if (lane == 0) {
+      const unsigned char* kq = a.kq + ((int64_t)first_slot * a.G + grp) * (kParts * L::kqPart);
+      const unsigned char* cp = a.cp + ((int64_t)first_slot * a.H + h) * (kParts * L::cpPart);
+      const int64_t kq_step = (int64_t)a.G * kParts * L::kqPart, cp_step = (int64_t)a.H * kParts * L::cpPart;
+      int begun = 0, begun_cp = 0;
+      for (int c = 0; c < chunks; ++c) {
+        // the images' places are free behind the last chunk's first product and its last one
+        if (c > 0) ok = dc_wait(&bars.y_done, (c - 1) & 1, bars);
+        if (!ok) break;
+        for (int e = 0; e < kParts; ++e) {
+          mbar_expect_tx(&bars.kq_full[e], L::kqPart);
+          bulk_load(sm + L::kq + e * L::kqPart, kq + c * kq_step + e * L::kqPart, L::kqPart, &bars.kq_full[e]);
+        }
+        ++begun;
+        if (c > 0) ok = dc_wait(&bars.o_done, (c - 1) & 1, bars);
+        if (!ok) break;
+        mbar_expect_tx(&bars.cp_full, kParts * L::cpPart);
+        bulk_load(sm + L::cp, cp + c * cp_step, kParts * L::cpPart, &bars.cp_full);
+        ++begun_cp;
+      }
+      if (!ok) {         // the copies in flight land before the CTA ends
+        auto land = [&](uint64_t* bar, int n) {
+          for (uint32_t spins = 0; n > 0 && !mbar_try_wait(bar, (n - 1) & 1) && spins < kSpins; ++spins) {}
+        };
+        for (int e = 0; e < kParts; ++e) land(&bars.kq_full[e], begun);
+        land(&bars.cp_full, begun_cp);
+      }
+    }
+  } else if (warp == 8) {
+    // ----------------------------- products -----------------------------
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint64_t kq_d = umma_smem_desc(smem_u32(sm + L::kq), 16, 1024);
+    const uint64_t cp_d = umma_smem_desc(smem_u32(sm + L::cp), 16, 1024);
+    const uint64_t s_d = cols_desc(smem_u32(sm + L::s), L::sPart);
+    const uint64_t r_d = cols_desc(smem_u32(sm + L::r), L::rPart);
+    // the left operand's part e meets the first 3 - e parts of the right one
+    auto product = [&](uint32_t d, int e, int ks, uint64_t left, uint64_t right) {
+      umma_ss_warp(tm + d + e * kCols, left, right, umma_idesc(true, 128, kCols * (kParts - e), false, true),
+                   (e > 0 || ks > 0) ? 1u : 0u);
+    };
+    // 128 rows of [C; P T] from row `row` on, times R
+    auto product_r = [&](uint32_t d, int row) {
+#pragma unroll
+      for (int e = 0; e < kParts; ++e)
+#pragma unroll
+        for (int ks = 0; ks < kChunk / 16; ++ks)
+          product(d, e, ks, umma_desc_add(cp_d, e * L::cpPart + row * 128 + ks * 32), umma_desc_add(r_d, ks * 1024));
+    };
+    for (int c = 0; c < chunks && ok; ++c) {
+      const uint32_t ph = c & 1;
+      ok = dc_wait_warp(&bars.s_full, ph, bars);
+#pragma unroll
+      for (int e = 0; e < kParts; ++e) {
+        ok = ok && dc_wait_warp(&bars.kq_full[e], ph, bars);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          product(kY, e, ks, umma_desc_add(kq_d, e * L::kqPart + (ks >> 2) * kPanel + (ks & 3) * 32), umma_desc_add(s_d, ks * 1024));
+      }
+      if (!ok) break;
+      umma_commit_warp(&bars.y_done);
+      ok = dc_wait_warp(&bars.cp_full, ph, bars) && dc_wait_warp(&bars.r_full, ph, bars) &&
+           (c == 0 || dc_wait_warp(&bars.o_free, ph ^ 1, bars));
+      if (!ok) break;
+      tc_fence_after();
+      product_r(kS, 0);                    // heads of 64: C and P T at once
+      umma_commit_warp(&bars.s_done);
+      if (D == 128) product_r(kO, 64);     // lanes 64 .. 127: P T (the others: C's second half again, not read)
+      umma_commit_warp(&bars.o_done);
+    }
+    if (!ok) {           // products in flight end before TMEM is given back
+      umma_commit_warp(&bars.drain);
+      for (uint32_t spins = 0; !mbar_try_wait(&bars.drain, 0) && spins < kSpins; ++spins) {}
+    }
+    __syncwarp();
+  } else if (warp < 8) {
+    // -------------------- products to operands, state --------------------
+    const int q4 = warp & 3, half = warp >> 2, row = q4 * 32 + lane;   // TMEM lane
+    const bool early = q4 < 2;             // rows 0 .. 63, the chunk's tokens: R
+    const int col0 = vt * kCols + half * 16;
+    const uint32_t my = tmem + ((uint32_t)(q4 * 32) << 16) + half * 16;
+    const bool keyed = row < D;            // a key channel's thread
+    float* st = a.state + (((int64_t)seq_slot * a.H + h) * a.Dv + col0) * D + row;
+    float* carry = a.carry + (((int64_t)b * a.H + h) * a.Dv + col0) * D + row;
+    const float* gw = a.gw + ((int64_t)first_slot * a.H + h) * kChunk;
+    float2 S[8];
+    {
+      const float* from = a.first > 0 ? carry : st;
+      const bool zero = !keyed || (a.first == 0 && start <= 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        S[j] = zero ? make_float2(0.f, 0.f) : make_float2(from[(int64_t)(2 * j) * D], from[(int64_t)(2 * j + 1) * D]);
+    }
+    if (keyed) put_parts(sm + L::s, L::sPart, row, half, S);
+    fence_proxy_async_smem();
+    mbar_arrive(&bars.s_full);
+
+    for (int c = 0; c < chunks; ++c) {
+      const uint32_t ph = c & 1;
+      const float g_all = gw[kChunk - 1];
+      // ---- K S -> R = V - G K S ----
+      if (early) {
+        const int tok = (a.first + c) * kChunk + row;       // within the portion
+        const float g_t = -gw[row];
+        float4 v[4];
+        {
+          const float4* p = reinterpret_cast<const float4*>(a.qkv + (int64_t)(t0 + tok) * a.qkv_stride + 2 * a.G * D + h * a.Dv + col0);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = tok < n_all ? p[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        ok = dc_wait_warp(&bars.y_done, ph, bars);
+        if (!ok) break;
+        tc_fence_after();
+        float2 o[8], not_finite = make_float2(0.f, 0.f);
+        take_product(my + kY, o);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          o[j] = __ffma2_rn(make_float2(g_t, g_t), o[j], j & 1 ? make_float2(v[j / 2].z, v[j / 2].w) : make_float2(v[j / 2].x, v[j / 2].y));
+          not_finite = __ffma2_rn(o[j], make_float2(0.f, 0.f), not_finite);
+        }
+        if (!(not_finite.x + not_finite.y == 0.f)) {
+          auto check = [&](float& x, int j) {
+            if (!(fabsf(x) <= 3.3e38f)) {
+              atomicMin(&bars.bad[ph][half * 16 + j], row);
+              x = 0.f;
+            }
+          };
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            check(o[j].x, 2 * j);
+            check(o[j].y, 2 * j + 1);
+          }
+          bars.any_bad[ph] = 1;
+        }
+        put_parts(sm + L::r, L::rPart, row, half, o);
+        fence_proxy_async_smem();
+        tc_fence_before();
+        mbar_arrive(&bars.r_full);
+      }
+      // ---- the state behind the chunk ----
+      ok = dc_wait_warp(&bars.s_done, ph, bars);
+      if (!ok) break;
+      tc_fence_after();
+      if (warp == 0) {                     // the last chunk's, whose readers are through (s_full, o_free)
+        bars.bad[ph ^ 1][lane] = kChunk;
+        if (lane == 0) bars.any_bad[ph ^ 1] = 0;
+      }
+      float2 x[8];
+      take_product(my + kS, x);
+      if (*const_cast<volatile int*>(&bars.any_bad[ph])) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (bars.bad[ph][half * 16 + 2 * j] < kChunk) x[j].x = __int_as_float(0x7fc00000);
+          if (bars.bad[ph][half * 16 + 2 * j + 1] < kChunk) x[j].y = __int_as_float(0x7fc00000);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) S[j] = __ffma2_rn(make_float2(g_all, g_all), S[j], x[j]);
+      if (keyed) put_parts(sm + L::s, L::sPart, row, half, S);
+      fence_proxy_async_smem();
+      tc_fence_before();
+      mbar_arrive(&bars.s_full);
+      gw += (int64_t)a.H * kChunk;
+    }
+    if (keyed) {
+      const bool ends = (a.first + chunks) * kChunk >= n_all;
+      float* to = ends ? (seq_slot != a.reserved_slot ? st : nullptr) : carry;
+      const float nan = __int_as_float(0x7fc00000);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (to) {
+          to[(int64_t)(2 * j) * D] = ok ? S[j].x : nan;
+          to[(int64_t)(2 * j + 1) * D] = ok ? S[j].y : nan;
+        }
+    }
+    if (!ok && tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
+  } else if ((warp & 3) >= 2) {
+    // ------------------------------ outputs ------------------------------
+    const int q4 = warp & 3, half = (warp >> 2) - 2, t = (q4 - 2) * 32 + lane;   // TMEM lanes 64 .. 127: tokens
+    const int col0 = vt * kCols + half * 16;
+    const uint32_t my = tmem + ((uint32_t)(q4 * 32) << 16) + half * 16;
+    const float* gw = a.gw + ((int64_t)first_slot * a.H + h) * kChunk + t;
+    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + a.first * kChunk + t) * a.out_stride + h * a.Dv + col0;
+    const T* gate = static_cast<const T*>(a.gate) + (int64_t)(t0 + a.first * kChunk + t) * a.gate_stride + a.gate_off + h * a.Dv + col0;
+    constexpr int kPieces = sizeof(T);     // 16 numbers in 16-byte pieces
+    uint4 z[kPieces];
+    int left = n_all - a.first * kChunk - t;   // tokens of the portion from this thread's on
+    auto load_gate = [&]() {
+#pragma unroll
+      for (int j = 0; j < kPieces; ++j) z[j] = left > 0 ? *reinterpret_cast<const uint4*>(gate + j * (16 / sizeof(T))) : make_uint4(0, 0, 0, 0);
+    };
+    float g_t = *gw;
+    load_gate();
+    mbar_arrive(&bars.s_full);
+    for (int c = 0; c < chunks; ++c) {
+      const uint32_t ph = c & 1;
+      float2 o[8], x[8];
+      ok = dc_wait_warp(&bars.y_done, ph, bars);
+      if (!ok) break;
+      tc_fence_after();
+      take_product(my + kY, o);
+      tc_fence_before();
+      mbar_arrive(&bars.s_full);           // Q S may be overwritten
+      ok = dc_wait_warp(&bars.o_done, ph, bars);
+      if (!ok) break;
+      tc_fence_after();
+      take_product(my + (D == 128 ? kO : kS), x);
+      tc_fence_before();
+      if (*const_cast<volatile int*>(&bars.any_bad[ph])) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (t >= bars.bad[ph][half * 16 + 2 * j]) x[j].x = __int_as_float(0x7fc00000);
+          if (t >= bars.bad[ph][half * 16 + 2 * j + 1]) x[j].y = __int_as_float(0x7fc00000);
+        }
+      }
+      mbar_arrive(&bars.o_free);
+      float2 sq = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        o[j] = __ffma2_rn(make_float2(g_t, g_t), o[j], x[j]);
+        sq = __ffma2_rn(o[j], o[j], sq);
+      }
+      float ss = sq.x + sq.y;
+      if (t == 0 && half == 0) mbar_expect_tx(&bars.norm[ph], VT * 2 * kChunk * sizeof(float));
+      float* mine = &bars.part[ph][vt * 2 + half][t];
+      for (int r = 0; r < VT; ++r)
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(mapa_u32(mine, r)),
+                     "r"(__float_as_uint(ss)), "r"(mapa_u32(&bars.norm[ph], r))
+                     : "memory");
+      // ---- weight and gate, and the next chunk's ----
+      auto gated = [&](float v, int j, float gz) { return v * bars.norm_w[half * 16 + j] * silu_fast(gz); };
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float2 gz;
+        if constexpr (sizeof(T) == 2) {
+          const uint32_t w[4] = {z[j / 4].x, z[j / 4].y, z[j / 4].z, z[j / 4].w};
+          gz = unpack2<true>(w[j & 3]);
+        } else {
+          gz = j & 1 ? make_float2(__uint_as_float(z[j / 2].z), __uint_as_float(z[j / 2].w))
+                     : make_float2(__uint_as_float(z[j / 2].x), __uint_as_float(z[j / 2].y));
+        }
+        o[j] = make_float2(gated(o[j].x, 2 * j, gz.x), gated(o[j].y, 2 * j + 1, gz.y));
+      }
+      const bool real = left > 0;
+      if (c + 1 < chunks) {
+        left -= kChunk;
+        gw += (int64_t)a.H * kChunk;
+        gate += (int64_t)kChunk * a.gate_stride;
+        g_t = *gw;
+        load_gate();
+      }
+      // ---- unit norm over the columns of all CTAs ----
+      ok = dc_wait_warp(&bars.norm[ph], (c >> 1) & 1, bars);
+      if (!ok) break;
+      ss = 0.f;
+      for (int r = 0; r < 2 * VT; ++r) ss += bars.part[ph][r][t];
+      const float inv = 1.0f / sqrtf(ss / (float)a.Dv + a.eps);
+      if (real) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = __fmul2_rn(o[j], make_float2(inv, inv));
+        if constexpr (sizeof(T) == 2) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<uint4*>(out + 8 * j) =
+                make_uint4(pack2<true>(o[4 * j].x, o[4 * j].y), pack2<true>(o[4 * j + 1].x, o[4 * j + 1].y),
+                           pack2<true>(o[4 * j + 2].x, o[4 * j + 2].y), pack2<true>(o[4 * j + 3].x, o[4 * j + 3].y));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(out + 4 * j) = make_float4(o[2 * j].x, o[2 * j].y, o[2 * j + 1].x, o[2 * j + 1].y);
+        }
+      }
+      out += (int64_t)kChunk * a.out_stride;
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (VT > 1) cluster_sync_all();          // nobody leaves while its sums may still be written
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+struct ChunkPlan {
+  int windows, per_seq, slots, compact;
+  size_t kq, cp, dots, gw, carry, bytes;
+};
+
+// Images take 116 KB per chunk and key head and 72 KB per chunk and head (heads of 128): 0.27 GB per 4096 tokens of 16 / 32
+// heads.  Above `kMost` the portions are taken in windows of chunks, the state carried between the launches.
+constexpr size_t kMost = (size_t)640 << 20;
+
+ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
+  ChunkPlan p{};
+  const size_t kq = (size_t)G * kParts * (D / 64) * kPanel, cp = (size_t)H * kParts * (D + kChunk) * 128;
+  const size_t dots = (size_t)G * kUnits * 256 * sizeof(float), gw = (size_t)H * kChunk * sizeof(float);
+  const int64_t all = tokens / kChunk + B;      // t0 / 64 + b + c is below this
+  p.per_seq = cdiv(max_new, kChunk);
+  p.compact = 1;
+  p.windows = 1;
+  int64_t slots = all;
+  if ((size_t)all * (kq + cp + dots + gw) > kMost) {
+    const int64_t most = (int64_t)(kMost / (kq + cp + dots + gw));
+    p.per_seq = (int)std::max<int64_t>(1, std::min<int64_t>(most / B, p.per_seq));
+    p.compact = 0;
+    p.windows = cdiv(cdiv(max_new, kChunk), p.per_seq);
+    slots = (int64_t)p.per_seq * B;
+  }
+  p.slots = (int)slots;
+  p.kq = 0;
+  p.cp = p.kq + slots * kq;
+  p.dots = p.cp + slots * cp;
+  p.gw = p.dots + slots * dots;
+  p.carry = p.gw + slots * gw;
+  p.bytes = p.carry + (p.windows > 1 ? (size_t)B * H * Dv * D * sizeof(float) : 0);
+  return p;
+}
+
+template <typename T, int D>
+int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) {
+  static std::atomic<uint64_t> attr_r{0}, attr_k{0}, attr_c{0};
+  constexpr size_t smem_r = (size_t)kParts * (D / 64) * kPanel + 1024, smem_k = CoefSmem<D>::total + 1024,
+                   smem_c = ChunkSmem<D>::total + 1024;
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_rows_kernel<D>, (int)smem_r, attr_r));
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_coef_kernel<T, D>, (int)smem_k, attr_k));
+  CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_chunk_kernel<T, D>, (int)smem_c, attr_c));
+  const int VT = a.Dv / kCols;
+  for (int w = 0; w < p.windows; ++w) {
+    a.first = w * p.per_seq;
+    delta_rows_kernel<D><<<dim3(p.per_seq, a.G, B), kPrepThreads, smem_r, st>>>(a);
+    delta_coef_kernel<T, D><<<dim3(p.per_seq, a.H, B), kPrepThreads, smem_k, st>>>(a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.H * VT, B);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = smem_c;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = VT;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = VT > 1 ? 1 : 0;
+    CVLLM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, delta_chunk_kernel<T, D>, a));
+  }
+  CVLLM_CHECK_LAUNCHES(3 * p.windows);
+  return CVLLM_OK;
+}
+
+}  // namespace
+}  // namespace cvllm
+
+using namespace cvllm;
+
+extern "C" size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
+  if (tokens <= 0 || B <= 0 || max_new <= 0 || H <= 0 || G <= 0) return 0;
+  if (test_options().gla_layout.load() > 0 || max_new < kChunk) return 0;
+  if ((D != 64 && D != 128) || Dv <= 0 || Dv % kCols != 0 || Dv > 8 * kCols || H % G != 0) return 0;
+  return chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
+}
+
+extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* proj, int64_t proj_stride, int b_off,
+                                       int a_off, const float* A_log, const float* dt_bias, float* state, const void* gate,
+                                       int64_t gate_stride, int gate_off, const float* norm_w, int norm_head_stride, float eps,
+                                       const int32_t* cu_seqlens_q, const int32_t* seq_start, const int32_t* batch_mapping,
+                                       int64_t tokens, int B, int max_new, void* out, int64_t out_stride, int H, int G, int D,
+                                       int Dv, int reserved_slot, int dtype, void* workspace, size_t workspace_bytes,
+                                       cvllm_stream_t stream) {
+  drop_stale_error();
+  CVLLM_CHECK_ARG(tokens >= 0 && B >= 0 && max_new >= 0 && H > 0 && G > 0 && H % G == 0 && D > 0 && Dv > 0);
+  if (B == 0 || max_new == 0 || tokens == 0) return CVLLM_OK;
+  CVLLM_CHECK_ARG(qkv && proj && A_log && dt_bias && state && gate && norm_w && cu_seqlens_q && seq_start && batch_mapping &&
+                  out && workspace && (dtype == CVLLM_BF16 || dtype == CVLLM_F32));
+  CVLLM_CHECK_SUPPORTED((D == 64 || D == 128) && Dv % kCols == 0 && Dv <= 8 * kCols && H <= 65535 && B <= 65535 &&
+                        tokens / kChunk + B < (1 << 24));
+  const int64_t E = dtype == CVLLM_BF16 ? 8 : 4;
+  CVLLM_CHECK_ALIGN(aligned16(qkv) && qkv_stride % 4 == 0 && aligned16(out) && out_stride % E == 0 && aligned16(gate) &&
+                    gate_stride % E == 0 && gate_off % E == 0 && aligned16(workspace));
+  const ChunkPlan p = chunk_plan(tokens, B, max_new, H, G, D, Dv);
+  if (workspace_bytes < p.bytes) {
+    set_last_error("workspace too small for cvllm_delta_rule_chunks");
+    return CVLLM_E_WORKSPACE;
+  }
+  unsigned char* ws = static_cast<unsigned char*>(workspace);
+  DeltaChunkArgs a{qkv, qkv_stride, proj_stride, gate_stride, out_stride, proj, gate, b_off, a_off, gate_off, A_log, dt_bias, norm_w,
+                   norm_head_stride, eps, state, out, H, G, Dv, reserved_slot, {cu_seqlens_q, seq_start, nullptr, batch_mapping},
+                   0, p.per_seq, p.compact, ws + p.kq, ws + p.cp,
+                   reinterpret_cast<float*>(ws + p.dots), reinterpret_cast<float*>(ws + p.gw),
+                   reinterpret_cast<float*>(ws + p.carry)};
+  auto st = static_cast<cudaStream_t>(stream);
+  if (dtype == CVLLM_BF16)
+    return D == 128 ? launch_chunks<__nv_bfloat16, 128>(a, p, B, st) : launch_chunks<__nv_bfloat16, 64>(a, p, B, st);
+  return D == 128 ? launch_chunks<float, 128>(a, p, B, st) : launch_chunks<float, 64>(a, p, B, st);
+}
+
+extern "C" int cvllm_delta_chunk_aborts(int* count) {
+  CVLLM_CHECK_ARG(count);
+  CVLLM_CHECK_CUDA(cudaMemcpyFromSymbol(count, g_delta_chunk_aborts, sizeof(int)));
+  return CVLLM_OK;
+}

@@ -27,46 +27,10 @@
 // Recurrence kernels: a cluster of one to eight CTAs per (head, sequence), the state in registers; see below.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "recur_common.cuh"
 
 namespace cvllm {
 namespace {
-
-template <typename T>
-__device__ __forceinline__ float to_f(T v);
-template <>
-__device__ __forceinline__ float to_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T>
-__device__ __forceinline__ T from_f(float v);
-template <>
-__device__ __forceinline__ float from_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
-__device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
-
-struct StepGeom {
-  const int32_t* cu_q;        // [B + 1] or NULL
-  const int32_t* seq_start;   // [B] (with cu_q)
-  const int32_t* positions;   // [B] (without cu_q)
-  const int32_t* slots;       // [B]
-};
-
-__device__ __forceinline__ void portion(const StepGeom& g, int b, int& t0, int& n_new, int& start) {
-  if (g.cu_q) {
-    t0 = g.cu_q[b];
-    n_new = g.cu_q[b + 1] - t0;
-    start = g.seq_start[b];
-  } else {
-    t0 = b;
-    n_new = 1;
-    start = g.positions[b];
-  }
-}
 
 // ---------------------------------------------------------------------------------------------------------
 // Token shift.  grid (token tiles, B), 256 threads over the width.

@@ -786,6 +786,19 @@ int cvllm_delta_rule(const float* qkv, int64_t qkv_stride, const void* proj, int
                      int max_new, void* out, int64_t out_stride, int H, int G, int D, int Dv, int reserved_slot,
                      int dtype, cvllm_stream_t stream);
 
+/* The same portions in chunks of 64 tokens on the tensor cores, operands in three bfloat16 parts (D 64 or 128, Dv a
+ * multiple of 32 up to 256; qkv, gate, out and workspace on 16 bytes, rows in multiples of 16 bytes).  `tokens`: rows of qkv,
+ * cu_seqlens_q[B] at most.  The workspace size is 0 where cvllm_delta_rule is the one to call (other sizes, short portions). */
+size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv);
+int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* proj, int64_t proj_stride, int b_off, int a_off,
+                            const float* A_log, const float* dt_bias, float* state, const void* gate, int64_t gate_stride,
+                            int gate_off, const float* norm_w, int norm_head_stride, float eps, const int32_t* cu_seqlens_q,
+                            const int32_t* seq_start, const int32_t* batch_mapping, int64_t tokens, int B, int max_new, void* out,
+                            int64_t out_stride, int H, int G, int D, int Dv, int reserved_slot, int dtype, void* workspace,
+                            size_t workspace_bytes, cvllm_stream_t stream);
+/* CTAs of its kernel that gave up a wait since the library was loaded (0 in sound operation). */
+int cvllm_delta_chunk_aborts(int* count);
+
 /* wkv: r, k, v, w_raw rows of H * D numbers (model type); w = exp(-exp(w_raw + w0)) per head and key channel;
  *   o = (S + diag(bonus_h) k v^T)^T r;  S <- diag(w) S + k v^T.   Dv = D. */
 int cvllm_wkv_scan(const void* r, int64_t r_stride, const void* k, int64_t k_stride, const void* v, int64_t v_stride,
