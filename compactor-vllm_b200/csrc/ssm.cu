@@ -14,45 +14,12 @@
 // Geometry of a step: cu_q [B + 1] token offsets and seq_start [B] first positions of the portions, batch_mapping [B]
 // slots; cu_q == NULL means one token per sequence at positions[b] (decode steps, CUDA-graph replays).
 // Everything but the stored projections is fp32.
-#include "common.cuh"
+#include <type_traits>
+
+#include "recur_common.cuh"
 
 namespace cvllm {
 namespace {
-
-template <typename T>
-__device__ __forceinline__ float to_f(T v);
-template <>
-__device__ __forceinline__ float to_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T>
-__device__ __forceinline__ T from_f(float v);
-template <>
-__device__ __forceinline__ float from_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
-
-struct StepGeom {
-  const int32_t* cu_q;        // [B + 1] or NULL
-  const int32_t* seq_start;   // [B] (with cu_q)
-  const int32_t* positions;   // [B] (without cu_q)
-  const int32_t* slots;       // [B]
-};
-
-__device__ __forceinline__ void portion(const StepGeom& g, int b, int& t0, int& n_new, int& start) {
-  if (g.cu_q) {
-    t0 = g.cu_q[b];
-    n_new = g.cu_q[b + 1] - t0;
-    start = g.seq_start[b];
-  } else {
-    t0 = b;
-    n_new = 1;
-    start = g.positions[b];
-  }
-}
 
 constexpr int kMaxTaps = 16;
 constexpr int kConvTokens = 8;   // tokens per CTA of the convolution
@@ -140,6 +107,95 @@ __global__ void __launch_bounds__(128) causal_conv_run_kernel(const T* __restric
     out[(int64_t)(t0 + j) * o_stride + ch] = from_f<TO>(MODE == 0 ? silu_f(acc) : acc);
 #pragma unroll
     for (int k = 0; k < TAPS - 1; ++k) win[k] = win[k + 1];
+  }
+}
+
+// The same with four neighbouring channels per thread (rows of 16-bit inputs in 8-byte, of fp32 ones in 16-byte pieces; outputs
+// likewise) and four tokens' rows loaded before the first is used.  An output is 4 multiply-adds and a silu: with one channel
+// per thread, a row at a time and a division's branch per silu, 4096 tokens of 8192 channels took 88 us where their bytes (0.2
+// GB) take 31.  grid (token runs, B, channel tiles of 512), 128 threads.
+template <typename T>
+struct Four {   // four numbers of type T as they lie in memory
+  using raw = typename std::conditional<sizeof(T) == 2, uint2, uint4>::type;
+  __device__ static __forceinline__ raw zero() {
+    raw r;
+    if constexpr (sizeof(T) == 2) r = make_uint2(0, 0);
+    else r = make_uint4(0, 0, 0, 0);
+    return r;
+  }
+  __device__ static __forceinline__ void get(const raw& r, float (&v)[4]) {
+    if constexpr (sizeof(T) == 2) {
+      const float2 a = unpack2<true>(r.x), b = unpack2<true>(r.y);
+      v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+    } else {
+      v[0] = __uint_as_float(r.x), v[1] = __uint_as_float(r.y), v[2] = __uint_as_float(r.z), v[3] = __uint_as_float(r.w);
+    }
+  }
+  __device__ static __forceinline__ raw put(const float (&v)[4]) {
+    raw r;
+    if constexpr (sizeof(T) == 2) r = make_uint2(pack2<true>(v[0], v[1]), pack2<true>(v[2], v[3]));
+    else r = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+    return r;
+  }
+};
+
+template <typename T, typename TO, int TAPS, int MODE>
+__global__ void __launch_bounds__(128) causal_conv_quads_kernel(const T* __restrict__ proj, int64_t p_stride, int x_off,
+                                                                int C, const float* __restrict__ w,
+                                                                const float* __restrict__ bias,
+                                                                const T* __restrict__ conv_state, StepGeom g,
+                                                                TO* __restrict__ out, int64_t o_stride) {
+  using In = typename Four<T>::raw;
+  using Out = typename Four<TO>::raw;
+  const int b = blockIdx.y;
+  int t0, n_new, start;
+  portion(g, b, t0, n_new, start);
+  const int j0 = blockIdx.x * kConvRun;
+  if (j0 >= n_new) return;
+  const int ch = (blockIdx.z * 128 + threadIdx.x) * 4;
+  if (ch >= C) return;
+  const int slot = g.slots[b];
+  float wk[4][TAPS], bv[4], win[TAPS][4];   // win[k] = inputs at j - (TAPS - 1 - k)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) wk[i][k] = w[(int64_t)(ch + i) * TAPS + k];
+    bv[i] = bias ? bias[ch + i] : 0.f;
+  }
+  const T* st = conv_state + (int64_t)slot * (TAPS - 1) * C + ch;
+  const T* in = proj + (int64_t)t0 * p_stride + x_off + ch;
+#pragma unroll
+  for (int k = 0; k < TAPS - 1; ++k) {
+    const int src = j0 - (TAPS - 1 - k);
+    In r = Four<T>::zero();
+    if (src >= 0) r = *reinterpret_cast<const In*>(in + (int64_t)src * p_stride);
+    else if (start + src >= 0) r = *reinterpret_cast<const In*>(st + (int64_t)(TAPS - 1 + src) * C);
+    Four<T>::get(r, win[k]);
+  }
+  const int j1 = min(j0 + kConvRun, n_new);
+  for (int j = j0; j < j1; j += 4) {
+    In row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = j + u < j1 ? *reinterpret_cast<const In*>(in + (int64_t)(j + u) * p_stride) : Four<T>::zero();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (j + u >= j1) break;
+      Four<T>::get(row[u], win[TAPS - 1]);
+      float y[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float acc = bv[i];
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) acc = fmaf(wk[i][k], win[k][i], acc);
+        if (MODE == 1) acc += win[TAPS - 1][i];
+        y[i] = MODE == 0 ? silu_fast(acc) : acc;
+      }
+      *reinterpret_cast<Out*>(out + (int64_t)(t0 + j + u) * o_stride + ch) = Four<TO>::put(y);
+#pragma unroll
+      for (int k = 0; k < TAPS - 1; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) win[k][i] = win[k + 1][i];
+    }
   }
 }
 
@@ -630,7 +686,20 @@ int launch_conv(const void* proj, int64_t proj_stride, int x_off, int channels, 
   const T* in = static_cast<const T*>(proj);
   const T* cs = static_cast<const T*>(conv_state);
   TO* o = static_cast<TO*>(out);
-  if (taps >= 2 && taps <= 4) {
+  // four channels a thread where their pieces are aligned and a portion fills a run (a few tokens are latency: more CTAs)
+  const auto pieces = [](const void* p, int64_t stride, size_t elem) {
+    return reinterpret_cast<uintptr_t>(p) % (4 * elem) == 0 && stride % 4 == 0;
+  };
+  if (taps >= 2 && taps <= 4 && max_new >= kConvRun && channels % 4 == 0 && x_off % 4 == 0 && pieces(proj, proj_stride, sizeof(T)) &&
+      pieces(conv_state, 0, sizeof(T)) && pieces(out, out_stride, sizeof(TO))) {
+    const dim3 qgrid(cdiv(max_new, kConvRun), B, cdiv(channels, 512));
+    if (taps == 2)
+      causal_conv_quads_kernel<T, TO, 2, MODE><<<qgrid, 128, 0, st>>>(in, proj_stride, x_off, channels, weight, bias, cs, g, o, out_stride);
+    else if (taps == 3)
+      causal_conv_quads_kernel<T, TO, 3, MODE><<<qgrid, 128, 0, st>>>(in, proj_stride, x_off, channels, weight, bias, cs, g, o, out_stride);
+    else
+      causal_conv_quads_kernel<T, TO, 4, MODE><<<qgrid, 128, 0, st>>>(in, proj_stride, x_off, channels, weight, bias, cs, g, o, out_stride);
+  } else if (taps >= 2 && taps <= 4) {
     const dim3 rgrid(cdiv(max_new, kConvRun), B, cdiv(channels, 128));
     if (taps == 2)
       causal_conv_run_kernel<T, TO, 2, MODE><<<rgrid, 128, 0, st>>>(in, proj_stride, x_off, channels, weight, bias, cs, g, o, out_stride);
