@@ -126,7 +126,7 @@ class DeltaRuleMixer(nn.Module):
                                                          out.stride(0) * out.element_size(), C * 4)):
             need = lib.cvllm_delta_rule_chunks_workspace_bytes(T, B, max_new, H, G, D, Dv)
         if need:
-            ws = N.workspace(dev, need, "delta_rule_chunks")
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to some hundred MB: given back after the call
             N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], N.ptr(slots), T, B, max_new, N.ptr(out),
                                                 out.stride(0), H, G, D, Dv, RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st),
                     "cvllm_delta_rule_chunks")

@@ -275,7 +275,7 @@ struct CoefSmem {
 // k <= row.
 template <bool CAUSAL>
 __device__ __forceinline__ void block_mul(float (&acc)[4], const float* left, int pitch, const float* right, int row, int col) {
-#pragma unroll
+#pragma unroll 4
   for (int k = 0; k < 16; ++k) {
     const float4 r = *reinterpret_cast<const float4*>(right + k * kPitchX + col);
     const float l = left[row * pitch + k];
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
   if (warp == 0) {      // G_t and w_63t by scans of products, two tokens a lane
     const float ga = s_tok[2 * lane].x, gb = s_tok[2 * lane + 1].x;
     float up = ga * gb, down = up, low = up;
-#pragma unroll
+#pragma unroll 1
     for (int o = 1; o < 32; o <<= 1) {
       const float lo = __shfl_up_sync(0xffffffffu, up, o), hi = __shfl_down_sync(0xffffffffu, down, o);
       const float in = __shfl_down_sync(0xffffffffu, low, o);
@@ -979,8 +979,8 @@ struct ChunkPlan {
 };
 
 // Images take 116 KB per chunk and key head and 72 KB per chunk and head (heads of 128): 0.27 GB per 4096 tokens of 16 / 32
-// heads.  Above `kMost` the portions are taken in windows of chunks, the state carried between the launches.
-constexpr size_t kMost = (size_t)640 << 20;
+// heads.  Above `kMost` the portions are taken in windows of chunks of equal length, the state carried between the launches.
+constexpr size_t kMost = (size_t)320 << 20;
 
 ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
   ChunkPlan p{};
@@ -993,9 +993,10 @@ ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, in
   int64_t slots = all;
   if ((size_t)all * (kq + cp + dots + gw) > kMost) {
     const int64_t most = (int64_t)(kMost / (kq + cp + dots + gw));
-    p.per_seq = (int)std::max<int64_t>(1, std::min<int64_t>(most / B, p.per_seq));
+    const int chunks = p.per_seq, longest = (int)std::max<int64_t>(1, std::min<int64_t>(most / B, chunks));
     p.compact = 0;
-    p.windows = cdiv(cdiv(max_new, kChunk), p.per_seq);
+    p.per_seq = cdiv(chunks, cdiv(chunks, longest));
+    p.windows = cdiv(chunks, p.per_seq);
     slots = (int64_t)p.per_seq * B;
   }
   p.slots = (int)slots;
@@ -1048,7 +1049,8 @@ extern "C" size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B,
   if (tokens <= 0 || B <= 0 || max_new <= 0 || H <= 0 || G <= 0) return 0;
   if (test_options().gla_layout.load() > 0 || max_new < kChunk) return 0;
   if ((D != 64 && D != 128) || Dv <= 0 || Dv % kCols != 0 || Dv > 8 * kCols || H % G != 0) return 0;
-  return chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
+  const size_t bytes = chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
+  return bytes <= 2 * kMost ? bytes : 0;   // a chunk of every sequence would take more: very many portions at once
 }
 
 extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* proj, int64_t proj_stride, int b_off,

@@ -1,0 +1,52 @@
+"""The gated delta rule's portions in chunks of 64 tokens (one tile of the tensor cores), against the recurrence token by token
+in 64 bits: chunks that are full, one token short and one token long, heads that share keys, clusters of one to eight CTAs,
+both types, and portions whose images exceed the workspace's bound and are taken in windows; the convolution in front with
+its rows in four-channel pieces and without.
+
+Tolerances are those of test_gpu_delta_layouts.py: operands in three bfloat16 parts are good to 2^-26, the sums are fp32."""
+import pytest
+import torch
+
+from test_gpu_delta_layouts import recurrence, setup
+
+pytestmark = pytest.mark.gpu
+
+
+def check(size, lens, starts, dtype, seed=5, odd_rows=False):
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context, set_context
+
+    m, state, cols, ctx = setup(*size, lens, starts, dtype, seed)
+    if odd_rows:       # a view whose rows do not start on 16 bytes: the kernels of the shorter portions
+        wide = torch.zeros(cols.shape[0], cols.shape[1] + 1, dtype=dtype, device=cols.device)
+        wide[:, 1:] = cols
+        cols = wide[:, 1:]
+    else:
+        heads, kv, dim, vdim = size
+        assert N.lib().cvllm_delta_rule_chunks_workspace_bytes(sum(lens), len(lens), max(lens), heads, kv, dim, vdim) > 0
+    want, want_state = recurrence(m, state, cols, lens, starts)
+    untouched = state.matrix_state[0].clone()
+    set_context(**ctx)
+    try:
+        got = m(None, cols, state).double()
+    finally:
+        reset_context()
+    err = lambda x, y: ((x - y).norm() / y.norm()).item()
+    assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
+    assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5
+    assert torch.equal(state.matrix_state[0], untouched)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens, starts", [([64], [0]), ([65, 1, 128, 63], [7, 0, 0, 3]), ([127, 200], [0, 9])])
+@pytest.mark.parametrize("size", [(2, 1, 128, 128), (4, 2, 64, 64), (3, 1, 128, 32), (2, 2, 64, 96), (1, 1, 128, 256)], ids=str)
+def test_chunks(size, lens, starts, dtype):
+    check(size, lens, starts, dtype)
+
+
+def test_rows_off_the_grid():
+    check((2, 1, 128, 128), [130, 70], [0, 4], torch.float32, odd_rows=True)
+
+
+def test_windows():
+    check((32, 32, 128, 128), [7000, 300], [0, 11], torch.bfloat16)
