@@ -71,7 +71,7 @@ uint64_t cvllm_launch_count(void);
  *                            rows wherever it serves (portions and decode)
  *   "ssm_segment" n          tokens per segment of cvllm_ssm_scan (0 = the product's choice; tests use short segments)
  *   "gla_layout" n           100 * CTAs per (head, sequence) + columns per thread of cvllm_gla_scan and of the portions of
- *                            cvllm_delta_rule (0 = chosen per step)
+ *                            cvllm_delta_rule (0 = chosen per step; < 0: cvllm_delta_rule_chunks for portions of any length)
  *   "select_passes" 1|0      cvllm_select_store_topk: the chain of launches also where one cluster per sequence would do
  *   "grs_debug_host_ptr" p   pinned host buffer (64 words per CTA) for cvllm_gemm_allreduce's timeout records
  * Returns CVLLM_E_ARG for an unknown name. */

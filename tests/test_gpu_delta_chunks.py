@@ -7,6 +7,7 @@ Tolerances are those of test_gpu_delta_layouts.py: operands in three bfloat16 pa
 import pytest
 import torch
 
+import test_gpu_delta_layouts as layouts
 from test_gpu_delta_layouts import recurrence, setup
 
 pytestmark = pytest.mark.gpu
@@ -17,6 +18,7 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
     from compactor_vllm.utils.context import reset_context, set_context
 
     m, state, cols, ctx = setup(*size, lens, starts, dtype, seed)
+    N.set_test_option("gla_layout", -1)       # chunks whatever the length
     if odd_rows:       # a view whose rows do not start on 16 bytes: the kernels of the shorter portions
         wide = torch.zeros(cols.shape[0], cols.shape[1] + 1, dtype=dtype, device=cols.device)
         wide[:, 1:] = cols
@@ -30,6 +32,7 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
     try:
         got = m(None, cols, state).double()
     finally:
+        N.set_test_option("gla_layout", 0)
         reset_context()
     err = lambda x, y: ((x - y).norm() / y.norm()).item()
     assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
@@ -46,6 +49,19 @@ def test_chunks(size, lens, starts, dtype):
 
 def test_rows_off_the_grid():
     check((2, 1, 128, 128), [130, 70], [0, 4], torch.float32, odd_rows=True)
+
+
+@pytest.mark.parametrize("at", [1, 15, 16, 34, 63, 64, 69])
+def test_what_is_not_finite_stays_behind_its_token(at):
+    layouts.test_what_is_not_finite_stays_behind_its_token(at, -1)
+
+
+def test_the_rule():
+    """Short portions and batches of mostly short ones are the other kernel's."""
+    from compactor_vllm import _native as N
+
+    need = lambda *a: N.lib().cvllm_delta_rule_chunks_workspace_bytes(*a, 16, 8, 128, 128)
+    assert need(128, 1, 128) > 0 and need(127, 1, 127) == 0 and need(191, 2, 128) == 0 and need(192, 2, 128) > 0
 
 
 def test_windows():
