@@ -1047,7 +1047,12 @@ using namespace cvllm;
 
 extern "C" size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
   if (tokens <= 0 || B <= 0 || max_new <= 0 || H <= 0 || G <= 0) return 0;
-  if (test_options().gla_layout.load() > 0 || max_new < kChunk) return 0;
+  // From where it is faster: the chunks' three launches take 35 - 45 us for 64 tokens, as long as the kernel of blocks of four takes
+  // for 90 (one portion of 16 or 32 heads of 64 or 128: 44 / 47 us at 64 tokens, 57 / 53 at 100, 60 / 51 at 128, 162 / 94 at
+  // 512, the blocks' time first), and every sequence fills whole chunks (7 single tokens and a portion of 90: 95 / 121 us; 300, 200,
+  // 100, 50, 25 and 12 tokens: 186 / 162).  Test option gla_layout: > 0 the other kernel, < 0 chunks.
+  const int forced = test_options().gla_layout.load();
+  if (forced > 0 || (forced == 0 && (max_new < 2 * kChunk || tokens < 96 * (int64_t)B))) return 0;
   if ((D != 64 && D != 128) || Dv <= 0 || Dv % kCols != 0 || Dv > 8 * kCols || H % G != 0) return 0;
   const size_t bytes = chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
   return bytes <= 2 * kMost ? bytes : 0;   // a chunk of every sequence would take more: very many portions at once
