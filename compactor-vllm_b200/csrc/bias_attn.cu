@@ -710,7 +710,7 @@ __device__ __forceinline__ void store8<float>(float* p, const float* v) {
 // LPR lanes (a power of two, 8 elements each) share a head row, so a warp takes 32 / LPR rows at once and a CTA
 // 4 * 32 / LPR; grid = (groups of TOKS tokens, row groups): a decode step's few tokens still spread over many CTAs.  A lane
 // keeps its piece of the row in registers between the sum of squares and the scaled write; TOKS tokens' pieces are loaded
-// before the first is used.  With TOKS > 1 the cache length of a slot is raised by the last token of an ascending run of its
+// before the first is used.  Above 64 tokens the cache length of a slot is raised by the last token of an ascending run of its
 // positions alone: a portion's tokens all hit the same few words (4096 tokens of 32 + 8 + 8 heads of 128: 38 us with an atomic per token
 // and a token per CTA, 32 us now, cold; the bytes take 15).
 template <typename T, int TOKS>
@@ -747,9 +747,11 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
     __syncthreads();
   }
   const float* w = (norm & 1) && !is_v ? (is_q ? q_w : k_w) : nullptr;
-  float wr[8];
+  float wr[TOKS > 1 ? 8 : 1];   // one token: read where they are used
+  if constexpr (TOKS > 1) {
 #pragma unroll
-  for (int e = 0; e < 8; ++e) wr[e] = w && mine ? w[cb + e] : 1.f;
+    for (int e = 0; e < 8; ++e) wr[e] = w && mine ? w[cb + e] : 1.f;
+  }
 #pragma unroll
   for (int u = 0; u < TOKS; ++u) {
     const int t = first + u;
@@ -774,7 +776,10 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
     if ((is_q || is_k) && mine) {
       const float inv = (norm & 1) ? 1.0f / sqrtf(ss / (float)D + eps) : 1.0f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[u][e] = x[u][e] * inv * wr[e];
+      for (int e = 0; e < 8; ++e) {
+        if constexpr (TOKS > 1) x[u][e] = x[u][e] * inv * wr[e];
+        else x[u][e] = w ? x[u][e] * inv * w[cb + e] : x[u][e] * inv;
+      }
       T* dst = is_q ? q_out + ((int64_t)t * H + r) * D : k_cache + cache_row(c, slot[u], r - H, pos[u]) * D;
       store8<T>(dst + cb, x[u]);
     }
@@ -789,7 +794,7 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
         store8<T>(v_cache + cache_row(c, slot[u], g, pos[u]) * Dv + cb, x[u]);
       }
       if (cb == 0 && bh_lens) {
-        const bool more = TOKS > 1 && t + 1 < tokens && token_slot[t + 1] == slot[u] && positions[t + 1] > pos[u];
+        const bool more = tokens > 64 && t + 1 < tokens && token_slot[t + 1] == slot[u] && positions[t + 1] > pos[u];
         if (!more) atomicMax(bh_lens + slot[u] * G + g, pos[u] + 1);
       }
     }
@@ -1279,8 +1284,9 @@ static int rope_qknorm_store_impl(const double* inv_freq, int rot_dims, int norm
     while (lpr * 8 < (D > Dv ? D : Dv)) lpr <<= 1;
     const int row_groups = cdiv(H + 2 * G, 4 * (32 / lpr));
     CVLLM_CHECK_SUPPORTED(row_groups <= 65535);
-    // four tokens a CTA from where that still leaves every SM eight CTAs
-    const bool fours = (int64_t)T * row_groups >= 32 * (int64_t)sm_count() && 4 * rsmem <= 32 * 1024;
+    // four tokens a CTA from where that still leaves every SM 32 CTAs (4096 tokens of 48 rows of 128: 165.4 -> 160.4 us with the
+    // attention behind; 3748 of 32 rows of 64, a third of that work, 76.5 us with four and 74.8 with one)
+    const bool fours = (int64_t)T * row_groups >= 128 * (int64_t)sm_count() && 4 * rsmem <= 32 * 1024;
     const dim3 grid(fours ? cdiv(T, 4) : T, row_groups);
 #define CVLLM_QKNORM(TT, KK)                                                                                                    \
   qknorm_store_vec_kernel<TT, KK><<<grid, 128, KK * rsmem, st>>>(                                                               \
