@@ -14,7 +14,10 @@
 // 2^-26 of the value), every product takes the six pairs of parts down to 2^-18, and pairs of one magnitude share an
 // accumulator: with the three parts of the right operand side by side in N, the left operand's first part meets all three
 // parts, its second part the first two (32 accumulator columns further on) and its third part the first.  Three products
-// of 96, 64 and 32 columns read the left operand three times instead of six, and the three sums are added smallest first.
+// of 96, 64 and 32 columns read the left operand three times instead of six, and the three sums are added smallest first.  The
+// tensor pipe truncates its sums, which with keys that share a direction is a bias: the largest sum of [K; Q] S has four
+// accumulators of a quarter of the channels each (one accumulator: twice the state's error behind a last chunk of few tokens),
+// and the coefficients are 64-bit (delta_coef_kernel).
 //
 // A chunk's images (operands as they lie in shared memory, 128-byte swizzle) are written once by the first kernels and copied
 // by untiled bulk copies.
@@ -72,7 +75,7 @@ struct DeltaChunkArgs {
   int first, per_seq, compact;
   unsigned char* kq;           // [slots, G, parts, D / 64, panel]: rows 0 .. 63 k, 64 .. 127 q
   unsigned char* cp;           // [slots, H, parts, D + 64 rows of 128 bytes]: rows 0 .. D - 1 C, then P T
-  float* dots;                 // [slots, G, 2, 10, 16, 16]: lower blocks of K K^T and Q K^T
+  double* dots;                // [slots, G, 2, 10, 16, 16]: lower blocks of K K^T and Q K^T
   float* gw;                   // [slots, H, 64]: G_t
   float* carry;                // [B, H, Dv, D] between launches
   __device__ __forceinline__ int slot(int b, int t0, int c) const { return compact ? t0 / kChunk + b + c : b * per_seq + c - first; }
@@ -99,6 +102,16 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
 __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// A number of a unit row (|x| <= 1) as x0 + 2^-12 x1 + 2^-24 x2, each a float16: x0 a multiple of 2^-11, so that a sum of such
+// products (multiples of 2^-22, at most 1 for two unit rows) is exact in fp32; x1 and x2 what is left, 11 bits each.
+__device__ __forceinline__ void slice3(float2 x, uint32_t& x0, uint32_t& x1, uint32_t& x2) {
+  const float2 near0 = make_float2((x.x + 6144.f) - 6144.f, (x.y + 6144.f) - 6144.f);   // 6144: last place 2^-11
+  x0 = pack2<false>(near0.x, near0.y);
+  x = make_float2((x.x - near0.x) * 4096.f, (x.y - near0.y) * 4096.f);
+  x1 = pack2<false>(x.x, x.y);
+  const float2 h = unpack2<false>(x1);
+  x2 = pack2<false>((x.x - h.x) * 4096.f, (x.y - h.y) * 4096.f);
 }
 // acc of two 8-column tiles (i: which) += A . B on three parts each; the largest pair apart from the others
 __device__ __forceinline__ void mma_parts(float (&big)[4], float (&rest)[4], const uint32_t (&fa)[3][4], const uint32_t (&fb)[3][4],
@@ -133,7 +146,9 @@ __device__ __forceinline__ int panel_at(int row, int piece) { return row * 128 +
 
 // ---------------------------------------------------------------------------------------------------------
 // Unit rows and their products.  grid (chunks, G, B), 256 threads: k and q rows to unit length and into parts, the image out
-// by a bulk copy; K K^T and Q K^T (lower blocks of 16) from the parts on mma.sync.
+// by a bulk copy; K K^T and Q K^T (lower blocks of 16) on mma.sync, from float16 slices that take the image's place.  The largest
+// sum is exact and the others are 2^-12 and 2^-24 of it, so a product is good to 2^-32: 63 of them enter every u_t, and keys that
+// share a direction (products near 1) make the sum as large as the values.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kPrepThreads = 256;
 constexpr int kUnits = 20;    // lower blocks of 16 x 16 of two matrices
@@ -202,34 +217,41 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const Delta
         if (at >= left) from |= o, at -= left;
       }
       const float inv = __shfl_sync(0xffffffffu, inv_mine, from, LR);
-      uint32_t p[kParts][2];
-      split3(x[i].x * inv, x[i].y * inv, p[0][0], p[1][0], p[2][0]);
-      split3(x[i].z * inv, x[i].w * inv, p[0][1], p[1][1], p[2][1]);
-      const int t = (i % kPasses) * (8 * RW) + warp * RW + sub, row = i < kPasses ? kChunk + t : t;
-#pragma unroll
-      for (int e = 0; e < kParts; ++e)
-        *reinterpret_cast<uint2*>(img + e * kPartBytes + off0 + panel_at(row, piece)) = make_uint2(p[e][0], p[e][1]);
+      x[i] = make_float4(x[i].x * inv, x[i].y * inv, x[i].z * inv, x[i].w * inv);
     }
+    auto put = [&](auto&& cut) {
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        uint32_t p[kParts][2];
+        cut(make_float2(x[i].x, x[i].y), p[0][0], p[1][0], p[2][0]);
+        cut(make_float2(x[i].z, x[i].w), p[0][1], p[1][1], p[2][1]);
+        const int t = (i % kPasses) * (8 * RW) + warp * RW + sub, row = i < kPasses ? kChunk + t : t;
+#pragma unroll
+        for (int e = 0; e < kParts; ++e)
+          *reinterpret_cast<uint2*>(img + e * kPartBytes + off0 + panel_at(row, piece)) = make_uint2(p[e][0], p[e][1]);
+      }
+    };
+    put([](float2 v, uint32_t& e0, uint32_t& e1, uint32_t& e2) { split3(v, e0, e1, e2); });
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      unsigned char* dst = a.kq + ((int64_t)slot * a.G + grp) * (kParts * kPartBytes);
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(img)),
+                   "r"(kParts * kPartBytes)
+                   : "memory");
+      bulk_commit();
+      bulk_wait_read<0>();
+    }
+    __syncthreads();
+    put([](float2 v, uint32_t& e0, uint32_t& e1, uint32_t& e2) { slice3(v, e0, e1, e2); });
   }
-  fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0) {
-    unsigned char* dst = a.kq + ((int64_t)slot * a.G + grp) * (kParts * kPartBytes);
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(img)),
-                 "r"(kParts * kPartBytes)
-                 : "memory");
-    bulk_commit();
-  }
 
   // ---- K K^T and Q K^T: 20 lower blocks over eight warps ----
   constexpr int kRounds = (kUnits + 7) / 8;
 #pragma unroll 1
   for (int r = 0; r < kRounds; ++r) {
-    float big[2][4], rest[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) big[i][e] = rest[i][e] = 0.f;
+    float acc[3][2][4] = {};     // sums of 1, 2^-12, 2^-24
     const int u = warp + 8 * r;
     if (u < kUnits) {
       int m, mt, nt;
@@ -245,64 +267,96 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const Delta
           ldmatrix4(fa[e], base + e * kPartBytes + (pa >> 3) * kPanel + panel_at(row_a, pa & 7));
           ldmatrix4(fb[e], base + e * kPartBytes + (pb >> 3) * kPanel + panel_at(row_b, pb & 7));
         }
-        mma_parts(big[0], rest[0], fa, fb, 0);
-        mma_parts(big[1], rest[1], fa, fb, 1);
+#pragma unroll
+        for (int ea = 0; ea < kParts; ++ea)
+#pragma unroll
+          for (int eb = 0; eb + ea < kParts; ++eb)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              mma16816<false>(acc[ea + eb][i], fa[ea][0], fa[ea][1], fa[ea][2], fa[ea][3], fb[eb][2 * i], fb[eb][2 * i + 1]);
       }
-      float* dst = a.dots + (((int64_t)slot * a.G + grp) * kUnits + u) * 256;
+      double* dst = a.dots + (((int64_t)slot * a.G + grp) * kUnits + u) * 256;
+      auto sum = [&](int i, int e) { return (double)acc[0][i][e] + 0x1p-12 * ((double)acc[1][i][e] + 0x1p-12 * (double)acc[2][i][e]); };
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int e = 0; e < 2; ++e)
-          *reinterpret_cast<float2*>(dst + ((lane >> 2) + 8 * e) * 16 + i * 8 + (lane & 3) * 2) =
-              make_float2(big[i][2 * e] + rest[i][2 * e], big[i][2 * e + 1] + rest[i][2 * e + 1]);
+          *reinterpret_cast<double2*>(dst + ((lane >> 2) + 8 * e) * 16 + i * 8 + (lane & 3) * 2) =
+              make_double2(sum(i, 2 * e), sum(i, 2 * e + 1));
     }
   }
   if (tid == 0) bulk_wait<0>();
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Coefficients of the chunks.  grid (chunks, H, B), 256 threads: decays; A (beta_t w_ts k_t . k_s, t > s) and P; the inverse X
-// of I + A in blocks of 16 tokens - diagonal blocks by forward substitution, a column per thread, then halves of 32 and of 64
-// from X_21 = -X_22 (A_21 X_11), half a block per warp; C = K^T diag(w_63) X diag(beta) from three parts on mma.sync; and
-// P X diag(beta).  Row t of X and of P X is made of rows up to t alone, by sums that stop at t: what is not finite stays behind
-// its token.
+// Coefficients of the chunks.  grid (chunks, H, B), 256 threads: decays; A (beta_t w_ts k_t . k_s, t > s); the inverse X of
+// I + A in blocks of 16 tokens - diagonal blocks by forward substitution, a column per thread, then halves of 32 and of 64 from
+// X_21 = -X_22 (A_21 X_11); C = K^T diag(w_63) X diag(beta) from three parts on mma.sync; P and P X diag(beta).
+//
+// A, X, P and P X are 64-bit (the products on mma.sync in f64, 64 multiply-adds per cycle and SM, as many as without it): with keys
+// that share a direction their sums cancel, and what 32 bits lose there is two to three times what the kernel of blocks of four
+// loses in all.  Rounded once, into the parts of C and P T.
+//
+// A token whose decay, beta or key is not finite makes itself and all that follow NaN, and no more: its rows of A are left out
+// (a product would carry them to earlier tokens as 0 * NaN), its rows of P T and all of C become NaN.  A query's own row needs
+// no care.
 // ---------------------------------------------------------------------------------------------------------
-constexpr int kPitchX = 68;   // X: rows read four columns at a time
-constexpr int kPitchA = 65;   // the others: sixteen rows' entries of a column at a time
+constexpr int kPitchD = 20;              // numbers per row of a block of 16 x 16: fragment loads without bank conflicts
+constexpr int kBlk = 16 * kPitchD;
 template <int D>
 struct CoefSmem {
   static constexpr int kRow = kChunk * 128;                  // one part's panel of K rows
   static constexpr int k = 0;                                // [parts][D / 64][64 rows], then C's image
-  static constexpr int a = kParts * (D / 64) * kRow;         // A, then the parts of diag(w) T, then P T's image
-  static constexpr int p = a + kParts * kRow;
-  static constexpr int x = p + kChunk * kPitchA * 4;
-  static constexpr int total = x + kChunk * kPitchX * 4;
+  static constexpr int a = kParts * (D / 64) * kRow;         // A, then the parts of diag(w) T, then P, then P T's image
+  static constexpr int x = a + 10 * kBlk * 8;
+  static constexpr int total = x + 10 * kBlk * 8;
 };
+static_assert(kParts * kChunk * 128 <= 10 * kBlk * 8, "the parts fit in A's place");
 
-// acc[4] += (row `row` of `left`, 16 numbers) x (16 rows of `right`, four columns from col).  CAUSAL: number k only where
-// k <= row.
-template <bool CAUSAL>
-__device__ __forceinline__ void block_mul(float (&acc)[4], const float* left, int pitch, const float* right, int row, int col) {
-#pragma unroll 4
-  for (int k = 0; k < 16; ++k) {
-    const float4 r = *reinterpret_cast<const float4*>(right + k * kPitchX + col);
-    const float l = left[row * pitch + k];
-    if (!CAUSAL || k <= row) {
-      acc[0] = fmaf(l, r.x, acc[0]);
-      acc[1] = fmaf(l, r.y, acc[1]);
-      acc[2] = fmaf(l, r.z, acc[2]);
-      acc[3] = fmaf(l, r.w, acc[3]);
-    }
+// lower block (i, j)
+__device__ __forceinline__ int blk_at(int i, int j) { return (i * (i + 1) / 2 + j) * kBlk; }
+
+// acc (16 x 8) += left (16 x 16) . right (16 rows, 8 columns from `right` on)
+__device__ __forceinline__ void block_mul(double (&acc)[4], const double* left, const double* right, int lane) {
+  const double* pa = left + (lane >> 2) * kPitchD + (lane & 3);
+  const double* pb = right + (lane & 3) * kPitchD + (lane >> 2);
+  double fa[8], fb[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    fa[2 * k] = pa[4 * k];
+    fa[2 * k + 1] = pa[8 * kPitchD + 4 * k];
+    fb[k] = pb[4 * k * kPitchD];
   }
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, "
+      "{%0,%1,%2,%3};"
+      : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
+      : "d"(fa[0]), "d"(fa[1]), "d"(fa[2]), "d"(fa[3]), "d"(fa[4]), "d"(fa[5]), "d"(fa[6]), "d"(fa[7]), "d"(fb[0]), "d"(fb[1]),
+        "d"(fb[2]), "d"(fb[3]));
+}
+__device__ __forceinline__ void block_put(double* m, const double (&v)[4], double sign, int lane) {
+  double* p = m + (lane >> 2) * kPitchD + (lane & 3) * 2;
+  *reinterpret_cast<double2*>(p) = make_double2(sign * v[0], sign * v[1]);
+  *reinterpret_cast<double2*>(p + 8 * kPitchD) = make_double2(sign * v[2], sign * v[3]);
+}
+// the three parts of two 64-bit numbers
+__device__ __forceinline__ void split3(double x, double y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack2<true>((float)x, (float)y);
+  const float2 h = unpack2<true>(hi);
+  const float2 r = make_float2((float)(x - (double)h.x), (float)(y - (double)h.y));
+  mid = pack2<true>(r.x, r.y);
+  const float2 m = unpack2<true>(mid);
+  lo = pack2<true>(r.x - m.x, r.y - m.y);
 }
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const DeltaChunkArgs a) {
   using L = CoefSmem<D>;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ float2 s_tok[kChunk];          // decays and betas
+  __shared__ float2 s_tok[kChunk];                    // decays and betas
   __shared__ uint64_t s_bar;
-  __shared__ float s_w[kChunk], s_rest[32]; // products of the decays behind token s: of the chunk's, of the first 32
+  __shared__ double s_pre[kChunk], s_suf[kChunk];     // products of the decays of a token's block up to it, and behind it
+  __shared__ int s_bad;                               // first token that is not finite
   const int b = blockIdx.z, h = blockIdx.y, c = a.first + blockIdx.x, grp = h / (a.H / a.G);
   int t0, n_new, start;
   portion(a.g, b, t0, n_new, start);
@@ -310,168 +364,163 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
   if (n <= 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = a.slot(b, t0, c);
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  float *A = reinterpret_cast<float*>(sm + L::a), *P = reinterpret_cast<float*>(sm + L::p), *X = reinterpret_cast<float*>(sm + L::x);
+  double *A = reinterpret_cast<double*>(sm + L::a), *X = reinterpret_cast<double*>(sm + L::x);
+  const double* dots = a.dots + ((int64_t)slot * a.G + grp) * kUnits * 256;
 
-  float z_decay = 0.f, z_beta = 0.f;
-  if (tid < n) {
-    const T* pr = static_cast<const T*>(a.proj) + (int64_t)(t0 + c * kChunk + tid) * a.proj_stride;
-    z_decay = to_f<T>(pr[a.a_off + h]) + a.dt_bias[h];
-    z_beta = to_f<T>(pr[a.b_off + h]);
-  }
-  const float rate = a.A_log[h];
   if (tid == 0) {       // k's rows, used by the product at the end
     mbar_init(&s_bar, 1);
     mbar_fence_init();
     const unsigned char* kq = a.kq + ((int64_t)slot * a.G + grp) * (kParts * (D / 64) * kPanel);
     mbar_expect_tx(&s_bar, kParts * (D / 64) * L::kRow);
     for (int i = 0; i < kParts * (D / 64); ++i) bulk_load(sm + L::k + i * L::kRow, kq + i * kPanel, L::kRow, &s_bar);
+    s_bad = kChunk;
   }
-  // the dots' blocks to their places in A and P
-  {
-    const float4* src = reinterpret_cast<const float4*>(a.dots + ((int64_t)slot * a.G + grp) * kUnits * 256);
-    float4 x[5];
+  // of the dots: threads 0 .. 63 a column of a diagonal block, the others eight numbers of the blocks below
+  const int dblk = tid >> 4, dcol = tid & 15;
+  auto diag_at = [&](int m) { return dots + (m * 10 + dblk * (dblk + 1) / 2 + dblk) * 256 + dcol; };
+  auto below = [&](int i, int& bi, int& bj, int& t, int& s) {   // number i of this thread
+    const int e = (i * 192 + tid - kChunk), q = e >> 8;         // blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+    bi = q < 1 ? 1 : q < 3 ? 2 : 3;
+    bj = q - (bi * (bi - 1)) / 2;
+    t = (e >> 4) & 15;
+    s = e & 15;
+  };
+  double dot[16];
+  auto load_dots = [&](int m) {
+    if (tid < kChunk) {
 #pragma unroll
-    for (int i = 0; i < 5; ++i) x[i] = src[i * kPrepThreads + tid];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const int e = i * kPrepThreads + tid;     // four numbers each; 64 per block
-      int m, mt, nt;
-      unit_of(e >> 6, m, mt, nt);
-      float* dst = (m ? P : A) + (mt * 16 + ((e >> 2) & 15)) * kPitchA + nt * 16 + (e & 3) * 4;
-      dst[0] = x[i].x;
-      dst[1] = x[i].y;
-      dst[2] = x[i].z;
-      dst[3] = x[i].w;
-    }
-  }
-  if (tid < kChunk)     // missing tokens: decay 1, beta 0
-    s_tok[tid] = tid < n ? make_float2(exp_1ulp(-expf(rate) * softplus_f(z_decay)), sigmoid_f(z_beta)) : make_float2(1.f, 0.f);
-  __syncthreads();
-  if (warp == 0) {      // G_t and w_63t by scans of products, two tokens a lane
-    const float ga = s_tok[2 * lane].x, gb = s_tok[2 * lane + 1].x;
-    float up = ga * gb, down = up, low = up;
-#pragma unroll 1
-    for (int o = 1; o < 32; o <<= 1) {
-      const float lo = __shfl_up_sync(0xffffffffu, up, o), hi = __shfl_down_sync(0xffffffffu, down, o);
-      const float in = __shfl_down_sync(0xffffffffu, low, o);
-      if (lane >= o) up *= lo;
-      if (lane + o < 32) down *= hi;
-      if ((lane & 15) + o < 16) low *= in;
-    }
-    const float before = __shfl_up_sync(0xffffffffu, up, 1), behind = __shfl_down_sync(0xffffffffu, down, 1);
-    const float in = __shfl_down_sync(0xffffffffu, low, 1);
-    const float prev = lane ? before : 1.f, next = lane < 31 ? behind : 1.f, next_low = lane < 15 ? in : 1.f;
-    if (lane < 16) {
-      s_rest[2 * lane] = next_low * gb;
-      s_rest[2 * lane + 1] = next_low;
-    }
-    s_w[2 * lane] = next * gb;
-    s_w[2 * lane + 1] = next;
-    *reinterpret_cast<float2*>(a.gw + ((int64_t)slot * a.H + h) * kChunk + 2 * lane) = make_float2(prev * ga, up);
-  }
-  __syncthreads();
-
-  // ---- A and P in the dots' place: a thread per column and half of it ----
-  {
-    const int s = tid & 63, upper = (tid >> 6) & 1, of_q = tid >> 7;
-    float* m = of_q ? P : A;
-    const int lo = upper ? max(32, s + 1) : s + 1, hi = upper ? kChunk : 32;
-    float w = upper && s < 32 ? s_rest[s] : 1.f;
-#pragma unroll 1
-    for (int t8 = lo & ~7; t8 < hi; t8 += 8) {   // eight at a time: their loads before their stores
-      float x[8];
-      float2 tok[8];
+      for (int t = 0; t < 16; ++t) dot[t] = t >= dcol ? diag_at(m)[t * 16] : 0.0;
+    } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        x[i] = m[(t8 + i) * kPitchA + s];
-        tok[i] = s_tok[t8 + i];
+        int bi, bj, t, s;
+        below(i, bi, bj, t, s);
+        dot[i] = dots[(m * 10 + bi * (bi + 1) / 2 + bj) * 256 + t * 16 + s];
       }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (t8 + i >= lo) {
-          w *= tok[i].x;
-          m[(t8 + i) * kPitchA + s] = x[i] * (of_q ? w : tok[i].y * w);
-        }
     }
+  };
+  load_dots(0);
+  __syncthreads();      // s_bad
+  if (tid < kChunk) {
+    float2 tok = make_float2(1.f, 0.f);     // missing tokens: decay 1, beta 0
+    if (tid < n) {
+      const T* pr = static_cast<const T*>(a.proj) + (int64_t)(t0 + c * kChunk + tid) * a.proj_stride;
+      tok = make_float2(exp_1ulp(-expf(a.A_log[h]) * softplus_f(to_f<T>(pr[a.a_off + h]) + a.dt_bias[h])),
+                        sigmoid_f(to_f<T>(pr[a.b_off + h])));
+    }
+    s_tok[tid] = tok;
+    double own = 0.0;                       // the key's product with itself
+#pragma unroll
+    for (int t = 0; t < 16; ++t)
+      if (t == dcol) own = dot[t];
+    if (!(fabsf(tok.x) + fabsf(tok.y) + fabsf((float)own) < 1e30f)) atomicMin(&s_bad, tid);
+    double up = tok.x, down = tok.x;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const double lo = __shfl_up_sync(0xffffffffu, up, o, 16), hi = __shfl_down_sync(0xffffffffu, down, o, 16);
+      if (dcol >= o) up *= lo;
+      if (dcol + o < 16) down *= hi;
+    }
+    const double behind = __shfl_down_sync(0xffffffffu, down, 1, 16);
+    s_pre[tid] = up;
+    s_suf[tid] = dcol < 15 ? behind : 1.0;
   }
   __syncthreads();
-
-  // ---- X ----
-  if (tid < kChunk) {      // diagonal blocks
-    const int blk = tid >> 4, col = tid & 15;
-    const float* d = A + blk * 16 * kPitchA + blk * 16;
-    float x[16];
+  const int bad = s_bad;
+  auto whole = [&](int i) { return s_pre[i * 16 + 15]; };   // a block's decays
+  // w of the blocks below: behind s, the blocks between, up to t
+  auto below_w = [&](int bi, int bj, int t, int s) {
+    double w = s_suf[bj * 16 + s] * s_pre[bi * 16 + t];
+    for (int i = bj + 1; i < bi; ++i) w *= whole(i);
+    return w;
+  };
+  if (tid < kChunk) {   // G_t, and the diagonal blocks of A and X
+    double g = s_pre[tid];
+    for (int i = 0; i < dblk; ++i) g *= whole(i);
+    a.gw[((int64_t)slot * a.H + h) * kChunk + tid] = (float)g;
+    double* d = A + blk_at(dblk, dblk);
+    double w = 1.0;
+#pragma unroll
+    for (int t = 1; t < 16; ++t)
+      if (t > dcol) {
+        w *= (double)s_tok[dblk * 16 + t].x;
+        d[t * kPitchD + dcol] = dblk * 16 + t < bad ? (double)s_tok[dblk * 16 + t].y * w * dot[t] : 0.0;
+      }
+    __syncwarp();
+    double x[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
-      float acc0 = t == col ? 1.f : 0.f, acc1 = 0.f;
+      double acc0 = t == dcol ? 1.0 : 0.0, acc1 = 0.0;
 #pragma unroll
       for (int s = 0; s < t; ++s) {
-        const float r = d[t * kPitchA + s];
-        if (s & 1) acc1 = fmaf(-r, x[s], acc1);
-        else acc0 = fmaf(-r, x[s], acc0);
+        const double r = d[t * kPitchD + s];
+        if (s & 1) acc1 = fma(-r, x[s], acc1);
+        else acc0 = fma(-r, x[s], acc0);
       }
       x[t] = acc0 + acc1;
+      X[blk_at(dblk, dblk) + t * kPitchD + dcol] = t < dcol ? 0.0 : x[t];
     }
+  } else {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) X[(blk * 16 + t) * kPitchX + blk * 16 + col] = t < col ? 0.f : x[t];
-  }
-  // half a block per warp: a row and four columns a lane
-  const int row = lane >> 1, col = (warp & 1) * 8 + (lane & 1) * 4, q4 = warp >> 1;
-  auto A_at = [&](int i, int j) { return A + i * 16 * kPitchA + j * 16; };
-  auto P_at = [&](int i, int j) { return P + i * 16 * kPitchA + j * 16; };
-  auto X_at = [&](int i, int j) { return X + i * 16 * kPitchX + j * 16; };
-  auto put = [&](float* m, const float (&v)[4], float sign) {
-    *reinterpret_cast<float4*>(m + row * kPitchX + col) = make_float4(sign * v[0], sign * v[1], sign * v[2], sign * v[3]);
-  };
-  __syncthreads();
-  if (q4 < 2) {            // blocks (1, 0) and (3, 2); sums on the way lie in the blocks above the diagonal
-    const int i = 2 * q4 + 1, j = 2 * q4;
-    float acc[4] = {}, res[4] = {};
-    block_mul<false>(acc, A_at(i, j), kPitchA, X_at(j, j), row, col);
-    put(X_at(j, i), acc, -1.f);
-    __syncwarp();
-    block_mul<true>(res, X_at(i, i), kPitchX, X_at(j, i), row, col);
-    put(X_at(i, j), res, 1.f);
-  }
-  __syncthreads();
-  {
-    const int i = 2 + (q4 >> 1), j = q4 & 1;     // blocks (2, 0), (2, 1), (3, 0), (3, 1)
-    float acc[4] = {};
-    if (j == 0) {
-      block_mul<false>(acc, A_at(i, 0), kPitchA, X_at(0, 0), row, col);
-      block_mul<false>(acc, A_at(i, 1), kPitchA, X_at(1, 0), row, col);
-    } else {
-      block_mul<false>(acc, A_at(i, 1), kPitchA, X_at(1, 1), row, col);
+    for (int i = 0; i < 8; ++i) {
+      int bi, bj, t, s;
+      below(i, bi, bj, t, s);
+      A[blk_at(bi, bj) + t * kPitchD + s] =
+          bi * 16 + t < bad ? (double)s_tok[bi * 16 + t].y * below_w(bi, bj, t, s) * dot[i] : 0.0;
     }
-    put(X_at(j, i), acc, -1.f);
-    __syncthreads();
-    float res[4] = {};
-    if (i == 3) block_mul<false>(res, X_at(3, 2), kPitchX, X_at(j, 2), row, col);
-    block_mul<true>(res, X_at(i, i), kPitchX, X_at(j, i), row, col);
-    put(X_at(i, j), res, 1.f);
   }
   __syncthreads();
 
-  // ---- diag(w) X diag(beta) in parts (a later token's beta may be NaN: left out, not multiplied) ----
-  for (int i = tid; i < kChunk * 8; i += kPrepThreads) {
-    const int t = i >> 3, s0 = (i & 7) * 8;
-    const float w = s_w[t];
+  // ---- X below the diagonal: eight columns a warp; sums on the way lie in A's diagonal blocks ----
+  const int half = (warp & 1) * 8, pair = warp >> 1;
+  auto S_at = [&](int i) { return A + blk_at(i, i) + half; };
+  if (pair < 2) {          // blocks (1, 0) and (3, 2)
+    const int i = 2 * pair + 1, j = 2 * pair;
+    double acc[4] = {}, res[4] = {};
+    block_mul(acc, A + blk_at(i, j), X + blk_at(j, j) + half, lane);
+    block_put(S_at(j), acc, -1.0, lane);
+    __syncwarp();
+    block_mul(res, X + blk_at(i, i), S_at(j), lane);
+    block_put(X + blk_at(i, j) + half, res, 1.0, lane);
+  }
+  __syncthreads();
+  if (pair < 2) {          // blocks (2, j) and (3, j)
+    const int j = pair;
+    double s2[4] = {}, s3[4] = {}, x2[4] = {}, x3[4] = {};
+    for (int k = j; k < 2; ++k) {
+      block_mul(s2, A + blk_at(2, k), X + blk_at(k, j) + half, lane);
+      block_mul(s3, A + blk_at(3, k), X + blk_at(k, j) + half, lane);
+    }
+    block_put(S_at(2 * j), s2, -1.0, lane);
+    block_put(S_at(2 * j + 1), s3, -1.0, lane);
+    __syncwarp();
+    block_mul(x2, X + blk_at(2, 2), S_at(2 * j), lane);
+    block_mul(x3, X + blk_at(3, 2), S_at(2 * j), lane);
+    block_mul(x3, X + blk_at(3, 3), S_at(2 * j + 1), lane);
+    block_put(X + blk_at(2, j) + half, x2, 1.0, lane);
+    block_put(X + blk_at(3, j) + half, x3, 1.0, lane);
+  }
+  __syncthreads();
+
+  // ---- diag(w) X diag(beta) in parts: the lower blocks' rows in pieces of eight (the others are not read) ----
+  for (int i = tid; i < 320; i += kPrepThreads) {
+    const int q = i >> 5, bi = q < 1 ? 0 : q < 3 ? 1 : q < 6 ? 2 : 3, bj = q - bi * (bi + 1) / 2, t = (i >> 1) & 15, s0 = (i & 1) * 8;
+    double w = s_suf[bi * 16 + t];
+    for (int k = bi + 1; k < 4; ++k) w *= whole(k);
+    const double2* x = reinterpret_cast<const double2*>(X + blk_at(bi, bj) + t * kPitchD + s0);
     uint32_t p[kParts][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int s = s0 + 2 * q;
-      float2 v = make_float2(0.f, 0.f);
-      if (s <= t) {
-        v = *reinterpret_cast<const float2*>(X + t * kPitchX + s);
-        v.x *= w * s_tok[s].y;
-        v.y = s < t ? v.y * (w * s_tok[s + 1].y) : 0.f;
-      }
-      split3(v, p[0][q], p[1][q], p[2][q]);
+    for (int e = 0; e < 4; ++e) {
+      const double2 v = x[e];
+      const int s = bj * 16 + s0 + 2 * e;
+      split3(v.x * (w * (double)s_tok[s].y), v.y * (w * (double)s_tok[s + 1].y), p[0][e], p[1][e], p[2][e]);
     }
 #pragma unroll
     for (int e = 0; e < kParts; ++e)
-      *reinterpret_cast<uint4*>(sm + L::a + e * L::kRow + panel_at(t, i & 7)) = make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
+      *reinterpret_cast<uint4*>(sm + L::a + e * L::kRow + panel_at(bi * 16 + t, bj * 2 + (i & 1))) =
+          make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
   }
+  load_dots(1);
   __syncthreads();
   {
     uint32_t spins = 0;
@@ -483,14 +532,9 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
       }
   }
 
-  // ---- C: 16 channels a warp, all 64 columns; column block nb has rows of token blocks kb >= nb ----
-  float big[4][2][4], rest[4][2][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) big[i][j][e] = rest[i][j][e] = 0.f;
+  // ---- C: 16 channels a warp, all 64 columns; column block nb has rows of token blocks kb >= nb.  The largest pair's sums
+  // leave the tensor pipe, which truncates, after each 16 tokens ----
+  float big[4][2][4] = {}, rest[4][2][4] = {};
   if (warp < D / 16) {
     const uint32_t kb_at = smem_u32(sm + L::k), tb_at = smem_u32(sm + L::a);
     const int piece_a = 2 * warp + ((lane >> 3) & 1), row_a = (lane & 7) + ((lane >> 4) << 3), row_b = (lane & 7) + (((lane >> 3) & 1) << 3);
@@ -505,13 +549,19 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
         uint32_t fb[kParts][4];
 #pragma unroll
         for (int e = 0; e < kParts; ++e) ldmatrix4_trans(fb[e], tb_at + e * L::kRow + panel_at(kb * 16 + row_b, nb * 2 + (lane >> 4)));
-        mma_parts(big[nb][0], rest[nb][0], fa, fb, 0);
-        mma_parts(big[nb][1], rest[nb][1], fa, fb, 1);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float part[4] = {};
+          mma_parts(part, rest[nb][i], fa, fb, i);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) big[nb][i][e] += part[e];
+        }
       }
     }
   }
-  __syncthreads();   // K and the parts are read: the images take their places
+  __syncthreads();   // K and the parts are read: C's image and P take their places
   if (warp < D / 16) {
+    const float nan = __int_as_float(0x7fc00000);
 #pragma unroll
     for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
@@ -519,38 +569,63 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           uint32_t p[kParts];
-          split3(big[nb][i][2 * e] + rest[nb][i][2 * e], big[nb][i][2 * e + 1] + rest[nb][i][2 * e + 1], p[0], p[1], p[2]);
+          const float u = big[nb][i][2 * e] + rest[nb][i][2 * e], v = big[nb][i][2 * e + 1] + rest[nb][i][2 * e + 1];
+          split3(bad < kChunk ? nan : u, bad < kChunk ? nan : v, p[0], p[1], p[2]);
           const int at = panel_at(warp * 16 + (lane >> 2) + 8 * e, nb * 2 + i) + (lane & 3) * 4;
 #pragma unroll
           for (int q = 0; q < kParts; ++q) *reinterpret_cast<uint32_t*>(sm + L::k + q * D * 128 + at) = p[q];
         }
   }
-  // ---- P X diag(beta): the ten lower blocks, five block products a pair of warps; blocks above the diagonal are zero ----
-  auto put_pt = [&](int i, int j, const float (&acc)[4]) {
-    float v[4];
+  if (tid < kChunk) {
+    double* d = A + blk_at(dblk, dblk);
+    double w = 1.0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = i > j || (i == j && col + q <= row) ? acc[q] * s_tok[j * 16 + col + q].y : 0.f;
-    uint32_t p[kParts][2];
-    split3(v[0], v[1], p[0][0], p[1][0], p[2][0]);
-    split3(v[2], v[3], p[0][1], p[1][1], p[2][1]);
+    for (int t = 0; t < 16; ++t) {
+      if (t > dcol) w *= (double)s_tok[dblk * 16 + t].x;
+      d[t * kPitchD + dcol] = t >= dcol ? w * dot[t] : 0.0;
+    }
+  } else {
 #pragma unroll
-    for (int e = 0; e < kParts; ++e)
-      *reinterpret_cast<uint2*>(sm + L::a + e * L::kRow + panel_at(i * 16 + row, (j * 16 + col) >> 3) + (col & 4) * 2) =
-          make_uint2(p[e][0], p[e][1]);
-  };
-  const uint32_t blocks = q4 == 0 ? 0x0030u : q4 == 1 ? 0x3220u : q4 == 2 ? 0x1031u : 0x33221121u;   // a byte each: row, column
-#pragma unroll 1
-  for (int q = 0; q < (q4 == 3 ? 4 : 2); ++q) {
-    const int i = (blocks >> (8 * q + 4)) & 15, j = (blocks >> (8 * q)) & 15;
-    float acc[4] = {};
-#pragma unroll 1
-    for (int k = j; k < i; ++k) block_mul<false>(acc, P_at(i, k), kPitchA, X_at(k, j), row, col);
-    block_mul<true>(acc, P_at(i, i), kPitchA, X_at(i, j), row, col);
-    put_pt(i, j, acc);
+    for (int i = 0; i < 8; ++i) {
+      int bi, bj, t, s;
+      below(i, bi, bj, t, s);
+      A[blk_at(bi, bj) + t * kPitchD + s] = below_w(bi, bj, t, s) * dot[i];
+    }
   }
+  __syncthreads();
+
+  // ---- P X: the ten lower blocks, five block products a pair of warps, eight columns a warp ----
+  const uint32_t blocks = pair == 0 ? 0x0030u : pair == 1 ? 0x3220u : pair == 2 ? 0x1031u : 0x33221121u;   // a byte each: row, column
+  double acc[4][4] = {};
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (q < 2 || pair == 3) {
+      const int i = (blocks >> (8 * q + 4)) & 15, j = (blocks >> (8 * q)) & 15;
+#pragma unroll 1
+      for (int k = j; k <= i; ++k) block_mul(acc[q], A + blk_at(i, k), X + blk_at(k, j) + half, lane);
+    }
+  __syncthreads();   // P is read: the image takes its place
+  auto put_pt = [&](int i, int j, const double (&v)[4]) {
+    const int s = j * 16 + half + (lane & 3) * 2;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = i * 16 + (lane >> 2) + 8 * e;
+      double u0 = s <= t ? v[2 * e] * (double)s_tok[s].y : 0.0, u1 = s < t ? v[2 * e + 1] * (double)s_tok[s + 1].y : 0.0;
+      if (t >= bad) u0 = s <= t ? nan : 0.0, u1 = s < t ? nan : 0.0;
+      uint32_t p[kParts];
+      split3(u0, u1, p[0], p[1], p[2]);
+#pragma unroll
+      for (int q = 0; q < kParts; ++q)
+        *reinterpret_cast<uint32_t*>(sm + L::a + q * L::kRow + panel_at(t, s >> 3) + (s & 7) * 2) = p[q];
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (q < 2 || pair == 3) put_pt((blocks >> (8 * q + 4)) & 15, (blocks >> (8 * q)) & 15, acc[q]);
   {
-    const float zero[4] = {};
-    for (int q = q4; q < 6; q += 4) {
+    const double zero[4] = {};
+    for (int q = pair; q < 6; q += 4) {
       const int i = q < 3 ? 0 : q < 5 ? 1 : 2, j = q < 3 ? q + 1 : q < 5 ? q - 1 : 3;
       put_pt(i, j, zero);
     }
@@ -646,6 +721,29 @@ __device__ __forceinline__ void take_product(uint32_t addr, float2 (&v)[8]) {
   for (int j = 0; j < 8; ++j) v[j] = __fadd2_rn(pair(0, j), __fadd2_rn(pair(1, j), pair(2, j)));
 }
 
+// [K; Q] S: the largest sum lies in four accumulators, a quarter of the key channels each, behind them the two others
+constexpr int kFirst = 4;
+__device__ __forceinline__ void take_first(uint32_t addr, float2 (&v)[8]) {
+  auto pair = [](const uint32_t (&x)[16], int j) { return make_float2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])); };
+  uint32_t x[3][16];
+  float2 small[8];
+  tmem_ld16(addr + kFirst * kCols, x[0]);
+  tmem_ld16(addr + (kFirst + 1) * kCols, x[1]);
+  tmem_ld16(addr, x[2]);
+  tc_wait_ld();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    small[j] = __fadd2_rn(pair(x[0], j), pair(x[1], j));
+    v[j] = pair(x[2], j);
+  }
+#pragma unroll
+  for (int e = 1; e < kFirst; ++e) tmem_ld16(addr + e * kCols, x[e - 1]);
+  tc_wait_ld();
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    v[j] = __fadd2_rn(__fadd2_rn(__fadd2_rn(v[j], pair(x[0], j)), __fadd2_rn(pair(x[1], j), pair(x[2], j))), small[j]);
+}
+
 template <typename T, int D>
 __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArgs a) {
   using L = ChunkSmem<D>;
@@ -689,7 +787,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
   tc_fence_after();
   if (VT > 1) cluster_sync_all();          // barriers exist before a neighbour writes to them
   const uint32_t tmem = bars.tmem_base;
-  constexpr uint32_t kY = 0, kS = 128, kO = 256;   // TMEM columns of the products
+  constexpr uint32_t kY = 0, kS = 256, kO = 384;   // TMEM columns of the products
   const int first_slot = a.slot(b, t0, a.first);
   bool ok = true;
 
@@ -752,8 +850,14 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          product(kY, e, ks, umma_desc_add(kq_d, e * L::kqPart + (ks >> 2) * kPanel + (ks & 3) * 32), umma_desc_add(s_d, ks * 1024));
+        for (int ks = 0; ks < D / 16; ++ks) {
+          constexpr int kStep = D / 16 / kFirst;      // products per accumulator of the largest sum
+          const uint64_t left = umma_desc_add(kq_d, e * L::kqPart + (ks >> 2) * kPanel + (ks & 3) * 32), right = umma_desc_add(s_d, ks * 1024);
+          if (e == 0)
+            umma_ss_warp(tm + kY + (ks / kStep) * kCols, left, right, umma_idesc(true, 128, kCols, false, true), ks % kStep > 0);
+          umma_ss_warp(tm + kY + (kFirst + (e == 2)) * kCols, left, e == 0 ? umma_desc_add(right, L::sPart) : right,
+                       umma_idesc(true, 128, e == 2 ? kCols : 2 * kCols, false, true), e > 0 || ks > 0);
+        }
       }
       if (!ok) break;
       umma_commit_warp(&bars.y_done);
@@ -810,7 +914,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         if (!ok) break;
         tc_fence_after();
         float2 o[8], not_finite = make_float2(0.f, 0.f);
-        take_product(my + kY, o);
+        take_first(my + kY, o);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           o[j] = __ffma2_rn(make_float2(g_t, g_t), o[j], j & 1 ? make_float2(v[j / 2].z, v[j / 2].w) : make_float2(v[j / 2].x, v[j / 2].y));
@@ -896,7 +1000,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
       ok = dc_wait_warp(&bars.y_done, ph, bars);
       if (!ok) break;
       tc_fence_after();
-      take_product(my + kY, o);
+      take_first(my + kY, o);
       tc_fence_before();
       mbar_arrive(&bars.s_full);           // Q S may be overwritten
       ok = dc_wait_warp(&bars.o_done, ph, bars);
@@ -993,7 +1097,7 @@ constexpr size_t kMost = (size_t)320 << 20;
 ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
   ChunkPlan p{};
   const size_t kq = (size_t)G * kParts * (D / 64) * kPanel, cp = (size_t)H * kParts * (D + kChunk) * 128;
-  const size_t dots = (size_t)G * kUnits * 256 * sizeof(float), gw = (size_t)H * kChunk * sizeof(float);
+  const size_t dots = (size_t)G * kUnits * 256 * sizeof(double), gw = (size_t)H * kChunk * sizeof(float);
   const int64_t all = tokens / kChunk + B;      // t0 / 64 + b + c is below this
   p.per_seq = cdiv(max_new, kChunk);
   p.compact = 1;
@@ -1092,7 +1196,7 @@ extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, con
   DeltaChunkArgs a{qkv, qkv_stride, proj_stride, gate_stride, out_stride, proj, gate, b_off, a_off, gate_off, A_log, dt_bias, norm_w,
                    norm_head_stride, eps, state, out, H, G, Dv, reserved_slot, {cu_seqlens_q, seq_start, nullptr, batch_mapping},
                    0, p.per_seq, p.compact, ws + p.kq, ws + p.cp,
-                   reinterpret_cast<float*>(ws + p.dots), reinterpret_cast<float*>(ws + p.gw),
+                   reinterpret_cast<double*>(ws + p.dots), reinterpret_cast<float*>(ws + p.gw),
                    reinterpret_cast<float*>(ws + p.carry)};
   auto st = static_cast<cudaStream_t>(stream);
   if (dtype == CVLLM_BF16)

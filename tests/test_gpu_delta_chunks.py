@@ -47,6 +47,54 @@ def test_chunks(size, lens, starts, dtype):
     check(size, lens, starts, dtype)
 
 
+def shared_direction(kind, m, cols, seed):
+    """Keys that share a direction, as a convolution with silu leaves them: a drift under noise, one key for all tokens, one
+    token repeated, and keys of alternating sign with beta and decays near 1."""
+    draw = torch.Generator().manual_seed(seed)
+    r = lambda n: torch.randn(n, generator=draw).to(cols.device)
+    qk, values, C = 2 * m.kv_heads * m.dim, m.heads * m.vdim, m.conv_channels
+    if kind == "drift":
+        cols[:, :qk] = 0.5 * cols[:, :qk] + 1.5 * r(qk)
+    elif kind == "one key":
+        cols[:, :qk] = r(qk)
+    elif kind == "one token":
+        cols[:, :C] = r(C)
+    elif kind == "alternating":
+        sign = torch.ones(cols.shape[0], 1, device=cols.device)
+        sign[::2] = -1
+        cols[:, :qk] = sign * 4 * r(qk) + 0.01 * cols[:, :qk]
+        cols[:, C + values:C + values + m.heads] = 6.0 + 0.1 * cols[:, C + values:C + values + m.heads]
+        m.A_log.fill_(-6.0)
+
+
+@pytest.mark.parametrize("size", [(4, 2, 128, 128), (4, 2, 64, 64)], ids=str)
+@pytest.mark.parametrize("lens", [[1000], [128], [130, 70, 333]], ids=str)
+@pytest.mark.parametrize("kind", ["random", "drift", "one key", "one token", "alternating"])
+def test_no_farther_from_64_bits_than_the_blocks_of_four(kind, lens, size):
+    """Root mean square over six draws of both kernels' distances from 64 bits, 32-bit rows, outputs and states.  The chunks lie
+    at 0.3 to 0.9 of the blocks of four; with 32-bit coefficients, or all of K S in one accumulator, at up to 2.4."""
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context, set_context
+
+    square = {-1: [0.0, 0.0], 102: [0.0, 0.0]}
+    for seed in range(3, 9):
+        for layout, sums in square.items():
+            m, state, cols, ctx = setup(*size, lens, [0] * len(lens), torch.float32, seed)
+            shared_direction(kind, m, cols, seed + 100)
+            want, want_state = recurrence(m, state, cols, lens, [0] * len(lens))
+            set_context(**ctx)
+            N.set_test_option("gla_layout", layout)
+            try:
+                got = m(None, cols, state).double()
+            finally:
+                N.set_test_option("gla_layout", 0)
+                reset_context()
+            for i, (x, y) in enumerate([(got, want), (state.matrix_state[1:].double(), want_state[1:])]):
+                sums[i] += ((x - y).norm() / y.norm()).item() ** 2
+    for chunks, blocks in zip(square[-1], square[102]):
+        assert chunks <= blocks, ((chunks / 6) ** 0.5, (blocks / 6) ** 0.5)
+
+
 def test_rows_off_the_grid():
     check((2, 1, 128, 128), [130, 70], [0, 4], torch.float32, odd_rows=True)
 
