@@ -767,8 +767,8 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     mbar_init(&bars.s_full, 384);          // eight warps of the state, four of the outputs (Q S is read)
     mbar_init(&bars.r_full, 128);
     mbar_init(&bars.o_free, 128);
-    mbar_init(&bars.norm[0], 1);
-    mbar_init(&bars.norm[1], 1);
+    mbar_init(&bars.norm[0], VT > 1 ? 1 : 2 * kChunk);
+    mbar_init(&bars.norm[1], VT > 1 ? 1 : 2 * kChunk);
     mbar_init(&bars.drain, 1);
     bars.any_bad[0] = bars.any_bad[1] = 0;
     bars.abort = 0;
@@ -1023,12 +1023,17 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         sq = __ffma2_rn(o[j], o[j], sq);
       }
       float ss = sq.x + sq.y;
-      if (t == 0 && half == 0) mbar_expect_tx(&bars.norm[ph], VT * 2 * kChunk * sizeof(float));
       float* mine = &bars.part[ph][vt * 2 + half][t];
-      for (int r = 0; r < VT; ++r)
-        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(mapa_u32(mine, r)),
-                     "r"(__float_as_uint(ss)), "r"(mapa_u32(&bars.norm[ph], r))
-                     : "memory");
+      if (VT > 1) {
+        if (t == 0 && half == 0) mbar_expect_tx(&bars.norm[ph], VT * 2 * kChunk * sizeof(float));
+        for (int r = 0; r < VT; ++r)
+          asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(mapa_u32(mine, r)),
+                       "r"(__float_as_uint(ss)), "r"(mapa_u32(&bars.norm[ph], r))
+                       : "memory");
+      } else {       // a launch without clusters: st.async is an illegal instruction there
+        *mine = ss;
+        mbar_arrive(&bars.norm[ph]);
+      }
       // ---- weight and gate, and the next chunk's ----
       auto gated = [&](float v, int j, float gz) { return v * bars.norm_w[half * 16 + j] * silu_fast(gz); };
 #pragma unroll

@@ -19,21 +19,28 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
 
     m, state, cols, ctx = setup(*size, lens, starts, dtype, seed)
     N.set_test_option("gla_layout", -1)       # chunks whatever the length
-    if odd_rows:       # a view whose rows do not start on 16 bytes: the kernels of the shorter portions
-        wide = torch.zeros(cols.shape[0], cols.shape[1] + 1, dtype=dtype, device=cols.device)
-        wide[:, 1:] = cols
-        cols = wide[:, 1:]
+    # rows on 16 bytes, or a view whose rows do not start there: the kernels of the shorter portions
+    wide = torch.zeros(cols.shape[0], (cols.shape[1] + 8) // 8 * 8, dtype=dtype, device=cols.device)
+    at = 1 if odd_rows else 0
+    wide[:, at:at + cols.shape[1]] = cols
+    cols = wide[:, at:at + cols.shape[1]]
+    if odd_rows:
+        assert cols.data_ptr() % 16 != 0
     else:
         heads, kv, dim, vdim = size
         assert N.lib().cvllm_delta_rule_chunks_workspace_bytes(sum(lens), len(lens), max(lens), heads, kv, dim, vdim) > 0
     want, want_state = recurrence(m, state, cols, lens, starts)
     untouched = state.matrix_state[0].clone()
     set_context(**ctx)
+    launched = N.lib().cvllm_launch_count()
     try:
         got = m(None, cols, state).double()
     finally:
         N.set_test_option("gla_layout", 0)
         reset_context()
+    # the convolution, its state, then one kernel, or three per window of chunks
+    launched = N.lib().cvllm_launch_count() - launched - 2
+    assert launched == 1 if odd_rows else launched >= 3 and launched % 3 == 0
     err = lambda x, y: ((x - y).norm() / y.norm()).item()
     assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
     assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5
