@@ -38,8 +38,9 @@
 // warps beside the issuing one (269); copies paced to arrive between the products (the same).
 //
 // Every wait has a limit.  A wait that runs out sets the CTA's abort flag; all roles then leave their loops, copies and
-// products in flight are waited for (with a limit), the CTA's state becomes NaN and a counter that the host can read
-// (cvllm_delta_chunk_aborts) goes up.
+// products in flight are waited for (with a limit), the CTA's state and its columns of the launch's rows become NaN and a counter
+// that the host can read (cvllm_delta_chunk_aborts) goes up, once per CTA.  In the coefficients' kernel it voids the chunk: its
+// decays, and with them the outputs from there on and the state, become NaN.
 #include <algorithm>
 
 #include "mma.cuh"
@@ -57,6 +58,7 @@ constexpr int kCols = 32;                        // value columns of a CTA
 constexpr int kPanel = 128 * 128;                // 128 rows of 64 16-bit numbers
 constexpr int kParts = 3;
 constexpr uint32_t kSpins = 1u << 20;            // tries of a wait, each up to kSleep ns: about two seconds
+constexpr uint32_t kSpinsHeld = 1u << 9;         // in tests whose waits run out: about a millisecond
 constexpr uint32_t kSleep = 2000;
 
 struct DeltaChunkArgs {
@@ -78,6 +80,8 @@ struct DeltaChunkArgs {
   double* dots;                // [slots, G, 2, 10, 16, 16]: lower blocks of K K^T and Q K^T
   float* gw;                   // [slots, H, 64]: G_t
   float* carry;                // [B, H, Dv, D] between launches
+  uint32_t spins;              // limit of a wait, in tries of up to kSleep ns
+  int hold;                    // tests: copies of chunk hold - 1 never begin for CTA 0 (coefficients: of chunk -hold - 1 for head 0)
   __device__ __forceinline__ int slot(int b, int t0, int c) const { return compact ? t0 / kChunk + b + c : b * per_seq + c - first; }
 };
 
@@ -372,7 +376,8 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
     mbar_fence_init();
     const unsigned char* kq = a.kq + ((int64_t)slot * a.G + grp) * (kParts * (D / 64) * kPanel);
     mbar_expect_tx(&s_bar, kParts * (D / 64) * L::kRow);
-    for (int i = 0; i < kParts * (D / 64); ++i) bulk_load(sm + L::k + i * L::kRow, kq + i * kPanel, L::kRow, &s_bar);
+    if (h > 0 || a.hold >= 0 || c != -a.hold - 1)
+      for (int i = 0; i < kParts * (D / 64); ++i) bulk_load(sm + L::k + i * L::kRow, kq + i * kPanel, L::kRow, &s_bar);
     s_bad = kChunk;
   }
   // of the dots: threads 0 .. 63 a column of a diagonal block, the others eight numbers of the blocks below
@@ -521,15 +526,21 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
           make_uint4(p[e][0], p[e][1], p[e][2], p[e][3]);
   }
   load_dots(1);
-  __syncthreads();
   {
     uint32_t spins = 0;
-    while (!dc_try(&s_bar, 0))
-      if (++spins > kSpins) {     // the chunk's coefficients are void: its decays, and with them the state, become NaN
-        if (tid < kChunk) a.gw[((int64_t)slot * a.H + h) * kChunk + tid] = __int_as_float(0x7fc00000);
-        if (tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
-        break;
+    bool ok = dc_try(&s_bar, 0);
+    while (!ok && spins < a.spins) {
+      ++spins;
+      ok = dc_try(&s_bar, 0);
+    }
+    if (!__syncthreads_and(ok)) {    // the chunk is void
+      if (tid < kChunk) a.gw[((int64_t)slot * a.H + h) * kChunk + tid] = __int_as_float(0x7fc00000);
+      if (tid == 0) {
+        atomicAdd(&g_delta_chunk_aborts, 1);
+        for (spins = 0; !dc_try(&s_bar, 0) && spins < a.spins; ++spins) {}   // the loads land before the CTA ends
       }
+      return;
+    }
   }
 
   // ---- C: 16 channels a warp, all 64 columns; column block nb has rows of token blocks kb >= nb.  The largest pair's sums
@@ -675,7 +686,7 @@ struct ChunkBars {
   float part[2][16][kChunk];             // sums of squares: [CTA * 2 + column half][token]
   float norm_w[kCols];
   int bad[2][kCols], any_bad[2];         // first token of the chunk whose R is not finite, per column
-  uint32_t tmem_base;
+  uint32_t tmem_base, spins;
   volatile uint32_t abort;
 };
 
@@ -683,7 +694,7 @@ __device__ __forceinline__ bool dc_wait(uint64_t* bar, uint32_t parity, ChunkBar
   uint32_t spins = 0;
   while (!dc_try(bar, parity)) {
     if (b.abort) return false;
-    if (++spins > kSpins) {
+    if (++spins > b.spins) {
       b.abort = 1;
       return false;
     }
@@ -772,6 +783,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     mbar_init(&bars.drain, 1);
     bars.any_bad[0] = bars.any_bad[1] = 0;
     bars.abort = 0;
+    bars.spins = a.spins;
     mbar_fence_init();
   }
   if (tid < kCols) {
@@ -804,7 +816,8 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         if (!ok) break;
         for (int e = 0; e < kParts; ++e) {
           mbar_expect_tx(&bars.kq_full[e], L::kqPart);
-          bulk_load(sm + L::kq + e * L::kqPart, kq + c * kq_step + e * L::kqPart, L::kqPart, &bars.kq_full[e]);
+          if (blockIdx.x > 0 || a.first + c != a.hold - 1)
+            bulk_load(sm + L::kq + e * L::kqPart, kq + c * kq_step + e * L::kqPart, L::kqPart, &bars.kq_full[e]);
         }
         ++begun;
         if (c > 0) ok = dc_wait(&bars.o_done, (c - 1) & 1, bars);
@@ -813,9 +826,9 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         bulk_load(sm + L::cp, cp + c * cp_step, kParts * L::cpPart, &bars.cp_full);
         ++begun_cp;
       }
-      if (!ok) {         // the copies in flight land before the CTA ends
+      {                  // copies in flight land before the CTA ends, also those that nobody waits for any more
         auto land = [&](uint64_t* bar, int n) {
-          for (uint32_t spins = 0; n > 0 && !mbar_try_wait(bar, (n - 1) & 1) && spins < kSpins; ++spins) {}
+          for (uint32_t spins = 0; n > 0 && !dc_try(bar, (n - 1) & 1) && spins < a.spins; ++spins) {}
         };
         for (int e = 0; e < kParts; ++e) land(&bars.kq_full[e], begun);
         land(&bars.cp_full, begun_cp);
@@ -872,7 +885,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     }
     if (!ok) {           // products in flight end before TMEM is given back
       umma_commit_warp(&bars.drain);
-      for (uint32_t spins = 0; !mbar_try_wait(&bars.drain, 0) && spins < kSpins; ++spins) {}
+      for (uint32_t spins = 0; !dc_try(&bars.drain, 0) && spins < a.spins; ++spins) {}
     }
     __syncwarp();
   } else if (warp < 8) {
@@ -967,15 +980,13 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     if (keyed) {
       const bool ends = (a.first + chunks) * kChunk >= n_all;
       float* to = ends ? (seq_slot != a.reserved_slot ? st : nullptr) : carry;
-      const float nan = __int_as_float(0x7fc00000);
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (to) {
-          to[(int64_t)(2 * j) * D] = ok ? S[j].x : nan;
-          to[(int64_t)(2 * j + 1) * D] = ok ? S[j].y : nan;
+          to[(int64_t)(2 * j) * D] = S[j].x;
+          to[(int64_t)(2 * j + 1) * D] = S[j].y;
         }
     }
-    if (!ok && tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
   } else if ((warp & 3) >= 2) {
     // ------------------------------ outputs ------------------------------
     const int q4 = warp & 3, half = (warp >> 2) - 2, t = (q4 - 2) * 32 + lane;   // TMEM lanes 64 .. 127: tokens
@@ -1083,7 +1094,23 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (VT > 1) cluster_sync_all();          // nobody leaves while its sums may still be written
+  if (bars.abort) {                        // whichever role gave up
+    const float nan = __int_as_float(0x7fc00000);
+    const int64_t cols = (int64_t)h * a.Dv + vt * kCols;
+    const bool ends = (a.first + chunks) * kChunk >= n_all;
+    float* to = ends ? (seq_slot != a.reserved_slot ? a.state + (int64_t)seq_slot * a.H * a.Dv * D : nullptr)
+                     : a.carry + (int64_t)b * a.H * a.Dv * D;
+    if (to)
+      for (int i = tid; i < kCols * D; i += 512) to[cols * D + i] = nan;
+    const int rows = min(n_all - a.first * kChunk, chunks * kChunk);
+    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + a.first * kChunk) * a.out_stride + cols;
+    for (int i = tid; i < rows * kCols; i += 512) out[(int64_t)(i / kCols) * a.out_stride + i % kCols] = from_f<T>(nan);
+    if (tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
+  }
+  if (VT > 1) {
+    cluster_sync_all();                    // nobody leaves while its sums may still be written:
+    if (bars.abort) __nanosleep(20000);    // here a neighbour's last ones may be under way, for nobody waited for them
+  }
   if (warp == 8) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -1202,7 +1229,8 @@ extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, con
                    norm_head_stride, eps, state, out, H, G, Dv, reserved_slot, {cu_seqlens_q, seq_start, nullptr, batch_mapping},
                    0, p.per_seq, p.compact, ws + p.kq, ws + p.cp,
                    reinterpret_cast<double*>(ws + p.dots), reinterpret_cast<float*>(ws + p.gw),
-                   reinterpret_cast<float*>(ws + p.carry)};
+                   reinterpret_cast<float*>(ws + p.carry), kSpins, test_options().delta_chunk_hold.load()};
+  if (a.hold != 0) a.spins = kSpinsHeld;
   auto st = static_cast<cudaStream_t>(stream);
   if (dtype == CVLLM_BF16)
     return D == 128 ? launch_chunks<__nv_bfloat16, 128>(a, p, B, st) : launch_chunks<__nv_bfloat16, 64>(a, p, B, st);

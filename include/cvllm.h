@@ -72,6 +72,8 @@ uint64_t cvllm_launch_count(void);
  *   "ssm_segment" n          tokens per segment of cvllm_ssm_scan (0 = the product's choice; tests use short segments)
  *   "gla_layout" n           100 * CTAs per (head, sequence) + columns per thread of cvllm_gla_scan and of the portions of
  *                            cvllm_delta_rule (0 = chosen per step; < 0: cvllm_delta_rule_chunks for portions of any length)
+ *   "delta_chunk_hold" n     cvllm_delta_rule_chunks: the copies of chunk n - 1 never begin for the first CTA (n < 0: of chunk
+ *                            -n - 1 for head 0 of the coefficients), so that waits run out, after a millisecond each
  *   "select_passes" 1|0      cvllm_select_store_topk: the chain of launches also where one cluster per sequence would do
  *   "grs_debug_host_ptr" p   pinned host buffer (64 words per CTA) for cvllm_gemm_allreduce's timeout records
  * Returns CVLLM_E_ARG for an unknown name. */
@@ -796,7 +798,8 @@ int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* pr
                             const int32_t* seq_start, const int32_t* batch_mapping, int64_t tokens, int B, int max_new, void* out,
                             int64_t out_stride, int H, int G, int D, int Dv, int reserved_slot, int dtype, void* workspace,
                             size_t workspace_bytes, cvllm_stream_t stream);
-/* CTAs of its kernel that gave up a wait since the library was loaded (0 in sound operation). */
+/* CTAs of its kernels that gave up a wait since the library was loaded (0 in sound operation).  What such a CTA would have written
+ * is NaN: its value columns of the rows and of the state. */
 int cvllm_delta_chunk_aborts(int* count);
 
 /* wkv: r, k, v, w_raw rows of H * D numbers (model type); w = exp(-exp(w_raw + w0)) per head and key channel;

@@ -4,6 +4,8 @@ both types, and portions whose images exceed the workspace's bound and are taken
 its rows in four-channel pieces and without.
 
 Tolerances are those of test_gpu_delta_layouts.py: operands in three bfloat16 parts are good to 2^-26, the sums are fp32."""
+import ctypes
+
 import pytest
 import torch
 
@@ -30,7 +32,7 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
         heads, kv, dim, vdim = size
         assert N.lib().cvllm_delta_rule_chunks_workspace_bytes(sum(lens), len(lens), max(lens), heads, kv, dim, vdim) > 0
     want, want_state = recurrence(m, state, cols, lens, starts)
-    untouched = state.matrix_state[0].clone()
+    untouched, before = state.matrix_state[0].clone(), aborts()
     set_context(**ctx)
     launched = N.lib().cvllm_launch_count()
     try:
@@ -41,6 +43,7 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
     # the convolution, its state, then one kernel, or three per window of chunks
     launched = N.lib().cvllm_launch_count() - launched - 2
     assert launched == 1 if odd_rows else launched >= 3 and launched % 3 == 0
+    assert aborts() == before
     err = lambda x, y: ((x - y).norm() / y.norm()).item()
     assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
     assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5
@@ -117,6 +120,54 @@ def test_the_rule():
 
     need = lambda *a: N.lib().cvllm_delta_rule_chunks_workspace_bytes(*a, 16, 8, 128, 128)
     assert need(128, 1, 128) > 0 and need(127, 1, 127) == 0 and need(191, 2, 128) == 0 and need(192, 2, 128) > 0
+
+
+def aborts():
+    from compactor_vllm import _native as N
+
+    count = ctypes.c_int(-1)
+    N.check(N.lib().cvllm_delta_chunk_aborts(ctypes.byref(count)), "aborts")
+    return count.value
+
+
+@pytest.mark.parametrize("lens", [[200, 64], [192]], ids=str)
+@pytest.mark.parametrize("hold", [1, 2, 3, -1, -2, -3])
+@pytest.mark.parametrize("vdim", [32, 64])
+def test_a_wait_that_runs_out(vdim, hold, lens):
+    """Copies that never begin (a flag that nothing sets): the call ends, the counter goes up, what the affected CTAs would have
+    written is NaN - rows and state of head 0, the cluster's other columns too, which wait for its sums - and the other heads' work
+    is what it was."""
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context, set_context
+
+    def once(held):
+        m, state, cols, ctx = setup(2, 1, 64, vdim, lens, [0] * len(lens), torch.float32, 11)
+        set_context(**ctx)
+        N.set_test_option("gla_layout", -1)
+        N.set_test_option("delta_chunk_hold", held)
+        try:
+            out = m(None, cols, state)
+        finally:
+            N.set_test_option("delta_chunk_hold", 0)
+            N.set_test_option("gla_layout", 0)
+            reset_context()
+        return out.view(-1, 2, vdim), state.matrix_state
+
+    before = aborts()
+    clean, clean_state = once(0)
+    assert aborts() == before and torch.isfinite(clean).all() and torch.isfinite(clean_state).all()
+    got, state = once(hold)
+    assert aborts() > before
+    at = 0
+    for b, n in enumerate(lens):
+        if n > 64 * (abs(hold) - 1):
+            first = 0 if hold > 0 else 64 * (-hold - 1)        # a chunk kernel's rows are void, a coefficient's from its chunk on
+            assert torch.isnan(got[at + first:at + n, 0]).all() and torch.isnan(state[b + 1, 0]).all()
+            assert torch.equal(got[at:at + first, 0], clean[at:at + first, 0])
+        else:
+            assert torch.equal(got[at:at + n, 0], clean[at:at + n, 0]) and torch.equal(state[b + 1, 0], clean_state[b + 1, 0])
+        at += n
+    assert torch.equal(got[:, 1], clean[:, 1]) and torch.equal(state[1:, 1], clean_state[1:, 1])
 
 
 def test_windows():
