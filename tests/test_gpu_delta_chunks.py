@@ -172,3 +172,37 @@ def test_a_wait_that_runs_out(vdim, hold, lens):
 
 def test_windows():
     check((32, 32, 128, 128), [7000, 300], [0, 11], torch.bfloat16)
+
+
+def test_silu_without_a_division():
+    """The convolution's rows in four-channel pieces make their silu from an approximate reciprocal and a correction, rows off the
+    16-byte grid by a division: the same bits over the whole range, where the denominator's reciprocal is subnormal too, and for
+    infinities and NaN."""
+    from compactor_vllm import _native as N
+
+    C, T, dev = 4096, 256, "cuda"
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    x = torch.linspace(-104.0, 104.0, T * C, device=dev)[torch.randperm(T * C, generator=torch.Generator().manual_seed(1)).to(dev)].view(T, C)
+    x[:, :256] = torch.linspace(-88.8, -87.2, T * 256, device=dev).view(T, 256)
+    x[-3] = 0.0          # what follows a number that is not finite is NaN: its weight is 0
+    x[-2] = torch.tensor([float("inf"), -float("inf"), float("nan"), 3e38, -3e38, 1e-40, -1e-40, -0.0], device=dev).repeat(C // 8)
+    weight = torch.zeros(C, 2, device=dev)
+    weight[:, 1] = 1.0
+    state, cu, zero, slot = torch.zeros(2, 1, C, device=dev), i32([0, T]), i32([0]), i32([1])
+
+    def silu(off):
+        rows = torch.zeros(T, C + 4, device=dev)
+        rows[:, off:off + C] = x
+        out = torch.empty(T, C, device=dev)
+        N.check(N.lib().cvllm_causal_conv(N.ptr(rows), rows.stride(0), off, C, 2, N.ptr(weight), None, N.ptr(state), N.ptr(cu),
+                                          N.ptr(zero), None, N.ptr(slot), 1, T, N.ptr(out), C, N.block_dtype_code(x.dtype),
+                                          N.stream(out.device)), "cvllm_causal_conv")
+        return out
+
+    got, want = silu(0), silu(1)
+    assert torch.equal(got.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0)) and torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(torch.signbit(got[:-1]), torch.signbit(want[:-1]))
+    exact = x[:-3].double() * torch.sigmoid(x[:-3].double())
+    # expf is good to 2^-22, the sum and the quotient to 2^-24 each; below 1e-30 e^-z nears the end of fp32's range
+    normal = exact.abs() > 1e-30
+    assert ((got[:-3].double() - exact)[normal].abs() <= (2 ** -22 + 2 ** -23) * exact[normal].abs()).all()
