@@ -42,6 +42,7 @@
 // that the host can read (cvllm_delta_chunk_aborts) goes up, once per CTA.  In the coefficients' kernel it voids the chunk: its
 // decays, and with them the outputs from there on and the state, become NaN.
 #include <algorithm>
+#include <utility>
 
 #include "mma.cuh"
 #include "recur_common.cuh"
@@ -73,17 +74,39 @@ struct DeltaChunkArgs {
   void* out;
   int H, G, Dv, reserved_slot;
   StepGeom g;
-  // a launch takes the chunks [first, first + per_seq) of every sequence; their images lie at slot(b, chunk)
-  int first, per_seq, compact;
+  // a launch takes a window of `slots` chunks, whose images lie at places from 0 on.  per_seq == 0: the chunks of all sequences in
+  // a row, chunk c of sequence b at cu_q[b] / 64 + b + c, from `window` on.  per_seq > 0: the chunks from `window` on of every
+  // sequence, per_seq places each.
+  int B, window, slots, per_seq;
   unsigned char* kq;           // [slots, G, parts, D / 64, panel]: rows 0 .. 63 k, 64 .. 127 q
   unsigned char* cp;           // [slots, H, parts, D + 64 rows of 128 bytes]: rows 0 .. D - 1 C, then P T
   double* dots;                // [slots, G, 2, 10, 16, 16]: lower blocks of K K^T and Q K^T
   float* gw;                   // [slots, H, 64]: G_t
-  float* carry;                // [B, H, Dv, D] between launches
+  float *carry_in, *carry_out; // [H, Dv, D]: the state of the sequence that the window before (this one) ends in, or every sequence's
   uint32_t spins;              // limit of a wait, in tries of up to kSleep ns
   int hold;                    // tests: copies of chunk hold - 1 never begin for CTA 0 (coefficients: of chunk -hold - 1 for head 0)
-  __device__ __forceinline__ int slot(int b, int t0, int c) const { return compact ? t0 / kChunk + b + c : b * per_seq + c - first; }
 };
+// the chunk at place blockIdx.x of the window: false where a sequence's last chunk is not followed by the next sequence's first
+__device__ __forceinline__ bool chunk_of_block(const DeltaChunkArgs& a, int& b, int& c, int& t0, int& n) {
+  const int at = a.window + blockIdx.x;
+  b = 0;
+  if (a.per_seq > 0) {
+    b = blockIdx.x / a.per_seq;
+  } else if (a.B > 1) {
+    int before = 0;      // sequences that begin here or before
+    for (int i0 = 0; i0 < a.B && before == i0; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      before += __syncthreads_count(i < a.B && a.g.cu_q[i] / kChunk + i <= at);
+    }
+    if (before == 0) return false;
+    b = before - 1;
+  }
+  int n_new, start;
+  portion(a.g, b, t0, n_new, start);
+  c = a.per_seq > 0 ? at - b * a.per_seq : at - (t0 / kChunk + b);
+  n = min(kChunk, n_new - c * kChunk);
+  return c >= 0 && n > 0;
+}
 
 // x = hi + mid + lo, each a bfloat16; two numbers a word
 __device__ __forceinline__ void split3(float2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -149,7 +172,7 @@ __device__ __forceinline__ bool dc_try(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ int panel_at(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
 
 // ---------------------------------------------------------------------------------------------------------
-// Unit rows and their products.  grid (chunks, G, B), 256 threads: k and q rows to unit length and into parts, the image out
+// Unit rows and their products.  grid (chunks, G), 256 threads: k and q rows to unit length and into parts, the image out
 // by a bulk copy; K K^T and Q K^T (lower blocks of 16) on mma.sync, from float16 slices that take the image's place.  The largest
 // sum is exact and the others are 2^-12 and 2^-24 of it, so a product is good to 2^-32: 63 of them enter every u_t, and keys that
 // share a direction (products near 1) make the sum as large as the values.
@@ -166,12 +189,10 @@ __device__ __forceinline__ void unit_of(int u, int& m, int& mt, int& nt) {
 template <int D>
 __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const DeltaChunkArgs a) {
   extern __shared__ unsigned char smem_raw[];
-  const int b = blockIdx.z, grp = blockIdx.y, c = a.first + blockIdx.x;
-  int t0, n_new, start;
-  portion(a.g, b, t0, n_new, start);
-  const int n = min(kChunk, n_new - c * kChunk);
-  if (n <= 0) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = a.slot(b, t0, c);
+  const int grp = blockIdx.y;
+  int b, c, t0, n;
+  if (!chunk_of_block(a, b, c, t0, n)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = blockIdx.x;
   unsigned char* img = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   constexpr int kPartBytes = (D / 64) * kPanel;
 
@@ -293,7 +314,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const Delta
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Coefficients of the chunks.  grid (chunks, H, B), 256 threads: decays; A (beta_t w_ts k_t . k_s, t > s); the inverse X of
+// Coefficients of the chunks.  grid (chunks, H), 256 threads: decays; A (beta_t w_ts k_t . k_s, t > s); the inverse X of
 // I + A in blocks of 16 tokens - diagonal blocks by forward substitution, a column per thread, then halves of 32 and of 64 from
 // X_21 = -X_22 (A_21 X_11); C = K^T diag(w_63) X diag(beta) from three parts on mma.sync; P and P X diag(beta).
 //
@@ -361,12 +382,10 @@ __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const Delta
   __shared__ uint64_t s_bar;
   __shared__ double s_pre[kChunk], s_suf[kChunk];     // products of the decays of a token's block up to it, and behind it
   __shared__ int s_bad;                               // first token that is not finite
-  const int b = blockIdx.z, h = blockIdx.y, c = a.first + blockIdx.x, grp = h / (a.H / a.G);
-  int t0, n_new, start;
-  portion(a.g, b, t0, n_new, start);
-  const int n = min(kChunk, n_new - c * kChunk);
-  if (n <= 0) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = a.slot(b, t0, c);
+  const int h = blockIdx.y, grp = h / (a.H / a.G);
+  int b, c, t0, n;
+  if (!chunk_of_block(a, b, c, t0, n)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = blockIdx.x;
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   double *A = reinterpret_cast<double*>(sm + L::a), *X = reinterpret_cast<double*>(sm + L::x);
   const double* dots = a.dots + ((int64_t)slot * a.G + grp) * kUnits * 256;
@@ -764,7 +783,8 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int t0, n_all, start;
   portion(a.g, b, t0, n_all, start);
-  const int chunks = min(a.per_seq, cdiv(max(n_all, 0), kChunk) - a.first);
+  const int base = a.per_seq > 0 ? 0 : t0 / kChunk + b, first = max(0, a.window - base);
+  const int chunks = min(cdiv(max(n_all, 0), kChunk), a.window + (a.per_seq > 0 ? a.per_seq : a.slots) - base) - first;
   if (chunks <= 0) return;                 // the same for every CTA of the cluster
   const int seq_slot = a.g.slots[b], grp = h / (a.H / a.G);
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -800,7 +820,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
   if (VT > 1) cluster_sync_all();          // barriers exist before a neighbour writes to them
   const uint32_t tmem = bars.tmem_base;
   constexpr uint32_t kY = 0, kS = 256, kO = 384;   // TMEM columns of the products
-  const int first_slot = a.slot(b, t0, a.first);
+  const int first_slot = base + first - a.window + b * a.per_seq;
   bool ok = true;
 
   if (warp == 9) {
@@ -816,7 +836,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
         if (!ok) break;
         for (int e = 0; e < kParts; ++e) {
           mbar_expect_tx(&bars.kq_full[e], L::kqPart);
-          if (blockIdx.x > 0 || a.first + c != a.hold - 1)
+          if (blockIdx.x > 0 || first + c != a.hold - 1)
             bulk_load(sm + L::kq + e * L::kqPart, kq + c * kq_step + e * L::kqPart, L::kqPart, &bars.kq_full[e]);
         }
         ++begun;
@@ -896,12 +916,12 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     const uint32_t my = tmem + ((uint32_t)(q4 * 32) << 16) + half * 16;
     const bool keyed = row < D;            // a key channel's thread
     float* st = a.state + (((int64_t)seq_slot * a.H + h) * a.Dv + col0) * D + row;
-    float* carry = a.carry + (((int64_t)b * a.H + h) * a.Dv + col0) * D + row;
+    const int64_t carried = (((int64_t)(a.per_seq > 0 ? b : 0) * a.H + h) * a.Dv + col0) * D + row;
     const float* gw = a.gw + ((int64_t)first_slot * a.H + h) * kChunk;
     float2 S[8];
     {
-      const float* from = a.first > 0 ? carry : st;
-      const bool zero = !keyed || (a.first == 0 && start <= 0);
+      const float* from = first > 0 ? a.carry_in + carried : st;
+      const bool zero = !keyed || (first == 0 && start <= 0);
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         S[j] = zero ? make_float2(0.f, 0.f) : make_float2(from[(int64_t)(2 * j) * D], from[(int64_t)(2 * j + 1) * D]);
@@ -915,7 +935,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
       const float g_all = gw[kChunk - 1];
       // ---- K S -> R = V - G K S ----
       if (early) {
-        const int tok = (a.first + c) * kChunk + row;       // within the portion
+        const int tok = (first + c) * kChunk + row;       // within the portion
         const float g_t = -gw[row];
         float4 v[4];
         {
@@ -978,8 +998,8 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
       gw += (int64_t)a.H * kChunk;
     }
     if (keyed) {
-      const bool ends = (a.first + chunks) * kChunk >= n_all;
-      float* to = ends ? (seq_slot != a.reserved_slot ? st : nullptr) : carry;
+      const bool ends = (first + chunks) * kChunk >= n_all;
+      float* to = ends ? (seq_slot != a.reserved_slot ? st : nullptr) : a.carry_out + carried;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (to) {
@@ -993,11 +1013,11 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
     const int col0 = vt * kCols + half * 16;
     const uint32_t my = tmem + ((uint32_t)(q4 * 32) << 16) + half * 16;
     const float* gw = a.gw + ((int64_t)first_slot * a.H + h) * kChunk + t;
-    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + a.first * kChunk + t) * a.out_stride + h * a.Dv + col0;
-    const T* gate = static_cast<const T*>(a.gate) + (int64_t)(t0 + a.first * kChunk + t) * a.gate_stride + a.gate_off + h * a.Dv + col0;
+    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + first * kChunk + t) * a.out_stride + h * a.Dv + col0;
+    const T* gate = static_cast<const T*>(a.gate) + (int64_t)(t0 + first * kChunk + t) * a.gate_stride + a.gate_off + h * a.Dv + col0;
     constexpr int kPieces = sizeof(T);     // 16 numbers in 16-byte pieces
     uint4 z[kPieces];
-    int left = n_all - a.first * kChunk - t;   // tokens of the portion from this thread's on
+    int left = n_all - first * kChunk - t;   // tokens of the portion from this thread's on
     auto load_gate = [&]() {
 #pragma unroll
       for (int j = 0; j < kPieces; ++j) z[j] = left > 0 ? *reinterpret_cast<const uint4*>(gate + j * (16 / sizeof(T))) : make_uint4(0, 0, 0, 0);
@@ -1097,13 +1117,13 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
   if (bars.abort) {                        // whichever role gave up
     const float nan = __int_as_float(0x7fc00000);
     const int64_t cols = (int64_t)h * a.Dv + vt * kCols;
-    const bool ends = (a.first + chunks) * kChunk >= n_all;
+    const bool ends = (first + chunks) * kChunk >= n_all;
     float* to = ends ? (seq_slot != a.reserved_slot ? a.state + (int64_t)seq_slot * a.H * a.Dv * D : nullptr)
-                     : a.carry + (int64_t)b * a.H * a.Dv * D;
+                     : a.carry_out + (int64_t)(a.per_seq > 0 ? b : 0) * a.H * a.Dv * D;
     if (to)
       for (int i = tid; i < kCols * D; i += 512) to[cols * D + i] = nan;
-    const int rows = min(n_all - a.first * kChunk, chunks * kChunk);
-    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + a.first * kChunk) * a.out_stride + cols;
+    const int rows = min(n_all - first * kChunk, chunks * kChunk);
+    T* out = static_cast<T*>(a.out) + (int64_t)(t0 + first * kChunk) * a.out_stride + cols;
     for (int i = tid; i < rows * kCols; i += 512) out[(int64_t)(i / kCols) * a.out_stride + i % kCols] = from_f<T>(nan);
     if (tid == 0) atomicAdd(&g_delta_chunk_aborts, 1);
   }
@@ -1118,38 +1138,41 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArg
 }
 
 struct ChunkPlan {
-  int windows, per_seq, slots, compact;
-  size_t kq, cp, dots, gw, carry, bytes;
+  int windows, slots, per_seq;
+  size_t cp, dots, gw, carry, other_carry, bytes;
 };
 
-// Images take 116 KB per chunk and key head and 72 KB per chunk and head (heads of 128): 0.27 GB per 4096 tokens of 16 / 32
-// heads.  Above `kMost` the portions are taken in windows of chunks of equal length, the state carried between the launches.
+// Images take 98 KB per chunk and key head and 74 KB per chunk and head (heads of 128), products 41 KB per key head: 0.3 GB per 4096
+// tokens of 16 / 32 heads.  Above `kMost` the chunks are taken in windows of equal length: the row of all chunks is cut, so that a
+// window is full however the tokens are spread (8000 tokens beside 15 times 500, 32 / 16 heads: 2.83 -> 1.64 ms against a range of
+// every sequence's chunks; 6000 beside 31 single tokens: 3.38 -> 0.93 ms), and ends in at most one sequence, whose state is
+// carried to the next.  Where a window of the row would hold too few sequences for the SMs and the sequences are about equally long,
+// a window takes a range of every sequence's chunks instead (8 times 4096 tokens, 8 heads of 128 x 64: 1.10 -> 0.74 ms).
 constexpr size_t kMost = (size_t)320 << 20;
 
 ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
   ChunkPlan p{};
   const size_t kq = (size_t)G * kParts * (D / 64) * kPanel, cp = (size_t)H * kParts * (D + kChunk) * 128;
   const size_t dots = (size_t)G * kUnits * 256 * sizeof(double), gw = (size_t)H * kChunk * sizeof(float);
-  const int64_t all = tokens / kChunk + B;      // t0 / 64 + b + c is below this
-  p.per_seq = cdiv(max_new, kChunk);
-  p.compact = 1;
-  p.windows = 1;
-  int64_t slots = all;
-  if ((size_t)all * (kq + cp + dots + gw) > kMost) {
-    const int64_t most = (int64_t)(kMost / (kq + cp + dots + gw));
-    const int chunks = p.per_seq, longest = (int)std::max<int64_t>(1, std::min<int64_t>(most / B, chunks));
-    p.compact = 0;
-    p.per_seq = cdiv(chunks, cdiv(chunks, longest));
+  const size_t state = (size_t)H * Dv * D * sizeof(float);
+  const int64_t all = tokens / kChunk + B;      // cu_q[b] / 64 + b + c is below this
+  const int64_t most = std::max<int64_t>(1, (int64_t)(kMost / (kq + cp + dots + gw)));
+  const int chunks = cdiv(max_new, kChunk);
+  p.windows = (int)((all + most - 1) / most);
+  p.slots = (int)((all + p.windows - 1) / p.windows);
+  if (p.windows > 1 && B <= most && B * state <= kMost && 4 * tokens >= 3 * (int64_t)B * max_new &&
+      (p.slots / chunks + 1) * (int64_t)H * (Dv / kCols) < sm_count()) {
+    p.per_seq = (int)std::min<int64_t>(most / B, chunks);
     p.windows = cdiv(chunks, p.per_seq);
-    slots = (int64_t)p.per_seq * B;
+    p.per_seq = cdiv(chunks, p.windows);
+    p.slots = p.per_seq * B;
   }
-  p.slots = (int)slots;
-  p.kq = 0;
-  p.cp = p.kq + slots * kq;
-  p.dots = p.cp + slots * cp;
-  p.gw = p.dots + slots * dots;
-  p.carry = p.gw + slots * gw;
-  p.bytes = p.carry + (p.windows > 1 ? (size_t)B * H * Dv * D * sizeof(float) : 0);
+  p.cp = p.slots * kq;
+  p.dots = p.cp + p.slots * cp;
+  p.gw = p.dots + p.slots * dots;
+  p.carry = p.gw + p.slots * gw;
+  p.other_carry = p.carry + (p.per_seq > 0 ? 0 : state);       // of its own: one sequence's is read while another's is written
+  p.bytes = p.windows == 1 ? p.carry : p.per_seq > 0 ? p.carry + B * state : p.other_carry + state;
   return p;
 }
 
@@ -1163,9 +1186,10 @@ int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) 
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_chunk_kernel<T, D>, (int)smem_c, attr_c));
   const int VT = a.Dv / kCols;
   for (int w = 0; w < p.windows; ++w) {
-    a.first = w * p.per_seq;
-    delta_rows_kernel<D><<<dim3(p.per_seq, a.G, B), kPrepThreads, smem_r, st>>>(a);
-    delta_coef_kernel<T, D><<<dim3(p.per_seq, a.H, B), kPrepThreads, smem_k, st>>>(a);
+    a.window = w * (p.per_seq > 0 ? p.per_seq : p.slots);
+    if (w > 0) std::swap(a.carry_in, a.carry_out);
+    delta_rows_kernel<D><<<dim3(p.slots, a.G), kPrepThreads, smem_r, st>>>(a);
+    delta_coef_kernel<T, D><<<dim3(p.slots, a.H), kPrepThreads, smem_k, st>>>(a);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.H * VT, B);
     cfg.blockDim = dim3(512);
@@ -1199,7 +1223,7 @@ extern "C" size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B,
   if (forced > 0 || (forced == 0 && (max_new < 2 * kChunk || tokens < 96 * (int64_t)B))) return 0;
   if ((D != 64 && D != 128) || Dv <= 0 || Dv % kCols != 0 || Dv > 8 * kCols || H % G != 0) return 0;
   const size_t bytes = chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
-  return bytes <= 2 * kMost ? bytes : 0;   // a chunk of every sequence would take more: very many portions at once
+  return bytes <= 2 * kMost ? bytes : 0;   // one chunk of very many heads
 }
 
 extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* proj, int64_t proj_stride, int b_off,
@@ -1227,9 +1251,9 @@ extern "C" int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, con
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   DeltaChunkArgs a{qkv, qkv_stride, proj_stride, gate_stride, out_stride, proj, gate, b_off, a_off, gate_off, A_log, dt_bias, norm_w,
                    norm_head_stride, eps, state, out, H, G, Dv, reserved_slot, {cu_seqlens_q, seq_start, nullptr, batch_mapping},
-                   0, p.per_seq, p.compact, ws + p.kq, ws + p.cp,
+                   B, 0, p.slots, p.per_seq, ws, ws + p.cp,
                    reinterpret_cast<double*>(ws + p.dots), reinterpret_cast<float*>(ws + p.gw),
-                   reinterpret_cast<float*>(ws + p.carry), kSpins, test_options().delta_chunk_hold.load()};
+                   reinterpret_cast<float*>(ws + p.carry), reinterpret_cast<float*>(ws + p.other_carry), kSpins, test_options().delta_chunk_hold.load()};
   if (a.hold != 0) a.spins = kSpinsHeld;
   auto st = static_cast<cudaStream_t>(stream);
   if (dtype == CVLLM_BF16)

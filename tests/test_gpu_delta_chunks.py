@@ -48,6 +48,7 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
     assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
     assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5
     assert torch.equal(state.matrix_state[0], untouched)
+    return launched
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -170,8 +171,15 @@ def test_a_wait_that_runs_out(vdim, hold, lens):
     assert torch.equal(got[:, 1], clean[:, 1]) and torch.equal(state[1:, 1], clean_state[1:, 1])
 
 
-def test_windows():
-    check((32, 32, 128, 128), [7000, 300], [0, 11], torch.bfloat16)
+@pytest.mark.parametrize("size, lens, windows", [
+    ((32, 32, 128, 128), [7000, 300], 3), ((32, 32, 128, 128), [1, 2500, 64, 1, 3000, 127, 900], 3),
+    ((32, 16, 128, 128), [6000] + [1] * 31, 2), ((2, 1, 64, 64), [1] * 300 + [130, 70], 1),
+    ((8, 8, 128, 64), [3300, 3200, 3100, 3000], 2)], ids=["two", "seven", "one long", "many", "about equal"])
+def test_windows(size, lens, windows):
+    """Chunks of all sequences in one row, cut into windows of 320 MB: what a window holds does not depend on how the tokens are
+    spread over the sequences.  The last: a range of every sequence's chunks, for few heads and sequences about equally long."""
+    starts = [11 * (i % 2) for i in range(len(lens))]
+    assert check(size, lens, starts, torch.bfloat16) == 3 * windows
 
 
 def test_silu_without_a_division():
