@@ -1213,14 +1213,31 @@ int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) 
 
 using namespace cvllm;
 
+// From where the chunks are faster than the blocks of four (cvllm_delta_rule).  The three launches take 35 to 45 us for 64 tokens, the
+// blocks of four 0.23 us a token (heads of 128) or 0.16 (64) while they are few; with `pairs` (head, sequence) pairs at work at once
+// both grow.  Coefficients cost the same whatever Dv, and the blocks of four pass value sizes of 32 and 64 at twice the rate per column.
+// Blocks' time / chunks' in us, at the lines (32 or 16 heads, lengths x sequences):
+//   128 x 128: 192 x 1: 54 / 46; 128 x 1: 39 / 43; 128 x 4, 16 heads (64 pairs): 56 / 62; 128 x 4, 32 heads (128): 108 / 83
+//   64 x 256: 256 x 1, 32 heads: 70 / 74; 384 x 1: 99 / 90; 64 x 128: 128 x 16, 16 heads (256): 137 / 141; 192 x 16: 210 / 187
+//   128 x 64: 256 x 2, 16 heads: 53 / 56; 512 x 2, 32 heads: 125 / 92; 512 x 16, 8 heads (128): 177 / 203
+//   128 x 32: 512 x 2, 16 heads: 90 / 67; 1024 x 4, 16 heads (64): 178 / 191; 64 x 32: 1024 x 8, 16 heads: 168 / 239
+// Every sequence fills whole chunks: 96 tokens a sequence on average at least (7 single tokens and 762: 293 / 179).
+// Of 2886 measured batches (D 64 and 128, Dv 32 to 256, 4 to 64 heads, 1 to 32 equal or ragged sequences) none is slower by the rule.
+static bool chunks_are_faster(int64_t tokens, int B, int max_new, int H, int D, int Dv) {
+  if (max_new < 2 * kChunk || tokens < 96 * (int64_t)B) return false;
+  const int64_t work = H * tokens;             // pairs * max_new
+  auto pairs_above = [&](int64_t n) { return work > n * max_new; };
+  if (Dv >= 3 * kCols) {
+    if (D == 128) return max_new >= 192 || pairs_above(64);
+    return max_new >= (pairs_above(32) ? 256 : 384) || pairs_above(256);
+  }
+  return max_new >= (pairs_above(16) ? 512 : 256) && !pairs_above(sm_count() / (Dv == 2 * kCols ? 2 : 3));
+}
+
 extern "C" size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv) {
   if (tokens <= 0 || B <= 0 || max_new <= 0 || H <= 0 || G <= 0) return 0;
-  // From where it is faster: the chunks' three launches take 35 - 45 us for 64 tokens, as long as the kernel of blocks of four takes
-  // for 90 (one portion of 16 or 32 heads of 64 or 128: 44 / 47 us at 64 tokens, 57 / 53 at 100, 60 / 51 at 128, 162 / 94 at
-  // 512, the blocks' time first), and every sequence fills whole chunks (7 single tokens and a portion of 90: 95 / 121 us; 300, 200,
-  // 100, 50, 25 and 12 tokens: 186 / 162).  Test option gla_layout: > 0 the other kernel, < 0 chunks.
-  const int forced = test_options().gla_layout.load();
-  if (forced > 0 || (forced == 0 && (max_new < 2 * kChunk || tokens < 96 * (int64_t)B))) return 0;
+  const int forced = test_options().gla_layout.load();   // tests and measurements: > 0 the other kernel, < 0 chunks
+  if (forced > 0 || (forced == 0 && !chunks_are_faster(tokens, B, max_new, H, D, Dv))) return 0;
   if ((D != 64 && D != 128) || Dv <= 0 || Dv % kCols != 0 || Dv > 8 * kCols || H % G != 0) return 0;
   const size_t bytes = chunk_plan(tokens, B, max_new, H, G, D, Dv).bytes;
   return bytes <= 2 * kMost ? bytes : 0;   // one chunk of very many heads

@@ -116,11 +116,19 @@ def test_what_is_not_finite_stays_behind_its_token(at):
 
 
 def test_the_rule():
-    """Short portions and batches of mostly short ones are the other kernel's."""
+    """Short portions, batches of mostly short ones and, for few value columns, many (head, sequence) pairs are the other
+    kernel's."""
     from compactor_vllm import _native as N
 
-    need = lambda *a: N.lib().cvllm_delta_rule_chunks_workspace_bytes(*a, 16, 8, 128, 128)
-    assert need(128, 1, 128) > 0 and need(127, 1, 127) == 0 and need(191, 2, 128) == 0 and need(192, 2, 128) > 0
+    def need(lens, heads, dim, vdim):
+        return N.lib().cvllm_delta_rule_chunks_workspace_bytes(sum(lens), len(lens), max(lens), heads, heads // 2, dim, vdim) > 0
+
+    assert need([192], 16, 128, 128) and not need([191], 16, 128, 128)
+    assert need([128] * 5, 16, 128, 128) and not need([128] * 4, 16, 128, 128) and not need([127] * 8, 16, 128, 128)
+    assert need([959, 1], 16, 128, 128) and not need([959] + [1] * 10, 16, 128, 128)
+    assert need([384], 32, 64, 256) and not need([383], 32, 64, 256) and need([256] * 2, 32, 64, 256) and need([128] * 9, 32, 64, 256)
+    assert need([256], 16, 128, 64) and need([512] * 2, 32, 128, 64) and not need([511] * 2, 32, 128, 64)
+    assert not need([4096] * 3, 32, 64, 64) and need([512] * 3, 16, 128, 32) and not need([4096] * 4, 16, 128, 32)
 
 
 def aborts():
