@@ -107,32 +107,31 @@ class DeltaRuleMixer(nn.Module):
         slots = ctx.batch_mapping
         C = self.conv_channels
         qkv = torch.empty((T, C), dtype=torch.float32, device=dev)
-        N.check(lib.cvllm_causal_conv(N.ptr(cols), cols.stride(0), 0, C, self.taps, N.ptr(self.conv_weight), None,
-                                      N.ptr(state.conv_state), *geom, N.ptr(slots), B, max_new, N.ptr(qkv),
-                                      qkv.stride(0), code, st), "cvllm_causal_conv")
-        N.check(lib.cvllm_conv_state_update(N.ptr(cols), cols.stride(0), 0, C, self.taps, N.ptr(state.conv_state),
-                                            *geom, N.ptr(slots), B, RESERVED_BATCH, code, st),
-                "cvllm_conv_state_update")
         out = torch.empty((T, H * Dv), dtype=cols.dtype, device=dev)
+        x, x_row, qkv_at, out_at, slots_at = N.ptr(cols), cols.stride(0), N.ptr(qkv), N.ptr(out), N.ptr(slots)
+        N.check(lib.cvllm_causal_conv(x, x_row, 0, C, self.taps, N.ptr(self.conv_weight), None, N.ptr(state.conv_state), *geom,
+                                      slots_at, B, max_new, qkv_at, C, code, st), "cvllm_causal_conv")
+        N.check(lib.cvllm_conv_state_update(x, x_row, 0, C, self.taps, N.ptr(state.conv_state), *geom, slots_at, B,
+                                            RESERVED_BATCH, code, st), "cvllm_conv_state_update")
         g_off = C
         b_off = C + H * Dv
-        rows = (N.ptr(qkv), qkv.stride(0), N.ptr(cols), cols.stride(0), b_off, b_off + H, N.ptr(self.A_log),
-                N.ptr(self.dt_bias), N.ptr(state.matrix_state), N.ptr(cols), cols.stride(0), g_off, N.ptr(self.norm_weight),
-                0, self.eps)
-        # portions in chunks on the tensor cores where the library has them for these sizes and rows lie on 16 bytes
+        rows = (qkv_at, C, x, x_row, b_off, b_off + H, N.ptr(self.A_log), N.ptr(self.dt_bias), N.ptr(state.matrix_state), x,
+                x_row, g_off, N.ptr(self.norm_weight), 0, self.eps)
+        # portions in chunks on the tensor cores where the library has them for these sizes (never below one chunk of 64 tokens)
+        # and rows lie on 16 bytes
         need = 0
-        if geom[2] is None and all(x % 16 == 0 for x in (qkv.data_ptr(), cols.data_ptr(), out.data_ptr(),
-                                                         cols.stride(0) * cols.element_size(), g_off * cols.element_size(),
-                                                         out.stride(0) * out.element_size(), C * 4)):
+        if max_new >= 64 and geom[2] is None:
             need = lib.cvllm_delta_rule_chunks_workspace_bytes(T, B, max_new, H, G, D, Dv)
+            size = cols.element_size()
+            if need and any(v % 16 for v in (qkv_at, x, out_at, x_row * size, g_off * size, H * Dv * size, C * 4)):
+                need = 0
         if need:
             ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to some hundred MB: given back after the call
-            N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], N.ptr(slots), T, B, max_new, N.ptr(out),
-                                                out.stride(0), H, G, D, Dv, RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st),
-                    "cvllm_delta_rule_chunks")
+            N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], slots_at, T, B, max_new, out_at, H * Dv, H, G, D, Dv,
+                                                RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st), "cvllm_delta_rule_chunks")
         else:
-            N.check(lib.cvllm_delta_rule(*rows, *geom, N.ptr(slots), B, max_new, N.ptr(out), out.stride(0), H, G, D, Dv,
-                                         RESERVED_BATCH, code, st), "cvllm_delta_rule")
+            N.check(lib.cvllm_delta_rule(*rows, *geom, slots_at, B, max_new, out_at, H * Dv, H, G, D, Dv, RESERVED_BATCH, code,
+                                         st), "cvllm_delta_rule")
         return self.o_proj(out)
 
 
