@@ -126,7 +126,11 @@ class DeltaRuleMixer(nn.Module):
             if need and any(v % 16 for v in (qkv_at, x, out_at, x_row * size, g_off * size, H * Dv * size, C * 4)):
                 need = 0
         if need:
-            ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to some hundred MB: given back after the call
+            try:
+                ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to 320 MB: given back after the call
+            except torch.OutOfMemoryError:      # the other kernel needs none
+                need = 0
+        if need:
             N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], slots_at, T, B, max_new, out_at, H * Dv, H, G, D, Dv,
                                                 RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st), "cvllm_delta_rule_chunks")
         else:

@@ -190,6 +190,32 @@ def test_windows(size, lens, windows):
     assert check(size, lens, starts, torch.bfloat16) == 3 * windows
 
 
+def test_without_memory_for_the_images(monkeypatch):
+    """A device that has no room left for the workspace: the kernel that needs none, as before there were chunks."""
+    from compactor_vllm import _native as N
+    from compactor_vllm.utils.context import reset_context, set_context
+
+    m, state, cols, ctx = setup(4, 2, 128, 128, [400], [0], torch.float32, 6)
+    want, want_state = recurrence(m, state, cols, [400], [0])
+    empty = torch.empty
+
+    def full(*args, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", full)
+    set_context(**ctx)
+    launched = N.lib().cvllm_launch_count()
+    try:
+        got = m(None, cols, state)
+    finally:
+        reset_context()
+    assert N.lib().cvllm_launch_count() - launched == 3
+    for x, y in ((got, want), (state.matrix_state[1:], want_state[1:])):
+        assert ((x.double() - y).norm() / y.norm()).item() < 1e-5
+
+
 def test_silu_without_a_division():
     """The convolution's rows in four-channel pieces make their silu from an approximate reciprocal and a correction, rows off the
     16-byte grid by a division: the same bits over the whole range, where the denominator's reciprocal is subnormal too, and for
