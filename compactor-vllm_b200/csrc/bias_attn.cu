@@ -708,19 +708,89 @@ __device__ __forceinline__ void store8<float>(float* p, const float* v) {
 
 // q / k norm + store with 16-byte accesses: D and Dv multiples of 8 and at most 256, rows 16-byte aligned.
 // LPR lanes (a power of two, 8 elements each) share a head row, so a warp takes 32 / LPR rows at once and a CTA
-// 4 * 32 / LPR; grid = (groups of TOKS tokens, row groups): a decode step's few tokens still spread over many CTAs.  A lane
-// keeps its piece of the row in registers between the sum of squares and the scaled write; TOKS tokens' pieces are loaded
-// before the first is used.  Above 64 tokens the cache length of a slot is raised by the last token of an ascending run of its
-// positions alone: a portion's tokens all hit the same few words (4096 tokens of 32 + 8 + 8 heads of 128: 38 us with an atomic per token
-// and a token per CTA, 32 us now, cold; the bytes take 15).
-template <typename T, int TOKS>
+// 4 * 32 / LPR; grid = (tokens, row groups): a decode step's few tokens still spread over many CTAs.  A lane keeps its
+// piece of the row in registers between the sum of squares and the scaled write.
+template <typename T>
 __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
+    const T* __restrict__ qkv, int64_t qkv_stride, const float* __restrict__ q_w, const float* __restrict__ k_w,
+    float eps, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_slot, T* __restrict__ q_out,
+    T* __restrict__ k_cache, T* __restrict__ v_cache, PagedKV c, int32_t* __restrict__ bh_lens, int H, int G, int D,
+    int Dv, int reserved_slot, int lpr, Rotation rot, int norm) {
+  extern __shared__ float rot_cs[];   // cos [dims / 2], sin [dims / 2]
+  const int t = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = token_slot[t];
+  const int pos = positions[t];
+  const int half = rot.inv_freq ? rot.dims / 2 : 0;
+  if (half > 0) {
+    fill_rotation(rot_cs, rot_cs + half, rot, pos);
+    __syncthreads();
+  }
+  const T* row = qkv + (int64_t)t * qkv_stride;
+  const int rows_per_warp = 32 / lpr;
+  const int r = (blockIdx.y * 4 + warp) * rows_per_warp + lane / lpr;
+  const int cb = (lane % lpr) * 8;
+  const bool is_q = r < H, is_k = r >= H && r < H + G, is_v = r >= H + G && r < H + 2 * G;
+  const bool stores = slot != reserved_slot;
+  float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if ((is_q || (is_k && stores)) && cb < D) load8<T>(row + (int64_t)r * D + cb, x);
+  if (is_v && stores && cb < Dv) load8<T>(row + (int64_t)(H + G) * D + (int64_t)(r - H - G) * Dv + cb, x);
+  if (half > 0 && (is_q || is_k)) {   // the lane's four pairs of neighbours
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const int p = (cb + e) >> 1;
+      if (p < half) {
+        const float u = x[e], v = x[e + 1];
+        x[e] = u * rot_cs[p] - v * rot_cs[half + p];
+        x[e + 1] = v * rot_cs[p] + u * rot_cs[half + p];
+      }
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
+  for (int o = lpr >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // every lane takes part
+  if ((is_q || (is_k && stores)) && cb < D) {
+    const float inv = (norm & 1) ? 1.0f / sqrtf(ss / (float)D + eps) : 1.0f;
+    const float* w = (norm & 1) ? (is_q ? q_w : k_w) : nullptr;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = w ? x[e] * inv * w[cb + e] : x[e] * inv;
+    T* dst = is_q ? q_out + ((int64_t)t * H + r) * D : k_cache + cache_row(c, slot, r - H, pos) * D;
+    store8<T>(dst + cb, x);
+  }
+  if (is_v && stores) {
+    const int g = r - H - G;
+    if (cb < Dv) {
+      if (norm & 2) {
+        const float inv = 1.0f / sqrtf(ss / (float)Dv + eps);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] *= inv;
+      }
+      store8<T>(v_cache + cache_row(c, slot, g, pos) * Dv + cb, x);
+    }
+    if (cb == 0 && bh_lens) atomicMax(bh_lens + slot * G + g, pos + 1);
+  }
+}
+
+template <typename T>
+struct Raw8 {   // eight numbers as they lie in memory
+  struct alignas(16) type { uint4 v[sizeof(T) / 2]; };
+};
+
+// The same for portions: kNormTokens tokens per CTA, whose pieces are all loaded before the first is used and kept as they lie in
+// memory (as fp32 numbers they take 92 registers, 5 CTAs an SM, and
+// 16384 tokens of 20 rows of 128 took 62 us where one token a CTA takes 50 and this 45).  The
+// cache length of a slot is raised by the last token of an ascending run of its positions alone: a portion's tokens all hit
+// the same few words.  4096 tokens of 32 + 8 + 8 heads of 128: 35.3 -> 24.7 us (the bytes take 15), 16 + 2 + 2 heads: 13.6 -> 12.0.
+constexpr int kNormTokens = 4;
+template <typename T>
+__global__ void __launch_bounds__(128) qknorm_store_many_kernel(
     const T* __restrict__ qkv, int64_t qkv_stride, const float* __restrict__ q_w, const float* __restrict__ k_w,
     float eps, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_slot, T* __restrict__ q_out,
     T* __restrict__ k_cache, T* __restrict__ v_cache, PagedKV c, int32_t* __restrict__ bh_lens, int tokens, int H, int G, int D,
     int Dv, int reserved_slot, int lpr, Rotation rot, int norm) {
   extern __shared__ float rot_cs[];   // per token: cos [dims / 2], sin [dims / 2]
-  const int first = blockIdx.x * TOKS;
+  const int first = blockIdx.x * kNormTokens;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows_per_warp = 32 / lpr;
   const int r = (blockIdx.y * 4 + warp) * rows_per_warp + lane / lpr;
@@ -729,59 +799,66 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
   const int width = is_v ? Dv : D;
   const bool mine = (is_q || is_k || is_v) && cb < width;
   const int64_t at = is_v ? (int64_t)(H + G) * D + (int64_t)(r - H - G) * Dv + cb : (int64_t)r * D + cb;
-  int slot[TOKS], pos[TOKS];
-  float x[TOKS][8];
+  int slot[kNormTokens], pos[kNormTokens];
+  typename Raw8<T>::type raw[kNormTokens];
 #pragma unroll
-  for (int u = 0; u < TOKS; ++u) {
+  for (int u = 0; u < kNormTokens; ++u) {
     const bool real = first + u < tokens;
     slot[u] = real ? token_slot[first + u] : reserved_slot;
     pos[u] = real ? positions[first + u] : 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[u][e] = 0.f;
-    if (mine && real) load8<T>(qkv + (int64_t)(first + u) * qkv_stride + at, x[u]);
+    raw[u] = {};
+    if (mine && real) raw[u] = *reinterpret_cast<const typename Raw8<T>::type*>(qkv + (int64_t)(first + u) * qkv_stride + at);
+  }
+  const bool counts = is_v && cb == 0 && bh_lens;
+  int next_slot = reserved_slot, next_pos = 0;   // the token behind: loaded here, not where the kernel would wait for it
+  if (counts && first + kNormTokens < tokens) {
+    next_slot = token_slot[first + kNormTokens];
+    next_pos = positions[first + kNormTokens];
   }
   const int half = rot.inv_freq ? rot.dims / 2 : 0;
   if (half > 0) {
-#pragma unroll
-    for (int u = 0; u < TOKS; ++u) fill_rotation(rot_cs + u * 2 * half, rot_cs + u * 2 * half + half, rot, pos[u]);
+    for (int i = threadIdx.x; i < kNormTokens * half; i += blockDim.x) {   // the tokens' sines and cosines beside one another
+      const int u = i / half, p = i - u * half;
+      double sv, cv;
+      sincos((double)(first + u < tokens ? positions[first + u] : 0) * rot.inv_freq[p], &sv, &cv);
+      rot_cs[u * 2 * half + p] = (float)cv;
+      rot_cs[u * 2 * half + half + p] = (float)sv;
+    }
     __syncthreads();
   }
   const float* w = (norm & 1) && !is_v ? (is_q ? q_w : k_w) : nullptr;
-  float wr[TOKS > 1 ? 8 : 1];   // one token: read where they are used
-  if constexpr (TOKS > 1) {
+  float wr[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) wr[e] = w && mine ? w[cb + e] : 1.f;
-  }
+  for (int e = 0; e < 8; ++e) wr[e] = w && mine ? w[cb + e] : 1.f;
 #pragma unroll
-  for (int u = 0; u < TOKS; ++u) {
+  for (int u = 0; u < kNormTokens; ++u) {
     const int t = first + u;
+    float x[8];
+    load8<T>(reinterpret_cast<const T*>(&raw[u]), x);
     if (half > 0 && (is_q || is_k)) {   // the lane's four pairs of neighbours
       const float* cs = rot_cs + u * 2 * half;
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
         const int p = (cb + e) >> 1;
         if (p < half) {
-          const float a = x[u][e], b = x[u][e + 1];
-          x[u][e] = a * cs[p] - b * cs[half + p];
-          x[u][e + 1] = b * cs[p] + a * cs[half + p];
+          const float a = x[e], b = x[e + 1];
+          x[e] = a * cs[p] - b * cs[half + p];
+          x[e + 1] = b * cs[p] + a * cs[half + p];
         }
       }
     }
     float ss = 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) ss += x[u][e] * x[u][e];
+    for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
     for (int o = lpr >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // every lane takes part
     const bool stores = slot[u] != reserved_slot;
     if (t >= tokens || !(is_q || stores)) continue;
     if ((is_q || is_k) && mine) {
       const float inv = (norm & 1) ? 1.0f / sqrtf(ss / (float)D + eps) : 1.0f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if constexpr (TOKS > 1) x[u][e] = x[u][e] * inv * wr[e];
-        else x[u][e] = w ? x[u][e] * inv * w[cb + e] : x[u][e] * inv;
-      }
+      for (int e = 0; e < 8; ++e) x[e] = x[e] * inv * wr[e];
       T* dst = is_q ? q_out + ((int64_t)t * H + r) * D : k_cache + cache_row(c, slot[u], r - H, pos[u]) * D;
-      store8<T>(dst + cb, x[u]);
+      store8<T>(dst + cb, x);
     }
     if (is_v) {
       const int g = r - H - G;
@@ -789,13 +866,14 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
         if (norm & 2) {
           const float inv = 1.0f / sqrtf(ss / (float)Dv + eps);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) x[u][e] *= inv;
+          for (int e = 0; e < 8; ++e) x[e] *= inv;
         }
-        store8<T>(v_cache + cache_row(c, slot[u], g, pos[u]) * Dv + cb, x[u]);
+        store8<T>(v_cache + cache_row(c, slot[u], g, pos[u]) * Dv + cb, x);
       }
-      if (cb == 0 && bh_lens) {
-        const bool more = tokens > 64 && t + 1 < tokens && token_slot[t + 1] == slot[u] && positions[t + 1] > pos[u];
-        if (!more) atomicMax(bh_lens + slot[u] * G + g, pos[u] + 1);
+      if (counts) {
+        const int after = u + 1 < kNormTokens ? u + 1 : 0;
+        const int s1 = after ? slot[after] : next_slot, p1 = after ? pos[after] : next_pos;
+        if (!(s1 == slot[u] && p1 > pos[u])) atomicMax(bh_lens + slot[u] * G + g, pos[u] + 1);
       }
     }
   }
@@ -1284,22 +1362,35 @@ static int rope_qknorm_store_impl(const double* inv_freq, int rot_dims, int norm
     while (lpr * 8 < (D > Dv ? D : Dv)) lpr <<= 1;
     const int row_groups = cdiv(H + 2 * G, 4 * (32 / lpr));
     CVLLM_CHECK_SUPPORTED(row_groups <= 65535);
-    // four tokens a CTA from where that still leaves every SM 32 CTAs (4096 tokens of 48 rows of 128: 165.4 -> 160.4 us with the
-    // attention behind; 3748 of 32 rows of 64, a third of that work, 76.5 us with four and 74.8 with one)
-    const bool fours = (int64_t)T * row_groups >= 128 * (int64_t)sm_count() && 4 * rsmem <= 32 * 1024;
-    const dim3 grid(fours ? cdiv(T, 4) : T, row_groups);
-#define CVLLM_QKNORM(TT, KK)                                                                                                    \
-  qknorm_store_vec_kernel<TT, KK><<<grid, 128, KK * rsmem, st>>>(                                                               \
-      static_cast<const TT*>(qkv), qkv_stride, q_weight, k_weight, eps, positions, token_slot, static_cast<TT*>(q_out),         \
-      static_cast<TT*>(k_cache), static_cast<TT*>(v_cache), c, bh_lens, T, H, G, D, Dv, reserved_slot, lpr, rot, norm)
-    if (dtype == CVLLM_BF16) {
-      if (fours) CVLLM_QKNORM(__nv_bfloat16, 4);
-      else CVLLM_QKNORM(__nv_bfloat16, 1);
+    // several tokens a CTA from 96 single-token CTAs per SM on: 2523 tokens of 32 rows of 128 (68 an SM) take 16.5 / 11.3 us (one / four)
+    // in front of their attention, 4096 of 20 rows 13.6 / 12.0, 8192 of 10 rows 17.4 / 15.4; but with fewer row groups the CTAs'
+    // longer chains count: 2522 of 10 rows (34 an SM) 7.4 / 8.2, 5640 of 10 rows of 64 (38 an SM) 8.4 / 10.3
+    const int forced = test_options().qknorm_tokens.load();
+    const bool many = (forced ? forced > 1 : T > 64 && (int64_t)T * row_groups >= 96 * (int64_t)sm_count()) &&
+                      kNormTokens * rsmem <= 32 * 1024;
+    const dim3 grid(many ? cdiv(T, kNormTokens) : T, row_groups);
+    if (many) {
+      if (dtype == CVLLM_BF16)
+        qknorm_store_many_kernel<__nv_bfloat16><<<grid, 128, kNormTokens * rsmem, st>>>(
+            static_cast<const __nv_bfloat16*>(qkv), qkv_stride, q_weight, k_weight, eps, positions, token_slot,
+            static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), c,
+            bh_lens, T, H, G, D, Dv, reserved_slot, lpr, rot, norm);
+      else
+        qknorm_store_many_kernel<float><<<grid, 128, kNormTokens * rsmem, st>>>(
+            static_cast<const float*>(qkv), qkv_stride, q_weight, k_weight, eps, positions, token_slot, static_cast<float*>(q_out),
+            static_cast<float*>(k_cache), static_cast<float*>(v_cache), c, bh_lens, T, H, G, D, Dv, reserved_slot, lpr, rot, norm);
+    } else if (dtype == CVLLM_BF16) {
+      qknorm_store_vec_kernel<__nv_bfloat16><<<grid, 128, rsmem, st>>>(
+          static_cast<const __nv_bfloat16*>(qkv), qkv_stride, q_weight, k_weight, eps, positions, token_slot,
+          static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache),
+          static_cast<__nv_bfloat16*>(v_cache), c, bh_lens, H, G, D, Dv, reserved_slot, lpr, rot, norm);
     } else {
-      if (fours) CVLLM_QKNORM(float, 4);
-      else CVLLM_QKNORM(float, 1);
+      qknorm_store_vec_kernel<float><<<grid, 128, rsmem, st>>>(static_cast<const float*>(qkv), qkv_stride, q_weight,
+                                                           k_weight, eps, positions, token_slot,
+                                                           static_cast<float*>(q_out), static_cast<float*>(k_cache),
+                                                           static_cast<float*>(v_cache), c, bh_lens, H, G, D, Dv,
+                                                           reserved_slot, lpr, rot, norm);
     }
-#undef CVLLM_QKNORM
     CVLLM_CHECK_LAUNCH();
     return CVLLM_OK;
   }

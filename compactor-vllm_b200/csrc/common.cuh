@@ -101,6 +101,7 @@ struct TestOptions {
   std::atomic<int> ssm_segment{0};            // > 0: tokens per segment of the state-space scan (0: chosen per step)
   std::atomic<int> gla_layout{0};             // > 0: 100 * CTAs per (head, sequence) + columns per thread (2, 4) of the gated linear attention and the delta rule
   std::atomic<int> delta_chunk_hold{0};       // != 0: copies of one chunk of cvllm_delta_rule_chunks never begin, its waits run out after a millisecond
+  std::atomic<int> qknorm_tokens{0};          // 1, 4: tokens per CTA of the norm and store of heads (0: chosen per step)
   std::atomic<int> recur_layout{0};           // > 0: 100 * CTAs per (head, sequence) + register slice of the matrix-state mixers (0: chosen per step)
 };
 TestOptions& test_options();

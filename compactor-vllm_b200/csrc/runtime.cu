@@ -113,6 +113,7 @@ extern "C" int cvllm_set_test_option(const char* name, double value) {
   else if (!strcmp(name, "select_passes")) o.select_passes = (int)value;
   else if (!strcmp(name, "gla_layout")) o.gla_layout = (int)value;
   else if (!strcmp(name, "delta_chunk_hold")) o.delta_chunk_hold = (int)value;
+  else if (!strcmp(name, "qknorm_tokens")) o.qknorm_tokens = (int)value;
   else if (!strcmp(name, "recur_layout")) o.recur_layout = (int)value;
   else {
     cvllm::set_last_error("unknown test option");

@@ -72,6 +72,7 @@ uint64_t cvllm_launch_count(void);
  *   "ssm_segment" n          tokens per segment of cvllm_ssm_scan (0 = the product's choice; tests use short segments)
  *   "gla_layout" n           100 * CTAs per (head, sequence) + columns per thread of cvllm_gla_scan and of the portions of
  *                            cvllm_delta_rule (0 = chosen per step; < 0: cvllm_delta_rule_chunks for portions of any length)
+ *   "qknorm_tokens" 1|4      tokens per CTA of cvllm_qknorm_store and cvllm_rope_qknorm_store (0 = chosen per step)
  *   "delta_chunk_hold" n     cvllm_delta_rule_chunks: the copies of chunk n - 1 never begin for the first CTA (n < 0: of chunk
  *                            -n - 1 for head 0 of the coefficients), so that waits run out, after a millisecond each
  *   "select_passes" 1|0      cvllm_select_store_topk: the chain of launches also where one cluster per sequence would do
