@@ -124,7 +124,7 @@ uint64_t launches();
 // OFF by default (test option "pdl" = 1 turns it on): measured on the selection chain it takes 15-19 us off the eager
 // chain run alone and nothing off its CUDA-graph replay, but INSIDE the prefill step — where every SM is held by an
 // attention CTA that uses all its shared memory and registers — the early-scheduled CTAs sit on SMs while they wait,
-// and the step gets 1-2 % slower (tools/ab_pdl.py, tools/ab_overlap.py).  Without the attribute `pdl_begin()` is a no-op.
+// and the step gets 1-2 % slower (measured in alternation).  Without the attribute `pdl_begin()` is a no-op.
 // ---------------------------------------------------------------------------
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_begin() {

@@ -292,7 +292,7 @@ def _reference_arithmetic_on_device(keys, lens, phi, chunk, reg=5e-3):
     sequence (cuBLAS GEMM on the transposed view, in-place mean subtraction, batched Gram GEMM, 16-bit roundings
     where torch puts them) — with the `gesvda` SVD replaced by the factorisation it approximates: fp64 `eigh`
     of the fp32 Gram, S = |lambda|.  On the B200 the unmodified reference is itself only 99.25 % within 2e-2 of
-    this on low-rank keys (profiles/r02c_leverage_selfdistance.json: ref_eigh64_vs_ref) while this repo is at
+    this on low-rank keys (profiles/leverage_selfdistance_exact_order.json: ref_eigh64_vs_ref) while this repo is at
     100.00 % (ours_vs_eigh64), so this is the tighter pin."""
     X = torch.matmul(keys.transpose(0, 1), phi)  # [H, N, k]
     H, N, k = X.shape

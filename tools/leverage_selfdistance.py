@@ -1,6 +1,6 @@
 """How far is the reference's leverage scorer from ITSELF, and how far is this repo from it? 
 
-    python tools/leverage_selfdistance.py            # both sides as subprocesses -> gpurun_out/r02_leverage_selfdistance.json
+    python tools/leverage_selfdistance.py            # both sides as subprocesses -> leverage_selfdistance.json in $CVLLM_REPORTS
 
 `approximate_leverage_scores` (reference compression/compactor.py:113-221) inverts 48x48 Gram matrices that were
 rounded to bf16 entrywise; with low-rank keys the small singular values of that rounded Gram are rounding noise, so
@@ -198,9 +198,9 @@ def compare(n_tok):
         rows["full_chain_ours_vs_ref"] = full
         rows["blend_formula_check_ref"] = _stats(torch, e2e_ref, a[f"{kind}/ref_e2e"])
         rep["inputs"][kind] = rows
-    out = ROOT / "gpurun_out"
-    out.mkdir(exist_ok=True)
-    (out / "r02_leverage_selfdistance.json").write_text(json.dumps(rep, indent=1))
+    out = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports"))
+    out.mkdir(parents=True, exist_ok=True)
+    (out / "leverage_selfdistance.json").write_text(json.dumps(rep, indent=1))
     print(json.dumps(rep, indent=1))
 
 
@@ -218,8 +218,8 @@ def main():
         t0 = time.time()
         p = subprocess.run([sys.executable, __file__, "--side", side, "--tokens", str(a.tokens)], env=env,
                            capture_output=True, text=True, timeout=1200)
-        log = ROOT / "gpurun_out" / f"levself_{side}.log"
-        log.parent.mkdir(exist_ok=True)
+        log = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports")) / f"levself_{side}.log"
+        log.parent.mkdir(parents=True, exist_ok=True)
         log.write_text(p.stdout[-20000:] + "\n--- stderr ---\n" + p.stderr[-20000:])
         print(f"[{side}] rc={p.returncode} {time.time() - t0:.0f}s", flush=True)
         if p.returncode != 0:

@@ -5,11 +5,12 @@ from cuBLAS / torch: the sketch X = K.PHI (bf16), the chunk mean (bf16), the cen
 Ours come from the library's workspace (mean, Gram) and from the fused norm+RoPE kernel's sketch output (same
 fragment order as the leverage kernel, tests/test_gpu_prepath.py); theirs are the reference's torch calls restated
 on the same device (torch.matmul / mean / sub_, same shapes, strides and batching as the reference issues).
--> gpurun_out/r02_leverage_stage_diff.json
+-> leverage_stage_diff.json in $CVLLM_REPORTS
 """
 from __future__ import annotations
 
 import json
+import os
 import math
 import sys
 from pathlib import Path
@@ -84,9 +85,9 @@ def main():
         r["our_gram_vs_exactly_rounded_entries_differ"] = int((Go != ex).sum())
         rep[kind] = r
         print(kind, json.dumps(r), flush=True)
-    out = ROOT / "gpurun_out"
-    out.mkdir(exist_ok=True)
-    (out / "r02_leverage_stage_diff.json").write_text(json.dumps(rep, indent=1))
+    out = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports"))
+    out.mkdir(parents=True, exist_ok=True)
+    (out / "leverage_stage_diff.json").write_text(json.dumps(rep, indent=1))
 
 
 if __name__ == "__main__":

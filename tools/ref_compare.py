@@ -9,7 +9,7 @@ packages expose the same names and signatures, so the SAME driver code below run
 drop-in claim made executable.  Inputs come from seeded CUDA generators (identical on both sides), outputs are
 compared by the parent: attention within the bf16 tolerance, scores within 2e-2*max(1,|s|), kept sets / bh_lens /
 stored rows bit-exact given identical scores.  Timings: CUDA events, warm-up first (Triton autotune), L2 flushed
-before every timed call.  Report -> gpurun_out/ref_compare.json (+ a table on stdout).
+before every timed call.  Report -> ref_compare.json in $CVLLM_REPORTS (default: build/reports) (+ a table on stdout).
 """
 from __future__ import annotations
 
@@ -369,8 +369,8 @@ def compare():
         speed[key] = {"ref": r[key], "ours": o[key], "ratio": o[key] / r[key]}
     rep = {"what": "unmodified reference (Triton, baseline/_ref) vs this repo on the same B200, same seeded inputs",
            "reference_build_notes": r.get("build_notes", {}), "parity": par, "timing": speed}
-    out = ROOT / "gpurun_out"
-    out.mkdir(exist_ok=True)
+    out = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports"))
+    out.mkdir(parents=True, exist_ok=True)
     (out / "ref_compare.json").write_text(json.dumps(rep, indent=1))
     print(json.dumps(rep, indent=1))
 
@@ -389,8 +389,8 @@ def main():
         t0 = time.time()
         cmd = [sys.executable, __file__, "--side", side] + (["--quick"] if a.quick else [])
         p = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=1500)
-        log = ROOT / "gpurun_out" / f"ref_compare_{side}.log"
-        log.parent.mkdir(exist_ok=True)
+        log = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports")) / f"ref_compare_{side}.log"
+        log.parent.mkdir(parents=True, exist_ok=True)
         log.write_text(p.stdout[-20000:] + "\n--- stderr ---\n" + p.stderr[-20000:])
         print(f"[{side}] rc={p.returncode} {time.time() - t0:.0f}s", flush=True)
         if p.returncode != 0:

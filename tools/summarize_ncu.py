@@ -1,16 +1,17 @@
-"""Turn gpurun_out/{launches.csv, prof_*.ncu-rep} into the tracked summaries under profiles/.
+"""Turn $CVLLM_REPORTS/{launches.csv, prof_*.ncu-rep} into the tracked summaries under profiles/.
 
-    python tools/summarize_ncu.py r01            # prefix for the output files
+    python tools/summarize_ncu.py dense            # prefix for the output files
 """
 import collections
 import csv
 import json
+import os
 import subprocess
 import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
-OUT = ROOT / "gpurun_out"
+OUT = Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports"))
 PROF = ROOT / "profiles"
 KEYS = [
     "gpu__time_duration.sum", "dram__bytes_read.sum", "dram__bytes_write.sum",

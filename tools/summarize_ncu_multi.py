@@ -1,11 +1,12 @@
 """Per-kernel summary of one multi-kernel `ncu --set full` report -> profiles/<prefix>_<tag>.json
 
-    python tools/summarize_ncu_multi.py gpurun_out/prof_scoring.ncu-rep r02 scoring_kernels
+    python tools/summarize_ncu_multi.py prof_scoring.ncu-rep dense scoring_kernels
 One entry per distinct kernel name (the LAST launch of each: warm caches for code, same data), with duration, DRAM
 bytes, achieved DRAM GB/s, tensor / xu / fma pipe utilisation, issue-slot utilisation, occupancy, registers.
 """
 import csv
 import json
+import os
 import subprocess
 import sys
 from pathlib import Path

@@ -43,4 +43,4 @@ for g in (0, 1):
     issued = t[1 + 2 * g]  # S_g(j+1) issued at row 1/3 of iteration j
     print(f"  head {g}: S(j+1) issued -> softmax woke {med(w[1:] - issued[:-1]):.0f} | softmax woke -> arrived {med(a - w):.0f} | "
           f"arrived -> issuer woke {med(t[2 * g] - a):.0f}")
-np.save(str(ROOT / "gpurun_out" / f"prefill_trace_{os.environ.get('CVLLM_LIB', 'default').split('/')[-1]}.npy"), buf)
+np.save(str(Path(os.environ.get("CVLLM_REPORTS", ROOT / "build" / "reports")) / f"prefill_trace_{os.environ.get('CVLLM_LIB', 'default').split('/')[-1]}.npy"), buf)
