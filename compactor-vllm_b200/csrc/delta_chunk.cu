@@ -755,23 +755,22 @@ __device__ __forceinline__ void take_product(uint32_t addr, float2 (&v)[8]) {
 constexpr int kFirst = 4;
 __device__ __forceinline__ void take_first(uint32_t addr, float2 (&v)[8]) {
   auto pair = [](const uint32_t (&x)[16], int j) { return make_float2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])); };
-  uint32_t x[3][16];
-  float2 small[8];
-  tmem_ld16(addr + kFirst * kCols, x[0]);
-  tmem_ld16(addr + (kFirst + 1) * kCols, x[1]);
-  tmem_ld16(addr, x[2]);
+  uint32_t x[2][16];
+  tmem_ld16(addr, x[0]);
+  tmem_ld16(addr + kCols, x[1]);
   tc_wait_ld();
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    small[j] = __fadd2_rn(pair(x[0], j), pair(x[1], j));
-    v[j] = pair(x[2], j);
-  }
-#pragma unroll
-  for (int e = 1; e < kFirst; ++e) tmem_ld16(addr + e * kCols, x[e - 1]);
+  for (int j = 0; j < 8; ++j) v[j] = __fadd2_rn(pair(x[0], j), pair(x[1], j));
+  tmem_ld16(addr + 2 * kCols, x[0]);
+  tmem_ld16(addr + 3 * kCols, x[1]);
   tc_wait_ld();
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
-    v[j] = __fadd2_rn(__fadd2_rn(__fadd2_rn(v[j], pair(x[0], j)), __fadd2_rn(pair(x[1], j), pair(x[2], j))), small[j]);
+  for (int j = 0; j < 8; ++j) v[j] = __fadd2_rn(v[j], __fadd2_rn(pair(x[0], j), pair(x[1], j)));
+  tmem_ld16(addr + 4 * kCols, x[0]);
+  tmem_ld16(addr + 5 * kCols, x[1]);
+  tc_wait_ld();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = __fadd2_rn(v[j], __fadd2_rn(pair(x[0], j), pair(x[1], j)));
 }
 
 template <typename T, int D>

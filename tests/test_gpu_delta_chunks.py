@@ -3,7 +3,10 @@ in 64 bits: chunks that are full, one token short and one token long, heads that
 both types, and portions whose images exceed the workspace's bound and are taken in windows; the convolution in front with
 its rows in four-channel pieces and without.
 
-Tolerances are those of test_gpu_delta_layouts.py: operands in three bfloat16 parts are good to 2^-26, the sums are fp32."""
+Tolerances: operands in three bfloat16 parts are good to 2^-26, coefficients are 64-bit, the tensor pipe's sums of 64 and 128
+products fp32.  Measured over the sizes here 1.2e-7 to 3.5e-7 in 32-bit outputs and states; the bound is about twice that, where
+a build without the third parts lies at 4e-6 and above.  bfloat16 rows are rounded at the output only: 2^-9 / sqrt(3) = 1.1e-3,
+and 2.5e-3 is twice that."""
 import ctypes
 
 import pytest
@@ -45,8 +48,9 @@ def check(size, lens, starts, dtype, seed=5, odd_rows=False):
     assert launched == 1 if odd_rows else launched >= 3 and launched % 3 == 0
     assert aborts() == before
     err = lambda x, y: ((x - y).norm() / y.norm()).item()
-    assert err(got, want) < (1e-5 if dtype == torch.float32 else 2.5e-3)
-    assert err(state.matrix_state[1:].double(), want_state[1:]) < 1e-5
+    near = 1e-5 if odd_rows else 7e-7       # the blocks of four: test_gpu_delta_layouts.py
+    assert err(got, want) < (near if dtype == torch.float32 else 2.5e-3), err(got, want)
+    assert err(state.matrix_state[1:].double(), want_state[1:]) < near, err(state.matrix_state[1:].double(), want_state[1:])
     assert torch.equal(state.matrix_state[0], untouched)
     return launched
 
