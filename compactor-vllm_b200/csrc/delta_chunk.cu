@@ -29,13 +29,14 @@
 // What is not finite stays behind its token: an element of R that is infinite or NaN would meet zeros of P T in earlier
 // tokens' rows, so it enters the products as 0 and its column becomes NaN from that token on.
 //
-// Measured (one portion of 4096 tokens, 32 / 16 heads of 128 x 128, which took the kernel of blocks of four 950 us): rows 45 us (their
-// bytes take 29), coefficients 120 us (issue, 0.45 instructions per scheduler and cycle, and the barriers between short phases, two
-// CTAs an SM), chunks 226 us.  What bounds the last: a chain per chunk of two products (24 of 128 x 96, 64 and 32, 12 of the same)
-// and two turns through registers of some 1000 cycles each, on 128 SMs; and shared memory, which carries 450 KB a chunk (operand
-// reads 288, copies 168).  Tried: three products in sequence without C (248 us, coefficients and rows together 113); the columns in
-// two groups that alternate (339: twice the operand reads); K S alone at 64 rows with Q S behind it (277); the gates' factors on two
-// warps beside the issuing one (269); copies paced to arrive between the products (the same).
+// Measured (one portion of 4096 tokens, 32 / 16 heads of 128 x 128, which takes the kernel of blocks of four 927 us): rows 58 us (their
+// bytes take 32; 45 with products in 32 bits), coefficients 126 us (barriers between short phases, 3.4 of the 11 cycles between two
+// instructions of a warp, two CTAs an SM; 120 in 32 bits), chunks 214 us.  What bounds the last: a chain per chunk of two
+// products (32 + 64, 64 and 32 columns of 128, 12 of 96, 64 and 32) and two turns through registers of some 1000 cycles each, on 128
+// SMs; and shared memory, whose operand reads and copies take about two thirds of a chunk's cycles at 128 bytes each.  Tried: three
+// products in sequence without C (248 us where this form then took 226); the columns in two groups that alternate (339: twice the
+// operand reads); K S alone at 64 rows with Q S behind it (277); the gates' factors on two warps beside the issuing one (269);
+// copies paced to arrive between the products (the same).
 //
 // Every wait has a limit.  A wait that runs out sets the CTA's abort flag; all roles then leave their loops, copies and
 // products in flight are waited for (with a limit), the CTA's state and its columns of the launch's rows become NaN and a counter
