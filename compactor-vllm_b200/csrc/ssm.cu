@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128) causal_conv_run_kernel(const T* __restric
 // The same with four neighbouring channels per thread (rows of 16-bit inputs in 8-byte, of fp32 ones in 16-byte pieces; outputs
 // likewise) and four tokens' rows loaded before the first is used.  An output is 4 multiply-adds and a silu: with one channel
 // per thread, a row at a time and a division's branch per silu, 4096 tokens of 8192 channels took 88 us where their bytes (0.2
-// GB) take 31.  grid (token runs, B, channel tiles of 512), 128 threads.
+// GB) take 31; now 51, bound by issue.  grid (token runs, B, channel tiles of 512), 128 threads.
 template <typename T>
 struct Four {   // four numbers of type T as they lie in memory
   using raw = typename std::conditional<sizeof(T) == 2, uint2, uint4>::type;
@@ -686,7 +686,9 @@ int launch_conv(const void* proj, int64_t proj_stride, int x_off, int channels, 
   const T* in = static_cast<const T*>(proj);
   const T* cs = static_cast<const T*>(conv_state);
   TO* o = static_cast<TO*>(out);
-  // four channels a thread where their pieces are aligned and a portion fills a run (a few tokens are latency: more CTAs)
+  // four channels a thread where their pieces are aligned and a portion fills a run (one channel / four, us: 32 tokens of 512
+  // channels 9.0 / 8.2, of 8192 9.2 / 8.2, 4096 of 512 10.2 / 8.7, 512 and 15 times 20 of 2048 12.5 / 11.0; below, where more CTAs are
+  // under way with one channel a thread, 4 tokens 3.1 / 3.4, 8 of 512 4.1 / 4.2, 16 5.9 / 5.7)
   const auto pieces = [](const void* p, int64_t stride, size_t elem) {
     return reinterpret_cast<uintptr_t>(p) % (4 * elem) == 0 && stride % 4 == 0;
   };
