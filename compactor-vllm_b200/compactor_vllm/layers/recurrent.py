@@ -127,7 +127,7 @@ class DeltaRuleMixer(nn.Module):
                 need = 0
         if need:
             try:
-                ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to 320 MB: given back after the call
+                ws = torch.empty(need, dtype=torch.uint8, device=dev)   # up to 400 MB: given back after the call
             except torch.OutOfMemoryError:      # the other kernel needs none
                 need = 0
         if need:

@@ -1160,7 +1160,7 @@ ChunkPlan chunk_plan(int64_t tokens, int B, int max_new, int H, int G, int D, in
   const int chunks = cdiv(max_new, kChunk);
   p.windows = (int)((all + most - 1) / most);
   p.slots = (int)((all + p.windows - 1) / p.windows);
-  if (p.windows > 1 && B <= most && B * state <= kMost && 4 * tokens >= 3 * (int64_t)B * max_new &&
+  if (p.windows > 1 && B <= most && B * state <= kMost / 4 && 4 * tokens >= 3 * (int64_t)B * max_new &&
       (p.slots / chunks + 1) * (int64_t)H * (Dv / kCols) < sm_count()) {
     p.per_seq = (int)std::min<int64_t>(most / B, chunks);
     p.windows = cdiv(chunks, p.per_seq);

@@ -791,7 +791,7 @@ int cvllm_delta_rule(const float* qkv, int64_t qkv_stride, const void* proj, int
 
 /* The same portions in chunks of 64 tokens on the tensor cores, operands in three bfloat16 parts (D 64 or 128, Dv a
  * multiple of 32 up to 256; qkv, gate, out and workspace on 16 bytes, rows in multiples of 16 bytes).  `tokens`: rows of qkv,
- * cu_seqlens_q[B] at least.  The workspace (up to 320 MB and two states; above that the chunks are taken in windows) has size 0
+ * cu_seqlens_q[B] at least.  The workspace (up to 400 MB; images above 320 MB are taken in windows of chunks) has size 0
  * where cvllm_delta_rule is the one to call: other sizes, and where it is the faster. */
 size_t cvllm_delta_rule_chunks_workspace_bytes(int64_t tokens, int B, int max_new, int H, int G, int D, int Dv);
 int cvllm_delta_rule_chunks(const float* qkv, int64_t qkv_stride, const void* proj, int64_t proj_stride, int b_off, int a_off,
