@@ -8,7 +8,7 @@
 //   X   = round16(K_h . PHI)                mma.sync, K rows straight from global
 //   Xc  = round16(X - round16(mean_t X))    per chunk
 //   G   = fp32(round16(Xc^T Xc)) + reg*I    mma.sync on the transposed sketch
-//   G   = V diag(lam) V^T                   Householder + implicit QL, fp32, one warp per matrix
+//   G   = V diag(lam) V^T                   Householder + divide and conquer, fp64, one CTA per matrix
 //   u   = round16(Xc . round16(V |lam|^-1/2));  score = round16(sum_j round16(u_j^2))
 //
 // The reference keeps X, Xc, G, V S^-1/2, U and the row sums in K's 16-bit
@@ -21,6 +21,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "leverage_eig.cuh"
 #include "mma.cuh"
 
 namespace cvllm {
@@ -251,356 +252,7 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const Lev
   if (tid < kSk) p.mean[(int64_t)(ch * p.HKV + h) * kSk + tid] = sm.mean[tid];
 }
 
-// ---- kernel 2: symmetric eigendecomposition in fp64, one 128-thread CTA per 48x48 matrix ----
-// Why fp64: the reference's gesvda result agrees with the EXACT (fp64) eigendecomposition of the same
-// fp32 Gram to 99.3 % of the scores within 2e-2 on low-rank keys, while any norm-wise backward-stable
-// fp32 solver (cuSOLVER gesvd / gesvdj, and an earlier fp32 QL here) only reaches 60-85 %
-// (profiles/leverage_selfdistance_before.json): |lam| ranges over 1e-2 .. 1e5, and an absolute
-// error of eps32 * |lam|_max ~ 1e-2 destroys the small eigenpairs that dominate x^T |G|^-1 x.
-//
-// Structure (EISPACK tred2 / tql2 restated for a CTA):
-//   phase 1  all 4 warps: Householder reduction to tridiagonal form (matvec and rank-2 update spread over
-//            128 threads, lanes own COLUMNS so every shared-memory access is conflict-free).
-//   phase 2  warps 1-3: accumulate the reflectors into Z (in place)        } concurrently
-//   phase 3  warp 0: implicit-shift QL on (d, e) ONLY — the rotations do   }
-//            not depend on Z, so they are streamed through a ring in shared memory as (c, s) pairs, one
-//            sweep at a time, and warps 1-2 apply them to the rows of Z behind the producer.
-// The QL recurrence is the latency chain (~2000 dependent rotations).  It is rewritten so that one
-// rotation costs fma -> rsqrt -> mul on the dependent path:  with r^2 = p^2 + e_i^2, c = p/r, s = e_i/r,
-//   p_next = c d_i - s (c_prev e_i) = (p d_i - e_i^2 c_prev) / r,
-// and the numerator does not wait for 1/r.  1/r = rsqrt.approx.f64 + one third-order (Halley) step.
-// out: sv[mat][48][48] = round16(V |lam|^-1/2)   (compactor.py:197: S of a symmetric G is |lam|);
-// the column (eigenpair) order is arbitrary, the score sums over all of them.
-constexpr int kEigThreads = 128;
-constexpr int kEigRing = 1024;  // (c, s) entries; one sweep needs <= 48
-struct EigSmem {
-  double a[kSk][kSk + 1];  // A, then Z in place
-  double d[kSk], e[kSk], hh[kSk], hinv[kSk], u[kSk], q[kSk];
-  double part[2][64];
-  double2 ring[kEigRing];
-  double2 pr[kSk];  // (p_i, 1/r_i) of the current QL sweep
-  int produced, done;
-  int consumed[2];
-};
-
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ double rsqrt64(double x) {  // x > 0, normal: seed 2^-22, Halley -> fp64
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ double rcp64(double x) {  // x != 0, normal
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
-}
-__device__ __forceinline__ void bar_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-__device__ __forceinline__ int ld_volatile_s(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
-__device__ __forceinline__ void st_volatile_s(int* p, int v) { *reinterpret_cast<volatile int*>(p) = v; }
-
-template <bool BF16>
-__global__ void __launch_bounds__(kEigThreads) leverage_eig_kernel(const float* __restrict__ gram,
-                                                                   float* __restrict__ sv_out,
-                                                                   const int32_t* __restrict__ chunk_offsets,
-                                                                   int HKV, int mats, double* __restrict__ dbg_lam,
-                                                                   double* __restrict__ dbg_vec,
-                                                                   long long* __restrict__ dbg_clk) {
-  __shared__ __align__(16) EigSmem s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int mat = blockIdx.x;
-  if (mat >= mats) return;
-  if (chunk_offsets) {
-    const int ch = mat / HKV;
-    if (chunk_offsets[ch + 1] - chunk_offsets[ch] <= 0) return;
-  }
-  constexpr int n = kSk;
-  constexpr int R1 = kEigRing - 1;
-  const float* gin = gram + (int64_t)mat * n * n;
-  for (int i = tid; i < n * n; i += kEigThreads) s.a[i / n][i % n] = (double)gin[i];
-  if (tid == 0) { s.produced = 0; s.done = 0; s.consumed[0] = 0; s.consumed[1] = 0; }
-  __syncthreads();
-  if (dbg_clk && tid == 0) dbg_clk[mat * 6 + 0] = clock64();
-
-  // ---- phase 1: Householder reduction to tridiagonal form; u^(i) is parked in column i (rows < i) ----
-  {
-    const int col = tid & 63, half = tid >> 6;
-    for (int i = n - 1; i >= 2; --i) {
-      // every warp forms the reflector of row i redundantly (no broadcast round trip)
-      double x0 = (lane < i) ? s.a[i][lane] : 0.0;
-      double x1 = (lane + 32 < i) ? s.a[i][lane + 32] : 0.0;
-      const double h = warp_sum_d(fma(x0, x0, x1 * x1));
-      if (!(h > 1e-280)) {  // row already reduced (or not finite): H_i = I.  Uniform over the CTA.
-        if (tid == 0) { s.e[i] = 0.0; s.hh[i] = 0.0; s.hinv[i] = 0.0; s.d[i] = s.a[i][i]; }
-        continue;
-      }
-      const double f = s.a[i][i - 1];
-      const double g = -copysign(h * rsqrt64(h), f);
-      const double hi = h - f * g;
-      const double rh = rcp64(hi);
-      if (lane == ((i - 1) & 31)) {
-        if (i - 1 < 32) x0 = f - g; else x1 = f - g;
-      }
-      if (warp == 0) {
-        if (lane < i) { s.u[lane] = x0; s.a[lane][i] = x0; }
-        if (lane + 32 < i) { s.u[lane + 32] = x1; s.a[lane + 32][i] = x1; }
-        if (lane == 0) { s.e[i] = g; s.hh[i] = hi; s.hinv[i] = rh; s.d[i] = s.a[i][i]; }
-      }
-      __syncthreads();
-      // p = A u / h: thread (col, half) sums rows k = half, half+2, ... of column col (A is symmetric)
-      if (col < i) {
-        double acc0 = 0.0, acc1 = 0.0;
-        int k = half;
-        for (; k + 2 < i; k += 4) {
-          acc0 = fma(s.a[k][col], s.u[k], acc0);
-          acc1 = fma(s.a[k + 2][col], s.u[k + 2], acc1);
-        }
-        for (; k < i; k += 2) acc0 = fma(s.a[k][col], s.u[k], acc0);
-        s.part[half][col] = acc0 + acc1;
-      }
-      __syncthreads();
-      const double p0 = (lane < i) ? (s.part[0][lane] + s.part[1][lane]) * rh : 0.0;
-      const double p1 = (lane + 32 < i) ? (s.part[0][lane + 32] + s.part[1][lane + 32]) * rh : 0.0;
-      const double K = warp_sum_d(fma(x0, p0, x1 * p1)) * 0.5 * rh;
-      if (warp == 0) {
-        if (lane < i) s.q[lane] = fma(-K, x0, p0);
-        if (lane + 32 < i) s.q[lane + 32] = fma(-K, x1, p1);
-      }
-      __syncthreads();
-      // A <- A - u q^T - q u^T on the leading i x i block (kept fully symmetric)
-      if (col < i) {
-        const double uc = s.u[col], qc = s.q[col];
-        for (int j = half; j < i; j += 2) s.a[j][col] -= fma(s.u[j], qc, s.q[j] * uc);
-      }
-      __syncthreads();
-    }
-    if (tid == 0) {
-      s.d[0] = s.a[0][0]; s.d[1] = s.a[1][1];
-      s.e[1] = s.a[1][0]; s.e[0] = 0.0;
-      s.a[0][0] = 1.0;
-    }
-    __syncthreads();
-  }
-
-  if (dbg_clk && tid == 0) dbg_clk[mat * 6 + 1] = clock64();
-  if (warp == 0) {
-    // ---- phase 3 (producer): implicit-shift QL on (d, e); rotations -> ring ----
-    {
-      const double e0 = s.e[lane + 1];
-      const double e1 = (lane + 33 < n) ? s.e[lane + 33] : 0.0;
-      __syncwarp();
-      s.e[lane] = e0;
-      if (lane + 32 < n) s.e[lane + 32] = e1;
-      __syncwarp();
-    }
-    double fsh = 0.0, tst1 = 0.0;
-    int prod = 0;
-    const double eps = 2.3e-13;  // 2^-42: |lam| is needed to ~1e-4 relative at |lam| >= reg = 5e-3
-    for (int l = 0; l < n; ++l) {
-      tst1 = fmax(tst1, fabs(s.d[l]) + fabs(s.e[l]));
-      // first m >= l with a negligible e[m] (e[n-1] == 0 ends the scan): two ballots instead of a serial walk
-      int m;
-      {
-        const double thr = eps * tst1;
-        const bool n0 = (lane >= l) && !(fabs(s.e[lane]) > thr);
-        const bool n1 = (lane + 32 >= l) && (lane + 32 >= n || !(fabs(s.e[lane + 32 < n ? lane + 32 : n - 1]) > thr));
-        const unsigned b0 = __ballot_sync(0xffffffffu, n0), b1 = __ballot_sync(0xffffffffu, n1);
-        m = b0 ? (__ffs(b0) - 1) : (32 + __ffs(b1) - 1);
-        if (m > n - 1) m = n - 1;
-      }
-      if (m > l) {
-        int iter = 0;
-        double el_abs;
-        do {
-          ++iter;
-          const double g0 = s.d[l], el = s.e[l], el1 = s.e[l + 1];
-          const double pp = (s.d[l + 1] - g0) * rcp64(2.0 * el);
-          const double x2 = fma(pp, pp, 1.0);
-          double rr = x2 * rsqrt64(x2);
-          if (pp < 0.0) rr = -rr;
-          const double ppr = pp + rr;
-          const double inv = rcp64(ppr);
-          const double dl = el * inv, dl1 = el * ppr;
-          const double hs = g0 - dl;
-          const double dj0 = s.d[lane], dj1 = (lane + 32 < n) ? s.d[lane + 32] : 0.0;
-          __syncwarp();
-          if (lane >= l + 2) s.d[lane] = dj0 - hs;
-          if (lane + 32 >= l + 2 && lane + 32 < n) s.d[lane + 32] = dj1 - hs;
-          if (lane == 0) { s.d[l] = dl; s.d[l + 1] = dl1; }
-          __syncwarp();
-          fsh += hs;
-          double p = s.d[m];
-          // ring space for this sweep: header + (m - l) rotations
-          const int need = m - l + 1;
-          while (prod + need - min(ld_volatile_s(&s.consumed[0]), ld_volatile_s(&s.consumed[1])) > kEigRing)
-            __nanosleep(64);
-          if (lane == 0) s.ring[prod & R1] = make_double2((double)l, (double)m);
-          // Warps issue in order, so anything between two links of the dependent chain delays it.  The loop
-          // therefore carries ONLY the recurrence (12 fp64 ops, p -> r^2 -> 1/r -> p on the chain) and parks
-          // (p_i, 1/r_i) in shared memory; the new d / e entries and the (c, s) ring records of the whole sweep
-          // are then formed by the lanes in parallel, one rotation per lane.  198 -> 86 cycles per rotation
-          // (tools/ubench/ql_chain.cu).
-          {
-            double c = 1.0;
-            double ei = s.e[m - 1], di = s.d[m - 1];
-            for (int i = m - 1; i >= l; --i) {
-              const double ein = (i > l) ? s.e[i - 1] : 0.0, din = (i > l) ? s.d[i - 1] : 0.0;  // prefetch
-              const double t = ei * ei;
-              const double r2 = fma(p, p, fma(ei, ei, 1e-300));  // > 0: no guard on the chain
-              const double qv = fma(p, di, -(t * c));            // r (c_new d_i - s_new g): does not wait for 1/r
-              double y;
-              asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-              const double er = fma(-r2 * y, y, 1.0);
-              const double ri = fma(y * er, fma(0.375, er, 0.5), y);
-              if (lane == 0) s.pr[i] = make_double2(p, ri);
-              c = p * ri;
-              p = ri * qv;
-              ei = ein; di = din;
-            }
-          }
-          __syncwarp();
-          // rotation i = m-1-k on lane k (and k+32): reads first, then writes (e[i+1] is another lane's e_i)
-          double o_e[2], o_d[2], o_c[2], o_s[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int k = lane + 32 * u, i = m - 1 - k;
-            o_e[u] = o_d[u] = o_c[u] = o_s[u] = 0.0;
-            if (i >= l) {
-              const double2 a = s.pr[i];
-              const double e_i = s.e[i], d_i = s.d[i];
-              const double c_i = a.x * a.y, s_i = e_i * a.y;
-              double c_p = 1.0, s_p = 0.0;
-              if (i < m - 1) {
-                const double2 b = s.pr[i + 1];
-                c_p = b.x * b.y;
-                s_p = s.e[i + 1] * b.y;
-              }
-              const double g = c_p * e_i, h = c_p * a.x;
-              const double r = fma(a.x, a.x, e_i * e_i) * a.y;
-              o_e[u] = s_p * r;
-              o_d[u] = h + s_i * fma(c_i, g, s_i * d_i);
-              o_c[u] = c_i;
-              o_s[u] = s_i;
-            }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int k = lane + 32 * u, i = m - 1 - k;
-            if (i >= l) {
-              s.e[i + 1] = o_e[u];
-              s.d[i + 1] = o_d[u];
-              s.ring[(prod + 1 + k) & R1] = make_double2(o_c[u], o_s[u]);
-            }
-          }
-          __syncwarp();
-          // s_l, s_{l+1}, c_l, c_{l+2} of this sweep (absent rotations: s = 0, c = 1)
-          const int nrot = m - l;
-          const double2 q0 = s.ring[(prod + nrot) & R1];
-          const double sn = q0.y, c = q0.x;
-          const double s2 = (nrot >= 2) ? s.ring[(prod + nrot - 1) & R1].y : 0.0;
-          const double c3 = (nrot >= 3) ? s.ring[(prod + nrot - 2) & R1].x : 1.0;
-          const double pe = -sn * s2 * c3 * el1 * inv;  // = -s s2 c3 e[l+1] e[l] / d[l+1] with d[l+1] = e[l] (pp + rr)
-          el_abs = fabs(sn * pe);
-          __syncwarp();
-          if (lane == 0) { s.e[l] = sn * pe; s.d[l] = c * pe; }
-          prod += need;
-          __threadfence_block();
-          if (lane == 0) st_volatile_s(&s.produced, prod);
-          __syncwarp();
-        } while (el_abs > eps * tst1 && iter < 60);
-      }
-      __syncwarp();
-      if (lane == 0) { s.d[l] += fsh; s.e[l] = 0.0; }
-      __syncwarp();
-    }
-    __threadfence_block();
-    if (lane == 0) st_volatile_s(&s.done, 1);
-    if (dbg_clk && lane == 0) { dbg_clk[mat * 6 + 2] = clock64(); dbg_clk[mat * 6 + 5] = prod; }
-  } else {
-    // ---- phase 2 (warps 1-3): Z = H_{n-1} ... H_2, built in place; thread owns (column, row parity) ----
-    const int t2 = tid - 32, zc = t2 % n, zp = t2 / n;
-    for (int i = 2; i <= n; ++i) {
-      // row / column i-1 of the growing block become the identity (column i-1 held u^(i-1), consumed)
-      for (int idx = t2; idx < i - 1; idx += 96) { s.a[i - 1][idx] = 0.0; s.a[idx][i - 1] = 0.0; }
-      if (t2 == 0) s.a[i - 1][i - 1] = 1.0;
-      bar_sync(1, 96);
-      if (i < n && s.hh[i] != 0.0) {
-        if (zc < i) {
-          double acc0 = 0.0, acc1 = 0.0;
-          int k = zp;
-          for (; k + 2 < i; k += 4) {
-            acc0 = fma(s.a[k][i], s.a[k][zc], acc0);
-            acc1 = fma(s.a[k + 2][i], s.a[k + 2][zc], acc1);
-          }
-          for (; k < i; k += 2) acc0 = fma(s.a[k][i], s.a[k][zc], acc0);
-          s.part[zp][zc] = acc0 + acc1;
-        }
-        bar_sync(1, 96);
-        if (zc < i) {
-          const double g = (s.part[0][zc] + s.part[1][zc]) * s.hinv[i];
-          for (int k = zp; k < i; k += 2) s.a[k][zc] = fma(-g, s.a[k][i], s.a[k][zc]);
-        }
-        bar_sync(1, 96);
-      }
-    }
-    if (dbg_clk && t2 == 0) dbg_clk[mat * 6 + 3] = clock64();
-    // ---- phase 3 (consumers, warps 1-2): apply the rotation stream to the rows of Z ----
-    if (warp <= 2) {
-      const bool active = t2 < n;
-      const int row = active ? t2 : 0;
-      int cons = 0;
-      for (;;) {
-        const int dn = ld_volatile_s(&s.done);
-        const int pr = ld_volatile_s(&s.produced);
-        __threadfence_block();
-        if (pr == cons) {
-          if (dn) break;
-          __nanosleep(100);
-          continue;
-        }
-        while (cons < pr) {  // whole sweeps are published at once
-          const double2 hd = s.ring[cons & R1];
-          const int l = (int)hd.x, m = (int)hd.y, cnt = m - l;
-          double z = s.a[row][m];
-          int slot = (cons + 1) & R1;
-          for (int k = 0, i = m - 1; k < cnt; ++k, --i) {
-            const double2 cs = s.ring[slot];
-            slot = (slot + 1) & R1;
-            const double y = s.a[row][i];
-            if (active) s.a[row][i + 1] = fma(cs.y, y, cs.x * z);
-            z = fma(cs.x, y, -cs.y * z);
-          }
-          if (active) s.a[row][l] = z;
-          cons += cnt + 1;
-        }
-        __syncwarp();
-        __threadfence_block();
-        if (lane == 0) st_volatile_s(&s.consumed[warp - 1], cons);
-      }
-    }
-  }
-  __syncthreads();
-  if (tid < n) s.u[tid] = rsqrt(fabs(s.d[tid]));
-  __syncthreads();
-  float* out = sv_out + (int64_t)mat * n * n;
-  for (int i = tid; i < n * n; i += kEigThreads) {
-    const int a = i / n, b = i - a * n;
-    out[i] = round16<BF16>((float)(s.a[a][b] * s.u[b]));
-    if (dbg_vec) dbg_vec[(int64_t)mat * n * n + i] = s.a[a][b];
-  }
-  if (dbg_lam && tid < n) dbg_lam[(int64_t)mat * n + tid] = s.d[tid];
-  if (dbg_clk && tid == 0) dbg_clk[mat * 6 + 4] = clock64();
-}
+// ---- kernel 2: symmetric eigendecomposition, leverage_eig.cuh ----
 
 // ---- kernel 3: grid (n_chunks, HKV): score_t = round16(sum_j round16(round16(xc_t . sv_j)^2)) ----
 template <bool BF16>
@@ -735,6 +387,12 @@ __global__ void __launch_bounds__(256) leverage_finalize_kernel(const float* __r
 
 using namespace cvllm;
 
+template <bool BF16>
+static cudaError_t ensure_eig_smem() {
+  static std::atomic<uint64_t> done{0};
+  return ensure_max_dyn_smem((const void*)leverage_eig_kernel<BF16>, (int)sizeof(EigSmem), done);
+}
+
 static size_t lev_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
 extern "C" size_t cvllm_leverage_scores_workspace_bytes(int N, int HKV, int sketch, int n_chunks) {
@@ -778,15 +436,17 @@ static int leverage_launch(const void* k_pre, int64_t k_stride_n, int64_t k_stri
   if (dtype == CVLLM_BF16) {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<true>, (int)smem, attr_g[1]));
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<true>, (int)smem, attr_s[1]));
+    CVLLM_CHECK_CUDA(ensure_eig_smem<true>());
     leverage_gram_kernel<true><<<grid, kLevThreads, smem, st>>>(p);
-    leverage_eig_kernel<true><<<(unsigned)mats, kEigThreads, 0, st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
+    leverage_eig_kernel<true><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
     leverage_score_kernel<true><<<grid, kLevThreads, smem, st>>>(p);
     leverage_finalize_kernel<true><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
   } else {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<false>, (int)smem, attr_g[0]));
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<false>, (int)smem, attr_s[0]));
+    CVLLM_CHECK_CUDA(ensure_eig_smem<false>());
     leverage_gram_kernel<false><<<grid, kLevThreads, smem, st>>>(p);
-    leverage_eig_kernel<false><<<(unsigned)mats, kEigThreads, 0, st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
+    leverage_eig_kernel<false><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
     leverage_score_kernel<false><<<grid, kLevThreads, smem, st>>>(p);
     leverage_finalize_kernel<false><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
   }
@@ -824,10 +484,11 @@ extern "C" int cvllm_selftest_eig(const float* gram, double* lam_out, double* ve
   CVLLM_CHECK_ARG(gram && lam_out && vec_out && sv_out && mats > 0);
   CVLLM_CHECK_ARG(dtype == CVLLM_F16 || dtype == CVLLM_BF16);
   auto st = static_cast<cudaStream_t>(stream);
+  CVLLM_CHECK_CUDA(dtype == CVLLM_BF16 ? ensure_eig_smem<true>() : ensure_eig_smem<false>());
   if (dtype == CVLLM_BF16)
-    leverage_eig_kernel<true><<<mats, kEigThreads, 0, st>>>(gram, sv_out, nullptr, 1, mats, lam_out, vec_out, clk_out);
+    leverage_eig_kernel<true><<<mats, kEigThreads, sizeof(EigSmem), st>>>(gram, sv_out, nullptr, 1, mats, lam_out, vec_out, clk_out);
   else
-    leverage_eig_kernel<false><<<mats, kEigThreads, 0, st>>>(gram, sv_out, nullptr, 1, mats, lam_out, vec_out, clk_out);
+    leverage_eig_kernel<false><<<mats, kEigThreads, sizeof(EigSmem), st>>>(gram, sv_out, nullptr, 1, mats, lam_out, vec_out, clk_out);
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }

@@ -414,12 +414,11 @@ int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_stride_n,
                         int pool_segment, float* out, int dtype, void* workspace,
                         size_t workspace_bytes, cvllm_stream_t stream);
 
-/* Test entry: the fp64 symmetric eigensolver of the leverage chain alone (csrc/score_leverage.cu).
+/* Test entry: the fp64 symmetric eigensolver of the leverage chain alone (csrc/leverage_eig.cuh).
  * gram fp32 [mats,48,48]; lam_out fp64 [mats,48]; vec_out fp64 [mats,48,48] (columns = eigenvectors, any
  * order); sv_out fp32 [mats,48,48] = round16(V |lam|^-1/2), what the score kernel consumes
  * (reference compression/compactor.py:177,197).  clk_out (optional, int64 [mats,6]): SM clock at kernel entry,
- * after the tridiagonal reduction, at the end of the QL producer, at the end of the reflector accumulation, at
- * exit, and the number of ring entries produced (profiling). */
+ * after the tridiagonal reduction, the leaves, the merges to 24, the merge to 48 and at exit (profiling). */
 int cvllm_selftest_eig(const float* gram, double* lam_out, double* vec_out, float* sv_out, int mats,
                        int dtype, long long* clk_out, cvllm_stream_t stream);
 

@@ -129,7 +129,7 @@ def _gram_like(mats, rank, noise, seed, dtype=torch.bfloat16):
 
 
 def test_eigensolver_vs_fp64_eigh():
-    """The fp64 CTA-per-matrix tred2/tql2 (csrc/score_leverage.cu) against torch.linalg.eigh in fp64 on
+    """The fp64 CTA-per-matrix solver (csrc/leverage_eig.cuh) against torch.linalg.eigh in fp64 on
     graded, indefinite Gram matrices plus degenerate cases (reg*I, diagonal, a zero row/column block,
     repeated eigenvalues): eigenvalues to 1e-10 |lam|_max, residual and orthogonality to 1e-9, and the product
     output round16(V |lam|^-1/2) reproduced from the returned (lam, V)."""
@@ -164,6 +164,54 @@ def test_eigensolver_vs_fp64_eigh():
     assert orth.max().item() <= 1e-9, orth.max().item()
     want = (vec * lam.abs().rsqrt().unsqueeze(1)).float().to(torch.bfloat16).float()
     assert torch.equal(sv, want)
+
+
+def test_eigensolver_hard_matrices():
+    """Matrices that the merges of the divide and conquer find hard: equal poles, halves that mirror each other, couplings of
+    all sizes, rank one, tiny and zero norms.  Bounds: a merge moves equal poles 2^-52 of a norm below 8 max |T_ij| apart, 47
+    of them at most, in four rounds: 4 * 47 * 8 * 2^-52 = 3.4e-13."""
+    from compactor_vllm import _native as N
+    n, i = 48, torch.arange(48, dtype=torch.float64)
+    off = lambda v: torch.diag(v, 1) + torch.diag(v, -1)  # noqa: E731
+    one, g = torch.ones(47, dtype=torch.float64), torch.Generator().manual_seed(5)
+    x = torch.randn(n, generator=g, dtype=torch.float64)
+    q = torch.linalg.qr(torch.randn((n, n), generator=g, dtype=torch.float64))[0]
+    mats = torch.stack([torch.ones(n, n, dtype=torch.float64), off(one), torch.diag((i - 24).abs()) + off(one),
+                        torch.diag((i - 23.5).abs()) + off(one), torch.diag(2.0 ** -i) + off(0.3 * 2.0 ** -i[:47]),
+                        torch.outer(x, x) * 1e4 + 5e-3 * torch.eye(n), 1e-25 * torch.diag(i), torch.zeros(n, n),
+                        q @ torch.diag(torch.where(i < 24, 1.0, 1e-6).double()) @ q.T, off(1e-9 * one) + torch.eye(n),
+                        off(torch.where(i[:47] % 3 == 2, 0.0, 1.0).double()), q @ torch.diag((-1.0) ** i) @ q.T]).float()
+    mats = torch.triu(mats) + torch.triu(mats, 1).transpose(1, 2)
+    M, G = mats.shape[0], mats.to(DEV)
+    lam, vec = torch.empty((M, n), dtype=torch.float64, device=DEV), torch.empty((M, n, n), dtype=torch.float64, device=DEV)
+    sv = torch.empty((M, n, n), device=DEV)
+    N.check(N.lib().cvllm_selftest_eig(N.ptr(G), N.ptr(lam), N.ptr(vec), N.ptr(sv), M, N.CVLLM_F16, None, N.stream()), "eig")
+    lam, vec, G64 = lam.cpu(), vec.cpu(), mats.double()
+    ref = torch.linalg.eigvalsh(G64)
+    scale = ref.abs().amax(dim=1).clamp_min(1e-30)
+    assert ((lam.sort(dim=1).values - ref).abs().amax(dim=1) / scale).max().item() <= 3.4e-13
+    resid = (G64 @ vec - vec * lam.unsqueeze(1)).abs().amax(dim=(1, 2)) / scale
+    assert resid.max().item() <= 3.4e-13, resid
+    orth = (vec.transpose(1, 2) @ vec - torch.eye(n, dtype=torch.float64)).abs().max().item()
+    assert orth <= 48 ** 2 * 2.0 ** -53, orth
+
+
+@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
+@pytest.mark.parametrize("at", [(0, 0), (5, 30), (47, 47)])
+def test_eigensolver_not_finite(bad, at):
+    """A matrix with an entry that is not finite gives NaN throughout, its neighbours what they give alone."""
+    from compactor_vllm import _native as N
+    G = _gram_like(3, 12, 0.05, 7)
+    G[1][at] = G[1][at[::-1]] = bad
+    G = G.to(DEV)
+    lam, vec = torch.empty((3, 48), dtype=torch.float64, device=DEV), torch.empty((3, 48, 48), dtype=torch.float64, device=DEV)
+    sv, alone = torch.empty((3, 48, 48), device=DEV), torch.empty((1, 48, 48), device=DEV)
+    call = N.lib().cvllm_selftest_eig
+    N.check(call(N.ptr(G), N.ptr(lam), N.ptr(vec), N.ptr(sv), 3, N.CVLLM_BF16, None, N.stream()), "eig")
+    assert sv[1].isnan().all() and lam[1].isnan().all()
+    last = G[2:].contiguous()
+    N.check(call(N.ptr(last), N.ptr(lam), N.ptr(vec), N.ptr(alone), 1, N.CVLLM_BF16, None, N.stream()), "eig")
+    assert torch.equal(sv[2], alone[0]) and sv[0].isfinite().all()
 
 
 def _structured_keys(N, H, D, dtype, seed):
@@ -317,7 +365,7 @@ def _reference_arithmetic_on_device(keys, lens, phi, chunk, reg=5e-3):
 def test_leverage_matches_reference_arithmetic_on_device(dtype, lens, chunk):
     """Low-rank keys, where one flipped ulp of the 16-bit sketch moves a chunk's scores by O(1): the kernel
     chain has to reproduce the reference's cuBLAS bits through the Gram (natural-k sketch chain, sequential
-    Gram accumulation) and factorise exactly (fp64 tridiagonal QL).  Bar: >= 99.95 % of the scores within
+    Gram accumulation) and factorise exactly (fp64).  Bar: >= 99.95 % of the scores within
     2e-2 * max(1, |s|), none beyond 0.1, top-half overlap >= 99.9 %."""
     N, H, D = sum(lens), 8, 128
     scale = 1.0 if dtype == torch.bfloat16 else 0.1  # fp16: keep the Gram below 65504
