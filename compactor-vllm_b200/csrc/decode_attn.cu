@@ -22,7 +22,8 @@
 //     layout, O^T += V^T.P^T
 //   * partial (m, l, O) of a range that does not cover its whole head goes to
 //     a scratch slot; the CTA that completes a head merges (atomic ticket),
-//     every warp folding a strided subset of the slots with independent loads
+//     every warp folding a strided subset of the slots with independent loads.
+//     Ranges of short heads end at heads' ends (heads_whole), and need none of it
 // HBM-bound: 4*D bytes per cached (token, head).
 //
 // BIAS: the same streaming for the biased attention's decode steps (cvllm_launch_bias_decode, called by
@@ -47,6 +48,17 @@ constexpr int kDecThreads = kDecCons + 32;  // + producer warp
 constexpr int kMaxSlots = 6;      // ring slots (one K unit or one V unit each): 6 when G <= 4, else 5
 constexpr int kSlotBytes = kUnit * 256;     // 32 KB at D = 128, 16-bit (half of it used at D = 64)
 constexpr int kHalfBytes = kUnit * 128;     // one 64-column half of a slot
+
+// Whether the ranges of the C CTAs end at heads' ends (`most` units in the longest head, U in all).  A cut costs some 4.5 us at
+// the end (a partial state through memory, a ticket, the fold); a head left whole costs what its CTA has more than the even
+// share, where a unit takes 0.7 us on a chip that has few and 1.4 on a full one.  Measured in a graph, cut / whole, us, 32 / 8 heads,
+// longest head 1.5 times the mean: 8 x 384 14.8 / 10.5, 8 x 600 15.1 / 13.1, 16 x 600 21.0 / 17.9, 32 x 200 21.2 / 17.2, 64 x 400
+// 34.7 / 31.5, but 24 x 650 26.4 / 27.9, 48 x 600 35.6 / 37.4, 32 x 800 32.5 / 34.8 (shares above 6 units), 1 x 500 10.2 / 10.8,
+// 4 x 1000 13.8 / 18.4 (long beside the share).
+__device__ __forceinline__ bool heads_whole(int most, int64_t U, int C) {
+  if (U > 6 * (int64_t)C) return most <= 5;
+  return most <= 8 && (int64_t)C * (most - (U >= C ? 6 : 4)) <= U;
+}
 
 struct DecodeParams {
   const void* q;
@@ -145,6 +157,64 @@ __device__ __forceinline__ float bias_inv(const BiasDecodeParams& p, int hq, flo
 
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kDecCons) : "memory"); }
 
+// The partial states of a cut head, slots c_first .. c_last, into s_merge's rows: each consumer warp folds the slots c_first + warp,
+// + 8, ... into a running (m, l, O), the loads of AHEAD slots in flight together; lane owns d = 2*lane, 2*lane+1, 64 + 2*lane,
+// 65 + 2*lane.  A function of its own: its registers beside the streaming loop's would make that loop spill.
+template <int NQ, int AHEAD>
+__device__ __noinline__ void fold_slots(const float* scratch, float* s_merge, int head, int G, int c_first, int c_last, int U, int C) {
+  constexpr int ROW = 128 + 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* mw = s_merge + warp * G * ROW;
+  float M[NQ], ls[NQ];
+  float2 oa[NQ], ob[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    M[q] = -INFINITY; ls[q] = 0.f;
+    oa[q] = make_float2(0.f, 0.f); ob[q] = make_float2(0.f, 0.f);
+  }
+  for (int cc = c_first + warp; cc <= c_last; cc += AHEAD * kDecWarps) {
+    float2 va[AHEAD][NQ], vb[AHEAD][NQ], ml[AHEAD][NQ];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int ci = cc + i * kDecWarps;
+      // CTAs with an empty unit range (U < C) never wrote their slot
+      const bool used = ci <= c_last && (int)((int64_t)U * ci / C) < (int)((int64_t)U * (ci + 1) / C);
+      const float* sl = scratch + (int64_t)(head + ci) * G * ROW;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        ml[i][q] = make_float2(-INFINITY, 0.f);
+        va[i][q] = vb[i][q] = make_float2(0.f, 0.f);
+        if (used && q < G) {
+          va[i][q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + 2 * lane));
+          vb[i][q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + 64 + 2 * lane));
+          ml[i][q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + 128));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const float Mn = fmaxf(M[q], ml[i][q].x);
+        const float so = (M[q] > -INFINITY) ? ex2(M[q] - Mn) : 0.f;
+        const float sn = (ml[i][q].x > -INFINITY) ? ex2(ml[i][q].x - Mn) : 0.f;
+        oa[q].x = oa[q].x * so + va[i][q].x * sn; oa[q].y = oa[q].y * so + va[i][q].y * sn;
+        ob[q].x = ob[q].x * so + vb[i][q].x * sn; ob[q].y = ob[q].y * so + vb[i][q].y * sn;
+        ls[q] = ls[q] * so + ml[i][q].y * sn;
+        M[q] = Mn;
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    if (q < G) {
+      *reinterpret_cast<float2*>(mw + q * ROW + 2 * lane) = oa[q];
+      *reinterpret_cast<float2*>(mw + q * ROW + 64 + 2 * lane) = ob[q];
+      if (lane == 0) *reinterpret_cast<float2*>(mw + q * ROW + 128) = make_float2(M[q], ls[q]);
+    }
+  }
+}
+
 template <bool BF16, int D, bool BIAS = false>
 __global__ void __launch_bounds__(kDecThreads, 1)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -165,9 +235,9 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   uint64_t* bar_full = reinterpret_cast<uint64_t*>(smem_raw + kSlots * kSlotBytes);
   uint64_t* bar_empty = bar_full + kMaxSlots;
   float* s_merge = reinterpret_cast<float*>(bar_empty + kMaxSlots);   // [kDecWarps][G][ROW]
-  float* s_final = s_merge + kDecWarps * p.G * ROW;                   // [G][ROW]
-  int32_t* s_prefix = reinterpret_cast<int32_t*>(s_final + p.G * ROW);  // [BH + 1]
-  __shared__ int32_t s_warp_tot[NW];
+  int32_t* s_prefix = reinterpret_cast<int32_t*>(s_merge + kDecWarps * p.G * ROW);  // [BH + 1]
+  int32_t* s_map = s_prefix + BH + 1;                                 // [B] batch_mapping
+  __shared__ int32_t s_warp_tot[NW], s_warp_max[NW];
   __shared__ int s_last;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -206,15 +276,24 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   {
     const int per = cdiv(BH, kDecThreads);
     const int beg = min(BH, tid * per), end = min(BH, beg + per);
-    int local = 0;
-    for (int i = beg; i < end; ++i) local += units_of(i);
+    int local = 0, most = 0;
+    for (int i = tid; i < p.B; i += kDecThreads) s_map[i] = p.batch_mapping[i];   // in flight with the lengths
+    for (int i = beg; i < end; ++i) {
+      const int n = units_of(i);
+      local += n;
+      most = max(most, n);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
     int incl = local;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
-    if (lane == 31) s_warp_tot[warp] = incl;
+    if (lane == 31) {
+      s_warp_tot[warp] = incl;
+      s_warp_max[warp] = most;
+    }
     __syncthreads();
     int base = 0;
     for (int w = 0; w < warp; ++w) base += s_warp_tot[w];
@@ -239,10 +318,6 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   }
   if (U == 0) return;
 
-  const int u_begin = (int)((int64_t)U * c / C);
-  const int u_end = (int)((int64_t)U * (c + 1) / C);
-  if (u_begin >= u_end) return;
-
   // largest i with s_prefix[i] <= u
   auto find_head = [&](int u) {
     int lo = 0, hi = BH;
@@ -252,6 +327,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     return lo;
   };
+  int most = 0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) most = max(most, s_warp_max[w]);
+  const bool uncut = (BIAS || G <= 4) && heads_whole(most, U, C);
+  auto range_at = [&](int t) {   // first unit of CTA t
+    const int x = (int)((int64_t)U * t / C);
+    if (!uncut || t == C) return x;
+    const int i = find_head(x);
+    return x - s_prefix[i] < s_prefix[i + 1] - x ? s_prefix[i] : s_prefix[i + 1];
+  };
+  const int u_begin = range_at(c), u_end = range_at(c + 1);
+  if (u_begin >= u_end) return;
 
   // =========================== producer warp ================================
   if (warp == kDecWarps) {
@@ -277,7 +364,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           const int pg = tok / p.PS;
           const int32_t* pt;
           if constexpr (BIAS) pt = p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head;
-          else pt = p.page_table + ((int64_t)p.batch_mapping[b] * p.HKV + h) * p.NLP;
+          else pt = p.page_table + ((int64_t)s_map[b] * p.HKV + h) * p.NLP;
           row = pt[pg] * p.PS + (tok - pg * p.PS);
         }
       }
@@ -319,6 +406,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
   // =========================== consumer warps ===============================
   const int r = lane >> 2, j = lane & 3;
+  // P as the sum of two 16-bit numbers (see the top): biased attention, and heads left whole.  Their one running maximum
+  // leaves fewer keys with the exact probability 1 than the cut ones' many, 2 % more error at 400 keys a head; so, it is
+  // a third less.
+  const bool low_parts = G <= 4 && (BIAS || uncut);
   const uint32_t ring_u32 = smem_u32(ring);
   int c_slot = 0;        // ring position of the next item to consume
   uint32_t c_par = 0;    // and its mbarrier phase parity
@@ -335,8 +426,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if constexpr (BIAS) return UnitList(p, b);
       else return UnitList{};
     }();
-    // biased attention: this lane's query columns 2j, 2j + 1 (columns 4 .. 7 of a small group carry the low parts of P)
-    const bool low_cols = BIAS && G <= 4 && j >= 2;
+    // this lane's query columns 2j, 2j + 1 (columns 4 .. 7 of a small group carry the low parts of P)
+    const bool low_cols = low_parts && j >= 2;
     const int qc = low_cols ? 2 * j - 4 : 2 * j;
     float slope0 = 0.f, slope1 = 0.f;
     if constexpr (BIAS) {
@@ -364,153 +455,161 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     for (int t = 0; t < MT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
-    for (int uu = ua; uu < ub; ++uu) {
-      // ring positions of this unit's K and V items (advanced without divisions)
-      const int ks_slot = c_slot;
-      const uint32_t k_par = c_par;
-      if (++c_slot == kSlots) { c_slot = 0; c_par ^= 1u; }
-      const int vs_slot = c_slot;
-      const uint32_t v_par = c_par;
-      if (++c_slot == kSlots) { c_slot = 0; c_par ^= 1u; }
-      const uint32_t k_base = ring_u32 + ks_slot * kSlotBytes, v_base = ring_u32 + vs_slot * kSlotBytes;
-      const int t0 = warp * 16;                               // this warp's rows inside the unit
-      const int unit0 = BIAS ? list.base(uu) : uu * kUnit;    // position of the unit's first key
-      const int n_valid = min(16, L - (unit0 + t0));          // <= 0: nothing for this warp
-      // what distance and head add to this lane's four logits, requested before the unit's data is waited for
-      float bias0 = 0.f, bias1 = 0.f, bias2 = 0.f, bias3 = 0.f;
-      if constexpr (BIAS) {
-        const int n_lo = list.pi - (unit0 + t0 + r), n_hi = n_lo - 8;
-        bias0 = -slope0 * (float)n_lo; bias1 = -slope1 * (float)n_lo;
-        bias2 = -slope0 * (float)n_hi; bias3 = -slope1 * (float)n_hi;
-        if (p.dist_bias && qc < G) {
-          const float* t_lo = p.dist_bias + (int64_t)min(max(n_lo, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
-          const float* t_hi = p.dist_bias + (int64_t)min(max(n_hi, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
-          bias0 = fmaf(t_lo[0], 1.4426950408889634f, bias0);
-          bias2 = fmaf(t_hi[0], 1.4426950408889634f, bias2);
-          if (qc + 1 < G) {
-            bias1 = fmaf(t_lo[1], 1.4426950408889634f, bias1);
-            bias3 = fmaf(t_hi[1], 1.4426950408889634f, bias3);
-          }
-        }
-      }
-
-      // every warp waits (so nobody can run a full ring ahead) and releases the slots
-      mbar_wait(&bar_full[ks_slot], k_par);
-      if (tid == 0 && u == u_begin && uu == ua) DEC_TRACE(2);
-      if (n_valid > 0 && p.mode == 0) {
-        Slice<D> cur;
-#pragma unroll
-        for (int cc = 0; cc < KC; ++cc) {
-          cur.k_lo[cc] = lds_v4(slot_addr(k_base, t0 + r, kchunk(j, cc)));
-          cur.k_hi[cc] = lds_v4(slot_addr(k_base, t0 + r + 8, kchunk(j, cc)));
-        }
-        // V rows of keys past the head's length are uninitialised memory: P is 0 there but
-        // 0 * NaN would poison O, so those rows are read as zeros.  V is fetched before the
-        // S chain so its shared-memory latency hides behind the mma / softmax dependency chain.
-        mbar_wait(&bar_full[vs_slot], v_par);
-        {
-          const uint4 z = make_uint4(0, 0, 0, 0);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int key = 2 * j + (i & 1) + ((i >> 1) << 3);
-            bool ok = key < n_valid;
-            if constexpr (BIAS) ok = ok && (unit0 + t0 + key >= list.lo || unit0 + t0 + key < p.keep);
-            cur.v[i][0] = ok ? lds_v4(slot_addr(v_base, t0 + key, r)) : z;
-            if constexpr (D == 128) cur.v[i][D / 64 - 1] = ok ? lds_v4(slot_addr(v_base, t0 + key, 8 + r)) : z;
-          }
-        }
-        // ---- S^T[16 keys x 8 queries]: two accumulators halve the dependent mma chain ----
-        float s[4] = {0.f, 0.f, 0.f, 0.f}, s_b[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int ks = 0; ks < KSTEPS; ++ks) {
-          const int cc = ks >> 1;
-          const uint32_t a0 = (ks & 1) ? cur.k_lo[cc].z : cur.k_lo[cc].x;
-          const uint32_t a1 = (ks & 1) ? cur.k_hi[cc].z : cur.k_hi[cc].x;
-          const uint32_t a2 = (ks & 1) ? cur.k_lo[cc].w : cur.k_lo[cc].y;
-          const uint32_t a3 = (ks & 1) ? cur.k_hi[cc].w : cur.k_hi[cc].y;
-          if (ks & 1) mma16816<BF16>(s_b, a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
-          else mma16816<BF16>(s, a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[e] += s_b[e];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);  // K rows are in registers: free the slot now
-        bool ok_lo = r < n_valid, ok_hi = r + 8 < n_valid;
+    auto stream_units = [&](auto parts) {
+      constexpr bool LOW = decltype(parts)::value;
+      for (int uu = ua; uu < ub; ++uu) {
+        // ring positions of this unit's K and V items (advanced without divisions)
+        const int ks_slot = c_slot;
+        const uint32_t k_par = c_par;
+        if (++c_slot == kSlots) { c_slot = 0; c_par ^= 1u; }
+        const int vs_slot = c_slot;
+        const uint32_t v_par = c_par;
+        if (++c_slot == kSlots) { c_slot = 0; c_par ^= 1u; }
+        const uint32_t k_base = ring_u32 + ks_slot * kSlotBytes, v_base = ring_u32 + vs_slot * kSlotBytes;
+        const int t0 = warp * 16;                               // this warp's rows inside the unit
+        const int unit0 = BIAS ? list.base(uu) : uu * kUnit;    // position of the unit's first key
+        const int n_valid = min(16, L - (unit0 + t0));          // <= 0: nothing for this warp
+        // what distance and head add to this lane's four logits, requested before the unit's data is waited for
+        float bias0 = 0.f, bias1 = 0.f, bias2 = 0.f, bias3 = 0.f;
         if constexpr (BIAS) {
-          const int kp = unit0 + t0 + r;
-          ok_lo = ok_lo && (kp >= list.lo || kp < p.keep);
-          ok_hi = ok_hi && (kp + 8 >= list.lo || kp + 8 < p.keep);
-          if (G <= 4) {   // columns 4 .. 7 repeat the scores of columns 0 .. 3: same maximum, same probabilities
+          const int n_lo = list.pi - (unit0 + t0 + r), n_hi = n_lo - 8;
+          bias0 = -slope0 * (float)n_lo; bias1 = -slope1 * (float)n_lo;
+          bias2 = -slope0 * (float)n_hi; bias3 = -slope1 * (float)n_hi;
+          if (p.dist_bias && qc < G) {
+            const float* t_lo = p.dist_bias + (int64_t)min(max(n_lo, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
+            const float* t_hi = p.dist_bias + (int64_t)min(max(n_hi, 0), p.dist_rows - 1) * p.HQ + h * G + qc;
+            bias0 = fmaf(t_lo[0], 1.4426950408889634f, bias0);
+            bias2 = fmaf(t_hi[0], 1.4426950408889634f, bias2);
+            if (qc + 1 < G) {
+              bias1 = fmaf(t_lo[1], 1.4426950408889634f, bias1);
+              bias3 = fmaf(t_hi[1], 1.4426950408889634f, bias3);
+            }
+          }
+        }
+
+        // every warp waits (so nobody can run a full ring ahead) and releases the slots
+        mbar_wait(&bar_full[ks_slot], k_par);
+        if (tid == 0 && u == u_begin && uu == ua) DEC_TRACE(2);
+        if (n_valid > 0 && p.mode == 0) {
+          Slice<D> cur;
+#pragma unroll
+          for (int cc = 0; cc < KC; ++cc) {
+            cur.k_lo[cc] = lds_v4(slot_addr(k_base, t0 + r, kchunk(j, cc)));
+            cur.k_hi[cc] = lds_v4(slot_addr(k_base, t0 + r + 8, kchunk(j, cc)));
+          }
+          // V rows of keys past the head's length are uninitialised memory: P is 0 there but
+          // 0 * NaN would poison O, so those rows are read as zeros.  V is fetched before the
+          // S chain so its shared-memory latency hides behind the mma / softmax dependency chain.
+          mbar_wait(&bar_full[vs_slot], v_par);
+          {
+            const uint4 z = make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int key = 2 * j + (i & 1) + ((i >> 1) << 3);
+              bool ok = key < n_valid;
+              if constexpr (BIAS) ok = ok && (unit0 + t0 + key >= list.lo || unit0 + t0 + key < p.keep);
+              cur.v[i][0] = ok ? lds_v4(slot_addr(v_base, t0 + key, r)) : z;
+              if constexpr (D == 128) cur.v[i][D / 64 - 1] = ok ? lds_v4(slot_addr(v_base, t0 + key, 8 + r)) : z;
+            }
+          }
+          // ---- S^T[16 keys x 8 queries]: two accumulators halve the dependent mma chain ----
+          float s[4] = {0.f, 0.f, 0.f, 0.f}, s_b[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int ks = 0; ks < KSTEPS; ++ks) {
+            const int cc = ks >> 1;
+            const uint32_t a0 = (ks & 1) ? cur.k_lo[cc].z : cur.k_lo[cc].x;
+            const uint32_t a1 = (ks & 1) ? cur.k_hi[cc].z : cur.k_hi[cc].x;
+            const uint32_t a2 = (ks & 1) ? cur.k_lo[cc].w : cur.k_lo[cc].y;
+            const uint32_t a3 = (ks & 1) ? cur.k_hi[cc].w : cur.k_hi[cc].y;
+            if (ks & 1) mma16816<BF16>(s_b, a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
+            else mma16816<BF16>(s, a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[e] += s_b[e];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);  // K rows are in registers: free the slot now
+          bool ok_lo = r < n_valid, ok_hi = r + 8 < n_valid;
+          if constexpr (BIAS) {
+            const int kp = unit0 + t0 + r;
+            ok_lo = ok_lo && (kp >= list.lo || kp < p.keep);
+            ok_hi = ok_hi && (kp + 8 >= list.lo || kp + 8 < p.keep);
+          }
+          if constexpr (LOW) {   // columns 4 .. 7 repeat the scores of columns 0 .. 3: same maximum, same probabilities
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float other = __shfl_xor_sync(0xffffffffu, s[e], 2);
               if (low_cols) s[e] = other;
             }
           }
-        }
-        const float x0 = ok_lo ? (BIAS ? fmaf(s[0], p.scale_log2, bias0) : s[0] * p.scale_log2) : -INFINITY;
-        const float x1 = ok_lo ? (BIAS ? fmaf(s[1], p.scale_log2, bias1) : s[1] * p.scale_log2) : -INFINITY;
-        const float x2 = ok_hi ? (BIAS ? fmaf(s[2], p.scale_log2, bias2) : s[2] * p.scale_log2) : -INFINITY;
-        const float x3 = ok_hi ? (BIAS ? fmaf(s[3], p.scale_log2, bias3) : s[3] * p.scale_log2) : -INFINITY;
-        float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
+          const float x0 = ok_lo ? (BIAS ? fmaf(s[0], p.scale_log2, bias0) : s[0] * p.scale_log2) : -INFINITY;
+          const float x1 = ok_lo ? (BIAS ? fmaf(s[1], p.scale_log2, bias1) : s[1] * p.scale_log2) : -INFINITY;
+          const float x2 = ok_hi ? (BIAS ? fmaf(s[2], p.scale_log2, bias2) : s[2] * p.scale_log2) : -INFINITY;
+          const float x3 = ok_hi ? (BIAS ? fmaf(s[3], p.scale_log2, bias3) : s[3] * p.scale_log2) : -INFINITY;
+          float mx0 = fmaxf(x0, x2), mx1 = fmaxf(x1, x3);
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-          mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-          mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-        }
-        if constexpr (BIAS) {   // a first unit may be all masked: the lowest finite reference, so that every score can pass it
-          m0 = fmaxf(m0, -3.402823466e38f);
-          m1 = fmaxf(m1, -3.402823466e38f);
-        }
-        float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-        // a NaN/-inf column max (garbage q) must not poison the rest
-        if (!(mn0 > -INFINITY)) mn0 = 0.f;
-        if (!(mn1 > -INFINITY)) mn1 = 0.f;
-        const float al0 = ex2(m0 - mn0), al1 = ex2(m1 - mn1);
-        m0 = mn0; m1 = mn1;
-        const float p0 = ex2(x0 - mn0), p1 = ex2(x1 - mn1), p2 = ex2(x2 - mn0), p3 = ex2(x3 - mn1);
-        l0 = l0 * al0 + p0 + p2;
-        l1 = l1 * al1 + p1 + p3;
-        if (__any_sync(0xffffffffu, (al0 != 1.f) | (al1 != 1.f))) {
-#pragma unroll
-          for (int t = 0; t < MT; ++t) {
-            acc[t][0] *= al0; acc[t][1] *= al1; acc[t][2] *= al0; acc[t][3] *= al1;
+          for (int o = 4; o < 32; o <<= 1) {
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
           }
-        }
-        uint32_t hi01 = pack2<BF16>(p0, p1), hi23 = pack2<BF16>(p2, p3), lo01 = 0u, lo23 = 0u;
-        if constexpr (BIAS) {
-          lo01 = pack2<true>(p0 - __uint_as_float(hi01 << 16), p1 - __uint_as_float(hi01 & 0xffff0000u));
-          lo23 = pack2<true>(p2 - __uint_as_float(hi23 << 16), p3 - __uint_as_float(hi23 & 0xffff0000u));
-          if (low_cols) { hi01 = lo01; hi23 = lo23; }
-        }
-        const uint32_t pb0 = movmatrix_trans(hi01);
-        const uint32_t pb1 = movmatrix_trans(hi23);
+          if constexpr (BIAS) {   // a first unit may be all masked: the lowest finite reference, so that every score can pass it
+            m0 = fmaxf(m0, -3.402823466e38f);
+            m1 = fmaxf(m1, -3.402823466e38f);
+          }
+          float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
+          // a NaN/-inf column max (garbage q) must not poison the rest
+          if (!(mn0 > -INFINITY)) mn0 = 0.f;
+          if (!(mn1 > -INFINITY)) mn1 = 0.f;
+          const float al0 = ex2(m0 - mn0), al1 = ex2(m1 - mn1);
+          m0 = mn0; m1 = mn1;
+          const float p0 = ex2(x0 - mn0), p1 = ex2(x1 - mn1), p2 = ex2(x2 - mn0), p3 = ex2(x3 - mn1);
+          l0 = l0 * al0 + p0 + p2;
+          l1 = l1 * al1 + p1 + p3;
+          if (__any_sync(0xffffffffu, (al0 != 1.f) | (al1 != 1.f))) {
+#pragma unroll
+            for (int t = 0; t < MT; ++t) {
+              acc[t][0] *= al0; acc[t][1] *= al1; acc[t][2] *= al0; acc[t][3] *= al1;
+            }
+          }
+          uint32_t hi01 = pack2<BF16>(p0, p1), hi23 = pack2<BF16>(p2, p3), lo01 = 0u, lo23 = 0u;
+          if constexpr (BIAS || LOW) {
+            const float2 h01 = unpack2<BF16>(hi01), h23 = unpack2<BF16>(hi23);
+            lo01 = pack2<BF16>(p0 - h01.x, p1 - h01.y);
+            lo23 = pack2<BF16>(p2 - h23.x, p3 - h23.y);
+            if (low_cols) { hi01 = lo01; hi23 = lo23; }
+          }
+          const uint32_t pb0 = movmatrix_trans(hi01);
+          const uint32_t pb1 = movmatrix_trans(hi23);
 
-        // ---- O^T[D x 8] += V^T[D x 16] . P^T[16 x 8] ----
-        // tile t: rows r and r + 8 are numbers 8 r + t and 64 + 8 r + t (D = 64: 8 r + t and 8 r + 4 + t) of the value rows
-        auto add_pv = [&](uint32_t b0, uint32_t b1) {
+          // ---- O^T[D x 8] += V^T[D x 16] . P^T[16 x 8] ----
+          // tile t: rows r and r + 8 are numbers 8 r + t and 64 + 8 r + t (D = 64: 8 r + t and 8 r + 4 + t) of the value rows
+          auto add_pv = [&](uint32_t b0, uint32_t b1) {
 #pragma unroll
-          for (int t = 0; t < MT; ++t) {
-            const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
-            const int w = t >> 1, c2 = D / 64 - 1, w2 = D == 128 ? w : w + 2;
-            const uint32_t a0 = __byte_perm(u4_get(cur.v[0][0], w), u4_get(cur.v[1][0], w), sel);
-            const uint32_t a1 = __byte_perm(u4_get(cur.v[0][c2], w2), u4_get(cur.v[1][c2], w2), sel);
-            const uint32_t a2 = __byte_perm(u4_get(cur.v[2][0], w), u4_get(cur.v[3][0], w), sel);
-            const uint32_t a3 = __byte_perm(u4_get(cur.v[2][c2], w2), u4_get(cur.v[3][c2], w2), sel);
-            mma16816<BF16>(acc[t], a0, a1, a2, a3, b0, b1);
+            for (int t = 0; t < MT; ++t) {
+              const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
+              const int w = t >> 1, c2 = D / 64 - 1, w2 = D == 128 ? w : w + 2;
+              const uint32_t a0 = __byte_perm(u4_get(cur.v[0][0], w), u4_get(cur.v[1][0], w), sel);
+              const uint32_t a1 = __byte_perm(u4_get(cur.v[0][c2], w2), u4_get(cur.v[1][c2], w2), sel);
+              const uint32_t a2 = __byte_perm(u4_get(cur.v[2][0], w), u4_get(cur.v[3][0], w), sel);
+              const uint32_t a3 = __byte_perm(u4_get(cur.v[2][c2], w2), u4_get(cur.v[3][c2], w2), sel);
+              mma16816<BF16>(acc[t], a0, a1, a2, a3, b0, b1);
+            }
+          };
+          add_pv(pb0, pb1);
+          if constexpr (BIAS) {
+            if (G > 4) add_pv(movmatrix_trans(lo01), movmatrix_trans(lo23));   // no free columns: a second product
           }
-        };
-        add_pv(pb0, pb1);
-        if constexpr (BIAS) {
-          if (G > 4) add_pv(movmatrix_trans(lo01), movmatrix_trans(lo23));   // no free columns: a second product
+        } else {
+          if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);
+          mbar_wait(&bar_full[vs_slot], v_par);
         }
-      } else {
-        if (lane == 0) mbar_arrive(&bar_empty[ks_slot]);
-        mbar_wait(&bar_full[vs_slot], v_par);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_empty[vs_slot]);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_empty[vs_slot]);
-    }
+    };
+    // two loops, the long heads' first: 16 x 10240 rows take 114.1 us so, 115.3 with the other one first, 115.7 with one loop and
+    // branches in it
+    if (__builtin_expect(!low_parts, 1)) stream_units(std::false_type{});
+    else stream_units(std::true_type{});
 
     if (tid == 0) DEC_TRACE(3);
     // ---- per-warp state -> smem ----
@@ -519,13 +618,11 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       l0 += __shfl_xor_sync(0xffffffffu, l0, o);
       l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     }
-    if constexpr (BIAS) {
-      if (G <= 4) {   // the low parts' products join their columns
+    if (low_parts) {   // the low parts' products join their columns
 #pragma unroll
-        for (int t = 0; t < MT; ++t)
+      for (int t = 0; t < MT; ++t)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[t][e] += __shfl_xor_sync(0xffffffffu, acc[t][e], 2);
-      }
+        for (int e = 0; e < 4; ++e) acc[t][e] += __shfl_xor_sync(0xffffffffu, acc[t][e], 2);
     }
     {
       float* mw = s_merge + warp * G * ROW;
@@ -533,135 +630,86 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       constexpr int kRow2 = D == 128 ? 64 : 4;   // where a tile's second eight rows lie (see add_pv)
       if (q0 < G) {
 #pragma unroll
-        for (int t = 0; t < MT; ++t) {
-          mw[q0 * ROW + 8 * r + t] = acc[t][0];
-          mw[q0 * ROW + kRow2 + 8 * r + t] = acc[t][2];
+        for (int t = 0; t < MT; t += 2) {
+          *reinterpret_cast<float2*>(mw + q0 * ROW + 8 * r + t) = make_float2(acc[t][0], acc[t + 1][0]);
+          *reinterpret_cast<float2*>(mw + q0 * ROW + kRow2 + 8 * r + t) = make_float2(acc[t][2], acc[t + 1][2]);
         }
         if (r == 0) { mw[q0 * ROW + D] = m0; mw[q0 * ROW + D + 1] = l0; }
       }
       if (q1 < G) {
 #pragma unroll
-        for (int t = 0; t < MT; ++t) {
-          mw[q1 * ROW + 8 * r + t] = acc[t][1];
-          mw[q1 * ROW + kRow2 + 8 * r + t] = acc[t][3];
+        for (int t = 0; t < MT; t += 2) {
+          *reinterpret_cast<float2*>(mw + q1 * ROW + 8 * r + t) = make_float2(acc[t][1], acc[t + 1][1]);
+          *reinterpret_cast<float2*>(mw + q1 * ROW + kRow2 + 8 * r + t) = make_float2(acc[t][3], acc[t + 1][3]);
         }
         if (r == 0) { mw[q1 * ROW + D] = m1; mw[q1 * ROW + D + 1] = l1; }
       }
     }
     cons_bar();
 
-    // ---- merge the 8 warps' rows -> s_final[q][ROW] (unnormalised O, m, l) ----
-    auto fold_warps = [&]() {
-      for (int e = tid; e < G * ROW; e += kDecCons) {
-        const int q = e / ROW, d = e - q * ROW;
-        float M = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, s_merge[(w * G + q) * ROW + D]);
-        float val = 0.f;
-        if (d == D) {
-          val = M;
-        } else {
-          const int src = d < D ? d : D + 1;
-#pragma unroll
-          for (int w = 0; w < kDecWarps; ++w) {
-            const float mw = s_merge[(w * G + q) * ROW + D];
-            const float sc = (mw > -INFINITY) ? ex2(mw - M) : 0.f;
-            val += s_merge[(w * G + q) * ROW + src] * sc;
-          }
-        }
-        s_final[e] = val;
-      }
-    };
-    auto write_out = [&]() {
-      uint32_t* orow = out_row(b, h);
-      for (int e = tid; e < G * D / 2; e += kDecCons) {
+    // ---- merge the 8 warps' rows: put(q, pair, O (unnormalised), m, l) ----
+    auto fold_warps = [&](auto put) {
+      for (int e = tid; e < G * (D / 2); e += kDecCons) {
         const int q = e / (D / 2), d2 = e - q * (D / 2);
-        const float lq = s_final[q * ROW + D + 1];
-        float inv = lq > 0.f ? 1.f / lq : 0.f;
-        if constexpr (BIAS) inv = bias_inv(p, h * G + q, s_final[q * ROW + D], lq);
-        orow[e] = pack2<BF16>(s_final[q * ROW + 2 * d2] * inv, s_final[q * ROW + 2 * d2 + 1] * inv);
+        float2 ml[kDecWarps], o = make_float2(0.f, 0.f);
+        float M = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+          ml[w] = *reinterpret_cast<const float2*>(s_merge + (w * G + q) * ROW + D);
+          M = fmaxf(M, ml[w].x);
+        }
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+          const float2 v = *reinterpret_cast<const float2*>(s_merge + (w * G + q) * ROW + 2 * d2);
+          const float sc = (ml[w].x > -INFINITY) ? ex2(ml[w].x - M) : 0.f;
+          l += ml[w].y * sc;
+          o.x += v.x * sc;
+          o.y += v.y * sc;
+        }
+        put(q, d2, o, M, l);
       }
     };
-    fold_warps();
-    cons_bar();
+    auto write_out = [&](int q, int d2, float2 o, float M, float l) {
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if constexpr (BIAS) inv = bias_inv(p, h * G + q, M, l);
+      out_row(b, h)[q * (D / 2) + d2] = pack2<BF16>(o.x * inv, o.y * inv);
+    };
 
     const bool whole = (ua == 0) && (ub == h_end - h_beg);
     if (whole) {
-      write_out();
+      fold_warps(write_out);
     } else {
       // publish the partial, then take a ticket; the CTA completing the head merges
       float* slot = p.scratch + (int64_t)(head + c) * G * ROW;
-      for (int e = tid; e < G * ROW; e += kDecCons) __stcg(slot + e, s_final[e]);
-      if constexpr (BIAS) {
-        cons_bar();   // s_merge / s_final reused by the next segment; bias_decode_fold_kernel merges
+      fold_warps([&](int q, int d2, float2 o, float M, float l) {
+        __stcg(reinterpret_cast<float2*>(slot + q * ROW + 2 * d2), o);
+        if (d2 == 0) __stcg(reinterpret_cast<float2*>(slot + q * ROW + D), make_float2(M, l));
+      });
+      cons_bar();
+      if constexpr (BIAS) {   // s_merge reused by the next segment; bias_decode_fold_kernel merges
         u = seg_end;
         continue;
       }
-      __threadfence();
-      cons_bar();
       if (tid == 0) {
+        __threadfence();      // the CTA's partial (behind the barrier) before its ticket
         const int done = atomicAdd(p.counters + head, ub - ua) + (ub - ua);
+        __threadfence();
         s_last = (done == h_end - h_beg);
       }
       cons_bar();
       if (tid == 0) DEC_TRACE(6);
       if (s_last) {
-        __threadfence();
         const int c_first = (int)((((int64_t)h_beg + 1) * C - 1) / U);
         const int c_last = (int)(((int64_t)h_end * C - 1) / U);
-        // Each warp folds the slots c_first + warp, + 8, ... into a running (m, l, O) with all
-        // loads of a slot independent; lane owns d = 2*lane, 2*lane+1, 64 + 2*lane, 65 + 2*lane.
-        float* mw = s_merge + warp * G * ROW;
-        float M[8], ls[8];
-        float2 oa[8], ob[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          M[q] = -INFINITY; ls[q] = 0.f;
-          oa[q] = make_float2(0.f, 0.f); ob[q] = make_float2(0.f, 0.f);
-        }
-        for (int cc = c_first + warp; cc <= c_last; cc += kDecWarps) {
-          // CTAs with an empty unit range (U < C) never wrote their slot
-          if ((int)((int64_t)U * cc / C) >= (int)((int64_t)U * (cc + 1) / C)) continue;
-          const float* sl = p.scratch + (int64_t)(head + cc) * G * ROW;
-          float2 va[8], vb[8], ml[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            if (q < G) {
-              va[q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + 2 * lane));
-              vb[q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + 64 + 2 * lane));
-              ml[q] = __ldcg(reinterpret_cast<const float2*>(sl + q * ROW + D));
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            if (q < G) {
-              const float Mn = fmaxf(M[q], ml[q].x);
-              const float so = (M[q] > -INFINITY) ? ex2(M[q] - Mn) : 0.f;
-              const float sn = (ml[q].x > -INFINITY) ? ex2(ml[q].x - Mn) : 0.f;
-              oa[q].x = oa[q].x * so + va[q].x * sn; oa[q].y = oa[q].y * so + va[q].y * sn;
-              ob[q].x = ob[q].x * so + vb[q].x * sn; ob[q].y = ob[q].y * so + vb[q].y * sn;
-              ls[q] = ls[q] * so + ml[q].y * sn;
-              M[q] = Mn;
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          if (q < G) {
-            *reinterpret_cast<float2*>(mw + q * ROW + 2 * lane) = oa[q];
-            *reinterpret_cast<float2*>(mw + q * ROW + 64 + 2 * lane) = ob[q];
-            if (lane == 0) { mw[q * ROW + D] = M[q]; mw[q * ROW + D + 1] = ls[q]; }
-          }
-        }
+        if (G <= 4) fold_slots<4, 3>(p.scratch, s_merge, head, G, c_first, c_last, U, C);
+        else fold_slots<8, 1>(p.scratch, s_merge, head, G, c_first, c_last, U, C);
         cons_bar();
         if (tid == 0) DEC_TRACE(7);
-        fold_warps();
-        cons_bar();
-        write_out();
+        fold_warps(write_out);
         if (tid == 0) p.counters[head] = 0;
       }
     }
-    cons_bar();  // s_merge / s_final reused by the next segment
+    cons_bar();  // s_merge reused by the next segment
 #ifdef CVLLM_DECODE_TRACE
     if (tid == 0 && p.trace) {
       DEC_TRACE(4);
@@ -683,9 +731,10 @@ __global__ void __launch_bounds__(256) bias_decode_fold_kernel(const BiasDecodeP
   __shared__ float s_o[8][D];
   __shared__ float s_l[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int before = 0, all = 0;   // units of the sequences before, and of all
+  int before = 0, all = 0, most = 0;   // units of the sequences before, of all, of the longest
   for (int i = lane; i < p.B; i += 32) {
     const int n = UnitList(p, i).count;
+    most = max(most, n);
     all += n;
     if (i < b) before += n;
   }
@@ -696,7 +745,9 @@ __global__ void __launch_bounds__(256) bias_decode_fold_kernel(const BiasDecodeP
   }
   const int n = UnitList(p, b).count;
   if (n == 0) return;
-  const int64_t U = (int64_t)all * p.HKV, h_beg = (int64_t)before * p.HKV + (int64_t)h * n, h_end = h_beg + n;
+  const int64_t U = (int64_t)all * p.HKV;
+  if (heads_whole(__reduce_max_sync(0xffffffffu, most), U, C)) return;
+  const int64_t h_beg = (int64_t)before * p.HKV + (int64_t)h * n, h_end = h_beg + n;
   const int c_first = (int)(((h_beg + 1) * C - 1) / U), c_last = (int)((h_end * C - 1) / U);
   if (c_first == c_last) return;   // one CTA had the whole head and has written it
   auto used = [&](int c) { return U * c / C < U * (c + 1) / C; };   // CTAs without units wrote nothing
@@ -823,7 +874,7 @@ static int launch_decode_attn(const void* q, void* out, const void* k_cache, con
 
   // ring depth: as many 32 KB slots as fit beside the merge rows (6 for G <= 4, else 5)
   constexpr int kMaxSmem = 224 * 1024;  // 227 KB opt-in limit minus static smem
-  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)(kDecWarps + 1) * G * (D + 2) * 4 + (BH + 1) * 4;
+  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)kDecWarps * G * (D + 2) * 4 + (BH + 1 + B) * 4;
   CVLLM_CHECK_SUPPORTED(fixed + 2 * (size_t)kSlotBytes <= (size_t)kMaxSmem);
   int slots = (int)(((size_t)kMaxSmem - fixed) / kSlotBytes);
   if (slots > kMaxSlots) slots = kMaxSlots;
@@ -886,7 +937,7 @@ int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_c
   }
   constexpr int kMaxSmem = 224 * 1024;
   const int BH = B * G, C = sm_count();
-  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)(kDecWarps + 1) * p.G * (D + 2) * 4 + ((size_t)BH + 1) * 4;
+  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)kDecWarps * p.G * (D + 2) * 4 + ((size_t)BH + 1 + B) * 4;
   CVLLM_CHECK_SUPPORTED(fixed + 2 * (size_t)kSlotBytes <= (size_t)kMaxSmem);
   p.slots = (int)(((size_t)kMaxSmem - fixed) / kSlotBytes);
   if (p.slots > kMaxSlots) p.slots = kMaxSlots;

@@ -147,3 +147,19 @@ def test_decode_step_matches_store_then_attend_with_reserved_rows():
     assert torch.equal(kc.view(torch.int16), kc2.view(torch.int16)) and torch.equal(vc.view(torch.int16), vc2.view(torch.int16))
     assert torch.equal(out[live], ref[live])
     assert (out[~live] == 0).all()
+
+
+@pytest.mark.parametrize("HQ,HKV,PS", [(32, 8, 128), (8, 1, 64)])
+@pytest.mark.parametrize("B,units", [(1, 4), (1, 5), (2, 8), (20, 6), (40, 7), (40, 8), (40, 9), (130, 5), (130, 6)])
+def test_decode_whole_and_cut_heads(HQ, HKV, PS, B, units):
+    """Both sides of the rule that leaves short heads whole (longest head 4, 5, 6, 8 units of 128 rows beside shares of under
+    one, up to six and more than six units per CTA), with empty heads, one-row heads and NaN behind every head's end."""
+    dtype, D = torch.bfloat16, 128
+    g = torch.Generator().manual_seed(100 * B + units)
+    lens = torch.randint(1, units * 128 + 1, (B, HKV), generator=g)
+    lens[torch.rand((B, HKV), generator=g) < 0.15] = 0
+    lens[B // 2, 0], lens[0, -1] = 1, units * 128
+    kc, vc, pt, bm = make_paged(B, HKV, D, PS, lens.tolist(), dtype, DEV, seed=B + units, poison=True)
+    q = torch.randn((B, HQ, D), generator=g).to(dtype).to(DEV)
+    out = _check(q, kc, vc, lens.to(torch.int32).to(DEV), pt, bm, HKV, PS, dtype)
+    assert (out.cpu()[(lens == 0).repeat_interleave(HQ // HKV, dim=1)] == 0).all()
