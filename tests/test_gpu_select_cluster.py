@@ -122,3 +122,40 @@ def test_sequences_longer_than_the_bound(H, bound, kind):
     b = evict(scores, lens, retain, H, True, slots, True, 1)
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("D", [8, 32, 64, 128, 256])
+@pytest.mark.parametrize("H,lens,ratio", [(1, [1], 1.0), (16, [255, 257, 1], 0.5), (8, [3000, 512], 0.37), (3, [777] * 9, 0.9),
+                                          (2, [160000, 300], 0.05), (8, [2048], 0.0005)])
+def test_kept_rows_are_where_they_belong(D, H, lens, ratio):
+    """Rows of 16 to 512 bytes, one to eight copy CTAs per tile: every head's kept tokens in ascending order, nothing else moved."""
+    from compactor_vllm.compression.common import extract_and_store_top_kv
+
+    B, PS, n = len(lens), 64, sum(lens)
+    g = torch.Generator(device=DEV).manual_seed(D + H)
+    flat = torch.randn(n * H, generator=g, device=DEV)
+    scores = flat.view(n, H)
+    k, v = (torch.randn(n, H, D, generator=g, device=DEV).bfloat16() for _ in range(2))
+    pages = max(lens) // PS + 2
+    table = torch.randperm((B + 1) * H * pages, generator=g, device=DEV).to(torch.int32).view(B + 1, H, pages).contiguous()
+    kc, vc = (torch.full((table.numel() * PS, D), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    want_k, want_v = kc.clone(), vc.clone()
+    lens0 = torch.randint(0, 3, (B, H), generator=g, device=DEV).to(torch.int32)
+    start, want_lens, cu, retain = lens0.clone(), lens0.clone(), [0], []
+    for b, m in enumerate(lens):
+        at, keep = cu[-1], int(ratio * m * H)
+        cu.append(at + m)
+        retain.append(keep)
+        kept = torch.zeros(m * H, dtype=torch.bool, device=DEV)
+        kept[flat[at * H:(at + m) * H].argsort(descending=True, stable=True)[:keep]] = True
+        for h in range(H):
+            tok = kept.view(m, H)[:, h].nonzero()[:, 0]
+            pos = start[b, h] + torch.arange(tok.numel(), device=DEV)
+            rows = table[b + 1, h, (pos // PS).long()].long() * PS + pos % PS
+            want_k[rows], want_v[rows] = k[at + tok, h], v[at + tok, h]
+            want_lens[b, h] += tok.numel()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    extract_and_store_top_kv(scores=scores, cu_seqlens_k=i32(cu), max_k_len=max(lens), top_k=max(lens) * H, H=H, new_keys=k,
+                             new_vals=v, num_tokens_to_retain=i32(retain), page_table=table, batch_mapping=i32(list(range(1, B + 1))),
+                             bh_lens=lens0, k_cache=kc, v_cache=vc, PAGE_SIZE=PS, PAD_TO_PAGE_SIZE=False)
+    assert torch.equal(lens0, want_lens) and torch.equal(kc, want_k) and torch.equal(vc, want_v)
