@@ -5,6 +5,8 @@
 Each csrc/*.cu is compiled to build/<name>.o (rebuilt when it or a header is
 newer), then linked into lib/libcompactor_sm100.so.  No CMake, no torch: the
 library is a plain C-ABI .so (include/cvllm.h) loaded with ctypes.
+csrc/host/py_call.cpp, which calls it with tensors, becomes lib/_cvllm_call.so
+(against the Python and torch of this interpreter).
 """
 from __future__ import annotations
 
@@ -20,6 +22,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 BUILD = HERE / "build"
 LIB = HERE / "lib" / "libcompactor_sm100.so"
+CALL_SRC, CALL = CSRC / "host" / "py_call.cpp", HERE / "lib" / "_cvllm_call.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -51,6 +54,28 @@ def _compile(src: Path, obj: Path, verbose: bool) -> str:
     return res.stderr if verbose else ""
 
 
+def _build_call(force: bool) -> None:
+    import sysconfig
+
+    import torch
+    stamp = BUILD / "py_call.made_for"           # the torch and Python that it was built against
+    made_for = f"{torch.__version__} {sys.version}"
+    if (not force and CALL.exists() and stamp.exists() and stamp.read_text() == made_for
+            and CALL.stat().st_mtime >= max(CALL_SRC.stat().st_mtime, _newest_header())):
+        return
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+           sysconfig.get_paths()["include"], HERE.parent / "include"]
+    cmd = ["g++", "-O2", "-std=c++20", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-isystem{i}" for i in inc), str(CALL_SRC), "-o", str(CALL), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu",
+           "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {CALL_SRC.name}:\n{res.stdout}\n{res.stderr}")
+    stamp.write_text(made_for)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
     LIB.parent.mkdir(exist_ok=True)
@@ -73,6 +98,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_call(force)
     return LIB
 
 

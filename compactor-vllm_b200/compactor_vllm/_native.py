@@ -1,4 +1,5 @@
-"""ctypes binding of libcompactor_sm100.so (C ABI in include/cvllm.h).
+"""Binding of libcompactor_sm100.so (C ABI in include/cvllm.h): ctypes, and for the calls of a model's step the functions of
+csrc/host/py_call.cpp, which take tensors where the ABI takes pointers.
 
 There is deliberately NO fallback: if the library is missing or a call fails the
 caller gets an exception.  PyTorch is used only for device memory and streams.
@@ -7,7 +8,10 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import importlib.machinery
+import importlib.util
 import os
+import types
 from pathlib import Path
 
 import torch
@@ -153,14 +157,25 @@ _SIGNATURES = {
 }
 
 _lib = None
+CALL_PATH = _PKG_ROOT / "lib" / "_cvllm_call.so"
 
 
 class NativeLibraryError(RuntimeError):
     pass
 
 
-def lib() -> C.CDLL:
-    """Load (once) and return the shared library; raise loudly if absent."""
+def _load_calls() -> types.ModuleType:
+    if not CALL_PATH.exists():
+        raise NativeLibraryError(f"{CALL_PATH} not found: build it with `python compactor-vllm_b200/build.py`")
+    loader = importlib.machinery.ExtensionFileLoader("_cvllm_call", str(CALL_PATH))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_cvllm_call", loader))
+    loader.exec_module(module)
+    return module
+
+
+def lib() -> types.SimpleNamespace:
+    """Load (once) and return the shared library's functions; raise loudly if absent.  Beside them: `call`, the module of
+    csrc/host/py_call.cpp, and `decode_address` / `prefill_address`, what its two whole entry points are given."""
     global _lib
     if _lib is None:
         if not LIB_PATH.exists():
@@ -169,13 +184,18 @@ def lib() -> C.CDLL:
                 "(there is no CPU or PyTorch fallback for this path)"
             )
         handle = C.CDLL(str(LIB_PATH))
+        calls = _load_calls()
+        made = types.SimpleNamespace(handle=handle, call=calls)
         for name, (res, args) in _SIGNATURES.items():
             fn = getattr(handle, name)  # AttributeError if the ABI drifted
             fn.restype = res
             fn.argtypes = args
+            setattr(made, name, calls.bind(name, C.cast(fn, C.c_void_p).value, fn) or fn)
+        made.decode_address = calls.address(C.cast(handle.cvllm_decode_attention, C.c_void_p).value)
+        made.prefill_address = calls.address(C.cast(handle.cvllm_prefill_attention_bounded, C.c_void_p).value)
         if handle.cvllm_abi_version() != 1:
             raise NativeLibraryError("libcompactor_sm100.so ABI version mismatch")
-        _lib = handle
+        _lib = made
     return _lib
 
 

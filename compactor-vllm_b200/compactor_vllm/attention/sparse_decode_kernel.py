@@ -34,6 +34,11 @@ def head_sparse_decode_attention(
     None, :94-103), fixed grid, scratch from torch's caching allocator.  Rows
     whose head is empty are zeros (uninitialised in the reference, :281-283).
     """
+    L = N.lib()
+    out = L.call.decode_attention(L.decode_address, N._WORKSPACES, q, k, v, seq_lens_bh, global_page_table, batch_mapping, HKV,
+                                  PAGE_SIZE, sm_scale)
+    if out is not None:
+        return out
     if q.ndim != 3:
         assert q.ndim == 4
         B, HQ, S, D = q.shape
@@ -56,14 +61,13 @@ def head_sparse_decode_attention(
     out = torch.empty_like(q)
     if B == 0:
         return out
-    L = N.lib()
     ws_bytes = N.sized(dev.index, "cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
     # one workspace per (B, HQ, HKV): the ticket region's size depends on B*HKV, and the "zero on
     # entry, zero on exit" contract only holds while the layout stays the same
     ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
     rc = L.cvllm_decode_attention(
-        N.ptr(q), N.ptr(out), N.ptr(k), N.ptr(v), N.ptr(seq_lens_bh), N.ptr(global_page_table),
-        N.ptr(batch_mapping), N.ptr(ws), ws.numel(), B, HQ, HKV, D, int(PAGE_SIZE),
+        q, out, k, v, seq_lens_bh, global_page_table,
+        batch_mapping, ws, ws.numel(), B, HQ, HKV, D, int(PAGE_SIZE),
         global_page_table.shape[-1], float(sm_scale), N.dtype_code(q.dtype), 0, N.stream(dev),
     )
     N.check(rc, "cvllm_decode_attention")
@@ -107,9 +111,9 @@ def decode_append_and_attend(
     ws_bytes = N.sized(dev.index, "cvllm_decode_attention_workspace_bytes", B, HQ, HKV, D, 0)
     ws = N.workspace(dev, ws_bytes, ("decode_attn", B, HQ, HKV), zero=True)
     rc = L.cvllm_decode_step(
-        N.ptr(key), N.ptr(value), key.stride(0), key.stride(1), value.stride(0), value.stride(1),
-        N.ptr(q), N.ptr(out), N.ptr(k_cache), N.ptr(v_cache), N.ptr(bh_seq_lens), N.ptr(global_page_table),
-        N.ptr(batch_mapping), N.ptr(ws), ws.numel(), B, HQ, HKV, D, int(PAGE_SIZE),
+        key, value, key.stride(0), key.stride(1), value.stride(0), value.stride(1),
+        q, out, k_cache, v_cache, bh_seq_lens, global_page_table,
+        batch_mapping, ws, ws.numel(), B, HQ, HKV, D, int(PAGE_SIZE),
         global_page_table.shape[-1], float(sm_scale), N.dtype_code(q.dtype), int(reserved_batch), 0,
         N.stream(dev),
     )

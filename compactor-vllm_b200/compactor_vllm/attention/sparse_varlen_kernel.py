@@ -35,6 +35,11 @@ def causal_sparse_varlen_with_cache(
     `max_seqlen_k_cache`, the longest prefix, only chooses the order of the work
     (the reference uses it as an autotune key, :164); a wrong one costs speed.
     """
+    L = N.lib()
+    out = L.call.prefill_attention(L.prefill_address, q, k, v, k_cache, v_cache, seq_lens_bh, global_page_table, batch_mapping,
+                                   cu_seqlens_q, max_seqlen_q, max_seqlen_k_cache, HKV, PAGE_SIZE, sm_scale)
+    if out is not None:
+        return out
     assert q.ndim == 3, "q should be [N, HQ, D]"
     Ntok, HQ, D = q.shape
     assert (D & (D - 1)) == 0, "D must be power of two"
@@ -60,7 +65,7 @@ def causal_sparse_varlen_with_cache(
         sm_scale = 1.0 / math.sqrt(D)
     out = torch.empty((Ntok, HQ, D), dtype=q.dtype, device=dev)
     max_past = min(max_seqlen_k_cache, 2 ** 31 - 1) if isinstance(max_seqlen_k_cache, int) else -1
-    rc = N.lib().cvllm_prefill_attention_bounded(
+    rc = L.cvllm_prefill_attention_bounded(
         N.ptr(q), N.ptr(k), N.ptr(v), N.ptr(out), N.ptr(k_cache), N.ptr(v_cache),
         N.ptr(lens), N.ptr(pt), N.ptr(bm), N.ptr(cu),
         B, Ntok, HQ, HKV, D, int(PAGE_SIZE), pt.shape[-1], CACHE_SIZE,

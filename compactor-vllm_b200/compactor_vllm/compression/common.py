@@ -141,10 +141,10 @@ def extract_and_store_top_kv(
     sk_n, sk_h, _ = new_keys.stride()
     sv_n, sv_h, _ = new_vals.stride()
     rc = L.cvllm_select_store_topk_bounded(
-        N.ptr(scores), scores.stride(0), N.ptr(new_keys), N.ptr(new_vals), sk_n, sk_h, sv_n, sv_h,
-        N.ptr(retain), N.ptr(cu), N.ptr(bm), N.ptr(bh_lens), N.ptr(page_table),
-        N.ptr(k_cache), N.ptr(v_cache), B, N_total, H, D, int(PAGE_SIZE), page_table.shape[2],
+        scores, scores.stride(0), new_keys, new_vals, sk_n, sk_h, sv_n, sv_h,
+        retain, cu, bm, bh_lens, page_table,
+        k_cache, v_cache, B, N_total, H, D, int(PAGE_SIZE), page_table.shape[2],
         new_keys.element_size(), int(bool(PAD_TO_PAGE_SIZE)), int(_RESERVED), max_k_len,
-        N.ptr(ws), ws.numel(), N.stream(dev),
+        ws, ws.numel(), N.stream(dev),
     )
     N.check(rc, "cvllm_select_store_topk")

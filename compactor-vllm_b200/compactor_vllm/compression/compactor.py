@@ -151,9 +151,9 @@ def approximate_leverage_scores(
     ws = N.workspace(dev, ws_bytes, "leverage")
     phi = PHI.contiguous()
     rc = L.cvllm_leverage_scores(
-        N.ptr(key_states), key_states.stride(0), key_states.stride(1), N.ptr(offsets), n_chunks,
-        max(chunk_lens), N.ptr(phi), N.ptr(out), Ntok, H, D, sketch, float(regularizer),
-        int(bool(normalize)), N.dtype_code(key_states.dtype), N.ptr(ws), ws.numel(), N.stream(dev),
+        key_states, key_states.stride(0), key_states.stride(1), offsets, n_chunks,
+        max(chunk_lens), phi, out, Ntok, H, D, sketch, float(regularizer),
+        int(bool(normalize)), N.dtype_code(key_states.dtype), ws, ws.numel(), N.stream(dev),
     )
     N.check(rc, "cvllm_leverage_scores")
     return out
@@ -177,8 +177,8 @@ def _leverage_from_sketch(sketch_rows, context_lens, regularizer, normalize, chu
     ws_bytes = L.cvllm_leverage_scores_workspace_bytes(Ntok, H, sketch, n_chunks)
     ws = N.workspace(dev, ws_bytes, "leverage")
     rc = L.cvllm_leverage_scores_from_sketch(
-        N.ptr(sketch_rows), N.ptr(offsets), n_chunks, max(chunk_lens), None, N.ptr(out), Ntok, H, sketch,
-        float(regularizer), int(bool(normalize)), N.dtype_code(sketch_rows.dtype), N.ptr(ws), ws.numel(),
+        sketch_rows, offsets, n_chunks, max(chunk_lens), None, out, Ntok, H, sketch,
+        float(regularizer), int(bool(normalize)), N.dtype_code(sketch_rows.dtype), ws, ws.numel(),
         N.stream(dev),
     )
     N.check(rc, "cvllm_leverage_scores_from_sketch")
@@ -240,10 +240,10 @@ def non_causal_attn_scores(
     ws_bytes = L.cvllm_chunk_attn_scores_workspace_bytes(B, Ntok, HKV, int(chunk_size))
     ws = N.workspace(dev, ws_bytes, "chunk_attn")
     rc = L.cvllm_chunk_attn_scores(
-        N.ptr(q), N.ptr(k), q.stride(0), k.stride(0), N.ptr(cu), B, Ntok, HQ, HKV, D,
+        q, k, q.stride(0), k.stride(0), cu, B, Ntok, HQ, HKV, D,
         int(chunk_size), int(max_seqlen_qk), float(sm_scale), int(bool(normalize)),
-        N.ptr(accum_scores), acc_dtype, acc_stride, blend, N.ptr(pf), N.ptr(pl), N.ptr(out),
-        N.dtype_code(q.dtype), N.ptr(ws), ws.numel(), N.stream(dev),
+        accum_scores, acc_dtype, acc_stride, blend, pf, pl, out,
+        N.dtype_code(q.dtype), ws, ws.numel(), N.stream(dev),
     )
     N.check(rc, "cvllm_chunk_attn_scores")
     return out

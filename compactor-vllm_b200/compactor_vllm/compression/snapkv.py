@@ -71,9 +71,9 @@ def query_aware_key_scores(
     ws_bytes = N.sized(dev.index, "cvllm_snapkv_scores_workspace_bytes", B, N_k, Hq, Hk, w)
     ws = N.workspace(dev, ws_bytes, "snapkv")
     rc = L.cvllm_snapkv_scores(
-        N.ptr(q), N.ptr(k), q.stride(0), k.stride(0), N.ptr(cu_q), N.ptr(cu_k), w, B, N_k, Hq, Hk,
-        D, N_k, float(sm_scale), KPOOL, int(pool_segment), N.ptr(out), N.dtype_code(q.dtype),
-        N.ptr(ws), ws.numel(), N.stream(dev),
+        q, k, q.stride(0), k.stride(0), cu_q, cu_k, w, B, N_k, Hq, Hk,
+        D, N_k, float(sm_scale), KPOOL, int(pool_segment), out, N.dtype_code(q.dtype),
+        ws, ws.numel(), N.stream(dev),
     )
     N.check(rc, "cvllm_snapkv_scores")
     if accum_scores is not None:

@@ -352,23 +352,23 @@ class BiasedChunkAttention(nn.Module):
         dev, code, lib = qkv.device, N.block_dtype_code(qkv.dtype), N.lib()
         q = torch.empty((T, H, D), dtype=qkv.dtype, device=dev)
         pt = self.page_table
-        table = (N.ptr(pt), pt.stride(0), pt.stride(1), int(self.page_size))
+        table = (pt, pt.stride(0), pt.stride(1), int(self.page_size))
         field = self._field
         rot, q_w, k_w = field("inv_freq"), field("q_norm_weight"), field("k_norm_weight")
         if self.row_norm:
-            caches = (None, None) if s is not None else (N.ptr(self.k_cache), N.ptr(self.v_cache))
+            caches = (None, None) if s is not None else (self.k_cache, self.v_cache)
             N.check(lib.cvllm_row_norm_rope_store(
-                N.ptr(qkv), qkv.stride(0), N.ptr(rot), 0 if rot is None else 2 * rot.numel(), N.ptr(q_w),
-                N.ptr(k_w), self.eps, N.ptr(ctx.positions_i32), N.ptr(ctx.token_slot), N.ptr(q), *caches,
-                *table, N.ptr(self.bh_seq_lens), T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
+                qkv, qkv.stride(0), rot, 0 if rot is None else 2 * rot.numel(), q_w,
+                k_w, self.eps, ctx.positions_i32, ctx.token_slot, q, *caches,
+                *table, self.bh_seq_lens, T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
                 "cvllm_row_norm_rope_store")
             return self.attend(q, out=out)
         N.check(lib.cvllm_rope_qknorm_store(
-            N.ptr(qkv), qkv.stride(0), N.ptr(rot), 0 if rot is None else 2 * rot.numel(),
+            qkv, qkv.stride(0), rot, 0 if rot is None else 2 * rot.numel(),
             int(self.norm) + 2 * int(self.value_norm),
-            N.ptr(q_w), N.ptr(k_w), self.eps,
-            N.ptr(ctx.positions_i32), N.ptr(ctx.token_slot), N.ptr(q), N.ptr(self.k_cache), N.ptr(self.v_cache),
-            *table, N.ptr(self.bh_seq_lens), T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
+            q_w, k_w, self.eps,
+            ctx.positions_i32, ctx.token_slot, q, self.k_cache, self.v_cache,
+            *table, self.bh_seq_lens, T, H, G, D, Dv, RESERVED_BATCH, code, N.stream(dev)),
             "cvllm_rope_qknorm_store")
         return self.attend(q, out=out)
 
@@ -381,7 +381,7 @@ class BiasedChunkAttention(nn.Module):
         assert q.is_contiguous() and q.dtype == self.k_cache.dtype
         dev, code, lib = q.device, N.block_dtype_code(q.dtype), N.lib()
         pt = self.page_table
-        table = (N.ptr(pt), pt.stride(0), pt.stride(1), int(self.page_size))
+        table = (pt, pt.stride(0), pt.stride(1), int(self.page_size))
         v_cache, v_stride = (self.k_cache, D) if self.values_in_keys else (self.v_cache, Dv)
         keep = Dv
         if (out is None and self.values_in_keys and ctx.is_prefill and q.dtype == torch.bfloat16 and D == 128 and Dv < D
@@ -402,13 +402,13 @@ class BiasedChunkAttention(nn.Module):
             self.refresh_distance_bias()
             db = field("dist_bias")
         slopes, sink_logits = field("slopes"), field("sink_logits")
-        dist = (self.window, self.keep_first, N.ptr(db), 0 if db is None else db.shape[0])
+        dist = (self.window, self.keep_first, db, 0 if db is None else db.shape[0])
         if ctx.is_prefill:
             B = ctx.batch_mapping.numel()
             N.check(lib.cvllm_bias_attn_varlen_dist(
-                N.ptr(q), N.ptr(self.k_cache), N.ptr(v_cache), *table, N.ptr(ctx.cu_seqlens_q),
-                N.ptr(ctx.seq_start), N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink),
-                N.ptr(sink_logits), self.scale, N.ptr(out), o_stride, B, int(ctx.max_seqlen_q), H, G, D, Dv, T,
+                q, self.k_cache, v_cache, *table, ctx.cu_seqlens_q,
+                ctx.seq_start, ctx.batch_mapping, slopes, self.chunk, *dist, int(self.sink),
+                sink_logits, self.scale, out, o_stride, B, int(ctx.max_seqlen_q), H, G, D, Dv, T,
                 self.k_cache.shape[0], pt.shape[-1], v_stride, code, N.stream(dev)), "cvllm_bias_attn_varlen")
         else:
             assert ctx.batch_mapping.numel() == T
@@ -418,18 +418,18 @@ class BiasedChunkAttention(nn.Module):
                     and (q_at | k_at | v_at) % 16 == 0):
                 ws = N.workspace(dev, N.sized(dev.index, "cvllm_bias_decode_workspace_bytes", T, H, G, D), "bias_attn_stream")
                 N.check(lib.cvllm_bias_attn_decode_stream(
-                    q_at, k_at, v_at, self.k_cache.shape[0], *table, N.ptr(ctx.positions_i32),
-                    N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
-                    self.scale, o_at, o_stride, T, H, G, D, RESERVED_BATCH, N.ptr(ws), ws.numel(), N.stream(dev)),
+                    q_at, k_at, v_at, self.k_cache.shape[0], *table, ctx.positions_i32,
+                    ctx.batch_mapping, slopes, self.chunk, *dist, int(self.sink), sink_logits,
+                    self.scale, o_at, o_stride, T, H, G, D, RESERVED_BATCH, ws, ws.numel(), N.stream(dev)),
                     "cvllm_bias_attn_decode_stream")
             else:
                 splits = self.decode_splits(T, max_keys)
                 ws = N.workspace(dev, 4 * T * H * splits * (2 + Dv), "bias_attn_decode") if splits > 1 else None
                 N.check(lib.cvllm_bias_attn_decode_dist(
-                    q_at, k_at, v_at, *table, N.ptr(ctx.positions_i32),
-                    N.ptr(ctx.batch_mapping), N.ptr(slopes), self.chunk, *dist, int(self.sink), N.ptr(sink_logits),
+                    q_at, k_at, v_at, *table, ctx.positions_i32,
+                    ctx.batch_mapping, slopes, self.chunk, *dist, int(self.sink), sink_logits,
                     self.scale, o_at, o_stride, T, H, G, D, Dv, self.k_cache.shape[0], RESERVED_BATCH, splits,
-                    N.ptr(ws), ws.numel() if ws is not None else 0, v_stride, code, N.stream(dev)), "cvllm_bias_attn_decode")
+                    ws, ws.numel() if ws is not None else 0, v_stride, code, N.stream(dev)), "cvllm_bias_attn_decode")
         if keep != Dv:
             out = out.view(T, H, Dv)[:, :, :keep]
             return out.reshape(T, H * keep) if flat else out

@@ -109,9 +109,9 @@ class DeltaRuleMixer(nn.Module):
         qkv = torch.empty((T, C), dtype=torch.float32, device=dev)
         out = torch.empty((T, H * Dv), dtype=cols.dtype, device=dev)
         x, x_row, qkv_at, out_at, slots_at = N.ptr(cols), cols.stride(0), N.ptr(qkv), N.ptr(out), N.ptr(slots)
-        N.check(lib.cvllm_causal_conv(x, x_row, 0, C, self.taps, N.ptr(self.conv_weight), None, N.ptr(state.conv_state), *geom,
+        N.check(lib.cvllm_causal_conv(x, x_row, 0, C, self.taps, self.conv_weight, None, state.conv_state, *geom,
                                       slots_at, B, max_new, qkv_at, C, code, st), "cvllm_causal_conv")
-        N.check(lib.cvllm_conv_state_update(x, x_row, 0, C, self.taps, N.ptr(state.conv_state), *geom, slots_at, B,
+        N.check(lib.cvllm_conv_state_update(x, x_row, 0, C, self.taps, state.conv_state, *geom, slots_at, B,
                                             RESERVED_BATCH, code, st), "cvllm_conv_state_update")
         g_off = C
         b_off = C + H * Dv
@@ -132,7 +132,7 @@ class DeltaRuleMixer(nn.Module):
                 need = 0
         if need:
             N.check(lib.cvllm_delta_rule_chunks(*rows, geom[0], geom[1], slots_at, T, B, max_new, out_at, H * Dv, H, G, D, Dv,
-                                                RESERVED_BATCH, code, N.ptr(ws), ws.numel(), st), "cvllm_delta_rule_chunks")
+                                                RESERVED_BATCH, code, ws, ws.numel(), st), "cvllm_delta_rule_chunks")
         else:
             N.check(lib.cvllm_delta_rule(*rows, *geom, slots_at, B, max_new, out_at, H * Dv, H, G, D, Dv, RESERVED_BATCH, code,
                                          st), "cvllm_delta_rule")
