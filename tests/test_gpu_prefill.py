@@ -136,3 +136,34 @@ def test_prefill_correction_path(threshold, rescale_threshold):
     ref = torch_prefill_fp32(q, k, v, torch.nan_to_num(kc), torch.nan_to_num(vc), l, pt, bm, cu, HKV, PS)
     assert torch.isfinite(out).all()
     assert (out.float() - ref).abs().max().item() <= ATOL[dtype]
+
+
+@pytest.mark.parametrize("bound", [0, 1 << 20])      # the order by tiles and the one by pairs
+@pytest.mark.parametrize("past", [0, 700])
+def test_prefill_batch_equals_its_sequences(past, bound):
+    """CTAs that go on to other tiles, heads and sequences (some 1300 tiles of one to eight key tiles, and as many places of the grid
+    past a sequence's end) leave nothing behind: every sequence gets what it gets alone, a launch of a wave at most, to the bit but for
+    the 2^-125 that a masked key counts, of a neighbour's values here and of none there (1e-36 where values are below 16)."""
+    dtype, HQ, HKV, D, PS = torch.bfloat16, 32, 8, 128, 128
+    g = torch.Generator().manual_seed(past)
+    lens = torch.randint(1, 260, (48,), generator=g).tolist()
+    lens[3], lens[17], lens[40], lens[47] = 1000, 0, 128, 1
+    B = len(lens)
+    pl = torch.randint(0, past + 1, (B, HKV), generator=g)
+    kc, vc, pt, bm = make_paged(B, HKV, D, PS, pl.tolist(), dtype, DEV, seed=6, poison=True)
+    q, k, v = fused_qkv(sum(lens), HQ, HKV, D, dtype, DEV, seed=8)
+    pl = pl.to(torch.int32).to(DEV)
+
+    def run(q, k, v, pl, bm, cu):
+        return causal_sparse_varlen_with_cache(q, k, v, kc, vc, pl, pt, bm, torch.tensor(cu, dtype=torch.int32, device=DEV),
+                                               max(lens), bound, HKV, PS)
+
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    got = run(q, k, v, pl, bm, cu)
+    for b, n in enumerate(lens):
+        if n:
+            at = slice(cu[b], cu[b + 1])
+            alone = run(q[at], k[at], v[at], pl[b:b + 1].contiguous(), bm[b:b + 1].contiguous(), [0, n])
+            assert (got[at].double() - alone.double()).abs().max().item() <= 128 * 16 * 2.0 ** -125, b
