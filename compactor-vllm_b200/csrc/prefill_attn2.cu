@@ -27,10 +27,10 @@
 // control) and goes on with its tile: barriers, TMEM and the K / V ring stay as they are, the next Q, K and V are loaded beside the
 // last PV, and its first S is made while the softmax groups still write the tile before out.  A launch per tile had 3 us each of
 // set-up, first loads and drain.  The order of the tiles is the grid's, as it was.
-// Measured in a burst (us, before -> after): 32768 tokens 6180 -> 6150 (7080 -> 7060 under the power limit), 4000 + 2077 + 911 + 3301 after
-// up to 3480 cached 533 -> 522, 1000 + 900 + 1100 + 400 53.3 -> 48.1, 4096 119 -> 116, twelve of 500 after up to 2400 178 -> 170.
+// Measured in a burst (us, before -> after): 32768 tokens 6180 -> 6100 (7080 -> 7060 under the power limit), 4000 + 2077 + 911 + 3301 after
+// up to 3480 cached 526 -> 517, 1000 + 900 + 1100 + 400 53.3 -> 47.5, 4096 117.8 -> 113.7, twelve of 500 after up to 2400 176 -> 169.
 // Numbers that the compiler does not know to be the warp's own (an item read from shared memory) stay in vector registers and
-// cost the softmax loop 5 %: next_item passes them through a shuffle.
+// cost the softmax loop 5 %: next_item passes them through a reduction (a shuffle helps less, 522 and 115.7 us above).
 //
 // TMEM (512 columns): S0 [0,128)  S1 [128,256)  O0 [256,384)  O1 [384,512).
 #include <stdlib.h>
@@ -198,12 +198,12 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     mbar_wait(&sm.item_full[i], ((k - 1) >> 1) & 1);
     it = sm.item[i];
     if (mask == 0xffffffffu) {   // numbers that the compiler knows to be the warp's own: they cost the loops no registers
-      it.b = __shfl_sync(mask, it.b, 0);
-      it.hq0 = __shfl_sync(mask, it.hq0, 0);
-      it.qt = __shfl_sync(mask, it.qt, 0);
-      it.q_beg = __shfl_sync(mask, it.q_beg, 0);
-      it.La = __shfl_sync(mask, it.La, 0);
-      it.Lc = __shfl_sync(mask, it.Lc, 0);
+      it.b = __reduce_max_sync(mask, it.b);
+      it.hq0 = __reduce_max_sync(mask, it.hq0);
+      it.qt = __reduce_max_sync(mask, it.qt);
+      it.q_beg = __reduce_max_sync(mask, it.q_beg);
+      it.La = __reduce_max_sync(mask, it.La);
+      it.Lc = __reduce_max_sync(mask, it.Lc);
     }
     if (lane == 0) mbar_arrive(&sm.item_empty[i]);
     return it.b >= 0;
