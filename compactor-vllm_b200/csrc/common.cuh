@@ -89,7 +89,6 @@ struct TestOptions {
   std::atomic<int> decode_mode{0};            // decode_attn.cu profiling modes (0 = product)
   std::atomic<int> decode_slots{0};           // >= 2: cap the decode TMA ring depth
   std::atomic<int> eig_trace{0};
-  std::atomic<int> snap_v1{0};                // 1: the mma.sync SnapKV kernels
   std::atomic<int> chunk_scores_v1{0};        // 1: the mma.sync chunk scorer (A/B against the tcgen05 one)
   std::atomic<int> pdl{0};                    // 1: launch the selection chain with programmatic dependent launch (A/B; off in the product)
   std::atomic<int> select_passes{0};          // 1: the selection as a chain of launches also where one cluster would do

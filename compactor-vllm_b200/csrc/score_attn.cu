@@ -1,5 +1,5 @@
-// Attention-mass key scorers: Compactor's chunk-local non-causal scorer and
-// SnapKV's observation-window scorer.
+// Attention-mass key scorers: Compactor's chunk-local non-causal scorer, and the call of SnapKV's observation-window scorer
+// (score_snap_umma.cu).
 //
 // Reference: compression/compactor.py:338-599 (K11 + z-score epilogue + blend
 // + protection) and compression/snapkv.py:39-276,332-448 (K12 writes ALL
@@ -316,200 +316,6 @@ __global__ void __launch_bounds__(256) chunk_finalize_kernel(const ChunkFinalize
   }
 }
 
-// ===========================================================================
-// SnapKV
-// ===========================================================================
-struct SnapParams {
-  const void* q;
-  const void* k;
-  int64_t q_stride_n, k_stride_n;
-  const int32_t* cu_q;
-  const int32_t* cu_k;
-  float* stats;  // [B, HKV, n_splits, rows_pad, 2] partial (m, l) per row per key split
-  float* out;    // [Nk, HKV]
-  int HQ, HKV, G, w, rows_pad, n_splits, keys_per_split, kpool, pool_segment;
-  float scale_log2;
-};
-
-// rows = (q_off, g): row R -> query token q_end - w + R / G, head hk*G + R % G (snapkv.py:106-113)
-__device__ __forceinline__ const char* snap_qrow(const SnapParams& p, int R, int q_end, int hk) {
-  if (R >= p.w * p.G) return nullptr;
-  const int qo = R / p.G, g = R - qo * p.G;
-  return reinterpret_cast<const char*>(p.q) +
-         ((int64_t)(q_end - p.w + qo) * p.q_stride_n + (int64_t)(hk * p.G + g) * 128) * 2;
-}
-
-// pass 1, grid (n_splits, HKV, B): running (max, sum) of every row over this split's keys
-template <bool BF16>
-__global__ void __launch_bounds__(kScThreads, 1) snap_stats_kernel(const SnapParams p) {
-  extern __shared__ __align__(16) unsigned char s_k[];
-  const int sp = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const int kb = p.cu_k[b], keff = p.cu_k[b + 1] - p.w, q_end = p.cu_q[b + 1];
-  const int n_keys_seq = keff - kb;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, j = lane & 3;
-  const int n_mt = p.rows_pad / 16;
-  float* st = p.stats + ((((int64_t)b * p.HKV + hk) * p.n_splits + sp) * p.rows_pad) * 2;
-  const int k_lo = sp * p.keys_per_split;
-  const int k_hi = min(n_keys_seq, k_lo + p.keys_per_split);
-  if (n_keys_seq <= 0 || k_lo >= k_hi) {
-    for (int R = threadIdx.x; R < p.rows_pad; R += kScThreads) { st[2 * R] = -INFINITY; st[2 * R + 1] = 0.f; }
-    return;
-  }
-  // each warp keeps the stats of its m-tiles in registers across key tiles (<= 2 m-tiles per warp)
-  float m_run[2][2], l_run[2][2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) m_run[t][0] = m_run[t][1] = -INFINITY, l_run[t][0] = l_run[t][1] = 0.f;
-
-  for (int kt = k_lo; kt < k_hi; kt += kKeyTile) {
-    const int nk = min(kKeyTile, k_hi - kt);
-    __syncthreads();
-    stage_k_tile(s_k, reinterpret_cast<const char*>(p.k) + ((int64_t)(kb + kt) * p.k_stride_n + hk * 128) * 2,
-                 p.k_stride_n * 2, nk);
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int mt = warp + t * (kScThreads / 32);
-      if (mt >= n_mt) continue;
-      AFrag128 a;
-      a.load(snap_qrow(p, mt * 16 + r, q_end, hk), snap_qrow(p, mt * 16 + r + 8, q_end, hk), j);
-      float acc[16][4];
-      qk_tile<BF16>(acc, a, s_k, r, j);
-      float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-      for (int nt = 0; nt < 16; ++nt) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const bool ok = (nt * 8 + 2 * j + e) < nk;
-          acc[nt][e] = ok ? acc[nt][e] * p.scale_log2 : -INFINITY;
-          acc[nt][2 + e] = ok ? acc[nt][2 + e] * p.scale_log2 : -INFINITY;
-          mx0 = fmaxf(mx0, acc[nt][e]);
-          mx1 = fmaxf(mx1, acc[nt][2 + e]);
-        }
-      }
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-      const float n0 = fmaxf(m_run[t][0], mx0), n1 = fmaxf(m_run[t][1], mx1);
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-      for (int nt = 0; nt < 16; ++nt) {
-        s0 += ex2(acc[nt][0] - n0) + ex2(acc[nt][1] - n0);
-        s1 += ex2(acc[nt][2] - n1) + ex2(acc[nt][3] - n1);
-      }
-      s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-      s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-      s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-      s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-      l_run[t][0] = l_run[t][0] * ex2(m_run[t][0] - n0) + s0;
-      l_run[t][1] = l_run[t][1] * ex2(m_run[t][1] - n1) + s1;
-      m_run[t][0] = n0;
-      m_run[t][1] = n1;
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int mt = warp + t * (kScThreads / 32);
-    if (mt >= n_mt || j != 0) continue;
-    const int R0 = mt * 16 + r, R1 = R0 + 8;
-    st[2 * R0] = m_run[t][0]; st[2 * R0 + 1] = l_run[t][0];
-    st[2 * R1] = m_run[t][1]; st[2 * R1 + 1] = l_run[t][1];
-  }
-}
-
-// pass 2, grid (key tiles, HKV, B): column sums of exp2(s - m_row) / l_row, pooled, written out
-template <bool BF16>
-__global__ void __launch_bounds__(kScThreads, 1) snap_scores_kernel(const SnapParams p) {
-  extern __shared__ __align__(16) unsigned char s_k[];
-  __shared__ float s_col[kScThreads / 32][kKeyTile];
-  __shared__ float s_raw[kKeyTile];
-  __shared__ float s_m[256], s_il[256];
-  const int tile = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const int kb = p.cu_k[b], ke = p.cu_k[b + 1], keff = ke - p.w, q_end = p.cu_q[b + 1];
-  const int len = ke - kb;
-  const int k0 = tile * kKeyTile;  // relative to the sequence start
-  if (k0 >= len) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, j = lane & 3;
-  const int n_keys_seq = keff - kb;
-  if (p.w <= 0 || n_keys_seq <= 0) {
-    // L <= w: the reference leaves these rows uninitialised (snapkv.py:94-95,204-205); zeros here
-    if ((int)threadIdx.x < min(kKeyTile, len - k0)) p.out[(int64_t)(kb + k0 + threadIdx.x) * p.HKV + hk] = 0.f;
-    return;
-  }
-  const int nk = max(0, min(kKeyTile, n_keys_seq - k0));  // scored keys in this tile
-  if (nk > 0) {
-    // combine the per-split row stats
-    for (int R = threadIdx.x; R < p.rows_pad; R += kScThreads) {
-      const float* st = p.stats + (((int64_t)b * p.HKV + hk) * p.n_splits * p.rows_pad + R) * 2;
-      float M = -INFINITY;
-      for (int s = 0; s < p.n_splits; ++s) M = fmaxf(M, st[(int64_t)s * p.rows_pad * 2]);
-      float L = 0.f;
-      for (int s = 0; s < p.n_splits; ++s) {
-        const float ms = st[(int64_t)s * p.rows_pad * 2];
-        if (ms > -INFINITY) L += st[(int64_t)s * p.rows_pad * 2 + 1] * ex2(ms - M);
-      }
-      s_m[R] = M;
-      s_il[R] = (R < p.w * p.G && L > 0.f) ? 1.f / L : 0.f;
-    }
-    stage_k_tile(s_k, reinterpret_cast<const char*>(p.k) + ((int64_t)(kb + k0) * p.k_stride_n + hk * 128) * 2,
-                 p.k_stride_n * 2, nk);
-    __syncthreads();
-    float colacc[16][2];
-#pragma unroll
-    for (int nt = 0; nt < 16; ++nt) colacc[nt][0] = colacc[nt][1] = 0.f;
-    const int n_mt = p.rows_pad / 16;
-    for (int mt = warp; mt < n_mt; mt += kScThreads / 32) {
-      const int R0 = mt * 16 + r, R1 = R0 + 8;
-      AFrag128 a;
-      a.load(snap_qrow(p, R0, q_end, hk), snap_qrow(p, R1, q_end, hk), j);
-      float acc[16][4];
-      qk_tile<BF16>(acc, a, s_k, r, j);
-      const float m0 = s_m[R0], m1 = s_m[R1], i0 = s_il[R0], i1 = s_il[R1];
-#pragma unroll
-      for (int nt = 0; nt < 16; ++nt) {
-        colacc[nt][0] += ex2(acc[nt][0] * p.scale_log2 - m0) * i0 + ex2(acc[nt][2] * p.scale_log2 - m1) * i1;
-        colacc[nt][1] += ex2(acc[nt][1] * p.scale_log2 - m0) * i0 + ex2(acc[nt][3] * p.scale_log2 - m1) * i1;
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 16; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float v = colacc[nt][e];
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (r == 0) s_col[warp][nt * 8 + 2 * j + e] = v;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < kKeyTile) {
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < kScThreads / 32; ++w) v += s_col[w][threadIdx.x];
-      s_raw[threadIdx.x] = v;
-    }
-    __syncthreads();
-  }
-  // causal kpool-tap mean inside pool_segment-key segments (snapkv.py:253-262); window <- +inf
-  if (threadIdx.x < kKeyTile) {
-    const int i = threadIdx.x;
-    const int kabs = k0 + i;
-    if (kabs < len) {
-      float v;
-      if (i < nk) {
-        const int lo = max(i - (p.kpool - 1), (i / p.pool_segment) * p.pool_segment);
-        float s = 0.f;
-        for (int t = lo; t <= i; ++t) s += s_raw[t];
-        v = s / (float)(i + 1 - lo);
-      } else {
-        v = INFINITY;
-      }
-      p.out[(int64_t)(kb + kabs) * p.HKV + hk] = v;
-    }
-  }
-}
-
 }  // namespace cvllm
 
 using namespace cvllm;
@@ -521,7 +327,7 @@ int cvllm_launch_chunk_scores_umma(const void* q, const void* k, int64_t q_strid
 
 size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV);
 int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
-                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nq, int Nk, int HQ, int HKV,
+                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nk, int HQ, int HKV,
                            int max_seqlen_k, float scale_log2, int kpool, int pool_segment, float* out, float* stats,
                            bool bf16, cudaStream_t st);
 
@@ -598,25 +404,9 @@ extern "C" int cvllm_chunk_attn_scores(const void* q, const void* k, int64_t q_s
                            workspace, workspace_bytes, stream);
 }
 
-static void snap_geometry(int max_seqlen_k, int HQ, int HKV, int w, int* rows_pad, int* n_splits,
-                          int* keys_per_split) {
-  const int G = HQ / HKV;
-  *rows_pad = ((w * G + 15) / 16) * 16;
-  // ~2048 keys per pass-1 CTA keeps the partial-stat traffic small and still fills the chip at 40K
-  int kps = 2048;
-  int ns = (max_seqlen_k + kps - 1) / kps;
-  if (ns < 1) ns = 1;
-  *n_splits = ns;
-  *keys_per_split = kps;
-}
-
 extern "C" size_t cvllm_snapkv_scores_workspace_bytes(int B, int N, int HQ, int HKV, int w) {
   if (B <= 0 || N <= 0 || HKV <= 0 || HQ <= 0) return 256;
-  int rows_pad, n_splits, kps;
-  snap_geometry(N, HQ, HKV, w, &rows_pad, &n_splits, &kps);
-  const size_t v1 = (size_t)B * HKV * n_splits * rows_pad * 2 * sizeof(float);
-  const size_t v2 = cvllm_snap_umma_workspace_bytes(B, N, HKV);  // tcgen05 route (w * G <= 128)
-  return al256(v1 > v2 ? v1 : v2);
+  return al256(cvllm_snap_umma_workspace_bytes(B, N, HKV));
 }
 
 extern "C" int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
@@ -633,29 +423,12 @@ extern "C" int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_strid
   CVLLM_CHECK_SUPPORTED(w * (HQ / HKV) <= 256);
   CVLLM_CHECK_ALIGN(aligned16(q) && aligned16(k) && q_stride_n % 8 == 0 && k_stride_n % 8 == 0);
   CVLLM_CHECK_ARG(workspace_bytes >= cvllm_snapkv_scores_workspace_bytes(B, max_seqlen_k, HQ, HKV, w));
-  if (w > 0 && w * (HQ / HKV) <= 128 && test_options().snap_v1.load() == 0) {
-    // product path for the engine's window (w = 32, G <= 4): tcgen05 tiles fed by TMA (score_snap_umma.cu).
-    // Nq: the q tensor has at least cu_seqlens_q[B] = Nk rows on the prefill path (queries and keys are the same tokens)
-    return cvllm_launch_snap_umma(q, k, q_stride_n, k_stride_n, cu_seqlens_q, cu_seqlens_k, w, B, Nk, Nk, HQ, HKV,
-                                  max_seqlen_k, sm_scale * 1.4426950408889634f, kpool, pool_segment, out,
-                                  reinterpret_cast<float*>(workspace), dtype == CVLLM_BF16,
-                                  static_cast<cudaStream_t>(stream));
-  }
-  SnapParams p;
-  p.q = q; p.k = k; p.q_stride_n = q_stride_n; p.k_stride_n = k_stride_n;
-  p.cu_q = cu_seqlens_q; p.cu_k = cu_seqlens_k; p.stats = reinterpret_cast<float*>(workspace); p.out = out;
-  p.HQ = HQ; p.HKV = HKV; p.G = HQ / HKV; p.w = w; p.kpool = kpool; p.pool_segment = pool_segment;
-  snap_geometry(max_seqlen_k, HQ, HKV, w, &p.rows_pad, &p.n_splits, &p.keys_per_split);
-  p.scale_log2 = sm_scale * 1.4426950408889634f;
   auto st = static_cast<cudaStream_t>(stream);
-  const dim3 g1(p.n_splits, HKV, B), g2((max_seqlen_k + kKeyTile - 1) / kKeyTile, HKV, B);
-  if (dtype == CVLLM_BF16) {
-    snap_stats_kernel<true><<<g1, kScThreads, kScSmem, st>>>(p);
-    snap_scores_kernel<true><<<g2, kScThreads, kScSmem, st>>>(p);
-  } else {
-    snap_stats_kernel<false><<<g1, kScThreads, kScSmem, st>>>(p);
-    snap_scores_kernel<false><<<g2, kScThreads, kScSmem, st>>>(p);
+  if (w == 0) {   // no rows: nothing is scored, and no key is in the window
+    CVLLM_CHECK_CUDA(cudaMemsetAsync(out, 0, (size_t)Nk * HKV * sizeof(float), st));
+    return CVLLM_OK;
   }
-  CVLLM_CHECK_LAUNCHES(2);
-  return CVLLM_OK;
+  return cvllm_launch_snap_umma(q, k, q_stride_n, k_stride_n, cu_seqlens_q, cu_seqlens_k, w, B, Nk, HQ, HKV, max_seqlen_k,
+                                sm_scale * 1.4426950408889634f, kpool, pool_segment, out, reinterpret_cast<float*>(workspace),
+                                dtype == CVLLM_BF16, st);
 }

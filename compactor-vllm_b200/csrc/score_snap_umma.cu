@@ -1,7 +1,8 @@
 // SnapKV observation-window scorer on tcgen05 (reference: compression/snapkv.py:39-276,332-448; K12 + K13).
 //
-// Rows = the last w query tokens x the G query heads of one kv head (w * G <= 128: one UMMA tile; the mma.sync
-// kernels of score_attn.cu serve larger windows), columns = 128-key tiles of the sequence's non-window keys.
+// Rows = the last w query tokens x the G query heads of one kv head (w * G <= 256: R = 1 or 2 row tiles of 128), columns =
+// 128-key tiles of the sequence's non-window keys.  A unit is a key tile against a row tile, R to a key tile, in turn
+// through the four TMEM buffers.
 // Two launches over the same (key split, kv head, sequence) grid, one CTA per split:
 //   pass 1  S = Qwin . K_tile^T (lane = row, column = key): running (max, sum) of every row over the split's
 //           keys -> stats[part][row]
@@ -10,17 +11,21 @@
 //           window keys <- +inf                                                            -> out[key, hk]
 // Roles per CTA as in score_chunk_umma.cu: warp 8 TMA producer (Q window once: a 3-D box {64 d, G heads, w tokens}
 // lands in shared memory already in row order (token, g); K tiles through a 4-slot ring), warp 9 UMMA issuer (four
-// 128-column TMEM buffers), warps 0-7 two warpgroups.  Pass 1: each warpgroup owns one half of the key columns of
-// every tile, a thread keeps its row's 64 logits in registers, and each half writes its own partial statistics
-// (parts = 2 x splits).  Pass 2: the warpgroups take alternate tiles; with the operands swapped a thread owns one
-// KEY, so the sum over the rows stays in its registers, with the rows' statistics read from shared memory as
-// broadcasts.  With lane = row it took 62 shuffles a thread, two barriers of all eight warps a tile and nothing
-// to overlap them with.  40960 keys, 32 / 8 heads, both passes and the call: 88 -> 50 us with the splits below, 131072
-// keys 288 -> 130 us; error against 64 bits (rms, relative) 9.3e-8 -> 5.2e-8.
-// What bounds the passes: pass 1 the read of K, pass 2 the exponentials (128 x 128 a tile at 16 per clock: 1024
-// clocks).  A CTA holds the SM (TMEM, 160 KB of shared memory), so the grid runs in waves of 148 CTAs and a start
-// (barriers, TMEM, the first tile's latency, in pass 2 the statistics) costs as much as four tiles: see
-// snap_split_tiles() for how many CTAs a call is cut into.
+// 128-column TMEM buffers), warps 0-7 two warpgroups.  Pass 1: the warpgroups take alternate tiles (with half the columns of every
+// tile each they loaded TMEM at the same time and took exponentials at the same time), a thread keeps its row's 128
+// logits in registers, and each writes its own partial statistics (parts = 2 x splits).  Pass 2: the warpgroups take
+// alternate tiles; with the operands swapped a thread owns one KEY, so the sum over the rows stays in its registers, with the
+// rows' statistics read from shared memory as broadcasts.  With lane = row it took 62 shuffles a thread, two barriers of
+// all eight warps a tile and nothing to overlap them with.  40960 keys, 32 / 8 heads, both passes and the call: 88 -> 50 us
+// with the splits below, 131072 keys 288 -> 130 us; error against 64 bits (rms, relative) 9.3e-8 -> 5.2e-8.
+// What bounds the passes: pass 1 the read of K (84 MB of 40960 keys: 13 us), pass 2 the exponentials (128 x 128 a tile at 16
+// per clock: 1024 clocks), both the start: a CTA holds the SM (TMEM, 200 KB of shared memory), so the grid runs in waves of 148
+// CTAs and a start (barriers, TMEM, the first tile's latency, in pass 2 the statistics) costs as much as four tiles: see
+// snap_split_tiles() for how many CTAs a call is cut into.  Alternate tiles in pass 1, a unit's row of TMEM in one load, all
+// parts' statistics in flight together, and pass 2 launched while pass 1 ends: 50.0 -> 46.9 us, short prompts 18.2 -> 14.8.
+// Two row tiles (16 / 2 heads, 32 tokens): 153 us on mma.sync, which served them, 26.6 here, and half the error.
+// Two key tiles at a time in pass 2, to read the statistics once for both, took 33.8 us for 29.4: with nine pairs a CTA one
+// warpgroup has a fifth more to do, and shared memory was not the bound.
 #include <algorithm>
 
 #include "common.cuh"
@@ -29,7 +34,7 @@
 namespace cvllm {
 
 namespace sn {
-constexpr int kTile = 128, kHD = 128, kHalf = 64;
+constexpr int kTile = 128, kHD = 128;
 constexpr int kTileBytes = kTile * kHD * 2;  // 32 KB
 constexpr int kBoxBytes = kTileBytes / 2;
 constexpr int kSlots = 4;
@@ -48,9 +53,9 @@ struct SnapUmmaParams {
 };
 
 struct SnapUmmaSmem {
-  unsigned char q[sn::kTileBytes];
+  unsigned char q[2 * sn::kTileBytes];   // two halves of 64 numbers, each of 128 R rows
   unsigned char ring[sn::kSlots][sn::kTileBytes];
-  float2 row_stat[2 * sn::kTile];  // pass 2: (-m, 1 / l) of every row; the second half: (m, l) of the other warpgroup
+  float2 row_stat[2 * sn::kTile];  // pass 2: (-m, 1 / l) of every row; R = 1, second half: (m, l) of the other warpgroup
   float raw[2][2][sn::kTile];      // pass 2: [warpgroup][its tile's parity] column sums before the mean over taps
   uint64_t q_full;
   uint64_t full[sn::kSlots], empty[sn::kSlots];
@@ -58,10 +63,12 @@ struct SnapUmmaSmem {
   uint32_t tmem_base;
 };
 
+// until the launch before is through and its writes are visible
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void snap_bar_256() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ void snap_bar_wg(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory"); }
 
-template <bool BF16, bool PASS2>
+template <bool BF16, bool PASS2, int R>
 __global__ void __launch_bounds__(sn::kThreads, 1)
 snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const SnapUmmaParams p) {
@@ -69,6 +76,9 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   extern __shared__ unsigned char smem_raw[];
   SnapUmmaSmem& sm = *reinterpret_cast<SnapUmmaSmem*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  // pass 2 is launched when the last CTAs of pass 1 are: its CTAs take over the SMs one by one, and set up, load and make
+  // their first S while pass 1 ends elsewhere
+  if constexpr (!PASS2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sp = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int kb = p.cu_k[b], len = p.cu_k[b + 1] - kb, q_end = p.cu_q[b + 1];
@@ -93,6 +103,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float v = n_scored > 0 ? INFINITY : 0.f;
       for (int k = k_lo + threadIdx.x; k < min(len, k_lo + p.split); k += kThreads)
         p.out[(int64_t)(kb + k) * p.HKV + hk] = v;
+      dependency_wait();   // nothing after this launch may begin before pass 1 is through
     }
     return;
   }
@@ -100,7 +111,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(&sm.q_full, 1);
     for (int i = 0; i < kSlots; ++i) { mbar_init(&sm.full[i], 1); mbar_init(&sm.empty[i], 1); }
-    for (int i = 0; i < 4; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], PASS2 ? 128 : 256); }
+    for (int i = 0; i < 4; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], 128); }
     mbar_fence_init();
   }
   if (warp == 9) {
@@ -108,9 +119,9 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tmem_relinquish();
   }
   // rows >= w * G of the Q tile are never loaded: zero them (their logits are then 0, not NaN from stale smem)
-  for (int i = threadIdx.x; i < (kTile - rows) * 16; i += kThreads) {
+  for (int i = threadIdx.x; i < (R * kTile - rows) * 16; i += kThreads) {
     const int r = rows + i / 16, c = i % 16;
-    *reinterpret_cast<uint4*>(sm.q + (c >> 3) * kBoxBytes + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(sm.q + (c >> 3) * R * kBoxBytes + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
   }
   fence_proxy_async_smem();
   tc_fence_before();
@@ -124,7 +135,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (lane == 0) {
       mbar_expect_tx(&sm.q_full, 2 * rows * 128);
       tma_load_3d(sm.q, &tm_q, &sm.q_full, 0, hk * p.G, q_end - p.w);
-      tma_load_3d(sm.q + kBoxBytes, &tm_q, &sm.q_full, 64, hk * p.G, q_end - p.w);
+      tma_load_3d(sm.q + R * kBoxBytes, &tm_q, &sm.q_full, 64, hk * p.G, q_end - p.w);
       for (int t = 0; t < n_tiles; ++t) {
         const int slot = t % kSlots;
         mbar_wait(&sm.empty[slot], ((t / kSlots) & 1) ^ 1);
@@ -140,23 +151,27 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);  // provably warp-uniform for the compiler
     mbar_wait(&sm.q_full, 0);
     for (int t = 0; t < n_tiles; ++t) {
-      const int slot = t % kSlots, buf = t & 3;
+      const int slot = t % kSlots;
       mbar_wait(&sm.full[slot], (t / kSlots) & 1);
-      mbar_wait(&sm.s_empty[buf], ((t >> 2) & 1) ^ 1);
-      tc_fence_after();
-      if (lane == 0) {
-        const uint64_t q_desc = umma_smem_desc(smem_u32(sm.q), 16, 1024);
-        const uint64_t k_desc = umma_smem_desc(smem_u32(sm.ring[slot]), 16, 1024);
 #pragma unroll
-        for (int kk = 0; kk < kHD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBoxBytes + (kk & 3) * 32;
-          const uint64_t qd = umma_desc_add(q_desc, off), kd = umma_desc_add(k_desc, off);
-          umma_ss(tmem_u + buf * kTile, PASS2 ? kd : qd, PASS2 ? qd : kd, idesc, kk > 0 ? 1u : 0u);
+      for (int x = 0; x < R; ++x) {
+        const int unit = t * R + x, buf = unit & 3;
+        mbar_wait(&sm.s_empty[buf], ((unit >> 2) & 1) ^ 1);
+        tc_fence_after();
+        if (lane == 0) {
+          const uint64_t q_desc = umma_smem_desc(smem_u32(sm.q) + x * kBoxBytes, 16, 1024);
+          const uint64_t k_desc = umma_smem_desc(smem_u32(sm.ring[slot]), 16, 1024);
+#pragma unroll
+          for (int kk = 0; kk < kHD / 16; ++kk) {
+            const uint64_t qd = umma_desc_add(q_desc, (kk >> 2) * R * kBoxBytes + (kk & 3) * 32);
+            const uint64_t kd = umma_desc_add(k_desc, (kk >> 2) * kBoxBytes + (kk & 3) * 32);
+            umma_ss(tmem_u + buf * kTile, PASS2 ? kd : qd, PASS2 ? qd : kd, idesc, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(&sm.s_full[buf]);
+          if (x == R - 1) umma_commit(&sm.empty[slot]);
         }
-        umma_commit(&sm.s_full[buf]);
-        umma_commit(&sm.empty[slot]);
+        __syncwarp();
       }
-      __syncwarp();
     }
   } else if (warp < 8) {
     // ====================== softmax statistics / column sums ======================
@@ -166,47 +181,52 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int st = threadIdx.x;        // 0..255
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
     if constexpr (!PASS2) {
-      float m_run = -INFINITY, l_run = 0.f;  // this half's running statistics of the row
-      for (int t = 0; t < n_tiles; ++t) {
-        const int buf = t & 3;
-        const int nk = min(kTile, k_hi - (k_lo + t * kTile));  // scored keys in this tile
-        mbar_wait(&sm.s_full[buf], (t >> 2) & 1);
+      // the running statistics of the row over this warpgroup's units: every second tile, or with R = 2 its row tile's all
+      float m_run = -INFINITY, l_run = 0.f;
+      for (int unit = wg; unit < n_tiles * R; unit += 2) {
+        const int buf = unit & 3;
+        const int nk = min(kTile, k_hi - (k_lo + unit / R * kTile));  // scored keys in this tile
+        mbar_wait(&sm.s_full[buf], (unit >> 2) & 1);
         tc_fence_after();
-        uint32_t r0[32], r1[32];
-        tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base, r0);
-        tmem_ld32(tmem + buf * kTile + wg * kHalf + lane_base + 32, r1);
+        float2 sv[kTile / 2];
+#pragma unroll
+        for (int c = 0; c < kTile / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + buf * kTile + lane_base + 32 * c, r);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) sv[16 * c + i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+        }
         tc_wait_ld();
         tc_fence_before();
         mbar_arrive(&sm.s_empty[buf]);
-        float sv[kHalf];
+        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          sv[i] = __uint_as_float(r0[i]) * p.scale_log2;
-          sv[32 + i] = __uint_as_float(r1[i]) * p.scale_log2;
-        }
+        for (int i = 0; i < kTile / 2; ++i) sv[i] = __fmul2_rn(sv[i], sc2);
         if (nk < kTile) {
 #pragma unroll
-          for (int i = 0; i < kHalf; ++i)
-            if (wg * kHalf + i >= nk) sv[i] = -INFINITY;
+          for (int i = 0; i < kTile / 2; ++i) {
+            if (2 * i >= nk) sv[i].x = -INFINITY;
+            if (2 * i + 1 >= nk) sv[i].y = -INFINITY;
+          }
         }
-        float m0 = sv[0], m1 = sv[1], m2 = sv[2], m3 = sv[3];
+        float m0 = sv[0].x, m1 = sv[0].y, m2 = sv[1].x, m3 = sv[1].y;
 #pragma unroll
-        for (int i = 4; i < kHalf; i += 4) {
-          m0 = fmaxf(m0, sv[i]); m1 = fmaxf(m1, sv[i + 1]); m2 = fmaxf(m2, sv[i + 2]); m3 = fmaxf(m3, sv[i + 3]);
+        for (int i = 2; i < kTile / 2; i += 2) {
+          m0 = fmaxf(m0, sv[i].x); m1 = fmaxf(m1, sv[i].y); m2 = fmaxf(m2, sv[i + 1].x); m3 = fmaxf(m3, sv[i + 1].y);
         }
         // The reference point is rounded up to a whole number: every later change of it, here and where the parts
         // meet, is then a power of two and adds no error (ex2's is one-sided and would add up along the chain).
         const float m_new = fmaxf(m_run, ceilf(fmaxf(fmaxf(m0, m1), fmaxf(m2, m3))));
-        if (m_new > -INFINITY) {  // else: every key of this half is masked so far
-          float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        if (m_new > -INFINITY) {  // else: every key is masked so far
+          const float2 nm2 = make_float2(-m_new, -m_new);
+          float2 a[4];
 #pragma unroll
-          for (int i = 0; i < kHalf; i += 4) {
-            s0 += ex2(sv[i] - m_new);
-            s1 += ex2(sv[i + 1] - m_new);
-            s2 += ex2(sv[i + 2] - m_new);
-            s3 += ex2(sv[i + 3] - m_new);
+          for (int i = 0; i < kTile / 2; ++i) {
+            const float2 x = __fadd2_rn(sv[i], nm2), e = make_float2(ex2(x.x), ex2(x.y));
+            a[i % 4] = i < 4 ? e : __fadd2_rn(a[i % 4], e);
           }
-          l_run = l_run * ex2(m_run - m_new) + ((s0 + s1) + (s2 + s3));  // ex2(-inf) = 0 on the first live tile
+          const float2 u = __fadd2_rn(__fadd2_rn(a[0], a[1]), __fadd2_rn(a[2], a[3]));
+          l_run = l_run * ex2(m_run - m_new) + (u.x + u.y);  // ex2(-inf) = 0 on the first live tile
           m_run = m_new;
         }
       }
@@ -214,55 +234,79 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       stp[0] = m_run;
       stp[1] = l_run;
     } else {
-      // the rows' final statistics: a thread combines one row's parts of one half (part & 1 == wg), then the
-      // first 128 threads the two halves
+      // the rows' final statistics: a thread combines one row's parts of one warpgroup (part & 1 == wg), then with R = 1 the
+      // first 128 threads the two warpgroups'
       {
+        dependency_wait();
         const float2* parts_of = reinterpret_cast<const float2*>(st_base) + (int64_t)wg * kTile + row;
         float M = -INFINITY, L = 0.f;
-#pragma unroll 4
-        for (int s = 0; s < p.n_splits; ++s) M = fmaxf(M, parts_of[(int64_t)s * 2 * kTile].x);
-#pragma unroll 4
-        for (int s = 0; s < p.n_splits; ++s) {
-          const float2 ml = parts_of[(int64_t)s * 2 * kTile];
-          if (ml.x > -INFINITY) L += ml.y * ex2(ml.x - M);
+        constexpr int kAhead = 20;   // parts in flight together (one sequence of 8 KV heads has 18)
+        for (int s0 = 0; s0 < p.n_splits; s0 += kAhead) {
+          float2 ml[kAhead];
+          float m = M;
+#pragma unroll
+          for (int s = 0; s < kAhead; ++s)
+            ml[s] = s0 + s < p.n_splits ? parts_of[(int64_t)(s0 + s) * 2 * kTile] : make_float2(-INFINITY, 0.f);
+#pragma unroll
+          for (int s = 0; s < kAhead; ++s) m = fmaxf(m, ml[s].x);
+          if (m > -INFINITY) {
+            L *= ex2(M - m);          // whole references: a power of two
+#pragma unroll
+            for (int s = 0; s < kAhead; ++s) L += ml[s].y * ex2(ml[s].x - m);
+            M = m;
+          }
         }
-        if (wg == 1) sm.row_stat[kTile + row] = make_float2(M, L);
-        snap_bar_256();
-        if (wg == 0) {
-          const float2 o = sm.row_stat[kTile + row];
-          const float Mt = fmaxf(M, o.x);
-          float Lt = 0.f;
-          if (M > -INFINITY) Lt += L * ex2(M - Mt);
-          if (o.x > -INFINITY) Lt += o.y * ex2(o.x - Mt);
-          sm.row_stat[row] = make_float2(Mt > -INFINITY ? -Mt : 0.f, (row < rows && Lt > 0.f) ? 1.f / Lt : 0.f);
+        auto put = [&](int r, float m, float l) {
+          sm.row_stat[r] = make_float2(m > -INFINITY ? -m : 0.f, (r < rows && l > 0.f) ? 1.f / l : 0.f);
+        };
+        if constexpr (R == 2) {
+          put(wg * kTile + row, M, L);
+        } else {
+          if (wg == 1) sm.row_stat[kTile + row] = make_float2(M, L);
+          snap_bar_256();
+          if (wg == 0) {
+            const float2 o = sm.row_stat[kTile + row];
+            const float Mt = fmaxf(M, o.x);
+            float Lt = 0.f;
+            if (M > -INFINITY) Lt += L * ex2(M - Mt);
+            if (o.x > -INFINITY) Lt += o.y * ex2(o.x - Mt);
+            put(row, Mt, Lt);
+          }
         }
         snap_bar_256();
       }
       const int blocks = (rows + 31) >> 5;  // 32-row column blocks that hold rows
       for (int t = wg; t < n_tiles; t += 2) {
-        const int buf = t & 3;
         const int nk = min(kTile, k_hi - (k_lo + t * kTile));  // scored keys in this tile
-        mbar_wait(&sm.s_full[buf], (t >> 2) & 1);
-        tc_fence_after();
-        float total = 0.f;  // of at most four blocks, each a tree over eight chains of four: short chains of roundings
-        for (int c = 0; c < blocks; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tmem + buf * kTile + lane_base + 32 * c, r);
-          tc_wait_ld();
-          const float4* rs = reinterpret_cast<const float4*>(sm.row_stat + 32 * c);
-          float a[8];
+        float total = 0.f;  // of at most four blocks a row tile, each a tree over eight chains of four: short chains of roundings
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float4 u = rs[i / 2];  // (-m, 1 / l) of two rows
-            const float e0 = ex2(fmaf(__uint_as_float(r[i]), p.scale_log2, u.x));
-            const float e1 = ex2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, u.z));
-            a[i % 8] = i < 8 ? e0 * u.y : fmaf(e0, u.y, a[i % 8]);
-            a[i % 8 + 1] = i < 8 ? e1 * u.w : fmaf(e1, u.w, a[i % 8 + 1]);
+        for (int x = 0; x < R; ++x) {
+          const int unit = t * R + x, buf = unit & 3;
+          mbar_wait(&sm.s_full[buf], (unit >> 2) & 1);
+          tc_fence_after();
+          uint32_t r[4][32];   // the whole row: one wait a unit for TMEM, not four
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld32(tmem + buf * kTile + lane_base + 32 * c, r[c]);
+          tc_wait_ld();
+          tc_fence_before();
+          mbar_arrive(&sm.s_empty[buf]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (4 * x + c < blocks) {
+              const float4* rs = reinterpret_cast<const float4*>(sm.row_stat + kTile * x + 32 * c);
+              float a[8];
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                const float4 u = rs[i / 2];  // (-m, 1 / l) of two rows
+                const float e0 = ex2(fmaf(__uint_as_float(r[c][i]), p.scale_log2, u.x));
+                const float e1 = ex2(fmaf(__uint_as_float(r[c][i + 1]), p.scale_log2, u.z));
+                a[i % 8] = i < 8 ? e0 * u.y : fmaf(e0, u.y, a[i % 8]);
+                a[i % 8 + 1] = i < 8 ? e1 * u.w : fmaf(e1, u.w, a[i % 8 + 1]);
+              }
+              total += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+            }
           }
-          total += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
         }
-        tc_fence_before();
-        mbar_arrive(&sm.s_empty[buf]);
         // causal kpool-tap mean inside pool_segment-key segments (snapkv.py:253-262); window keys <- +inf.  The
         // buffer of this parity is written again two tiles on, behind the next tile's barrier, which every
         // reader of this one passes first
@@ -336,13 +380,14 @@ size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV) {
 }
 
 int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
-                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nq, int Nk, int HQ, int HKV,
+                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nk, int HQ, int HKV,
                            int max_seqlen_k, float scale_log2, int kpool, int pool_segment, float* out, float* stats,
                            bool bf16, cudaStream_t st) {
   const int G = HQ / HKV;
   CUtensorMap tm_q, tm_k;
   const uint32_t boxq[3] = {64, (uint32_t)G, (uint32_t)w};
-  const uint64_t dq[3] = {(uint64_t)sn::kHD, (uint64_t)HQ, (uint64_t)Nq};
+  // the queries' number is not known here (theirs may be another packing than the keys'); a box ends with its sequence
+  const uint64_t dq[3] = {(uint64_t)sn::kHD, (uint64_t)HQ, (uint64_t)0x7fffffff};
   const uint64_t sq[2] = {(uint64_t)sn::kHD * 2, (uint64_t)q_stride_n * 2};
   int rc = make_tmap_16b(&tm_q, q, 3, dq, sq, boxq, bf16);
   if (rc) return rc;
@@ -358,18 +403,32 @@ int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int
   p.kpool = kpool; p.pool_segment = pool_segment; p.scale_log2 = scale_log2;
   const dim3 grid(p.n_splits, HKV, B);
   const int smem = (int)sizeof(SnapUmmaSmem) + 1024;
-  static std::atomic<uint64_t> attr[4] = {{0}, {0}, {0}, {0}};
-  if (bf16) {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)snap_umma_kernel<true, false>, smem, attr[0]));
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)snap_umma_kernel<true, true>, smem, attr[1]));
-    snap_umma_kernel<true, false><<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
-    snap_umma_kernel<true, true><<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
-  } else {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)snap_umma_kernel<false, false>, smem, attr[2]));
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)snap_umma_kernel<false, true>, smem, attr[3]));
-    snap_umma_kernel<false, false><<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
-    snap_umma_kernel<false, true><<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
-  }
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, SnapUmmaParams);
+  static std::atomic<uint64_t> attr[4][2] = {};
+  auto both = [&](Kernel pass1, Kernel pass2, std::atomic<uint64_t>(&done)[2]) -> int {
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)pass1, smem, done[0]));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)pass2, smem, done[1]));
+    pass1<<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(sn::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CVLLM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, pass2, tm_q, tm_k, p));
+    return CVLLM_OK;
+  };
+  if (w * G <= sn::kTile)
+    rc = bf16 ? both(snap_umma_kernel<true, false, 1>, snap_umma_kernel<true, true, 1>, attr[0])
+              : both(snap_umma_kernel<false, false, 1>, snap_umma_kernel<false, true, 1>, attr[1]);
+  else
+    rc = bf16 ? both(snap_umma_kernel<true, false, 2>, snap_umma_kernel<true, true, 2>, attr[2])
+              : both(snap_umma_kernel<false, false, 2>, snap_umma_kernel<false, true, 2>, attr[3]);
+  if (rc) return rc;
   CVLLM_CHECK_LAUNCHES(2);
   return CVLLM_OK;
 }

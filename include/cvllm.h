@@ -60,7 +60,7 @@ uint64_t cvllm_launch_count(void);
  *   "prefill_threshold" t    lazy-rescale threshold of the prefill softmax in log2 units (0 exercises the
  *                            O-correction path on every growing row max); negative = built-in default
  *   "decode_mode" m          decode_attn.cu profiling modes (0 = product), "decode_slots" n  TMA ring depth cap
- *   "chunk_scores_v1" / "snap_v1" 1|0   the mma.sync scorers instead of the tcgen05 ones (A/B)
+ *   "chunk_scores_v1" 1|0    the mma.sync scorer instead of the tcgen05 one (A/B)
  *   "pdl" 1|0                launch the selection chain with programmatic dependent launch (A/B; off by default)
  *   "grs_pairs" n            cap the CTA pairs of cvllm_gemm_allreduce (several virtual ranks on one GPU: the tests)
  *   "grs_rows_per_round" r   rows per reduce round of cvllm_gemm_allreduce (multiple of 256; 0 = default 256)

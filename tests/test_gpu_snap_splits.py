@@ -21,6 +21,10 @@ CASES = [
     ([9000], 3, 1, 32),                        # 96 of 128 rows, one head: 71 tiles on 148 CTAs
     ([40, 6000, 32, 1, 129], 16, 4, 32),       # unequal sequences: more waves, empty splits
     ([1300, 700, 260, 64, 33, 2200, 90, 515, 300, 1025], 16, 8, 16),   # 80 pairs: the fixed split, 32 rows
+    ([33, 500, 9000], 16, 2, 32),              # two row tiles, both full
+    ([200, 3000], 8, 1, 17),                   # two row tiles, 8 rows in the second
+    ([5000], 12, 2, 40),                       # 240 rows
+    ([1300, 700, 260, 64, 33, 2200, 90, 515, 300, 1025] * 4, 16, 2, 32),   # 80 pairs of two row tiles: the fixed split
 ]
 
 
@@ -38,3 +42,26 @@ def test_splits_match_oracle(lens, hq, hkv, w, dtype):
         # 128 products of 2^-24 each, and its exponential by as much relative to itself, once in the
         # numerator and once in the row's sum
         assert ((out[ok] - ref[ok]).abs() <= 4 * 2**-16 * ref[ok].abs() + 1e-7).all()
+
+
+@pytest.mark.parametrize("hq,hkv,w", [(32, 8, 32), (16, 2, 32), (4, 4, 1)])
+def test_queries_packed_otherwise_than_keys(hq, hkv, w):
+    """The query window ends where cu_seqlens_q says, in a packing with more tokens than the keys'."""
+    lens = [300, 40, 1111]
+    q, _, _ = fused_qkv(3 * sum(lens), hq, hkv, 128, torch.bfloat16, DEV, seed=1)
+    _, k, _ = fused_qkv(sum(lens), hq, hkv, 128, torch.bfloat16, DEV, seed=2)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    out = query_aware_key_scores(q, k, (3 * cu).to(DEV), cu.to(DEV), w).cpu()
+    tail = torch.cat([q[3 * e - n:3 * e] for e, n in zip(cu[1:].tolist(), lens)]).contiguous()
+    assert torch.equal(out, query_aware_key_scores(tail, k, cu.to(DEV), cu.to(DEV), w).cpu())
+
+
+def test_no_window_scores_nothing():
+    from compactor_vllm import _native as N
+
+    q, k, _ = fused_qkv(300, 8, 2, 128, torch.float16, DEV, seed=3)
+    cu, out = torch.tensor([0, 300], dtype=torch.int32, device=DEV), torch.full((300, 2), 7.0, device=DEV)
+    ws = torch.empty(1 << 20, dtype=torch.uint8, device=DEV)
+    N.check(N.lib().cvllm_snapkv_scores(q, k, q.stride(0), k.stride(0), cu, cu, 0, 1, 300, 8, 2, 128, 300, 0.1, 5, 64, out, 0, ws,
+                                        ws.numel(), N.stream(out.device)), "snapkv")
+    assert (out == 0).all()
