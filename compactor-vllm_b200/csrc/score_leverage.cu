@@ -39,7 +39,6 @@ struct LevParams {
   const void* sketch;  // optional [N, HKV, 48] 16-bit = round16(K.PHI) from rope.cu; null: derive it from k
   float* raw;       // [N, HKV] fp32 (values already rounded to 16-bit)
   float* gram;      // [n_chunks*HKV][48][48] fp32
-  float* mean;      // [n_chunks*HKV][48] fp32
   float* sv;        // [n_chunks*HKV][48][48] fp32 (values rounded to 16-bit)
   uint16_t* xc;     // centred sketch, 16-bit: chunk ch / head h at (c_beg*HKV + h*c_len)*48, [48][c_len] sketch-major
   int HKV;
@@ -62,18 +61,52 @@ __device__ __forceinline__ float from16(uint16_t x) {
   else return __half2float(__ushort_as_half(x));
 }
 
-struct LevSmem {
-  uint16_t phiT[kSk][128 + 8];        // PHI^T: sketch-major, d contiguous (68-word rows: conflict-free LDS.32 fragments)
+// 48 rows of 520 and 136 16-bit numbers: rows a multiple of 16 bytes apart and 4 banks on, so that eight rows' 16-byte pieces
+// (ldmatrix, stmatrix) lie in separate banks
+struct GramSmem {
+  uint16_t phiT[kSk][128 + 8];        // PHI^T: sketch-major, d contiguous
   uint16_t xt[kSk][kXtStride];        // X^T tile: sketch-major, token contiguous
-  float g[kSk][kSk + 1];              // Gram accumulator (gram kernel) / unused (score kernel)
-  float sv[kSk][kSk];                 // round16(V |lam|^-1/2) (score kernel) / staging (gram kernel)
+  uint16_t stage[kLevThreads / 32][16][128 + 8];   // 16 key rows per warp
+  float g[kSk][kSk + 1];              // Gram accumulator (upper triangle)
   float colsum[kSk];
   float mean[kSk];
 };
+struct ScoreSmem {
+  uint16_t xt[kSk][kXtStride];
+  float sv[kSk][kSk];                 // round16(V |lam|^-1/2)
+};
 
-// X^T tile for tokens [t0, t0+nt): xt[c][t] = round16(sum_d K[t][d] * PHI[d][c]) (optionally centred)
+__device__ __forceinline__ uint32_t lev_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+// 16 bytes, or as many zeros
+__device__ __forceinline__ void lev_copy16(void* dst, const void* src, bool real) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(lev_addr(dst)), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void lev_copies_done() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* row) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(lev_addr(row))
+               : "memory");
+}
+// the right operand of two neighbouring column tiles (rows col, col + 1, .. of `m`, 16 numbers from k0 on): b[0..1] and b[2..3]
+template <int PITCH>
+__device__ __forceinline__ void load_pair(uint32_t (&b)[4], const uint16_t (*m)[PITCH], int col, int k0, int lane) {
+  ldmatrix4(b, &m[col + (lane >> 4) * 8 + (lane & 7)][k0 + ((lane >> 3) & 1) * 8]);
+}
+// the left operand: rows row .. row + 15, 16 numbers from k0 on
+template <int PITCH>
+__device__ __forceinline__ void load_left(uint32_t (&a)[4], const uint16_t (*m)[PITCH], int row, int k0, int lane) {
+  ldmatrix4(a, &m[row + ((lane >> 3) & 1) * 8 + (lane & 7)][k0 + (lane >> 4) * 8]);
+}
+
+// X^T tile for tokens [t0, t0+nt): xt[c][t] = round16(sum_d K[t][d] * PHI[d][c]) (optionally centred).  A warp's 16 key rows come
+// by asynchronous copies while it multiplies the 16 before them; the product's fragments are stored transposed.  Loads of
+// four bytes a lane, four stores of two bytes for every eight columns and the right operand's 96 loads a tile took two
+// thirds of the L1's cycles (the kernel 33 us for 256 chunks, 22 now).
 template <bool BF16>
-__device__ __forceinline__ void sketch_tile(LevSmem& sm, const LevParams& p, int h, int tok0, int nt,
+__device__ __forceinline__ void sketch_tile(GramSmem& sm, const LevParams& p, int h, int tok0, int nt,
                                             bool centre) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, j = lane & 3;
   const char* kb = reinterpret_cast<const char*>(p.k);
@@ -97,53 +130,79 @@ __device__ __forceinline__ void sketch_tile(LevSmem& sm, const LevParams& p, int
     }
     return;
   }
+  uint16_t(*stage)[128 + 8] = sm.stage[warp];
+  auto fetch = [&](int mt) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 2 * i + (lane >> 4), piece = lane & 15, t = mt * 16 + row;
+      lev_copy16(&stage[row][piece * 8], kb + ((int64_t)(tok0 + min(t, nt - 1)) * p.k_stride_n + (int64_t)h * p.k_stride_h) * 2 + piece * 16,
+                 t < nt);
+    }
+  };
+  if (warp < n_mt) fetch(warp);
   for (int mt = warp; mt < n_mt; mt += kLevThreads / 32) {
+    uint32_t a[8][4];
+    lev_copies_done();
+    __syncwarp();
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) load_left(a[ks], stage, 0, 16 * ks, lane);
+    __syncwarp();
+    if (mt + kLevThreads / 32 < n_mt) fetch(mt + kLevThreads / 32);
     const int t_lo = mt * 16 + r, t_hi = t_lo + 8;
-    auto krow = [&](int t) -> const char* {
-      return t < nt ? kb + ((int64_t)(tok0 + t) * p.k_stride_n + (int64_t)h * p.k_stride_h) * 2 : nullptr;
-    };
-    // natural-k chain (mma.cuh): the bits of the reference's cuBLAS GEMM at compactor.py:158
-    FragNat128 alo, ahi;
-    alo.load(reinterpret_cast<const uint16_t*>(krow(t_lo)), j);
-    ahi.load(reinterpret_cast<const uint16_t*>(krow(t_hi)), j);
 #pragma unroll
-    for (int nn = 0; nn < kSk / 8; ++nn) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t* prow = reinterpret_cast<const uint32_t*>(sm.phiT[nn * 8 + r]);
+    for (int nn = 0; nn < kSk / 16; ++nn) {
+      float acc[2][4] = {};
+      // natural-k chain (mma.cuh): the bits of the reference's cuBLAS GEMM at compactor.py:158
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        mma16816<BF16>(acc, alo.w[2 * ks], ahi.w[2 * ks], alo.w[2 * ks + 1], ahi.w[2 * ks + 1], prow[8 * ks + j],
-                       prow[8 * ks + 4 + j]);
-      // acc: rows t_lo / t_hi, sketch cols nn*8 + 2j, +1
-      const int c0 = nn * 8 + 2 * j;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float x0 = round16<BF16>(acc[e]), x1 = round16<BF16>(acc[2 + e]);
-        if (centre) {
-          x0 = round16<BF16>(x0 - sm.mean[c0 + e]);
-          x1 = round16<BF16>(x1 - sm.mean[c0 + e]);
-        }
-        sm.xt[c0 + e][t_lo] = (t_lo < nt) ? to16<BF16>(x0) : 0;
-        sm.xt[c0 + e][t_hi] = (t_hi < nt) ? to16<BF16>(x1) : 0;
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t b[4];
+        load_pair(b, sm.phiT, 16 * nn, 16 * ks, lane);
+        mma16816<BF16>(acc[0], a[ks][0], a[ks][1], a[ks][2], a[ks][3], b[0], b[1]);
+        mma16816<BF16>(acc[1], a[ks][0], a[ks][1], a[ks][2], a[ks][3], b[2], b[3]);
       }
+      // acc[u]: rows t_lo / t_hi, sketch cols 16 nn + 8 u + 2 j, + 1
+      uint32_t m[4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x[e] = round16<BF16>(acc[u][e]);
+          if (centre) x[e] = round16<BF16>(x[e] - sm.mean[16 * nn + 8 * u + 2 * j + (e & 1)]);
+        }
+        m[2 * u] = t_lo < nt ? pack2<BF16>(x[0], x[1]) : 0u;
+        m[2 * u + 1] = t_hi < nt ? pack2<BF16>(x[2], x[3]) : 0u;
+      }
+      asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(
+                       lev_addr(&sm.xt[16 * nn + (lane >> 4) * 8 + (lane & 7)][mt * 16 + ((lane >> 3) & 1) * 8])),
+                   "r"(m[0]), "r"(m[1]), "r"(m[2]), "r"(m[3])
+                   : "memory");
     }
   }
 }
 
-__device__ __forceinline__ void load_phi(LevSmem& sm, const LevParams& p) {
-  const uint16_t* phi = reinterpret_cast<const uint16_t*>(p.phi);
-  for (int i = threadIdx.x; i < 128 * kSk; i += kLevThreads) {
-    const int d = i / kSk, c = i - d * kSk;
-    sm.phiT[c][d] = phi[i];
+__device__ __forceinline__ void load_phi(GramSmem& sm, const LevParams& p) {
+  if (reinterpret_cast<uintptr_t>(p.phi) & 15) {
+    const uint16_t* phi = reinterpret_cast<const uint16_t*>(p.phi);
+    for (int i = threadIdx.x; i < 128 * kSk; i += kLevThreads) sm.phiT[i % kSk][i / kSk] = phi[i];
+    return;
+  }
+  const uint4* phi = reinterpret_cast<const uint4*>(p.phi);   // 6 pieces of eight columns a row
+  for (int i = threadIdx.x; i < 128 * (kSk / 8); i += kLevThreads) {
+    const int d = i / (kSk / 8), c = i % (kSk / 8) * 8;
+    const uint4 v = phi[i];
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sm.phiT[c + e][d] = (uint16_t)(w[e >> 1] >> ((e & 1) * 16));
   }
 }
 
 // ---- kernel 1: grid (n_chunks, HKV): column means + Gram of the centred sketch ----
-// out: gram[(ch*HKV+h)][48][48] = fp32(round16(Xc^T Xc)) + reg*I ; mean[(ch*HKV+h)][48]
+// out: gram[(ch*HKV+h)][48][48] = fp32(round16(Xc^T Xc)) + reg*I
 template <bool BF16>
 __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const LevParams p) {
   extern __shared__ __align__(16) unsigned char lev_smem_raw[];
-  LevSmem& sm = *reinterpret_cast<LevSmem*>(lev_smem_raw);
+  GramSmem& sm = *reinterpret_cast<GramSmem*>(lev_smem_raw);
   const int ch = blockIdx.x, h = blockIdx.y;
   const int c_beg = p.chunk_offsets[ch], c_len = p.chunk_offsets[ch + 1] - c_beg;
   if (c_len <= 0) return;
@@ -214,31 +273,30 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const Lev
       }
     }
     __syncthreads();
-    const int r = lane >> 2, j = lane & 3;
-    // 3 m-tiles (16 sketch rows) x 6 n-tiles (8 sketch cols) = 18 output tiles over 8 warps
-    for (int tile = warp; tile < 18; tile += kLevThreads / 32) {
-      const int mt = tile / 6, nn = tile - mt * 6;
+    // the tiles that hold the upper triangle: 16 sketch rows from `rows` on, columns 16 pair .. 16 pair + 15, for six warps
+    if (warp < 6) {
+      const int rows = warp < 3 ? 0 : warp < 5 ? 16 : 32, pair = warp < 3 ? warp : warp < 5 ? warp - 2 : 2;
       // the accumulator is CARRIED across token tiles (not summed per tile and added): one sequential
       // k16 chain over the whole chunk, the order a non-split-K library GEMM accumulates in — the Gram is
       // rounded to 16 bit next, and on low-rank keys one flipped ulp there moves a chunk's scores by O(1)
-      const int gi = mt * 16 + r, gj = nn * 8 + 2 * j;
-      float acc[4] = {sm.g[gi][gj], sm.g[gi][gj + 1], sm.g[gi + 8][gj], sm.g[gi + 8][gj + 1]};
-      const uint16_t* a_lo = sm.xt[mt * 16 + r];
-      const uint16_t* a_hi = sm.xt[mt * 16 + r + 8];
-      const uint16_t* b_r = sm.xt[nn * 8 + r];
+      const int gi = rows + (lane >> 2), gj = 16 * pair + 2 * (lane & 3);
+      float acc[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[u][e] = sm.g[gi + 8 * (e >> 1)][gj + 8 * u + (e & 1)];
+#pragma unroll 4
       for (int k0 = 0; k0 < nt16; k0 += 16) {
-        const uint32_t a0 = *reinterpret_cast<const uint32_t*>(a_lo + k0 + 2 * j);
-        const uint32_t a1 = *reinterpret_cast<const uint32_t*>(a_hi + k0 + 2 * j);
-        const uint32_t a2 = *reinterpret_cast<const uint32_t*>(a_lo + k0 + 8 + 2 * j);
-        const uint32_t a3 = *reinterpret_cast<const uint32_t*>(a_hi + k0 + 8 + 2 * j);
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(b_r + k0 + 2 * j);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(b_r + k0 + 8 + 2 * j);
-        mma16816<BF16>(acc, a0, a1, a2, a3, b0, b1);
+        uint32_t a[4], b[4];
+        load_left(a, sm.xt, rows, k0, lane);
+        load_pair(b, sm.xt, 16 * pair, k0, lane);
+        mma16816<BF16>(acc[0], a[0], a[1], a[2], a[3], b[0], b[1]);
+        mma16816<BF16>(acc[1], a[0], a[1], a[2], a[3], b[2], b[3]);
       }
-      sm.g[gi][gj] = acc[0];
-      sm.g[gi][gj + 1] = acc[1];
-      sm.g[gi + 8][gj] = acc[2];
-      sm.g[gi + 8][gj + 1] = acc[3];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sm.g[gi + 8 * (e >> 1)][gj + 8 * u + (e & 1)] = acc[u][e];
     }
     __syncthreads();
   }
@@ -249,7 +307,6 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const Lev
     const int a = i / kSk, b = i - a * kSk;
     gout[i] = round16<BF16>(a <= b ? sm.g[a][b] : sm.g[b][a]) + ((a == b) ? p.reg : 0.f);
   }
-  if (tid < kSk) p.mean[(int64_t)(ch * p.HKV + h) * kSk + tid] = sm.mean[tid];
 }
 
 // ---- kernel 2: symmetric eigendecomposition, leverage_eig.cuh ----
@@ -258,19 +315,35 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_gram_kernel(const Lev
 template <bool BF16>
 __global__ void __launch_bounds__(kLevThreads, 2) leverage_score_kernel(const LevParams p) {
   extern __shared__ __align__(16) unsigned char lev_smem_raw[];
-  LevSmem& sm = *reinterpret_cast<LevSmem*>(lev_smem_raw);
+  ScoreSmem& sm = *reinterpret_cast<ScoreSmem*>(lev_smem_raw);
   const int ch = blockIdx.x, h = blockIdx.y;
   const int c_beg = p.chunk_offsets[ch], c_len = p.chunk_offsets[ch + 1] - c_beg;
   if (c_len <= 0) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, j = lane & 3;
+  const bool vec_ok = (c_len & 7) == 0;
+  const uint16_t* xc = p.xc + ((int64_t)c_beg * p.HKV + (int64_t)h * c_len) * kSk;
+  // the centred sketch's tile from token t0 on; whole pieces in flight beside what follows
+  auto fetch = [&](int t0) {
+    const int nt = min(kTokTile, c_len - t0);
+    for (int c = warp; c < kSk; c += kLevThreads / 32) {
+      const uint16_t* src = xc + (int64_t)c * c_len + t0;
+      for (int t8 = lane * 8; t8 < nt; t8 += 256) {
+        if (vec_ok) {
+          lev_copy16(&sm.xt[c][t8], src + t8, true);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sm.xt[c][t8 + e] = (t8 + e < nt) ? src[t8 + e] : (uint16_t)0;
+        }
+      }
+    }
+  };
+  fetch(0);
   {
-    const float* svin = p.sv + (int64_t)(ch * p.HKV + h) * kSk * kSk;
-    for (int i = tid; i < kSk * kSk; i += kLevThreads) (&sm.sv[0][0])[i] = svin[i];
-    if (tid < kSk) sm.mean[tid] = p.mean[(int64_t)(ch * p.HKV + h) * kSk + tid];
+    const float4* svin = reinterpret_cast<const float4*>(p.sv + (int64_t)(ch * p.HKV + h) * kSk * kSk);
+    for (int i = tid; i < kSk * kSk / 4; i += kLevThreads) reinterpret_cast<float4*>(&sm.sv[0][0])[i] = svin[i];
   }
   __syncthreads();
   // B fragments of U = Xc . SV (k = sketch column c, n = eigen-column): SV's entries are 16-bit values held in fp32
-  const int warp = tid >> 5, lane = tid & 31, r = lane >> 2, j = lane & 3;
   uint32_t bfr[3][6][2];
 #pragma unroll
   for (int ks = 0; ks < 3; ++ks)
@@ -279,23 +352,10 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_score_kernel(const Le
       bfr[ks][nn][0] = pack2<BF16>(sm.sv[16 * ks + 2 * j][nn * 8 + r], sm.sv[16 * ks + 2 * j + 1][nn * 8 + r]);
       bfr[ks][nn][1] = pack2<BF16>(sm.sv[16 * ks + 8 + 2 * j][nn * 8 + r], sm.sv[16 * ks + 9 + 2 * j][nn * 8 + r]);
     }
-  const bool vec_ok = (c_len & 7) == 0;
   for (int t0 = 0; t0 < c_len; t0 += kTokTile) {
     const int nt = min(kTokTile, c_len - t0);
-    {
-      const uint16_t* xc = p.xc + ((int64_t)c_beg * p.HKV + (int64_t)h * c_len) * kSk;
-      for (int c = warp; c < kSk; c += kLevThreads / 32) {
-        const uint16_t* src = xc + (int64_t)c * c_len + t0;
-        for (int t8 = lane * 8; t8 < nt; t8 += 256) {
-          if (vec_ok) {
-            *reinterpret_cast<uint4*>(&sm.xt[c][t8]) = *reinterpret_cast<const uint4*>(src + t8);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sm.xt[c][t8 + e] = (t8 + e < nt) ? src[t8 + e] : (uint16_t)0;
-          }
-        }
-      }
-    }
+    if (t0 > 0) fetch(t0);
+    lev_copies_done();
     __syncthreads();
     // U[16 tokens x 48] per m-tile on mma.sync (the scalar form was 48 x 48 FFMA per token); the A operand is read
     // straight out of the sketch-major tile with ldmatrix.trans
@@ -400,7 +460,7 @@ extern "C" size_t cvllm_leverage_scores_workspace_bytes(int N, int HKV, int sket
   if (N <= 0 || HKV <= 0) return 256;
   const size_t mats = (size_t)(n_chunks > 0 ? n_chunks : 0) * HKV;
   return lev_align((size_t)N * HKV * sizeof(float)) + 2 * lev_align(mats * kSk * kSk * sizeof(float)) +
-         lev_align(mats * kSk * sizeof(float)) + lev_align((size_t)N * HKV * kSk * sizeof(uint16_t));
+         lev_align((size_t)N * HKV * kSk * sizeof(uint16_t));
 }
 
 static int leverage_launch(const void* k_pre, int64_t k_stride_n, int64_t k_stride_h, const void* sketch_rows,
@@ -427,27 +487,24 @@ static int leverage_launch(const void* k_pre, int64_t k_stride_n, int64_t k_stri
   wsb += lev_align(mats * kSk * kSk * sizeof(float));
   p.sv = reinterpret_cast<float*>(wsb);
   wsb += lev_align(mats * kSk * kSk * sizeof(float));
-  p.mean = reinterpret_cast<float*>(wsb);
-  wsb += lev_align(mats * kSk * sizeof(float));
   p.xc = reinterpret_cast<uint16_t*>(wsb);
-  const size_t smem = sizeof(LevSmem);
   static std::atomic<uint64_t> attr_g[2] = {{0}, {0}}, attr_s[2] = {{0}, {0}};
   const dim3 grid(n_chunks, HKV);
   if (dtype == CVLLM_BF16) {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<true>, (int)smem, attr_g[1]));
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<true>, (int)smem, attr_s[1]));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<true>, (int)sizeof(GramSmem), attr_g[1]));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<true>, (int)sizeof(ScoreSmem), attr_s[1]));
     CVLLM_CHECK_CUDA(ensure_eig_smem<true>());
-    leverage_gram_kernel<true><<<grid, kLevThreads, smem, st>>>(p);
+    leverage_gram_kernel<true><<<grid, kLevThreads, sizeof(GramSmem), st>>>(p);
     leverage_eig_kernel<true><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
-    leverage_score_kernel<true><<<grid, kLevThreads, smem, st>>>(p);
+    leverage_score_kernel<true><<<grid, kLevThreads, sizeof(ScoreSmem), st>>>(p);
     leverage_finalize_kernel<true><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
   } else {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<false>, (int)smem, attr_g[0]));
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<false>, (int)smem, attr_s[0]));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<false>, (int)sizeof(GramSmem), attr_g[0]));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<false>, (int)sizeof(ScoreSmem), attr_s[0]));
     CVLLM_CHECK_CUDA(ensure_eig_smem<false>());
-    leverage_gram_kernel<false><<<grid, kLevThreads, smem, st>>>(p);
+    leverage_gram_kernel<false><<<grid, kLevThreads, sizeof(GramSmem), st>>>(p);
     leverage_eig_kernel<false><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
-    leverage_score_kernel<false><<<grid, kLevThreads, smem, st>>>(p);
+    leverage_score_kernel<false><<<grid, kLevThreads, sizeof(ScoreSmem), st>>>(p);
     leverage_finalize_kernel<false><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
   }
   CVLLM_CHECK_LAUNCHES(4);

@@ -360,6 +360,29 @@ def _reference_arithmetic_on_device(keys, lens, phi, chunk, reg=5e-3):
     return torch.cat(out, dim=0)
 
 
+@pytest.mark.parametrize("lens,chunk", [([1], 512), ([15, 17, 33], 512), ([500, 511, 513], 512), ([100, 900], 129), ([700, 1300], 0)])
+def test_leverage_layouts(lens, chunk):
+    """Rows of a wider projection, a sketch matrix that is not on 16 bytes, tiles that end inside 16 and 8 rows, chunks of several
+    tiles: the same bits as from plain tensors, and from the sketch's own rows where those are given."""
+    n, H = sum(lens), 5
+    wide = (_structured_keys(n, H + 2, 128, torch.float32, seed=n)).to(torch.bfloat16).to(DEV)
+    keys = wide[:, 1:1 + H]
+    phi = make_phi(128, 48, torch.bfloat16, DEV)
+    odd = torch.empty(128 * 48 + 1, dtype=phi.dtype, device=DEV)[1:].view(128, 48)
+    odd.copy_(phi)
+    assert odd.data_ptr() % 16 and odd.is_contiguous()
+    run = lambda k, f, **kw: approximate_leverage_scores(k, lens, f, normalize=False, chunk_size=chunk, **kw)  # noqa: E731
+    want = run(keys.contiguous(), phi)
+    assert torch.equal(run(keys, phi), want) and torch.equal(run(keys, odd), want)
+    rows = torch.matmul(keys.transpose(0, 1).contiguous().double(), phi.double()).transpose(0, 1)
+    near = run(None, phi, sketch_rows=rows.to(torch.bfloat16).contiguous())
+    assert want.isfinite().all() and near.isfinite().all()
+    if chunk:
+        ref = _reference_arithmetic_on_device(keys.contiguous(), lens, phi, chunk).float()
+        long = torch.cat([torch.full((x,), x >= 96, dtype=torch.bool) for x in osc.split_into_chunks(lens, chunk)[1]]).to(DEV)
+        assert not long.any() or ((want.float() - ref).abs() <= 2e-2 * ref.abs().clamp_min(1.0))[long].float().mean() >= 0.99
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("lens,chunk", [([4096], 512), ([1536, 700, 49], 512), ([32768], 512)])
 def test_leverage_matches_reference_arithmetic_on_device(dtype, lens, chunk):
