@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(128) qknorm_store_kernel(
     float eps, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_slot, T* __restrict__ q_out,
     T* __restrict__ k_cache, T* __restrict__ v_cache, PagedKV c, int32_t* __restrict__ bh_lens, int H, int G, int D,
     int Dv, int reserved_slot, Rotation rot, int norm) {
+  pdl_trigger();   // a decode step's attention may be scheduled
   extern __shared__ float rot_cs[];   // cos [dims / 2], sin [dims / 2]
   const int t = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -716,6 +717,7 @@ __global__ void __launch_bounds__(128) qknorm_store_vec_kernel(
     float eps, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_slot, T* __restrict__ q_out,
     T* __restrict__ k_cache, T* __restrict__ v_cache, PagedKV c, int32_t* __restrict__ bh_lens, int H, int G, int D,
     int Dv, int reserved_slot, int lpr, Rotation rot, int norm) {
+  pdl_trigger();   // a decode step's attention may be scheduled
   extern __shared__ float rot_cs[];   // cos [dims / 2], sin [dims / 2]
   const int t = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -904,6 +906,7 @@ __global__ void __launch_bounds__(kRowNormThreads) row_norm_rope_store_kernel(
     float eps, const int32_t* __restrict__ positions, const int32_t* __restrict__ token_slot, T* __restrict__ q_out,
     T* __restrict__ k_cache, T* __restrict__ v_cache, PagedKV c, int32_t* __restrict__ bh_lens, int H, int G, int D,
     int Dv, int reserved_slot, Rotation rot, int has_kv) {
+  pdl_trigger();   // a decode step's attention may be scheduled
   extern __shared__ float rot_cs[];   // cos [dims / 2], sin [dims / 2]
   __shared__ float2 red[kRowNormThreads / 32];
   constexpr int V = VEC ? 8 : 2;

@@ -24,6 +24,9 @@
 //     a scratch slot; the CTA that completes a head merges (atomic ticket),
 //     every warp folding a strided subset of the slots with independent loads.
 //     Ranges of short heads end at heads' ends (heads_whole), and need none of it
+//   * the launch is scheduled beside the kernel in front of it where that one lets it (the norm and store of a step, another
+//     decode step): barriers and descriptors are ready when it ends.  One sequence of 8192 rows 17.9 -> 15.5 us a call back to
+//     back, 8 x 384 rows 12.3 -> 10.1, a biased step of 8 x 4096 rows, whose fold is scheduled beside it, 40.7 -> 37.3
 // HBM-bound: 4*D bytes per cached (token, head).
 //
 // BIAS: the same streaming for the biased attention's decode steps (cvllm_launch_bias_decode, called by
@@ -271,6 +274,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     mbar_fence_init();
   }
+  pdl_wait();      // what came before wrote the query, the cache's new rows and the lengths
+  pdl_trigger();   // the fold may start (behind the wait: what it reads ahead is then as this kernel finds it)
 
   // ---- phase 0: units per head, exclusive prefix over the BH heads ---------
   {
@@ -744,6 +749,7 @@ __global__ void __launch_bounds__(256) bias_decode_fold_kernel(const BiasDecodeP
     all += __shfl_xor_sync(0xffffffffu, all, o);
   }
   const int n = UnitList(p, b).count;
+  pdl_wait();   // for the states (what is read above was there when the kernel in front let this one start)
   if (n == 0) return;
   const int64_t U = (int64_t)all * p.HKV;
   if (heads_whole(__reduce_max_sync(0xffffffffu, most), U, C)) return;
@@ -889,9 +895,9 @@ static int launch_decode_attn(const void* q, void* out, const void* k_cache, con
   if (bf16) CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128>, kMaxSmem, attr_bf));
   else CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<false, 128>, kMaxSmem, attr_h));
   if (bf16) {
-    decode_attn_kernel<true, 128><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 128>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
   } else {
-    decode_attn_kernel<false, 128><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<false, 128>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
   }
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
@@ -945,14 +951,14 @@ int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_c
   static std::atomic<uint64_t> attr_128{0}, attr_64{0};
   if (D == 128) {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128, true>, kMaxSmem, attr_128));
-    decode_attn_kernel<true, 128, true><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 128, true>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
     CVLLM_CHECK_LAUNCH();
-    bias_decode_fold_kernel<128><<<B * H, 256, 0, st>>>(p, C);
+    CVLLM_CHECK_CUDA(launch_behind(bias_decode_fold_kernel<128>, dim3(B * H), dim3(256), 0, st, p, C));
   } else {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 64, true>, kMaxSmem, attr_64));
-    decode_attn_kernel<true, 64, true><<<C, kDecThreads, smem, st>>>(tm_k, tm_v, p);
+    CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 64, true>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
     CVLLM_CHECK_LAUNCH();
-    bias_decode_fold_kernel<64><<<B * H, 256, 0, st>>>(p, C);
+    CVLLM_CHECK_CUDA(launch_behind(bias_decode_fold_kernel<64>, dim3(B * H), dim3(256), 0, st, p, C));
   }
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;

@@ -63,8 +63,6 @@ struct SnapUmmaSmem {
   uint32_t tmem_base;
 };
 
-// until the launch before is through and its writes are visible
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void snap_bar_256() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ void snap_bar_wg(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory"); }
 
@@ -78,7 +76,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   // pass 2 is launched when the last CTAs of pass 1 are: its CTAs take over the SMs one by one, and set up, load and make
   // their first S while pass 1 ends elsewhere
-  if constexpr (!PASS2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if constexpr (!PASS2) pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sp = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int kb = p.cu_k[b], len = p.cu_k[b + 1] - kb, q_end = p.cu_q[b + 1];
@@ -103,7 +101,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float v = n_scored > 0 ? INFINITY : 0.f;
       for (int k = k_lo + threadIdx.x; k < min(len, k_lo + p.split); k += kThreads)
         p.out[(int64_t)(kb + k) * p.HKV + hk] = v;
-      dependency_wait();   // nothing after this launch may begin before pass 1 is through
+      pdl_wait();   // nothing after this launch may begin before pass 1 is through
     }
     return;
   }
@@ -237,7 +235,7 @@ snap_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       // the rows' final statistics: a thread combines one row's parts of one warpgroup (part & 1 == wg), then with R = 1 the
       // first 128 threads the two warpgroups'
       {
-        dependency_wait();
+        pdl_wait();
         const float2* parts_of = reinterpret_cast<const float2*>(st_base) + (int64_t)wg * kTile + row;
         float M = -INFINITY, L = 0.f;
         constexpr int kAhead = 20;   // parts in flight together (one sequence of 8 KV heads has 18)
@@ -409,17 +407,7 @@ int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)pass1, smem, done[0]));
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)pass2, smem, done[1]));
     pass1<<<grid, sn::kThreads, smem, st>>>(tm_q, tm_k, p);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(sn::kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CVLLM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, pass2, tm_q, tm_k, p));
+    CVLLM_CHECK_CUDA(launch_behind(pass2, grid, dim3(sn::kThreads), smem, st, tm_q, tm_k, p));
     return CVLLM_OK;
   };
   if (w * G <= sn::kTile)

@@ -20,6 +20,7 @@ __global__ void decode_store_kernel(const uint4* __restrict__ key, const uint4* 
                                     const int32_t* __restrict__ page_table, uint4* __restrict__ k_cache,
                                     uint4* __restrict__ v_cache, int B, int HKV, int PS, int NLP,
                                     int reserved_batch, int lens_by_slot) {
+  pdl_trigger();   // the attention behind it may be scheduled
   // strides here are already in uint4 units
   const int rows = B * HKV;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
