@@ -546,6 +546,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) leverage_eig_kernel(const floa
       mma884(v[t], c0[1] + c1[1], s.refl[8 * b + 2 * k4 + 1][8 * t + r8]);
     }
   }
+  pdl_trigger();   // late: kernels that wait on an SM keep others from it
   float* out = sv_out + (int64_t)mat * n * n;
   const int col = 8 * (tid >> 5) + r8;
   const double lam = s.d[col] * back, rs = rsqrt(fabs(lam));

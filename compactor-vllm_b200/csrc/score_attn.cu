@@ -256,6 +256,7 @@ struct ChunkFinalizeParams {
 // grid (tiles, B): every CTA re-reduces its sequence's partials in a fixed order (deterministic),
 // then finishes a tile of tokens: z-score, + blend*accum, protected tokens <- +inf
 __global__ void __launch_bounds__(256) chunk_finalize_kernel(const ChunkFinalizeParams p) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int seq_beg = p.cu[b], seq_end = p.cu[b + 1], len = seq_end - seq_beg;
   if (len <= 0) return;
@@ -387,7 +388,7 @@ static int chunk_scores_impl(const void* q, const void* k, int64_t q_stride_n, i
   f.accum_stride_n = accum_stride_n; f.blend = blend; f.prot_first = prot_first; f.prot_last = prot_last;
   f.HKV = HKV; f.chunk = chunk; f.max_chunks = max_chunks; f.normalize = normalize;
   const int tiles = max(1, min((max_seqlen * HKV + 255) / 256, 2 * sm_count()));
-  chunk_finalize_kernel<<<dim3(tiles, B), 256, 0, st>>>(f);
+  CVLLM_CHECK_CUDA(launch_behind(chunk_finalize_kernel, dim3(tiles, B), dim3(256), 0, st, f));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }

@@ -276,6 +276,7 @@ chunk_scores_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));  // warps 10, 11
   }
 
+  pdl_trigger();
   tc_fence_before();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem, 512);

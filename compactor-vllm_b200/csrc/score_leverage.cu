@@ -316,6 +316,7 @@ template <bool BF16>
 __global__ void __launch_bounds__(kLevThreads, 2) leverage_score_kernel(const LevParams p) {
   extern __shared__ __align__(16) unsigned char lev_smem_raw[];
   ScoreSmem& sm = *reinterpret_cast<ScoreSmem*>(lev_smem_raw);
+  pdl_wait();
   const int ch = blockIdx.x, h = blockIdx.y;
   const int c_beg = p.chunk_offsets[ch], c_len = p.chunk_offsets[ch + 1] - c_beg;
   if (c_len <= 0) return;
@@ -403,6 +404,7 @@ template <bool BF16>
 __global__ void __launch_bounds__(256) leverage_finalize_kernel(const float* __restrict__ raw,
                                                                 const int32_t* __restrict__ chunk_offsets,
                                                                 void* __restrict__ out, int HKV, int normalize) {
+  pdl_wait();
   const int ch = blockIdx.x;
   const int beg = chunk_offsets[ch], len = chunk_offsets[ch + 1] - beg;
   if (len <= 0) return;
@@ -489,6 +491,8 @@ static int leverage_launch(const void* k_pre, int64_t k_stride_n, int64_t k_stri
   wsb += lev_align(mats * kSk * kSk * sizeof(float));
   p.xc = reinterpret_cast<uint16_t*>(wsb);
   static std::atomic<uint64_t> attr_g[2] = {{0}, {0}}, attr_s[2] = {{0}, {0}};
+  // the last two are scheduled beside the end of the kernel in front; the eigensolver is not: its CTAs would come two to the SMs
+  // whose Gram is done first, where one each is faster (256 chunks 147 -> 149 us a call)
   const dim3 grid(n_chunks, HKV);
   if (dtype == CVLLM_BF16) {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<true>, (int)sizeof(GramSmem), attr_g[1]));
@@ -496,16 +500,18 @@ static int leverage_launch(const void* k_pre, int64_t k_stride_n, int64_t k_stri
     CVLLM_CHECK_CUDA(ensure_eig_smem<true>());
     leverage_gram_kernel<true><<<grid, kLevThreads, sizeof(GramSmem), st>>>(p);
     leverage_eig_kernel<true><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
-    leverage_score_kernel<true><<<grid, kLevThreads, sizeof(ScoreSmem), st>>>(p);
-    leverage_finalize_kernel<true><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
+    CVLLM_CHECK_CUDA(launch_behind(leverage_score_kernel<true>, grid, dim3(kLevThreads), sizeof(ScoreSmem), st, p));
+    CVLLM_CHECK_CUDA(launch_behind(leverage_finalize_kernel<true>, dim3(n_chunks), dim3(256), 0, st, p.raw, chunk_offsets, out_scores,
+                                   HKV, normalize));
   } else {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_gram_kernel<false>, (int)sizeof(GramSmem), attr_g[0]));
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)leverage_score_kernel<false>, (int)sizeof(ScoreSmem), attr_s[0]));
     CVLLM_CHECK_CUDA(ensure_eig_smem<false>());
     leverage_gram_kernel<false><<<grid, kLevThreads, sizeof(GramSmem), st>>>(p);
     leverage_eig_kernel<false><<<(unsigned)mats, kEigThreads, sizeof(EigSmem), st>>>(p.gram, p.sv, chunk_offsets, HKV, (int)mats, nullptr, nullptr, nullptr);
-    leverage_score_kernel<false><<<grid, kLevThreads, sizeof(ScoreSmem), st>>>(p);
-    leverage_finalize_kernel<false><<<n_chunks, 256, 0, st>>>(p.raw, chunk_offsets, out_scores, HKV, normalize);
+    CVLLM_CHECK_CUDA(launch_behind(leverage_score_kernel<false>, grid, dim3(kLevThreads), sizeof(ScoreSmem), st, p));
+    CVLLM_CHECK_CUDA(launch_behind(leverage_finalize_kernel<false>, dim3(n_chunks), dim3(256), 0, st, p.raw, chunk_offsets, out_scores,
+                                   HKV, normalize));
   }
   CVLLM_CHECK_LAUNCHES(4);
   return CVLLM_OK;

@@ -611,6 +611,7 @@ __global__ void __launch_bounds__(kClThreads) sel_cluster_kernel(
   }
   if (rank == 0 && tid < H)
     w.state_h[b * H + tid] = SegState{s_prefix[tid], s_remaining[tid], s_active[tid], 0};
+  pdl_trigger();   // late: the copy's CTAs wait on the SMs that the clusters leave free, and keep others from them
   // ---- phase 4: per tile / head: (#keys > T_h, #keys == T_h), a warp per tile ----
   const int subs = 32 / H;
   for (int t = tile0 + warp; t < tile1; t += kClThreads / 32) {
@@ -847,13 +848,17 @@ extern "C" size_t cvllm_select_store_workspace_bytes(int B, int H, int N) {
 }
 
 template <int V>
-static void launch_sel_gather(dim3 grid, cudaStream_t st, const float* scores, int64_t s_stride_n,
+static void launch_sel_gather(bool behind, dim3 grid, cudaStream_t st, const float* scores, int64_t s_stride_n,
                               const void* keys, const void* vals, int64_t sk_n, int64_t sk_h,
                               int64_t sv_n, int64_t sv_h, const int32_t* cu, const int32_t* bm,
                               const int32_t* pt, int32_t* bh_lens, void* kc, void* vc, int H, int PS,
                               int NLP, const SelWs& w) {
-  launch_pdl(sel_gather_kernel<V>, grid, dim3(kTileTok), 0, st, scores, s_stride_n, (const uint4*)keys,
-             (const uint4*)vals, sk_n, sk_h, sv_n, sv_h, cu, bm, pt, bh_lens, (uint4*)kc, (uint4*)vc, H, PS, NLP, w);
+  auto go = [&](auto launch) {
+    launch(sel_gather_kernel<V>, grid, dim3(kTileTok), 0, st, scores, s_stride_n, (const uint4*)keys, (const uint4*)vals, sk_n, sk_h,
+           sv_n, sv_h, cu, bm, pt, bh_lens, (uint4*)kc, (uint4*)vc, H, PS, NLP, w);
+  };
+  if (behind) go([](auto... a) { return launch_behind(a...); });
+  else go([](auto... a) { return launch_pdl(a...); });
 }
 
 extern "C" int cvllm_select_store_topk_bounded(const float* scores, int64_t s_stride_n, const void* keys,
@@ -907,7 +912,8 @@ extern "C" int cvllm_select_store_topk_bounded(const float* scores, int64_t s_st
   const int tiles_per_cta = cdiv(cdiv(longest, kTileTok), cluster);
   const size_t cl_smem = sel_cluster_smem(tiles_per_cta, HKV);
   constexpr size_t kClSmemMax = 226 * 1024;   // beside the static arrays
-  if (cl_smem <= kClSmemMax && test_options().select_passes.load() == 0) {
+  const bool one_launch = cl_smem <= kClSmemMax && test_options().select_passes.load() == 0;
+  if (one_launch) {
     static std::atomic<uint64_t> attr{0};
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)sel_cluster_kernel, (int)kClSmemMax, attr));
     cudaLaunchConfig_t cfg = {};
@@ -946,7 +952,7 @@ extern "C" int cvllm_select_store_topk_bounded(const float* scores, int64_t s_st
   const int tiles = cdiv(N, kTileTok) + (B - 1);   // at most: each sequence may end inside one
   const dim3 ggrid(grid.x, grid.y, max(1, min(8, 4 * sm_count() / tiles)));
 #define G(V)                                                                                            \
-  launch_sel_gather<V>(ggrid, st, scores, s_stride_n, keys, vals, sk_n / per16, sk_h / per16, sv_n / per16, \
+  launch_sel_gather<V>(one_launch, ggrid, st, scores, s_stride_n, keys, vals, sk_n / per16, sk_h / per16, sv_n / per16, \
                        sv_h / per16, cu_seqlens_k, batch_mapping, page_table, bh_lens, k_cache, v_cache,   \
                        HKV, PS, NLP, w)
   switch (vpr) {
