@@ -879,6 +879,7 @@ __global__ void __launch_bounds__(128) qknorm_store_many_kernel(
       }
     }
   }
+  pdl_trigger();   // late: the attention's CTAs hold an SM each
 }
 
 // ---------------------------------------------------------------------------------------------------------

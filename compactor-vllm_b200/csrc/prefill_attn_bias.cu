@@ -142,6 +142,7 @@ prefill_attn_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();      // the launch is scheduled beside the norm and store in front
   TileOrder at = {(int)(gridDim.x - 1 - blockIdx.x), (int)blockIdx.y, (int)blockIdx.z};
   int q_beg = p.cu_seqlens_q[at.b], q_end = p.cu_seqlens_q[at.b + 1], start = p.seq_start[at.b];
   if (p.by_tile && pasts_are_short(p.seq_start, p.B, kBM)) {   // (behind the loads above: see prefill_attn2.cu)
@@ -593,7 +594,7 @@ int launch_bias(const CUtensorMap& tm_q, const CUtensorMap& tm_kc, const CUtenso
   const dim3 grid((max_seqlen_q + pb::kBM - 1) / pb::kBM, p.HQ / 2, p.B);
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)prefill_attn_bias_kernel<HD, DIST, EXACT>, (int)smem, attr));
-  prefill_attn_bias_kernel<HD, DIST, EXACT><<<grid, pb::kThreads, smem, st>>>(tm_q, tm_kc, tm_vc, p);
+  CVLLM_CHECK_CUDA(launch_behind(prefill_attn_bias_kernel<HD, DIST, EXACT>, grid, dim3(pb::kThreads), smem, st, tm_q, tm_kc, tm_vc, p));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }
