@@ -189,6 +189,8 @@ __device__ __forceinline__ void unit_of(int u, int& m, int& mt, int& nt) {
 
 template <int D>
 __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const DeltaChunkArgs a) {
+  pdl_wait();      // each of the three kernels is scheduled beside the one in front
+  pdl_trigger();
   extern __shared__ unsigned char smem_raw[];
   const int grp = blockIdx.y;
   int b, c, t0, n;
@@ -377,6 +379,8 @@ __device__ __forceinline__ void split3(double x, double y, uint32_t& hi, uint32_
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kPrepThreads, 2) delta_coef_kernel(const DeltaChunkArgs a) {
+  pdl_wait();
+  pdl_trigger();
   using L = CoefSmem<D>;
   extern __shared__ unsigned char smem_raw[];
   __shared__ float2 s_tok[kChunk];                    // decays and betas
@@ -776,6 +780,7 @@ __device__ __forceinline__ void take_first(uint32_t addr, float2 (&v)[8]) {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(512, 1) delta_chunk_kernel(const DeltaChunkArgs a) {
+  pdl_wait();
   using L = ChunkSmem<D>;
   extern __shared__ unsigned char smem_raw[];
   __shared__ ChunkBars bars;
@@ -1188,20 +1193,22 @@ int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) 
   for (int w = 0; w < p.windows; ++w) {
     a.window = w * (p.per_seq > 0 ? p.per_seq : p.slots);
     if (w > 0) std::swap(a.carry_in, a.carry_out);
-    delta_rows_kernel<D><<<dim3(p.slots, a.G), kPrepThreads, smem_r, st>>>(a);
-    delta_coef_kernel<T, D><<<dim3(p.slots, a.H), kPrepThreads, smem_k, st>>>(a);
+    CVLLM_CHECK_CUDA(launch_behind(delta_rows_kernel<D>, dim3(p.slots, a.G), dim3(kPrepThreads), smem_r, st, a));
+    CVLLM_CHECK_CUDA(launch_behind(delta_coef_kernel<T, D>, dim3(p.slots, a.H), dim3(kPrepThreads), smem_k, st, a));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.H * VT, B);
     cfg.blockDim = dim3(512);
     cfg.dynamicSmemBytes = smem_c;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = VT;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = VT;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = VT > 1 ? 1 : 0;
+    cfg.numAttrs = VT > 1 ? 2 : 1;
     CVLLM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, delta_chunk_kernel<T, D>, a));
   }
   CVLLM_CHECK_LAUNCHES(3 * p.windows);

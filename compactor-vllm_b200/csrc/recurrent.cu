@@ -1452,6 +1452,7 @@ struct DeltaTile {
 template <typename T, int KS>
 __global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict__ qkv, const T* __restrict__ proj,
                                                          DeltaArgs da, RecurArgs a) {
+  pdl_wait();   // scheduled beside the convolution's state update
   namespace cg = cooperative_groups;
   constexpr int C = 4, DP = KS * kGlaRows;
   using Tile = DeltaTile<KS, C, 1>;
@@ -1530,6 +1531,7 @@ constexpr int kDeltaMain = 8;                   // most main warps
 template <typename T, int KS, int C>
 __global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers<C>) * 32, 1)
 delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, DeltaArgs da, RecurArgs a) {
+  pdl_wait();   // scheduled beside the convolution's state update
   namespace cg = cooperative_groups;
   constexpr int U = kGlaBlock, DP = KS * kGlaRows, HW = kDeltaHelpers<C>;
   using Coef = DeltaCoef<U>;
@@ -1928,19 +1930,25 @@ inline RecurShape recur_shape(int D, int Dv, int pairs, int max_new, int extra =
 }
 
 template <typename K, typename... Args>
-cudaError_t launch_clustered(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, Args... args) {
+cudaError_t launch_clustered(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, bool behind,
+                             Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (behind) {   // as launch_behind (common.cuh)
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
@@ -1948,7 +1956,7 @@ template <typename T, int KS, int C, int U>
 int launch_gla(const GlaShape& sh, dim3 grid, cudaStream_t st, const void* proj, const GlaArgs& ga, const RecurArgs& a) {
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)gla_scan_kernel<T, KS, C, U>, 200 * 1024, attr));
-  CVLLM_CHECK_CUDA(launch_clustered(gla_scan_kernel<T, KS, C, U>, grid, sh.warps * 32, sh.smem(sizeof(T)), st, sh.VT,
+  CVLLM_CHECK_CUDA(launch_clustered(gla_scan_kernel<T, KS, C, U>, grid, sh.warps * 32, sh.smem(sizeof(T)), st, sh.VT, false,
                                     static_cast<const T*>(proj), ga, a));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
@@ -1977,7 +1985,7 @@ int launch_delta(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* 
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)delta_scan_kernel<T, KS, C>, 200 * 1024, attr));
   CVLLM_CHECK_CUDA(launch_clustered(delta_scan_kernel<T, KS, C>, grid, (sh.warps + kDeltaHelpers<C>) * 32, sh.smem(sizeof(T)), st,
-                                    sh.VT, qkv, static_cast<const T*>(proj), da, a));
+                                    sh.VT, true, qkv, static_cast<const T*>(proj), da, a));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }
@@ -1985,7 +1993,7 @@ int launch_delta(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* 
 template <typename T, int KS>
 int launch_delta_step(const DeltaShape& sh, dim3 grid, cudaStream_t st, const float* qkv, const void* proj, const DeltaArgs& da,
                       const RecurArgs& a) {
-  CVLLM_CHECK_CUDA(launch_clustered(delta_step_kernel<T, KS>, grid, sh.warps * 32, sh.smem(sizeof(T)), st, sh.VT, qkv,
+  CVLLM_CHECK_CUDA(launch_clustered(delta_step_kernel<T, KS>, grid, sh.warps * 32, sh.smem(sizeof(T)), st, sh.VT, true, qkv,
                                     static_cast<const T*>(proj), da, a));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
@@ -2022,7 +2030,7 @@ int launch_wkv(dim3 grid, const RecurShape& sh, cudaStream_t st, const void* r, 
                const float* bonus, const RecurArgs& a) {
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)wkv_scan_kernel<T, R, MAXT>, max_recur_smem<R>(3), attr));
-  CVLLM_CHECK_CUDA(launch_clustered(wkv_scan_kernel<T, R, MAXT>, grid, sh.threads, sh.smem(3), st, sh.VT,
+  CVLLM_CHECK_CUDA(launch_clustered(wkv_scan_kernel<T, R, MAXT>, grid, sh.threads, sh.smem(3), st, sh.VT, false,
                                     static_cast<const T*>(r), r_stride, static_cast<const T*>(k), k_stride,
                                     static_cast<const T*>(v), v_stride, static_cast<const T*>(w_raw), w_stride, w0,
                                     bonus, a));
@@ -2036,7 +2044,7 @@ int launch_general_delta(dim3 grid, const RecurShape& sh, cudaStream_t st, const
                          const float* w0, float rate, const RecurArgs& a) {
   static std::atomic<uint64_t> attr{0};
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)general_delta_kernel<T, R, MAXT>, max_recur_smem<R>(5), attr));
-  CVLLM_CHECK_CUDA(launch_clustered(general_delta_kernel<T, R, MAXT>, grid, sh.threads, sh.smem(5), st, sh.VT,
+  CVLLM_CHECK_CUDA(launch_clustered(general_delta_kernel<T, R, MAXT>, grid, sh.threads, sh.smem(5), st, sh.VT, false,
                                     static_cast<const T*>(proj), proj_stride, r_off, k_off, v_off, a_off,
                                     static_cast<const T*>(w_raw), w_stride, w0, rate, a));
   CVLLM_CHECK_LAUNCH();
@@ -2051,7 +2059,7 @@ int launch_matrix_memory(dim3 grid, const RecurShape& sh, cudaStream_t st, const
   CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)matrix_memory_kernel<T, R, MAXT>, max_recur_smem<R>(2), attr));
   // + the warp that walks the gates; + the two stages' gate records
   CVLLM_CHECK_CUDA(launch_clustered(matrix_memory_kernel<T, R, MAXT>, grid, sh.threads + 32,
-                                    sh.smem(2) + sizeof(float) * 8 * kTokMax, st, sh.VT,
+                                    sh.smem(2) + sizeof(float) * 8 * kTokMax, st, sh.VT, false,
                                     static_cast<const T*>(proj), proj_stride, q_off, k_off, v_off, i_off, f_off, cap,
                                     q_scale, nvec, mstate, a));
   CVLLM_CHECK_LAUNCH();

@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(128) causal_conv_run_kernel(const T* __restric
                                                               const float* __restrict__ bias,
                                                               const T* __restrict__ conv_state, StepGeom g,
                                                               TO* __restrict__ out, int64_t o_stride) {
+  pdl_trigger();   // the state's update may be scheduled
   const int b = blockIdx.y;
   int t0, n_new, start;
   portion(g, b, t0, n_new, start);
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(128) causal_conv_quads_kernel(const T* __restr
                                                                 const float* __restrict__ bias,
                                                                 const T* __restrict__ conv_state, StepGeom g,
                                                                 TO* __restrict__ out, int64_t o_stride) {
+  pdl_trigger();
   using In = typename Four<T>::raw;
   using Out = typename Four<TO>::raw;
   const int b = blockIdx.y;
@@ -205,6 +207,8 @@ __global__ void __launch_bounds__(128) conv_state_update_kernel(const T* __restr
                                                                 int x_off, int C, int taps,
                                                                 T* __restrict__ conv_state, StepGeom g,
                                                                 int reserved_slot) {
+  pdl_wait();      // scheduled beside the convolution, which reads what this writes
+  pdl_trigger();   // the mixer's kernel may be scheduled
   const int b = blockIdx.x;
   const int ch = blockIdx.y * 128 + threadIdx.x;
   if (ch >= C) return;
@@ -768,13 +772,12 @@ extern "C" int cvllm_conv_state_update(const void* proj, int64_t proj_stride, in
   const StepGeom g{cu_seqlens_q, seq_start, positions, batch_mapping};
   const dim3 grid(B, cdiv(channels, 128));
   if (dtype == CVLLM_BF16)
-    conv_state_update_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(proj), proj_stride,
-                                                                  x_off, channels, taps,
-                                                                  static_cast<__nv_bfloat16*>(conv_state), g,
-                                                                  reserved_slot);
+    CVLLM_CHECK_CUDA(launch_behind(conv_state_update_kernel<__nv_bfloat16>, grid, dim3(128), 0, st,
+                                   static_cast<const __nv_bfloat16*>(proj), proj_stride, x_off, channels, taps,
+                                   static_cast<__nv_bfloat16*>(conv_state), g, reserved_slot));
   else
-    conv_state_update_kernel<float><<<grid, 128, 0, st>>>(static_cast<const float*>(proj), proj_stride, x_off, channels,
-                                                          taps, static_cast<float*>(conv_state), g, reserved_slot);
+    CVLLM_CHECK_CUDA(launch_behind(conv_state_update_kernel<float>, grid, dim3(128), 0, st, static_cast<const float*>(proj),
+                                   proj_stride, x_off, channels, taps, static_cast<float*>(conv_state), g, reserved_slot));
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;
 }
