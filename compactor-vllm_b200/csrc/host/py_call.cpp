@@ -131,11 +131,12 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
-// an ordinary CUDA tensor: no subclass, conjugate or negative view; the caller checks shapes and strides
+// an ordinary CUDA tensor: no subclass, conjugate or negative view, and memory of its own (a tensor that vmap or a transform of
+// torch.func stands in for has none); the caller checks shapes and strides
 const at::Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  return t.is_cuda() && t.layout() == at::kStrided && !t.is_conj() && !t.is_neg() ? &t : nullptr;
+  return t.is_cuda() && t.layout() == at::kStrided && t.has_storage() && !t.is_conj() && !t.is_neg() ? &t : nullptr;
 }
 bool index_on(const at::Tensor& t, const at::Device& dev) {
   return t.scalar_type() == at::kInt && t.device() == dev && t.is_contiguous();
@@ -194,13 +195,18 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* work = plain(ws);
   if (!work) Py_RETURN_NONE;
   const at::Tensor space = *work;     // held for the call: another thread may replace the entry
+  const auto call = reinterpret_cast<decltype(&cvllm_decode_attention)>(PyCapsule_GetPointer(a[0], nullptr));
+  if (!call) return nullptr;
   at::Tensor out = at::empty({B, HQ, D}, q->options());
+  // all that may throw or set an error comes before the lock is released
+  const void *q_at = q->data_ptr(), *k_at = k->data_ptr(), *v_at = v->data_ptr();
+  void *out_at = out.data_ptr(), *space_at = space.data_ptr();
+  const int32_t *lens_at = lens->data_ptr<int32_t>(), *pt_at = pt->data_ptr<int32_t>(), *bm_at = bm->data_ptr<int32_t>();
+  const size_t space_bytes = static_cast<size_t>(space.numel());
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = reinterpret_cast<decltype(&cvllm_decode_attention)>(PyCapsule_GetPointer(a[0], nullptr))(
-      q->data_ptr(), out.data_ptr(), k->data_ptr(), v->data_ptr(), lens->data_ptr<int32_t>(), pt->data_ptr<int32_t>(),
-      bm->data_ptr<int32_t>(), space.data_ptr(), static_cast<size_t>(space.numel()), static_cast<int>(B), static_cast<int>(HQ),
-      static_cast<int>(HKV), static_cast<int>(D), static_cast<int>(PS), static_cast<int>(NLP), scale, dtype, 0, stream);
+  rc = call(q_at, out_at, k_at, v_at, lens_at, pt_at, bm_at, space_at, space_bytes, static_cast<int>(B), static_cast<int>(HQ),
+            static_cast<int>(HKV), static_cast<int>(D), static_cast<int>(PS), static_cast<int>(NLP), scale, dtype, 0, stream);
   Py_END_ALLOW_THREADS
   if (rc != CVLLM_OK) Py_RETURN_NONE;
   return THPVariable_Wrap(out);
@@ -239,15 +245,21 @@ PyObject* prefill_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   if (max_past > 0x7fffffff) max_past = 0x7fffffff;
   if (max_past < -1) Py_RETURN_NONE;
+  const auto call = reinterpret_cast<decltype(&cvllm_prefill_attention_bounded)>(PyCapsule_GetPointer(a[0], nullptr));
+  if (!call) return nullptr;
   at::Tensor out = at::empty({T, HQ, D}, q->options());
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  // all that may throw or set an error comes before the lock is released
+  const void *q_at = q->data_ptr(), *k_at = k->data_ptr(), *v_at = v->data_ptr(), *kc_at = kc->data_ptr(), *vc_at = vc->data_ptr();
+  void* out_at = out.data_ptr();
+  const int32_t *lens_at = lens->data_ptr<int32_t>(), *pt_at = pt->data_ptr<int32_t>(), *bm_at = bm->data_ptr<int32_t>(),
+                *cu_at = cu->data_ptr<int32_t>();
+  const int64_t q_stride = q->stride(0), k_stride = k->stride(0), v_stride = v->stride(0), out_stride = out.stride(0);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = reinterpret_cast<decltype(&cvllm_prefill_attention_bounded)>(PyCapsule_GetPointer(a[0], nullptr))(
-      q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(), kc->data_ptr(), vc->data_ptr(), lens->data_ptr<int32_t>(),
-      pt->data_ptr<int32_t>(), bm->data_ptr<int32_t>(), cu->data_ptr<int32_t>(), static_cast<int>(B), static_cast<int>(T),
-      static_cast<int>(HQ), static_cast<int>(HKV), static_cast<int>(D), static_cast<int>(PS), static_cast<int>(NLP), rows, q->stride(0),
-      k->stride(0), v->stride(0), out.stride(0), static_cast<int>(max_q), static_cast<int>(max_past), scale, dtype, stream);
+  rc = call(q_at, k_at, v_at, out_at, kc_at, vc_at, lens_at, pt_at, bm_at, cu_at, static_cast<int>(B), static_cast<int>(T),
+            static_cast<int>(HQ), static_cast<int>(HKV), static_cast<int>(D), static_cast<int>(PS), static_cast<int>(NLP), rows, q_stride,
+            k_stride, v_stride, out_stride, static_cast<int>(max_q), static_cast<int>(max_past), scale, dtype, stream);
   Py_END_ALLOW_THREADS
   if (rc != CVLLM_OK) Py_RETURN_NONE;
   return THPVariable_Wrap(out);

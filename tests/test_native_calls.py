@@ -118,3 +118,39 @@ def test_prefill_forms(monkeypatch, form):
         call(pt=pt.long())
     _long_way(monkeypatch)
     assert torch.equal(got, call()) and got.shape == (n, HQ, 128)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("transform", ["vmap", "grad", "jvp", "vmap of lengths"])
+def test_tensors_without_memory_are_refused(transform):
+    """Inside vmap and the transforms of torch.func a tensor is of the exact type and contiguous, but has no address: an exception as
+    for every call that asks for one, and the next call works."""
+    B, HQ, HKV, PS, pages = 2, 8, 2, 128, 1
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q = torch.randn(B, HQ, 128, generator=g, device=DEV, dtype=torch.bfloat16)
+    kc, vc = (torch.randn((B + 1) * HKV * pages * PS, 128, generator=g, device=DEV).to(q.dtype) for _ in range(2))
+    k, v = (torch.randn(B, HKV, 128, generator=g, device=DEV).to(q.dtype) for _ in range(2))
+    pt = torch.randperm((B + 1) * HKV * pages, generator=g, device=DEV).to(torch.int32).view(B + 1, HKV, pages).contiguous()
+    lens = torch.full((B, HKV), 40, dtype=torch.int32, device=DEV)
+    bm, cu = torch.tensor([2, 1], dtype=torch.int32, device=DEV), torch.arange(B + 1, dtype=torch.int32, device=DEV)
+
+    def decode(q, lens=lens):
+        return head_sparse_decode_attention(q, kc, vc, lens, pt, bm, HKV, PS, 0.1)
+
+    def prefill(q, lens=lens):
+        return causal_sparse_varlen_with_cache(q, k, v, kc, vc, seq_lens_bh=lens, global_page_table=pt, batch_mapping=bm,
+                                               cu_seqlens_q=cu, max_seqlen_q=1, max_seqlen_k_cache=40, HKV=HKV, PAGE_SIZE=PS,
+                                               sm_scale=0.1)
+
+    for attend in (decode, prefill):
+        want = attend(q)                        # and the workspace
+        with pytest.raises(RuntimeError, match="Cannot access data pointer"):
+            if transform == "vmap":
+                torch.vmap(attend)(q[None].expand(3, -1, -1, -1).contiguous())
+            elif transform == "grad":
+                torch.func.grad(lambda x: attend(x).float().sum())(q)
+            elif transform == "jvp":
+                torch.func.jvp(attend, (q,), (q,))
+            else:
+                torch.vmap(lambda x: attend(q, x))(lens[None].expand(3, -1, -1).contiguous())
+        assert torch.equal(attend(q), want)
