@@ -2,7 +2,8 @@
 // what such a call costs on the host is what it costs: ctypes takes 4 to 5 us for 20 to 30 arguments and 0.3 us for every
 // tensor's address, and a dozen properties of the tensors 0.2 us each.  Two layers:
 //   * bind(name, address, otherwise): the function of include/cvllm.h at `address` as a callable that takes None, int, float and CUDA
-//     tensors; whatever else comes among the arguments goes to `otherwise` (the ctypes function) unchanged.
+//     tensors; with anything else among the arguments (a number of numpy's, a ctypes array) the call goes to `otherwise` (the ctypes
+//     function), tensors as their addresses.
 //   * decode_attention / prefill_attention: the whole of the two entry points for the plain form of their arguments (ordinary
 //     CUDA tensors of the documented types, shapes and strides).  They return None where anything is out of the ordinary, or
 //     where the library refuses; the caller then goes the long way, which converts, or says what is wrong.
@@ -86,13 +87,42 @@ struct Bound<int(A...)> {
     Py_END_ALLOW_THREADS
     return 1;
   }
+  // a tensor where the ABI takes a pointer -> its address, anything else as it came: 1 and a new reference, or -1
+  template <class T>
+  static int address(PyObject* o, PyObject*& out) {
+    if constexpr (std::is_pointer_v<T>) {
+      if (THPVariable_Check(o)) {
+        T at;
+        if (convert(o, at) != 1) return -1;
+        out = PyLong_FromVoidPtr(const_cast<void*>(static_cast<const void*>(at)));
+        return out ? 1 : -1;
+      }
+    }
+    out = Py_NewRef(o);
+    return 1;
+  }
+  template <size_t... I>
+  static PyObject* long_way(PyObject* otherwise, PyObject* const* args, Py_ssize_t n, std::index_sequence<I...>) {
+    PyObject* list = PyTuple_New(n);
+    if (!list) return nullptr;
+    int state = 1;
+    auto put = [&](Py_ssize_t i, auto convert_one) {
+      PyObject* item = nullptr;
+      if (state == 1 && i < n && (state = convert_one(args[i], item)) == 1) PyTuple_SET_ITEM(list, i, item);
+    };
+    (put(I, address<A>), ...);
+    for (Py_ssize_t i = sizeof...(A); i < n; ++i) put(i, address<int>);
+    PyObject* result = state == 1 ? PyObject_CallObject(otherwise, list) : nullptr;
+    Py_DECREF(list);
+    return result;
+  }
   static PyObject* run(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     int result = 0, state = 0;
     if (n == static_cast<Py_ssize_t>(sizeof...(A)))
       state = call(PyCapsule_GetPointer(PyTuple_GET_ITEM(self, 0), nullptr), args, result, std::index_sequence_for<A...>{});
     if (state < 0) return nullptr;
-    if (state == 0) return PyObject_Vectorcall(PyTuple_GET_ITEM(self, 1), args, n, nullptr);
+    if (state == 0) return long_way(PyTuple_GET_ITEM(self, 1), args, n, std::index_sequence_for<A...>{});
     return PyLong_FromLong(result);
     END_HANDLE_TH_ERRORS
   }

@@ -1,6 +1,7 @@
 """The calls that take tensors (csrc/host/py_call.cpp) against the long way: same results, same refusals."""
 import ctypes
 
+import numpy as np
 import pytest
 import torch
 
@@ -31,6 +32,32 @@ def test_other_arguments_go_to_ctypes():
         L.cvllm_decode_attention(1, 2)
     with pytest.raises(ctypes.ArgumentError):
         L.cvllm_decode_attention(*[None] * 8, 0, "one", 32, 8, 128, 128, 1, 0.1, 0, 0, None)
+
+
+class Placed(torch.Tensor):
+    """Says of itself that it lies on a GPU, at an address."""
+    is_cuda = True
+
+    def data_ptr(self):
+        return 4096
+
+
+@pytest.mark.parametrize("number", [np.int64, np.int32, torch.tensor], ids=["int64", "int32", "tensor"])
+def test_numbers_of_other_libraries_beside_tensors(number):
+    """ctypes takes what has an __index__ or a __float__ where the ABI has a number; beside it the tensors still pass as addresses."""
+    L, t = N.lib(), torch.zeros(1).as_subclass(Placed)
+    scale = np.float32(0.1) if number is not torch.tensor else torch.tensor(0.1)
+    rest = [number(x) for x in (8, 128, 128, 1)]
+    # B = 0: nothing is launched
+    assert L.cvllm_decode_attention(*[t] * 8, number(0), number(0), number(32), *rest, scale, number(0), number(0), None) == 0
+    with pytest.raises(AssertionError, match="CUDA tensors"):
+        L.cvllm_decode_attention(*[t] * 7, torch.zeros(1), 0, number(0), 32, 8, 128, 128, 1, 0.1, 0, 0, None)
+    seen = []
+    bound = L.call.bind("cvllm_decode_attention", 1, lambda *a: seen.append(a) or 5)
+    assert bound(*[t] * 7, None, 0, number(0), 32, 8, 128, 128, 1, 0.1, 0, 0, None) == 5
+    assert seen[0][:8] == (4096,) * 7 + (None,) and seen[0][10:] == (32, 8, 128, 128, 1, 0.1, 0, 0, None)
+    assert bound(t, t) == 5 and seen[1] == (4096, 4096)
+    assert bound(*[0] * 19, t) == 5 and seen[2][19] is t
 
 
 class Named(torch.Tensor):
