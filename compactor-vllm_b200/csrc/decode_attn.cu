@@ -38,6 +38,8 @@
 #include <stdlib.h>
 #include <type_traits>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "mma.cuh"
 #include "tma.cuh"
@@ -49,6 +51,7 @@ constexpr int kDecWarps = 8;      // consumer warps: 8 x 16 keys = one unit
 constexpr int kDecCons = kDecWarps * 32;
 constexpr int kDecThreads = kDecCons + 32;  // + producer warp
 constexpr int kMaxSlots = 6;      // ring slots (one K unit or one V unit each): 6 when G <= 4, else 5
+constexpr int kDecMaxSmem = 224 * 1024;     // 227 KB opt-in limit minus static smem
 constexpr int kSlotBytes = kUnit * 256;     // 32 KB at D = 128, 16-bit (half of it used at D = 64)
 constexpr int kHalfBytes = kUnit * 128;     // one 64-column half of a slot
 
@@ -76,6 +79,7 @@ struct DecodeParams {
   int slots;          // ring depth (<= kMaxSlots)
   int lens_by_slot;   // seq_lens_bh is the cache's [Bmax+1, HKV] table, indexed through batch_mapping
   int mode;           // 0 = normal; 1 = consumers only drain the ring (load ceiling, profiling only)
+  int map_in_smem;    // batch_mapping has a copy in shared memory (decode_smem)
   float scale_log2;
 #ifdef CVLLM_DECODE_TRACE
   unsigned long long* trace;  // profiling build only (tools/trace_decode.py): 8 globaltimer stamps per CTA
@@ -239,7 +243,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   uint64_t* bar_empty = bar_full + kMaxSlots;
   float* s_merge = reinterpret_cast<float*>(bar_empty + kMaxSlots);   // [kDecWarps][G][ROW]
   int32_t* s_prefix = reinterpret_cast<int32_t*>(s_merge + kDecWarps * p.G * ROW);  // [BH + 1]
-  int32_t* s_map = s_prefix + BH + 1;                                 // [B] batch_mapping
+  int32_t* s_map = s_prefix + BH + 1;                                 // [B] batch_mapping, where there is room
   __shared__ int32_t s_warp_tot[NW], s_warp_max[NW];
   __shared__ int s_last;
 
@@ -282,7 +286,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int per = cdiv(BH, kDecThreads);
     const int beg = min(BH, tid * per), end = min(BH, beg + per);
     int local = 0, most = 0;
-    for (int i = tid; i < p.B; i += kDecThreads) s_map[i] = p.batch_mapping[i];   // in flight with the lengths
+    if (p.map_in_smem)
+      for (int i = tid; i < p.B; i += kDecThreads) s_map[i] = p.batch_mapping[i];   // in flight with the lengths
     for (int i = beg; i < end; ++i) {
       const int n = units_of(i);
       local += n;
@@ -369,7 +374,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           const int pg = tok / p.PS;
           const int32_t* pt;
           if constexpr (BIAS) pt = p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head;
-          else pt = p.page_table + ((int64_t)s_map[b] * p.HKV + h) * p.NLP;
+          else pt = p.page_table + ((int64_t)(p.map_in_smem ? s_map[b] : p.batch_mapping[b]) * p.HKV + h) * p.NLP;
           row = pt[pg] * p.PS + (tok - pg * p.PS);
         }
       }
@@ -826,6 +831,19 @@ extern "C" size_t cvllm_decode_attention_workspace_bytes(int B, int HQ, int HKV,
   return decode_counter_bytes(BH) + slots * G * (D + 2) * sizeof(float);
 }
 
+// Shared memory of a launch: the merge rows, the prefix of the heads' units, as many 32 KB slots as fit beside them (6 for G <= 4, else 5;
+// fewer for thousands of heads), and the table of slot numbers where it costs no ring slot.  False: not even two slots fit.
+static bool decode_smem(DecodeParams& p, int D, bool want_map, size_t& bytes) {
+  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)kDecWarps * p.G * (D + 2) * 4 + ((size_t)p.B * p.HKV + 1) * 4;
+  const size_t map = want_map ? (size_t)p.B * 4 : 0;
+  if (fixed + 2 * (size_t)kSlotBytes > (size_t)kDecMaxSmem) return false;
+  p.slots = (int)std::min<size_t>(kMaxSlots, (kDecMaxSmem - fixed) / kSlotBytes);
+  bytes = fixed + (size_t)p.slots * kSlotBytes;
+  p.map_in_smem = want_map && bytes + map <= (size_t)kDecMaxSmem;
+  if (p.map_in_smem) bytes += map;
+  return true;
+}
+
 static int launch_decode_attn(const void* q, void* out, const void* k_cache, const void* v_cache,
                               const int32_t* seq_lens_bh, const int32_t* page_table,
                               const int32_t* batch_mapping, void* workspace, size_t workspace_bytes, int B,
@@ -878,22 +896,16 @@ static int launch_decode_attn(const void* q, void* out, const void* k_cache, con
     if (rc) return rc;
   }
 
-  // ring depth: as many 32 KB slots as fit beside the merge rows (6 for G <= 4, else 5)
-  constexpr int kMaxSmem = 224 * 1024;  // 227 KB opt-in limit minus static smem
-  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)kDecWarps * G * (D + 2) * 4 + (BH + 1 + B) * 4;
-  CVLLM_CHECK_SUPPORTED(fixed + 2 * (size_t)kSlotBytes <= (size_t)kMaxSmem);
-  int slots = (int)(((size_t)kMaxSmem - fixed) / kSlotBytes);
-  if (slots > kMaxSlots) slots = kMaxSlots;
+  size_t smem = 0;
+  CVLLM_CHECK_SUPPORTED(decode_smem(p, D, true, smem));
   {
     const int cap = test_options().decode_slots.load(std::memory_order_relaxed);  // profiling knob
-    if (cap >= 2 && cap < slots) slots = cap;
+    if (cap >= 2 && cap < p.slots) p.slots = cap;
   }
-  p.slots = slots;
-  const size_t smem = fixed + (size_t)slots * kSlotBytes;
   // raise the dynamic-smem cap once per (kernel, device)
   static std::atomic<uint64_t> attr_bf{0}, attr_h{0};
-  if (bf16) CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128>, kMaxSmem, attr_bf));
-  else CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<false, 128>, kMaxSmem, attr_h));
+  if (bf16) CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128>, kDecMaxSmem, attr_bf));
+  else CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<false, 128>, kDecMaxSmem, attr_h));
   if (bf16) {
     CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 128>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
   } else {
@@ -941,21 +953,17 @@ int cvllm_launch_bias_decode(const void* q, const void* k_cache, const void* v_c
     rc = make_tmap_16b(&tm_v, v_cache, 2, dims, strides, box, true);
     if (rc) return rc;
   }
-  constexpr int kMaxSmem = 224 * 1024;
-  const int BH = B * G, C = sm_count();
-  const size_t fixed = 1024 + 2 * kMaxSlots * 8 + (size_t)kDecWarps * p.G * (D + 2) * 4 + ((size_t)BH + 1 + B) * 4;
-  CVLLM_CHECK_SUPPORTED(fixed + 2 * (size_t)kSlotBytes <= (size_t)kMaxSmem);
-  p.slots = (int)(((size_t)kMaxSmem - fixed) / kSlotBytes);
-  if (p.slots > kMaxSlots) p.slots = kMaxSlots;
-  const size_t smem = fixed + (size_t)p.slots * kSlotBytes;
+  const int C = sm_count();
+  size_t smem = 0;
+  CVLLM_CHECK_SUPPORTED(decode_smem(p, D, false, smem));   // (the producer reads the slot numbers from memory)
   static std::atomic<uint64_t> attr_128{0}, attr_64{0};
   if (D == 128) {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128, true>, kMaxSmem, attr_128));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 128, true>, kDecMaxSmem, attr_128));
     CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 128, true>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
     CVLLM_CHECK_LAUNCH();
     CVLLM_CHECK_CUDA(launch_behind(bias_decode_fold_kernel<128>, dim3(B * H), dim3(256), 0, st, p, C));
   } else {
-    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 64, true>, kMaxSmem, attr_64));
+    CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)decode_attn_kernel<true, 64, true>, kDecMaxSmem, attr_64));
     CVLLM_CHECK_CUDA(launch_behind(decode_attn_kernel<true, 64, true>, dim3(C), dim3(kDecThreads), smem, st, tm_k, tm_v, p));
     CVLLM_CHECK_LAUNCH();
     CVLLM_CHECK_CUDA(launch_behind(bias_decode_fold_kernel<64>, dim3(B * H), dim3(256), 0, st, p, C));

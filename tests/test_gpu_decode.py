@@ -163,3 +163,27 @@ def test_decode_whole_and_cut_heads(HQ, HKV, PS, B, units):
     q = torch.randn((B, HQ, D), generator=g).to(dtype).to(DEV)
     out = _check(q, kc, vc, lens.to(torch.int32).to(DEV), pt, bm, HKV, PS, dtype)
     assert (out.cpu()[(lens == 0).repeat_interleave(HQ // HKV, dim=1)] == 0).all()
+
+
+@pytest.mark.parametrize("B,HQ,HKV", [
+    (4499, 32, 8), (31319, 8, 1),      # the most sequences that the heads' prefix leaves two ring slots for
+    (1600, 4, 1), (1900, 4, 1),        # the table of slot numbers beside six ring slots, and the first size where it would cost one
+    (3700, 4, 1)])                     # five slots without it
+def test_decode_many_sequences(B, HQ, HKV):
+    dtype, D, PS, pages = torch.bfloat16, 128, 32, 64
+    g = torch.Generator(device=DEV).manual_seed(B)
+    kc, vc = (torch.randn(pages * PS, D, generator=g, device=DEV).to(dtype) for _ in range(2))
+    pt = torch.randint(0, pages, (B + 1, HKV, 2), generator=g, device=DEV, dtype=torch.int32)
+    lens = torch.randint(0, 2 * PS + 1, (B, HKV), generator=g, device=DEV, dtype=torch.int32)
+    bm = (torch.randperm(B, generator=g, device=DEV) + 1).to(torch.int32)
+    q = torch.randn(B, HQ, D, generator=g, device=DEV).to(dtype)
+    out = head_sparse_decode_attention(q, kc, vc, lens, pt, bm, HKV, PS, 0.1)
+    for b0 in range(0, B, 1024):
+        s = slice(b0, b0 + 1024)
+        at = (pt[bm[s].long()].long()[..., None] * PS + torch.arange(PS, device=DEV)).flatten(-2)       # [b, HKV, 2 PS]
+        k, v = kc.float()[at], vc.float()[at]
+        x = torch.einsum("bhgd,bhnd->bhgn", q[s].float().view(-1, HKV, HQ // HKV, D), k) * 0.1
+        there = torch.arange(2 * PS, device=DEV) < lens[s][:, :, None]
+        x = x.masked_fill(~there[:, :, None], -torch.inf).softmax(-1).nan_to_num(0.0)
+        want = torch.einsum("bhgn,bhnd->bhgd", x, v).flatten(1, 2)
+        assert (out[s].float() - want).abs().max().item() <= TOL[dtype]
