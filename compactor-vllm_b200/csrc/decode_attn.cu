@@ -5,7 +5,8 @@
 //   * work = 128-token units of every (b, kv-head); the flattened unit list
 //     is cut into gridDim.x equal ranges (stream-K style), so ragged per-head
 //     lengths after compression are balanced exactly — the reference gives
-//     every head the same KEY_SPLIT regardless of its length (:303-306)
+//     every head the same KEY_SPLIT regardless of its length (:303-306).  Ranges
+//     over short heads end at heads' ends instead (heads_whole)
 //   * warp 8 is the TMA producer: it resolves (head, page) for 32 units at a
 //     time (one lane per unit/page piece), then streams K and V units through
 //     a ring of kSlots x 32 KB shared-memory slots (cp.async.bulk.tensor, 128B
@@ -22,8 +23,7 @@
 //     layout, O^T += V^T.P^T
 //   * partial (m, l, O) of a range that does not cover its whole head goes to
 //     a scratch slot; the CTA that completes a head merges (atomic ticket),
-//     every warp folding a strided subset of the slots with independent loads.
-//     Ranges of short heads end at heads' ends (heads_whole), and need none of it
+//     every warp folding every eighth of the states with independent loads
 //   * the launch is scheduled beside the kernel in front of it where that one lets it (the norm and store of a step, another
 //     decode step): barriers and descriptors are ready when it ends.  One sequence of 8192 rows 17.9 -> 15.5 us a call back to
 //     back, 8 x 384 rows 12.3 -> 10.1, a biased step of 8 x 4096 rows, whose fold is scheduled beside it, 40.7 -> 37.3
@@ -55,12 +55,13 @@ constexpr int kDecMaxSmem = 224 * 1024;     // 227 KB opt-in limit minus static 
 constexpr int kSlotBytes = kUnit * 256;     // 32 KB at D = 128, 16-bit (half of it used at D = 64)
 constexpr int kHalfBytes = kUnit * 128;     // one 64-column half of a slot
 
-// Whether the ranges of the C CTAs end at heads' ends (`most` units in the longest head, U in all).  A cut costs some 4.5 us at
-// the end (a partial state through memory, a ticket, the fold); a head left whole costs what its CTA has more than the even
-// share, where a unit takes 0.7 us on a chip that has few and 1.4 on a full one.  Measured in a graph, cut / whole, us, 32 / 8 heads,
-// longest head 1.5 times the mean: 8 x 384 14.8 / 10.5, 8 x 600 15.1 / 13.1, 16 x 600 21.0 / 17.9, 32 x 200 21.2 / 17.2, 64 x 400
-// 34.7 / 31.5, but 24 x 650 26.4 / 27.9, 48 x 600 35.6 / 37.4, 32 x 800 32.5 / 34.8 (shares above 6 units), 1 x 500 10.2 / 10.8,
-// 4 x 1000 13.8 / 18.4 (long beside the share).
+// Whether the ranges of the C CTAs end at heads' ends (`most` units in the longest head, U in all).  A cut costs 3 to 4 us at the
+// end where units outnumber the CTAs, 1 where they don't (a partial state through memory, a ticket, the fold); a head left whole
+// costs what its CTA has more than the even share, where a unit takes 0.7 us on a chip that has few and 1.4 on a full one.
+// Measured in a graph, cut / whole, us, 32 / 8 heads, longest head up to 1.4 times the rows given: 8 x 384 13.1 / 9.0, 8 x 600
+// 14.0 / 10.8, 16 x 600 15.2 / 12.5, 32 x 200 15.7 / 11.9, 64 x 400 32.3 / 29.7, 1 x 300 9.0 / 7.8, 4 x 300 9.1 / 8.1, but 24 x 650
+// 19.4 / 19.6, 48 x 600 33.4 / 34.9, 32 x 800 29.8 / 32.7 (shares above 6 units), 1 x 500 8.9 / 9.5, 4 x 500 9.2 / 10.0, 4 x 1000
+// 12.2 / 14.5 (long beside the share).
 __device__ __forceinline__ bool heads_whole(int most, int64_t U, int C) {
   if (U > 6 * (int64_t)C) return most <= 5;
   return most <= 8 && (int64_t)C * (most - (U >= C ? 6 : 4)) <= U;
@@ -164,11 +165,29 @@ __device__ __forceinline__ float bias_inv(const BiasDecodeParams& p, int hq, flo
 
 __device__ __forceinline__ void cons_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kDecCons) : "memory"); }
 
-// The partial states of a cut head, slots c_first .. c_last, into s_merge's rows: each consumer warp folds the slots c_first + warp,
-// + 8, ... into a running (m, l, O), the loads of AHEAD slots in flight together; lane owns d = 2*lane, 2*lane+1, 64 + 2*lane,
-// 65 + 2*lane.  A function of its own: its registers beside the streaming loop's would make that loop spill.
+// (a division of 64 bits takes 0.1 us, and some stand in front of all else)
+__device__ __forceinline__ int quotient(int64_t x, int d) {   // x >= 0, d > 0
+  return x >> 32 ? (int)(x / d) : (int)((uint32_t)x / (uint32_t)d);
+}
+// Where the partial states of a cut head lie: state k = 0 .. n - 1 in the slot of CTA cta(k).  With at least as many units as CTAs every
+// CTA from the head's first to its last has one; with fewer a unit is a state, and most CTAs between have none.  Going through
+// those too, with the two divisions that tell, was most of a fold.  One sequence of 700 rows, a head with a group of eight:
+// 19.0 -> 10 us back to back, a biased step over 1500 rows of it 24.7 -> 12.
+struct HeadStates {
+  int h_beg, U, C, c_first, n;
+  __device__ __forceinline__ HeadStates(int h_beg, int h_end, int U, int C) : h_beg(h_beg), U(U), C(C) {
+    c_first = holder(h_beg);
+    n = U < C ? h_end - h_beg : holder(h_end - 1) - c_first + 1;
+  }
+  __device__ __forceinline__ int holder(int u) const { return quotient((int64_t)(u + 1) * C - 1, U); }   // the CTA of unit u
+  __device__ __forceinline__ int cta(int k) const { return U < C ? holder(h_beg + k) : c_first + k; }
+};
+
+// The partial states of a cut head (units h_beg .. h_end - 1) into s_merge's rows: each consumer warp folds every eighth of them into a
+// running (m, l, O), the loads of AHEAD states in flight together; lane owns d = 2*lane, 2*lane+1, 64 + 2*lane, 65 + 2*lane.
+// A function of its own: its registers beside the streaming loop's would make that loop spill.
 template <int NQ, int AHEAD>
-__device__ __noinline__ void fold_slots(const float* scratch, float* s_merge, int head, int G, int c_first, int c_last, int U, int C) {
+__device__ __noinline__ void fold_slots(const float* scratch, float* s_merge, int head, int G, int h_beg, int h_end, int U, int C) {
   constexpr int ROW = 128 + 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* mw = s_merge + warp * G * ROW;
@@ -179,14 +198,14 @@ __device__ __noinline__ void fold_slots(const float* scratch, float* s_merge, in
     M[q] = -INFINITY; ls[q] = 0.f;
     oa[q] = make_float2(0.f, 0.f); ob[q] = make_float2(0.f, 0.f);
   }
-  for (int cc = c_first + warp; cc <= c_last; cc += AHEAD * kDecWarps) {
+  const HeadStates states(h_beg, h_end, U, C);
+  for (int k = warp; k < states.n; k += AHEAD * kDecWarps) {
     float2 va[AHEAD][NQ], vb[AHEAD][NQ], ml[AHEAD][NQ];
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
-      const int ci = cc + i * kDecWarps;
-      // CTAs with an empty unit range (U < C) never wrote their slot
-      const bool used = ci <= c_last && (int)((int64_t)U * ci / C) < (int)((int64_t)U * (ci + 1) / C);
-      const float* sl = scratch + (int64_t)(head + ci) * G * ROW;
+      const int ki = k + i * kDecWarps;
+      const bool used = ki < states.n;
+      const float* sl = scratch + (int64_t)(head + states.cta(ki)) * G * ROW;
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {
         ml[i][q] = make_float2(-INFINITY, 0.f);
@@ -417,8 +436,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   // =========================== consumer warps ===============================
   const int r = lane >> 2, j = lane & 3;
   // P as the sum of two 16-bit numbers (see the top): biased attention, and heads left whole.  Their one running maximum
-  // leaves fewer keys with the exact probability 1 than the cut ones' many, 2 % more error at 400 keys a head; so, it is
-  // a third less.
+  // leaves fewer keys with the exact probability 1 than the cut ones' many, 2 % more error at 384 keys a head; so, it is 16 %
+  // less in fp16 (2.07e-4 for 2.46e-4 of the result, twelve seeds) and 17 % in bf16 (1.66e-3 for 2.00e-3).
   const bool low_parts = G <= 4 && (BIAS || uncut);
   const uint32_t ring_u32 = smem_u32(ring);
   int c_slot = 0;        // ring position of the next item to consume
@@ -709,10 +728,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       cons_bar();
       if (tid == 0) DEC_TRACE(6);
       if (s_last) {
-        const int c_first = (int)((((int64_t)h_beg + 1) * C - 1) / U);
-        const int c_last = (int)(((int64_t)h_end * C - 1) / U);
-        if (G <= 4) fold_slots<4, 3>(p.scratch, s_merge, head, G, c_first, c_last, U, C);
-        else fold_slots<8, 1>(p.scratch, s_merge, head, G, c_first, c_last, U, C);
+        if (G <= 4) fold_slots<4, 3>(p.scratch, s_merge, head, G, h_beg, h_end, U, C);
+        else fold_slots<8, 1>(p.scratch, s_merge, head, G, h_beg, h_end, U, C);
         cons_bar();
         if (tid == 0) DEC_TRACE(7);
         fold_warps(write_out);
@@ -756,25 +773,21 @@ __global__ void __launch_bounds__(256) bias_decode_fold_kernel(const BiasDecodeP
   const int n = UnitList(p, b).count;
   pdl_wait();   // for the states (what is read above was there when the kernel in front let this one start)
   if (n == 0) return;
-  const int64_t U = (int64_t)all * p.HKV;
+  const int U = all * p.HKV, h_beg = before * p.HKV + h * n;
   if (heads_whole(__reduce_max_sync(0xffffffffu, most), U, C)) return;
-  const int64_t h_beg = (int64_t)before * p.HKV + (int64_t)h * n, h_end = h_beg + n;
-  const int c_first = (int)(((h_beg + 1) * C - 1) / U), c_last = (int)((h_end * C - 1) / U);
-  if (c_first == c_last) return;   // one CTA had the whole head and has written it
-  auto used = [&](int c) { return U * c / C < U * (c + 1) / C; };   // CTAs without units wrote nothing
-  auto row = [&](int c) { return p.scratch + ((int64_t)(head + c) * G + q) * ROW; };
+  const HeadStates states(h_beg, h_beg + n, U, C);
+  if (states.n == 1) return;   // one CTA had the whole head and has written it
+  auto row = [&](int k) { return p.scratch + ((int64_t)(head + states.cta(k)) * G + q) * ROW; };
   float M = -INFINITY;
-  for (int c = c_first + lane; c <= c_last; c += 32)
-    if (used(c)) M = fmaxf(M, __ldcg(row(c) + D));
+  for (int k = lane; k < states.n; k += 32) M = fmaxf(M, __ldcg(row(k) + D));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   float acc[PER], l = 0.f;
 #pragma unroll
   for (int i = 0; i < PER; ++i) acc[i] = 0.f;
 #pragma unroll 4
-  for (int c = c_first + warp; c <= c_last; c += 8) {
-    if (!used(c)) continue;
-    const float* x = row(c);
+  for (int k = warp; k < states.n; k += 8) {
+    const float* x = row(k);
     const float w = ex2(__ldcg(x + D) - M);
     l = fmaf(__ldcg(x + D + 1), w, l);
 #pragma unroll

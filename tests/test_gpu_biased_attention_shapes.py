@@ -237,6 +237,19 @@ def test_decoding_with_kept_tokens(D, page, window, keep, chunk):
     assert err(got) < 2.5e-3 and err(got) < 1.05 * err(decode(m, q, 1, KEPT)) + 1e-6
 
 
+@pytest.mark.parametrize("H,G,D", [(8, 1, 128), (16, 2, 64)])
+@pytest.mark.parametrize("units", [9, 40, 68, 69, 70, 142, 143, 144, 160])
+def test_decoding_cut_heads(H, G, D, units):
+    """A long sequence beside three short ones, (units + 5) G units in all: fewer than CTAs (148), as many, more."""
+    spans = [(0, 1), (128 * units - 1, 1), (127, 1), (300, 1), (700, 1)]
+    m, q, keys = make(H, G, D, 128, spans, units, **options(1, H, 0, True, "zero", 0, 0, 0))
+    want = formula(m, q, keys, spans)
+    want[4] = 0
+    got = decode(m, q, spans=spans)
+    assert torch.isfinite(got).all() and (got[4] == 0).all()
+    assert ((got - want).norm(dim=1) <= 2.5e-3 * want.norm(dim=1)).all()
+
+
 def test_decode_kernel_does_not_depend_on_earlier_steps():
     """What a step runs on follows from the step: a step on three key splits gives the same bits before and after a step that
     left a large workspace behind, and those are not the streaming kernel's."""

@@ -150,10 +150,11 @@ def test_decode_step_matches_store_then_attend_with_reserved_rows():
 
 
 @pytest.mark.parametrize("HQ,HKV,PS", [(32, 8, 128), (8, 1, 64)])
-@pytest.mark.parametrize("B,units", [(1, 4), (1, 5), (2, 8), (20, 6), (40, 7), (40, 8), (40, 9), (130, 5), (130, 6)])
+@pytest.mark.parametrize("B,units", [(1, 4), (1, 5), (2, 8), (20, 6), (40, 7), (40, 8), (40, 9), (130, 5), (130, 6),
+                                     (1, 20), (1, 147), (1, 148), (1, 149), (3, 49)])
 def test_decode_whole_and_cut_heads(HQ, HKV, PS, B, units):
     """Both sides of the rule that leaves short heads whole (longest head 4, 5, 6, 8 units of 128 rows beside shares of under
-    one, up to six and more than six units per CTA), with empty heads, one-row heads and NaN behind every head's end."""
+    one, up to six and more than six units per CTA), and cut heads over fewer, as many and more units than CTAs, with empty heads, one-row heads and NaN behind every head's end."""
     dtype, D = torch.bfloat16, 128
     g = torch.Generator().manual_seed(100 * B + units)
     lens = torch.randint(1, units * 128 + 1, (B, HKV), generator=g)
