@@ -23,7 +23,7 @@
 //   warp 11       idle (registers are handed out per 4-warp group: the third group gives its
 //                 registers to the softmax groups with setmaxnreg, 56 vs 224 per thread).
 //
-// A CTA that nears the end of its query tile takes over the next CTA of the grid that has not started (cluster launch
+// Where tiles are more than a wave, a CTA that nears the end of its tile takes over the next CTA of the grid that has not started (cluster launch
 // control) and goes on with its tile: barriers, TMEM and the K / V ring stay as they are, the next Q, K and V are loaded beside the
 // last PV, and its first S is made while the softmax groups still write the tile before out.  A launch per tile had 3 us each of
 // set-up, first loads and drain.  The order of the tiles is the grid's, as it was.
@@ -35,6 +35,7 @@
 //
 // TMEM (512 columns): S0 [0,128)  S1 [128,256)  O0 [256,384)  O1 [384,512).
 #include <stdlib.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tile_order.cuh"
@@ -129,7 +130,8 @@ __device__ long long g_p2_trace[8][256];
 #define P2_TRACE(rowi, jj) do { } while (0)
 #endif
 
-template <bool BF16, bool BY_TILE>
+// TAKE: CTAs go on with other tiles
+template <bool BF16, bool BY_TILE, bool TAKE>
 __global__ void __launch_bounds__(p2::kThreads, 1)
 prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kc,
@@ -218,7 +220,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (lane == 0) {
       int slot = 0;
       uint32_t ph = 0;
-      for (int k = 0; k == 0 || next_item(k, 1u); ++k) {
+      for (int k = 0; k == 0 || (TAKE && next_item(k, 1u)); ++k) {
         const int hkv = it.hq0 / p.G, n_pre = (it.Lc + kBN - 1) / kBN, n_loads = 2 * (n_pre + it.qt + 1);
         mbar_wait(&sm.q_empty, (k & 1) ^ 1);
         mbar_expect_tx(&sm.q_full, 2 * kTileBytes);
@@ -363,7 +365,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tc_fence_after();
     };
 
-    for (int k = 0; k == 0 || next_item(k, 0xffffffffu); ++k) {
+    for (int k = 0; k == 0 || (TAKE && next_item(k, 0xffffffffu)); ++k) {
       n_pre = (it.Lc + kBN - 1) / kBN;
       n_tiles = n_pre + it.qt + 1;
       mbar_wait(&sm.q_full, k & 1);
@@ -396,7 +398,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t o_tmem = tmem + 256 + t * kHD + lane_base;
     int done = 0;                   // KV tiles before this query tile
 
-    for (int k = 0; k == 0 || next_item(k, 0xffffffffu); ++k) {
+    for (int k = 0; k == 0 || (TAKE && next_item(k, 0xffffffffu)); ++k) {
       const int n_pre = (it.Lc + kBN - 1) / kBN, n_tiles = n_pre + it.qt + 1, Lc = it.Lc;
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < n_tiles; ++j) {
@@ -551,7 +553,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));  // warps 10, 11
-    if (warp == 10 && lane == 0) {
+    if (TAKE && warp == 10 && lane == 0) {
       // ======================== the next query tile ========================
       uint32_t answers = 0;
       for (int k = 1;; ++k) {
@@ -602,6 +604,10 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
   p.rescale_threshold = rescale_threshold;
   const size_t smem = sizeof(Prefill2Smem) + 1024;
   const dim3 grid((max_seqlen_q + p2::kBM - 1) / p2::kBM, HQ / 2, B);
+  // Where there is little more than a wave of tiles a CTA would take over one that soon has an SM of its own, the sooner the more CTAs
+  // lie past their sequence's end.  Left to the launch / taken over, us, back to back: 5 + 900 + 77 tokens (160 tiles, 32 / 8 heads)
+  // 19.1 / 20.5, 1250 (160) 21.5 / 22.3, but 700 + 100 + 650 (208) 22.1 / 20.9, 16 x 300 with 8 / 1 heads (192) 19.0 / 17.0.
+  const bool take = 4 * ctas_with_work(grid, N, p2::kBM) > 5 * (int64_t)sm_count();
   const bool by_tile = order_by_tile(grid, N, p2::kBM) && grid.x <= 65535 && past_is_short(max_past, max_seqlen_q);
   auto launch = [&](auto kernel, std::atomic<uint64_t>& attr) -> int {
     CVLLM_CHECK_CUDA(ensure_max_dyn_smem((const void*)kernel, (int)smem, attr));
@@ -609,10 +615,17 @@ int cvllm_launch_prefill2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, cons
                                    tm_kc, tm_vc, p));
     return CVLLM_OK;
   };
-  static std::atomic<uint64_t> attr[4] = {{0}, {0}, {0}, {0}};
-  int rc;
-  if (bf16) rc = by_tile ? launch(prefill_attn2_kernel<true, true>, attr[0]) : launch(prefill_attn2_kernel<true, false>, attr[1]);
-  else rc = by_tile ? launch(prefill_attn2_kernel<false, true>, attr[2]) : launch(prefill_attn2_kernel<false, false>, attr[3]);
+  static std::atomic<uint64_t> attr[2][2][2] = {};
+  auto choose = [&](auto is_bf16, auto tiles, auto takes) -> int {
+    return launch(prefill_attn2_kernel<is_bf16, tiles, takes>, attr[is_bf16][tiles][takes]);
+  };
+  auto with_take = [&](auto is_bf16, auto tiles) {
+    return take ? choose(is_bf16, tiles, std::true_type{}) : choose(is_bf16, tiles, std::false_type{});
+  };
+  auto with_order = [&](auto is_bf16) {
+    return by_tile ? with_take(is_bf16, std::true_type{}) : with_take(is_bf16, std::false_type{});
+  };
+  const int rc = bf16 ? with_order(std::true_type{}) : with_order(std::false_type{});
   if (rc) return rc;
   CVLLM_CHECK_LAUNCH();
   return CVLLM_OK;

@@ -27,12 +27,16 @@
 
 namespace cvllm {
 
-// Launches of one wave start all their tiles at once: no order to choose, and no past to read first.  Tiles of shorter
-// sequences that lie past their end cost nothing, so the CTAs that count are those of `tokens` new tokens in all: at most
-// one partial tile per sequence more than whole ones.
-inline bool order_by_tile(dim3 grid, int tokens, int tile_rows) {
+// CTAs of a launch that have a tile, at most.  Tiles of shorter sequences that lie past their end cost nothing: those of `tokens` new
+// tokens in all are one partial tile per sequence more than whole ones.
+inline int64_t ctas_with_work(dim3 grid, int tokens, int tile_rows) {
   const int64_t padded = (int64_t)grid.x * grid.y * grid.z;
-  const int64_t live = std::min(padded, ((int64_t)tokens / tile_rows + grid.z) * grid.y);
+  return std::min(padded, ((int64_t)tokens / tile_rows + grid.z) * grid.y);
+}
+
+// Launches of one wave start all their tiles at once: no order to choose, and no past to read first.
+inline bool order_by_tile(dim3 grid, int tokens, int tile_rows) {
+  const int64_t live = ctas_with_work(grid, tokens, tile_rows);
   return live > sm_count() && live <= 12 * (int64_t)sm_count();
 }
 
