@@ -189,7 +189,7 @@ __device__ __forceinline__ void unit_of(int u, int& m, int& mt, int& nt) {
 
 template <int D>
 __global__ void __launch_bounds__(kPrepThreads, 2) delta_rows_kernel(const DeltaChunkArgs a) {
-  pdl_wait();      // each of the three kernels is scheduled beside the one in front
+  pdl_wait();      // each of the three kernels may be scheduled beside the one in front
   pdl_trigger();
   extern __shared__ unsigned char smem_raw[];
   const int grp = blockIdx.y;
@@ -1193,8 +1193,17 @@ int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) 
   for (int w = 0; w < p.windows; ++w) {
     a.window = w * (p.per_seq > 0 ? p.per_seq : p.slots);
     if (w > 0) std::swap(a.carry_in, a.carry_out);
-    CVLLM_CHECK_CUDA(launch_behind(delta_rows_kernel<D>, dim3(p.slots, a.G), dim3(kPrepThreads), smem_r, st, a));
-    CVLLM_CHECK_CUDA(launch_behind(delta_coef_kernel<T, D>, dim3(p.slots, a.H), dim3(kPrepThreads), smem_k, st, a));
+    // Each beside the end of the one in front, for heads of 64.  With heads of 128 the next kernel's CTAs then come two to the SMs that are
+    // free first, where one each is faster: 300 + 200 tokens, 16 / 8 heads, 68.4 us for 63.3 one behind the other, 400 + 100 73.5 for
+    // 68.5, 400 with 32 / 16 93.3 for 89.9, 2000 183.2 for 180.6; heads of 64: 600 tokens 66.6 for 67.7, 2000 150.0 for 151.9.
+    constexpr bool kBehind = D == 64;
+    if constexpr (kBehind) {
+      CVLLM_CHECK_CUDA(launch_behind(delta_rows_kernel<D>, dim3(p.slots, a.G), dim3(kPrepThreads), smem_r, st, a));
+      CVLLM_CHECK_CUDA(launch_behind(delta_coef_kernel<T, D>, dim3(p.slots, a.H), dim3(kPrepThreads), smem_k, st, a));
+    } else {
+      delta_rows_kernel<D><<<dim3(p.slots, a.G), kPrepThreads, smem_r, st>>>(a);
+      delta_coef_kernel<T, D><<<dim3(p.slots, a.H), kPrepThreads, smem_k, st>>>(a);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.H * VT, B);
     cfg.blockDim = dim3(512);
@@ -1202,7 +1211,7 @@ int launch_chunks(DeltaChunkArgs a, const ChunkPlan& p, int B, cudaStream_t st) 
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = kBehind;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = VT;
     attr[1].val.clusterDim.y = 1;
