@@ -120,7 +120,7 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
 }
 
-#ifdef CVLLM_PREFILL_TRACE  // profiling build only (tools/trace_prefill.py): clock64 stamps of CTA (0,0,0), first 256 KV tiles
+#ifdef CVLLM_PREFILL_TRACE  // profiling build only (tools/trace_prefill.py): clock64 stamps of CTA (0,0,0), its first 256 KV tiles
 __device__ long long g_p2_trace[8][256];
 #define P2_TRACE(rowi, jj)                                                                              \
   do {                                                                                                  \
@@ -318,7 +318,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const uint32_t par = (done + j) & 1;
 #if CVLLM_PREFILL_P_SPLIT > 0
       mbar_wait(&sm.p_half[t], par);
-      P2_TRACE(2 * t, j);
+      P2_TRACE(2 * t, done + j);
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 2 * kPSplit; ++kk)
@@ -330,7 +330,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         umma_ts_warp(o_tmem, p_tmem + kk * 8, desc_at(v_desc, kk * 2048), idesc_pv, 1u);
 #else
       mbar_wait(&sm.p_full[t], par);
-      P2_TRACE(2 * t, j);
+      P2_TRACE(2 * t, done + j);
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < kBN / 16; ++kk)
@@ -380,10 +380,10 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           wait_k();
           issue_qk(0, j + 1);
         }
-        P2_TRACE(1, j);
+        P2_TRACE(1, done + j);
         issue_pv(1, j);
         if (more) issue_qk(1, j + 1);
-        P2_TRACE(3, j);
+        P2_TRACE(3, done + j);
       }
       done += n_tiles;
     }
@@ -403,13 +403,13 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < n_tiles; ++j) {
         mbar_wait(&sm.s_full[t], (done + j) & 1);
-        if (quad == 0) P2_TRACE(4 + 2 * t, j);
+        if (quad == 0) P2_TRACE(4 + 2 * t, done + j);
         tc_fence_after();
 #ifdef CVLLM_PROBE_NO_SOFTMAX  // timing probe only (wrong results): the issuer / TMA side alone — 6.4 ms at 32K
         tc_fence_before();
         mbar_arrive(&sm.p_half[t]);
         mbar_arrive(&sm.p_full[t]);
-        if (quad == 0) P2_TRACE(5 + 2 * t, j);
+        if (quad == 0) P2_TRACE(5 + 2 * t, done + j);
         continue;
 #endif
         float s[kBN];
@@ -522,7 +522,7 @@ prefill_attn2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(&sm.p_full[t]);
-        if (quad == 0) P2_TRACE(5 + 2 * t, j);
+        if (quad == 0) P2_TRACE(5 + 2 * t, done + j);
       }
 
       // ---- epilogue: O / l -> out ----

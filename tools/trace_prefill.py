@@ -1,5 +1,5 @@
 """Hand-off latencies of prefill_attn2_kernel from in-kernel clock64 stamps (CTA (0,0,0) = the heaviest query tile of
-head pair 0; first 256 KV tiles).  Needs a library built with -DCVLLM_PREFILL_TRACE (tools/build_variant.sh), selected
+head pair 0 and those that it goes on with; its first 256 KV tiles, which of 32768 tokens are the first query tile's).  Needs a library built with -DCVLLM_PREFILL_TRACE (tools/build_variant.sh), selected
 with CVLLM_LIB.  Rows: 0 issuer woke on p_full0, 1 issuer done issuing PV0(j) + S0(j+1), 2 woke on p_full1, 3 done
 issuing PV1(j) + S1(j+1), 4 / 6 softmax group 0 / 1 woke on s_full(j), 5 / 7 it arrived on p_full(j)."""
 import ctypes as C
