@@ -86,6 +86,8 @@ _SIGNATURES = {
     "cvllm_snapkv_scores_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
     "cvllm_snapkv_scores": (_i, [_p, _p, _i64, _i64, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _i,
                                  _i, _p, _i, _p, _sz, _p]),
+    "cvllm_snapkv_scores_bounded": (_i, [_p, _p, _i64, _i64, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i,
+                                 _i, _p, _i, _p, _sz, _p]),
     "cvllm_selftest_tile_order": (_i, [_p, _i, _i, _i, _i, _i, _i, _p, C.POINTER(_i), _p]),
     "cvllm_selftest_snap_split": (_i, [_i, _i, _i, _i]),
     "cvllm_selftest_umma": (_i, [_p, _p, _p, _i, _u32, _u32, _i, _p]),

@@ -70,8 +70,8 @@ def query_aware_key_scores(
     L = N.lib()
     ws_bytes = N.sized(dev.index, "cvllm_snapkv_scores_workspace_bytes", B, N_k, Hq, Hk, w)
     ws = N.workspace(dev, ws_bytes, "snapkv")
-    rc = L.cvllm_snapkv_scores(
-        q, k, q.stride(0), k.stride(0), cu_q, cu_k, w, B, N_k, Hq, Hk,
+    rc = L.cvllm_snapkv_scores_bounded(
+        q, k, q.stride(0), k.stride(0), cu_q, cu_k, w, B, N_q, N_k, Hq, Hk,
         D, N_k, float(sm_scale), KPOOL, int(pool_segment), out, N.dtype_code(q.dtype),
         ws, ws.numel(), N.stream(dev),
     )

@@ -133,8 +133,9 @@ struct Bound<int(A...)> {
   X(cvllm_prefill_attention_bounded) X(cvllm_rope_qknorm_store) X(cvllm_row_norm_rope_store)                                  \
   X(cvllm_bias_attn_varlen_dist) X(cvllm_bias_attn_decode_stream) X(cvllm_bias_attn_decode_dist)                              \
   X(cvllm_leverage_scores) X(cvllm_leverage_scores_from_sketch) X(cvllm_chunk_attn_scores) X(cvllm_snapkv_scores)             \
-  X(cvllm_select_store_topk_bounded) X(cvllm_causal_conv) X(cvllm_causal_conv_mode) X(cvllm_conv_state_update)                \
-  X(cvllm_delta_rule) X(cvllm_delta_rule_chunks) X(cvllm_rmsnorm) X(cvllm_residual_norm) X(cvllm_gated_act)
+  X(cvllm_snapkv_scores_bounded) X(cvllm_select_store_topk_bounded) X(cvllm_causal_conv) X(cvllm_causal_conv_mode)            \
+  X(cvllm_conv_state_update) X(cvllm_delta_rule) X(cvllm_delta_rule_chunks) X(cvllm_rmsnorm) X(cvllm_residual_norm)           \
+  X(cvllm_gated_act)
 
 PyMethodDef kBound[] = {
 #define X(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&Bound<decltype(name)>::run)), METH_FASTCALL, nullptr},

@@ -328,7 +328,7 @@ int cvllm_launch_chunk_scores_umma(const void* q, const void* k, int64_t q_strid
 
 size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV);
 int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
-                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nk, int HQ, int HKV,
+                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nq, int Nk, int HQ, int HKV,
                            int max_seqlen_k, float scale_log2, int kpool, int pool_segment, float* out, float* stats,
                            bool bf16, cudaStream_t st);
 
@@ -415,9 +415,18 @@ extern "C" int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_strid
                                    int Nk, int HQ, int HKV, int D, int max_seqlen_k, float sm_scale,
                                    int kpool, int pool_segment, float* out, int dtype, void* workspace,
                                    size_t workspace_bytes, cvllm_stream_t stream) {
+  return cvllm_snapkv_scores_bounded(q, k, q_stride_n, k_stride_n, cu_seqlens_q, cu_seqlens_k, w, B, 0x7fffffff, Nk, HQ, HKV, D,
+                                     max_seqlen_k, sm_scale, kpool, pool_segment, out, dtype, workspace, workspace_bytes, stream);
+}
+
+extern "C" int cvllm_snapkv_scores_bounded(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
+                                           const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int w, int B,
+                                           int Nq, int Nk, int HQ, int HKV, int D, int max_seqlen_k, float sm_scale,
+                                           int kpool, int pool_segment, float* out, int dtype, void* workspace,
+                                           size_t workspace_bytes, cvllm_stream_t stream) {
   CVLLM_CHECK_ARG(B > 0 && Nk >= 0 && HQ > 0 && HKV > 0 && w >= 0 && kpool >= 1 && max_seqlen_k >= 0);
   if (Nk == 0 || max_seqlen_k == 0) return CVLLM_OK;
-  CVLLM_CHECK_ARG(q && k && cu_seqlens_q && cu_seqlens_k && out && workspace);
+  CVLLM_CHECK_ARG(q && Nq > 0 && k && cu_seqlens_q && cu_seqlens_k && out && workspace);
   CVLLM_CHECK_ARG(HQ % HKV == 0 && (dtype == CVLLM_F16 || dtype == CVLLM_BF16));
   CVLLM_CHECK_SUPPORTED(D == 128);
   CVLLM_CHECK_SUPPORTED(pool_segment > 0 && kKeyTile % pool_segment == 0);
@@ -429,7 +438,7 @@ extern "C" int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_strid
     CVLLM_CHECK_CUDA(cudaMemsetAsync(out, 0, (size_t)Nk * HKV * sizeof(float), st));
     return CVLLM_OK;
   }
-  return cvllm_launch_snap_umma(q, k, q_stride_n, k_stride_n, cu_seqlens_q, cu_seqlens_k, w, B, Nk, HQ, HKV, max_seqlen_k,
+  return cvllm_launch_snap_umma(q, k, q_stride_n, k_stride_n, cu_seqlens_q, cu_seqlens_k, w, B, Nq, Nk, HQ, HKV, max_seqlen_k,
                                 sm_scale * 1.4426950408889634f, kpool, pool_segment, out, reinterpret_cast<float*>(workspace),
                                 dtype == CVLLM_BF16, st);
 }

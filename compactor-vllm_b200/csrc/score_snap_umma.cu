@@ -378,14 +378,13 @@ size_t cvllm_snap_umma_workspace_bytes(int B, int max_seqlen_k, int HKV) {
 }
 
 int cvllm_launch_snap_umma(const void* q, const void* k, int64_t q_stride_n, int64_t k_stride_n,
-                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nk, int HQ, int HKV,
+                           const int32_t* cu_q, const int32_t* cu_k, int w, int B, int Nq, int Nk, int HQ, int HKV,
                            int max_seqlen_k, float scale_log2, int kpool, int pool_segment, float* out, float* stats,
                            bool bf16, cudaStream_t st) {
   const int G = HQ / HKV;
   CUtensorMap tm_q, tm_k;
   const uint32_t boxq[3] = {64, (uint32_t)G, (uint32_t)w};
-  // the queries' number is not known here (theirs may be another packing than the keys'); a box ends with its sequence
-  const uint64_t dq[3] = {(uint64_t)sn::kHD, (uint64_t)HQ, (uint64_t)0x7fffffff};
+  const uint64_t dq[3] = {(uint64_t)sn::kHD, (uint64_t)HQ, (uint64_t)Nq};   // (their packing may be another than the keys')
   const uint64_t sq[2] = {(uint64_t)sn::kHD * 2, (uint64_t)q_stride_n * 2};
   int rc = make_tmap_16b(&tm_q, q, 3, dq, sq, boxq, bf16);
   if (rc) return rc;

@@ -405,7 +405,8 @@ int cvllm_chunk_attn_scores(const void* q, const void* k, int64_t q_stride_n,
  * last-w queries x G heads against keys [0, L-w), softmax over those keys,
  * column sums, causal `kpool`-tap mean pool inside `pool_segment`-key
  * segments (the reference's autotuned BLOCK_K, :160-168,253-262), window
- * keys <- +inf.  No logits scratch. */
+ * keys <- +inf.  No logits scratch.  _bounded: q has Nq rows; rows that cu_seqlens_q says lie past them count as zeros
+ * (without the bound they are read). */
 size_t cvllm_snapkv_scores_workspace_bytes(int B, int N, int HQ, int HKV, int w);
 int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_stride_n,
                         int64_t k_stride_n, const int32_t* cu_seqlens_q,
@@ -413,6 +414,12 @@ int cvllm_snapkv_scores(const void* q, const void* k, int64_t q_stride_n,
                         int HKV, int D, int max_seqlen_k, float sm_scale, int kpool,
                         int pool_segment, float* out, int dtype, void* workspace,
                         size_t workspace_bytes, cvllm_stream_t stream);
+int cvllm_snapkv_scores_bounded(const void* q, const void* k, int64_t q_stride_n,
+                                int64_t k_stride_n, const int32_t* cu_seqlens_q,
+                                const int32_t* cu_seqlens_k, int w, int B, int Nq, int Nk, int HQ,
+                                int HKV, int D, int max_seqlen_k, float sm_scale, int kpool,
+                                int pool_segment, float* out, int dtype, void* workspace,
+                                size_t workspace_bytes, cvllm_stream_t stream);
 
 /* Test entry: the fp64 symmetric eigensolver of the leverage chain alone (csrc/leverage_eig.cuh).
  * gram fp32 [mats,48,48]; lam_out fp64 [mats,48]; vec_out fp64 [mats,48,48] (columns = eigenvectors, any

@@ -56,6 +56,15 @@ def test_queries_packed_otherwise_than_keys(hq, hkv, w):
     assert torch.equal(out, query_aware_key_scores(tail, k, cu.to(DEV), cu.to(DEV), w).cpu())
 
 
+@pytest.mark.parametrize("hq,hkv,w", [(32, 8, 32), (16, 2, 32), (4, 4, 1)])
+def test_queries_past_the_end_count_as_zeros(hq, hkv, w):
+    lens, short = [300, 40, 1111], 5
+    q, k, _ = fused_qkv(sum(lens), hq, hkv, 128, torch.bfloat16, DEV, seed=7)
+    q[-short:] = 0
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    assert torch.equal(query_aware_key_scores(q[:-short], k, cu, cu, w), query_aware_key_scores(q, k, cu, cu, w))
+
+
 def test_no_window_scores_nothing():
     from compactor_vllm import _native as N
 
