@@ -1449,10 +1449,10 @@ struct DeltaTile {
 };
 
 // One token per sequence: the state's trip through the registers is the step.
+// (in functions of their own behind the kernels' wait: what is `const __restrict__` to a kernel may be read in front of it)
 template <typename T, int KS>
-__global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict__ qkv, const T* __restrict__ proj,
-                                                         DeltaArgs da, RecurArgs a) {
-  pdl_wait();   // scheduled beside the convolution's state update
+__device__ __forceinline__ void delta_step(const float* __restrict__ qkv, const T* __restrict__ proj, const DeltaArgs& da,
+                                           const RecurArgs& a) {
   namespace cg = cooperative_groups;
   constexpr int C = 4, DP = KS * kGlaRows;
   using Tile = DeltaTile<KS, C, 1>;
@@ -1506,6 +1506,11 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const float* __restrict
   tile_norm_rows<T>(a, so, sg, CP, part, part + 1, h, c0, ncol, t0, 1, 0);
   if (a.VT > 1) cg::this_cluster().sync();   // nobody leaves while its sums may still be read
 }
+template <typename T, int KS>
+__global__ void __launch_bounds__(512) delta_step_kernel(const float* qkv, const T* proj, const DeltaArgs da, const RecurArgs a) {
+  pdl_wait();   // scheduled beside the convolution's state update
+  delta_step<T, KS>(qkv, proj, da, a);
+}
 
 // Portions.  A cluster of VT CTAs serves one (head, sequence); each keeps CW value columns.  Warps have one of two roles:
 // `warps` main warps take the blocks through their state tiles; the others work for the stages (`tok` tokens) around the
@@ -1529,9 +1534,8 @@ constexpr int kDeltaHelpers = C == 2 ? 8 : 4;   // warps (four columns per threa
 constexpr int kDeltaMain = 8;                   // most main warps
 
 template <typename T, int KS, int C>
-__global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers<C>) * 32, 1)
-delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, DeltaArgs da, RecurArgs a) {
-  pdl_wait();   // scheduled beside the convolution's state update
+__device__ __forceinline__ void delta_scan(const float* __restrict__ qkv, const T* __restrict__ proj, const DeltaArgs& da,
+                                           const RecurArgs& a) {
   namespace cg = cooperative_groups;
   constexpr int U = kGlaBlock, DP = KS * kGlaRows, HW = kDeltaHelpers<C>;
   using Coef = DeltaCoef<U>;
@@ -1772,6 +1776,12 @@ delta_scan_kernel(const float* __restrict__ qkv, const T* __restrict__ proj, Del
     if (s <= stages) sync_all();
   }
   if (!helper && slot != a.reserved_slot) store_tile<KS, C>(S, a, slot, h, c0, col0, ncol, ks);
+}
+template <typename T, int KS, int C>
+__global__ void __launch_bounds__((kDeltaMain + kDeltaHelpers<C>) * 32, 1)
+delta_scan_kernel(const float* qkv, const T* proj, const DeltaArgs da, const RecurArgs a) {
+  pdl_wait();   // scheduled beside the convolution's state update
+  delta_scan<T, KS, C>(qkv, proj, da, a);
 }
 
 // How a (head, sequence) of the gated linear attention is laid out: KS key lanes, C columns per thread, `warps` warps per

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kLevThreads, 2) leverage_score_kernel(const Le
 
 // grid (n_chunks): z-score a chunk over all heads (compactor.py:224-269) and cast to the output dtype
 template <bool BF16>
-__global__ void __launch_bounds__(256) leverage_finalize_kernel(const float* __restrict__ raw,
+__global__ void __launch_bounds__(256) leverage_finalize_kernel(const float* raw,
                                                                 const int32_t* __restrict__ chunk_offsets,
                                                                 void* __restrict__ out, int HKV, int normalize) {
   pdl_wait();

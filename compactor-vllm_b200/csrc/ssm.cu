@@ -203,10 +203,9 @@ __global__ void __launch_bounds__(128) causal_conv_quads_kernel(const T* __restr
 
 // grid (B, channel tiles), 128 threads: a thread reads what it needs of its channel's old state, then writes the new.
 template <typename T>
-__global__ void __launch_bounds__(128) conv_state_update_kernel(const T* __restrict__ proj, int64_t p_stride,
+__global__ void __launch_bounds__(128) conv_state_update_kernel(const T* proj, int64_t p_stride,
                                                                 int x_off, int C, int taps,
-                                                                T* __restrict__ conv_state, StepGeom g,
-                                                                int reserved_slot) {
+                                                                T* conv_state, StepGeom g, int reserved_slot) {
   pdl_wait();      // scheduled beside the convolution, which reads what this writes
   pdl_trigger();   // the mixer's kernel may be scheduled
   const int b = blockIdx.x;
