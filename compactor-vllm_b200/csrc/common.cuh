@@ -116,24 +116,36 @@ int launch_decode_store(const void* key, const void* value, int64_t sk_b, int64_
 uint64_t launches();
 
 // ---------------------------------------------------------------------------
-// Programmatic dependent launch (a chain of short kernels on one stream): `launch_pdl` lets the NEXT kernel of the
-// stream be scheduled while this one is still running; a kernel launched that way calls `pdl_begin()` as its first
-// statement, which (a) allows ITS successor to be scheduled and (b) waits until every earlier kernel of the stream
-// has completed and its writes are visible.  Ordering and results are those of plain stream order.
-// OFF by default (test option "pdl" = 1 turns it on): measured on the selection chain it takes 15-19 us off the eager
-// chain run alone and nothing off its CUDA-graph replay, but INSIDE the prefill step — where every SM is held by an
-// attention CTA that uses all its shared memory and registers — the early-scheduled CTAs sit on SMs while they wait,
-// and the step gets 1-2 % slower (measured in alternation).  Without the attribute `pdl_begin()` is a no-op.
+// Programmatic dependent launch: a kernel that is scheduled while the one in front of it on the stream still runs.
+// Ordering and results are those of plain stream order.  Two forms:
+//
+// launch_behind + pdl_wait() / pdl_trigger(): always on.  The kernel may start once the threads of whatever is in front of it have
+// all called pdl_trigger() or ended (a kernel that never calls it just runs to its end).
+//   * It calls pdl_wait() in every CTA, also one that has nothing to do: a launch that ends first would let the next begin too early.
+//   * Before the wait it touches nothing that may be in an earlier kernel's hands, and what the kernel in front may have written is no
+//     `const __restrict__` parameter: the compiler may read those before the wait.  Two kernels read ahead all the same, because of
+//     what is in front of them:
+//     bias_decode_fold_kernel (the streaming kernel triggers only behind its own wait, so what lies further back has ended) and
+//     pass 2 of snap_umma_kernel (pass 1 is launched plainly).  Moving the streaming kernel's trigger above its wait, or
+//     launching pass 1 behind something, would break them.
+//   * It pays where a launch's start costs as much as its work (steps, short prompts, the last kernels of a chain), and not where its
+//     CTAs then come two to an SM (delta_chunk.cu).
+//   Inside the prefill step (attention on one stream, scores and eviction on another) the chains' overlapped launches neither help
+//   nor harm: overlapped / launched plainly, us, in alternation in one process: 4096 tokens 243.8 / 245.7, 8192 568 / 563,
+//   16384 2034 / 2012, 32768 7414 / 7449, where runs of one side spread by 1 to 2 %.  The chain alone in a graph: 4096 tokens
+//   134.7 / 137.0, 16384 201 / 201.
+//
+// launch_pdl + pdl_begin(): the selection chain of many short launches, off by default (test option "pdl" = 1).  pdl_begin(), the
+// kernel's first statement, lets its successor be scheduled and waits.  On, it takes 15-19 us off the eager chain run alone and
+// nothing off its CUDA-graph replay, but INSIDE the prefill step - where every SM is held by an attention CTA that uses all its
+// shared memory and registers - a dozen early-scheduled launches sit on SMs while they wait, and the step gets 1-2 % slower (measured
+// in alternation).  Without the attribute `pdl_begin()` is a no-op.
 // ---------------------------------------------------------------------------
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// The same for two launches that always belong together, whatever the option says: `launch_behind` schedules a kernel while the one
-// before it runs, once that one's threads have all called pdl_trigger() or ended.  The kernel calls pdl_wait() - in every CTA, also
-// one that has nothing to do: a launch that ends first would let the next one begin too early - before it touches what
-// earlier kernels write.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... KArgs, typename... Args>

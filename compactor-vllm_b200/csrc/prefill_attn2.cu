@@ -31,7 +31,8 @@
 // up to 3480 cached 526 -> 517, 1000 + 900 + 1100 + 400 53.3 -> 47.5, 4096 117.8 -> 113.7, twelve of 500 after up to 2400 176 -> 169.
 // Numbers that the compiler does not know to be the warp's own (an item read from shared memory) stay in vector registers and
 // cost the softmax loop 5 %: next_item passes them through a reduction (a shuffle helps less, 522 and 115.7 us above).
-// The launch is scheduled beside the kernel in front: eight prompts of 17 to 256 tokens back to back 12.3 -> 10.6 us.
+// The launch is scheduled beside the kernel in front where that one lets it, as another prefill does: eight prompts of 17 to 256 tokens
+// back to back 12.3 -> 10.6 us.  The rotation and the store of a layer do not; behind those it starts when they end.
 //
 // TMEM (512 columns): S0 [0,128)  S1 [128,256)  O0 [256,384)  O1 [384,512).
 #include <stdlib.h>
