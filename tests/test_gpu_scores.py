@@ -364,6 +364,8 @@ def _reference_arithmetic_on_device(keys, lens, phi, chunk, reg=5e-3):
 def test_leverage_layouts(lens, chunk):
     """Rows of a wider projection, a sketch matrix that is not on 16 bytes, tiles that end inside 16 and 8 rows, chunks of several
     tiles: the same bits as from plain tensors, and from the sketch's own rows where those are given."""
+    from compactor_vllm.layers.rotary_embedding import RotaryEmbedding
+
     n, H = sum(lens), 5
     wide = (_structured_keys(n, H + 2, 128, torch.float32, seed=n)).to(torch.bfloat16).to(DEV)
     keys = wide[:, 1:1 + H]
@@ -374,13 +376,17 @@ def test_leverage_layouts(lens, chunk):
     run = lambda k, f, **kw: approximate_leverage_scores(k, lens, f, normalize=False, chunk_size=chunk, **kw)  # noqa: E731
     want = run(keys.contiguous(), phi)
     assert torch.equal(run(keys, phi), want) and torch.equal(run(keys, odd), want)
-    rows = torch.matmul(keys.transpose(0, 1).contiguous().double(), phi.double()).transpose(0, 1)
-    near = run(None, phi, sketch_rows=rows.to(torch.bfloat16).contiguous())
-    assert want.isfinite().all() and near.isfinite().all()
-    if chunk:
-        ref = _reference_arithmetic_on_device(keys.contiguous(), lens, phi, chunk).float()
-        long = torch.cat([torch.full((x,), x >= 96, dtype=torch.bool) for x in osc.split_into_chunks(lens, chunk)[1]]).to(DEV)
-        assert not long.any() or ((want.float() - ref).abs() <= 2e-2 * ref.abs().clamp_min(1.0))[long].float().mean() >= 0.99
+    rope = RotaryEmbedding(128, 128, 8, 500000.0, None).to(DEV)
+    same = keys.contiguous()
+    _, _, rows = rope.forward_fused(torch.zeros(n, dtype=torch.int64, device=DEV), same, same.clone(), PHI=phi)
+    assert want.isfinite().all() and torch.equal(run(None, phi, sketch_rows=rows), want)
+    whole = chunk or max(lens)                              # 0: a chunk per sequence
+    chunks = osc.split_into_chunks(lens, whole)[1]
+    ref = _reference_arithmetic_on_device(keys.contiguous(), lens, phi, whole).float()
+    at = lambda which: torch.cat([torch.full((x,), which(x), dtype=torch.bool) for x in chunks]).to(DEV)  # noqa: E731
+    assert (want[at(lambda x: x == 1)] == 0).all()          # a single token is its own mean
+    long = at(lambda x: x >= 96)
+    assert not long.any() or ((want.float() - ref).abs() <= 2e-2 * ref.abs().clamp_min(1.0))[long].float().mean() >= 0.99
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])

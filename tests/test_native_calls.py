@@ -99,7 +99,9 @@ def test_decode_forms(monkeypatch, form, dtype):
         scale = 1
     run = lambda: head_sparse_decode_attention(q, kc, vc, lens, pt, bm, HKV, PS, scale)  # noqa: E731
     run()                                     # the workspace
-    got = run()
+    got, L = run(), N.lib()
+    short = L.call.decode_attention(L.decode_address, N._WORKSPACES, q, kc, vc, lens, pt, bm, HKV, PS, scale)
+    assert torch.equal(short, got) if form in ("plain", "default scale") else short is None
     with pytest.raises(AssertionError):
         head_sparse_decode_attention(q, kc, vc, lens, pt[:, :2].contiguous(), bm, HKV, PS, scale)
     with pytest.raises(AssertionError):
@@ -136,7 +138,10 @@ def test_prefill_forms(monkeypatch, form):
     call = lambda q=q, k=k, pt=pt: causal_sparse_varlen_with_cache(  # noqa: E731
         q, k, v, kc, vc, seq_lens_bh=past, global_page_table=pt, batch_mapping=bm, cu_seqlens_q=cu, max_seqlen_q=130,
         max_seqlen_k_cache=bound, HKV=HKV, PAGE_SIZE=PS, sm_scale=scale)
-    got = call()
+    got, L = call(), N.lib()
+    short = L.call.prefill_attention(L.prefill_address, q, k, v, kc, vc, past, pt, bm, cu, 130, bound, HKV, PS, scale)
+    served = ("plain", "views", "default scale", "bound of 64 bits")
+    assert torch.equal(short, got) if form in served else short is None
     with pytest.raises(AssertionError):
         call(k=k[:-1])
     with pytest.raises(AssertionError):
