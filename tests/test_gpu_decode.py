@@ -188,3 +188,48 @@ def test_decode_many_sequences(B, HQ, HKV):
         x = x.masked_fill(~there[:, :, None], -torch.inf).softmax(-1).nan_to_num(0.0)
         want = torch.einsum("bhgn,bhnd->bhgd", x, v).flatten(1, 2)
         assert (out[s].float() - want).abs().max().item() <= TOL[dtype]
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_decode_behind_another_stream(captured):
+    """The launch is scheduled beside the kernel in front of it: what it reads may come from another stream that was waited for just
+    before, or from a copy in front, and what follows may overwrite its inputs."""
+    dtype, B, HQ, HKV, D, PS = torch.bfloat16, 4, 32, 8, 128, 128
+    lens = torch.randint(1, 3000, (B, HKV), generator=torch.Generator().manual_seed(5))
+    kc, vc, pt, bm = make_paged(B, HKV, D, PS, lens.tolist(), dtype, DEV, seed=9)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    q = torch.randn((B, HQ, D), generator=g, device=DEV).to(dtype)
+    l = lens.to(torch.int32).to(DEV)
+    want = head_sparse_decode_attention(q, kc, vc, l, pt, bm, HKV, PS)
+    q_now, l_now, big = torch.zeros_like(q), torch.zeros_like(l), torch.randn((1 << 24,), device=DEV)
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def step():
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                big.mul_(1.0)               # the copies come late
+            q_now.copy_(q)
+            l_now.copy_(l)
+        first = head_sparse_decode_attention(q, kc, vc, l, pt, bm, HKV, PS)
+        main.wait_stream(side)
+        second = head_sparse_decode_attention(q_now, kc, vc, l_now, pt, bm, HKV, PS)
+        third = head_sparse_decode_attention(second.clone().copy_(q_now), kc, vc, l_now, pt, bm, HKV, PS)
+        q_now.zero_()
+        l_now.zero_()
+        return first, second, third
+
+    with torch.cuda.stream(main):
+        outs = step()
+        if captured:
+            main.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=main):
+                outs = step()
+            for o in outs:
+                o.zero_()
+            for _ in range(3):
+                graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
