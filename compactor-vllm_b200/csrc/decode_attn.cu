@@ -266,6 +266,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   float* s_merge = reinterpret_cast<float*>(bar_empty + kMaxSlots);   // [kDecWarps][G][ROW]
   int32_t* s_prefix = reinterpret_cast<int32_t*>(s_merge + kDecWarps * p.G * ROW);  // [BH + 1]
   int32_t* s_map = s_prefix + BH + 1;                                 // [B] batch_mapping, where there is room
+  // (as one pointer: chosen at every look-up, 16 x 10240 rows took 0.5 % longer)
+  const int32_t* slot_of = p.map_in_smem ? s_map : p.batch_mapping;
   __shared__ int32_t s_warp_tot[NW], s_warp_max[NW];
   __shared__ int s_near[2], s_last;
 
@@ -401,7 +403,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           const int pg = tok / p.PS;
           const int32_t* pt;
           if constexpr (BIAS) pt = p.page_table + p.batch_mapping[b] * p.pt_slot + h * p.pt_head;
-          else pt = p.page_table + ((int64_t)(p.map_in_smem ? s_map[b] : p.batch_mapping[b]) * p.HKV + h) * p.NLP;
+          else pt = p.page_table + ((int64_t)slot_of[b] * p.HKV + h) * p.NLP;
           row = pt[pg] * p.PS + (tok - pg * p.PS);
         }
       }
