@@ -661,7 +661,11 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
       for (int t = 0; t < MT; ++t)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[t][e] += __shfl_xor_sync(0xffffffffu, acc[t][e], 2);
+        for (int e = 0; e < 4; ++e) {
+          const float low = __shfl_xor_sync(0xffffffffu, acc[t][e], 2);
+          // the sum over an infinite value is infinite; its low part may be of the other sign, or 0 times infinity
+          if (BIAS || fabsf(acc[t][e]) < INFINITY) acc[t][e] += low;
+        }
     }
     {
       float* mw = s_merge + warp * G * ROW;

@@ -233,3 +233,22 @@ def test_decode_behind_another_stream(captured):
                 graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(o, want) for o in outs)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("HQ,HKV,rows", [(32, 8, 384), (16, 8, 130), (8, 1, 384), (32, 8, 6000)])     # whole heads; cut ones
+def test_decode_infinite_values(HQ, HKV, rows, dtype):
+    """An infinite value that a query sees makes its number infinite, not NaN, and leaves the others as they are."""
+    B, D, PS = 6, 128, 128
+    lens = torch.randint(rows // 2, rows + 1, (B, HKV), generator=torch.Generator().manual_seed(rows))
+    kc, vc, pt, bm = make_paged(B, HKV, D, PS, lens.tolist(), dtype, DEV, seed=rows)
+    g = torch.Generator(device=DEV).manual_seed(7)
+    q = (0.1 * torch.randn((B, HQ, D), generator=g, device=DEV)).to(dtype)
+    l = lens.to(torch.int32).to(DEV)
+    want = head_sparse_decode_attention(q, kc, vc, l, pt, bm, HKV, PS)
+    first = pt[bm.long(), :, 0].long().flatten() * PS
+    vc[first + 5, 3], vc[first + 9, 4] = torch.inf, -torch.inf
+    out = head_sparse_decode_attention(q, kc, vc, l, pt, bm, HKV, PS)
+    assert (out[..., 3] == torch.inf).all() and (out[..., 4] == -torch.inf).all()
+    rest = torch.arange(D, device=DEV).sub(3.5).abs() > 1
+    assert torch.equal(out[..., rest], want[..., rest])
