@@ -911,8 +911,8 @@ def main():
             g_gbs = comp_bytes / (comps["compress_graph_ms"] * 1e-3) / 1e9
             comps["roofline_compress"] = {"bound": "hbm", "achieved": g_gbs, "peak": pk["hbm"], "unit": "GB/s",
                                           "frac": g_gbs / pk["hbm"], "bytes": comp_bytes,
-                                          "note": "whole chain (22 launches, CUDA-graph replay): latency-bound by the "
-                                                  "eigensolver, not by bandwidth"}
+                                          "note": "whole chain (CUDA-graph replay): bound by latency (eigensolver, selection "
+                                                  "rounds), not by bandwidth"}
 
         # ---------------- the step in front of the path: fused q/k norm + sketch + RoPE ----------------
         try:
