@@ -33,6 +33,8 @@ def _run(seqs, new, past, pools, bound=None):
     # move their softmax reference point together (ragged tails against the oracle: test_gpu_prefill.py)
     ([640, 256, 128], [0, 600, 1], [(0, 1, 2), (1, 0, 2), (2, 1, 0)]),          # by pairs for the pasts, in three batch orders
     ([1280, 640, 128], [0, 2600, 1], [(0, 1, 2), (2, 0), (2, 1, 0), (1, 2)]),   # by pairs for the pasts; by tiles; pairs; one wave
+    ([1280, 640], [0, 100], [(0, 1), (0,), (1,)]),     # CTAs go on with other tiles; 160 CTAs, which don't; one wave
+    ([1280, 640], [2600, 0], [(0, 1), (0,)]),          # the same by pairs
     ([384] * 40, [0, 70] * 20, [tuple(range(40)), tuple(range(20)), tuple(range(20, 40))]),   # 1920 CTAs; 960
 ])
 def test_order_changes_nothing(dtype, new, past, calls):
